@@ -13,6 +13,7 @@ import torch  # noqa: F401  (loads libcudart.so.12 into the process)
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libarc_sdpa.so")
+BINDING_PATH = os.path.join(HERE, "_native.so")
 
 ARC_OK = 0
 ARC_ERR_BAD_SHAPE = 1
@@ -157,6 +158,25 @@ def load() -> C.CDLL:
     L.arc_sdpa_allgather_merge.argtypes = [vp, vp, C.c_int32, C.c_int32, C.c_int32, C.c_int32, vp, vp, vp, vp]
     _lib = L
     return L
+
+
+_native = None
+
+
+def native(workspace_of):
+    """The compiled tensor binding (``_native.so``, csrc/torch_binding.cpp), loaded once.
+    ``workspace_of(device index)`` gives it the default workspace of a device."""
+    global _native
+    if _native is None:
+        if not os.path.exists(BINDING_PATH):
+            raise RuntimeError(
+                f"{BINDING_PATH} is missing: build it with `python -m arcaine_b200.build` "
+                "(there is no CPU or PyTorch fallback for these operators)")
+        load()
+        from . import _native as module
+        module.setup(check, workspace_of)
+        _native = module
+    return _native
 
 
 class ArcError(RuntimeError):

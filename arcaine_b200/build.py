@@ -12,6 +12,7 @@ import subprocess
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libarc_sdpa.so")
+BINDING = os.path.join(HERE, "_native.so")
 BENCH_BIN = os.path.join(HERE, "arc_attention_bench")
 
 NVCC_FLAGS = [
@@ -35,7 +36,7 @@ def _stale(target: str, sources: list[str]) -> bool:
 
 
 def sources() -> list[str]:
-    out = [os.path.join(CSRC, f) for f in sorted(os.listdir(CSRC)) if f.endswith((".cu", ".cuh", ".hpp", ".cpp"))]
+    out = [os.path.join(CSRC, f) for f in sorted(os.listdir(CSRC)) if f.endswith((".cu", ".cuh", ".hpp", ".cpp")) and f != "torch_binding.cpp"]
     out.append(os.path.join(os.path.dirname(HERE), "include", "arc_sdpa.h"))
     return out
 
@@ -52,6 +53,27 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def build_binding(force: bool = False) -> str:
+    """Compile the torch tensor binding (``_native.so``) against the library and the torch in use."""
+    src = os.path.join(CSRC, "torch_binding.cpp")
+    header = os.path.join(os.path.dirname(HERE), "include", "arc_sdpa.h")
+    build_library()
+    if force or _stale(BINDING, [src, header]):
+        import sysconfig
+        import torch
+        from torch.utils import cpp_extension
+        lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+        cuda = os.path.dirname(os.path.dirname(_nvcc()))
+        subprocess.check_call([
+            shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", BINDING, src,
+            "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include"),
+            *("-isystem" + p for p in cpp_extension.include_paths()),
+            "-L" + HERE, "-larc_sdpa", "-Wl,-rpath,$ORIGIN", "-L" + lib, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch_python"])
+    return BINDING
+
+
 def build_attention_bench(force: bool = False) -> str:
     """Compile the kbench-style C++ program that drives the library through the
     reference-shaped C++ interface (``arcaine_attention.hpp``)."""
@@ -66,4 +88,5 @@ def build_attention_bench(force: bool = False) -> str:
 
 if __name__ == "__main__":
     print(build_library(force=True, verbose=True))
+    print(build_binding(force=True))
     print(build_attention_bench(force=True))
