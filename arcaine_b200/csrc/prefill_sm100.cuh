@@ -387,7 +387,9 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     const int cstep = CLUSTER ? (int)(gridDim.x / csize) : (int)gridDim.x;
     auto tile_of = [&](const TileCursor& c) { return CLUSTER ? decode_tile<HD>(p, c, csize, crank) : decode_tile<HD>(p, c); };
 
-    const int warp = threadIdx.x >> 5;
+    // (broadcast, so that the compiler knows them to be the same in every lane and keeps what follows from them —
+    // MMA descriptors above all — in uniform registers)
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     const long long rows_total = (long long)p.batch * p.seq * p.nq;
     const bool causal = (p.mask_type == 3);
@@ -435,7 +437,7 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     __syncthreads();
     tc_fence_after_sync();
     if constexpr (CLUSTER) cluster_sync_all();  // every CTA's barriers exist before anyone arrives on them
-    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
     // A call that finds a status word set does no work: every role walks an empty tile list and meets
     // the others at the end (in a cluster nobody may leave early anyway).
     const int total_tiles = *abort_slot ? 0 : p.total_tiles;
@@ -507,33 +509,32 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         // Per tile: the first NSB-1 score blocks; then for every block u:  S(u+NSB-1) into the
         // buffer P(u-1) just left (runs while the softmax warps work on S(u)), then
         // O += P(u) V(u) once P(u) is in tensor memory.  Counters run across tiles, so buffers,
-        // stages and barrier phases simply keep rotating.
-        if (lane == 0) {
+        // stages and barrier phases simply keep rotating.  The whole warp runs the code, one elected lane issues.
+        {
             constexpr uint32_t IDESC_QK = make_idesc_bf16(128, 128, false);
             constexpr uint32_t IDESC_PV = make_idesc_bf16(128, HD, true);
+            constexpr uint32_t TILE16 = C::TILE_BYTES >> 4, CHUNK16 = C::CHUNK_BYTES >> 4;  // descriptor units
             const uint32_t tO = tmem_base + C::COL_O;
-            const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
-            // Descriptors are built once; per MMA only the start-address field (bytes >> 4, low
-            // word) moves, so the issuing thread needs a handful of instructions per MMA.
-            const uint64_t dQ = make_smem_desc_sw128(aQ, 16, 1024);
-            const uint64_t dK = make_smem_desc_sw128(aK, 16, 1024);
-            const uint64_t dV = make_smem_desc_sw128(aV, C::CHUNK_BYTES, 1024);
-            int gs = 0, gp = 0, tc = 0;  // score blocks issued, P V blocks issued, non-empty tiles started
+            // Descriptors are built once; per MMA only the start-address field (bytes >> 4, low word) moves.
+            const uint64_t dQ = make_smem_desc_sw128(smem_u32(sQ), 16, 1024);
+            const uint64_t dK = make_smem_desc_sw128(smem_u32(sK), 16, 1024);
+            const uint64_t dV = make_smem_desc_sw128(smem_u32(sV), C::CHUNK_BYTES, 1024);
+            // score blocks issued, P V blocks issued, non-empty tiles started; ring positions of gs and gp
+            int gs = 0, gp = 0, tc = 0;
             auto issue_qk = [&]() -> bool {
-                if (!mbar_wait(&k_full[gs % KS], (gs / KS) & 1)) {
+                if (!mbar_wait_inline(&k_full[gs % KS], (gs / KS) & 1)) {
                     report_fault(p.fault, FAULT_WAIT_K, gs);
                     return false;
                 }
                 tc_fence_after_sync();
                 const uint32_t tS = tmem_base + C::COL_S + (gs % NSB) * 128;
-                const uint64_t dKu = dK + (uint64_t)(((gs % KS) * C::TILE_BYTES) >> 4);
-#pragma unroll
-                for (int kk = 0; kk < HD / 16; ++kk) {
-                    const uint32_t o = ((kk >> 2) * C::CHUNK_BYTES + (kk & 3) * 32) >> 4;
-                    umma_ss(tS, dQ + o, dKu + o, IDESC_QK, kk > 0 ? 1u : 0u);
-                }
-                umma_commit(&s_full[gs % NSB]);
-                umma_commit(&k_empty[gs % KS]);
+                uint64_t da = dQ, db = dK + (uint64_t)((gs % KS) * TILE16);
+                uint32_t acc = 0u;
+#pragma unroll 1
+                for (int c = 0; c < C::CH; ++c, da += CHUNK16, db += CHUNK16, acc = 1u)  // 64 head-dim columns a turn
+                    umma_ss_x4<2, 2>(tS, da, db, IDESC_QK, acc);
+                umma_commit_warp(&s_full[gs % NSB]);
+                umma_commit_warp(&k_empty[gs % KS]);
                 ++gs;
                 return true;
             };
@@ -542,51 +543,50 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
             for (cur.init(p, cfirst, cstep); ok && cur.w < total_tiles; cur.advance(p)) {
                 const TileWork tw = tile_of(cur);
                 if (tw.n_my == 0) continue;
-                if (!mbar_wait(q_full, tc & 1)) {
+                if (!mbar_wait_inline(q_full, tc & 1)) {
                     report_fault(p.fault, FAULT_WAIT_Q, tc);
                     break;
                 }
                 int issued = 0;  // score blocks of this tile issued so far
-                for (; ok && issued < NSB - 1 && issued < tw.n_my; ++issued) ok = issue_qk();
-                if (ok && issued == tw.n_my) umma_commit(q_empty);
-                for (int u = 0; ok && u < tw.n_my; ++u) {
+                // u < 0: the first scores; the loop is one so that the scores are issued from one place
+                for (int u = -(NSB - 1); ok && u < tw.n_my; ++u) {
                     if (issued < tw.n_my) {
                         ok = issue_qk();
                         if (!ok) break;
-                        if (++issued == tw.n_my) umma_commit(q_empty);
+                        if (++issued == tw.n_my) umma_commit_warp(q_empty);
                     }
-                    if (!mbar_wait(&p_full[gp % NSB], (gp / NSB) & 1)) {
-                        report_fault(p.fault, FAULT_WAIT_P, gp);
-                        ok = false;
-                        break;
-                    }
-                    if (!mbar_wait(&v_full[gp % VS], (gp / VS) & 1)) {
+                    if (u < 0) continue;
+                    // (P comes last: the others have long been there when it does)
+                    if (!mbar_wait_inline(&v_full[gp % VS], (gp / VS) & 1)) {
                         report_fault(p.fault, FAULT_WAIT_V, gp);
                         ok = false;
                         break;
                     }
-                    if (u == 0 && tc > 0 && !mbar_wait(o_empty, (tc - 1) & 1)) {
+                    if (u == 0 && tc > 0 && !mbar_wait_inline(o_empty, (tc - 1) & 1)) {
                         report_fault(p.fault, FAULT_WAIT_O, 0x100u + tc);
+                        ok = false;
+                        break;
+                    }
+                    if (!mbar_wait_inline(&p_full[gp % NSB], (gp / NSB) & 1)) {
+                        report_fault(p.fault, FAULT_WAIT_P, gp);
                         ok = false;
                         break;
                     }
                     tc_fence_after_sync();
                     // P from tensor memory: each 32-key chunk keeps its 16 bf16x2 columns at the start
-                    // of its own 32 score columns, so 16 keys = 8 columns at 32*(ks/2) + 8*(ks%2).  V is
+                    // of its own 32 score columns, so 32 keys are two MMAs 8 columns apart.  V is
                     // MN-major: 64-element head-dim chunks 16 KB apart (leading offset), 8-key groups
-                    // 1024 bytes apart (stride offset).
-                    const uint32_t tS = tmem_base + C::COL_S + (gp % NSB) * 128;
-                    const uint64_t dVu = dV + (uint64_t)(((gp % VS) * C::TILE_BYTES) >> 4);
-#pragma unroll
-                    for (int ks = 0; ks < C::BN / 16; ++ks) {
-                        umma_ts(tO, tS + (ks >> 1) * 32 + (ks & 1) * 8, dVu + (uint64_t)((ks * 2048) >> 4), IDESC_PV,
-                                (u > 0 || ks > 0) ? 1u : 0u);
-                    }
-                    umma_commit(&v_empty[gp % VS]);
-                    umma_commit(pv_done);
+                    // 1024 bytes apart (stride offset); 16 keys = 2048 bytes.
+                    uint32_t tP = tmem_base + C::COL_S + (gp % NSB) * 128, acc = u > 0 ? 1u : 0u;
+                    uint64_t dVu = dV + (uint64_t)((gp % VS) * TILE16);
+#pragma unroll 1
+                    for (int c = 0; c < C::BN / 32; ++c, tP += 32, dVu += 256, acc = 1u)
+                        umma_ts_x2<8, 128>(tO, tP, dVu, IDESC_PV, acc);
+                    umma_commit_warp(&v_empty[gp % VS]);
+                    umma_commit_warp(pv_done);
                     ++gp;
                 }
-                if (ok) umma_commit(o_full);
+                if (ok) umma_commit_warp(o_full);
                 ++tc;
             }
         }

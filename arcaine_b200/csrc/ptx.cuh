@@ -194,6 +194,16 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait<GROUP>(bar, parity));
 }
 
+// The same without the out-of-line loop, for a warp whose registers should not pass through a call (an MMA issuer).
+__device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity, long long limit_cycles = 2000000000LL) {
+    if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
+    const long long t0 = clock64();
+    do {
+        if (__all_sync(0xffffffffu, mbar_try_wait_hint(bar, parity, 200000u))) return true;
+    } while (clock64() - t0 < limit_cycles);
+    return false;
+}
+
 // ---------------------------------------------------------------------------
 // Thread-block clusters: rank, shared memory of the other CTAs (distributed shared memory) and
 // mbarriers across the cluster.  A CTA may only be read while it is alive: every CTA therefore
@@ -382,80 +392,64 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
         : "memory");
 }
 
-// Eight MMAs of one K = 128 slab in a single statement: the issuing thread spends eight issue
-// slots instead of eight rounds of address arithmetic, which matters because it shares an
-// instruction scheduler with busy softmax warps.  The first MMA accumulates only if asked to.
-__device__ __forceinline__ void umma_ss_x8(uint32_t d_tmem, const uint64_t (&a)[8], const uint64_t (&b)[8],
-                                           uint32_t idesc, uint32_t accumulate) {
+// Forms for a whole converged warp: every lane executes the statement with identical operands and one elected lane
+// issues.  The election belongs into the statement: with it the assembler keeps the descriptors in uniform registers,
+// where the instruction wants them (a branch or a predicate on the lane index costs ~50 clk per MMA instead).
+// Four MMAs of K = 16 each, operand addresses advancing by A_STEP / B_STEP; the first accumulates only if asked to.
+template <uint32_t A_STEP, uint32_t B_STEP>  // in descriptor units of 16 bytes
+__device__ __forceinline__ void umma_ss_x4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %18, 0;\n\t"
-        "setp.eq.b32 q, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %9, %17, p;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %2, %10, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %3, %11, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %4, %12, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %5, %13, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %6, %14, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %7, %15, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %8, %16, %17, q;\n\t}" ::"r"(d_tmem),
-        "l"(a[0]), "l"(a[1]), "l"(a[2]), "l"(a[3]), "l"(a[4]), "l"(a[5]), "l"(a[6]), "l"(a[7]), "l"(b[0]), "l"(b[1]),
-        "l"(b[2]), "l"(b[3]), "l"(b[4]), "l"(b[5]), "l"(b[6]), "l"(b[7]), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "add.s64 a, %1, %5;\n\tadd.s64 b, %2, %6;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+        "add.s64 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+        "add.s64 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
         : "memory");
 }
 
-// The same with the A operand in tensor memory.
-__device__ __forceinline__ void umma_ts_x8(uint32_t d_tmem, const uint32_t (&a)[8], const uint64_t (&b)[8],
-                                           uint32_t idesc, uint32_t accumulate) {
+// The same with A in tensor memory (A_STEP in columns).
+template <uint32_t A_STEP, uint32_t B_STEP>
+__device__ __forceinline__ void umma_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %18, 0;\n\t"
-        "setp.eq.b32 q, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %9, %17, p;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], %10, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%3], %11, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%4], %12, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%5], %13, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%6], %14, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%7], %15, %17, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%8], %16, %17, q;\n\t}" ::"r"(d_tmem),
-        "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "l"(b[0]), "l"(b[1]),
-        "l"(b[2]), "l"(b[3]), "l"(b[4]), "l"(b[5]), "l"(b[6]), "l"(b[7]), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "add.s32 a, %1, %5;\n\tadd.s64 b, %2, %6;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+        "add.s32 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+        "add.s32 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
         : "memory");
 }
 
-// Warp-uniform forms: every lane executes the statement with identical operands and only the
-// lane whose `leader` flag is set issues the instruction.  Keeping the surrounding address
-// arithmetic uniform across the warp lets it live in the uniform datapath, which matters when
-// the issuing warp shares its scheduler with busy warps.
-__device__ __forceinline__ void umma_ss_lead(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate, uint32_t leader) {
+// Two of them.
+template <uint32_t A_STEP, uint32_t B_STEP>
+__device__ __forceinline__ void umma_ts_x2(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "add.s32 a, %1, %5;\n\tadd.s64 b, %2, %6;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
         : "memory");
 }
 
-__device__ __forceinline__ void umma_ts_lead(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate, uint32_t leader) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit_lead(uint64_t* bar, uint32_t leader) {
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
-        "r"(leader)
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
         : "memory");
 }
 
