@@ -19,6 +19,7 @@
 #include "prefill_pair_sm100.cuh"
 #include "qkv_prepare_sm100.cuh"
 #include "prefill_sm100.cuh"
+#include "prefill_wide_sm100.cuh"
 
 namespace arc {
 
@@ -41,6 +42,7 @@ struct DeviceState {
     // [head dim 128 / 256][log2(cluster size)]: how many clusters of 2 or 4 CTAs of the cluster form of the
     // prefill kernel the device can hold at once (0: that size cannot be launched)
     int active_clusters[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    int wide_pairs = 0;  // CTA pairs of the head-dim-256 kernel the device holds at once
 };
 
 static DeviceState g_dev[kMaxDevices];
@@ -71,6 +73,25 @@ template <typename K>
 static cudaError_t opt_in_smem(K kernel, int bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
+
+// Configuration of a launch in thread-block clusters of `size` CTAs.
+struct ClusterLaunch {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    ClusterLaunch(int size, long long ctas, int threads, int smem, cudaStream_t stream) {
+        cfg.gridDim = dim3((unsigned)ctas);
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = (size_t)smem;
+        cfg.stream = stream;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)size;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    ClusterLaunch(const ClusterLaunch&) = delete;
+};
 
 // One-time set-up for the current device: status-word address, SM count, and the
 // dynamic shared memory opt-in of every kernel.
@@ -111,22 +132,24 @@ static int device_state(DeviceState** out) {
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<256, false, false, true>, PrefillCfg<256>::SMEM_BYTES));
             for (int hi = 0; hi < 2; ++hi) {
                 for (int cs = 2, lg = 1; cs <= 4; cs *= 2, ++lg) {
-                    cudaLaunchConfig_t cfg{};
-                    cfg.gridDim = dim3((unsigned)(s.sm_count / cs * cs));  // the answer is capped by the grid asked about
-                    cfg.blockDim = dim3(hi ? PrefillCfg<256>::THREADS : PrefillCfg<128>::THREADS);
-                    cfg.dynamicSmemBytes = hi ? PrefillCfg<256>::SMEM_BYTES : PrefillCfg<128>::SMEM_BYTES;
-                    cudaLaunchAttribute attr[1];
-                    attr[0].id = cudaLaunchAttributeClusterDimension;
-                    attr[0].val.clusterDim.x = (unsigned)cs;
-                    attr[0].val.clusterDim.y = 1;
-                    attr[0].val.clusterDim.z = 1;
-                    cfg.attrs = attr;
-                    cfg.numAttrs = 1;
+                    // (the answer is capped by the grid asked about)
+                    ClusterLaunch cl(cs, s.sm_count / cs * cs, hi ? PrefillCfg<256>::THREADS : PrefillCfg<128>::THREADS,
+                                     hi ? PrefillCfg<256>::SMEM_BYTES : PrefillCfg<128>::SMEM_BYTES, nullptr);
                     int n = 0;
-                    const cudaError_t e = hi ? cudaOccupancyMaxActiveClusters(&n, sdpa_prefill_kernel<256, false, false, true>, &cfg)
-                                             : cudaOccupancyMaxActiveClusters(&n, sdpa_prefill_kernel<128, false, false, true>, &cfg);
+                    const cudaError_t e = hi ? cudaOccupancyMaxActiveClusters(&n, sdpa_prefill_kernel<256, false, false, true>, &cl.cfg)
+                                             : cudaOccupancyMaxActiveClusters(&n, sdpa_prefill_kernel<128, false, false, true>, &cl.cfg);
                     if (e == cudaSuccess && n > 0) s.active_clusters[hi][lg] = n;
                     else cudaGetLastError();
+                }
+            }
+            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false>, WideCfg::SMEM_BYTES));
+            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true>, WideCfg::SMEM_BYTES));
+            {
+                ClusterLaunch cl(2, s.sm_count / 2 * 2, WideCfg::THREADS, WideCfg::SMEM_BYTES, nullptr);
+                ARC_CUDA(cudaOccupancyMaxActiveClusters(&s.wide_pairs, sdpa_prefill_wide_kernel<false>, &cl.cfg));
+                if (s.wide_pairs < 1) {
+                    std::snprintf(g_last_error, sizeof(g_last_error), "the device cannot hold a CTA pair of the prefill kernel");
+                    return ARC_ERR_CUDA;
                 }
             }
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1>, s.smem_optin - kDecodeStaticSmem));
@@ -165,13 +188,13 @@ static cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// (hd, heads, tokens, batch) view of a token-major bf16 tensor; box = 64 x 1 x 128 x 1, 128-byte swizzle.
+// (hd, heads, tokens, batch) view of a token-major bf16 tensor; box = 64 x 1 x box_rows x 1, 128-byte swizzle.
 static int make_tile_map(CUtensorMap* tm, const void* base, int hd, int heads, int tokens, int batch,
-                         int64_t stride_t, int64_t stride_b) {
+                         int64_t stride_t, int64_t stride_b, int box_rows = 128) {
     cuuint64_t dims[4] = {(cuuint64_t)hd, (cuuint64_t)heads, (cuuint64_t)tokens, (cuuint64_t)batch};
     cuuint64_t sb = (cuuint64_t)(batch > 1 ? stride_b : stride_t * (int64_t)tokens) * 2u;
     cuuint64_t strides[3] = {(cuuint64_t)hd * 2u, (cuuint64_t)stride_t * 2u, sb};
-    cuuint32_t box[4] = {64u, 1u, 128u, 1u};
+    cuuint32_t box[4] = {64u, 1u, (cuuint32_t)box_rows, 1u};
     cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
     CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -181,6 +204,16 @@ static int make_tile_map(CUtensorMap* tm, const void* base, int hd, int heads, i
         return ARC_ERR_CUDA;
     }
     return ARC_OK;
+}
+
+// Output and gate as the epilogue warps see them: boxes of 64 columns x 32 rows.
+static int make_out_maps(CUtensorMap* to, CUtensorMap* tg, const arc_sdpa_prefill_params* p) {
+    const int rc = make_tile_map(to, p->out, p->hd, p->nq, p->seq, p->batch, p->o_stride_t, p->o_stride_b, 32);
+    if (rc != ARC_OK || !p->gate) {
+        *tg = *to;
+        return rc;
+    }
+    return make_tile_map(tg, p->gate, p->hd, p->nq, p->seq, p->batch, p->o_stride_t, p->o_stride_b, 32);
 }
 
 // (nkv*hd, rows) view of a KV cache whose rows are `stride_t` elements apart;
@@ -272,7 +305,7 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const in
 template <int HD>
 static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& plan, DeviceState* ds,
                           cudaStream_t stream) {
-    CUtensorMap tq, tk, tv;
+    CUtensorMap tq, tk, tv, to, tg;
     int rc;
     if ((rc = make_tile_map(&tq, p->q, HD, p->nq, p->seq, p->batch, p->q_stride_t, p->q_stride_b)) != ARC_OK) return rc;
     if ((rc = make_tile_map(&tk, p->k, HD, p->nkv, p->kv_len, p->batch, p->k_stride_t, p->k_stride_b)) != ARC_OK) return rc;
@@ -349,13 +382,14 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
             const long long pair_units = cut_tail ? full_waves * sms : pair_tiles;
             kp.total_tiles = (int)pair_units;
             const unsigned ctas = (unsigned)(pair_units < ds->sm_count ? pair_units : ds->sm_count);
+            if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
             if (kp.n_copies > 0) {
-                if (kp.gate) sdpa_prefill_pair_kernel<true, true><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, kp);
-                else sdpa_prefill_pair_kernel<false, true><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, kp);
+                if (kp.gate) sdpa_prefill_pair_kernel<true, true><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, to, tg, kp);
+                else sdpa_prefill_pair_kernel<false, true><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, to, tg, kp);
             } else if (kp.gate) {
-                sdpa_prefill_pair_kernel<true, false><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, kp);
+                sdpa_prefill_pair_kernel<true, false><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, to, tg, kp);
             } else {
-                sdpa_prefill_pair_kernel<false, false><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, kp);
+                sdpa_prefill_pair_kernel<false, false><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, to, tg, kp);
             }
             g_launches.fetch_add(1, std::memory_order_relaxed);
             ARC_CUDA(cudaGetLastError());
@@ -378,6 +412,28 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         }
     }
 
+    // Head dim 256, whole tiles, no additive mask: pairs of CTAs (prefill_wide_sm100.cuh) take 2300-2500 clk per key block
+    // and pair of tiles where a CTA on its own takes 3700 per tile.
+    if (HD == 256 && plan.splits == 1 && plan.cluster == 0 && !(kp.mask_type == 1 && kp.mask != nullptr)) {
+        kp.head_pair = ((p->nq / p->nkv) & 1) == 0;
+        kp.cur_heads = kp.head_pair ? p->nq / 2 : p->nq;
+        kp.q_tiles = kp.head_pair ? plan.q_tiles : (p->seq + 255) / 256;
+        const long long units = (long long)kp.q_tiles * kp.cur_heads * p->batch;
+        if (units > 0x3fffffffLL) return ARC_ERR_TOO_LARGE;
+        kp.total_tiles = (int)units;
+        // Units differ in length only under a causal mask without a window; longest first then, unless the K and V
+        // that all heads and sequences together read would not stay in L2 (126 MB).
+        const bool windowed = p->window > 0 && p->window < p->kv_len;
+        kp.long_first = p->mask_type == ARC_MASK_CAUSAL && !windowed && units > ds->wide_pairs &&
+                        (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;
+        if ((rc = make_tile_map(&tk, p->k, HD, p->nkv, p->kv_len, p->batch, p->k_stride_t, p->k_stride_b, 64)) != ARC_OK) return rc;
+        if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
+        ClusterLaunch cl(2, 2 * (units < ds->wide_pairs ? units : ds->wide_pairs), WideCfg::THREADS, WideCfg::SMEM_BYTES, stream);
+        ARC_CUDA(cudaLaunchKernelEx(&cl.cfg, kp.gate ? sdpa_prefill_wide_kernel<true> : sdpa_prefill_wide_kernel<false>, tq, tk, tv, to, tg, kp));
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        return ARC_OK;
+    }
+
     kp.q_tiles = plan.q_tiles;
     kp.cur_heads = p->nq;
     kp.head_pair = 0;
@@ -390,19 +446,8 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         kp.total_tiles = (int)tiles;
         kp.num_splits = 1;
         const long long nclusters = tiles;  // the plan made sure that many are resident at once
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)(nclusters * plan.cluster));
-        cfg.blockDim = dim3(PrefillCfg<HD>::THREADS);
-        cfg.dynamicSmemBytes = PrefillCfg<HD>::SMEM_BYTES;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)plan.cluster;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        ARC_CUDA(cudaLaunchKernelEx(&cfg, sdpa_prefill_kernel<HD, false, false, true>, tq, tk, tv, kp));
+        ClusterLaunch cl(plan.cluster, nclusters * plan.cluster, PrefillCfg<HD>::THREADS, PrefillCfg<HD>::SMEM_BYTES, stream);
+        ARC_CUDA(cudaLaunchKernelEx(&cl.cfg, sdpa_prefill_kernel<HD, false, false, true>, tq, tk, tv, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
         return ARC_OK;
     }

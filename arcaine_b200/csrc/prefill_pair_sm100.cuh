@@ -52,10 +52,11 @@ struct PairCfg {
     static constexpr int COL_S = 0;    // + 128 * pipeline
     static constexpr int COL_O = 256;  // + 128 * pipeline
     // q_full[2] q_empty[2] k_full[KS] k_empty[KS] v_full[VS] v_empty[VS] then per pipeline:
-    // s_full p_half[2] o_full o_empty fin[2]
-    static constexpr int NUM_BARS = 4 + 2 * K_STAGES + 2 * V_STAGES + 14;
-    static constexpr int FIN_FLOATS = 2 * 2 * 128 * 2;  // [tile parity][pipeline][row] (row sum, row maximum)
-    static constexpr int SMEM_BYTES = (2 + K_STAGES + V_STAGES) * TILE_BYTES + NUM_BARS * 8 + 16 + FIN_FLOATS * 4 + 1024;
+    // s_full p_half[2] o_full o_empty fin[2]; then gate[4], one per epilogue warp
+    static constexpr int NUM_BARS = 4 + 2 * K_STAGES + 2 * V_STAGES + 18;
+    static constexpr int FIN_FLOATS = 2 * 2 * 128;  // [tile parity][pipeline][row] row sum
+    static constexpr int SMEM_BYTES = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 4 * 8192 + NUM_BARS * 8 + 16 + FIN_FLOATS * 4;  // (4 x 8 KB: output stage)
+    static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
     static constexpr int SOFTMAX_WARPS = 8;   // four per pipeline
     static constexpr int EPILOGUE_WARP = 8;   // four warps
     static constexpr int PRODUCER_WARP = 12;
@@ -164,6 +165,72 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&v)[32], uint32_t (&pk
     }
 }
 
+// Output of a 128-row tile through shared memory.  Thread = row, so a store of a thread's 16 bytes touches 32 lines per
+// warp instruction: written straight to global memory, a tile of 128 x 256 kept the accumulator and the load / store
+// unit busy for 9000 clk.  Instead a warp collects its 32 rows, 128 columns at a time, in 8 KB of shared memory (two
+// boxes of 64 columns, 128-byte swizzle: lanes of a quarter warp hit different banks) and hands them to TMA, whose
+// stores clip the rows past `seq`; the gate values come the same way, by TMA into the same buffer, and are replaced
+// by the products in place.
+constexpr int STAGE_WARP_BYTES = 8192;
+constexpr int STAGE_BYTES = 4 * STAGE_WARP_BYTES;  // four epilogue warps
+
+struct OutStage {
+    uint8_t* buf;        // this warp's 8 KB, 1024-byte aligned
+    uint64_t* gate_bar;  // this warp's
+    uint32_t gate_par;   // parity of the next gate load
+};
+
+// Begin 128 columns of the warp's 32 rows from (c0, h, t0, b) on: the buffer is free again; ask for the gate values.
+// Rows from p.seq on are the caller's to skip (t0 < seq).
+template <bool GATE>
+__device__ __forceinline__ void stage_begin(OutStage& s, const void* tm_gate, int lane, int c0, int h, int t0, int b) {
+    if (lane == 0) {
+        bulk_wait_read();
+        if (GATE) {
+            mbar_arrive_expect_tx(s.gate_bar, STAGE_WARP_BYTES);
+            for (int i = 0; i < 2; ++i) tma_load_4d(s.buf + i * 4096, tm_gate, s.gate_bar, c0 + i * 64, h, t0, b);
+        }
+    }
+    __syncwarp();
+}
+
+// Columns [32 c, 32 c + 32) of the round: the accumulator's values times `inv`, gated, as bf16 into the buffer (and
+// into w8 for the caller).
+template <bool GATE>
+__device__ __forceinline__ void stage_chunk(const OutStage& s, int lane, int c, const uint32_t (&acc)[32], float inv, uint32_t (&w8)[16]) {
+    const uint32_t row = smem_u32(s.buf) + (c >> 1) * 4096 + lane * 128;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t a = row + ((((c & 1) * 4 + i) ^ (lane & 7)) << 4);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            w8[4 * i + u] = pack_bf16x2(__uint_as_float(acc[8 * i + 2 * u]) * inv, __uint_as_float(acc[8 * i + 2 * u + 1]) * inv);
+        if (GATE) {
+            // bf16(attention) * sigmoid(gate): the rounding order of the two-launch form
+            uint32_t gw[4];
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(gw[0]), "=r"(gw[1]), "=r"(gw[2]), "=r"(gw[3]) : "r"(a));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t w = w8[4 * i + u];
+                const float a0 = __uint_as_float(w << 16), a1 = __uint_as_float(w & 0xffff0000u);
+                const float g0 = __uint_as_float(gw[u] << 16), g1 = __uint_as_float(gw[u] & 0xffff0000u);
+                w8[4 * i + u] = pack_bf16x2(a0 * (1.0f / (1.0f + __expf(-g0))), a1 * (1.0f / (1.0f + __expf(-g1))));
+            }
+        }
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(w8[4 * i]), "r"(w8[4 * i + 1]), "r"(w8[4 * i + 2]), "r"(w8[4 * i + 3]) : "memory");
+    }
+}
+
+// The round's 128 columns are in the buffer: send them off.
+__device__ __forceinline__ void stage_end(const OutStage& s, const void* tm_out, int lane, int c0, int h, int t0, int b) {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+        for (int i = 0; i < 2; ++i) tma_store_4d(tm_out, s.buf + i * 4096, c0 + i * 64, h, t0, b);
+        bulk_commit();
+    }
+}
+
 // One arrival for the warp, behind everything its lanes did before.
 __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
     __syncwarp();
@@ -175,17 +242,18 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
 template <bool GATE, bool COPIES>
 __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     sdpa_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                             const __grid_constant__ CUtensorMap tm_v, const PrefillParams p) {
+                             const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
+                             const __grid_constant__ CUtensorMap tm_gate, const PrefillParams p) {
     using C = PairCfg;
     constexpr int HD = C::HD;
     constexpr int KS = C::K_STAGES;
     constexpr int VS = C::V_STAGES;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) uint8_t smem[];  // (the swizzle pattern follows the address bits)
     uint8_t* sQ = smem;                       // [2] one per pipeline
     uint8_t* sK = smem + 2 * C::TILE_BYTES;   // [KS]
     uint8_t* sV = sK + KS * C::TILE_BYTES;    // [VS]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + VS * C::TILE_BYTES);
+    uint8_t* sOut = sV + VS * C::TILE_BYTES;  // output stage
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + STAGE_BYTES);
     uint64_t* q_full = bars;         // [2]
     uint64_t* q_empty = bars + 2;    // [2] the tile's last S = Q K^T has completed
     uint64_t* k_full = bars + 4;     // [KS]
@@ -196,16 +264,16 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     uint64_t* p_half = s_full + 2;   // [pipeline][half]: P of keys 0-63 / 64-127 of the block is in tensor memory
     uint64_t* o_full = p_half + 4;   // one phase per tile: the tile's last O += P V has completed
     uint64_t* o_empty = o_full + 2;  // one phase per tile: the epilogue warps have read O out
-    // fin[2 * s + (tile & 1)], one phase per second tile: the softmax warps have published the tile's row sums
-    // and maxima.  Two barriers per pipeline, used in turn, because a tile of one key block needs no
+    // fin[2 * s + (tile & 1)], one phase per second tile: the softmax warps have published the tile's row sums.  Two barriers per pipeline, used in turn, because a tile of one key block needs no
     // O += P V to finish: with one barrier the softmax warps could complete it for tile n + 1 while a slow
     // epilogue (stores held up) still waits for tile n's completion — and a parity wait cannot tell "twice"
     // from "not yet".  They cannot reach tile n + 2 before the epilogue has taken tile n (the first O += P V
     // of tile n + 1 waits for that), so two are enough.
     uint64_t* fin = o_empty + 2;
+    uint64_t* gate_bar = fin + 4;    // [epilogue warp]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
-    float2* fin_vals = reinterpret_cast<float2*>(tmem_slot + 4);  // [tile parity 2][pipeline 2][row 128] (row sum, row maximum)
+    float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [tile parity 2][pipeline 2][row 128] row sum
 
     grid_launch_dependents();  // a launch behind this one (the single-head tail of the unit list) may be scheduled as SMs free up
     // (broadcast, so that the compiler knows them to be the same in every lane and keeps what follows from them —
@@ -233,6 +301,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             mbar_init(&fin[2 * s], 4);
             mbar_init(&fin[2 * s + 1], 4);
         }
+        for (int w = 0; w < 4; ++w) mbar_init(&gate_bar[w], 1);
         for (int s = 0; s < KS; ++s) {
             mbar_init(&k_full[s], 1);
             mbar_init(&k_empty[s], 1);
@@ -487,16 +556,17 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
         int tq0 = 0, tq1 = 0;  // tiles with key blocks so far, per pipeline
         bool ok = true;
-        uint32_t wa[32];
+        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[quarter], 0u};
         TileCursor cur;
         for (cur.init(p); ok && cur.w < p.total_tiles; cur.advance(p)) {
             const PairWork pw = decode_pair(p, cur);
 #pragma unroll 1
             for (int s = 0; s < 2 && ok; ++s) {
-                const int t = pw.q0_of(s) + r;
+                const int t0 = pw.q0_of(s) + quarter * 32, t = t0 + lane, h = pw.h_of(s);
                 const bool store = pw.live_of(s) && t < p.seq;
-                const long long row = ((long long)pw.b * p.seq + t) * p.nq + pw.h_of(s);
-                const long long eoff = pw.b * p.o_stride_b + t * p.o_stride_t + (long long)pw.h_of(s) * HD;
+                const bool warp_store = pw.live_of(s) && t0 < p.seq;  // some row of the warp is stored
+                const long long row = ((long long)pw.b * p.seq + t) * p.nq + h;
+                const long long eoff = pw.b * p.o_stride_b + t * p.o_stride_t + (long long)h * HD;
                 if (pw.hi_of(s) == pw.lo_of(s)) {
                     // Nothing visible for this tile: zero output.
                     if (store) {
@@ -508,27 +578,34 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     }
                     continue;
                 }
+                if (warp_store) stage_begin<GATE>(stage, &tm_gate, lane, 0, h, t0, pw.b);
                 const int tq = s ? tq1 : tq0;
                 if (!mbar_wait_relaxed_warp<2>(&fin[2 * s + (tq & 1)], (tq >> 1) & 1)) {
                     report_fault(p.fault, FAULT_WAIT_FULL, 0x500u + s);
                     ok = false;
                     break;
                 }
-                const float2 fv = fin_vals[((tq & 1) * 2 + s) * 128 + r];
-                const float row_l = fv.x, row_m = fv.y;
+                const float row_l = fin_vals[((tq & 1) * 2 + s) * 128 + r];
                 if (!mbar_wait_relaxed_warp<2>(&o_full[s], tq & 1)) {
                     report_fault(p.fault, FAULT_WAIT_O, tq);
                     ok = false;
                     break;
                 }
+                if (GATE && warp_store) {
+                    if (!mbar_wait_relaxed_warp<2>(stage.gate_bar, stage.gate_par)) {
+                        report_fault(p.fault, FAULT_WAIT_FULL, 0x600u + s);
+                        ok = false;
+                        break;
+                    }
+                    stage.gate_par ^= 1u;
+                }
                 tc_fence_after_sync();
                 if (s) ++tq1; else ++tq0;
                 const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
                 const uint32_t tO = tmem_base + lane_sel + C::COL_O + s * 128;
-                uint16_t* dst = p.out + eoff;
-                const uint16_t* gp = GATE ? p.gate + eoff : nullptr;
 #pragma unroll 1
                 for (int c = 0; c < HD / 32; ++c) {
+                    uint32_t wa[32], w8[16];
                     tmem_ld32(tO + c * 32, wa);
                     tmem_wait_ld();
                     if (c + 1 == HD / 32) {
@@ -536,34 +613,21 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                         tc_fence_before_sync();
                         warp_arrive(&o_empty[s], lane);
                     }
-                    if (store) {
+                    if (warp_store) {
+                        stage_chunk<GATE>(stage, lane, c, wa, inv, w8);
+                        if (COPIES && store) {
+                            for (int k = 0; k < p.n_copies; ++k) {
+                                uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + eoff + c * 32);
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {  // 16 values = 32 bytes per round
-                            uint32_t w8[8];
-#pragma unroll
-                            for (int u = 0; u < 8; ++u)
-                                w8[u] = pack_bf16x2(__uint_as_float(wa[i * 16 + 2 * u]) * inv, __uint_as_float(wa[i * 16 + 2 * u + 1]) * inv);
-                            if (GATE) {
-                                // bf16(attention) * sigmoid(gate): the rounding order of the two-launch form
-                                const uint4 g0 = *reinterpret_cast<const uint4*>(gp + c * 32 + i * 16);
-                                const uint4 g1 = *reinterpret_cast<const uint4*>(gp + c * 32 + i * 16 + 8);
-                                const uint32_t gw[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-#pragma unroll
-                                for (int u = 0; u < 8; ++u) {
-                                    const float a0 = __uint_as_float(w8[u] << 16), a1 = __uint_as_float(w8[u] & 0xffff0000u);
-                                    const float g0f = __uint_as_float(gw[u] << 16), g1f = __uint_as_float(gw[u] & 0xffff0000u);
-                                    w8[u] = pack_bf16x2(a0 * (1.0f / (1.0f + __expf(-g0f))), a1 * (1.0f / (1.0f + __expf(-g1f))));
-                                }
+                                for (int i = 0; i < 4; ++i) d4[i] = make_uint4(w8[4 * i], w8[4 * i + 1], w8[4 * i + 2], w8[4 * i + 3]);
                             }
-                            store_bf16x16(dst + c * 32 + i * 16, w8);
-                            if (COPIES) store_copies_bf16x16(p.out_copies, p.n_copies, eoff + c * 32 + i * 16, w8);
                         }
                     }
                 }
-                if (store && p.out_lse)
-                    p.out_lse[row] = row_l > 0.f ? (row_m + fast_log2(row_l)) * 0.6931471805599453f : -CUDART_INF_F;
+                if (warp_store) stage_end(stage, &tm_out, lane, 0, h, t0, pw.b);
             }
         }
+        if (lane == 0) bulk_wait_read();  // the stage may go when its last rows have been read
     } else {
         // ------------------------------------------------------------------ softmax
         // Warps 0-3 serve tile A, warps 4-7 tile B; a thread owns one query row and takes its 128
@@ -678,9 +742,12 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 warp_arrive(&p_half[2 * s + 1], lane);
             }
             if (ok && hi > lo) {
-                // The tile's last key block is on its way: hand the row sum and maximum to the
-                // epilogue warps and go on with the next tile.
-                fin_vals[((tq & 1) * 2 + s) * 128 + r] = make_float2(l, m);
+                // The tile's last key block is on its way: hand the row sum to the epilogue warps and go on with
+                // the next tile.
+                fin_vals[((tq & 1) * 2 + s) * 128 + r] = l;
+                if (p.out_lse && pw.live_of(s) && t < p.seq)
+                    p.out_lse[((long long)pw.b * p.seq + t) * p.nq + pw.h_of(s)] =
+                        l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
                 warp_arrive(&fin[2 * s + (tq & 1)], lane);
                 ++tq;
             }

@@ -56,6 +56,7 @@ struct PrefillParams {
     // >= 0 (one-tile kernel): the launch covers the tail of a two-tile launch's unit list — tile w is head (w & 1)
     // of the head pair with unit index tail_base + (w >> 1), one tile per CTA; -1: the plain tile list
     int tail_base;
+    int long_first;  // prefill_wide_sm100.cuh: units in order of falling length
 };
 
 // One CTA per SM, persistent: it takes tiles (128 query tokens of one query head) round-robin

@@ -1,0 +1,523 @@
+// GQA flash-attention prefill kernel for sm_100a, head dim 256: a pair of CTAs works on 256 query rows together.
+//
+// What bounds head dim 256.  One key block of 128 keys costs a 128-row tile 2048 clk of the tensor pipe (16 MMAs of
+// 64 clk for S = Q K^T, 8 of 128 clk for O += P V) and 1024 clk of the ex2 unit; Q, one K and one V tile are 64 KB
+// each, so a CTA on its own has room for one stage of each and pulls 128 KB per block through L2: 64 bytes per clk
+// and SM at the tensor rate, more than L2 delivers to 148 SMs (the one-tile kernel takes 3700 clk per block).  The
+// MMAs of a CTA pair (cta_group::2, M = 256) take half of B from either CTA: each CTA loads 64 of the block's keys
+// for K and 128 of V's 256 columns — half the traffic, 32 KB stages, two of each.
+//
+// The pair's two tiles are the same 128 tokens of two query heads of one KV group (even group), else 256
+// consecutive tokens of one head.  Tensor memory per CTA: two score buffers of 128 columns, O 256 columns.  S(j+1)
+// is computed while the softmax warps work on S(j), so the tensor pipe only waits when a softmax takes longer than
+// 2048 clk.
+//
+// Warp roles of each CTA (320 threads, 200 registers): 0-3 softmax (one row per thread), 4-7 epilogue, 8 TMA producer
+// (its CTA's Q tile and halves of K and V), 9 MMA issuer (leader CTA only).  Full barriers live in the leader, which
+// expects the bytes of both CTAs; empty and score barriers are committed to both (commit with multicast — the loads
+// themselves use none).  The softmax and epilogue warps of both CTAs arrive on the leader's barriers.
+//
+// Masks, lazy rescaling, P over the scores, bounded waits and the status word are as in prefill_pair_sm100.cuh.
+#pragma once
+#include "prefill_pair_sm100.cuh"
+
+namespace arc {
+
+struct WideCfg {
+    static constexpr int HD = 256;
+    static constexpr int BM = 128;  // rows per CTA
+    static constexpr int BN = 128;  // keys per block
+    static constexpr int Q_BYTES = BM * HD * 2;
+    static constexpr int Q_CHUNK = 128 * 128;      // 128 rows x 64 columns
+    static constexpr int K_BYTES = BN / 2 * HD * 2;  // this CTA's 64 keys
+    static constexpr int K_CHUNK = 64 * 128;       // 64 keys x 64 columns
+    static constexpr int V_BYTES = BN * HD / 2 * 2;  // this CTA's 128 columns
+    static constexpr int V_CHUNK = 128 * 128;      // 128 keys x 64 columns
+    static constexpr int STAGES = 2;               // of K and of V
+    static constexpr int COL_S = 0;                // + 128 * buffer
+    static constexpr int COL_O = 256;
+    // q_full q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[2], gate[epilogue warp]
+    static constexpr int NUM_BARS = 2 + 8 + 2 + 4 + 4 + 4;
+    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 2 * 128 * 4;
+    static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
+    static constexpr int EPILOGUE_WARP = 4, PRODUCER_WARP = 8, ISSUER_WARP = 9;
+    static constexpr int THREADS = 320;
+};
+
+// One unit of the pair: this CTA's tile, and the key blocks [lo, hi) the pair walks (the union over both tiles).
+struct WideWork {
+    int q0, h, b, kvh, lo, hi;
+};
+
+__device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first, int q_last, int& lo, int& hi) {
+    const int off = p.kv_len - p.seq;
+    lo = 0;
+    hi = (p.kv_len + WideCfg::BN - 1) / WideCfg::BN;
+    if (p.mask_type == 3) {
+        q_last = min(q_last, p.seq - 1);
+        const int last_key = p.vis_hi ? p.vis_hi[q_last] - 1 : min(p.kv_len - 1, q_last + off);
+        hi = last_key >= 0 ? last_key / WideCfg::BN + 1 : 0;
+        if (p.window > 0 && p.window != 0x7fffffff) lo = max(0, q_first + off - p.window + 1) / WideCfg::BN;
+    }
+    if (hi < lo) hi = lo;
+}
+
+// Position of a CTA pair in the list of units.  Plain order: token tiles fastest, then heads, then sequences (pairs that
+// run side by side share K and V in L2).  long_first (causal without a window, several waves): the units with most key
+// blocks first, all heads of a token tile together, and every second wave in reverse order, so that the sums of a
+// pair's units are about equal.
+struct WideCursor {
+    int w, i, first, step;
+    __device__ __forceinline__ WideCursor(int first_, int step_) : w(first_), i(0), first(first_), step(step_) {}
+    __device__ __forceinline__ void advance(const PrefillParams& p) {
+        ++i;
+        w = i * step + (p.long_first && (i & 1) ? step - 1 - first : first);
+    }
+};
+
+__device__ __forceinline__ WideWork decode_wide(const PrefillParams& p, const WideCursor& cur, int rank) {
+    WideWork t;
+    int qt;
+    if (p.long_first) {
+        const int per = p.cur_heads * p.batch, rest = cur.w % per;
+        qt = p.q_tiles - 1 - cur.w / per;
+        t.h = rest % p.cur_heads;
+        t.b = rest / p.cur_heads;
+    } else {
+        const int rest = cur.w / p.q_tiles;
+        qt = cur.w % p.q_tiles;
+        t.h = rest % p.cur_heads;
+        t.b = rest / p.cur_heads;
+    }
+    const int rows = p.head_pair ? WideCfg::BM : 2 * WideCfg::BM;  // tokens of the unit
+    const int q0 = qt * rows;
+    wide_blocks(p, q0, q0 + rows - 1, t.lo, t.hi);
+    if (p.head_pair) {
+        t.h = t.h * 2 + rank;
+        t.q0 = q0;
+    } else {
+        t.q0 = q0 + rank * WideCfg::BM;
+    }
+    t.kvh = p.group_shift >= 0 ? (t.h >> p.group_shift) : t.h / p.group;
+    return t;
+}
+
+template <bool GATE>
+__global__ void __launch_bounds__(WideCfg::THREADS, 1)
+    sdpa_prefill_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                             const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
+                             const __grid_constant__ CUtensorMap tm_gate, const PrefillParams p) {
+    using C = WideCfg;
+    constexpr int HD = C::HD;
+    extern __shared__ __align__(1024) uint8_t smem[];  // (the swizzle pattern follows the address bits)
+    uint8_t* sQ = smem;
+    uint8_t* sK = sQ + C::Q_BYTES;               // [STAGES]
+    uint8_t* sV = sK + C::STAGES * C::K_BYTES;   // [STAGES]
+    uint8_t* sOut = sV + C::STAGES * C::V_BYTES;  // output stage
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + STAGE_BYTES);
+    uint64_t* q_full = bars;           // leader
+    uint64_t* q_empty = bars + 1;      // both: the tile's last S = Q K^T has completed
+    uint64_t* k_full = bars + 2;       // [2] leader
+    uint64_t* k_empty = bars + 4;      // [2] both
+    uint64_t* v_full = bars + 6;       // [2] leader
+    uint64_t* v_empty = bars + 8;      // [2] both
+    uint64_t* s_full = bars + 10;      // [2] both
+    uint64_t* p_half = bars + 12;      // [buffer][half] leader: eight warps' probabilities of keys 0-63 / 64-127
+    uint64_t* o_full = bars + 16;      // both: one phase per unit
+    uint64_t* o_empty = bars + 17;     // leader: eight epilogue warps have read O out
+    uint64_t* fin = bars + 18;         // [unit parity] own CTA: row sums are published
+    uint64_t* gate_bar = bars + 20;    // [epilogue warp] own CTA
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
+    uint32_t* abort_slot = tmem_slot + 1;
+    float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [unit parity][row] row sum
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    const int lane = threadIdx.x & 31;
+    const int rank = (int)cluster_ctarank();
+    const bool leader = rank == 0;
+
+    if (threadIdx.x == 32) {
+        prefetch_tensormap(&tm_q);
+        prefetch_tensormap(&tm_k);
+        prefetch_tensormap(&tm_v);
+    }
+    if (threadIdx.x == 0) {
+        const uint32_t fault_word = *reinterpret_cast<volatile uint32_t*>(p.fault);
+        mbar_init(q_full, 1);
+        mbar_init(q_empty, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&k_full[i], 1);
+            mbar_init(&k_empty[i], 1);
+            mbar_init(&v_full[i], 1);
+            mbar_init(&v_empty[i], 1);
+            mbar_init(&s_full[i], 1);
+            mbar_init(&p_half[2 * i], 8);
+            mbar_init(&p_half[2 * i + 1], 8);
+            mbar_init(&fin[i], 4);
+        }
+        for (int i = 0; i < 4; ++i) mbar_init(&gate_bar[i], 1);
+        mbar_init(o_full, 1);
+        mbar_init(o_empty, 8);
+        fence_mbar_init();
+        *abort_slot = fault_word != 0u ? 1u : 0u;
+    }
+    if (warp == C::PRODUCER_WARP) tmem_alloc_pair(tmem_slot, 512);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    cluster_sync_all();  // both CTAs' barriers exist before anyone arrives on the other's
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
+    const int total = *abort_slot ? 0 : p.total_tiles;  // a status is set: walk an empty list
+    const int first = (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
+
+    if (warp == C::PRODUCER_WARP) {
+        // ------------------------------------------------------------------ TMA producer
+        const uint32_t bq = map_to_cta(smem_u32(q_full), 0), bk = map_to_cta(smem_u32(k_full), 0), bv = map_to_cta(smem_u32(v_full), 0);
+        int gk = 0, gv = 0, n = 0;  // K blocks, V blocks and units loaded so far
+        bool ok = true;
+        auto load_k = [&](const WideWork& w, int j) {
+            const int st = gk & 1;
+            if (gk >= 2 && !mbar_wait_inline(&k_empty[st], ((gk >> 1) - 1) & 1)) {
+                if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x100u);
+                return false;
+            }
+            if (leader && lane == 0) mbar_arrive_expect_tx(&k_full[st], 2 * C::K_BYTES);
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                tma_load_4d_pair(sK + st * C::K_BYTES + c * C::K_CHUNK, &tm_k, bk + st * 8, c * 64, w.kvh, j * C::BN + rank * 64, w.b);
+            ++gk;
+            return true;
+        };
+        auto load_v = [&](const WideWork& w, int j) {
+            const int st = gv & 1;
+            if (gv >= 2 && !mbar_wait_inline(&v_empty[st], ((gv >> 1) - 1) & 1)) {
+                if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x200u);
+                return false;
+            }
+            if (leader && lane == 0) mbar_arrive_expect_tx(&v_full[st], 2 * C::V_BYTES);
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+                tma_load_4d_pair(sV + st * C::V_BYTES + c * C::V_CHUNK, &tm_v, bv + st * 8, rank * 128 + c * 64, w.kvh, j * C::BN, w.b);
+            ++gv;
+            return true;
+        };
+        WideCursor cur(first, step);
+        for (; ok && cur.w < total; cur.advance(p)) {
+            const WideWork w = decode_wide(p, cur, rank);
+            if (w.hi == w.lo) continue;
+            if (n > 0 && !mbar_wait_inline(q_empty, (n - 1) & 1)) {
+                if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u);
+                break;
+            }
+            if (leader && lane == 0) mbar_arrive_expect_tx(q_full, 2 * C::Q_BYTES);
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 4; ++c) tma_load_4d_pair(sQ + c * C::Q_CHUNK, &tm_q, bq, c * 64, w.h, w.q0, w.b);
+            ++n;
+            // in the order of use: K one block ahead of V
+            ok = load_k(w, w.lo);
+            for (int j = w.lo; ok && j < w.hi; ++j) {
+                if (j + 1 < w.hi) ok = load_k(w, j + 1);
+                if (ok) ok = load_v(w, j);
+            }
+        }
+    } else if (warp == C::ISSUER_WARP) {
+        // ------------------------------------------------------------------ MMA issuer (for both CTAs)
+        if (leader) {
+            constexpr uint32_t IDESC_QK = make_idesc_bf16(256, 128, false);
+            constexpr uint32_t IDESC_PV = make_idesc_bf16(256, 256, true);
+            const uint64_t dQ = make_smem_desc_sw128(smem_u32(sQ), 16, 1024);
+            const uint64_t dK = make_smem_desc_sw128(smem_u32(sK), 16, 1024);
+            const uint64_t dV = make_smem_desc_sw128(smem_u32(sV), C::V_CHUNK, 1024);
+            int gs = 0, gp = 0, nq = 0, no = 0;  // score blocks, P V blocks issued; units whose scores / P V have begun
+            bool ok = true;
+            // S(gs) of the unit's block j
+            auto scores = [&](const WideWork& w, int j) -> bool {
+                const int st = gs & 1;
+                if (j == w.lo) {
+                    if (!mbar_wait_inline(q_full, nq & 1)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_Q, nq);
+                        return false;
+                    }
+                    ++nq;
+                }
+                if (!mbar_wait_inline(&k_full[st], (gs >> 1) & 1)) {
+                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_K, gs);
+                    return false;
+                }
+                tc_fence_after_sync();
+                uint64_t da = dQ, db = dK + (uint64_t)(st * (C::K_BYTES >> 4));
+                uint32_t acc = 0u;
+#pragma unroll 1
+                for (int c = 0; c < 4; ++c, da += C::Q_CHUNK >> 4, db += C::K_CHUNK >> 4, acc = 1u)
+                    umma_pair_ss_x4<2, 2>(tmem_base + C::COL_S + st * 128, da, db, IDESC_QK, acc);
+                umma_commit_pair(&s_full[st]);
+                umma_commit_pair(&k_empty[st]);
+                if (j + 1 == w.hi) umma_commit_pair(q_empty);
+                ++gs;
+                return true;
+            };
+            WideCursor cur(first, step);
+            auto next_unit = [&](WideWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
+                for (; cur.w < total; cur.advance(p)) {
+                    w = decode_wide(p, cur, 0);
+                    if (w.hi > w.lo) {
+                        cur.advance(p);
+                        return true;
+                    }
+                }
+                return false;
+            };
+            WideWork w{}, wn{};
+            bool have = next_unit(w);
+            if (have) ok = scores(w, w.lo);
+            while (have && ok) {
+                const bool have_next = next_unit(wn);
+                for (int j = w.lo; j < w.hi; ++j) {
+                    // the next block's scores first: they run while the softmax warps work on this block's
+                    if (j + 1 < w.hi) ok = scores(w, j + 1);
+                    else if (have_next) ok = scores(wn, wn.lo);
+                    if (!ok) break;
+                    const int st = gp & 1;
+                    const uint32_t par = (gp >> 1) & 1;
+                    if (!mbar_wait_inline(&v_full[st], par)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_V, gp);
+                        ok = false;
+                        break;
+                    }
+                    if (j == w.lo) {
+                        if (no > 0 && !mbar_wait_inline(o_empty, (no - 1) & 1)) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x100u + no);
+                            ok = false;
+                            break;
+                        }
+                        ++no;
+                    }
+                    // P from tensor memory, 16 keys = 8 columns; V MN-major, 64-column chunks 16 KB apart, 16 keys =
+                    // 2048 bytes; the first 64 keys while the softmax warps still exponentiate the other 64
+                    uint32_t tP = tmem_base + C::COL_S + st * 128, acc = j > w.lo ? 1u : 0u;
+                    uint64_t dv = dV + (uint64_t)(st * (C::V_BYTES >> 4));
+#pragma unroll 1
+                    for (int half = 0; half < 2; ++half, tP += 32, dv += 512, acc = 1u) {
+                        if (!mbar_wait_inline(&p_half[2 * st + half], par)) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_P, gp);
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after_sync();
+                        umma_pair_ts_x4<8, 128>(tmem_base + C::COL_O, tP, dv, IDESC_PV, acc);
+                    }
+                    if (!ok) break;
+                    if (j + 1 == w.hi) umma_commit_pair(o_full);
+                    umma_commit_pair(&v_empty[st]);
+                    ++gp;
+                }
+                w = wn;
+                have = have_next;
+            }
+        }
+    } else if (warp >= C::EPILOGUE_WARP) {
+        // ------------------------------------------------------------------ epilogue: thread = query row
+        const int quarter = warp & 3;
+        const int r = quarter * 32 + lane;
+        const uint32_t tO = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::COL_O;
+        const uint32_t b_empty = map_to_cta(smem_u32(o_empty), 0);
+        int n = 0;  // units with key blocks so far
+        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[quarter], 0u};
+        WideCursor cur(first, step);
+        for (; cur.w < total; cur.advance(p)) {
+            const WideWork w = decode_wide(p, cur, rank);
+            const int t0 = w.q0 + quarter * 32, t = t0 + lane;
+            const bool store = t < p.seq, warp_store = t0 < p.seq;  // this row / some row of the warp is stored
+            const long long row = ((long long)w.b * p.seq + t) * p.nq + w.h;
+            const long long eoff = w.b * p.o_stride_b + t * p.o_stride_t + (long long)w.h * HD;
+            if (w.hi == w.lo) {  // nothing visible for the pair: zero output
+                if (store) {
+                    for (int c = -1; c < p.n_copies; ++c) {
+                        uint4* dst = reinterpret_cast<uint4*>((c < 0 ? p.out : reinterpret_cast<uint16_t*>(p.out_copies[c])) + eoff);
+                        for (int i = 0; i < HD / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                    if (p.out_lse) p.out_lse[row] = -CUDART_INF_F;
+                }
+                continue;
+            }
+            if (warp_store) stage_begin<GATE>(stage, &tm_gate, lane, 0, w.h, t0, w.b);
+            if (!mbar_wait_relaxed_warp<2>(&fin[n & 1], (n >> 1) & 1)) {
+                if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x500u);
+                break;
+            }
+            const float row_l = fin_vals[(n & 1) * 128 + r];
+            if (!mbar_wait_relaxed_warp<2>(o_full, n & 1)) {
+                if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, n);
+                break;
+            }
+            tc_fence_after_sync();
+            ++n;
+            const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
+            bool ok = true;
+#pragma unroll 1
+            for (int c = 0; c < HD / 32; ++c) {
+                uint32_t wa[32], w8[16];
+                if (warp_store && (c & 3) == 0) {
+                    if (c > 0) stage_begin<GATE>(stage, &tm_gate, lane, 128, w.h, t0, w.b);
+                    if (GATE) {
+                        if (!mbar_wait_relaxed_warp<2>(stage.gate_bar, stage.gate_par)) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x600u);
+                            ok = false;
+                            break;
+                        }
+                        stage.gate_par ^= 1u;
+                    }
+                }
+                tmem_ld32(tO + c * 32, wa);
+                tmem_wait_ld();
+                if (c + 1 == HD / 32) {  // O is in registers: the next unit may overwrite the accumulator
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_remote(b_empty);
+                }
+                if (warp_store) {
+                    stage_chunk<GATE>(stage, lane, c & 3, wa, inv, w8);
+                    if (store) {
+                        for (int k = 0; k < p.n_copies; ++k) {
+                            uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + eoff + c * 32);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) d4[i] = make_uint4(w8[4 * i], w8[4 * i + 1], w8[4 * i + 2], w8[4 * i + 3]);
+                        }
+                    }
+                    if ((c & 3) == 3) stage_end(stage, &tm_out, lane, (c >> 2) * 128, w.h, t0, w.b);
+                }
+            }
+            if (!ok) break;
+        }
+        if (lane == 0) bulk_wait_read();  // the stage may go when its last rows have been read
+    } else {
+        // ------------------------------------------------------------------ softmax: thread = query row
+        const int quarter = warp & 3;
+        const int r = quarter * 32 + lane;
+        const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
+        const uint32_t tO = tmem_base + lane_sel + C::COL_O;
+        const uint32_t b_half = map_to_cta(smem_u32(p_half), 0);
+        const float sl = p.scale_log2;
+        const uint64_t sl2 = pack_f32x2(sl, sl);
+        const bool causal = (p.mask_type == 3);
+        const bool windowed = causal && p.window > 0 && p.window != 0x7fffffff;
+        const int off = p.kv_len - p.seq;
+        int g = 0, n = 0;  // key blocks and units so far
+        bool ok = true;
+        uint32_t s0[32], s1[32], s2[32], s3[32];  // the row's 128 scores of the current block
+        WideCursor cur(first, step);
+        for (; ok && cur.w < total; cur.advance(p)) {
+            const WideWork w = decode_wide(p, cur, rank);
+            if (w.hi == w.lo) continue;
+            const int t = w.q0 + r;
+            int row_lo = 0, row_hi = p.kv_len;  // visible keys [row_lo, row_hi)
+            if (causal) {
+                const int diag = t + off;
+                row_hi = min(max(diag + 1, 0), p.kv_len);
+                if (p.vis_hi && t < p.seq) row_hi = p.vis_hi[t];  // a vision block's later keys are visible too
+                if (windowed) row_lo = max(0, diag - p.window + 1);
+                if (row_lo > row_hi) row_lo = row_hi;
+            }
+            const RowMask rm{row_lo, row_hi, p.kv_len, nullptr};
+            float m = -CUDART_INF_F;  // running max, log2 domain, possibly stale by <= 8
+            float l = 0.f;            // row sum
+            for (int j = w.lo; j < w.hi; ++j, ++g) {
+                const int kc = j * C::BN, st = g & 1;
+                const uint32_t tS = tmem_base + lane_sel + C::COL_S + st * 128;
+                if (!mbar_wait_inline(&s_full[st], (g >> 1) & 1)) {
+                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_S, g);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                tmem_ld32(tS, s0);
+                tmem_ld32(tS + 32, s1);
+                tmem_ld32(tS + 64, s2);
+                tmem_ld32(tS + 96, s3);
+                tmem_wait_ld();
+                if (!__all_sync(0xffffffffu, rm.lo <= kc && kc + C::BN <= rm.hi)) {  // window edge, diagonal, ragged end
+                    mask_chunk(s0, kc, rm);
+                    mask_chunk(s1, kc + 32, rm);
+                    mask_chunk(s2, kc + 64, rm);
+                    mask_chunk(s3, kc + 96, rm);
+                }
+                float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+                chunk_max<0>(s0, mr, sl, kc, rm);
+                chunk_max<0>(s1, mr, sl, kc, rm);
+                chunk_max<0>(s2, mr, sl, kc, rm);
+                chunk_max<0>(s3, mr, sl, kc, rm);
+                const float m_new = fmaxf(m, fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sl);
+                if (j == w.lo) {
+                    m = m_new;
+                } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
+                    // Rare: some row's maximum grows by more than 2^8.  Once O += P V of the previous block has landed
+                    // (it releases its V stage), rescale those rows of O in tensor memory.
+                    const bool need = m_new > m + 8.0f;
+                    const float alpha = need ? fast_exp2(m - m_new) : 1.0f;
+                    if (!mbar_wait_inline(&v_empty[st ^ 1], ((g - 1) >> 1) & 1)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x200u + g);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+#pragma unroll 1
+                    for (int c = 0; c < HD; c += 16) {
+                        uint32_t ww[16];
+                        tmem_ld16(tO + c, ww);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) ww[e] = __float_as_uint(__uint_as_float(ww[e]) * alpha);
+                        tmem_st16(tO + c, ww);
+                    }
+                    tmem_wait_st();
+                    l *= alpha;
+                    if (need) m = m_new;
+                }
+                // Probabilities as bf16, packed over the first 64 of the block's score columns; row sum in fp32.
+                // The first 64 keys are announced a chunk late: their stores have landed by then.
+                const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
+                const uint64_t nm2 = pack_f32x2(-m_eff, -m_eff);
+                uint64_t ls2[2] = {0ull, 0ull};
+                uint32_t pk[16];
+                exp_chunk(s0, pk, ls2, sl2, nm2);
+                tmem_st16(tS, pk);
+                exp_chunk(s1, pk, ls2, sl2, nm2);
+                tmem_st16(tS + 16, pk);
+                exp_chunk(s2, pk, ls2, sl2, nm2);
+                tmem_wait_st();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_remote(b_half + 16 * st);
+                tmem_st16(tS + 32, pk);
+                exp_chunk(s3, pk, ls2, sl2, nm2);
+                tmem_st16(tS + 48, pk);
+                float l0, l1, l2, l3;
+                unpack_f32x2(ls2[0], l0, l1);
+                unpack_f32x2(ls2[1], l2, l3);
+                l += (l0 + l1) + (l2 + l3);
+                tmem_wait_st();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_remote(b_half + 16 * st + 8);
+            }
+            if (ok) {
+                fin_vals[(n & 1) * 128 + r] = l;
+                if (p.out_lse && t < p.seq)
+                    p.out_lse[((long long)w.b * p.seq + t) * p.nq + w.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
+                warp_arrive(&fin[n & 1], lane);
+                ++n;
+            }
+        }
+    }
+
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync_all();  // neither CTA's barriers or tensor memory go before the other is through with them
+    if (warp == C::PRODUCER_WARP) tmem_dealloc_pair(tmem_base, 512);
+}
+
+}  // namespace arc

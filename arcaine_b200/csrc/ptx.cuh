@@ -256,6 +256,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
 }
 
+// The same without release at cluster scope, for arrivals that announce tensor-memory accesses only (completed by
+// tcgen05.wait and ordered by tcgen05.fence): the release costs the arriving warp about 600 clk.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+}
+
 // Bounded wait on a local mbarrier whose arrivals come from the whole cluster (acquire at cluster scope).
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, long long limit_cycles = 2000000000LL) {
     const long long t0 = clock64();
@@ -299,6 +305,20 @@ __device__ __forceinline__ void tma_prefetch_4d(const void* tmap, int c0, int c1
                  "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                  : "memory");
 }
+
+// Tile of shared memory to global memory (same swizzle as the loads; rows past the tensor's end are not written), in
+// the issuing thread's current bulk group.  The generic-proxy writes to the tile need fence_proxy_async_smem() first.
+__device__ __forceinline__ void tma_store_4d(const void* tmap, const void* smem_src, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
+                     reinterpret_cast<uint64_t>(tmap)),
+                 "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+                 : "memory");
+}
+
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+
+// Every bulk group of this thread has read its shared memory.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
 // 2-D tiled load (c0 innermost, multiple of 8 elements for 16-bit data).
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1) {
@@ -485,6 +505,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -504,6 +535,76 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
         "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// tcgen05 on a CTA pair (cta_group::2): two CTAs of a cluster of two hold 128 rows of D (and of A) each, and half of
+// B each; one thread of the leader CTA (rank 0) issues for both.  Allocation and release are done by one warp of each.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
+// Four MMAs of K = 16 each, as umma_ss_x4 / umma_ts_x4, for the pair.
+template <uint32_t A_STEP, uint32_t B_STEP>
+__device__ __forceinline__ void umma_pair_ss_x4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "add.s64 a, %1, %5;\n\tadd.s64 b, %2, %6;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t"
+        "add.s64 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t"
+        "add.s64 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
+        : "memory");
+}
+
+template <uint32_t A_STEP, uint32_t B_STEP>
+__device__ __forceinline__ void umma_pair_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "add.s32 a, %1, %5;\n\tadd.s64 b, %2, %6;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a], b, %3, t;\n\t"
+        "add.s32 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a], b, %3, t;\n\t"
+        "add.s32 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a], b, %3, t;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
+        : "memory");
+}
+
+// Arrive on the mbarrier at this address in BOTH CTAs once every MMA issued so far by this thread has completed.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b16 m;\n\tmov.b16 m, 3;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(
+            smem_u32(bar))
+        : "memory");
+}
+
+// TMA load into this CTA's shared memory whose bytes are counted on an mbarrier of the pair's leader (`bar`: cluster
+// address from map_to_cta).  Whole warp, one lane issues.
+__device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const void* tmap, uint32_t bar, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}" ::"r"(smem_u32(smem_dst)),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
 
