@@ -51,9 +51,9 @@ struct PairCfg {
     static constexpr int TMEM_COLS = 512;
     static constexpr int COL_S = 0;    // + 128 * pipeline
     static constexpr int COL_O = 256;  // + 128 * pipeline
-    // q_full[2] q_empty[2] k_full[KS] k_empty[KS] v_full[VS] v_empty[VS] then per pipeline:
-    // s_full p_half[2] o_full o_empty fin[2]; then gate[4], one per epilogue warp
-    static constexpr int NUM_BARS = 4 + 2 * K_STAGES + 2 * V_STAGES + 18;
+    // q_full[2] q_empty[2] k_first kv_full[2] kv_empty[2] then per pipeline:
+    // s_full p_part[2] o_full o_empty fin[2]; then gate[4], one per epilogue warp
+    static constexpr int NUM_BARS = 4 + 1 + 2 * K_STAGES + 18;
     static constexpr int FIN_FLOATS = 2 * 2 * 128;  // [tile parity][pipeline][row] row sum
     static constexpr int SMEM_BYTES = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 4 * 8192 + NUM_BARS * 8 + 16 + FIN_FLOATS * 4;  // (4 x 8 KB: output stage)
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
@@ -151,12 +151,13 @@ __device__ __forceinline__ void mask_chunk(uint32_t (&v)[32], int key0, const Ro
     for (int e = 0; e < 32; ++e) v[e] = (vis >> e) & 1u ? v[e] : 0xff800000u;
 }
 
-// 2^(score * scale - max) of one chunk, packed to bf16x2, added up in two pairs of partial sums.  Packed fp32
+// 2^(score * scale - max) of one chunk (or of its columns [E0, E1)), packed to bf16x2, added up in two pairs of partial sums.  Packed fp32
 // arithmetic: the pipe time is that of the scalar forms, the code is half as long.
+template <int E0 = 0, int E1 = 32>
 __device__ __forceinline__ void exp_chunk(const uint32_t (&v)[32], uint32_t (&pk)[16], uint64_t (&ls2)[2], uint64_t sl2,
                                           uint64_t nm2) {
 #pragma unroll
-    for (int e = 0; e < 32; e += 2) {
+    for (int e = E0; e < E1; e += 2) {
         float x0, x1;
         unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), sl2, nm2), x0, x1);
         const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
@@ -231,12 +232,6 @@ __device__ __forceinline__ void stage_end(const OutStage& s, const void* tm_out,
     }
 }
 
-// One arrival for the warp, behind everything its lanes did before.
-__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bar);
-}
-
 // The gated epilogue and the one that also stores copies of the output are instances of their own: code the
 // common kernel does not carry.
 template <bool GATE, bool COPIES>
@@ -256,13 +251,12 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + STAGE_BYTES);
     uint64_t* q_full = bars;         // [2]
     uint64_t* q_empty = bars + 2;    // [2] the tile's last S = Q K^T has completed
-    uint64_t* k_full = bars + 4;     // [KS]
-    uint64_t* k_empty = k_full + KS; // [KS]
-    uint64_t* v_full = k_empty + KS;
-    uint64_t* v_empty = v_full + VS; // [VS]
-    uint64_t* s_full = v_empty + VS; // [2] per pipeline from here on
-    uint64_t* p_half = s_full + 2;   // [pipeline][half]: P of keys 0-63 / 64-127 of the block is in tensor memory
-    uint64_t* o_full = p_half + 4;   // one phase per tile: the tile's last O += P V has completed
+    uint64_t* k_first = bars + 4;    // the first key block's K
+    uint64_t* kv_full = bars + 5;    // [2] V of a block and K of the block after it
+    uint64_t* kv_empty = bars + 7;   // [2] both have been used by both pipelines
+    uint64_t* s_full = kv_empty + 2; // [2] per pipeline from here on
+    uint64_t* p_part = s_full + 2;   // [pipeline][part]: P of keys 0-95 / 96-127 of the block is in tensor memory
+    uint64_t* o_full = p_part + 4;   // one phase per tile: the tile's last O += P V has completed
     uint64_t* o_empty = o_full + 2;  // one phase per tile: the epilogue warps have read O out
     // fin[2 * s + (tile & 1)], one phase per second tile: the softmax warps have published the tile's row sums.  Two barriers per pipeline, used in turn, because a tile of one key block needs no
     // O += P V to finish: with one barrier the softmax warps could complete it for tile n + 1 while a slow
@@ -294,21 +288,18 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             mbar_init(&q_full[s], 1);
             mbar_init(&q_empty[s], 1);
             mbar_init(&s_full[s], 1);
-            mbar_init(&p_half[2 * s], 4);
-            mbar_init(&p_half[2 * s + 1], 4);
+            mbar_init(&p_part[2 * s], 4);
+            mbar_init(&p_part[2 * s + 1], 4);
             mbar_init(&o_full[s], 1);
             mbar_init(&o_empty[s], 4);
             mbar_init(&fin[2 * s], 4);
             mbar_init(&fin[2 * s + 1], 4);
         }
         for (int w = 0; w < 4; ++w) mbar_init(&gate_bar[w], 1);
-        for (int s = 0; s < KS; ++s) {
-            mbar_init(&k_full[s], 1);
-            mbar_init(&k_empty[s], 1);
-        }
-        for (int s = 0; s < VS; ++s) {
-            mbar_init(&v_full[s], 1);
-            mbar_init(&v_empty[s], 1);
+        mbar_init(k_first, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&kv_full[s], 1);
+            mbar_init(&kv_empty[s], 1);
         }
         fence_mbar_init();
         *abort_slot = fault_word != 0u ? 1u : 0u;
@@ -328,48 +319,55 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         reg_dealloc<C::REGS_CONTROL>();
         if (warp == C::PRODUCER_WARP) {
             // -------------------------------------------------------------- TMA producer of K and V
-            if (lane == 0) {
-                prefetch_tensormap(&tm_k);
-                prefetch_tensormap(&tm_v);
-                int gk = 0, gv = 0;        // key blocks loaded into each ring so far
-                bool ok = true;
-                TileCursor cur;
-                for (cur.init(p); ok && cur.w < p.total_tiles; cur.advance(p)) {
-                    const PairWork pw = decode_pair(p, cur);
-                    // K stays at most two blocks ahead of V; both rings fill in the order of use.
-                    const int n = pw.uhi - pw.ulo;
-                    int uk = 0, uv = 0;
-                    while (ok && (uk < n || uv < n)) {
-                        if (uk < n && (uk <= uv + 1 || uv >= n)) {
-                            const int st = gk % KS;
-                            if (gk >= KS && !mbar_wait<1>(&k_empty[st], ((gk / KS) - 1) & 1)) {
-                                report_fault(p.fault, FAULT_WAIT_EMPTY, 0x100u);
-                                ok = false;
-                                break;
-                            }
-                            mbar_arrive_expect_tx(&k_full[st], C::TILE_BYTES);
+            // One stage holds what one step of the issuer takes: V of a key block and K of the block after it — in
+            // the next unit, if the block is a unit's last.  K of the very first block comes on its own.
+            int r = 0;  // ring position: key blocks whose K has been requested
+            bool ok = true;
+            auto load = [&](uint8_t* dst, const void* tm, uint64_t* bar, const PairWork& pw, int j) {
 #pragma unroll
-                            for (int c = 0; c < C::CH; ++c)
-                                tma_load_4d(sK + st * C::TILE_BYTES + c * C::CHUNK_BYTES, &tm_k, &k_full[st], c * 64, pw.kvh,
-                                            (pw.ulo + uk) * C::BN, pw.b);
-                            ++uk;
-                            ++gk;
-                        } else {
-                            const int st = gv % VS;
-                            if (gv >= VS && !mbar_wait<1>(&v_empty[st], ((gv / VS) - 1) & 1)) {
-                                report_fault(p.fault, FAULT_WAIT_EMPTY, 0x200u);
-                                ok = false;
-                                break;
-                            }
-                            mbar_arrive_expect_tx(&v_full[st], C::TILE_BYTES);
-#pragma unroll
-                            for (int c = 0; c < C::CH; ++c)
-                                tma_load_4d(sV + st * C::TILE_BYTES + c * C::CHUNK_BYTES, &tm_v, &v_full[st], c * 64, pw.kvh,
-                                            (pw.ulo + uv) * C::BN, pw.b);
-                            ++uv;
-                            ++gv;
+                for (int c = 0; c < C::CH; ++c)
+                    tma_load_4d_warp(dst + c * C::CHUNK_BYTES, tm, bar, c * 64, pw.kvh, j * C::BN, pw.b);
+            };
+            TileCursor cur;
+            PairWork last{};  // unit and index of the block requested last
+            int last_j = 0;
+            for (cur.init(p); ok && cur.w < p.total_tiles; cur.advance(p)) {
+                const PairWork pw = decode_pair(p, cur);
+                for (int j = pw.ulo; ok && j < pw.uhi; ++j, ++r) {
+                    if (r == 0) {
+                        if (lane == 0) mbar_arrive_expect_tx(k_first, C::TILE_BYTES);
+                        __syncwarp();
+                        load(sK, &tm_k, k_first, pw, j);
+                    } else {
+                        // V of block r - 1 and K of block r; both stages were used by step r - 3 (the first K by the
+                        // scores in front of all steps: its barrier's second phase — and the first one, or the wait
+                        // for the second would pass before the first has completed)
+                        uint64_t* full = &kv_full[(r - 1) & 1];
+                        const bool free = r < 2    ? true
+                                          : r == 2 ? mbar_wait_inline(k_first, 0u) && mbar_wait_inline(k_first, 1u)
+                                                   : mbar_wait_inline(&kv_empty[(r - 1) & 1], (((r - 1) >> 1) - 1) & 1);
+                        if (!free) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x100u);
+                            ok = false;
+                            break;
                         }
+                        if (lane == 0) mbar_arrive_expect_tx(full, 2 * C::TILE_BYTES);
+                        __syncwarp();
+                        load(sV + ((r - 1) & 1) * C::TILE_BYTES, &tm_v, full, last, last_j);
+                        load(sK + (r & 1) * C::TILE_BYTES, &tm_k, full, pw, j);
                     }
+                    last = pw;
+                    last_j = j;
+                }
+            }
+            if (ok && r > 0) {  // V of the last block of all
+                uint64_t* full = &kv_full[(r - 1) & 1];
+                if (r >= 3 && !mbar_wait_inline(&kv_empty[(r - 1) & 1], (((r - 1) >> 1) - 1) & 1)) {
+                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x200u);
+                } else {
+                    if (lane == 0) mbar_arrive_expect_tx(full, C::TILE_BYTES);
+                    __syncwarp();
+                    load(sV + ((r - 1) & 1) * C::TILE_BYTES, &tm_v, full, last, last_j);
                 }
             }
         } else if (warp == C::Q_PRODUCER_WARP) {
@@ -440,23 +438,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             uint32_t q_par = 0u;   // bit s: parity of its tiles whose first scores have been issued
             uint32_t o_par = 3u;   // bit s: parity to wait for before its next tile's first P V (starts "complete")
             bool ok = true;
-            // K (and Q for a tile's first block) of pipeline s's block j at ring position r.
-            auto await_scores = [&](const PairWork& pw, int s, int j, int r) -> bool {
-                if (!mbar_wait_inline(&k_full[r & 1], (r >> 1) & 1)) {
-                    report_fault(p.fault, FAULT_WAIT_K, r);
-                    return false;
-                }
-                if (j == pw.lo_of(s) && j < pw.hi_of(s)) {
-                    if (!mbar_wait_inline(&q_full[s], (q_par >> s) & 1u)) {
-                        report_fault(p.fault, FAULT_WAIT_Q, s);
-                        return false;
-                    }
-                    q_par ^= 1u << s;
-                }
-                return true;
-            };
-            // S = Q K(j)^T of pipeline s (a block the pipeline does not use: nothing); the second pipeline's turn
-            // releases the K stage.
+            // S = Q K(j)^T of pipeline s at ring position r (a block the pipeline does not use: nothing).
             auto issue_scores = [&](const PairWork& pw, int s, int j, int r) {
                 if (j >= pw.lo_of(s) && j < pw.hi_of(s)) {
                     const uint32_t tS = tmem_base + C::COL_S + s * 128;
@@ -466,7 +448,16 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     umma_commit_warp(&s_full[s]);
                     if (j + 1 == pw.hi_of(s)) umma_commit_warp(&q_empty[s]);
                 }
-                if (s == 1) umma_commit_warp(&k_empty[r & 1]);
+            };
+            // Q of a tile whose first scores come next
+            auto await_q = [&](const PairWork& pw, int s, int j) -> bool {
+                if (j != pw.lo_of(s) || j >= pw.hi_of(s)) return true;
+                if (!mbar_wait_inline(&q_full[s], (q_par >> s) & 1u)) {
+                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_Q, s);
+                    return false;
+                }
+                q_par ^= 1u << s;
+                return true;
             };
             TileCursor cur;
             cur.init(p);
@@ -482,33 +473,38 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             };
             PairWork pw{};
             bool have = next_unit(pw);
+            if (have && !mbar_wait_inline(k_first, 0)) {
+                if (lane == 0) report_fault(p.fault, FAULT_WAIT_K, 0u);
+                ok = false;
+            }
             for (int s = 0; have && ok && s < 2; ++s) {
-                ok = await_scores(pw, s, pw.ulo, 0);
+                ok = await_q(pw, s, pw.ulo);
                 tc_fence_after_sync();
                 if (ok) issue_scores(pw, s, pw.ulo, 0);
             }
+            umma_commit_warp(k_first);  // its second phase: the first block's K may be replaced
             while (have && ok) {
                 PairWork pn = pw;
                 const bool have_next = next_unit(pn);
                 for (int j = pw.ulo; ok && j < pw.uhi; ++j, ++gu) {
                     const bool more = j + 1 < pw.uhi;           // the next scores belong to this unit
                     const bool scores = more || have_next;
+                    if (!mbar_wait_inline(&kv_full[gu & 1], (gu >> 1) & 1)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_V, gu);
+                        ok = false;
+                        break;
+                    }
 #pragma unroll 1
                     for (int s = 0; s < 2; ++s) {
                         const bool act = j >= pw.lo_of(s) && j < pw.hi_of(s);
-                        if (s == 0 && !mbar_wait_inline(&v_full[gu & 1], (gu >> 1) & 1)) {
-                            report_fault(p.fault, FAULT_WAIT_V, gu);
-                            ok = false;
-                            break;
-                        }
-                        if (scores && !await_scores(more ? pw : pn, s, more ? j + 1 : pn.ulo, gu + 1)) {
+                        if (scores && !await_q(more ? pw : pn, s, more ? j + 1 : pn.ulo)) {
                             ok = false;
                             break;
                         }
                         if (act) {
                             if (j == pw.lo_of(s)) {
                                 if (!mbar_wait_inline(&o_empty[s], (o_par >> s) & 1u)) {
-                                    report_fault(p.fault, FAULT_WAIT_O, 0x100u + s);
+                                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x100u + s);
                                     ok = false;
                                     break;
                                 }
@@ -516,30 +512,31 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                             }
                             // P from tensor memory: 16 keys are 8 columns of packed bf16.  V is MN-major:
                             // 64-element head-dim chunks 16 KB apart, 8-key groups 1024 bytes apart; 16 keys =
-                            // 2048 bytes.  The first 64 keys go to the tensor pipe while the softmax warps are
-                            // still exponentiating the other 64.
+                            // 2048 bytes.  The first 96 keys go to the tensor pipe while the softmax warps are
+                            // still busy with the other 32: what is left for the chain is 128 clk.
                             const uint32_t tO = tmem_base + C::COL_O + s * 128, tP = tmem_base + C::COL_S + s * 128;
                             const uint64_t dv = dV + (uint64_t)((gu & 1) * TILE16);
                             const uint32_t par = (g_par >> s) & 1u;
-                            if (!mbar_wait_inline(&p_half[2 * s], par)) {
-                                report_fault(p.fault, FAULT_WAIT_P, gu);
+                            if (!mbar_wait_inline(&p_part[2 * s], par)) {
+                                if (lane == 0) report_fault(p.fault, FAULT_WAIT_P, gu);
                                 ok = false;
                                 break;
                             }
                             tc_fence_after_sync();
                             umma_ts_x4<8, 128>(tO, tP, dv, IDESC_PV, j > pw.lo_of(s) ? 1u : 0u);
-                            if (!mbar_wait_inline(&p_half[2 * s + 1], par)) {
-                                report_fault(p.fault, FAULT_WAIT_P, 0x1000u + gu);
+                            umma_ts_x2<8, 128>(tO, tP + 32, dv + 512, IDESC_PV, 1u);
+                            if (!mbar_wait_inline(&p_part[2 * s + 1], par)) {
+                                if (lane == 0) report_fault(p.fault, FAULT_WAIT_P, 0x1000u + gu);
                                 ok = false;
                                 break;
                             }
                             tc_fence_after_sync();
-                            umma_ts_x4<8, 128>(tO, tP + 32, dv + 512, IDESC_PV, 1u);
+                            umma_ts_x2<8, 128>(tO, tP + 48, dv + 768, IDESC_PV, 1u);
                             g_par ^= 1u << s;
                         }
                         if (scores) issue_scores(more ? pw : pn, s, more ? j + 1 : pn.ulo, gu + 1);
                         if (act && j + 1 == pw.hi_of(s)) umma_commit_warp(&o_full[s]);
-                        if (s == 1) umma_commit_warp(&v_empty[gu & 1]);
+                        if (s == 1) umma_commit_warp(&kv_empty[gu & 1]);
                     }
                 }
                 pw = pn;
@@ -611,7 +608,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     if (c + 1 == HD / 32) {
                         // O is in registers: the next tile may overwrite the accumulator.
                         tc_fence_before_sync();
-                        warp_arrive(&o_empty[s], lane);
+                        mbar_arrive_warp(&o_empty[s]);
                     }
                     if (warp_store) {
                         stage_chunk<GATE>(stage, lane, c, wa, inv, w8);
@@ -676,20 +673,23 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 tc_fence_after_sync();
                 const bool full = __all_sync(0xffffffffu, rm.lo <= kc && kc + C::BN <= rm.hi);
                 for (;;) {
+                    float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
                     tmem_ld32(tS, s0);
                     tmem_ld32(tS + 32, s1);
-                    tmem_ld32(tS + 64, s2);
-                    tmem_ld32(tS + 96, s3);
                     tmem_wait_ld();
+                    tmem_ld32(tS + 64, s2);  // lands while the maximum of the first half is taken
+                    tmem_ld32(tS + 96, s3);
                     if (!full) {  // window edge, diagonal, ragged end (two blocks in nine with a 1024-key window)
                         mask_chunk(s0, kc, rm);
                         mask_chunk(s1, kc + 32, rm);
+                    }
+                    chunk_max<0>(s0, mr, sl, kc, rm);
+                    chunk_max<0>(s1, mr, sl, kc, rm);
+                    tmem_wait_ld();
+                    if (!full) {
                         mask_chunk(s2, kc + 64, rm);
                         mask_chunk(s3, kc + 96, rm);
                     }
-                    float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                    chunk_max<0>(s0, mr, sl, kc, rm);
-                    chunk_max<0>(s1, mr, sl, kc, rm);
                     chunk_max<0>(s2, mr, sl, kc, rm);
                     chunk_max<0>(s3, mr, sl, kc, rm);
                     const float m_new = fmaxf(m, fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sl);
@@ -716,8 +716,8 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     if (need) m = m_new;
                 }
                 // Probabilities as bf16, packed over the first 64 of the block's score columns; row sum in fp32.
-                // The first 64 keys are announced a chunk late: by then their stores have landed and the wait for
-                // them costs nothing, and their share of O += P V still runs beside the last chunk.
+                // The first 96 keys are announced half a chunk late: by then their stores have landed and the wait
+                // for them costs nothing, and their share of O += P V still runs beside the rest.
                 const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
                 const uint64_t nm2 = pack_f32x2(-m_eff, -m_eff);
                 uint64_t ls2[2] = {0ull, 0ull};
@@ -727,11 +727,12 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 exp_chunk(s1, pk, ls2, sl2, nm2);
                 tmem_st16(tS + 16, pk);
                 exp_chunk(s2, pk, ls2, sl2, nm2);
+                tmem_st16(tS + 32, pk);
+                exp_chunk<0, 16>(s3, pk, ls2, sl2, nm2);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                warp_arrive(&p_half[2 * s], lane);
-                tmem_st16(tS + 32, pk);
-                exp_chunk(s3, pk, ls2, sl2, nm2);
+                mbar_arrive_warp(&p_part[2 * s]);
+                exp_chunk<16, 32>(s3, pk, ls2, sl2, nm2);
                 tmem_st16(tS + 48, pk);
                 float l0, l1, l2, l3;
                 unpack_f32x2(ls2[0], l0, l1);
@@ -739,7 +740,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 l += (l0 + l1) + (l2 + l3);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                warp_arrive(&p_half[2 * s + 1], lane);
+                mbar_arrive_warp(&p_part[2 * s + 1]);
             }
             if (ok && hi > lo) {
                 // The tile's last key block is on its way: hand the row sum to the epilogue warps and go on with
@@ -748,7 +749,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 if (p.out_lse && pw.live_of(s) && t < p.seq)
                     p.out_lse[((long long)pw.b * p.seq + t) * p.nq + pw.h_of(s)] =
                         l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
-                warp_arrive(&fin[2 * s + (tq & 1)], lane);
+                mbar_arrive_warp(&fin[2 * s + (tq & 1)]);
                 ++tq;
             }
         }

@@ -375,8 +375,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 tmem_wait_ld();
                 if (c + 1 == HD / 32) {  // O is in registers: the next unit may overwrite the accumulator
                     tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_remote(b_empty);
+                    mbar_arrive_remote_warp(b_empty);
                 }
                 if (warp_store) {
                     stage_chunk<GATE>(stage, lane, c & 3, wa, inv, w8);
@@ -489,8 +488,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 exp_chunk(s2, pk, ls2, sl2, nm2);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_remote(b_half + 16 * st);
+                mbar_arrive_remote_warp(b_half + 16 * st);
                 tmem_st16(tS + 32, pk);
                 exp_chunk(s3, pk, ls2, sl2, nm2);
                 tmem_st16(tS + 48, pk);
@@ -500,14 +498,13 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 l += (l0 + l1) + (l2 + l3);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_remote(b_half + 16 * st + 8);
+                mbar_arrive_remote_warp(b_half + 16 * st + 8);
             }
             if (ok) {
                 fin_vals[(n & 1) * 128 + r] = l;
                 if (p.out_lse && t < p.seq)
                     p.out_lse[((long long)w.b * p.seq + t) * p.nq + w.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
-                warp_arrive(&fin[n & 1], lane);
+                mbar_arrive_warp(&fin[n & 1]);
                 ++n;
             }
         }

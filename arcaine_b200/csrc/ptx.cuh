@@ -95,6 +95,16 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
                  : "memory");
 }
 
+// One arrival for a converged warp, behind everything its lanes did before.  (Predicated on an elected lane instead of
+// branching on the lane index: the branch costs the warp more than 100 clk.)
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
+    __syncwarp();
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b64 st;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q mbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
+}
+
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
                      smem_u32(bar)),
@@ -256,10 +266,14 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
 }
 
-// The same without release at cluster scope, for arrivals that announce tensor-memory accesses only (completed by
-// tcgen05.wait and ordered by tcgen05.fence): the release costs the arriving warp about 600 clk.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+// One arrival for a converged warp, without release at cluster scope: for arrivals that announce tensor-memory accesses
+// only (completed by tcgen05.wait and ordered by tcgen05.fence).  The release costs the arriving warp about 600 clk.
+__device__ __forceinline__ void mbar_arrive_remote_warp(uint32_t remote_bar) {
+    __syncwarp();
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(remote_bar)
+        : "memory");
 }
 
 // Bounded wait on a local mbarrier whose arrivals come from the whole cluster (acquire at cluster scope).
@@ -293,6 +307,16 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const void* tmap, ui
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(smem_dst)),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
+}
+
+// The same from a whole converged warp, one lane issuing.
+__device__ __forceinline__ void tma_load_4d_warp(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}" ::"r"(smem_u32(smem_dst)),
         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
