@@ -30,8 +30,6 @@ constexpr int kMaxDevices = 64;
 // The decode kernel keeps a few bytes of static shared memory; the dynamic part
 // may use the opt-in maximum minus this reserve.
 constexpr int kDecodeStaticSmem = 1024;
-// Dynamic shared memory the decode merge kernel may ask for (it is opted in to this much).
-constexpr int kMergeSmemOptin = 64 * 1024;
 
 struct DeviceState {
     std::atomic<bool> ready{false};  // set (release) once everything below is written
@@ -74,24 +72,27 @@ static cudaError_t opt_in_smem(K kernel, int bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-// Configuration of a launch in thread-block clusters of `size` CTAs.
-struct ClusterLaunch {
+// How many clusters of `size` CTAs of a kernel the device holds at once (0: none).
+template <typename K>
+static int clusters_at_once(K kernel, int size, int sm_count, int threads, int smem) {
     cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(sm_count / size * size));  // the answer is capped by the grid asked about
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
     cudaLaunchAttribute attr[1];
-    ClusterLaunch(int size, long long ctas, int threads, int smem, cudaStream_t stream) {
-        cfg.gridDim = dim3((unsigned)ctas);
-        cfg.blockDim = dim3((unsigned)threads);
-        cfg.dynamicSmemBytes = (size_t)smem;
-        cfg.stream = stream;
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)size;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
-    ClusterLaunch(const ClusterLaunch&) = delete;
-};
+    return n;
+}
 
 // One-time set-up for the current device: status-word address, SM count, and the
 // dynamic shared memory opt-in of every kernel.
@@ -132,34 +133,22 @@ static int device_state(DeviceState** out) {
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<256, false, false, true>, PrefillCfg<256>::SMEM_BYTES));
             for (int hi = 0; hi < 2; ++hi) {
                 for (int cs = 2, lg = 1; cs <= 4; cs *= 2, ++lg) {
-                    // (the answer is capped by the grid asked about)
-                    ClusterLaunch cl(cs, s.sm_count / cs * cs, hi ? PrefillCfg<256>::THREADS : PrefillCfg<128>::THREADS,
-                                     hi ? PrefillCfg<256>::SMEM_BYTES : PrefillCfg<128>::SMEM_BYTES, nullptr);
-                    int n = 0;
-                    const cudaError_t e = hi ? cudaOccupancyMaxActiveClusters(&n, sdpa_prefill_kernel<256, false, false, true>, &cl.cfg)
-                                             : cudaOccupancyMaxActiveClusters(&n, sdpa_prefill_kernel<128, false, false, true>, &cl.cfg);
-                    if (e == cudaSuccess && n > 0) s.active_clusters[hi][lg] = n;
-                    else cudaGetLastError();
+                    s.active_clusters[hi][lg] =
+                        hi ? clusters_at_once(sdpa_prefill_kernel<256, false, false, true>, cs, s.sm_count, PrefillCfg<256>::THREADS, PrefillCfg<256>::SMEM_BYTES)
+                           : clusters_at_once(sdpa_prefill_kernel<128, false, false, true>, cs, s.sm_count, PrefillCfg<128>::THREADS, PrefillCfg<128>::SMEM_BYTES);
                 }
             }
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true>, WideCfg::SMEM_BYTES));
-            {
-                ClusterLaunch cl(2, s.sm_count / 2 * 2, WideCfg::THREADS, WideCfg::SMEM_BYTES, nullptr);
-                ARC_CUDA(cudaOccupancyMaxActiveClusters(&s.wide_pairs, sdpa_prefill_wide_kernel<false>, &cl.cfg));
-                if (s.wide_pairs < 1) {
-                    std::snprintf(g_last_error, sizeof(g_last_error), "the device cannot hold a CTA pair of the prefill kernel");
-                    return ARC_ERR_CUDA;
-                }
+            s.wide_pairs = clusters_at_once(sdpa_prefill_wide_kernel<false>, 2, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
+            if (s.wide_pairs < 1) {
+                std::snprintf(g_last_error, sizeof(g_last_error), "the device cannot hold a CTA pair of the prefill kernel");
+                return ARC_ERR_CUDA;
             }
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2>, s.smem_optin - kDecodeStaticSmem));
-            ARC_CUDA(opt_in_smem(sdpa_decode_merge_kernel<128, false>, kMergeSmemOptin));
-            ARC_CUDA(opt_in_smem(sdpa_decode_merge_kernel<256, false>, kMergeSmemOptin));
-            ARC_CUDA(opt_in_smem(sdpa_decode_merge_kernel<128, true>, kMergeSmemOptin));
-            ARC_CUDA(opt_in_smem(sdpa_decode_merge_kernel<256, true>, kMergeSmemOptin));
             s.ready.store(true, std::memory_order_release);
         }
     }
@@ -167,22 +156,29 @@ static int device_state(DeviceState** out) {
     return ARC_OK;
 }
 
-// Launch `kernel` behind the previous kernel of `stream` with programmatic serialization: its CTAs
-// may be scheduled and run up to their grid_dependency_wait() while that kernel is still running,
-// which takes the launch latency of a small follow-up kernel (a merge) off the critical path.
+// Launch `kernel` behind the previous kernel of `stream` with programmatic serialization: its CTAs may be scheduled and
+// run up to their grid_dependency_wait() while that kernel is still running, which takes the launch latency and the
+// prologue off the critical path (2-3 us of a small call).  Every kernel of the library is launched this way, and every
+// one of them waits before it touches global memory and only then releases the kernel behind it
+// (grid_launch_dependents): so when a kernel may run, everything in front of its predecessor has completed, and no grid
+// completes before the one in front of it has.  cluster > 1: in clusters of that many CTAs along x.
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+static cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
                                     Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
@@ -323,10 +319,9 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     if (p->block_ids) {
         // span ends per query row, once per call: a few microseconds instead of a (seq, kv_len) f32 mask
         int* vis = reinterpret_cast<int*>(static_cast<unsigned char*>(p->workspace) + plan.split_bytes);
-        vision_span_kernel<<<(unsigned)((p->seq + 255) / 256), 256, 0, stream>>>(p->block_ids, p->block_ids_offset,
-                                                                               p->kv_len - p->seq, p->seq, p->kv_len, vis);
+        ARC_CUDA(launch_dependent(vision_span_kernel, dim3((unsigned)((p->seq + 255) / 256)), dim3(256), 0, stream, 1, p->block_ids,
+                                  p->block_ids_offset, p->kv_len - p->seq, p->seq, p->kv_len, vis));
         g_launches.fetch_add(1, std::memory_order_relaxed);
-        ARC_CUDA(cudaGetLastError());
         kp.vis_hi = vis;
     }
     kp.fault = ds->fault;
@@ -383,16 +378,10 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
             kp.total_tiles = (int)pair_units;
             const unsigned ctas = (unsigned)(pair_units < ds->sm_count ? pair_units : ds->sm_count);
             if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
-            if (kp.n_copies > 0) {
-                if (kp.gate) sdpa_prefill_pair_kernel<true, true><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, to, tg, kp);
-                else sdpa_prefill_pair_kernel<false, true><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, to, tg, kp);
-            } else if (kp.gate) {
-                sdpa_prefill_pair_kernel<true, false><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, to, tg, kp);
-            } else {
-                sdpa_prefill_pair_kernel<false, false><<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(tq, tk, tv, to, tg, kp);
-            }
+            auto kernel = kp.n_copies > 0 ? (kp.gate ? sdpa_prefill_pair_kernel<true, true> : sdpa_prefill_pair_kernel<false, true>)
+                                          : (kp.gate ? sdpa_prefill_pair_kernel<true, false> : sdpa_prefill_pair_kernel<false, false>);
+            ARC_CUDA(launch_dependent(kernel, dim3(ctas), dim3(PairCfg::THREADS), (size_t)PairCfg::SMEM_BYTES, stream, 1, tq, tk, tv, to, tg, kp));
             g_launches.fetch_add(1, std::memory_order_relaxed);
-            ARC_CUDA(cudaGetLastError());
             if (cut_tail) {
                 PrefillParams tp = kp;
                 tp.head_pair = 0;
@@ -403,9 +392,9 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
                 tp.num_splits = 1;
                 const dim3 grid((unsigned)(2 * left)), block(PrefillCfg<128>::THREADS);
                 if (tp.gate)
-                    ARC_CUDA(launch_dependent(sdpa_prefill_kernel<128, false, true>, grid, block, (size_t)PrefillCfg<128>::SMEM_BYTES, stream, tq, tk, tv, tp));
+                    ARC_CUDA(launch_dependent(sdpa_prefill_kernel<128, false, true>, grid, block, (size_t)PrefillCfg<128>::SMEM_BYTES, stream, 1, tq, tk, tv, tp));
                 else
-                    ARC_CUDA(launch_dependent(sdpa_prefill_kernel<128, false, false>, grid, block, (size_t)PrefillCfg<128>::SMEM_BYTES, stream, tq, tk, tv, tp));
+                    ARC_CUDA(launch_dependent(sdpa_prefill_kernel<128, false, false>, grid, block, (size_t)PrefillCfg<128>::SMEM_BYTES, stream, 1, tq, tk, tv, tp));
                 g_launches.fetch_add(1, std::memory_order_relaxed);
             }
             return ARC_OK;
@@ -428,8 +417,9 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
                         (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;
         if ((rc = make_tile_map(&tk, p->k, HD, p->nkv, p->kv_len, p->batch, p->k_stride_t, p->k_stride_b, 64)) != ARC_OK) return rc;
         if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
-        ClusterLaunch cl(2, 2 * (units < ds->wide_pairs ? units : ds->wide_pairs), WideCfg::THREADS, WideCfg::SMEM_BYTES, stream);
-        ARC_CUDA(cudaLaunchKernelEx(&cl.cfg, kp.gate ? sdpa_prefill_wide_kernel<true> : sdpa_prefill_wide_kernel<false>, tq, tk, tv, to, tg, kp));
+        ARC_CUDA(launch_dependent(kp.gate ? sdpa_prefill_wide_kernel<true> : sdpa_prefill_wide_kernel<false>,
+                                  dim3((unsigned)(2 * (units < ds->wide_pairs ? units : ds->wide_pairs))), dim3(WideCfg::THREADS),
+                                  (size_t)WideCfg::SMEM_BYTES, stream, 2, tq, tk, tv, to, tg, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
         return ARC_OK;
     }
@@ -446,8 +436,8 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         kp.total_tiles = (int)tiles;
         kp.num_splits = 1;
         const long long nclusters = tiles;  // the plan made sure that many are resident at once
-        ClusterLaunch cl(plan.cluster, nclusters * plan.cluster, PrefillCfg<HD>::THREADS, PrefillCfg<HD>::SMEM_BYTES, stream);
-        ARC_CUDA(cudaLaunchKernelEx(&cl.cfg, sdpa_prefill_kernel<HD, false, false, true>, tq, tk, tv, kp));
+        ARC_CUDA(launch_dependent(sdpa_prefill_kernel<HD, false, false, true>, dim3((unsigned)(nclusters * plan.cluster)),
+                                  dim3(PrefillCfg<HD>::THREADS), (size_t)PrefillCfg<HD>::SMEM_BYTES, stream, plan.cluster, tq, tk, tv, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
         return ARC_OK;
     }
@@ -457,14 +447,11 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     kp.total_tiles = (int)total_tiles;
     const unsigned ctas = (unsigned)(total_tiles < ds->sm_count ? total_tiles : ds->sm_count);
     // The additive-mask form is a kernel of its own: the common one stays small.
-    if (kp.mask_type == 1 && kp.mask != nullptr)
-        sdpa_prefill_kernel<HD, true, true><<<ctas, PrefillCfg<HD>::THREADS, PrefillCfg<HD>::SMEM_BYTES, stream>>>(tq, tk, tv, kp);
-    else if (kp.gate && plan.splits == 1)
-        sdpa_prefill_kernel<HD, false, true><<<ctas, PrefillCfg<HD>::THREADS, PrefillCfg<HD>::SMEM_BYTES, stream>>>(tq, tk, tv, kp);
-    else
-        sdpa_prefill_kernel<HD, false, false><<<ctas, PrefillCfg<HD>::THREADS, PrefillCfg<HD>::SMEM_BYTES, stream>>>(tq, tk, tv, kp);
+    auto kernel = kp.mask_type == 1 && kp.mask != nullptr ? sdpa_prefill_kernel<HD, true, true, false>
+                  : kp.gate && plan.splits == 1           ? sdpa_prefill_kernel<HD, false, true, false>
+                                                          : sdpa_prefill_kernel<HD, false, false, false>;
+    ARC_CUDA(launch_dependent(kernel, dim3(ctas), dim3(PrefillCfg<HD>::THREADS), (size_t)PrefillCfg<HD>::SMEM_BYTES, stream, 1, tq, tk, tv, kp));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    ARC_CUDA(cudaGetLastError());
 
     if (plan.splits > 1) {
         UniformMergeParams mp{};
@@ -485,7 +472,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         mp.out_copies = kp.out_copies;
         mp.n_copies = kp.n_copies;
         ARC_CUDA(launch_dependent(sdpa_uniform_merge_kernel<HD>, dim3((unsigned)((plan.rows + UMERGE_ROWS - 1) / UMERGE_ROWS)),
-                                  dim3(32 * UMERGE_ROWS), 0, stream, mp));
+                                  dim3(32 * UMERGE_ROWS), 0, stream, 1, mp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
     return ARC_OK;
@@ -499,7 +486,6 @@ struct DecodePlan {
     int smem_bytes = 0;
     long long parts = 0;
     size_t ws_bytes = 0;
-    size_t merge_smem = 0;
 };
 
 static int plan_decode(const arc_sdpa_decode_params* p, int sm_count, int smem_optin, DecodePlan* plan) {
@@ -546,11 +532,6 @@ static int plan_decode(const arc_sdpa_decode_params* p, int sm_count, int smem_o
     plan->ncta = ncta;
     plan->parts = ((long long)ncta + p->batch) * slices;
     plan->ws_bytes = (size_t)plan->parts * p->nq * ((size_t)p->hd + 1) * sizeof(float);
-    // the merge kernel keeps the length prefix, a row of partial sums per warp and one weight plus one
-    // list entry per record of a sequence (at most ncta + 1 shares) in shared memory
-    plan->merge_smem = (size_t)(p->batch + 2) * 8 + 8 * sizeof(float) + (size_t)(MERGE_THREADS / 32) * p->hd * sizeof(float) +
-                       (size_t)(ncta + 1) * slices * (sizeof(float) + sizeof(int));
-    if (plan->merge_smem > (size_t)kMergeSmemOptin) return ARC_ERR_TOO_LARGE;
     return ARC_OK;
 }
 
@@ -589,12 +570,9 @@ static int launch_decode(const arc_sdpa_decode_params* p, const DecodePlan& plan
     dim3 grid((unsigned)plan.ncta, (unsigned)plan.groups, 1);
     const unsigned threads = 32u * (unsigned)(plan.nkv_cta * plan.slices + 1);
     if (!empty_cache) {
-        if (plan.nt == 1)
-            sdpa_decode_kernel<HD, 1><<<grid, threads, plan.smem_bytes, stream>>>(tk, tv, kp);
-        else
-            sdpa_decode_kernel<HD, 2><<<grid, threads, plan.smem_bytes, stream>>>(tk, tv, kp);
+        ARC_CUDA(launch_dependent(plan.nt == 1 ? sdpa_decode_kernel<HD, 1> : sdpa_decode_kernel<HD, 2>, grid, dim3(threads),
+                                  (size_t)plan.smem_bytes, stream, 1, tk, tv, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
-        ARC_CUDA(cudaGetLastError());
     }
 
     DecodeMergeParams mp{};
@@ -619,15 +597,8 @@ static int launch_decode(const arc_sdpa_decode_params* p, const DecodePlan& plan
     mp.fault = ds->fault;
     dim3 mgrid((unsigned)p->nq, (unsigned)p->batch, 1);
     const bool xchg = mp.x_world > 1;
-    if (empty_cache) {
-        if (xchg) sdpa_decode_merge_kernel<HD, true><<<mgrid, MERGE_THREADS, plan.merge_smem, stream>>>(mp);
-        else sdpa_decode_merge_kernel<HD, false><<<mgrid, MERGE_THREADS, plan.merge_smem, stream>>>(mp);
-        ARC_CUDA(cudaGetLastError());
-    } else if (xchg) {
-        ARC_CUDA(launch_dependent(sdpa_decode_merge_kernel<HD, true>, mgrid, dim3(MERGE_THREADS), plan.merge_smem, stream, mp));
-    } else {
-        ARC_CUDA(launch_dependent(sdpa_decode_merge_kernel<HD, false>, mgrid, dim3(MERGE_THREADS), plan.merge_smem, stream, mp));
-    }
+    ARC_CUDA(launch_dependent(xchg ? sdpa_decode_merge_kernel<HD, true> : sdpa_decode_merge_kernel<HD, false>, mgrid,
+                              dim3(MERGE_THREADS), 0, stream, 1, mp));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return ARC_OK;
 }
@@ -814,12 +785,10 @@ extern "C" int arc_sdpa_merge(const float* part_out, const float* part_lse, int3
     if ((mp.o_part_stride & 3) != 0) return ARC_ERR_ALIGNMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned blocks = (unsigned)((rows + UMERGE_ROWS - 1) / UMERGE_ROWS);
-    if (hd == 128)
-        sdpa_uniform_merge_kernel<128><<<blocks, 32 * UMERGE_ROWS, 0, st>>>(mp);
-    else
-        sdpa_uniform_merge_kernel<256><<<blocks, 32 * UMERGE_ROWS, 0, st>>>(mp);
+    ARC_CUDA(launch_dependent(hd == 128 ? sdpa_uniform_merge_kernel<128> : sdpa_uniform_merge_kernel<256>, dim3(blocks),
+                              dim3(32 * UMERGE_ROWS), 0, st, 1, mp));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    return cudaGetLastError() == cudaSuccess ? ARC_OK : ARC_ERR_CUDA;
+    return ARC_OK;
 }
 
 extern "C" int arc_mul_sigmoid_inplace(void* a, const void* gate, int64_t n, void* stream) {
@@ -828,10 +797,10 @@ extern "C" int arc_mul_sigmoid_inplace(void* a, const void* gate, int64_t n, voi
     if (n == 0) return ARC_OK;
     long long blocks = (n + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    mul_sigmoid_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<uint16_t*>(a), static_cast<const uint16_t*>(gate), n);
+    ARC_CUDA(launch_dependent(mul_sigmoid_kernel, dim3((unsigned)blocks), dim3(256), 0, static_cast<cudaStream_t>(stream), 1,
+                              static_cast<uint16_t*>(a), static_cast<const uint16_t*>(gate), (long long)n));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    return cudaGetLastError() == cudaSuccess ? ARC_OK : ARC_ERR_CUDA;
+    return ARC_OK;
 }
 
 extern "C" int arc_qkv_prepare(const arc_qkv_prepare_params* p, void* stream) {
@@ -928,18 +897,15 @@ extern "C" int arc_qkv_prepare(const arc_qkv_prepare_params* p, void* stream) {
     auto launch = [&](auto hd_tag, auto qwen_tag) {
         constexpr int H = decltype(hd_tag)::value;
         constexpr bool Q = decltype(qwen_tag)::value;
-        if (ahead) qkv_prepare_kernel<H, Q, true><<<ctas, 256, 0, st>>>(kp, tpc);
-        else qkv_prepare_kernel<H, Q, false><<<ctas, 256, 0, st>>>(kp, tpc);
+        return launch_dependent(ahead ? qkv_prepare_kernel<H, Q, true> : qkv_prepare_kernel<H, Q, false>, dim3(ctas), dim3(256), 0, st, 1, kp, tpc);
     };
     auto launch_hd = [&](auto qwen_tag) {
-        if (p->hd == 128) launch(std::integral_constant<int, 128>{}, qwen_tag);
-        else if (p->hd == 256) launch(std::integral_constant<int, 256>{}, qwen_tag);
-        else launch(std::integral_constant<int, 512>{}, qwen_tag);
+        if (p->hd == 128) return launch(std::integral_constant<int, 128>{}, qwen_tag);
+        if (p->hd == 256) return launch(std::integral_constant<int, 256>{}, qwen_tag);
+        return launch(std::integral_constant<int, 512>{}, qwen_tag);
     };
-    if (qwen) launch_hd(std::true_type{});
-    else launch_hd(std::false_type{});
+    ARC_CUDA(qwen ? launch_hd(std::true_type{}) : launch_hd(std::false_type{}));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    ARC_CUDA(cudaGetLastError());
     return ARC_OK;
 }
 
@@ -963,14 +929,14 @@ static int fill_mask(float* mask, const int32_t* block_ids, int32_t q_len, int32
                      int32_t sliding_window, void* stream) {
     if (!mask) return ARC_ERR_NULL_POINTER;
     if (q_len < 0 || kv_len < 0) return ARC_ERR_BAD_SHAPE;
-    const long long n = (long long)q_len * kv_len;
-    if (n == 0) return ARC_OK;
-    long long blocks = (n + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    fill_causal_mask_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        mask, block_ids, q_len, kv_len, past_offset, sliding_window);
+    if (q_len == 0 || kv_len == 0) return ARC_OK;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // a block writes 1024 keys of a row; a grid's y extent ends at 65535, longer masks loop
+    const dim3 grid((unsigned)((kv_len + 1023) / 1024), (unsigned)(q_len < 65535 ? q_len : 65535));
+    ARC_CUDA(launch_dependent(block_ids ? fill_causal_mask_kernel<true> : fill_causal_mask_kernel<false>, grid, dim3(256), 0, st, 1,
+                              mask, block_ids, (int)q_len, (int)kv_len, (int)past_offset, (int)sliding_window));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    return cudaGetLastError() == cudaSuccess ? ARC_OK : ARC_ERR_CUDA;
+    return ARC_OK;
 }
 
 extern "C" int arc_sdpa_device_status(uint32_t* fault_code, uint32_t* fault_detail) {

@@ -57,21 +57,24 @@ struct DecodeParams {
     long long kv_rows_total;   // rows addressable from k and v
 };
 
-// Prefix sums of the per-sequence lengths into shared memory: cum[b] = keys
-// before sequence b, cum[batch] = total.  Called by every thread of the block.
-__device__ __forceinline__ void build_len_prefix(const int* kv_len, int kv_len_uniform, int batch,
-                                                 long long* cum) {
-    for (int b = threadIdx.x; b < batch; b += blockDim.x) {
-        int len = kv_len ? kv_len[b] : kv_len_uniform;
-        cum[b + 1] = len > 0 ? len : 0;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+// Prefix sums of the per-sequence lengths into shared memory: cum[b] = keys before sequence b, cum[batch] = total.
+// Called by every thread of the block; the first warp scans, 32 sequences a step (one thread adding them up in turn
+// took a microsecond for 64).
+__device__ __forceinline__ void build_len_prefix(const int* kv_len, int kv_len_uniform, int batch, long long* cum) {
+    if (threadIdx.x < 32) {
         long long run = 0;
-        cum[0] = 0;
-        for (int b = 0; b < batch; ++b) {
-            run += cum[b + 1];
-            cum[b + 1] = run;
+        if (threadIdx.x == 0) cum[0] = 0;
+        for (int b0 = 0; b0 < batch; b0 += 32) {
+            const int b = b0 + threadIdx.x;
+            const int len = b < batch ? (kv_len ? kv_len[b] : kv_len_uniform) : 0;
+            long long v = len > 0 ? len : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long up = __shfl_up_sync(0xffffffffu, v, o);
+                if ((int)threadIdx.x >= o) v += up;
+            }
+            if (b < batch) cum[b + 1] = run + v;
+            run += __shfl_sync(0xffffffffu, v, 31);
         }
     }
     __syncthreads();
@@ -113,26 +116,27 @@ __global__ void __launch_bounds__(288, 1)
     const int head0 = blockIdx.y * p.nkv_cta;  // first KV head of this CTA
     const int G = p.nq / p.nkv;
 
-    grid_launch_dependents();  // the merge kernel may be scheduled now; it waits for this grid before reading
-    // A fault recorded by an earlier CTA or launch: do not start new waits.
     __shared__ uint32_t abort_flag;
-    // Everything the prologue reads from global memory is asked for at once: after an L2 flush each of these is
-    // an HBM round trip, and taken one after the other (status word and lengths, then row offsets, then the
-    // descriptors at the first copy) they kept the first K / V request waiting for several microseconds.
-    if (p.kv_row_offset)
-        for (int b = threadIdx.x * 16; b < p.batch; b += blockDim.x * 16) prefetch_l2(p.kv_row_offset + b);
     if (threadIdx.x == 32) {
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
     }
     if (threadIdx.x == 0) {
-        abort_flag = *reinterpret_cast<volatile uint32_t*>(p.fault);
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], ncw);
         }
         fence_mbar_init();
     }
+    // Up to here nothing depends on the kernels in front; everything below may.
+    grid_dependency_wait();
+    grid_launch_dependents();  // the merge kernel may be scheduled now; it waits for this grid before reading
+    // A fault recorded by an earlier CTA or launch: do not start new waits.  Everything the prologue reads from global
+    // memory is asked for at once: after an L2 flush each of these is an HBM round trip, and taken one after the other
+    // (status word and lengths, then row offsets) they kept the first K / V request waiting.
+    if (p.kv_row_offset)
+        for (int b = threadIdx.x * 16; b < p.batch; b += blockDim.x * 16) prefetch_l2(p.kv_row_offset + b);
+    if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile uint32_t*>(p.fault);
     build_len_prefix(p.kv_len, p.kv_len_uniform, p.batch, cum);
     if (abort_flag != 0u) return;
     // Lengths and row offsets live on the device, so this is where they can be checked: a sequence
@@ -482,121 +486,106 @@ __device__ __forceinline__ float sigmoid_gate(float attn, uint16_t gate_bits) {
 
 constexpr int MERGE_THREADS = 256;
 
-// Block-wide max / sum over MERGE_THREADS threads (result to every thread).
-__device__ __forceinline__ float block_reduce(float v, bool is_max, float* scratch) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float t = __shfl_xor_sync(0xffffffffu, v, o);
-        v = is_max ? fmaxf(v, t) : v + t;
-    }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float r = scratch[0];
-#pragma unroll
-    for (int w = 1; w < MERGE_THREADS / 32; ++w) r = is_max ? fmaxf(r, scratch[w]) : r + scratch[w];
-    return r;
-}
-
 // XCHG: the instance that also exchanges records with other GPUs.  It keeps every source's values in
 // registers; the plain merge — hundreds of small blocks for a large batch — stays lean enough for five blocks
 // per SM.
 template <int HD, bool XCHG>
 __global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const DecodeMergeParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    long long* cum = reinterpret_cast<long long*>(smem_raw);
-    float* red = reinterpret_cast<float*>(cum + p.batch + 2);      // 8 floats
-    float* acc_sm = red + 8;                                        // (warps) x HD
-    float* wgt = acc_sm + (MERGE_THREADS / 32) * HD;                // one weight per record
-    __shared__ int n_live_sm;
-    // What does not depend on the decode kernel's results happens while it still runs: the length prefix, and
-    // requests for the lines the tail will need (this row's gate values, the status word) into L2.
-    if (p.gate && p.out && threadIdx.x < HD * 2 / 128)
-        prefetch_l2(p.gate + (long long)blockIdx.y * p.o_stride_b + (long long)blockIdx.x * HD + threadIdx.x * 64);
-    if (threadIdx.x == 32) prefetch_l2(p.fault);
-    build_len_prefix(p.kv_len, p.kv_len_uniform, p.batch, cum);
-    grid_dependency_wait();                                        // from here on its partial records are read
-    if (*reinterpret_cast<volatile uint32_t*>(p.fault) != 0u) return;  // block-uniform: a status is set, no work
+    // One row of output per block; what the block does before its one barrier every warp does for itself — where the
+    // row's records are, their maximum and weights — because that is a handful of loads, while three block-wide
+    // reductions and a list in shared memory made this kernel's tail 5 us.
+    constexpr int NW = MERGE_THREADS / 32;
+    __shared__ float acc_sm[NW * HD];
     const int h = blockIdx.x, b = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long total = cum[p.batch];
+    // (The decode kernel released this one after its own wait for the kernels in front: the lengths are final.)
+    long long k_begin = 0, total = 0, k_len = 0;
+    if (!p.kv_len) {
+        k_len = max(0, p.kv_len_uniform);
+        k_begin = (long long)b * k_len;
+        total = (long long)p.batch * k_len;
+    } else {
+        for (int i = lane; i < p.batch; i += 32) {
+            const int len = max(0, p.kv_len[i]);
+            total += len;
+            if (i < b) k_begin += len;
+            if (i == b) k_len = len;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            total += __shfl_xor_sync(0xffffffffu, total, o);
+            k_begin += __shfl_xor_sync(0xffffffffu, k_begin, o);
+            k_len += __shfl_xor_sync(0xffffffffu, k_len, o);
+        }
+    }
+    // requests for the lines the end will need
+    if (p.gate && p.out && threadIdx.x < HD * 2 / 128)
+        prefetch_l2(p.gate + (long long)b * p.o_stride_b + (long long)h * HD + threadIdx.x * 64);
     const long long per = share_size(total, p.ncta, 16 * p.slices);
-    const long long k_begin = cum[b], k_end = cum[b + 1];
+    const long long k_end = k_begin + k_len;
+    grid_dependency_wait();                                            // from here on the partial records are read
+    grid_launch_dependents();
+    if (*reinterpret_cast<volatile uint32_t*>(p.fault) != 0u) return;  // block-uniform: a status is set, no work
     constexpr int VPL = HD / 32;  // output values per lane
     float acc[VPL];
 #pragma unroll
     for (int j = 0; j < VPL; ++j) acc[j] = 0.f;
     float lse = -CUDART_INF_F, inv = 0.f;
-    if (k_end > k_begin) {  // block-uniform
+    if (k_len > 0) {  // block-uniform
         const int c_first = (int)(k_begin / per), c_last = (int)((k_end - 1) / per);
         const int n_parts = (c_last - c_first + 1) * p.slices;
         const long long part0 = ((long long)c_first + b) * p.slices;
-        // weights: every thread takes a strided set of records
+        const float* lses = p.part_lse + part0 * p.nq + h;
         float mx = -CUDART_INF_F;
-        for (int i = threadIdx.x; i < n_parts; i += MERGE_THREADS) {
-            const float li = p.part_lse[(part0 + i) * p.nq + h];
-            wgt[i] = li;
-            mx = fmaxf(mx, li);
-        }
-        mx = block_reduce(mx, true, red);
-        float z = 0.f;
+        for (int i = lane; i < n_parts; i += 32) mx = fmaxf(mx, lses[(long long)i * p.nq]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (mx > -CUDART_INF_F) {
-            for (int i = threadIdx.x; i < n_parts; i += MERGE_THREADS) {
-                const float w = __expf(wgt[i] - mx);  // exp(-inf) = 0 for empty records
-                wgt[i] = w;
+            // Most records carry no weight (the decode kernel folds the slices of a share's last segment into slice
+            // 0's slot and marks the others empty): the live ones are dealt to the warps in turn, in order, so the
+            // fold is spread evenly and always adds in the same order; four at a time, their loads in flight
+            // together; a lane owns VPL consecutive output values.
+            float z = 0.f;
+            int seen = 0;  // live records before this group of 32
+            for (int i0 = 0; i0 < n_parts; i0 += 32) {
+                const int i = i0 + lane;
+                const float w = i < n_parts ? __expf(lses[(long long)i * p.nq] - mx) : 0.f;  // exp(-inf) = 0 for empty records
                 z += w;
-            }
-        }
-        z = block_reduce(z, false, red);  // also orders the wgt[] writes before the reads below
-        if (z > 0.f) {
-            inv = 1.f / z;
-            lse = mx + __logf(z);
-            // Most records carry no weight (the decode kernel folds the slices of a share's last segment
-            // into slice 0's slot and marks the others empty; slots of other sequences' shares): warp 0
-            // lists the live ones, in order, so that the fold below is spread evenly and always adds in the
-            // same order.
-            int* live = reinterpret_cast<int*>(wgt + n_parts);
-            if (warp == 0) {
-                int base = 0;
-                for (int i0 = 0; i0 < n_parts; i0 += 32) {
-                    const int i = i0 + lane;
-                    const bool on = i < n_parts && wgt[i] != 0.f;
-                    const uint32_t bal = __ballot_sync(0xffffffffu, on);
-                    if (on) live[base + __popc(bal & ((1u << lane) - 1u))] = i;
-                    base += __popc(bal);
-                }
-                if (lane == 0) n_live_sm = base;
-            }
-            __syncthreads();
-            const int n_live = n_live_sm;
-            // each warp folds every 8th live record, four at a time so that their loads are in flight
-            // together (one record after the other, the loop ran at one L2 latency per record);
-            // a lane owns VPL consecutive output values
-            constexpr int NW = MERGE_THREADS / 32, U = 4;
-            for (int j0 = warp; j0 < n_live; j0 += NW * U) {
-                float w[U];
-                float4 ov[U][VPL / 4];
+                const uint32_t live = __ballot_sync(0xffffffffu, w != 0.f);
+                // this warp's: the record's rank among the live ones, modulo the warps
+                uint32_t mine = __ballot_sync(0xffffffffu, w != 0.f && ((seen + __popc(live & ((1u << lane) - 1u))) % NW) == warp);
+                seen += __popc(live);
+                while (mine) {
+                    constexpr int U = 4;
+                    float wu[U];
+                    float4 ov[U][VPL / 4];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int jj = j0 + u * NW;
-                    const int i = jj < n_live ? live[jj] : 0;
-                    w[u] = jj < n_live ? wgt[i] : 0.f;
-                    const float* src = p.part_o + ((part0 + i) * p.nq + h) * HD + lane * VPL;
+                    for (int u = 0; u < U; ++u) {
+                        const int src = mine ? __ffs(mine) - 1 : 0;
+                        wu[u] = __shfl_sync(0xffffffffu, w, src);
+                        if (!mine) wu[u] = 0.f;
+                        mine &= mine - 1;
+                        const float* rec = p.part_o + ((part0 + i0 + src) * p.nq + h) * HD + lane * VPL;
 #pragma unroll
-                    for (int j = 0; j < VPL / 4; ++j)
-                        ov[u][j] = w[u] != 0.f ? *reinterpret_cast<const float4*>(src + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
+                        for (int j = 0; j < VPL / 4; ++j)
+                            ov[u][j] = wu[u] != 0.f ? *reinterpret_cast<const float4*>(rec + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
+                    for (int u = 0; u < U; ++u) {
 #pragma unroll
-                    for (int j = 0; j < VPL / 4; ++j) {
-                        acc[4 * j] = fmaf(w[u], ov[u][j].x, acc[4 * j]);
-                        acc[4 * j + 1] = fmaf(w[u], ov[u][j].y, acc[4 * j + 1]);
-                        acc[4 * j + 2] = fmaf(w[u], ov[u][j].z, acc[4 * j + 2]);
-                        acc[4 * j + 3] = fmaf(w[u], ov[u][j].w, acc[4 * j + 3]);
+                        for (int j = 0; j < VPL / 4; ++j) {
+                            acc[4 * j] = fmaf(wu[u], ov[u][j].x, acc[4 * j]);
+                            acc[4 * j + 1] = fmaf(wu[u], ov[u][j].y, acc[4 * j + 1]);
+                            acc[4 * j + 2] = fmaf(wu[u], ov[u][j].z, acc[4 * j + 2]);
+                            acc[4 * j + 3] = fmaf(wu[u], ov[u][j].w, acc[4 * j + 3]);
+                        }
                     }
                 }
             }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+            inv = 1.f / z;
+            lse = mx + __logf(z);
         }
     }
 #pragma unroll
@@ -724,6 +713,7 @@ constexpr int UMERGE_ROWS = 8;  // rows per block of the uniform merge: one warp
 template <int HD>
 __global__ void __launch_bounds__(32 * UMERGE_ROWS) sdpa_uniform_merge_kernel(const UniformMergeParams p) {
     grid_dependency_wait();  // launched behind the kernel that writes the partials, possibly before it has finished
+    grid_launch_dependents();
     const long long row = (long long)blockIdx.x * UMERGE_ROWS + (threadIdx.x >> 5);
     if (row >= p.rows) return;
     const int lane = threadIdx.x & 31;
@@ -814,6 +804,8 @@ __global__ void __launch_bounds__(32 * UMERGE_ROWS) sdpa_uniform_merge_kernel(co
 
 // a[i] = bf16(f32(a[i]) * sigmoid(f32(gate[i]))) : src/modeling/qwen3_5_moe/kernels.hpp:80-88
 __global__ void mul_sigmoid_kernel(uint16_t* a, const uint16_t* gate, long long n) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const float g = bf16_bits_to_f32(gate[i]);
@@ -825,22 +817,33 @@ __global__ void mul_sigmoid_kernel(uint16_t* a, const uint16_t* gate, long long 
 // Additive causal / sliding-window mask : src/common/kernels/attention_mask.hpp:12-38; with
 // block_ids (one int per absolute position, -1 = text) tokens of the same non-negative block also
 // see each other's future: fill_causal_mask_with_block_ids, attention_mask.hpp:44-73.
-__global__ void fill_causal_mask_kernel(float* mask, const int* block_ids, int q_len, int kv_len, int past_offset,
-                                        int window) {
-    const long long n = (long long)q_len * kv_len;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const int qi = (int)(i / kv_len), kvj = (int)(i % kv_len);
+// Bound by the stores: a thread writes four consecutive keys of one row, 16 bytes at once where the row allows it, and
+// divides nothing (one element per thread and a division per element took 13 us for 1000 x 1300).
+template <bool IDS>
+__global__ void fill_causal_mask_kernel(float* mask, const int* block_ids, int q_len, int kv_len, int past_offset, int window) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const int j0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (j0 >= kv_len) return;
+    const int first = past_offset - (kv_len - q_len);  // absolute position of key 0
+    for (int qi = blockIdx.y; qi < q_len; qi += gridDim.y) {
         const int q_global = past_offset + qi;
-        const int kv_global = past_offset - (kv_len - q_len) + kvj;
-        bool same_block = false;
-        if (block_ids) {
-            const int qb = block_ids[q_global];
-            same_block = qb >= 0 && kv_global >= 0 && qb == block_ids[kv_global];
+        const int qb = IDS ? block_ids[q_global] : -1;
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int kv_global = first + j0 + e;
+            const bool same_block = IDS && qb >= 0 && kv_global >= 0 && j0 + e < kv_len && qb == block_ids[kv_global];
+            const bool causal = !same_block && kv_global > q_global;
+            const bool too_far = (window != 0x7fffffff) && (kv_global < q_global - window + 1);
+            v[e] = (causal || too_far) ? -CUDART_INF_F : 0.0f;
         }
-        const bool causal = !same_block && kv_global > q_global;
-        const bool too_far = (window != 0x7fffffff) && (kv_global < q_global - window + 1);
-        mask[i] = (causal || too_far) ? -CUDART_INF_F : 0.0f;
+        float* dst = mask + (long long)qi * kv_len + j0;
+        if (j0 + 4 <= kv_len && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+            *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+            for (int e = 0; e < 4 && j0 + e < kv_len; ++e) dst[e] = v[e];
+        }
     }
 }
 
@@ -849,6 +852,8 @@ __global__ void fill_causal_mask_kernel(float* mask, const int* block_ids, int q
 // contiguous) sees the block's later keys as well.  ids[base + j] is key j's id; row t sits at key
 // position t + off.  One thread per row; the scan runs to the end of the row's block at most.
 __global__ void vision_span_kernel(const int* ids, int base, int off, int seq, int kv_len, int* vis_hi) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= seq) return;
     const int self = t + off;  // key index of the query's own position

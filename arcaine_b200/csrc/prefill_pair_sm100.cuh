@@ -51,9 +51,9 @@ struct PairCfg {
     static constexpr int TMEM_COLS = 512;
     static constexpr int COL_S = 0;    // + 128 * pipeline
     static constexpr int COL_O = 256;  // + 128 * pipeline
-    // q_full[2] q_empty[2] k_first kv_full[2] kv_empty[2] then per pipeline:
+    // q_full[2] q_empty[2] k_first k_first_used kv_full[2] kv_empty[2] then per pipeline:
     // s_full p_part[2] o_full o_empty fin[2]; then gate[4], one per epilogue warp
-    static constexpr int NUM_BARS = 4 + 1 + 2 * K_STAGES + 18;
+    static constexpr int NUM_BARS = 4 + 2 + 2 * K_STAGES + 18;
     static constexpr int FIN_FLOATS = 2 * 2 * 128;  // [tile parity][pipeline][row] row sum
     static constexpr int SMEM_BYTES = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 4 * 8192 + NUM_BARS * 8 + 16 + FIN_FLOATS * 4;  // (4 x 8 KB: output stage)
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
@@ -251,9 +251,10 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + STAGE_BYTES);
     uint64_t* q_full = bars;         // [2]
     uint64_t* q_empty = bars + 2;    // [2] the tile's last S = Q K^T has completed
-    uint64_t* k_first = bars + 4;    // the first key block's K
-    uint64_t* kv_full = bars + 5;    // [2] V of a block and K of the block after it
-    uint64_t* kv_empty = bars + 7;   // [2] both have been used by both pipelines
+    uint64_t* k_first = bars + 4;       // the first key block's K
+    uint64_t* k_first_used = bars + 5;  // both pipelines' first scores have been computed
+    uint64_t* kv_full = bars + 6;       // [2] V of a block and K of the block after it
+    uint64_t* kv_empty = bars + 8;      // [2] both have been used by both pipelines
     uint64_t* s_full = kv_empty + 2; // [2] per pipeline from here on
     uint64_t* p_part = s_full + 2;   // [pipeline][part]: P of keys 0-95 / 96-127 of the block is in tensor memory
     uint64_t* o_full = p_part + 4;   // one phase per tile: the tile's last O += P V has completed
@@ -269,21 +270,17 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     uint32_t* abort_slot = tmem_slot + 1;
     float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [tile parity 2][pipeline 2][row 128] row sum
 
-    grid_launch_dependents();  // a launch behind this one (the single-head tail of the unit list) may be scheduled as SMs free up
     // (broadcast, so that the compiler knows them to be the same in every lane and keeps what follows from them —
     // MMA descriptors above all — in uniform registers)
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
 
-    // After an L2 flush the status word, the three descriptors and the first tiles are an HBM round trip each:
-    // the descriptors and the status word are requested at once, and the barriers are set up while they travel.
     if (threadIdx.x == 32) {
         prefetch_tensormap(&tm_q);
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
     }
     if (threadIdx.x == 0) {
-        const uint32_t fault_word = *reinterpret_cast<volatile uint32_t*>(p.fault);
         for (int s = 0; s < 2; ++s) {
             mbar_init(&q_full[s], 1);
             mbar_init(&q_empty[s], 1);
@@ -297,23 +294,27 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         }
         for (int w = 0; w < 4; ++w) mbar_init(&gate_bar[w], 1);
         mbar_init(k_first, 1);
+        mbar_init(k_first_used, 1);
         for (int s = 0; s < 2; ++s) {
             mbar_init(&kv_full[s], 1);
             mbar_init(&kv_empty[s], 1);
         }
         fence_mbar_init();
-        *abort_slot = fault_word != 0u ? 1u : 0u;
     }
-    __syncthreads();
-    if (*abort_slot) return;
     if (warp == C::PRODUCER_WARP) {
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
     }
+    // Up to here nothing depends on the kernels in front; everything below may.  A launch behind this one (the
+    // single-head tail of the unit list) may be scheduled from then on, as SMs free up.
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (threadIdx.x == 0) *abort_slot = *reinterpret_cast<volatile uint32_t*>(p.fault) != 0u ? 1u : 0u;
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
+    const int total_tiles = *abort_slot ? 0 : p.total_tiles;  // a status is set: walk an empty list
 
     if (warp >= C::PRODUCER_WARP) {
         reg_dealloc<C::REGS_CONTROL>();
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             TileCursor cur;
             PairWork last{};  // unit and index of the block requested last
             int last_j = 0;
-            for (cur.init(p); ok && cur.w < p.total_tiles; cur.advance(p)) {
+            for (cur.init(p); ok && cur.w < total_tiles; cur.advance(p)) {
                 const PairWork pw = decode_pair(p, cur);
                 for (int j = pw.ulo; ok && j < pw.uhi; ++j, ++r) {
                     if (r == 0) {
@@ -340,11 +341,10 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                         load(sK, &tm_k, k_first, pw, j);
                     } else {
                         // V of block r - 1 and K of block r; both stages were used by step r - 3 (the first K by the
-                        // scores in front of all steps: its barrier's second phase — and the first one, or the wait
-                        // for the second would pass before the first has completed)
+                        // scores in front of all steps)
                         uint64_t* full = &kv_full[(r - 1) & 1];
                         const bool free = r < 2    ? true
-                                          : r == 2 ? mbar_wait_inline(k_first, 0u) && mbar_wait_inline(k_first, 1u)
+                                          : r == 2 ? mbar_wait_inline(k_first_used, 0u)
                                                    : mbar_wait_inline(&kv_empty[(r - 1) & 1], (((r - 1) >> 1) - 1) & 1);
                         if (!free) {
                             if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x100u);
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 int tq0 = 0, tq1 = 0;  // tiles with key blocks loaded so far, per pipeline
                 bool ok = true;
                 TileCursor cur;
-                for (cur.init(p); ok && cur.w < p.total_tiles; cur.advance(p)) {
+                for (cur.init(p); ok && cur.w < total_tiles; cur.advance(p)) {
                     const PairWork pw = decode_pair(p, cur);
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     // memory) are asked into L2 now, a whole unit ahead of the load that needs them.
                     TileCursor nx = cur;
                     nx.advance(p);
-                    if (ok && nx.w < p.total_tiles) {
+                    if (ok && nx.w < total_tiles) {
                         const PairWork pn = decode_pair(p, nx);
 #pragma unroll
                         for (int s = 0; s < 2; ++s) {
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             TileCursor cur;
             cur.init(p);
             auto next_unit = [&](PairWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
-                for (; cur.w < p.total_tiles; cur.advance(p)) {
+                for (; cur.w < total_tiles; cur.advance(p)) {
                     w = decode_pair(p, cur);
                     if (w.uhi > w.ulo) {
                         cur.advance(p);
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 tc_fence_after_sync();
                 if (ok) issue_scores(pw, s, pw.ulo, 0);
             }
-            umma_commit_warp(k_first);  // its second phase: the first block's K may be replaced
+            umma_commit_warp(k_first_used);
             while (have && ok) {
                 PairWork pn = pw;
                 const bool have_next = next_unit(pn);
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         bool ok = true;
         OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[quarter], 0u};
         TileCursor cur;
-        for (cur.init(p); ok && cur.w < p.total_tiles; cur.advance(p)) {
+        for (cur.init(p); ok && cur.w < total_tiles; cur.advance(p)) {
             const PairWork pw = decode_pair(p, cur);
 #pragma unroll 1
             for (int s = 0; s < 2 && ok; ++s) {
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         uint32_t s0[32], s1[32], s2[32], s3[32];  // the row's 128 scores of the current block
 
         TileCursor cur;
-        for (cur.init(p); ok && cur.w < p.total_tiles; cur.advance(p)) {
+        for (cur.init(p); ok && cur.w < total_tiles; cur.advance(p)) {
             const PairWork pw = decode_pair(p, cur);
             if (pw.uhi == pw.ulo) continue;
             const int t = pw.q0_of(s) + r;

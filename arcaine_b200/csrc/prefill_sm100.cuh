@@ -397,11 +397,9 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     const bool windowed = causal && p.window > 0 && p.window != 0x7fffffff;
     const int off = p.kv_len - p.seq;
 
-    grid_launch_dependents();  // with key-range splits the merge kernel follows: it may be scheduled already
     constexpr int PRODUCER_WARP = C::SOFTMAX_WARPS;
     constexpr int MMA_WARP = C::SOFTMAX_WARPS + 1;
     if (threadIdx.x == 0) {
-        const uint32_t fault_word = *reinterpret_cast<volatile uint32_t*>(p.fault);
         mbar_init(q_full, 1);
         mbar_init(q_empty, 1);
         for (int s = 0; s < KS; ++s) {
@@ -422,7 +420,6 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         mbar_init(part_ready, csize);  // one arrival per CTA of the cluster
         mbar_init(read_done, csize);
         fence_mbar_init();
-        *abort_slot = fault_word != 0u ? 1u : 0u;
     }
     if (warp == PRODUCER_WARP) {
         if (lane == 0) {
@@ -434,6 +431,11 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
     }
+    // Up to here nothing depends on the kernels in front; everything below may.  (The tail of a two-tile launch runs
+    // beside that launch, which let it start only when the kernels before it had completed.)
+    if (p.tail_base < 0) grid_dependency_wait();
+    grid_launch_dependents();
+    if (threadIdx.x == 0) *abort_slot = *reinterpret_cast<volatile uint32_t*>(p.fault) != 0u ? 1u : 0u;
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();

@@ -36,9 +36,9 @@ struct WideCfg {
     static constexpr int STAGES = 2;               // of K and of V
     static constexpr int COL_S = 0;                // + 128 * buffer
     static constexpr int COL_O = 256;
-    // q_full q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[2], gate[epilogue warp]
-    static constexpr int NUM_BARS = 2 + 8 + 2 + 4 + 4 + 4;
-    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 2 * 128 * 4;
+    // q_full q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp]
+    static constexpr int NUM_BARS = 2 + 8 + 2 + 4 + 2 + 4 + 4;
+    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
     static constexpr int EPILOGUE_WARP = 4, PRODUCER_WARP = 8, ISSUER_WARP = 9;
     static constexpr int THREADS = 320;
@@ -125,11 +125,15 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     uint64_t* p_half = bars + 12;      // [buffer][half] leader: eight warps' probabilities of keys 0-63 / 64-127
     uint64_t* o_full = bars + 16;      // both: one phase per unit
     uint64_t* o_empty = bars + 17;     // leader: eight epilogue warps have read O out
-    uint64_t* fin = bars + 18;         // [unit parity] own CTA: row sums are published
-    uint64_t* gate_bar = bars + 20;    // [epilogue warp] own CTA
+    // [unit & 3] own CTA: the softmax warps have published the unit's row sums.  While the epilogue is still busy with
+    // unit n - 1, units n, n + 1 and n + 2 may be through the softmax when they have one key block each (scores are
+    // computed one block ahead; the first P V of n + 1 waits for the epilogue of n): with fewer slots a phase could
+    // complete twice before the epilogue has looked at it, which a parity wait cannot tell from "not yet".
+    uint64_t* fin = bars + 18;
+    uint64_t* gate_bar = bars + 22;    // [epilogue warp] own CTA
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
-    float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [unit parity][row] row sum
+    float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [unit & 3][row] row sum
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
@@ -142,7 +146,6 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         prefetch_tensormap(&tm_v);
     }
     if (threadIdx.x == 0) {
-        const uint32_t fault_word = *reinterpret_cast<volatile uint32_t*>(p.fault);
         mbar_init(q_full, 1);
         mbar_init(q_empty, 1);
         for (int i = 0; i < 2; ++i) {
@@ -153,15 +156,20 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             mbar_init(&s_full[i], 1);
             mbar_init(&p_half[2 * i], 8);
             mbar_init(&p_half[2 * i + 1], 8);
-            mbar_init(&fin[i], 4);
         }
-        for (int i = 0; i < 4; ++i) mbar_init(&gate_bar[i], 1);
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(&fin[i], 4);
+            mbar_init(&gate_bar[i], 1);
+        }
         mbar_init(o_full, 1);
         mbar_init(o_empty, 8);
         fence_mbar_init();
-        *abort_slot = fault_word != 0u ? 1u : 0u;
     }
     if (warp == C::PRODUCER_WARP) tmem_alloc_pair(tmem_slot, 512);
+    // Up to here nothing depends on the kernels in front; everything below may.
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (threadIdx.x == 0) *abort_slot = *reinterpret_cast<volatile uint32_t*>(p.fault) != 0u ? 1u : 0u;
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -344,11 +352,11 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 continue;
             }
             if (warp_store) stage_begin<GATE>(stage, &tm_gate, lane, 0, w.h, t0, w.b);
-            if (!mbar_wait_relaxed_warp<2>(&fin[n & 1], (n >> 1) & 1)) {
+            if (!mbar_wait_relaxed_warp<2>(&fin[n & 3], (n >> 2) & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x500u);
                 break;
             }
-            const float row_l = fin_vals[(n & 1) * 128 + r];
+            const float row_l = fin_vals[(n & 3) * 128 + r];
             if (!mbar_wait_relaxed_warp<2>(o_full, n & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, n);
                 break;
@@ -501,10 +509,10 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 mbar_arrive_remote_warp(b_half + 16 * st + 8);
             }
             if (ok) {
-                fin_vals[(n & 1) * 128 + r] = l;
+                fin_vals[(n & 3) * 128 + r] = l;
                 if (p.out_lse && t < p.seq)
                     p.out_lse[((long long)w.b * p.seq + t) * p.nq + w.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
-                mbar_arrive_warp(&fin[n & 1]);
+                mbar_arrive_warp(&fin[n & 3]);
                 ++n;
             }
         }

@@ -113,6 +113,8 @@ __global__ void __launch_bounds__(256) qkv_prepare_kernel(const QkvPrepareParams
             s_inv[pr] = 1.0f / powf(p.theta, 2.0f * pr / static_cast<float>(QWEN ? p.freq_denom : HD));
         __syncthreads();
     }
+    grid_dependency_wait();  // (the frequencies above depend on no kernel in front)
+    grid_launch_dependents();
     int it = 0;
     for (int rd = blockIdx.x; rd < rounds; rd += gridDim.x, ++it) {
         const int tk0 = rd * tpc;
