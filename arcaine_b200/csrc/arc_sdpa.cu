@@ -40,6 +40,7 @@ struct DeviceState {
     // [head dim 128 / 256][log2(cluster size)]: how many clusters of 2 or 4 CTAs of the cluster form of the
     // prefill kernel the device can hold at once (0: that size cannot be launched)
     int active_clusters[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    int decode_clusters[4] = {0, 0, 0, 0};  // [log2(size)]: clusters of the one-launch decode the device holds at once
     int wide_pairs = 0;  // CTA pairs of the head-dim-256 kernel the device holds at once
 };
 
@@ -145,10 +146,16 @@ static int device_state(DeviceState** out) {
                 std::snprintf(g_last_error, sizeof(g_last_error), "the device cannot hold a CTA pair of the prefill kernel");
                 return ARC_ERR_CUDA;
             }
-            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1>, s.smem_optin - kDecodeStaticSmem));
-            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2>, s.smem_optin - kDecodeStaticSmem));
-            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1>, s.smem_optin - kDecodeStaticSmem));
-            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, false>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, true>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, false>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, true>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, false>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, true>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, false>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, true>, s.smem_optin - kDecodeStaticSmem));
+            for (int lg = 0; lg < 4; ++lg)
+                s.decode_clusters[lg] = clusters_at_once(sdpa_decode_kernel<256, 1, true>, 1 << lg, s.sm_count, 288, s.smem_optin - kDecodeStaticSmem);
             s.ready.store(true, std::memory_order_release);
         }
     }
@@ -486,9 +493,67 @@ struct DecodePlan {
     int smem_bytes = 0;
     long long parts = 0;
     size_t ws_bytes = 0;
+    bool cluster = false;  // one launch: a cluster of `ncta` CTAs per sequence and group of KV heads
 };
 
-static int plan_decode(const arc_sdpa_decode_params* p, int sm_count, int smem_optin, DecodePlan* plan) {
+// Shared memory of a CTA that works on `nkv_cta` KV heads: slices, stages, bytes.  False: not even two stages fit.
+static bool size_decode_cta(int hd, int nkv_cta, int batch, int smem_optin, DecodePlan* plan) {
+    const int row_bytes = nkv_cta * hd * 2;
+    int slices = (64 * 1024) / (32 * row_bytes);
+    if (slices > 8 / nkv_cta) slices = 8 / nkv_cta;
+    if (slices < 1) slices = 1;
+    const int stage_bytes = 2 * 16 * slices * row_bytes;
+    const int fixed = 1024 + 2 * 8 * 8 + (batch + 2) * 8;
+    int stages = (smem_optin - kDecodeStaticSmem - fixed) / stage_bytes;
+    if (stages > 4) stages = 4;
+    plan->nkv_cta = nkv_cta;
+    plan->slices = slices;
+    plan->stages = stages;
+    plan->smem_bytes = stages * stage_bytes + fixed;
+    return stages >= 2;
+}
+
+// One launch or two?  A cluster of up to eight CTAs per sequence and group of heads finishes alone: 6 us plus the time its
+// CTAs take for their part of the longest sequence, at the 58 GB/s one CTA pulls at head dim 256 (four consumer warps) and
+// 93 at 128 (eight), or their share of the memory's rate.  Equal shares over all SMs read the total at 6.9 TB/s,
+// but cost 9 us and 0.12 us per sequence for the second launch and the records.  (Measured over
+// batches of 1 to 64 and lengths of 32 to 8192 for four head layouts; one token over 513 keys, 24/4 heads: 11.8 -> 7.6 us,
+// 64 sequences of 512 keys, 16/2 heads: 21.7 -> 10.3.)  Lengths on the device are not known here: the longest sequence is
+// taken to be as long as its bound says, or twice the mean of a packed cache, the others half of that.
+static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceState& ds, int nkv_cta, DecodePlan* plan) {
+    if (p->num_ctas != 0 || p->xchg_world > 1 || p->kv_rows_total == 0 || p->batch > 1024) return;
+    const int G = p->nq / p->nkv;
+    int heads = 0, csize = 0;  // the smallest group of heads and then the largest cluster that are all resident at once
+    for (int c = 1; c <= nkv_cta && !heads; ++c)
+        if (p->nkv % c == 0 && (long long)p->batch * (p->nkv / c) <= ds.decode_clusters[0]) heads = c;
+    for (int lg = 3; heads && lg >= 0 && !csize; --lg)
+        if ((long long)p->batch * (p->nkv / heads) <= ds.decode_clusters[lg]) csize = 1 << lg;
+    if (!csize) return;
+    double longest = (double)p->kv_len_uniform, total = longest * p->batch;
+    if (p->kv_len) {
+        longest = (double)(p->max_kv_len > 0 ? p->max_kv_len : p->kv_rows_total);
+        if (p->kv_row_offset && p->batch > 1 && longest > 2.0 * (double)p->kv_rows_total / p->batch)
+            longest = 2.0 * (double)p->kv_rows_total / p->batch;
+        total = longest * (0.5 * p->batch + 0.5);
+    }
+    double rate = p->hd == 256 ? 58e3 : 93e3;
+    const double even = 6.9e6 / ((double)p->batch * (p->nkv / heads) * csize);
+    if (rate > even) rate = even;
+    const double t_cluster = 6.0 + longest / csize * heads * p->hd * 4.0 / rate;
+    const double t_shares = 9.0 + 0.12 * p->batch + total * p->nkv * p->hd * 4.0 / 6.9e6;
+    if (t_cluster > t_shares) return;
+    DecodePlan one = *plan;
+    if (!size_decode_cta(p->hd, heads, 0, ds.smem_optin, &one)) return;
+    const int ncw = heads * one.slices;  // the records must fit where the stages were
+    if ((ncw * one.nt * 8 + heads * G) * (p->hd + 1) * 4 > one.stages * 2 * 16 * one.slices * heads * p->hd * 2) return;
+    one.cluster = true;
+    one.groups = p->nkv / heads;
+    one.ncta = csize;
+    *plan = one;
+}
+
+static int plan_decode(const arc_sdpa_decode_params* p, const DeviceState& ds, DecodePlan* plan) {
+    const int sm_count = ds.sm_count, smem_optin = ds.smem_optin;
     if (!p) return ARC_ERR_NULL_POINTER;
     if (p->batch <= 0 || p->nq <= 0 || p->nkv <= 0 || p->nq % p->nkv != 0) return ARC_ERR_BAD_SHAPE;
     if (p->batch > DECODE_MAX_BATCH) return ARC_ERR_TOO_LARGE;
@@ -512,26 +577,15 @@ static int plan_decode(const arc_sdpa_decode_params* p, int sm_count, int smem_o
     int nkv_cta = 1;
     for (int c = 1; c <= p->nkv && c <= max_heads; ++c)
         if (p->nkv % c == 0) nkv_cta = c;
-    plan->nkv_cta = nkv_cta;
+    if (!size_decode_cta(p->hd, nkv_cta, p->batch, smem_optin, plan)) return ARC_ERR_TOO_LARGE;
     plan->groups = p->nkv / nkv_cta;
-    const int row_bytes = nkv_cta * p->hd * 2;
-    int slices = (64 * 1024) / (32 * row_bytes);
-    if (slices > 8 / nkv_cta) slices = 8 / nkv_cta;
-    if (slices < 1) slices = 1;
-    plan->slices = slices;
-    const int stage_bytes = 2 * 16 * slices * row_bytes;
-    const int fixed = 1024 + 2 * 8 * 8 + (p->batch + 2) * 8;
-    int stages = (smem_optin - kDecodeStaticSmem - fixed) / stage_bytes;
-    if (stages > 4) stages = 4;
-    if (stages < 2) return ARC_ERR_TOO_LARGE;
-    plan->stages = stages;
-    plan->smem_bytes = stages * stage_bytes + fixed;
     int ncta = p->num_ctas > 0 ? p->num_ctas : sm_count / plan->groups;
     if (ncta < 1) ncta = 1;
     if (ncta > 1024) ncta = 1024;
     plan->ncta = ncta;
-    plan->parts = ((long long)ncta + p->batch) * slices;
+    plan->parts = ((long long)ncta + p->batch) * plan->slices;
     plan->ws_bytes = (size_t)plan->parts * p->nq * ((size_t)p->hd + 1) * sizeof(float);
+    plan_decode_cluster(p, ds, nkv_cta, plan);  // (the workspace asked for stays that of the form above)
     return ARC_OK;
 }
 
@@ -569,8 +623,20 @@ static int launch_decode(const arc_sdpa_decode_params* p, const DecodePlan& plan
 
     dim3 grid((unsigned)plan.ncta, (unsigned)plan.groups, 1);
     const unsigned threads = 32u * (unsigned)(plan.nkv_cta * plan.slices + 1);
+    if (plan.cluster) {
+        kp.gate = static_cast<const uint16_t*>(p->gate);
+        kp.out = static_cast<uint16_t*>(p->out);
+        kp.out_f32 = p->out_f32;
+        kp.out_lse = p->out_lse;
+        kp.o_stride_b = p->o_stride_b;
+        grid.z = (unsigned)p->batch;
+        ARC_CUDA(launch_dependent(plan.nt == 1 ? sdpa_decode_kernel<HD, 1, true> : sdpa_decode_kernel<HD, 2, true>, grid, dim3(threads),
+                                  (size_t)plan.smem_bytes, stream, plan.ncta, tk, tv, kp));
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        return ARC_OK;
+    }
     if (!empty_cache) {
-        ARC_CUDA(launch_dependent(plan.nt == 1 ? sdpa_decode_kernel<HD, 1> : sdpa_decode_kernel<HD, 2>, grid, dim3(threads),
+        ARC_CUDA(launch_dependent(plan.nt == 1 ? sdpa_decode_kernel<HD, 1, false> : sdpa_decode_kernel<HD, 2, false>, grid, dim3(threads),
                                   (size_t)plan.smem_bytes, stream, 1, tk, tv, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
@@ -669,7 +735,7 @@ extern "C" size_t arc_sdpa_decode_workspace_bytes(const arc_sdpa_decode_params* 
     DeviceState* ds = nullptr;
     if (device_state(&ds) != ARC_OK) return 0;
     DecodePlan plan;
-    if (plan_decode(p, ds->sm_count, ds->smem_optin, &plan) != ARC_OK) return 0;
+    if (plan_decode(p, *ds, &plan) != ARC_OK) return 0;
     return plan.ws_bytes;
 }
 
@@ -686,7 +752,7 @@ extern "C" int arc_sdpa_decode(const arc_sdpa_decode_params* p, void* stream) {
     int rc = device_state(&ds);
     if (rc != ARC_OK) return rc;
     DecodePlan plan;
-    if ((rc = plan_decode(p, ds->sm_count, ds->smem_optin, &plan)) != ARC_OK) return rc;
+    if ((rc = plan_decode(p, *ds, &plan)) != ARC_OK) return rc;
     if (!aligned16(p->q) || (p->kv_rows_total != 0 && (!aligned16(p->k) || !aligned16(p->v))) || (p->out && !aligned16(p->out)) ||
         (p->gate && !aligned16(p->gate)) || (p->out_f32 && !aligned16(p->out_f32)))
         return ARC_ERR_ALIGNMENT;

@@ -55,29 +55,32 @@ struct DecodeParams {
     int ncta;     // grid.x
     int max_kv_len;            // > 0: no sequence may be longer
     long long kv_rows_total;   // rows addressable from k and v
+    // The form that finishes in one launch (sdpa_decode_kernel<.., true>): the results
+    const uint16_t* gate;
+    uint16_t* out;
+    float* out_f32;
+    float* out_lse;
+    long long o_stride_b;
 };
 
 // Prefix sums of the per-sequence lengths into shared memory: cum[b] = keys before sequence b, cum[batch] = total.
-// Called by every thread of the block; the first warp scans, 32 sequences a step (one thread adding them up in turn
-// took a microsecond for 64).
+// Called by the first warp, which scans 32 sequences a step (one thread adding them up in turn took a microsecond for
+// 64); the caller's barrier follows.
 __device__ __forceinline__ void build_len_prefix(const int* kv_len, int kv_len_uniform, int batch, long long* cum) {
-    if (threadIdx.x < 32) {
-        long long run = 0;
-        if (threadIdx.x == 0) cum[0] = 0;
-        for (int b0 = 0; b0 < batch; b0 += 32) {
-            const int b = b0 + threadIdx.x;
-            const int len = b < batch ? (kv_len ? kv_len[b] : kv_len_uniform) : 0;
-            long long v = len > 0 ? len : 0;
+    long long run = 0;
+    if (threadIdx.x == 0) cum[0] = 0;
+    for (int b0 = 0; b0 < batch; b0 += 32) {
+        const int b = b0 + threadIdx.x;
+        const int len = b < batch ? (kv_len ? kv_len[b] : kv_len_uniform) : 0;
+        long long v = len > 0 ? len : 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long up = __shfl_up_sync(0xffffffffu, v, o);
-                if ((int)threadIdx.x >= o) v += up;
-            }
-            if (b < batch) cum[b + 1] = run + v;
-            run += __shfl_sync(0xffffffffu, v, 31);
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long up = __shfl_up_sync(0xffffffffu, v, o);
+            if ((int)threadIdx.x >= o) v += up;
         }
+        if (b < batch) cum[b + 1] = run + v;
+        run += __shfl_sync(0xffffffffu, v, 31);
     }
-    __syncthreads();
 }
 
 __device__ __forceinline__ long long share_size(long long total, int ncta, int tile_keys) {
@@ -86,12 +89,21 @@ __device__ __forceinline__ long long share_size(long long total, int ncta, int t
     return per > 0 ? per : tile_keys;
 }
 
+__device__ __forceinline__ float sigmoid_gate(float attn, uint16_t gate_bits) {
+    const float g = bf16_bits_to_f32(gate_bits);
+    return bf16_round(attn) * (1.0f / (1.0f + __expf(-g)));
+}
+
 // All consumer warps of the CTA (named barrier 1; the producer warp does not take part).
 __device__ __forceinline__ void consumer_sync(int consumer_warps) {
     asm volatile("bar.sync 1, %0;" ::"r"(consumer_warps * 32) : "memory");
 }
 
-template <int HD, int NT>
+// CLUSTER: a cluster of CTAs owns one sequence (grid.z) and one group of KV heads (grid.y); its CTAs take equal parts of
+// the sequence's keys, fold their slices as above, then fold each other's records through distributed shared
+// memory and write the result: one launch, no records in global memory, no merge kernel.  For calls so small that the
+// launches are what they cost; otherwise equal shares over all SMs win.
+template <int HD, int NT, bool CLUSTER>
 __global__ void __launch_bounds__(288, 1)
     sdpa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const DecodeParams p) {
@@ -116,7 +128,6 @@ __global__ void __launch_bounds__(288, 1)
     const int head0 = blockIdx.y * p.nkv_cta;  // first KV head of this CTA
     const int G = p.nq / p.nkv;
 
-    __shared__ uint32_t abort_flag;
     if (threadIdx.x == 32) {
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
@@ -131,36 +142,44 @@ __global__ void __launch_bounds__(288, 1)
     // Up to here nothing depends on the kernels in front; everything below may.
     grid_dependency_wait();
     grid_launch_dependents();  // the merge kernel may be scheduled now; it waits for this grid before reading
-    // A fault recorded by an earlier CTA or launch: do not start new waits.  Everything the prologue reads from global
-    // memory is asked for at once: after an L2 flush each of these is an HBM round trip, and taken one after the other
-    // (status word and lengths, then row offsets) they kept the first K / V request waiting.
-    if (p.kv_row_offset)
-        for (int b = threadIdx.x * 16; b < p.batch; b += blockDim.x * 16) prefetch_l2(p.kv_row_offset + b);
-    if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile uint32_t*>(p.fault);
-    build_len_prefix(p.kv_len, p.kv_len_uniform, p.batch, cum);
-    if (abort_flag != 0u) return;
-    // Lengths and row offsets live on the device, so this is where they can be checked: a sequence
-    // that reaches past the cache (the copies would read zero rows and fold them in as score-0
-    // keys) or past the stated bound stops the launch with a status instead of a wrong result.
+    // The status word, the lengths and the row offsets are asked for together: each is a trip to L2 or HBM.
+    // Lengths and row offsets live on the device, so this is where they can be checked: a sequence that reaches past the
+    // cache (the copies would read zero rows and fold them in as score-0 keys) or past the stated bound stops the
+    // launch with a status instead of a wrong result.  Every CTA checks all sequences and so none of them works.
+    bool bad = threadIdx.x == 0 && *reinterpret_cast<volatile uint32_t*>(p.fault) != 0u;
     for (int b = threadIdx.x; b < p.batch; b += blockDim.x) {
-        const long long len = cum[b + 1] - cum[b];
+        const int len = p.kv_len ? p.kv_len[b] : p.kv_len_uniform;
         const long long row0 = p.kv_row_offset ? p.kv_row_offset[b] : (long long)b * p.kv_stride_b;
         if ((len > 0 && (row0 < 0 || row0 + len > p.kv_rows_total)) || (p.max_kv_len > 0 && len > p.max_kv_len)) {
             report_fault(p.fault, FAULT_BAD_KV_RANGE, (uint32_t)b);
-            abort_flag = 1u;
+            bad = true;
         }
     }
-    __syncthreads();
-    if (abort_flag != 0u) return;
-    const long long total = cum[p.batch];
-    const long long per = share_size(total, p.ncta, tk);
-    const long long g0 = (long long)blockIdx.x * per;
-    const long long g1 = min(total, g0 + per);
-
-    if (g0 >= g1) return;  // (the barriers were set up before the prefix's block-wide syncs)
-
+    if (!CLUSTER && threadIdx.x < 32) build_len_prefix(p.kv_len, p.kv_len_uniform, p.batch, cum);
+    const int my_len = CLUSTER ? max(0, p.kv_len ? p.kv_len[blockIdx.z] : p.kv_len_uniform) : 0;
+    const bool work = !__syncthreads_or(bad);
+    long long g0, g1;  // this CTA's keys, counted over the sequences laid end to end (CLUSTER: of its own sequence)
     int b_first = 0;
-    while (b_first < p.batch - 1 && cum[b_first + 1] <= g0) ++b_first;
+    if constexpr (CLUSTER) {
+        b_first = blockIdx.z;
+        const int per = ((my_len + p.ncta - 1) / p.ncta + 15) / 16 * 16;
+        g0 = (long long)blockIdx.x * per;
+        g1 = work ? min((long long)my_len, g0 + per) : g0;
+    } else {
+        if (!work) return;
+        const long long total = cum[p.batch];
+        const long long per = share_size(total, p.ncta, tk);
+        g0 = (long long)blockIdx.x * per;
+        g1 = min(total, g0 + per);
+        if (g0 >= g1) return;
+        while (b_first < p.batch - 1 && cum[b_first + 1] <= g0) ++b_first;
+    }
+    // keys before sequence b / up to its end, in the count g0 and g1 use
+    auto seq_begin = [&](int b) { return CLUSTER ? 0ll : cum[b]; };
+    auto seq_end = [&](int b) { return CLUSTER ? (long long)my_len : cum[b + 1]; };
+    // CLUSTER: this CTA's folded record of every head of its group, behind the warps' records
+    float* crec = reinterpret_cast<float*>(stage_base) + (size_t)ncw * NT * 8 * (HD + 1);
+    float* crec_lse = crec + (size_t)p.nkv_cta * G * HD;
 
     if (warp == ncw) {
         // ------------------------------------------------------------------ producer
@@ -169,9 +188,9 @@ __global__ void __launch_bounds__(288, 1)
         int b = b_first;
         long long g = g0;
         while (ok && g < g1) {
-            while (cum[b + 1] <= g) ++b;
-            const long long seg_end = min(g1, cum[b + 1]);
-            const long long row0 = (p.kv_row_offset ? p.kv_row_offset[b] : (long long)b * p.kv_stride_b) + (g - cum[b]);
+            while (seq_end(b) <= g) ++b;
+            const long long seg_end = min(g1, seq_end(b));
+            const long long row0 = (p.kv_row_offset ? p.kv_row_offset[b] : (long long)b * p.kv_stride_b) + (g - seq_begin(b));
             const int seg_keys = (int)(seg_end - g);
             for (int k0 = 0; k0 < seg_keys; k0 += tk, ++it) {
                 const int st = it % p.stages;
@@ -217,8 +236,8 @@ __global__ void __launch_bounds__(288, 1)
         int b = b_first;
         long long g = g0;
         while (ok && g < g1) {
-            while (cum[b + 1] <= g) ++b;
-            const long long seg_end = min(g1, cum[b + 1]);
+            while (seq_end(b) <= g) ++b;
+            const long long seg_end = min(g1, seq_end(b));
             const int seg_keys = (int)(seg_end - g);
 
             // Q^T fragments (B operand, hd x 8 heads) for this head's GQA group.
@@ -346,10 +365,10 @@ __global__ void __launch_bounds__(288, 1)
             // The last segment of the share (for most CTAs the only one) is folded across the slices inside
             // the CTA first: the stages are free by then, so each warp leaves its record in shared memory,
             // and the warps of a KV head combine them into ONE record per (CTA, sequence), stored in slice
-            // 0's slot; the other slices' slots are marked empty (lse = -inf).  The merge kernel then reads
+            // 0's slot; the other slices' slots stay unwritten.  The merge kernel then reads
             // `slices` times fewer records.  Earlier segments (a sequence boundary inside the share) write
             // one record per slice.
-            const bool fold_here = p.slices > 1 && seg_end == g1;  // CTA-uniform
+            const bool fold_here = CLUSTER || (p.slices > 1 && seg_end == g1);  // CTA-uniform
             float* rec = reinterpret_cast<float*>(stage_base);     // [warp][NT * 8 heads][HD]
             float* rec_lse = rec + (size_t)ncw * NT * 8 * HD;      // [warp][NT * 8]
             if (fold_here) {
@@ -417,19 +436,81 @@ __global__ void __launch_bounds__(288, 1)
                         const float iz = 1.f / z;
                         acc = make_float4(acc.x * iz, acc.y * iz, acc.z * iz, acc.w * iz);
                     }
-                    const long long row = part0 * p.nq + (long long)kvh * G + n;
-                    *reinterpret_cast<float4*>(p.part_o + row * HD + d) = acc;
-                    if (d == 0) p.part_lse[row] = mx > -CUDART_INF_F ? mx + __logf(z) : -CUDART_INF_F;
+                    const float rec_l = mx > -CUDART_INF_F ? mx + __logf(z) : -CUDART_INF_F;
+                    if constexpr (CLUSTER) {
+                        *reinterpret_cast<float4*>(crec + (size_t)(hl * G + n) * HD + d) = acc;
+                        if (d == 0) crec_lse[hl * G + n] = rec_l;
+                    } else {
+                        const long long row = part0 * p.nq + (long long)kvh * G + n;
+                        *reinterpret_cast<float4*>(p.part_o + row * HD + d) = acc;
+                        if (d == 0) p.part_lse[row] = rec_l;
+                    }
                 }
-                if (slice > 0 && lane < G) p.part_lse[(part0 + slice) * p.nq + (long long)kvh * G + lane] = -CUDART_INF_F;
             }
             g = seg_end;
         }
         // A warp that gave up a wait never reached the fold: it still meets the others at both barriers.
-        if (p.slices > 1 && !folded) {
+        if (!folded && (CLUSTER || p.slices > 1)) {
             consumer_sync(ncw);
             consumer_sync(ncw);
         }
+        // (CLUSTER: no keys: an empty record)
+        if (CLUSTER && !folded)
+            for (int n = slice * 32 + lane; n < G; n += p.slices * 32) crec_lse[hl * G + n] = -CUDART_INF_F;
+    }
+    if constexpr (CLUSTER) {
+        __syncwarp();
+        cluster_sync_all();  // every CTA's records are in its shared memory
+        // this CTA's part of the (head, 4 columns) items, all records of an item in flight at once
+        const int heads = p.nkv_cta * G, items = heads * (HD / 4), C = p.ncta;
+        const uint32_t a_lse = smem_u32(crec_lse), a_rec = smem_u32(crec);
+        const int b = blockIdx.z;
+        for (int item = blockIdx.x * blockDim.x + threadIdx.x; work && item < items; item += C * blockDim.x) {
+            const int n = item / (HD / 4), d = (item % (HD / 4)) * 4;
+            const int h = head0 * G + n;
+            const long long eoff = (long long)b * p.o_stride_b + (long long)h * HD + d;
+            const uint2 gw = p.gate ? *reinterpret_cast<const uint2*>(p.gate + eoff) : make_uint2(0u, 0u);
+            float li[8];
+            float4 ov[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                li[c] = -CUDART_INF_F;
+                if (c < C) {
+                    li[c] = ld_cluster_f32(map_to_cta(a_lse + n * 4, c));
+                    ov[c] = ld_cluster_f32x4(map_to_cta(a_rec + (n * HD + d) * 4, c));
+                }
+            }
+            float mx = li[0];
+#pragma unroll
+            for (int c = 1; c < 8; ++c) mx = fmaxf(mx, li[c]);
+            float z = 0.f, a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                if (li[c] == -CUDART_INF_F) continue;  // an empty record may hold anything
+                const float wt = __expf(li[c] - mx);
+                z += wt;
+                a[0] = fmaf(wt, ov[c].x, a[0]);
+                a[1] = fmaf(wt, ov[c].y, a[1]);
+                a[2] = fmaf(wt, ov[c].z, a[2]);
+                a[3] = fmaf(wt, ov[c].w, a[3]);
+            }
+            const float iz = z > 0.f ? 1.f / z : 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[e] *= iz;
+            const long long row = (long long)b * p.nq + h;
+            if (p.out_f32) *reinterpret_cast<float4*>(p.out_f32 + row * HD + d) = make_float4(a[0], a[1], a[2], a[3]);
+            if (p.out_lse && d == 0) p.out_lse[row] = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
+            if (p.out) {
+                if (p.gate) {
+                    a[0] = sigmoid_gate(a[0], (uint16_t)(gw.x & 0xffffu));
+                    a[1] = sigmoid_gate(a[1], (uint16_t)(gw.x >> 16));
+                    a[2] = sigmoid_gate(a[2], (uint16_t)(gw.y & 0xffffu));
+                    a[3] = sigmoid_gate(a[3], (uint16_t)(gw.y >> 16));
+                }
+                *reinterpret_cast<uint2*>(p.out + eoff) = make_uint2(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]));
+            }
+        }
+        cluster_sync_all();  // nobody's shared memory goes while another CTA still reads it
     }
 }
 
@@ -479,10 +560,6 @@ __device__ __forceinline__ uint4 ld_volatile_v4(const uint4* p) {
     return v;
 }
 
-__device__ __forceinline__ float sigmoid_gate(float attn, uint16_t gate_bits) {
-    const float g = bf16_bits_to_f32(gate_bits);
-    return bf16_round(attn) * (1.0f / (1.0f + __expf(-g)));
-}
 
 constexpr int MERGE_THREADS = 256;
 
@@ -533,52 +610,45 @@ __global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const 
     float lse = -CUDART_INF_F, inv = 0.f;
     if (k_len > 0) {  // block-uniform
         const int c_first = (int)(k_begin / per), c_last = (int)((k_end - 1) / per);
-        const int n_parts = (c_last - c_first + 1) * p.slices;
         const long long part0 = ((long long)c_first + b) * p.slices;
-        const float* lses = p.part_lse + part0 * p.nq + h;
+        // Which records exist follows from the shares: a share whose last segment is this sequence's folded its slices
+        // into slice 0's record — every share but possibly the last, whose slices wrote one record each if the
+        // sequence ends before the share does.
+        const int n_full = c_last - c_first;
+        const int n_rec = n_full + (k_end == min(total, (c_last + 1) * per) ? 1 : p.slices);
+        auto rec_of = [&](int j) { return part0 + (j < n_full ? (long long)j * p.slices : (long long)n_full * p.slices + (j - n_full)); };
+        const float* lses = p.part_lse + h;
         float mx = -CUDART_INF_F;
-        for (int i = lane; i < n_parts; i += 32) mx = fmaxf(mx, lses[(long long)i * p.nq]);
+        for (int j = lane; j < n_rec; j += 32) mx = fmaxf(mx, lses[rec_of(j) * p.nq]);
+        // The records are dealt to the warps in turn, four at a time with their loads in flight together (and beside
+        // those of the weights); a lane owns VPL consecutive output values.  Always the same order of additions.
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (mx > -CUDART_INF_F) {
-            // Most records carry no weight (the decode kernel folds the slices of a share's last segment into slice
-            // 0's slot and marks the others empty): the live ones are dealt to the warps in turn, in order, so the
-            // fold is spread evenly and always adds in the same order; four at a time, their loads in flight
-            // together; a lane owns VPL consecutive output values.
             float z = 0.f;
-            int seen = 0;  // live records before this group of 32
-            for (int i0 = 0; i0 < n_parts; i0 += 32) {
-                const int i = i0 + lane;
-                const float w = i < n_parts ? __expf(lses[(long long)i * p.nq] - mx) : 0.f;  // exp(-inf) = 0 for empty records
-                z += w;
-                const uint32_t live = __ballot_sync(0xffffffffu, w != 0.f);
-                // this warp's: the record's rank among the live ones, modulo the warps
-                uint32_t mine = __ballot_sync(0xffffffffu, w != 0.f && ((seen + __popc(live & ((1u << lane) - 1u))) % NW) == warp);
-                seen += __popc(live);
-                while (mine) {
-                    constexpr int U = 4;
-                    float wu[U];
-                    float4 ov[U][VPL / 4];
+            for (int j = lane; j < n_rec; j += 32) z += __expf(lses[rec_of(j) * p.nq] - mx);  // exp(-inf) = 0: an empty slice
+            constexpr int U = 4;
+            for (int j0 = warp; j0 < n_rec; j0 += NW * U) {
+                float wu[U];
+                float4 ov[U][VPL / 4];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int src = mine ? __ffs(mine) - 1 : 0;
-                        wu[u] = __shfl_sync(0xffffffffu, w, src);
-                        if (!mine) wu[u] = 0.f;
-                        mine &= mine - 1;
-                        const float* rec = p.part_o + ((part0 + i0 + src) * p.nq + h) * HD + lane * VPL;
+                for (int u = 0; u < U; ++u) {
+                    const int j = j0 + u * NW;
+                    const long long rec = rec_of(j < n_rec ? j : j0);
+                    wu[u] = j < n_rec ? lses[rec * p.nq] : -CUDART_INF_F;
+                    const float* src = p.part_o + (rec * p.nq + h) * HD + lane * VPL;
 #pragma unroll
-                        for (int j = 0; j < VPL / 4; ++j)
-                            ov[u][j] = wu[u] != 0.f ? *reinterpret_cast<const float4*>(rec + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
+                    for (int i = 0; i < VPL / 4; ++i) ov[u][i] = *reinterpret_cast<const float4*>(src + 4 * i);
+                }
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
+                for (int u = 0; u < U; ++u) {
+                    const float w = __expf(wu[u] - mx);
 #pragma unroll
-                        for (int j = 0; j < VPL / 4; ++j) {
-                            acc[4 * j] = fmaf(wu[u], ov[u][j].x, acc[4 * j]);
-                            acc[4 * j + 1] = fmaf(wu[u], ov[u][j].y, acc[4 * j + 1]);
-                            acc[4 * j + 2] = fmaf(wu[u], ov[u][j].z, acc[4 * j + 2]);
-                            acc[4 * j + 3] = fmaf(wu[u], ov[u][j].w, acc[4 * j + 3]);
-                        }
+                    for (int i = 0; i < VPL / 4; ++i) {
+                        acc[4 * i] = fmaf(w, ov[u][i].x, acc[4 * i]);
+                        acc[4 * i + 1] = fmaf(w, ov[u][i].y, acc[4 * i + 1]);
+                        acc[4 * i + 2] = fmaf(w, ov[u][i].z, acc[4 * i + 2]);
+                        acc[4 * i + 3] = fmaf(w, ov[u][i].w, acc[4 * i + 3]);
                     }
                 }
             }

@@ -254,6 +254,12 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
     return v;
 }
 
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ float2 ld_cluster_f32x2(uint32_t addr) {
     float2 v;
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");

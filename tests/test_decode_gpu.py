@@ -264,3 +264,36 @@ def test_empty_cache_slice_gives_empty_records(ops):
     out, o32, lse = ops.sdpa_decode(q, k, k, scale=0.1, return_partial=True)
     assert torch.count_nonzero(out.float()) == 0 and torch.count_nonzero(o32) == 0
     assert torch.isinf(lse).all() and (lse < 0).all()
+
+
+@pytest.mark.parametrize("B,nq,nkv,hd,lens", [
+    (1, 24, 4, 256, [1]),                      # one key: seven of eight CTAs of a cluster have none
+    (1, 6, 1, 128, [1000]),                    # one group of heads
+    (5, 32, 2, 128, [129, 16, 0, 640, 333]),   # 16 query heads per KV head, an empty sequence
+    (37, 24, 4, 256, [i * 7 for i in range(37)]),   # as many clusters of one CTA as fit
+    (70, 16, 8, 256, [40 + i for i in range(70)]),  # several KV heads per CTA
+])
+def test_one_launch_form(ops, B, nq, nkv, hd, lens):
+    """Short calls: a cluster per sequence and group of heads writes the result itself (one launch), from a block cache and
+    from a packed one, with the gate and with the partial outputs."""
+    cap = max(lens)
+    q, k, v = seeded_bf16(B, nq, hd, seed=1), seeded_bf16(B, cap, nkv, hd, seed=2), seeded_bf16(B, cap, nkv, hd, seed=3)
+    g = seeded_bf16(B, nq, hd, seed=4)
+    kl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    before = ops.launch_count()
+    out, o32, lse = ops.sdpa_decode(q.cuda(), k.cuda(), v.cuda(), scale=hd ** -0.5, kv_len=kl, gate=g.cuda(), return_partial=True)
+    assert ops.launch_count() - before == 1
+    kp, vp = (torch.cat([t[b, :n] for b, n in enumerate(lens)]).cuda() for t in (k, v))
+    offs = torch.tensor([sum(lens[:b]) for b in range(B)], dtype=torch.int64, device="cuda")
+    packed = ops.sdpa_decode(q.cuda(), kp, vp, scale=hd ** -0.5, kv_len=kl, kv_row_offset=offs, gate=g.cuda())
+    two = ops.sdpa_decode(q.cuda(), k.cuda(), v.cuda(), scale=hd ** -0.5, kv_len=kl, gate=g.cuda(), num_ctas=148)  # shares and merge
+    assert_close(packed, two.float(), "packed", rel_tol=5e-3)
+    for b in range(0, B, max(1, B // 8)):
+        if lens[b] == 0:
+            assert torch.count_nonzero(out[b].float()) == 0 and torch.isinf(lse[b]).all()
+            continue
+        wf, _, wl = oracle_decode(q[b], k[b, :lens[b]], v[b, :lens[b]], hd ** -0.5)
+        _, wgb, _ = oracle_decode(q[b], k[b, :lens[b]], v[b, :lens[b]], hd ** -0.5, gate=g[b])
+        assert_close(o32[b], wf[0], f"seq {b} f32", rel_tol=3e-3, abs_tol=5e-3)
+        assert_close(out[b], wgb[0].float(), f"seq {b} gated")
+        assert torch.allclose(lse[b].cpu(), wl[0], atol=2e-3)
