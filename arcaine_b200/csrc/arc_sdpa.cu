@@ -139,9 +139,11 @@ static int device_state(DeviceState** out) {
                            : clusters_at_once(sdpa_prefill_kernel<128, false, false, true>, cs, s.sm_count, PrefillCfg<128>::THREADS, PrefillCfg<128>::SMEM_BYTES);
                 }
             }
-            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false>, WideCfg::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true>, WideCfg::SMEM_BYTES));
-            s.wide_pairs = clusters_at_once(sdpa_prefill_wide_kernel<false>, 2, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
+            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, false>, WideCfg::SMEM_BYTES));
+            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true, false>, WideCfg::SMEM_BYTES));
+            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, true>, WideCfg::SMEM_BYTES));
+            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true, true>, WideCfg::SMEM_BYTES));
+            s.wide_pairs = clusters_at_once(sdpa_prefill_wide_kernel<false, false>, 2, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
             if (s.wide_pairs < 1) {
                 std::snprintf(g_last_error, sizeof(g_last_error), "the device cannot hold a CTA pair of the prefill kernel");
                 return ARC_ERR_CUDA;
@@ -246,7 +248,8 @@ struct PrefillPlan {
     int cluster = 0;         // > 0: the splits are the CTAs of a thread-block cluster of this size, folded in the kernel
     long long rows = 0;
     size_t split_bytes = 0;  // partial records of key-range splits, at the start of the workspace
-    size_t ws_bytes = 0;     // all of the workspace: partial records, then the per-row span ends of block_ids
+    size_t ws_bytes = 0;     // what must be there: partial records, then the per-row span ends of block_ids
+    size_t mask_bytes = 0;   // behind it, if it is there: the classes and bits of an additive mask
 };
 
 static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const int* active_clusters, PrefillPlan* plan) {
@@ -263,6 +266,8 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const in
     const int kv_blocks = (p->kv_len + 127) / 128;
     int splits = p->num_splits;
     const long long tiles = (long long)plan->q_tiles * p->nq * p->batch;
+    const bool scanned_mask = p->mask_type == ARC_MASK_EXPLICIT && p->hd == 256 && p->num_splits <= 1;
+    if (splits == 0 && scanned_mask) splits = 1;
     if (splits == 0) {
         // Split the key range only when the tiles alone leave most SMs idle and there are enough key blocks
         // to pay for folding the parts again (measured: about 8 us for the fold against 1.3-2 us per key
@@ -298,6 +303,7 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const in
     plan->split_bytes = splits > 1 ? (size_t)splits * plan->rows * ((size_t)p->hd + 1) * sizeof(float) : 0;
     plan->split_bytes = (plan->split_bytes + 15) & ~(size_t)15;
     plan->ws_bytes = plan->split_bytes;
+    if (scanned_mask) plan->mask_bytes = (size_t)plan->q_tiles * kv_blocks * (128 * sizeof(uint4) + sizeof(uint32_t));
     if (p->block_ids) {
         if (p->mask_type != ARC_MASK_CAUSAL || p->block_ids_offset < 0) return ARC_ERR_BAD_SHAPE;
         plan->ws_bytes += ((size_t)p->seq * sizeof(int32_t) + 15) & ~(size_t)15;
@@ -410,21 +416,38 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
 
     // Head dim 256, whole tiles, no additive mask: pairs of CTAs (prefill_wide_sm100.cuh) take 2300-2500 clk per key block
     // and pair of tiles where a CTA on its own takes 3700 per tile.
-    if (HD == 256 && plan.splits == 1 && plan.cluster == 0 && !(kp.mask_type == 1 && kp.mask != nullptr)) {
+    const bool masked = kp.mask_type == 1 && kp.mask != nullptr;
+    // (a caller who brings no workspace for the scanned mask gets the one-tile kernel, which reads the mask itself)
+    if (HD == 256 && plan.splits == 1 && plan.cluster == 0 &&
+        (!masked || (plan.mask_bytes > 0 && plan.q_tiles < 16384 && p->workspace && aligned16(p->workspace) && p->workspace_bytes >= plan.ws_bytes + plan.mask_bytes))) {
+        if (masked) {
+            kp.mask_blocks = (p->kv_len + 127) / 128;
+            uint4* bits = reinterpret_cast<uint4*>(static_cast<unsigned char*>(p->workspace) + plan.ws_bytes);
+            uint32_t* cls = reinterpret_cast<uint32_t*>(bits + (size_t)plan.q_tiles * kp.mask_blocks * 128);
+            ARC_CUDA(launch_dependent(mask_scan_kernel, dim3((unsigned)kp.mask_blocks, (unsigned)plan.q_tiles * 4), dim3(256), 0, stream, 1,
+                                      kp.mask, (int)p->seq, (int)p->kv_len, kp.mask_blocks, cls, bits));
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+            kp.mask_bits = bits;
+            kp.mask_class = cls;
+        }
         kp.head_pair = ((p->nq / p->nkv) & 1) == 0;
         kp.cur_heads = kp.head_pair ? p->nq / 2 : p->nq;
         kp.q_tiles = kp.head_pair ? plan.q_tiles : (p->seq + 255) / 256;
         const long long units = (long long)kp.q_tiles * kp.cur_heads * p->batch;
         if (units > 0x3fffffffLL) return ARC_ERR_TOO_LARGE;
         kp.total_tiles = (int)units;
-        // Units differ in length only under a causal mask without a window; longest first then, unless the K and V
-        // that all heads and sequences together read would not stay in L2 (126 MB).
+        // Under a causal mask (as most additive ones are, too) units differ in length — with a window only the first tiles are shorter, which matters
+        // while there are few waves of units — and go longest first then, unless the K and V that all heads and
+        // sequences together read would not stay in L2 (126 MB).  (1531 tokens, window 1024, 96 units on 74 pairs:
+        // 36.5 -> 27 us.)
         const bool windowed = p->window > 0 && p->window < p->kv_len;
-        kp.long_first = p->mask_type == ARC_MASK_CAUSAL && !windowed && units > ds->wide_pairs &&
+        kp.long_first = p->mask_type != ARC_MASK_NONE && units > ds->wide_pairs && (!windowed || units < 8LL * ds->wide_pairs) &&
                         (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;
         if ((rc = make_tile_map(&tk, p->k, HD, p->nkv, p->kv_len, p->batch, p->k_stride_t, p->k_stride_b, 64)) != ARC_OK) return rc;
         if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
-        ARC_CUDA(launch_dependent(kp.gate ? sdpa_prefill_wide_kernel<true> : sdpa_prefill_wide_kernel<false>,
+        auto kernel = masked ? (kp.gate ? sdpa_prefill_wide_kernel<true, true> : sdpa_prefill_wide_kernel<false, true>)
+                             : (kp.gate ? sdpa_prefill_wide_kernel<true, false> : sdpa_prefill_wide_kernel<false, false>);
+        ARC_CUDA(launch_dependent(kernel,
                                   dim3((unsigned)(2 * (units < ds->wide_pairs ? units : ds->wide_pairs))), dim3(WideCfg::THREADS),
                                   (size_t)WideCfg::SMEM_BYTES, stream, 2, tq, tk, tv, to, tg, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -700,7 +723,7 @@ extern "C" size_t arc_sdpa_prefill_workspace_bytes(const arc_sdpa_prefill_params
     if (device_state(&ds) == ARC_OK) sm = ds->sm_count;
     PrefillPlan plan;
     if (plan_prefill(p, sm, ds ? ds->active_clusters[p && p->hd == 256 ? 1 : 0] : nullptr, &plan) != ARC_OK) return 0;
-    return plan.ws_bytes;
+    return plan.ws_bytes + plan.mask_bytes;
 }
 
 extern "C" int arc_sdpa_prefill(const arc_sdpa_prefill_params* p, void* stream) {

@@ -57,6 +57,10 @@ struct PrefillParams {
     // of the head pair with unit index tail_base + (w >> 1), one tile per CTA; -1: the plain tile list
     int tail_base;
     int long_first;  // prefill_wide_sm100.cuh: units in order of falling length
+    // The additive mask as mask_scan_kernel has read it (prefill_wide_sm100.cuh; mask_blocks key blocks per row tile)
+    const uint32_t* mask_class;  // [row tile][key block]: a byte per 32 rows, MASK_* bits
+    const uint4* mask_bits;      // [row tile][key block][row]: one bit per key, set where the mask is 0
+    int mask_blocks;
 };
 
 // One CTA per SM, persistent: it takes tiles (128 query tokens of one query head) round-robin

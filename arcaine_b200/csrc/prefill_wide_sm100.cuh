@@ -49,6 +49,95 @@ struct WideWork {
     int q0, h, b, kvh, lo, hi;
 };
 
+// ---------------------------------------------------------------------------
+// Additive masks.  Read element by element from every row, head and block, the (seq, kv_len) f32 buffer made an
+// attention of 1000 queries over 1300 keys take 180 us, of which the attention itself is 20.  In practice a mask is 0
+// where a key is visible and -inf where it is not, and the same for all heads: one pass over the buffer turns it into a
+// bit per key and a class per 32 rows x 128 keys.  The attention then skips key blocks nobody sees, tests nothing in
+// those everybody sees and selects by bits in the others; only where other values occur does it read the mask itself.
+// ---------------------------------------------------------------------------
+constexpr uint32_t MASK_SEEN = 1;     // some key is not -inf
+constexpr uint32_t MASK_HIDDEN = 2;   // some key is -inf or past the end
+constexpr uint32_t MASK_VALUES = 4;   // some value is neither 0 nor -inf
+
+// Block = 32 rows x 128 keys, warp = 4 rows; a lane reads keys lane + 32 c, so that reads coalesce whatever the row's
+// alignment and a ballot is the chunk's bits.
+__global__ void __launch_bounds__(256) mask_scan_kernel(const float* mask, int seq, int kv_len, int blocks, uint32_t* cls, uint4* bits) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int j = blockIdx.x, r0 = blockIdx.y * 32 + warp * 4;  // key block, first row
+    float v[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int key = j * 128 + c * 32 + lane;
+            v[i][c] = r0 + i < seq && key < kv_len ? mask[(long long)(r0 + i) * kv_len + key] : -CUDART_INF_F;
+        }
+    uint32_t c8 = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t w[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            w[c] = __ballot_sync(0xffffffffu, v[i][c] == 0.f);
+            if (r0 + i >= seq) continue;
+            if (__any_sync(0xffffffffu, v[i][c] != -CUDART_INF_F)) c8 |= MASK_SEEN;
+            if (__any_sync(0xffffffffu, v[i][c] == -CUDART_INF_F)) c8 |= MASK_HIDDEN;
+            if (__any_sync(0xffffffffu, v[i][c] != 0.f && v[i][c] != -CUDART_INF_F)) c8 |= MASK_VALUES;
+        }
+        const int row = r0 + i, tile = row >> 7;
+        if (lane == 0) bits[((long long)tile * blocks + j) * 128 + (row & 127)] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    const uint32_t a = __syncthreads_or(c8 & MASK_SEEN), b = __syncthreads_or(c8 & MASK_HIDDEN), d = __syncthreads_or(c8 & MASK_VALUES);
+    if (threadIdx.x == 0) {
+        const int row = blockIdx.y * 32;
+        reinterpret_cast<uint8_t*>(cls + (long long)(row >> 7) * blocks + j)[(row >> 5) & 3] =
+            static_cast<uint8_t>((a ? MASK_SEEN : 0u) | (b ? MASK_HIDDEN : 0u) | (d ? MASK_VALUES : 0u));
+    }
+}
+
+// Key blocks [lo, hi) between the first and the last one somebody in the row tiles [t0, t1) sees.  Whole warps.
+__device__ __forceinline__ void masked_blocks(const PrefillParams& p, int t0, int t1, int& lo, int& hi) {
+    const int lane = threadIdx.x & 31;
+    lo = hi = 0;
+    for (int j0 = 0; j0 < p.mask_blocks; j0 += 32) {
+        uint32_t c = 0;
+        if (j0 + lane < p.mask_blocks)
+            for (int t = t0; t < t1; ++t) c |= p.mask_class[(long long)t * p.mask_blocks + j0 + lane];
+        const uint32_t seen = __ballot_sync(0xffffffffu, (c & (MASK_SEEN * 0x01010101u)) != 0);
+        if (!seen) continue;
+        if (hi == 0) lo = j0 + __ffs(seen) - 1;
+        hi = j0 + 32 - __clz(seen);
+    }
+}
+
+// One chunk of 32 keys: hidden scores become -inf.
+__device__ __forceinline__ void select_chunk(uint32_t (&v)[32], uint32_t bits) {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) v[e] = (bits >> e) & 1u ? v[e] : 0xff800000u;
+}
+
+// A block with values: raw score + mask / scale, which the softmax scales like a score, back into tensor memory.
+// (Clamped, so that a large finite mask stays finite.)
+__device__ __forceinline__ void add_mask_values(uint32_t tS, const float* mask_row, int key0, int kv_len, float inv_scale) {
+#pragma unroll 1
+    for (int c = 0; c < 128; c += 32) {
+        uint32_t v[32];
+        tmem_ld32(tS + c, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+            const float m = mask_row && key0 + c + e < kv_len ? mask_row[key0 + c + e] : -CUDART_INF_F;
+            const float x = fminf(fmaxf(m * inv_scale, -3.0e38f), 3.0e38f);
+            v[e] = m == -CUDART_INF_F ? 0xff800000u : __float_as_uint(__uint_as_float(v[e]) + x);
+        }
+        tmem_st32(tS + c, v);
+    }
+    tmem_wait_st();
+}
+
 __device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first, int q_last, int& lo, int& hi) {
     const int off = p.kv_len - p.seq;
     lo = 0;
@@ -75,6 +164,7 @@ struct WideCursor {
     }
 };
 
+template <bool MASKED>
 __device__ __forceinline__ WideWork decode_wide(const PrefillParams& p, const WideCursor& cur, int rank) {
     WideWork t;
     int qt;
@@ -91,7 +181,8 @@ __device__ __forceinline__ WideWork decode_wide(const PrefillParams& p, const Wi
     }
     const int rows = p.head_pair ? WideCfg::BM : 2 * WideCfg::BM;  // tokens of the unit
     const int q0 = qt * rows;
-    wide_blocks(p, q0, q0 + rows - 1, t.lo, t.hi);
+    if constexpr (MASKED) masked_blocks(p, q0 >> 7, min(q0 + rows, p.seq + 127) >> 7, t.lo, t.hi);
+    else wide_blocks(p, q0, q0 + rows - 1, t.lo, t.hi);
     if (p.head_pair) {
         t.h = t.h * 2 + rank;
         t.q0 = q0;
@@ -102,7 +193,8 @@ __device__ __forceinline__ WideWork decode_wide(const PrefillParams& p, const Wi
     return t;
 }
 
-template <bool GATE>
+// MASKED: with an additive mask, as mask_scan_kernel has read it.
+template <bool GATE, bool MASKED>
 __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     sdpa_prefill_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
@@ -213,7 +305,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         };
         WideCursor cur(first, step);
         for (; ok && cur.w < total; cur.advance(p)) {
-            const WideWork w = decode_wide(p, cur, rank);
+            const WideWork w = decode_wide<MASKED>(p, cur, rank);
             if (w.hi == w.lo) continue;
             if (n > 0 && !mbar_wait_inline(q_empty, (n - 1) & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u);
@@ -270,7 +362,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             WideCursor cur(first, step);
             auto next_unit = [&](WideWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
                 for (; cur.w < total; cur.advance(p)) {
-                    w = decode_wide(p, cur, 0);
+                    w = decode_wide<MASKED>(p, cur, 0);
                     if (w.hi > w.lo) {
                         cur.advance(p);
                         return true;
@@ -336,7 +428,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[quarter], 0u};
         WideCursor cur(first, step);
         for (; cur.w < total; cur.advance(p)) {
-            const WideWork w = decode_wide(p, cur, rank);
+            const WideWork w = decode_wide<MASKED>(p, cur, rank);
             const int t0 = w.q0 + quarter * 32, t = t0 + lane;
             const bool store = t < p.seq, warp_store = t0 < p.seq;  // this row / some row of the warp is stored
             const long long row = ((long long)w.b * p.seq + t) * p.nq + w.h;
@@ -417,7 +509,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         uint32_t s0[32], s1[32], s2[32], s3[32];  // the row's 128 scores of the current block
         WideCursor cur(first, step);
         for (; ok && cur.w < total; cur.advance(p)) {
-            const WideWork w = decode_wide(p, cur, rank);
+            const WideWork w = decode_wide<MASKED>(p, cur, rank);
             if (w.hi == w.lo) continue;
             const int t = w.q0 + r;
             int row_lo = 0, row_hi = p.kv_len;  // visible keys [row_lo, row_hi)
@@ -440,12 +532,24 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                     break;
                 }
                 tc_fence_after_sync();
+                const long long at = MASKED ? (long long)(w.q0 >> 7) * p.mask_blocks + j : 0;
+                const uint32_t cls = MASKED && w.q0 < p.seq ? reinterpret_cast<const uint8_t*>(p.mask_class + at)[quarter] : 0u;
+                if (MASKED && (cls & MASK_VALUES))
+                    add_mask_values(tS, t < p.seq ? p.mask + (long long)t * p.kv_len : nullptr, kc, p.kv_len, 1.4426950408889634f / sl);
                 tmem_ld32(tS, s0);
                 tmem_ld32(tS + 32, s1);
                 tmem_ld32(tS + 64, s2);
                 tmem_ld32(tS + 96, s3);
                 tmem_wait_ld();
-                if (!__all_sync(0xffffffffu, rm.lo <= kc && kc + C::BN <= rm.hi)) {  // window edge, diagonal, ragged end
+                if constexpr (MASKED) {
+                    if ((cls & (MASK_HIDDEN | MASK_VALUES)) == MASK_HIDDEN) {
+                        const uint4 bits = p.mask_bits[at * 128 + r];
+                        select_chunk(s0, bits.x);
+                        select_chunk(s1, bits.y);
+                        select_chunk(s2, bits.z);
+                        select_chunk(s3, bits.w);
+                    }
+                } else if (!__all_sync(0xffffffffu, rm.lo <= kc && kc + C::BN <= rm.hi)) {  // window edge, diagonal, ragged end
                     mask_chunk(s0, kc, rm);
                     mask_chunk(s1, kc + 32, rm);
                     mask_chunk(s2, kc + 64, rm);

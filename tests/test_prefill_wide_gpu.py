@@ -51,3 +51,53 @@ def test_consecutive_one_block_units_keep_the_epilogue_in_step():
     assert ops.device_status() == (0, 0) and torch.equal(out, again)
     solo = ops.sdpa_prefill(q[1:, :128], k[1:, :128], v[1:, :128], scale=0.0625, mask_type=ops.MASK_CAUSAL, window=100, num_splits=1)
     assert torch.equal(out[1:, :128], solo)
+
+
+@pytest.mark.parametrize("seq,kv,nq,nkv,kind", [
+    (200, 333, 8, 4, "window"),   # rows of the buffer not 16-byte aligned
+    (129, 900, 6, 2, "random"),   # odd group; keys hidden at random
+    (300, 1300, 4, 2, "blocks"),  # whole key blocks nobody sees, at either end and inside; a row without any key
+    (150, 260, 4, 2, "values"),   # finite values, a bias per key, and -inf
+    (1, 1, 2, 1, "window"),
+])
+def test_additive_mask(seq, kv, nq, nkv, kind):
+    from arcaine_b200 import _lib, ops
+    import ctypes as C
+    ops.clear_device_status()
+    hd, inf = 256, float("inf")
+    g = torch.Generator().manual_seed(3)
+    mask = torch.zeros(seq, kv)
+    if kind == "window":
+        mask = torch.from_numpy(oracle.fill_causal_mask(seq, kv, kv - seq, 100))
+        assert torch.equal(ops.fill_causal_mask(seq, kv, kv - seq, 100).cpu(), mask)
+    elif kind == "random":
+        mask[torch.rand(seq, kv, generator=g) < 0.5] = -inf
+    elif kind == "blocks":
+        mask[:, :140], mask[:, 400:700], mask[:, 1200:] = -inf, -inf, -inf
+        mask[7] = -inf
+    else:
+        mask = torch.randn(seq, kv, generator=g) * 2
+        mask[:, 130:] = 0.0
+        mask[torch.rand(seq, kv, generator=g) < 0.2] = -inf
+    q, k, v = seeded_bf16(seq, nq, hd, seed=1), seeded_bf16(kv, nkv, hd, seed=2), seeded_bf16(kv, nkv, hd, seed=3)
+    gate = seeded_bf16(seq, nq, hd, seed=4)
+    dev = [t.cuda() for t in (q, k, v, gate, mask.float().contiguous())]
+    out, lse = ops.sdpa_prefill(dev[0], dev[1], dev[2], scale=0.0625, mask_type=ops.MASK_EXPLICIT, mask=dev[4], return_lse=True)
+    gated = ops.sdpa_prefill(dev[0], dev[1], dev[2], scale=0.0625, mask_type=ops.MASK_EXPLICIT, mask=dev[4], gate=dev[3])
+    want = oracle.sdpa_f32(q, k, v, scale=0.0625, mask_type=1, mask=mask.numpy(), want_lse=True)
+    assert_close(out, want[0], kind)
+    fin = torch.isfinite(want[2])
+    assert torch.equal(torch.isfinite(lse.cpu()), fin) and torch.allclose(lse.cpu()[fin], want[2][fin], atol=2e-3)
+    assert_close(gated, oracle.sdpa_f32(q, k, v, scale=0.0625, mask_type=1, mask=mask.numpy(), gate=gate)[1].float(), kind + " gated")
+    # without a workspace the call still works (the mask is then read by the attention kernel itself)
+    p = _lib.PrefillParams()
+    o2 = torch.empty_like(out)
+    p.q, p.k, p.v, p.out, p.mask = (t.data_ptr() for t in (dev[0], dev[1], dev[2], o2, dev[4]))
+    p.batch, p.seq, p.kv_len, p.nq, p.nkv, p.hd = 1, seq, kv, nq, nkv, hd
+    p.q_stride_t = p.o_stride_t = nq * hd
+    p.k_stride_t = p.v_stride_t = nkv * hd
+    p.q_stride_b, p.o_stride_b, p.k_stride_b, p.v_stride_b = seq * nq * hd, seq * nq * hd, kv * nkv * hd, kv * nkv * hd
+    p.scale, p.mask_type, p.window, p.num_splits = 0.0625, ops.MASK_EXPLICIT, ops.NO_WINDOW, 1
+    assert _lib.load().arc_sdpa_prefill(C.byref(p), torch.cuda.current_stream().cuda_stream) == _lib.ARC_OK
+    assert_close(o2, want[0], kind + " without a workspace")
+    assert ops.device_status() == (0, 0)
