@@ -91,7 +91,7 @@ __device__ __forceinline__ long long share_size(long long total, int ncta, int t
 
 __device__ __forceinline__ float sigmoid_gate(float attn, uint16_t gate_bits) {
     const float g = bf16_bits_to_f32(gate_bits);
-    return bf16_round(attn) * (1.0f / (1.0f + __expf(-g)));
+    return bf16_round(attn) * sigmoid(g);
 }
 
 // All consumer warps of the CTA (named barrier 1; the producer warp does not take part).
@@ -879,7 +879,7 @@ __global__ void mul_sigmoid_kernel(uint16_t* a, const uint16_t* gate, long long 
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const float g = bf16_bits_to_f32(gate[i]);
-        const float sig = 1.0f / (1.0f + __expf(-g));
+        const float sig = sigmoid(g);
         a[i] = __bfloat16_as_ushort(__float2bfloat16_rn(bf16_bits_to_f32(a[i]) * sig));
     }
 }

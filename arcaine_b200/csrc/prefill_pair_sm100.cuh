@@ -52,8 +52,8 @@ struct PairCfg {
     static constexpr int COL_S = 0;    // + 128 * pipeline
     static constexpr int COL_O = 256;  // + 128 * pipeline
     // q_full[2] q_empty[2] k_first k_first_used kv_full[2] kv_empty[2] then per pipeline:
-    // s_full p_part[2] o_full o_empty fin[2]; then gate[4], one per epilogue warp
-    static constexpr int NUM_BARS = 4 + 2 + 2 * K_STAGES + 18;
+    // s_full p_part[2] o_full o_empty fin[2]; then gate[4][2], two per epilogue warp
+    static constexpr int NUM_BARS = 4 + 2 + 2 * K_STAGES + 22;
     static constexpr int FIN_FLOATS = 2 * 2 * 128;  // [tile parity][pipeline][row] row sum
     static constexpr int SMEM_BYTES = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 4 * 8192 + NUM_BARS * 8 + 16 + FIN_FLOATS * 4;  // (4 x 8 KB: output stage)
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
@@ -168,67 +168,108 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&v)[32], uint32_t (&pk
 
 // Output of a 128-row tile through shared memory.  Thread = row, so a store of a thread's 16 bytes touches 32 lines per
 // warp instruction: written straight to global memory, a tile of 128 x 256 kept the accumulator and the load / store
-// unit busy for 9000 clk.  Instead a warp collects its 32 rows, 128 columns at a time, in 8 KB of shared memory (two
-// boxes of 64 columns, 128-byte swizzle: lanes of a quarter warp hit different banks) and hands them to TMA, whose
-// stores clip the rows past `seq`; the gate values come the same way, by TMA into the same buffer, and are replaced
-// by the products in place.
+// unit busy for 9000 clk.  Instead a warp collects its 32 rows, 64 columns a round, in one of two 4 KB buffers (128-byte
+// swizzle: lanes of a quarter warp hit different banks) and hands them to TMA, whose stores clip the rows past `seq`;
+// gate values come the same way, by TMA into the buffer a round ahead, and are replaced by the products in place.
 constexpr int STAGE_WARP_BYTES = 8192;
 constexpr int STAGE_BYTES = 4 * STAGE_WARP_BYTES;  // four epilogue warps
 
 struct OutStage {
-    uint8_t* buf;        // this warp's 8 KB, 1024-byte aligned
-    uint64_t* gate_bar;  // this warp's
-    uint32_t gate_par;   // parity of the next gate load
+    uint8_t* buf;        // this warp's 2 x 4 KB, 1024-byte aligned
+    uint64_t* gate_bar;  // [2] this warp's, one per buffer
+    uint32_t gate_par;   // bit i: parity of buffer i's next gate load
+    int h, t0, b;        // head, first of the warp's 32 rows, sequence
 };
 
-// Begin 128 columns of the warp's 32 rows from (c0, h, t0, b) on: the buffer is free again; ask for the gate values.
-// Rows from p.seq on are the caller's to skip (t0 < seq).
-template <bool GATE>
-__device__ __forceinline__ void stage_begin(OutStage& s, const void* tm_gate, int lane, int c0, int h, int t0, int b) {
+// Gate values of round c (columns [64 c, 64 c + 64)) into the round's buffer, which is free.  One lane.
+__device__ __forceinline__ void stage_load_gate(const OutStage& s, const void* tm_gate, int c) {
+    mbar_arrive_expect_tx(&s.gate_bar[c & 1], 4096);
+    tma_load_4d(s.buf + (c & 1) * 4096, tm_gate, &s.gate_bar[c & 1], c * 64, s.h, s.t0, s.b);
+}
+
+// Once per tile, before its accumulator is waited for.
+template <bool GATE, int HD>
+__device__ __forceinline__ void stage_open(OutStage& s, const void* tm_gate, int lane, int h, int t0, int b) {
+    s.h = h, s.t0 = t0, s.b = b;
     if (lane == 0) {
-        bulk_wait_read();
+        bulk_wait_read<0>();
         if (GATE) {
-            mbar_arrive_expect_tx(s.gate_bar, STAGE_WARP_BYTES);
-            for (int i = 0; i < 2; ++i) tma_load_4d(s.buf + i * 4096, tm_gate, s.gate_bar, c0 + i * 64, h, t0, b);
+            stage_load_gate(s, tm_gate, 0);
+            stage_load_gate(s, tm_gate, 1);
+            for (int c = 2; c < HD / 64; ++c) tma_prefetch_4d(tm_gate, c * 64, h, t0, b);  // (the later rounds' into L2)
         }
     }
     __syncwarp();
 }
 
-// Columns [32 c, 32 c + 32) of the round: the accumulator's values times `inv`, gated, as bf16 into the buffer (and
-// into w8 for the caller).
+// The epilogue takes STAGE_COLS columns a turn of a rolled loop: its code runs beside the softmax loop out of the same
+// instruction cache, and what does not fit beside it costs 50 clk per 128 bytes on every turn.  (Gated, 32 columns a
+// turn are 6 KB of code and took 2500 clk, 16 columns 2.5 KB.)
 template <bool GATE>
-__device__ __forceinline__ void stage_chunk(const OutStage& s, int lane, int c, const uint32_t (&acc)[32], float inv, uint32_t (&w8)[16]) {
-    const uint32_t row = smem_u32(s.buf) + (c >> 1) * 4096 + lane * 128;
+constexpr int STAGE_COLS = GATE ? 16 : 32;
+
+// Before turn k of a tile of HD columns.  False: the gate values never came.
+template <bool GATE, int HD>
+__device__ __forceinline__ bool stage_before(OutStage& s, const void* tm_gate, int lane, int k) {
+    constexpr int TURNS = 64 / STAGE_COLS<GATE>;  // per round
+    const int c = k / TURNS, i = c & 1;
+    if (k % TURNS == 0) {
+        if (GATE) {
+            if (!mbar_wait_warp<2>(&s.gate_bar[i], (s.gate_par >> i) & 1u)) return false;
+            s.gate_par ^= 1u << i;
+        } else if (c >= 2) {
+            if (lane == 0) bulk_wait_read<1>();  // round c - 2 has left the buffer
+            __syncwarp();
+        }
+    } else if (GATE && k % TURNS == TURNS / 2 && c >= 1 && c + 1 < HD / 64) {
+        if (lane == 0) {
+            bulk_wait_read<0>();  // round c - 1 has left its buffer: the one of round c + 1
+            stage_load_gate(s, tm_gate, c + 1);
+        }
+        __syncwarp();
+    }
+    return true;
+}
+
+// Turn k: the accumulator's values times `inv`, gated, as bf16 into the buffer (and into w8 for the caller); after a
+// round's last turn the round is sent off.  taken(): called once acc has been used, so that the next turn's values
+// can be on their way while this turn's are gated.
+template <bool GATE, typename F, int N = STAGE_COLS<GATE>>
+__device__ __forceinline__ void stage_turn(const OutStage& s, const void* tm_out, int lane, int k, const uint32_t (&acc)[N], float inv,
+                                           uint32_t (&w8)[N / 2], F&& taken) {
+    constexpr int TURNS = 64 / N;
+    const int c = k / TURNS;
+    const uint32_t row = smem_u32(s.buf) + (c & 1) * 4096 + lane * 128;
+    uint32_t at[N / 8], gw[N / 2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t a = row + ((((c & 1) * 4 + i) ^ (lane & 7)) << 4);
+    for (int i = 0; i < N / 8; ++i) {
+        at[i] = row + ((((k % TURNS) * (N / 8) + i) ^ (lane & 7)) << 4);
+        if (GATE)
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(gw[4 * i]), "=r"(gw[4 * i + 1]), "=r"(gw[4 * i + 2]), "=r"(gw[4 * i + 3]) : "r"(at[i]));
+    }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            w8[4 * i + u] = pack_bf16x2(__uint_as_float(acc[8 * i + 2 * u]) * inv, __uint_as_float(acc[8 * i + 2 * u + 1]) * inv);
+    for (int u = 0; u < N / 2; ++u) w8[u] = pack_bf16x2(__uint_as_float(acc[2 * u]) * inv, __uint_as_float(acc[2 * u + 1]) * inv);
+    taken();
+#pragma unroll
+    for (int i = 0; i < N / 8; ++i) {
         if (GATE) {
             // bf16(attention) * sigmoid(gate): the rounding order of the two-launch form
-            uint32_t gw[4];
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(gw[0]), "=r"(gw[1]), "=r"(gw[2]), "=r"(gw[3]) : "r"(a));
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t w = w8[4 * i + u];
-                const float a0 = __uint_as_float(w << 16), a1 = __uint_as_float(w & 0xffff0000u);
+            for (int u = 4 * i; u < 4 * i + 4; ++u) {
+                const float a0 = __uint_as_float(w8[u] << 16), a1 = __uint_as_float(w8[u] & 0xffff0000u);
                 const float g0 = __uint_as_float(gw[u] << 16), g1 = __uint_as_float(gw[u] & 0xffff0000u);
-                w8[4 * i + u] = pack_bf16x2(a0 * (1.0f / (1.0f + __expf(-g0))), a1 * (1.0f / (1.0f + __expf(-g1))));
+                w8[u] = pack_bf16x2(a0 * sigmoid(g0), a1 * sigmoid(g1));
             }
         }
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(w8[4 * i]), "r"(w8[4 * i + 1]), "r"(w8[4 * i + 2]), "r"(w8[4 * i + 3]) : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at[i]), "r"(w8[4 * i]), "r"(w8[4 * i + 1]), "r"(w8[4 * i + 2]), "r"(w8[4 * i + 3]) : "memory");
     }
-}
-
-// The round's 128 columns are in the buffer: send them off.
-__device__ __forceinline__ void stage_end(const OutStage& s, const void* tm_out, int lane, int c0, int h, int t0, int b) {
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) {
-        for (int i = 0; i < 2; ++i) tma_store_4d(tm_out, s.buf + i * 4096, c0 + i * 64, h, t0, b);
-        bulk_commit();
+    if (k % TURNS == TURNS - 1) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_4d(tm_out, s.buf + (c & 1) * 4096, c * 64, s.h, s.t0, s.b);
+            bulk_commit();
+        }
     }
 }
 
@@ -265,7 +306,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     // from "not yet".  They cannot reach tile n + 2 before the epilogue has taken tile n (the first O += P V
     // of tile n + 1 waits for that), so two are enough.
     uint64_t* fin = o_empty + 2;
-    uint64_t* gate_bar = fin + 4;    // [epilogue warp]
+    uint64_t* gate_bar = fin + 4;    // [epilogue warp][buffer]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
     float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [tile parity 2][pipeline 2][row 128] row sum
@@ -292,7 +333,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             mbar_init(&fin[2 * s], 4);
             mbar_init(&fin[2 * s + 1], 4);
         }
-        for (int w = 0; w < 4; ++w) mbar_init(&gate_bar[w], 1);
+        for (int w = 0; w < 8; ++w) mbar_init(&gate_bar[w], 1);
         mbar_init(k_first, 1);
         mbar_init(k_first_used, 1);
         for (int s = 0; s < 2; ++s) {
@@ -553,7 +594,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
         int tq0 = 0, tq1 = 0;  // tiles with key blocks so far, per pipeline
         bool ok = true;
-        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[quarter], 0u};
+        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0};
         TileCursor cur;
         for (cur.init(p); ok && cur.w < total_tiles; cur.advance(p)) {
             const PairWork pw = decode_pair(p, cur);
@@ -575,56 +616,56 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     }
                     continue;
                 }
-                if (warp_store) stage_begin<GATE>(stage, &tm_gate, lane, 0, h, t0, pw.b);
+                if (warp_store) stage_open<GATE, HD>(stage, &tm_gate, lane, h, t0, pw.b);
                 const int tq = s ? tq1 : tq0;
-                if (!mbar_wait_relaxed_warp<2>(&fin[2 * s + (tq & 1)], (tq >> 1) & 1)) {
+                if (!mbar_wait_warp<2>(&fin[2 * s + (tq & 1)], (tq >> 1) & 1)) {
                     report_fault(p.fault, FAULT_WAIT_FULL, 0x500u + s);
                     ok = false;
                     break;
                 }
                 const float row_l = fin_vals[((tq & 1) * 2 + s) * 128 + r];
-                if (!mbar_wait_relaxed_warp<2>(&o_full[s], tq & 1)) {
+                if (!mbar_wait_warp<2>(&o_full[s], tq & 1)) {
                     report_fault(p.fault, FAULT_WAIT_O, tq);
                     ok = false;
                     break;
-                }
-                if (GATE && warp_store) {
-                    if (!mbar_wait_relaxed_warp<2>(stage.gate_bar, stage.gate_par)) {
-                        report_fault(p.fault, FAULT_WAIT_FULL, 0x600u + s);
-                        ok = false;
-                        break;
-                    }
-                    stage.gate_par ^= 1u;
                 }
                 tc_fence_after_sync();
                 if (s) ++tq1; else ++tq0;
                 const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
                 const uint32_t tO = tmem_base + lane_sel + C::COL_O + s * 128;
+                constexpr int SC = STAGE_COLS<GATE>;
+                uint32_t wa[SC], w8[SC / 2];
+                tmem_ld(tO, wa);
 #pragma unroll 1
-                for (int c = 0; c < HD / 32; ++c) {
-                    uint32_t wa[32], w8[16];
-                    tmem_ld32(tO + c * 32, wa);
+                for (int c = 0; c < HD / SC; ++c) {
+                    if (warp_store && !stage_before<GATE, HD>(stage, &tm_gate, lane, c)) {
+                        report_fault(p.fault, FAULT_WAIT_FULL, 0x600u + s);
+                        ok = false;
+                        break;
+                    }
                     tmem_wait_ld();
-                    if (c + 1 == HD / 32) {
-                        // O is in registers: the next tile may overwrite the accumulator.
+                    if (c + 1 == HD / SC) {  // O is in registers: the next unit may overwrite the accumulator
                         tc_fence_before_sync();
                         mbar_arrive_warp(&o_empty[s]);
                     }
+                    auto next = [&]() {
+                        if (c + 1 < HD / SC) tmem_ld(tO + (c + 1) * SC, wa);
+                    };
+                    if (!warp_store) next();
                     if (warp_store) {
-                        stage_chunk<GATE>(stage, lane, c, wa, inv, w8);
+                        stage_turn<GATE>(stage, &tm_out, lane, c, wa, inv, w8, next);
                         if (COPIES && store) {
                             for (int k = 0; k < p.n_copies; ++k) {
-                                uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + eoff + c * 32);
+                                uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + eoff + c * SC);
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) d4[i] = make_uint4(w8[4 * i], w8[4 * i + 1], w8[4 * i + 2], w8[4 * i + 3]);
+                                for (int i = 0; i < SC / 8; ++i) d4[i] = make_uint4(w8[4 * i], w8[4 * i + 1], w8[4 * i + 2], w8[4 * i + 3]);
                             }
                         }
                     }
                 }
-                if (warp_store) stage_end(stage, &tm_out, lane, 0, h, t0, pw.b);
             }
         }
-        if (lane == 0) bulk_wait_read();  // the stage may go when its last rows have been read
+        if (lane == 0) bulk_wait_read<0>();  // the stage may go when its last rows have been read
     } else {
         // ------------------------------------------------------------------ softmax
         // Warps 0-3 serve tile A, warps 4-7 tile B; a thread owns one query row and takes its 128

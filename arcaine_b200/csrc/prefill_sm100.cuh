@@ -146,7 +146,7 @@ __device__ __forceinline__ void store_copies_bf16x16(const unsigned long long* c
 // output (src/modeling/qwen3_5_moe/kernels.hpp:80-88).
 __device__ __forceinline__ float sigmoid_gate_bits(float attn, uint16_t gate_bits) {
     const float g = bf16_bits_to_f32(gate_bits);
-    return bf16_round(attn) * (1.0f / (1.0f + __expf(-g)));
+    return bf16_round(attn) * sigmoid(g);
 }
 
 // Maximum of one 32-column chunk, folded into four independent running maxima.
@@ -1054,7 +1054,7 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
 #pragma unroll
                                     for (int u = 0; u < 8; ++u) {
                                         const float gf = bf16_bits_to_f32(static_cast<uint16_t>(gw[u >> 1] >> ((u & 1) * 16)));
-                                        const float sig = 1.0f / (1.0f + __expf(-gf));
+                                        const float sig = sigmoid(gf);
                                         o[u] = bf16_round(o[u]) * sig;
                                     }
                                 }

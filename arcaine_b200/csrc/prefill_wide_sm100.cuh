@@ -36,8 +36,8 @@ struct WideCfg {
     static constexpr int STAGES = 2;               // of K and of V
     static constexpr int COL_S = 0;                // + 128 * buffer
     static constexpr int COL_O = 256;
-    // q_full q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp]
-    static constexpr int NUM_BARS = 2 + 8 + 2 + 4 + 2 + 4 + 4;
+    // q_full q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp][2]
+    static constexpr int NUM_BARS = 2 + 8 + 2 + 4 + 2 + 4 + 8;
     static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
     static constexpr int EPILOGUE_WARP = 4, PRODUCER_WARP = 8, ISSUER_WARP = 9;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     // computed one block ahead; the first P V of n + 1 waits for the epilogue of n): with fewer slots a phase could
     // complete twice before the epilogue has looked at it, which a parity wait cannot tell from "not yet".
     uint64_t* fin = bars + 18;
-    uint64_t* gate_bar = bars + 22;    // [epilogue warp] own CTA
+    uint64_t* gate_bar = bars + 22;    // [epilogue warp][buffer] own CTA
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
     float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [unit & 3][row] row sum
@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         }
         for (int i = 0; i < 4; ++i) {
             mbar_init(&fin[i], 4);
-            mbar_init(&gate_bar[i], 1);
+            mbar_init(&gate_bar[2 * i], 1);
+            mbar_init(&gate_bar[2 * i + 1], 1);
         }
         mbar_init(o_full, 1);
         mbar_init(o_empty, 8);
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         const uint32_t tO = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::COL_O;
         const uint32_t b_empty = map_to_cta(smem_u32(o_empty), 0);
         int n = 0;  // units with key blocks so far
-        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[quarter], 0u};
+        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0};
         WideCursor cur(first, step);
         for (; cur.w < total; cur.advance(p)) {
             const WideWork w = decode_wide<MASKED>(p, cur, rank);
@@ -443,13 +444,13 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 }
                 continue;
             }
-            if (warp_store) stage_begin<GATE>(stage, &tm_gate, lane, 0, w.h, t0, w.b);
-            if (!mbar_wait_relaxed_warp<2>(&fin[n & 3], (n >> 2) & 1)) {
+            if (warp_store) stage_open<GATE, HD>(stage, &tm_gate, lane, w.h, t0, w.b);
+            if (!mbar_wait_warp<2>(&fin[n & 3], (n >> 2) & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x500u);
                 break;
             }
             const float row_l = fin_vals[(n & 3) * 128 + r];
-            if (!mbar_wait_relaxed_warp<2>(o_full, n & 1)) {
+            if (!mbar_wait_warp<2>(o_full, n & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, n);
                 break;
             }
@@ -457,41 +458,39 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             ++n;
             const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
             bool ok = true;
+            constexpr int SC = STAGE_COLS<GATE>;
+            uint32_t wa[SC], w8[SC / 2];
+            tmem_ld(tO, wa);
 #pragma unroll 1
-            for (int c = 0; c < HD / 32; ++c) {
-                uint32_t wa[32], w8[16];
-                if (warp_store && (c & 3) == 0) {
-                    if (c > 0) stage_begin<GATE>(stage, &tm_gate, lane, 128, w.h, t0, w.b);
-                    if (GATE) {
-                        if (!mbar_wait_relaxed_warp<2>(stage.gate_bar, stage.gate_par)) {
-                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x600u);
-                            ok = false;
-                            break;
-                        }
-                        stage.gate_par ^= 1u;
-                    }
+            for (int c = 0; c < HD / SC; ++c) {
+                if (warp_store && !stage_before<GATE, HD>(stage, &tm_gate, lane, c)) {
+                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x600u);
+                    ok = false;
+                    break;
                 }
-                tmem_ld32(tO + c * 32, wa);
                 tmem_wait_ld();
-                if (c + 1 == HD / 32) {  // O is in registers: the next unit may overwrite the accumulator
+                if (c + 1 == HD / SC) {  // O is in registers: the next unit may overwrite the accumulator
                     tc_fence_before_sync();
                     mbar_arrive_remote_warp(b_empty);
                 }
+                auto next = [&]() {
+                    if (c + 1 < HD / SC) tmem_ld(tO + (c + 1) * SC, wa);
+                };
+                if (!warp_store) next();
                 if (warp_store) {
-                    stage_chunk<GATE>(stage, lane, c & 3, wa, inv, w8);
+                    stage_turn<GATE>(stage, &tm_out, lane, c, wa, inv, w8, next);
                     if (store) {
                         for (int k = 0; k < p.n_copies; ++k) {
-                            uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + eoff + c * 32);
+                            uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + eoff + c * SC);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) d4[i] = make_uint4(w8[4 * i], w8[4 * i + 1], w8[4 * i + 2], w8[4 * i + 3]);
+                            for (int i = 0; i < SC / 8; ++i) d4[i] = make_uint4(w8[4 * i], w8[4 * i + 1], w8[4 * i + 2], w8[4 * i + 3]);
                         }
                     }
-                    if ((c & 3) == 3) stage_end(stage, &tm_out, lane, (c >> 2) * 128, w.h, t0, w.b);
                 }
             }
             if (!ok) break;
         }
-        if (lane == 0) bulk_wait_read();  // the stage may go when its last rows have been read
+        if (lane == 0) bulk_wait_read<0>();  // the stage may go when its last rows have been read
     } else {
         // ------------------------------------------------------------------ softmax: thread = query row
         const int quarter = warp & 3;

@@ -175,27 +175,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
     return mbar_wait_slow<GROUP>(bar, parity, limit_cycles);
 }
 
-// The same for waits that are long and not urgent (an epilogue waiting for a whole tile): the
-// thread sleeps between polls, so that it does not take issue slots from the warps that work.
-template <int GROUP>
-__device__ __noinline__ bool mbar_wait_relaxed_slow(uint64_t* bar, uint32_t parity, long long limit_cycles) {
-    long long t0 = clock64();
-    uint32_t spins = 0;
-    while (!mbar_try_wait(bar, parity)) {
-        __nanosleep(100);
-        if ((++spins & 0x3Fu) == 0 && clock64() - t0 > limit_cycles) return false;
-    }
-    return true;
-}
-
-template <int GROUP = 0>
-__device__ __forceinline__ bool mbar_wait_relaxed_warp(uint64_t* bar, uint32_t parity,
-                                                       long long limit_cycles = 2000000000LL) {
-    bool ok = mbar_try_wait(bar, parity);
-    if (!ok) ok = mbar_wait_relaxed_slow<GROUP>(bar, parity, limit_cycles);
-    return __all_sync(0xffffffffu, ok);
-}
-
 // Same, with a warp-uniform answer (every lane polls; all must succeed), so the
 // warp-collective tcgen05 / ldmatrix instructions that follow never see a
 // partially exited warp.
@@ -347,8 +326,11 @@ __device__ __forceinline__ void tma_store_4d(const void* tmap, const void* smem_
 
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 
-// Every bulk group of this thread has read its shared memory.
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// All but the last PENDING bulk groups of this thread have read their shared memory.
+template <int PENDING>
+__device__ __forceinline__ void bulk_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory");
+}
 
 // 2-D tiled load (c0 innermost, multiple of 8 elements for 16-bit data).
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1) {
@@ -546,6 +528,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
+
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -689,6 +674,14 @@ __device__ __forceinline__ float bf16_bits_to_f32(uint16_t b) {
 
 __device__ __forceinline__ float bf16_round(float x) {
     return __bfloat162float(__float2bfloat16_rn(x));
+}
+
+// 1 / (1 + e^-x) with the hardware's exponential and reciprocal (a few ulp of fp32; an IEEE division is many times the
+// instructions and made gated epilogues the longest part of a tile).
+__device__ __forceinline__ float sigmoid(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(1.0f + fast_exp2(x * -1.4426950408889634f)));
+    return y;
 }
 
 // ---------------------------------------------------------------------------
