@@ -965,28 +965,29 @@ extern "C" int arc_qkv_prepare(const arc_qkv_prepare_params* p, void* stream) {
         const int rh = kp.rot_half;
         if (rh < 8 || (rh & (rh - 1)) != 0 || rh > p->hd / 4 || p->n_active_pairs > rh) return ARC_ERR_BAD_SHAPE;
     }
-    // A CTA works on `tpc` consecutive tokens per round: enough (token, head) rows for its eight warps
-    // (each takes 512 / hd rows per pass), within the shared-memory angle table of 1024 pairs.
+    const bool qwen = kp.rot_half != p->hd / 2 || kp.freq_denom != p->hd || kp.mrope_pos != nullptr || kp.v_copy;
+    // A warp takes a token at a time, or a part of a token's passes: whatever gives the last warp the fewest passes,
+    // the start of a unit (the token's angles) counted as 0.7 of one; whole tokens where there are several for every warp.
     const long long tokens = (long long)p->batch * p->seq;
     if (tokens > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
-    const int rows = row_count;
-    const int rows_per_pass = 8 * (512 / p->hd);
-    int tpc = (8 * rows_per_pass + rows - 1) / rows;  // about eight passes per warp and round
-    const int max_tpc = 1024 / (p->hd / 2);
-    if (tpc > max_tpc) tpc = max_tpc;
-    if (tpc < 1) tpc = 1;
-    const long long rounds = (tokens + tpc - 1) / tpc;
-    const long long cap = (long long)ds->sm_count * 8;  // eight CTAs per SM keep enough loads in flight
-    const unsigned ctas = (unsigned)(rounds < cap ? rounds : cap);
+    const int passes = (row_count + 512 / p->hd - 1) / (512 / p->hd);
+    const long long warps = (long long)ds->sm_count * (qwen ? PREP_CTAS<true> : PREP_CTAS<false>) * PREP_WARPS;
+    int chunk = passes, chunks = 1;
+    long long best = 0;
+    for (int c = passes; tokens < 4 * warps; c = (c + 1) / 2) {
+        const int n = (passes + c - 1) / c;
+        const long long cost = (tokens * n + warps - 1) / warps * (10 * c + 7);
+        if (best == 0 || cost < best) best = cost, chunk = c, chunks = n;
+        if (c == 1) break;
+    }
+    if (tokens * chunks + warps > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
+    const long long units = tokens * chunks;
+    const unsigned ctas = (unsigned)((units < warps ? units : warps) + PREP_WARPS - 1) / PREP_WARPS;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool qwen = kp.rot_half != p->hd / 2 || kp.freq_denom != p->hd || kp.mrope_pos != nullptr || kp.v_copy;
-    // (measured on config 3's pre-processing: 64 rows per token 220 -> 207 us with the look-ahead form, 8 rows per
-    // token 43 -> 45 us)
-    const bool ahead = rows >= 24;
     auto launch = [&](auto hd_tag, auto qwen_tag) {
         constexpr int H = decltype(hd_tag)::value;
         constexpr bool Q = decltype(qwen_tag)::value;
-        return launch_dependent(ahead ? qkv_prepare_kernel<H, Q, true> : qkv_prepare_kernel<H, Q, false>, dim3(ctas), dim3(256), 0, st, 1, kp, tpc);
+        return launch_dependent(qkv_prepare_kernel<H, Q>, dim3(ctas), dim3(32 * PREP_WARPS), 0, st, 1, kp, chunk, chunks);
     };
     auto launch_hd = [&](auto qwen_tag) {
         if (p->hd == 128) return launch(std::integral_constant<int, 128>{}, qwen_tag);

@@ -13,12 +13,18 @@
 // works on those rounded values.  cos / sin come from a caller table (seq x n_active_pairs, as
 // the reference's RopeTable) or are computed per token: angle = (offset + token) / theta^(2p/hd).
 //
-// Mapping: one CTA per group of consecutive tokens at a time (grid-stride), cos / sin of those
-// tokens staged once in shared memory and shared by all their heads (the reference's "Fused"
-// mode), one warp per
-// (token, head) row segment: a lane holds eight consecutive elements of the row's first half and
-// the matching eight of the second half (16-byte loads), so a rotation pair never leaves the lane
-// and a warp covers 4 / 2 / 1 rows at once for head dim 128 / 256 / 512.
+// Mapping: a warp on its own takes a unit of work — a token, or a part of a token's rows where there are few tokens — and
+// walks it 32 / (hd / 16) rows a pass: a lane holds eight consecutive elements of a row's first half and the matching
+// eight of the second half (16-byte loads), so a rotation pair never leaves the lane and a warp covers 4 / 2 / 1 rows at
+// once for head dim 128 / 256 / 512.  The token's cos / sin are worked out once, a pair per lane, into shared memory of
+// the warp's own; nothing but the norm weights and the frequencies is shared, so there is one barrier in all.
+//
+// What bounds it: for prompts the instructions of a pass (about 250 for 2 KB moved) as much as HBM.  Hence pointers
+// per unit instead of per row, carries instead of divisions between units, weights and angles read from shared memory
+// (in registers they cost the third CTA per SM: 208 us), one pass of loads ahead (two: 198 us).  For a few tokens it is
+// the latency of one pass, so their rows are spread over all warps.  4 x 8192 tokens, 32/16 heads of 128 (1.07 GB):
+// 206 -> 193 us against a CTA per four tokens with angles behind a barrier per round; 64 tokens, 24/4 heads of 256:
+// 10.4 -> 3.3 us.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -73,211 +79,219 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
     return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
 }
 
-__device__ __forceinline__ float bf16_rne(float x) {
-    return __uint_as_float(static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(x))) << 16);
-}
+// Rows of a token per pass of a warp.
+template <int HD>
+constexpr int PREP_RPW = 512 / HD;
+constexpr int PREP_WARPS = 8;
+// CTAs per SM (the Qwen3.5 form does not fit 80 registers).
+template <bool QWEN>
+constexpr int PREP_CTAS = QWEN ? 2 : 3;
 
-// 256 threads = 8 warps.  A row of HD values is held by HD/16 lanes, each with eight consecutive
-// values of the row's first half and the matching eight of the second half (two 16-byte loads),
-// so a warp works on 32 / (HD/16) rows at once: 4 (HD 128), 2 (HD 256) or 1 (HD 512).  A CTA
-// takes `tpc` consecutive tokens per round (the host picks tpc so that a round has work for all
-// eight warps even when a rank holds only a few heads).
-// QWEN: the Qwen3.5 form (pairs rot_half apart, per-axis positions, V copied); the common instance does not
-// carry its branches.
-// AHEAD: a warp issues the loads of its next pass before it works on this one (64 registers, four CTAs per SM:
-// faster when a token has many rows); without it 40 registers and six CTAs per SM (faster for the few rows per
-// token of a rank that holds a few heads).
-template <int HD, bool QWEN, bool AHEAD>
-__global__ void __launch_bounds__(256) qkv_prepare_kernel(const QkvPrepareParams p, const int tpc) {
+// QWEN: the Qwen3.5 form (pairs rot_half apart, per-axis positions, V copied); the common instance does not carry its
+// branches.  chunk: passes per unit; chunks: units per token.
+template <int HD, bool QWEN>
+__global__ void __launch_bounds__(32 * PREP_WARPS, PREP_CTAS<QWEN>) qkv_prepare_kernel(const QkvPrepareParams p, const int chunk, const int chunks) {
     constexpr int LPR = HD / 16;    // lanes per row
-    constexpr int RPW = 32 / LPR;   // rows per warp and pass
-    constexpr int MAX_TPC = 1024 / (HD / 2);
-    __shared__ float s_cos2[2][1024];  // [round parity][token in round][pair]: one barrier per round is enough
-    __shared__ float s_sin2[2][1024];
-    __shared__ float s_inv[HD / 2];    // rotation frequencies, computed once
-    __shared__ int s_bt[2][2 * 16];     // [round parity][token in round] -> (batch index, token in sequence)
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int sub = lane / LPR;     // which of the warp's rows
+    constexpr int RPW = PREP_RPW<HD>;
+    __shared__ float s_inv[HD / 2];                      // rotation frequencies
+    __shared__ __align__(16) float s_cos[PREP_WARPS][HD / 2], s_sin[PREP_WARPS][HD / 2];  // per warp: the token's angles
+    __shared__ __align__(16) float s_w[2][HD];           // norm weights of Q and K (1 where there are none: the product is then exact)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int sub = lane / LPR;     // which of the pass's rows
     const int li = lane % LPR;      // position inside the row
+    if (p.nap > 0 && !p.rope_cos) {
+        for (int pr = threadIdx.x; pr < p.nap; pr += blockDim.x)
+            s_inv[pr] = 1.0f / powf(p.theta, 2.0f * pr / static_cast<float>(QWEN ? p.freq_denom : HD));
+    }
+    grid_dependency_wait();  // (the frequencies above depend on no kernel in front)
+    grid_launch_dependents();
+    for (int i = threadIdx.x; i < HD; i += blockDim.x) {
+        s_w[0][i] = p.q_weight ? bf16_bits_to_f32(p.q_weight[i]) : 1.0f;
+        s_w[1][i] = p.k_weight ? bf16_bits_to_f32(p.k_weight[i]) : 1.0f;
+    }
+
     const int rows_q = p.q ? p.nq : 0;
     const int rows_k = p.k_src && p.k_dst ? p.nkv : 0;
     const int rows_v = p.v_dst ? p.nkv : 0;
     const int rows = rows_q + rows_k + rows_v;
-    const int tokens = p.batch * p.seq;  // the host refuses more than 2^31 - 1 tokens
-    const int rounds = (tokens + tpc - 1) / tpc;
-    (void)MAX_TPC;
+    const int units = p.batch * p.seq * chunks;  // the host keeps this below 2^31
+    const int stride = gridDim.x * PREP_WARPS;
 
-    if (p.nap > 0 && !p.rope_cos) {
-        for (int pr = threadIdx.x; pr < p.nap; pr += blockDim.x)
-            s_inv[pr] = 1.0f / powf(p.theta, 2.0f * pr / static_cast<float>(QWEN ? p.freq_denom : HD));
-        __syncthreads();
-    }
-    grid_dependency_wait();  // (the frequencies above depend on no kernel in front)
-    grid_launch_dependents();
-    int it = 0;
-    for (int rd = blockIdx.x; rd < rounds; rd += gridDim.x, ++it) {
-        const int tk0 = rd * tpc;
-        float* s_cos = s_cos2[it & 1];
-        float* s_sin = s_sin2[it & 1];
-        // The tokens of this round, split into (sequence, position) once: the row loop below would
-        // otherwise divide per row.
-        int* s_tok = s_bt[it & 1];
-        if (threadIdx.x < tpc && tk0 + (int)threadIdx.x < tokens) {
-            const int tk = tk0 + threadIdx.x;
-            const int b = tk / p.seq;
-            s_tok[2 * threadIdx.x] = b;
-            s_tok[2 * threadIdx.x + 1] = tk - b * p.seq;
+    // A unit and its rows [r0, r1).  Row r of the token sits r * HD elements behind the pointer of its part (so K's
+    // pointer is set back by Q's rows, V's by Q's and K's), this lane's columns included.
+    struct Unit {
+        int id, b, t, c, r0, r1;
+    };
+    auto set_rows = [&](Unit& u) {
+        u.r0 = u.c * chunk * RPW;
+        u.r1 = u.id < units ? min(rows, u.r0 + chunk * RPW) : u.r0;
+    };
+    auto first_unit = [&]() {
+        Unit u;
+        u.id = blockIdx.x * PREP_WARPS + warp;
+        const int tk = u.id / chunks;
+        u.c = u.id - tk * chunks;
+        u.b = tk / p.seq;
+        u.t = tk - u.b * p.seq;
+        set_rows(u);
+        return u;
+    };
+    // `stride` units on, by carries instead of divisions
+    const int stk = stride / chunks, sc = stride - stk * chunks, sb = stk / p.seq, stt = stk - sb * p.seq;
+    auto advance = [&](Unit& u) {
+        u.id += stride;
+        u.c += sc;
+        const int c1 = u.c >= chunks ? 1 : 0;
+        u.c -= c1 * chunks;
+        u.t += stt + c1;
+        const int c2 = u.t >= p.seq ? 1 : 0;
+        u.t -= c2 * p.seq;
+        u.b += sb + c2;
+        set_rows(u);
+    };
+    const int k0 = rows_q, v0 = rows_q + rows_k;  // first K row, first V row
+    // The walk of the loads, a pass ahead of the work: unit fu, rows from fr on.
+    Unit fu = first_unit();
+    int fr = 0;
+    const uint16_t *fq, *fk, *fv;
+    auto begin_loads = [&]() {
+        fr = fu.r0;
+        fq = p.q + fu.b * p.q_stride_b + fu.t * p.q_stride_t + li * 8;
+        const uint16_t* kr = p.k_src + fu.b * p.ks_stride_b + fu.t * p.ks_stride_t + li * 8;
+        fk = kr - k0 * HD;
+        fv = (p.v_src ? p.v_src + fu.b * p.vs_stride_b + fu.t * p.vs_stride_t + li * 8 : kr) - v0 * HD;
+    };
+    auto fetch = [&](uint4& lo, uint4& hi) {
+        if (fr < fu.r1) {
+            const int r = fr + sub;
+            lo = hi = make_uint4(0u, 0u, 0u, 0u);
+            if (r < fu.r1) {
+                const uint16_t* src = (r < k0 ? fq : r < v0 ? fk : fv) + r * HD;
+                lo = *reinterpret_cast<const uint4*>(src);
+                hi = *reinterpret_cast<const uint4*>(src + HD / 2);
+            }
+            fr += RPW;
+            if (fr >= fu.r1 && fu.id < units - stride) {  // the next unit's first rows follow at once
+                advance(fu);
+                begin_loads();
+            }
         }
-        if (p.nap > 0) {
-            for (int idx = threadIdx.x; idx < tpc * p.nap; idx += blockDim.x) {
-                const int tl = idx / p.nap, pr = idx - tl * p.nap;
-                const int tk = tk0 + tl;
-                if (tk >= tokens) break;
-                const int b = tk / p.seq;
-                const int t = tk - b * p.seq;
-                float c, s;
+    };
+    begin_loads();
+    uint4 nl, nh;
+    nl = nh = make_uint4(0u, 0u, 0u, 0u);
+    fetch(nl, nh);
+    __syncthreads();  // frequencies and weights, while the first rows are on their way
+
+    for (Unit u = first_unit(); u.id < units; advance(u)) {
+        uint32_t turns = 0;  // bit e: element e is rotated
+        const int dl = QWEN ? p.rot_half >> 3 : 0;
+        const bool split = QWEN && p.rot_half != HD / 2;  // pairs inside the row's first half
+        const int pr0 = split ? (li & (dl - 1)) * 8 : li * 8;
+        if (p.nap > 0 && u.r0 < rows_q + rows_k) {
+            __syncwarp();
+            for (int pr = lane; pr < p.nap; pr += 32) {
+                float cv, sv;
                 if (p.rope_cos) {
-                    const long long ti = (long long)b * p.rope_stride_b + (long long)t * p.nap + pr;
-                    c = p.rope_cos[ti];
-                    s = p.rope_sin[ti];
+                    const long long ti = (long long)u.b * p.rope_stride_b + (long long)u.t * p.nap + pr;
+                    cv = p.rope_cos[ti];
+                    sv = p.rope_sin[ti];
                 } else {
                     const int pos = (QWEN && p.mrope_pos)
-                                        ? p.mrope_pos[((long long)b * 3 + mrope_axis(pr, p.sec1, p.sec2)) * p.seq + t]
-                                        : (p.pos_offset ? p.pos_offset[b] : p.pos0) + t;
-                    sincosf(static_cast<float>(pos) * s_inv[pr], &s, &c);
+                                        ? p.mrope_pos[((long long)u.b * 3 + mrope_axis(pr, p.sec1, p.sec2)) * p.seq + u.t]
+                                        : (p.pos_offset ? p.pos_offset[u.b] : p.pos0) + u.t;
+                    sincosf(static_cast<float>(pos) * s_inv[pr], &sv, &cv);
                 }
-                s_cos[tl * (HD / 2) + pr] = c;
-                s_sin[tl * (HD / 2) + pr] = s;
+                s_cos[warp][pr] = cv;
+                s_sin[warp][pr] = sv;
             }
+            __syncwarp();
+            const int n = min(max(p.nap - pr0, 0), 8);
+            turns = split && li >= 2 * dl ? 0u : (1u << n) - 1u;
         }
-        // Readers of these buffers two rounds ago finished before every thread reached the previous
-        // round's barrier, so one barrier per round orders both directions.
-        __syncthreads();
-        const float inv_rows = 1.0f / static_cast<float>(rows);
-        const int slots = tpc * rows;  // (token in round, row) pairs of this round
-        // AHEAD: the addresses of the next pass's rows are worked out and their loads issued before this pass's
-        // rows are processed, so that a warp has two passes' worth of loads in flight instead of waiting out one
-        // DRAM latency per pass.
-        struct Pass {
-            const uint16_t* weight;
-            uint16_t* dst;
-            uint4 rl, rh;
-            int tl;
-            bool valid, rope, norm;
-        };
-        auto fetch = [&](int r0) -> Pass {
-            Pass f;
-            const int slot = r0 + sub;
-            f.tl = static_cast<int>((static_cast<float>(slot) + 0.5f) * inv_rows);  // exact: slot < 2^20
-            const int r = slot - f.tl * rows;
-            const int tk = tk0 + f.tl;
-            f.valid = slot < slots && tk < tokens;
-            const int b = f.valid ? s_tok[2 * f.tl] : 0;
-            const int t = f.valid ? s_tok[2 * f.tl + 1] : 0;
-            const uint16_t* src = nullptr;
-            f.dst = nullptr;
-            f.weight = nullptr;
-            f.rope = false;
-            f.norm = true;
-            if (f.valid) {
-                if (r < rows_q) {
-                    src = f.dst = p.q + b * p.q_stride_b + t * p.q_stride_t + (long long)r * HD;
-                    f.weight = p.q_weight;
-                    f.rope = true;
-                } else if (r < rows_q + rows_k) {
-                    const int h = r - rows_q;
-                    src = p.k_src + b * p.ks_stride_b + t * p.ks_stride_t + (long long)h * HD;
-                    f.dst = p.k_dst + b * p.kd_stride_b + t * p.kd_stride_t + (long long)h * HD;
-                    f.weight = p.k_weight;
-                    f.rope = true;
-                } else {
-                    const int h = r - rows_q - rows_k;
-                    src = p.v_src ? p.v_src + b * p.vs_stride_b + t * p.vs_stride_t + (long long)h * HD
-                                  : p.k_src + b * p.ks_stride_b + t * p.ks_stride_t + (long long)h * HD;
-                    f.dst = p.v_dst + b * p.vd_stride_b + t * p.vd_stride_t + (long long)h * HD;
-                    f.norm = !(QWEN && p.v_copy);
-                }
-            }
-            f.rl = make_uint4(0u, 0u, 0u, 0u);
-            f.rh = f.rl;
-            if (f.valid) {
-                f.rl = *reinterpret_cast<const uint4*>(src + li * 8);
-                f.rh = *reinterpret_cast<const uint4*>(src + HD / 2 + li * 8);
-            }
-            return f;
-        };
-        Pass nxt;
-        if (AHEAD) nxt = fetch(warp * RPW);
-        for (int r0 = warp * RPW; r0 < slots; r0 += 8 * RPW) {
-            const Pass cur = AHEAD ? nxt : fetch(r0);
-            if (AHEAD && r0 + 8 * RPW < slots) nxt = fetch(r0 + 8 * RPW);
-            const bool valid = cur.valid, rope = cur.rope, norm = cur.norm;
-            const int tl = cur.tl;
-            const uint16_t* weight = cur.weight;
-            uint16_t* dst = cur.dst;
-            const uint4 rl = cur.rl, rh = cur.rh;
-            float lo[8], hi[8];
-            unpack8(rl, lo);
-            unpack8(rh, hi);
-            float ss = 0.f;
+        uint16_t* dq = p.q + u.b * p.q_stride_b + u.t * p.q_stride_t + li * 8;
+        uint16_t* dk = p.k_dst + u.b * p.kd_stride_b + u.t * p.kd_stride_t + li * 8 - k0 * HD;
+        uint16_t* dv = p.v_dst + u.b * p.vd_stride_b + u.t * p.vd_stride_t + li * 8 - v0 * HD;
+        for (int r0 = u.r0; r0 < u.r1; r0 += RPW) {
+            const uint4 rl = nl, rh = nh;
+            fetch(nl, nh);
+            const int r = r0 + sub;
+            const bool is_v = r >= v0;
+            uint16_t* dst = (r < k0 ? dq : r < v0 ? dk : dv) + r * HD;
+            uint4 ol = rl, oh = rh;
+            if (!(QWEN && p.v_copy && r0 >= v0)) {  // (rows of the warp that are only copied need no norm)
+                float lo[8], hi[8];
+                unpack8(rl, lo);
+                unpack8(rh, hi);
+                float ss = 0.f;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) ss += lo[e] * lo[e] + hi[e] * hi[e];
+                for (int e = 0; e < 8; ++e) ss += lo[e] * lo[e] + hi[e] * hi[e];
 #pragma unroll
-            for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            const float rms_inv = rsqrtf(ss / static_cast<float>(HD) + p.eps);
-            if (!norm) {
-                // appended as it is
-            } else if (weight) {
-                float wl[8], wh[8];
-                unpack8(*reinterpret_cast<const uint4*>(weight + li * 8), wl);
-                unpack8(*reinterpret_cast<const uint4*>(weight + HD / 2 + li * 8), wh);
+                for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                const float rms_inv = rsqrtf(ss / static_cast<float>(HD) + p.eps);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    lo[e] = bf16_rne(lo[e] * rms_inv * wl[e]);
-                    hi[e] = bf16_rne(hi[e] * rms_inv * wh[e]);
-                }
-            } else {
+                for (int e = 0; e < 8; ++e) lo[e] *= rms_inv, hi[e] *= rms_inv;
+                if (r0 < v0) {  // some row of the pass is a Q or K row
+                    const float* w = s_w[r < k0 ? 0 : 1] + li * 8;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    lo[e] = bf16_rne(lo[e] * rms_inv);
-                    hi[e] = bf16_rne(hi[e] * rms_inv);
-                }
-            }
-            if (QWEN && p.rot_half != HD / 2) {
-                // Pairs (f, f + rot_half) both sit in the row's first half, rot_half / 8 lanes apart: the
-                // partner's values come by shuffle (every lane takes part; only the rotary lanes update).
-                const int dl = p.rot_half >> 3;
-                const bool mine = rope && li < 2 * dl;
-                const bool first = (li & dl) == 0;
-                const float* tc = s_cos + tl * (HD / 2);
-                const float* ts = s_sin + tl * (HD / 2);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const float other = __shfl_xor_sync(0xffffffffu, lo[e], dl);
-                    const int pr = (li & (dl - 1)) * 8 + e;
-                    if (mine && pr < p.nap) {
-                        const float c = tc[pr], s = ts[pr];
-                        lo[e] = first ? lo[e] * c - other * s : other * s + lo[e] * c;
+                    for (int e = 0; e < 8; e += 4) {
+                        const float4 a = *reinterpret_cast<const float4*>(w + e), b = *reinterpret_cast<const float4*>(w + HD / 2 + e);
+                        if (r0 + RPW <= v0 || !is_v) {
+                            lo[e] *= a.x, lo[e + 1] *= a.y, lo[e + 2] *= a.z, lo[e + 3] *= a.w;
+                            hi[e] *= b.x, hi[e + 1] *= b.y, hi[e + 2] *= b.z, hi[e + 3] *= b.w;
+                        }
                     }
                 }
-            } else if (rope) {
-                const float* tc = s_cos + tl * (HD / 2);
-                const float* ts = s_sin + tl * (HD / 2);
+                ol = pack8(lo);
+                oh = pack8(hi);
+                if (r0 < v0 && p.nap > 0) {
+                    unpack8(ol, lo);  // the rotation works on the rounded values
+                    unpack8(oh, hi);
+                    float c[8], s[8];  // (from nap on whatever was there: not used)
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const int pr = li * 8 + e;
-                    if (pr < p.nap) {
-                        const float c = tc[pr], s = ts[pr];
-                        const float x0 = lo[e], x1 = hi[e];
-                        lo[e] = x0 * c - x1 * s;
-                        hi[e] = x0 * s + x1 * c;
+                    for (int e = 0; e < 8; e += 4) {
+                        const float4 cv = *reinterpret_cast<const float4*>(&s_cos[warp][pr0 + e]), sv = *reinterpret_cast<const float4*>(&s_sin[warp][pr0 + e]);
+                        c[e] = cv.x, c[e + 1] = cv.y, c[e + 2] = cv.z, c[e + 3] = cv.w;
+                        s[e] = sv.x, s[e + 1] = sv.y, s[e + 2] = sv.z, s[e + 3] = sv.w;
+                    }
+                    if (split) {
+                        // Pairs (f, f + rot_half) both sit in the row's first half, rot_half / 8 lanes apart: the
+                        // partner's values come by shuffle (every lane takes part; only the rotary lanes update).
+                        const bool first = (li & dl) == 0;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const float other = __shfl_xor_sync(0xffffffffu, lo[e], dl);
+                            if ((turns >> e) & 1u) lo[e] = first ? lo[e] * c[e] - other * s[e] : other * s[e] + lo[e] * c[e];
+                        }
+                    } else if (p.nap == HD / 2) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const float x0 = lo[e], x1 = hi[e];
+                            lo[e] = x0 * c[e] - x1 * s[e];
+                            hi[e] = x0 * s[e] + x1 * c[e];
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const float x0 = lo[e], x1 = hi[e];
+                            const bool on = (turns >> e) & 1u;
+                            lo[e] = on ? x0 * c[e] - x1 * s[e] : x0;
+                            hi[e] = on ? x0 * s[e] + x1 * c[e] : x1;
+                        }
+                    }
+                    if (r0 + RPW <= v0) {
+                        ol = pack8(lo);
+                        oh = pack8(hi);
+                    } else if (!is_v) {  // (V rows beside K rows are not rotated)
+                        ol = pack8(lo);
+                        oh = pack8(hi);
                     }
                 }
+                if (QWEN && p.v_copy && is_v) ol = rl, oh = rh;
             }
-            if (valid) {
-                *reinterpret_cast<uint4*>(dst + li * 8) = pack8(lo);
-                *reinterpret_cast<uint4*>(dst + HD / 2 + li * 8) = pack8(hi);
+            if (r < u.r1) {
+                *reinterpret_cast<uint4*>(dst) = ol;
+                *reinterpret_cast<uint4*>(dst + HD / 2) = oh;
             }
         }
     }
