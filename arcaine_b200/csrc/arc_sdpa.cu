@@ -329,8 +329,12 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     kp.out_lse = p->out_lse;
     kp.part_o = plan.splits > 1 ? static_cast<float*>(p->workspace) : nullptr;
     kp.part_lse = kp.part_o ? kp.part_o + (size_t)plan.splits * plan.rows * HD : nullptr;
-    if (p->block_ids) {
-        // span ends per query row, once per call: a few microseconds instead of a (seq, kv_len) f32 mask
+    // CTA pairs (prefill_wide_sm100.cuh) look vision blocks up themselves; the one-tile kernel wants the span end of every
+    // row (a few microseconds instead of a (seq, kv_len) f32 mask).
+    const bool wide = HD == 256 && plan.splits == 1 && plan.cluster == 0;
+    if (p->block_ids && wide) {
+        kp.ids = p->block_ids + p->block_ids_offset;
+    } else if (p->block_ids) {
         int* vis = reinterpret_cast<int*>(static_cast<unsigned char*>(p->workspace) + plan.split_bytes);
         ARC_CUDA(launch_dependent(vision_span_kernel, dim3((unsigned)((p->seq + 255) / 256)), dim3(256), 0, stream, 1, p->block_ids,
                                   p->block_ids_offset, p->kv_len - p->seq, p->seq, p->kv_len, vis));
@@ -418,7 +422,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     // and pair of tiles where a CTA on its own takes 3700 per tile.
     const bool masked = kp.mask_type == 1 && kp.mask != nullptr;
     // (a caller who brings no workspace for the scanned mask gets the one-tile kernel, which reads the mask itself)
-    if (HD == 256 && plan.splits == 1 && plan.cluster == 0 &&
+    if (wide &&
         (!masked || (plan.mask_bytes > 0 && plan.q_tiles < 16384 && p->workspace && aligned16(p->workspace) && p->workspace_bytes >= plan.ws_bytes + plan.mask_bytes))) {
         if (masked) {
             kp.mask_blocks = (p->kv_len + 127) / 128;

@@ -61,6 +61,7 @@ struct PrefillParams {
     const uint32_t* mask_class;  // [row tile][key block]: a byte per 32 rows, MASK_* bits
     const uint4* mask_bits;      // [row tile][key block][row]: one bit per key, set where the mask is 0
     int mask_blocks;
+    const int* ids;  // prefill_wide_sm100.cuh: vision-block ids, ids[j] that of key j (instead of vis_hi)
 };
 
 // One CTA per SM, persistent: it takes tiles (128 query tokens of one query head) round-robin

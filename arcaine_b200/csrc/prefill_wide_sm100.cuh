@@ -138,13 +138,54 @@ __device__ __forceinline__ void add_mask_values(uint32_t tS, const float* mask_r
     tmem_wait_st();
 }
 
+// ---------------------------------------------------------------------------
+// Vision blocks (a query inside a block of equal non-negative ids also sees the block's later keys).  The ends are looked
+// up where they are needed: a launch of its own for one end per row took 4.5 us in front of a kernel of 20.
+// ---------------------------------------------------------------------------
+// First key after `key` that does not carry `id`.  Whole warps, 128 keys a step.
+__device__ __forceinline__ int run_end(const int* ids, int kv_len, int key, int id) {
+    const int lane = threadIdx.x & 31;
+    for (int k0 = key + 1;; k0 += 128) {
+        bool other[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) other[i] = k0 + 32 * i + lane >= kv_len || ids[k0 + 32 * i + lane] != id;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t found = __ballot_sync(0xffffffffu, other[i]);
+            if (found) return k0 + 32 * i + __ffs(found) - 1;
+        }
+    }
+}
+
+// First key the row at key position `self` does not see.  Same position in every lane.
+__device__ __forceinline__ int vision_end(const PrefillParams& p, int self) {
+    const int plain = min(max(self + 1, 0), p.kv_len);
+    if (self < 0 || self >= p.kv_len) return plain;
+    const int id = p.ids[self];
+    return id >= 0 ? run_end(p.ids, p.kv_len, self, id) : plain;
+}
+
+// The same for a warp's 32 consecutive rows, one per lane (row: t < seq).
+__device__ __forceinline__ int vision_ends(const PrefillParams& p, int self, bool row) {
+    const int lane = threadIdx.x & 31;
+    const int id = row && self >= 0 && self < p.kv_len ? p.ids[self] : -1;
+    const int next_id = __shfl_down_sync(0xffffffffu, id, 1);  // (all lanes take part; lane 31 does not use it)
+    const uint32_t breaks = __ballot_sync(0xffffffffu, lane < 31 && id != next_id);
+    const int last_id = __shfl_sync(0xffffffffu, id, 31), last = __shfl_sync(0xffffffffu, self, 31);
+    const int end = last_id >= 0 ? run_end(p.ids, p.kv_len, last, last_id) : 0;  // of the block that leaves the warp's rows
+    if (id < 0) return min(max(self + 1, 0), p.kv_len);
+    const uint32_t ahead = breaks >> lane;
+    return ahead ? self + __ffs(ahead) : end;
+}
+
 __device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first, int q_last, int& lo, int& hi) {
     const int off = p.kv_len - p.seq;
     lo = 0;
     hi = (p.kv_len + WideCfg::BN - 1) / WideCfg::BN;
     if (p.mask_type == 3) {
         q_last = min(q_last, p.seq - 1);
-        const int last_key = p.vis_hi ? p.vis_hi[q_last] - 1 : min(p.kv_len - 1, q_last + off);
+        // (the span ends are monotone in the row, so the last row decides)
+        const int last_key = p.ids ? vision_end(p, q_last + off) - 1 : min(p.kv_len - 1, q_last + off);
         hi = last_key >= 0 ? last_key / WideCfg::BN + 1 : 0;
         if (p.window > 0 && p.window != 0x7fffffff) lo = max(0, q_first + off - p.window + 1) / WideCfg::BN;
     }
@@ -515,14 +556,25 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             if (causal) {
                 const int diag = t + off;
                 row_hi = min(max(diag + 1, 0), p.kv_len);
-                if (p.vis_hi && t < p.seq) row_hi = p.vis_hi[t];  // a vision block's later keys are visible too
+                if (p.ids) row_hi = vision_ends(p, diag, t < p.seq);
                 if (windowed) row_lo = max(0, diag - p.window + 1);
                 if (row_lo > row_hi) row_lo = row_hi;
             }
             const RowMask rm{row_lo, row_hi, p.kv_len, nullptr};
             float m = -CUDART_INF_F;  // running max, log2 domain, possibly stale by <= 8
             float l = 0.f;            // row sum
+            // (MASKED: a block's class is asked for a block ahead, its bits before its scores are waited for)
+            auto class_of = [&](int j) -> uint32_t {
+                return MASKED && w.q0 < p.seq && j < w.hi
+                           ? reinterpret_cast<const uint8_t*>(p.mask_class + (long long)(w.q0 >> 7) * p.mask_blocks + j)[quarter]
+                           : 0u;
+            };
+            uint32_t cls = class_of(w.lo);
             for (int j = w.lo; j < w.hi; ++j, ++g) {
+                const uint32_t next_cls = class_of(j + 1);
+                const bool by_bits = (cls & (MASK_HIDDEN | MASK_VALUES)) == MASK_HIDDEN;
+                uint4 bits = make_uint4(0u, 0u, 0u, 0u);
+                if (MASKED && by_bits) bits = p.mask_bits[((long long)(w.q0 >> 7) * p.mask_blocks + j) * 128 + r];
                 const int kc = j * C::BN, st = g & 1;
                 const uint32_t tS = tmem_base + lane_sel + C::COL_S + st * 128;
                 if (!mbar_wait_inline(&s_full[st], (g >> 1) & 1)) {
@@ -531,8 +583,6 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                     break;
                 }
                 tc_fence_after_sync();
-                const long long at = MASKED ? (long long)(w.q0 >> 7) * p.mask_blocks + j : 0;
-                const uint32_t cls = MASKED && w.q0 < p.seq ? reinterpret_cast<const uint8_t*>(p.mask_class + at)[quarter] : 0u;
                 if (MASKED && (cls & MASK_VALUES))
                     add_mask_values(tS, t < p.seq ? p.mask + (long long)t * p.kv_len : nullptr, kc, p.kv_len, 1.4426950408889634f / sl);
                 tmem_ld32(tS, s0);
@@ -541,8 +591,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 tmem_ld32(tS + 96, s3);
                 tmem_wait_ld();
                 if constexpr (MASKED) {
-                    if ((cls & (MASK_HIDDEN | MASK_VALUES)) == MASK_HIDDEN) {
-                        const uint4 bits = p.mask_bits[at * 128 + r];
+                    if (by_bits) {
                         select_chunk(s0, bits.x);
                         select_chunk(s1, bits.y);
                         select_chunk(s2, bits.z);
@@ -603,6 +652,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 tmem_st16(tS + 32, pk);
                 exp_chunk(s3, pk, ls2, sl2, nm2);
                 tmem_st16(tS + 48, pk);
+                cls = next_cls;
                 float l0, l1, l2, l3;
                 unpack_f32x2(ls2[0], l0, l1);
                 unpack_f32x2(ls2[1], l2, l3);

@@ -101,3 +101,22 @@ def test_additive_mask(seq, kv, nq, nkv, kind):
     assert _lib.load().arc_sdpa_prefill(C.byref(p), torch.cuda.current_stream().cuda_stream) == _lib.ARC_OK
     assert_close(o2, want[0], kind + " without a workspace")
     assert ops.device_status() == (0, 0)
+
+
+def test_vision_blocks_longer_than_a_search_step():
+    """Block ids looked up in the kernel (128 keys a step, 32 rows a warp) against the additive buffer of the same rule:
+    blocks of one token, next to each other, across warps and tiles, longer than a step, and up to the last key."""
+    from arcaine_b200 import ops
+    ops.clear_device_status()
+    seq, kv, nq, nkv, hd = 900, 1000, 12, 4, 256
+    ids = torch.full((kv,), -1, dtype=torch.int32)
+    for i, (a, b) in enumerate([(30, 31), (31, 100), (140, 160), (227, 260), (260, 261), (300, 711), (840, 1000)]):
+        ids[a:b] = i
+    q, k, v = (seeded_bf16(n, h, hd, seed=40 + h).cuda() for n, h in ((seq, nq), (kv, nkv), (kv, nkv)))
+    for window in (oracle.INT_MAX, 200):
+        mask = ops.fill_causal_mask_with_block_ids(ids.cuda(), seq, kv, kv - seq, window)
+        want = ops.sdpa_prefill(q, k, v, scale=0.0625, mask_type=ops.MASK_EXPLICIT, mask=mask)
+        got = ops.sdpa_prefill(q, k, v, scale=0.0625, mask_type=ops.MASK_CAUSAL, window=window, block_ids=ids.cuda())
+        # the same visible keys; blocks may be skipped in one form and fully masked in the other
+        assert_close(got, want.float(), f"window {window}", rel_tol=2e-3, abs_tol=8e-3)
+    assert ops.device_status() == (0, 0)
