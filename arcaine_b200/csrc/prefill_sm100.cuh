@@ -90,7 +90,7 @@ struct PrefillCfg {
     static constexpr int NSB = (HD == 128) ? 3 : 2;  // score buffers: S = Q K^T runs NSB-1 blocks ahead of the softmax
     static constexpr int COL_S = 0;                  // NSB buffers of 128 fp32 columns; P (bf16) is written over them
     static constexpr int COL_O = NSB * 128;          // HD fp32 columns
-    static constexpr int NUM_BARS = 2 + 2 * K_STAGES + 2 * V_STAGES + 2 * NSB + 1 + 2 + 2;  // the last two: cluster merge
+    static constexpr int NUM_BARS = 2 + 2 * K_STAGES + 2 * V_STAGES + 2 * NSB + 2 + 2 + 2;  // the last two: cluster merge
     static constexpr int XCH_FLOATS = 2 * 2 * 128 + 2 * 128 + 2 * 128;  // row-max exchange (2 phases), row-sum exchange, (max, sum) per row for the cluster merge
     static constexpr int SMEM_BYTES = (1 + K_STAGES + V_STAGES) * TILE_BYTES + NUM_BARS * 8 + 16 + XCH_FLOATS * 4 + 1024;
     static constexpr int SOFTMAX_WARPS = 8;
@@ -377,8 +377,12 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     uint64_t* v_empty = v_full + VS;
     uint64_t* s_full = v_empty + VS;    // [NSB] score buffers
     uint64_t* p_full = s_full + NSB;    // [NSB]
-    uint64_t* pv_done = p_full + NSB;   // one phase per key block: O += P V of that block has completed
-    uint64_t* o_full = pv_done + 1;     // one phase per tile: the tile's last O += P V has completed
+    // [key block & 1]: O += P V of that block has completed.  Two barriers, because with three score buffers a softmax warp
+    // may ask for block g's while that of block g - 1 still runs: on one barrier the parity it waits for is then also
+    // that of block g - 2, and it would rescale O under the MMA.  (P V of block g - 2 has completed: the scores it has of
+    // block g + 1 were computed behind it.)
+    uint64_t* pv_done = p_full + NSB;
+    uint64_t* o_full = pv_done + 2;     // one phase per tile: the tile's last O += P V has completed
     uint64_t* o_empty = o_full + 1;     // one phase per tile: the softmax warps have read O out
     uint64_t* part_ready = o_empty + 1;  // cluster merge, one phase per tile: every CTA's share of the tile is in its shared memory
     uint64_t* read_done = part_ready + 1; // cluster merge, one phase per tile: every CTA has finished reading this CTA's share
@@ -419,7 +423,8 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
             mbar_init(&s_full[s], 1);
             mbar_init(&p_full[s], 32 * C::SOFTMAX_WARPS);
         }
-        mbar_init(pv_done, 1);
+        mbar_init(&pv_done[0], 1);
+        mbar_init(&pv_done[1], 1);
         mbar_init(o_full, 1);
         mbar_init(o_empty, 32 * C::SOFTMAX_WARPS);
         mbar_init(part_ready, csize);  // one arrival per CTA of the cluster
@@ -591,7 +596,7 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
                     for (int c = 0; c < C::BN / 32; ++c, tP += 32, dVu += 256, acc = 1u)
                         umma_ts_x2<8, 128>(tO, tP, dVu, IDESC_PV, acc);
                     umma_commit_warp(&v_empty[gp % VS]);
-                    umma_commit_warp(pv_done);
+                    umma_commit_warp(&pv_done[gp & 1]);
                     ++gp;
                 }
                 if (ok) umma_commit_warp(o_full);
@@ -900,7 +905,7 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
                         // memory (the row's other thread takes the same decision from the same values).
                         const float alpha = (m_new == -CUDART_INF_F) ? 1.0f : fast_exp2(m - m_new);
                         tmem_wait_ld();
-                        if (!mbar_wait_warp(pv_done, g & 1)) {
+                        if (!mbar_wait_warp(&pv_done[g & 1], (g >> 1) & 1)) {
                             report_fault(p.fault, FAULT_WAIT_O, g);
                             ok = false;
                             continue;
@@ -957,7 +962,7 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
                         // landed, rescale this thread's half of O in tensor memory (the row's other thread takes
                         // the same decision from the same values).
                         const float alpha = (m_new == -CUDART_INF_F) ? 1.0f : fast_exp2(m - m_new);
-                        if (!mbar_wait_warp(pv_done, (g - 1) & 1)) {
+                        if (!mbar_wait_warp(&pv_done[(g - 1) & 1], ((g - 1) >> 1) & 1)) {
                             report_fault(p.fault, FAULT_WAIT_O, g);
                             ok = false;
                             continue;

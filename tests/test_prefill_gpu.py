@@ -316,3 +316,18 @@ def test_gemma4_decode_wrappers(ops):
     got1 = ops.gemma4_full_decode_attention(q1.cuda(), k1.cuda(), v1.cuda(), n, nq1, hd1)
     want1, _ = oracle.sdpa_f32(q1[None], k1, v1, scale=1.0)
     assert_close(got1, want1[0], "gemma4 full-attention decode, one KV head")
+
+
+@pytest.mark.parametrize("window", [523, 540, 600])
+def test_few_keys_in_the_first_block_repeat_bit_for_bit(ops, window):
+    """A window that leaves most rows a few keys of their first key block: the next block raises their maximum by far
+    more than 2^8, so the accumulator is rescaled while earlier P V products may still run.  One-tile kernel."""
+    seq, kv_len, nq, nkv, hd = 400, 1466, 16, 8, 128
+    q, k, v = seeded_bf16(1, seq, nq, hd, seed=61), seeded_bf16(1, kv_len, nkv, hd, seed=62), seeded_bf16(1, kv_len, nkv, hd, seed=63)
+    want = oracle.sdpa_f32(q[0], k[0], v[0], scale=hd ** -0.5, mask_type=3, window=window)[0]
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    run = lambda: ops.sdpa_prefill(qd, kd, vd, scale=hd ** -0.5, mask_type=3, window=window, num_splits=1)  # noqa: E731
+    first = run()
+    assert_close(first[0], want, f"window {window}")
+    for _ in range(40):
+        assert torch.equal(first, run())
