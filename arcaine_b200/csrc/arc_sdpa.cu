@@ -9,6 +9,7 @@
 
 #include <atomic>
 #include <cmath>
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -31,6 +32,14 @@ constexpr int kMaxDevices = 64;
 // may use the opt-in maximum minus this reserve.
 constexpr int kDecodeStaticSmem = 1024;
 
+// What the device holds of the CTA pairs of prefill_wide_sm100.cuh at once (the defaults: a B200).
+struct WideRoom {
+    static constexpr int MOST_FOLDED = WideCfg::MOST_FOLDED;
+    int pairs = 74;
+    int folded[MOST_FOLDED + 1] = {0, 0, 33, 22};  // clusters of that many pairs
+    int clusters(int parts) const { return parts <= MOST_FOLDED ? folded[parts] : 0; }
+};
+
 struct DeviceState {
     std::atomic<bool> ready{false};  // set (release) once everything below is written
     uint32_t* fault = nullptr;
@@ -39,9 +48,8 @@ struct DeviceState {
     // largest cluster size (2, 4 or 8; 0 = none) the cluster form of the prefill kernel can be launched with, per head dim
     // [head dim 128 / 256][log2(cluster size)]: how many clusters of 2 or 4 CTAs of the cluster form of the
     // prefill kernel the device can hold at once (0: that size cannot be launched)
-    int active_clusters[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
     int decode_clusters[4] = {0, 0, 0, 0};  // [log2(size)]: clusters of the one-launch decode the device holds at once
-    int wide_pairs = 0;  // CTA pairs of the head-dim-256 kernel the device holds at once
+    WideRoom wide;
 };
 
 static DeviceState g_dev[kMaxDevices];
@@ -127,24 +135,16 @@ static int device_state(DeviceState** out) {
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, false, false>, PrefillCfg<128>::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, false, true>, PrefillCfg<128>::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, true, true>, PrefillCfg<128>::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<256, false, false>, PrefillCfg<256>::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<256, false, true>, PrefillCfg<256>::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<256, true, true>, PrefillCfg<256>::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, false, false, true>, PrefillCfg<128>::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<256, false, false, true>, PrefillCfg<256>::SMEM_BYTES));
-            for (int hi = 0; hi < 2; ++hi) {
-                for (int cs = 2, lg = 1; cs <= 4; cs *= 2, ++lg) {
-                    s.active_clusters[hi][lg] =
-                        hi ? clusters_at_once(sdpa_prefill_kernel<256, false, false, true>, cs, s.sm_count, PrefillCfg<256>::THREADS, PrefillCfg<256>::SMEM_BYTES)
-                           : clusters_at_once(sdpa_prefill_kernel<128, false, false, true>, cs, s.sm_count, PrefillCfg<128>::THREADS, PrefillCfg<128>::SMEM_BYTES);
-                }
-            }
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, false>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true, false>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, true>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true, true>, WideCfg::SMEM_BYTES));
-            s.wide_pairs = clusters_at_once(sdpa_prefill_wide_kernel<false, false>, 2, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
-            if (s.wide_pairs < 1) {
+            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, false, true>, WideCfg::SMEM_BYTES));
+            s.wide.pairs = clusters_at_once(sdpa_prefill_wide_kernel<false, false>, 2, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
+            for (int parts = 2; parts <= WideRoom::MOST_FOLDED; ++parts)
+                s.wide.folded[parts] = clusters_at_once(sdpa_prefill_wide_kernel<false, false, true>, 2 * parts, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
+            if (s.wide.pairs < 1) {
                 std::snprintf(g_last_error, sizeof(g_last_error), "the device cannot hold a CTA pair of the prefill kernel");
                 return ARC_ERR_CUDA;
             }
@@ -245,14 +245,36 @@ static int make_cache_map(CUtensorMap* tm, const void* base, int row_elems, int6
 struct PrefillPlan {
     int q_tiles = 0;
     int splits = 1;
-    int cluster = 0;         // > 0: the splits are the CTAs of a thread-block cluster of this size, folded in the kernel
     long long rows = 0;
     size_t split_bytes = 0;  // partial records of key-range splits, at the start of the workspace
     size_t ws_bytes = 0;     // what must be there: partial records, then the per-row span ends of block_ids
     size_t mask_bytes = 0;   // behind it, if it is there: the classes and bits of an additive mask
 };
 
-static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const int* active_clusters, PrefillPlan* plan) {
+// Head dim 256: units of the CTA pairs' list, and how many parts the key range of each is worth when the units alone
+// would leave pairs idle.  Measured (us): a key block of a pair 1.13; records and fold 3 + 0.04 per pair in a cluster, 2.5 +
+// 0.06 per pair with a merge launch (every pair writes its 256 rows as f32, 32 bytes per clk and SM), whatever the number
+// of parts.  (256 queries of 16 heads over 2304 keys: 26.7 us whole, 19.1 in three parts, 19.6 in four; of 8 heads 26.2,
+// 15.6 in six.)
+static long long wide_units(const arc_sdpa_prefill_params* p, int q_tiles) {
+    const bool head_pair = ((p->nq / p->nkv) & 1) == 0;
+    return (head_pair ? (long long)q_tiles * (p->nq / 2) : (long long)((p->seq + 255) / 256) * p->nq) * p->batch;
+}
+
+static int choose_wide_splits(const arc_sdpa_prefill_params* p, int q_tiles, const WideRoom& room) {
+    const long long units = wide_units(p, q_tiles);
+    int most = (p->kv_len + 127) / 128;  // key blocks of the longest unit
+    if (p->mask_type == ARC_MASK_CAUSAL && p->window > 0 && p->window < p->kv_len && !p->block_ids) most = std::min(most, (p->window + 255) / 128 + 1);
+    int best = 1;
+    double least = 1.13 * most;
+    for (int s = 2; s <= 8 && s <= most && units * s <= room.pairs; ++s) {
+        const double t = 1.13 * ((most + s - 1) / s) + (units <= room.clusters(s) ? 3.0 + 0.04 * (units * s) : 2.5 + 0.06 * (units * s));
+        if (t < least) least = t, best = s;
+    }
+    return best;
+}
+
+static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const WideRoom& room, PrefillPlan* plan) {
     if (!p) return ARC_ERR_NULL_POINTER;
     if (p->batch <= 0 || p->seq <= 0 || p->kv_len <= 0 || p->nq <= 0 || p->nkv <= 0 || p->nq % p->nkv != 0)
         return ARC_ERR_BAD_SHAPE;
@@ -268,6 +290,7 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const in
     const long long tiles = (long long)plan->q_tiles * p->nq * p->batch;
     const bool scanned_mask = p->mask_type == ARC_MASK_EXPLICIT && p->hd == 256 && p->num_splits <= 1;
     if (splits == 0 && scanned_mask) splits = 1;
+    if (splits == 0 && p->hd == 256) splits = choose_wide_splits(p, plan->q_tiles, room);
     if (splits == 0) {
         // Split the key range only when the tiles alone leave most SMs idle and there are enough key blocks
         // to pay for folding the parts again (measured: about 8 us for the fold against 1.3-2 us per key
@@ -283,22 +306,6 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const in
     }
     if (splits > kv_blocks) splits = kv_blocks;
     if (splits > 64) splits = 64;
-    // A split the library chose itself is run as a thread-block cluster where the device allows it: the
-    // CTAs of a tile fold their accumulators through distributed shared memory in the same launch, no
-    // partial records, no merge kernel, no workspace.  An explicit num_splits keeps the two-launch form.
-    // All tiles' clusters must be resident at once (clusters are placed inside one GPC each, so fewer fit
-    // than SMs / size suggests; a second wave would double the time).  Head dim 256 only: at head dim 128 the two-launch form measured
-    // 5-7 us faster (the cluster instance of that kernel does not fit its register budget without spills).
-    if (p->num_splits == 0 && (splits == 2 || splits == 4) && p->hd == 256 && active_clusters &&
-        p->mask_type != ARC_MASK_EXPLICIT) {
-        // (two or four parts: with eight, a CTA reads seven eighths of its rows from the others and the
-        // two-launch form measured 2-3 us faster; three parts would have to become two)
-        const int lg = splits == 2 ? 1 : 2;
-        if (active_clusters[lg] >= tiles) {
-            plan->cluster = splits;
-            splits = 1;
-        }
-    }
     plan->splits = splits;
     plan->split_bytes = splits > 1 ? (size_t)splits * plan->rows * ((size_t)p->hd + 1) * sizeof(float) : 0;
     plan->split_bytes = (plan->split_bytes + 15) & ~(size_t)15;
@@ -306,8 +313,34 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const in
     if (scanned_mask) plan->mask_bytes = (size_t)plan->q_tiles * kv_blocks * (128 * sizeof(uint4) + sizeof(uint32_t));
     if (p->block_ids) {
         if (p->mask_type != ARC_MASK_CAUSAL || p->block_ids_offset < 0) return ARC_ERR_BAD_SHAPE;
-        plan->ws_bytes += ((size_t)p->seq * sizeof(int32_t) + 15) & ~(size_t)15;
+        if (p->hd == 128) plan->ws_bytes += ((size_t)p->seq * sizeof(int32_t) + 15) & ~(size_t)15;
     }
+    return ARC_OK;
+}
+
+// The parts of a split key range, folded, gated and stored.
+template <int HD>
+static int launch_fold(const arc_sdpa_prefill_params* p, const PrefillPlan& plan, const PrefillParams& kp, cudaStream_t stream) {
+    UniformMergeParams mp{};
+    mp.part_o = kp.part_o;
+    mp.part_lse = kp.part_lse;
+    mp.gate = kp.gate;
+    mp.out = kp.out;
+    mp.out_f32 = nullptr;
+    mp.out_lse = p->out_lse;
+    mp.rows = plan.rows;
+    mp.num_parts = plan.splits;
+    mp.o_part_stride = plan.rows * HD;
+    mp.lse_part_stride = plan.rows;
+    mp.seq = p->seq;
+    mp.nq = p->nq;
+    mp.o_stride_b = p->o_stride_b;
+    mp.o_stride_t = p->o_stride_t;
+    mp.out_copies = kp.out_copies;
+    mp.n_copies = kp.n_copies;
+    ARC_CUDA(launch_dependent(plan.splits <= 4 ? sdpa_uniform_merge_kernel<HD, 4> : sdpa_uniform_merge_kernel<HD, 8>, dim3((unsigned)((plan.rows + UMERGE_ROWS - 1) / UMERGE_ROWS)),
+                              dim3(32 * UMERGE_ROWS), 0, stream, 1, mp));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
     return ARC_OK;
 }
 
@@ -331,7 +364,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     kp.part_lse = kp.part_o ? kp.part_o + (size_t)plan.splits * plan.rows * HD : nullptr;
     // CTA pairs (prefill_wide_sm100.cuh) look vision blocks up themselves; the one-tile kernel wants the span end of every
     // row (a few microseconds instead of a (seq, kv_len) f32 mask).
-    const bool wide = HD == 256 && plan.splits == 1 && plan.cluster == 0;
+    const bool wide = HD == 256 && (plan.splits == 1 || p->mask_type != ARC_MASK_EXPLICIT);
     if (p->block_ids && wide) {
         kp.ids = p->block_ids + p->block_ids_offset;
     } else if (p->block_ids) {
@@ -361,7 +394,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
 
     // Head dim 128: two query tiles per CTA (prefill_pair_sm100.cuh) when that is the faster way to cover
     // the tiles.  ARC_SDPA_PREFILL_KERNEL=single|pair overrides the choice (for A/B measurements).
-    if (HD == 128 && plan.splits == 1 && plan.cluster == 0 && !(kp.mask_type == 1 && kp.mask != nullptr) && kp.vis_hi == nullptr) {
+    if (HD == 128 && plan.splits == 1 && !(kp.mask_type == 1 && kp.mask != nullptr) && kp.vis_hi == nullptr) {
         static const int forced = [] {
             const char* e = std::getenv("ARC_SDPA_PREFILL_KERNEL");
             if (!e) return 0;
@@ -434,10 +467,11 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
             kp.mask_bits = bits;
             kp.mask_class = cls;
         }
+        const bool split = plan.splits > 1;
         kp.head_pair = ((p->nq / p->nkv) & 1) == 0;
         kp.cur_heads = kp.head_pair ? p->nq / 2 : p->nq;
         kp.q_tiles = kp.head_pair ? plan.q_tiles : (p->seq + 255) / 256;
-        const long long units = (long long)kp.q_tiles * kp.cur_heads * p->batch;
+        const long long units = wide_units(p, plan.q_tiles) * plan.splits;
         if (units > 0x3fffffffLL) return ARC_ERR_TOO_LARGE;
         kp.total_tiles = (int)units;
         // Under a causal mask (as most additive ones are, too) units differ in length — with a window only the first tiles are shorter, which matters
@@ -445,71 +479,43 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         // sequences together read would not stay in L2 (126 MB).  (1531 tokens, window 1024, 96 units on 74 pairs:
         // 36.5 -> 27 us.)
         const bool windowed = p->window > 0 && p->window < p->kv_len;
-        kp.long_first = p->mask_type != ARC_MASK_NONE && units > ds->wide_pairs && (!windowed || units < 8LL * ds->wide_pairs) &&
+        kp.long_first = !split && p->mask_type != ARC_MASK_NONE && units > ds->wide.pairs && (!windowed || units < 8LL * ds->wide.pairs) &&
                         (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;
         if ((rc = make_tile_map(&tk, p->k, HD, p->nkv, p->kv_len, p->batch, p->k_stride_t, p->k_stride_b, 64)) != ARC_OK) return rc;
-        if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
-        auto kernel = masked ? (kp.gate ? sdpa_prefill_wide_kernel<true, true> : sdpa_prefill_wide_kernel<false, true>)
-                             : (kp.gate ? sdpa_prefill_wide_kernel<true, false> : sdpa_prefill_wide_kernel<false, false>);
+        if (split) {
+            to = tg = tq;  // (not used)
+        } else if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) {
+            return rc;
+        }
+        // (a cluster is placed inside one GPC, so fewer fit than pairs / parts)
+        kp.fold = split && wide_units(p, plan.q_tiles) <= ds->wide.clusters(plan.splits);
+        auto kernel = split    ? sdpa_prefill_wide_kernel<false, false, true>
+                      : masked ? (kp.gate ? sdpa_prefill_wide_kernel<true, true> : sdpa_prefill_wide_kernel<false, true>)
+                               : (kp.gate ? sdpa_prefill_wide_kernel<true, false> : sdpa_prefill_wide_kernel<false, false>);
         ARC_CUDA(launch_dependent(kernel,
-                                  dim3((unsigned)(2 * (units < ds->wide_pairs ? units : ds->wide_pairs))), dim3(WideCfg::THREADS),
-                                  (size_t)WideCfg::SMEM_BYTES, stream, 2, tq, tk, tv, to, tg, kp));
+                                  dim3((unsigned)(2 * (split || units < ds->wide.pairs ? units : ds->wide.pairs))), dim3(WideCfg::THREADS),
+                                  (size_t)WideCfg::SMEM_BYTES, stream, kp.fold ? 2 * plan.splits : 2, tq, tk, tv, to, tg, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
-        return ARC_OK;
+        return split && !kp.fold ? launch_fold<HD>(p, plan, kp, stream) : ARC_OK;
     }
 
     kp.q_tiles = plan.q_tiles;
     kp.cur_heads = p->nq;
     kp.head_pair = 0;
-    if (plan.cluster > 0) {
-        // Few tiles: the key range of every tile is split over the CTAs of a thread-block cluster, which
-        // fold their accumulators through distributed shared memory — one launch, nothing in global memory
-        // but the result.  Clusters walk the tile list together.
-        const long long tiles = (long long)plan.q_tiles * p->nq * p->batch;
-        if (tiles > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
-        kp.total_tiles = (int)tiles;
-        kp.num_splits = 1;
-        const long long nclusters = tiles;  // the plan made sure that many are resident at once
-        ARC_CUDA(launch_dependent(sdpa_prefill_kernel<HD, false, false, true>, dim3((unsigned)(nclusters * plan.cluster)),
-                                  dim3(PrefillCfg<HD>::THREADS), (size_t)PrefillCfg<HD>::SMEM_BYTES, stream, plan.cluster, tq, tk, tv, kp));
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        return ARC_OK;
-    }
     // Persistent grid: one CTA per SM (fewer if there are fewer tiles), tiles dealt round-robin.
     const long long total_tiles = (long long)plan.q_tiles * p->nq * p->batch * plan.splits;
     if (total_tiles > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
     kp.total_tiles = (int)total_tiles;
     const unsigned ctas = (unsigned)(total_tiles < ds->sm_count ? total_tiles : ds->sm_count);
     // The additive-mask form is a kernel of its own: the common one stays small.
-    auto kernel = kp.mask_type == 1 && kp.mask != nullptr ? sdpa_prefill_kernel<HD, true, true, false>
-                  : kp.gate && plan.splits == 1           ? sdpa_prefill_kernel<HD, false, true, false>
-                                                          : sdpa_prefill_kernel<HD, false, false, false>;
+    void (*kernel)(CUtensorMap, CUtensorMap, CUtensorMap, PrefillParams) = sdpa_prefill_kernel<HD, true, true>;
+    if constexpr (HD == 128) {
+        if (!masked) kernel = kp.gate && plan.splits == 1 ? sdpa_prefill_kernel<HD, false, true> : sdpa_prefill_kernel<HD, false, false>;
+    }
     ARC_CUDA(launch_dependent(kernel, dim3(ctas), dim3(PrefillCfg<HD>::THREADS), (size_t)PrefillCfg<HD>::SMEM_BYTES, stream, 1, tq, tk, tv, kp));
     g_launches.fetch_add(1, std::memory_order_relaxed);
 
-    if (plan.splits > 1) {
-        UniformMergeParams mp{};
-        mp.part_o = kp.part_o;
-        mp.part_lse = kp.part_lse;
-        mp.gate = kp.gate;
-        mp.out = kp.out;
-        mp.out_f32 = nullptr;
-        mp.out_lse = p->out_lse;
-        mp.rows = plan.rows;
-        mp.num_parts = plan.splits;
-        mp.o_part_stride = plan.rows * HD;
-        mp.lse_part_stride = plan.rows;
-        mp.seq = p->seq;
-        mp.nq = p->nq;
-        mp.o_stride_b = p->o_stride_b;
-        mp.o_stride_t = p->o_stride_t;
-        mp.out_copies = kp.out_copies;
-        mp.n_copies = kp.n_copies;
-        ARC_CUDA(launch_dependent(sdpa_uniform_merge_kernel<HD>, dim3((unsigned)((plan.rows + UMERGE_ROWS - 1) / UMERGE_ROWS)),
-                                  dim3(32 * UMERGE_ROWS), 0, stream, 1, mp));
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-    }
-    return ARC_OK;
+    return plan.splits > 1 ? launch_fold<HD>(p, plan, kp, stream) : ARC_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -723,10 +729,9 @@ extern "C" const char* arc_sdpa_status_string(int status) {
 
 extern "C" size_t arc_sdpa_prefill_workspace_bytes(const arc_sdpa_prefill_params* p) {
     DeviceState* ds = nullptr;
-    int sm = 148;
-    if (device_state(&ds) == ARC_OK) sm = ds->sm_count;
+    const bool known = device_state(&ds) == ARC_OK;
     PrefillPlan plan;
-    if (plan_prefill(p, sm, ds ? ds->active_clusters[p && p->hd == 256 ? 1 : 0] : nullptr, &plan) != ARC_OK) return 0;
+    if (plan_prefill(p, known ? ds->sm_count : 148, known ? ds->wide : WideRoom{}, &plan) != ARC_OK) return 0;
     return plan.ws_bytes + plan.mask_bytes;
 }
 
@@ -739,7 +744,12 @@ extern "C" int arc_sdpa_prefill(const arc_sdpa_prefill_params* p, void* stream) 
     int rc = device_state(&ds);
     if (rc != ARC_OK) return rc;
     PrefillPlan plan;
-    if ((rc = plan_prefill(p, ds->sm_count, ds->active_clusters[p->hd == 256 ? 1 : 0], &plan)) != ARC_OK) return rc;
+    if ((rc = plan_prefill(p, ds->sm_count, ds->wide, &plan)) != ARC_OK) return rc;
+    if (p->hd == 256 && p->num_splits == 0 && plan.splits > 1 && (!p->workspace || p->workspace_bytes < plan.ws_bytes)) {
+        arc_sdpa_prefill_params whole = *p;  // no room for the parts of a split the caller has not asked for: none, then
+        whole.num_splits = 1;
+        if ((rc = plan_prefill(&whole, ds->sm_count, ds->wide, &plan)) != ARC_OK) return rc;
+    }
     if (!aligned16(p->q) || !aligned16(p->k) || !aligned16(p->v) || !aligned16(p->out) ||
         (p->gate && !aligned16(p->gate)))
         return ARC_ERR_ALIGNMENT;
@@ -878,7 +888,7 @@ extern "C" int arc_sdpa_merge(const float* part_out, const float* part_lse, int3
     if ((mp.o_part_stride & 3) != 0) return ARC_ERR_ALIGNMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned blocks = (unsigned)((rows + UMERGE_ROWS - 1) / UMERGE_ROWS);
-    ARC_CUDA(launch_dependent(hd == 128 ? sdpa_uniform_merge_kernel<128> : sdpa_uniform_merge_kernel<256>, dim3(blocks),
+    ARC_CUDA(launch_dependent(hd == 128 ? sdpa_uniform_merge_kernel<128, 4> : sdpa_uniform_merge_kernel<256, 4>, dim3(blocks),
                               dim3(32 * UMERGE_ROWS), 0, st, 1, mp));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return ARC_OK;

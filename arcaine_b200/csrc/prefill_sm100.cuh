@@ -1,6 +1,6 @@
-// GQA flash-attention prefill / canvas kernel for sm_100a, one query tile at a time per CTA: the
-// kernel for head dim 256, additive masks, key-range splits and small problems (head dim 128
-// with enough tiles runs two tiles per CTA, prefill_pair_sm100.cuh).
+// GQA flash-attention prefill kernel for sm_100a, one query tile at a time per CTA: the kernel for small problems, split
+// key ranges, additive masks and vision blocks of head dim 128 (with enough tiles prefill_pair_sm100.cuh runs two per
+// CTA), and at head dim 256 for additive masks without a workspace (prefill_wide_sm100.cuh does the rest).
 //
 // One CTA owns a tile of 128 query tokens of one query head and walks the key
 // blocks (128 keys) that tile can see.  Q, K and V tiles are staged in shared
@@ -61,6 +61,7 @@ struct PrefillParams {
     const uint32_t* mask_class;  // [row tile][key block]: a byte per 32 rows, MASK_* bits
     const uint4* mask_bits;      // [row tile][key block][row]: one bit per key, set where the mask is 0
     int mask_blocks;
+    int fold;        // prefill_wide_sm100.cuh: the parts of a unit are the pairs of one cluster, which folds them itself
     const int* ids;  // prefill_wide_sm100.cuh: vision-block ids, ids[j] that of key j (instead of vis_hi)
 };
 
@@ -90,8 +91,8 @@ struct PrefillCfg {
     static constexpr int NSB = (HD == 128) ? 3 : 2;  // score buffers: S = Q K^T runs NSB-1 blocks ahead of the softmax
     static constexpr int COL_S = 0;                  // NSB buffers of 128 fp32 columns; P (bf16) is written over them
     static constexpr int COL_O = NSB * 128;          // HD fp32 columns
-    static constexpr int NUM_BARS = 2 + 2 * K_STAGES + 2 * V_STAGES + 2 * NSB + 2 + 2 + 2;  // the last two: cluster merge
-    static constexpr int XCH_FLOATS = 2 * 2 * 128 + 2 * 128 + 2 * 128;  // row-max exchange (2 phases), row-sum exchange, (max, sum) per row for the cluster merge
+    static constexpr int NUM_BARS = 2 + 2 * K_STAGES + 2 * V_STAGES + 2 * NSB + 2 + 2;
+    static constexpr int XCH_FLOATS = 2 * 2 * 128 + 2 * 128;  // row-max exchange (2 phases), row-sum exchange
     static constexpr int SMEM_BYTES = (1 + K_STAGES + V_STAGES) * TILE_BYTES + NUM_BARS * 8 + 16 + XCH_FLOATS * 4 + 1024;
     static constexpr int SOFTMAX_WARPS = 8;
     static constexpr int THREADS = 32 * (SOFTMAX_WARPS + 2);
@@ -258,9 +259,6 @@ __device__ __forceinline__ void pair_sync(int quarter) {
     asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
 }
 
-// All eight softmax warps (named barrier 5; barriers 1-4 belong to pair_sync).
-__device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 5, 256;" ::: "memory"); }
-
 // One unit of work of the persistent kernel.
 struct TileWork {
     int q0, h, b, split, kvh;
@@ -274,11 +272,9 @@ struct TileWork {
 struct TileCursor {
     int w, qt, h, z;
     int dqt, dh, dz, step;
-    __device__ __forceinline__ void init(const PrefillParams& p) { init(p, blockIdx.x, gridDim.x); }
-    // first tile and stride given explicitly (a cluster of CTAs walks the list together)
-    __device__ __forceinline__ void init(const PrefillParams& p, int first, int step_) {
-        w = first;
-        step = step_;
+    __device__ __forceinline__ void init(const PrefillParams& p) {
+        w = blockIdx.x;
+        step = gridDim.x;
         if (p.tail_base >= 0) {  // (the grid holds one CTA per tile: the strides below are never used)
             const int idx = p.tail_base + (w >> 1);
             qt = idx % p.q_tiles;
@@ -309,24 +305,18 @@ struct TileCursor {
     }
 };
 
-// nsplit > 0: the key range is split over the CTAs of a cluster (split = the CTA's rank) and the
-// tile list holds whole tiles; else the split is part of the tile index (z = batch * num_splits + split).
+// The split is part of the tile index (z = batch * num_splits + split).
 template <int HD>
-__device__ __forceinline__ TileWork decode_tile(const PrefillParams& p, const TileCursor& cur, int nsplit = 0, int split = 0) {
+__device__ __forceinline__ TileWork decode_tile(const PrefillParams& p, const TileCursor& cur) {
     using C = PrefillCfg<HD>;
     TileWork t;
     t.h = cur.h;
-    if (nsplit > 0) {
-        t.b = cur.z;
-        t.split = split;
-    } else if (p.num_splits == 1) {
+    if (p.num_splits == 1) {
         t.b = cur.z;
         t.split = 0;
-        nsplit = 1;
     } else {
         t.b = cur.z / p.num_splits;
         t.split = cur.z % p.num_splits;
-        nsplit = p.num_splits;
     }
     t.kvh = p.group_shift >= 0 ? (t.h >> p.group_shift) : t.h / p.group;
     t.q0 = cur.qt * C::BM;
@@ -342,7 +332,7 @@ __device__ __forceinline__ TileWork decode_tile(const PrefillParams& p, const Ti
         if (windowed) blk_lo = max(0, t.q0 + off - p.window + 1) / C::BN;
     }
     const int nblk = max(0, blk_hi - blk_lo);
-    const int per = (nblk + nsplit - 1) / nsplit;
+    const int per = p.num_splits == 1 ? nblk : (nblk + p.num_splits - 1) / p.num_splits;
     t.my_lo = blk_lo + t.split * per;
     t.n_my = max(0, min(blk_hi, t.my_lo + per) - t.my_lo);
     return t;
@@ -350,12 +340,7 @@ __device__ __forceinline__ TileWork decode_tile(const PrefillParams& p, const Ti
 
 // ADD_MASK and GATE select code that most calls do not need (an additive mask row per query, the
 // sigmoid-gated epilogue); the common instance carries neither and stays small.
-// CLUSTER: the kernel is launched in thread-block clusters; the CTAs of a cluster share a tile and
-// split its key range, then fold their accumulators through distributed shared memory — each CTA
-// writes its unnormalised O and (max, sum) per row into its own shared memory (the K / V buffers are
-// free by then), and merges a share of the rows reading all of them.  One launch, no partial records
-// in global memory, no merge kernel.
-template <int HD, bool ADD_MASK, bool GATE, bool CLUSTER = false>
+template <int HD, bool ADD_MASK, bool GATE>
 __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     sdpa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                         const __grid_constant__ CUtensorMap tm_v, const PrefillParams p) {
@@ -384,18 +369,11 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     uint64_t* pv_done = p_full + NSB;
     uint64_t* o_full = pv_done + 2;     // one phase per tile: the tile's last O += P V has completed
     uint64_t* o_empty = o_full + 1;     // one phase per tile: the softmax warps have read O out
-    uint64_t* part_ready = o_empty + 1;  // cluster merge, one phase per tile: every CTA's share of the tile is in its shared memory
-    uint64_t* read_done = part_ready + 1; // cluster merge, one phase per tile: every CTA has finished reading this CTA's share
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
     float* xch_max = reinterpret_cast<float*>(tmem_slot + 4);  // [phase 2][key half 2][row 128]
     float* xch_sum = xch_max + 2 * 2 * 128;                    // [key half 2][row 128]
-    float2* cl_stat = reinterpret_cast<float2*>(xch_sum + 2 * 128);  // [row 128] (max, sum) of this CTA's key range
-    const int csize = CLUSTER ? (int)cluster_nctarank() : 1;
-    const int crank = CLUSTER ? (int)cluster_ctarank() : 0;
-    const int cfirst = CLUSTER ? (int)(blockIdx.x / csize) : (int)blockIdx.x;  // this CTA's (cluster's) first tile
-    const int cstep = CLUSTER ? (int)(gridDim.x / csize) : (int)gridDim.x;
-    auto tile_of = [&](const TileCursor& c) { return CLUSTER ? decode_tile<HD>(p, c, csize, crank) : decode_tile<HD>(p, c); };
+
 
     // (broadcast, so that the compiler knows them to be the same in every lane and keeps what follows from them —
     // MMA descriptors above all — in uniform registers)
@@ -427,8 +405,6 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         mbar_init(&pv_done[1], 1);
         mbar_init(o_full, 1);
         mbar_init(o_empty, 32 * C::SOFTMAX_WARPS);
-        mbar_init(part_ready, csize);  // one arrival per CTA of the cluster
-        mbar_init(read_done, csize);
         fence_mbar_init();
     }
     if (warp == PRODUCER_WARP) {
@@ -441,6 +417,9 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
     }
+    // (the divisions, ahead of the wait: they took 1000 clk between the kernel's release and its first load)
+    TileCursor cursor;
+    cursor.init(p);
     // Up to here nothing depends on the kernels in front; everything below may.  (The tail of a two-tile launch runs
     // beside that launch, which let it start only when the kernels before it had completed.)
     if (p.tail_base < 0) grid_dependency_wait();
@@ -449,30 +428,20 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    if constexpr (CLUSTER) cluster_sync_all();  // every CTA's barriers exist before anyone arrives on them
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
     // A call that finds a status word set does no work: every role walks an empty tile list and meets
-    // the others at the end (in a cluster nobody may leave early anyway).
+    // the others at the end.
     const int total_tiles = *abort_slot ? 0 : p.total_tiles;
 
     if (warp == PRODUCER_WARP) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
             int gk = 0, gv = 0, tc = 0;  // K blocks, V blocks and non-empty tiles loaded so far
-            int tn = 0;                  // tiles seen (cluster merge: one phase of read_done each)
             bool ok = true;
-            TileCursor cur;
-            for (cur.init(p, cfirst, cstep); ok && cur.w < total_tiles; cur.advance(p), ++tn) {
-                const TileWork tw = tile_of(cur);
+            TileCursor cur = cursor;
+            for (; ok && cur.w < total_tiles; cur.advance(p)) {
+                const TileWork tw = decode_tile<HD>(p, cur);
                 if (tw.n_my == 0) continue;
-                if constexpr (CLUSTER) {
-                    // the K / V buffers held this CTA's share of the previous tile: wait until the whole
-                    // cluster has read it
-                    if (tn > 0 && !mbar_wait_cluster(read_done, (tn - 1) & 1)) {
-                        report_fault(p.fault, FAULT_WAIT_EMPTY, 0x400u);
-                        break;
-                    }
-                }
                 if (tc > 0 && !mbar_wait(q_empty, (tc - 1) & 1)) {
                     report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u);
                     break;
@@ -552,9 +521,9 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
                 return true;
             };
             bool ok = true;
-            TileCursor cur;
-            for (cur.init(p, cfirst, cstep); ok && cur.w < total_tiles; cur.advance(p)) {
-                const TileWork tw = tile_of(cur);
+            TileCursor cur = cursor;
+            for (; ok && cur.w < total_tiles; cur.advance(p)) {
+                const TileWork tw = decode_tile<HD>(p, cur);
                 if (tw.n_my == 0) continue;
                 if (!mbar_wait_inline(q_full, tc & 1)) {
                     report_fault(p.fault, FAULT_WAIT_Q, tc);
@@ -618,171 +587,14 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         constexpr bool has_mask = ADD_MASK;  // the additive-mask form is a kernel of its own: the common one stays small
 
         int gb = 0, tc = 0;  // key blocks and non-empty tiles processed so far
-        int tn = 0;          // tiles seen (cluster merge: one phase of part_ready / read_done each)
         bool ok = true;
         uint32_t va[32], vb[32];  // this thread's 64 scores of the current block
 
-        // Cluster merge at the end of a tile.  has_blocks: this CTA's key range of the tile is not empty
-        // (m, l_share are then its row maximum and this thread's share of the row sum).
-        //
-        // Every CTA writes its unnormalised accumulator and (max, sum) per row into its own shared memory,
-        // tells the cluster with one arrival per CTA, and folds rows [crank * 128 / CS, +128 / CS): a warp
-        // takes an eighth of them, a lane 4 consecutive columns (twice for head dim 256) of every CTA's
-        // share.  A lane's 16 (32) remote 16-byte loads are issued eight at a time before any is used — the
-        // fold is bound by the latency of distributed shared memory, not by arithmetic.
-        auto fold_rows = [&](const TileWork& tw, auto cs_tag) {
-            constexpr int CS = decltype(cs_tag)::value;
-            constexpr int WROWS = 128 / CS / C::SOFTMAX_WARPS;  // rows per warp
-            constexpr int PIECES = HD / 128;                    // 16-byte pieces of a row per lane
-            constexpr int ITEMS = WROWS * PIECES;               // (row, piece) items per lane
-            constexpr int IB = CS >= 8 ? 1 : 8 / CS;            // items per batch: eight 16-byte loads in flight
-            float* opart = reinterpret_cast<float*>(sK);
-            const int row0 = crank * (128 / CS) + warp * WROWS;
-            uint2 gv[IB];
-            auto load_gates = [&](int it0) {
-                if (!p.gate) return;
-#pragma unroll
-                for (int b = 0; b < IB; ++b) {
-                    const int i = (it0 + b) / PIECES, j = (it0 + b) % PIECES;
-                    const int tt = tw.q0 + row0 + i;
-                    const long long eoff = tw.b * p.o_stride_b + tt * p.o_stride_t + (long long)tw.h * HD;
-                    gv[b] = tt < p.seq ? *reinterpret_cast<const uint2*>(p.gate + eoff + (lane + 32 * j) * 4) : make_uint2(0u, 0u);
-                }
-            };
-            // The gate values of the first batch depend on nothing here: request them before waiting for
-            // the cluster (those of a later batch go out together with its loads).
-            load_gates(0);
-            if (!__all_sync(0xffffffffu, mbar_wait_cluster(part_ready, tn & 1))) {
-                report_fault(p.fault, FAULT_WAIT_FULL, 0x700u);
-                ok = false;
-            }
-            if (!ok) return;
-            const uint32_t st_base = smem_u32(cl_stat), op_base = smem_u32(opart);
-#pragma unroll 1
-            for (int it0 = 0; it0 < ITEMS; it0 += IB) {
-                float4 o[IB][CS];
-                float2 st[IB][CS];
-                if (it0 > 0) load_gates(it0);
-#pragma unroll
-                for (int b = 0; b < IB; ++b) {
-                    const int i = (it0 + b) / PIECES, j = (it0 + b) % PIECES;
-                    const int rr = row0 + i;
-                    const uint32_t off = (uint32_t)(rr * HD + (((lane + 32 * j) ^ (rr & 7)) << 2)) * 4u;
-#pragma unroll
-                    for (int c = 0; c < CS; ++c) {
-                        st[b][c] = ld_cluster_f32x2(map_to_cta(st_base + rr * 8, c));
-                        o[b][c] = ld_cluster_f32x4(map_to_cta(op_base + off, c));
-                    }
-                }
-#pragma unroll
-                for (int b = 0; b < IB; ++b) {
-                    const int i = (it0 + b) / PIECES, j = (it0 + b) % PIECES;
-                    const int rr = row0 + i;
-                    float mx = -CUDART_INF_F, ltot = 0.f;
-                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (int c = 0; c < CS; ++c) mx = fmaxf(mx, st[b][c].x);
-#pragma unroll
-                    for (int c = 0; c < CS; ++c) {
-                        // a CTA without key blocks wrote no rows: whatever was read from it is not used
-                        const float w = st[b][c].x != -CUDART_INF_F ? fast_exp2(st[b][c].x - mx) : 0.f;
-                        ltot = fmaf(w, st[b][c].y, ltot);
-                        if (w != 0.f) {
-                            acc.x = fmaf(w, o[b][c].x, acc.x);
-                            acc.y = fmaf(w, o[b][c].y, acc.y);
-                            acc.z = fmaf(w, o[b][c].z, acc.z);
-                            acc.w = fmaf(w, o[b][c].w, acc.w);
-                        }
-                    }
-                    const float inv = ltot > 0.f ? 1.0f / ltot : 0.f;
-                    const int tt = tw.q0 + rr;
-                    if (tt >= p.seq) continue;
-                    const long long eoff = tw.b * p.o_stride_b + tt * p.o_stride_t + (long long)tw.h * HD;
-                    float o4[4] = {acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv};
-                    if (p.gate) {
-                        o4[0] = sigmoid_gate_bits(o4[0], (uint16_t)(gv[b].x & 0xffffu));
-                        o4[1] = sigmoid_gate_bits(o4[1], (uint16_t)(gv[b].x >> 16));
-                        o4[2] = sigmoid_gate_bits(o4[2], (uint16_t)(gv[b].y & 0xffffu));
-                        o4[3] = sigmoid_gate_bits(o4[3], (uint16_t)(gv[b].y >> 16));
-                    }
-                    const uint2 packed = make_uint2(pack_bf16x2(o4[0], o4[1]), pack_bf16x2(o4[2], o4[3]));
-                    *reinterpret_cast<uint2*>(p.out + eoff + (lane + 32 * j) * 4) = packed;
-                    for (int c = 0; c < p.n_copies; ++c)
-                        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.out_copies[c]) + eoff + (lane + 32 * j) * 4) = packed;
-                    if (j == 0 && lane == 0 && p.out_lse)
-                        p.out_lse[((long long)tw.b * p.seq + tt) * p.nq + tw.h] =
-                            ltot > 0.f ? (mx + fast_log2(ltot)) * 0.6931471805599453f : -CUDART_INF_F;
-                }
-            }
-        };
-        auto cluster_tile_end = [&](const TileWork& tw, float m, float l_share, bool has_blocks) {
-            float* opart = reinterpret_cast<float*>(sK);  // [128 rows][HD] fp32, 16-byte pieces swizzled by row & 7
-            float l = 0.f;
-            // the previous tile's share (rows and statistics) must have been read by the whole cluster before
-            // this one overwrites it
-            if (tn > 0 && !__all_sync(0xffffffffu, mbar_wait_cluster(read_done, (tn - 1) & 1))) {
-                report_fault(p.fault, FAULT_WAIT_EMPTY, 0x500u);
-                ok = false;
-            }
-            if (has_blocks) {
-                xch_sum[kh * 128 + r] = l_share;
-                pair_sync(quarter);
-                l = xch_sum[r] + xch_sum[128 + r];
-                if (ok && !mbar_wait_warp(o_full, tc & 1)) {
-                    report_fault(p.fault, FAULT_WAIT_O, tc);
-                    ok = false;
-                }
-                ++tc;
-                if (ok) {
-                    tc_fence_after_sync();
-                    // this thread's half of the row, unnormalised, into this CTA's shared memory (every MMA
-                    // that read the K / V buffers has completed: o_full follows them)
-#pragma unroll 1
-                    for (int c = 0; c < OC / 32; c += 2) {
-                        tmem_ld32(tO + c * 32, va);
-                        tmem_ld32(tO + c * 32 + 32, vb);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int e = 0; e < 64; e += 4) {
-                            const uint32_t* src = e < 32 ? va + e : vb + (e - 32);
-                            const int piece = (kh * OC + c * 32 + e) >> 2;
-                            *reinterpret_cast<float4*>(opart + r * HD + ((piece ^ (r & 7)) << 2)) =
-                                make_float4(__uint_as_float(src[0]), __uint_as_float(src[1]), __uint_as_float(src[2]),
-                                            __uint_as_float(src[3]));
-                        }
-                    }
-                    tc_fence_before_sync();
-                    mbar_arrive(o_empty);  // the accumulator is out: the next tile may overwrite it
-                }
-            }
-            if (kh == 0) cl_stat[r] = make_float2(has_blocks ? m : -CUDART_INF_F, l);
-            // my CTA's share is written once all 256 softmax threads are here: one thread tells every CTA of
-            // the cluster (release at cluster scope, cumulative over what the barrier ordered before it)
-            const uint32_t pr = smem_u32(part_ready), rd = smem_u32(read_done);
-            softmax_sync();
-            if (threadIdx.x == 0) {
-                fence_acq_rel_cluster();
-                for (int c = 0; c < csize; ++c) mbar_arrive_cluster(map_to_cta(pr, c));
-            }
-            if (csize == 2) fold_rows(tw, std::integral_constant<int, 2>{});  // the host launches clusters of 2 or 4
-            else fold_rows(tw, std::integral_constant<int, 4>{});
-            // every softmax thread of this CTA is done reading the cluster's shared memory
-            softmax_sync();
-            if (threadIdx.x == 0) {
-                for (int c = 0; c < csize; ++c) mbar_arrive_cluster(map_to_cta(rd, c));
-            }
-            ++tn;
-        };
-
-        TileCursor cur;
-        for (cur.init(p, cfirst, cstep); cur.w < total_tiles; cur.advance(p)) {
-            const TileWork tw = tile_of(cur);
+        TileCursor cur = cursor;
+        for (; cur.w < total_tiles; cur.advance(p)) {
+            const TileWork tw = decode_tile<HD>(p, cur);
             const int t = tw.q0 + r;
             const long long row = ((long long)tw.b * p.seq + t) * p.nq + tw.h;
-            if (CLUSTER && tw.n_my == 0) {
-                cluster_tile_end(tw, -CUDART_INF_F, 0.f, false);  // the other CTAs of the cluster may have key blocks
-                continue;
-            }
             if (tw.n_my == 0) {
                 // Nothing visible: zero output (or an empty partial) for this tile.
                 if (t < p.seq) {
@@ -995,11 +807,6 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
                 }
             }
             gb += tw.n_my;
-            if constexpr (CLUSTER) {
-                cluster_tile_end(tw, m, l, true);
-                continue;
-            }
-
             // Row sum = the two threads' shares.
             xch_sum[kh * 128 + r] = l;
             pair_sync(quarter);
@@ -1085,9 +892,6 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     // grid only, so this grid does not complete before the one in front of it has: every CTA ends on the
     // grid-dependency wait (a no-op for launches without the attribute).
     if (p.tail_base >= 0) grid_dependency_wait();
-    // A CTA's shared memory may be read by the others only while it is alive: nobody leaves before the
-    // whole cluster is through (all threads are still running here).
-    if constexpr (CLUSTER) cluster_sync_all();
 }
 
 }  // namespace arc

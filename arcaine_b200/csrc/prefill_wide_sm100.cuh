@@ -19,6 +19,7 @@
 //
 // Masks, lazy rescaling, P over the scores, bounded waits and the status word are as in prefill_pair_sm100.cuh.
 #pragma once
+#include "decode_sm100.cuh"
 #include "prefill_pair_sm100.cuh"
 
 namespace arc {
@@ -38,8 +39,9 @@ struct WideCfg {
     static constexpr int COL_O = 256;
     // q_full q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp][2]
     static constexpr int NUM_BARS = 2 + 8 + 2 + 4 + 2 + 4 + 8;
-    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4;
+    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4 + 32;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
+    static constexpr int MOST_FOLDED = 3;  // parts of a split unit that fold themselves as one cluster
     static constexpr int EPILOGUE_WARP = 4, PRODUCER_WARP = 8, ISSUER_WARP = 9;
     static constexpr int THREADS = 320;
 };
@@ -47,6 +49,7 @@ struct WideCfg {
 // One unit of the pair: this CTA's tile, and the key blocks [lo, hi) the pair walks (the union over both tiles).
 struct WideWork {
     int q0, h, b, kvh, lo, hi;
+    int part;  // SPLIT: which part of the key range
 };
 
 // ---------------------------------------------------------------------------
@@ -205,37 +208,56 @@ struct WideCursor {
     }
 };
 
-template <bool MASKED>
-__device__ __forceinline__ WideWork decode_wide(const PrefillParams& p, const WideCursor& cur, int rank) {
+// The unit at the cursor, without its key blocks: nothing here depends on memory.
+template <bool SPLIT>
+__device__ __forceinline__ WideWork wide_place(const PrefillParams& p, const WideCursor& cur, int rank) {
     WideWork t;
     int qt;
-    if (p.long_first) {
+    t.part = SPLIT ? cur.w % p.num_splits : 0;
+    if (!SPLIT && p.long_first) {
         const int per = p.cur_heads * p.batch, rest = cur.w % per;
         qt = p.q_tiles - 1 - cur.w / per;
         t.h = rest % p.cur_heads;
         t.b = rest / p.cur_heads;
     } else {
-        const int rest = cur.w / p.q_tiles;
-        qt = cur.w % p.q_tiles;
+        const int w = SPLIT ? cur.w / p.num_splits : cur.w;
+        const int rest = w / p.q_tiles;
+        qt = w % p.q_tiles;
         t.h = rest % p.cur_heads;
         t.b = rest / p.cur_heads;
     }
-    const int rows = p.head_pair ? WideCfg::BM : 2 * WideCfg::BM;  // tokens of the unit
-    const int q0 = qt * rows;
-    if constexpr (MASKED) masked_blocks(p, q0 >> 7, min(q0 + rows, p.seq + 127) >> 7, t.lo, t.hi);
-    else wide_blocks(p, q0, q0 + rows - 1, t.lo, t.hi);
     if (p.head_pair) {
         t.h = t.h * 2 + rank;
-        t.q0 = q0;
+        t.q0 = qt * WideCfg::BM;
     } else {
-        t.q0 = q0 + rank * WideCfg::BM;
+        t.q0 = (qt * 2 + rank) * WideCfg::BM;
     }
     t.kvh = p.group_shift >= 0 ? (t.h >> p.group_shift) : t.h / p.group;
     return t;
 }
 
+template <bool MASKED, bool SPLIT>
+__device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int rank, WideWork& t) {
+    const int rows = p.head_pair ? WideCfg::BM : 2 * WideCfg::BM;  // tokens of the unit
+    const int q0 = p.head_pair ? t.q0 : t.q0 - rank * WideCfg::BM;
+    if constexpr (MASKED) masked_blocks(p, q0 >> 7, min(q0 + rows, p.seq + 127) >> 7, t.lo, t.hi);
+    else wide_blocks(p, q0, q0 + rows - 1, t.lo, t.hi);
+    if (SPLIT) {
+        const int lo = t.lo, n = t.hi - t.lo;
+        t.lo = lo + n * t.part / p.num_splits;
+        t.hi = lo + n * (t.part + 1) / p.num_splits;
+    }
+}
+
 // MASKED: with an additive mask, as mask_scan_kernel has read it.
-template <bool GATE, bool MASKED>
+// SPLIT: a unit is one of num_splits parts of the key blocks, one unit per pair, for calls whose tiles would leave most
+// pairs idle.  The part's normalised rows go to the partial records as f32 with their log-sum-exp.  Two or three parts
+// are the pairs of one cluster (p.fold): each CTA stores only the rows the other parts' CTAs fold, and after a cluster
+// barrier folds its own share of rows; more parts are folded by sdpa_uniform_merge_kernel.  The rows pass through L2:
+// read out of the other CTAs' shared memory, 11 bytes per clk and SM, the fold took 5 us.  Every instruction here runs
+// once per launch and is fetched cold, 50 clk per 128 bytes of code, so the loops are rolled: with five rows unrolled
+// the fold itself took 8700 clk.
+template <bool GATE, bool MASKED, bool SPLIT = false>
 __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     sdpa_prefill_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
@@ -267,10 +289,12 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
     float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [unit & 3][row] row sum
+    WideWork* first_unit = reinterpret_cast<WideWork*>(fin_vals + 4 * 128);
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
-    const int rank = (int)cluster_ctarank();
+    const int cta = SPLIT ? (int)cluster_ctarank() : 0;                   // in the cluster, which may hold several pairs
+    const int lead = cta & ~1, rank = SPLIT ? cta & 1 : (int)cluster_ctarank();  // the pair's leader; rank in the pair
     const bool leader = rank == 0;
 
     if (threadIdx.x == 32) {
@@ -300,21 +324,83 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         fence_mbar_init();
     }
     if (warp == C::PRODUCER_WARP) tmem_alloc_pair(tmem_slot, 512);
+    // One warp finds the first unit for all; its divisions, and the code that every role would fetch for them, took 2500 clk
+    // between the kernel's release and its first load.
+    const int first = (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
+    const bool blocks_in_memory = MASKED || p.ids;
+    WideWork w_first{};
+    if (warp == C::EPILOGUE_WARP) {
+        w_first = wide_place<SPLIT>(p, WideCursor(first, step), rank);
+        if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
+    }
+    cluster_sync_all();  // both CTAs' barriers exist before anyone arrives on the other's
     // Up to here nothing depends on the kernels in front; everything below may.
     grid_dependency_wait();
     grid_launch_dependents();
     if (threadIdx.x == 0) *abort_slot = *reinterpret_cast<volatile uint32_t*>(p.fault) != 0u ? 1u : 0u;
+    if (warp == C::EPILOGUE_WARP) {
+        if (blocks_in_memory) wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
+        if (lane == 0) *first_unit = w_first;
+    }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    cluster_sync_all();  // both CTAs' barriers exist before anyone arrives on the other's
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
     const int total = *abort_slot ? 0 : p.total_tiles;  // a status is set: walk an empty list
-    const int first = (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
+    auto unit_at = [&](const WideCursor& cur) {
+        if (SPLIT || cur.i == 0) return *first_unit;
+        WideWork w = wide_place<SPLIT>(p, cur, rank);
+        wide_find_blocks<MASKED, SPLIT>(p, rank, w);
+        return w;
+    };
+
+    // SPLIT: columns [col, col + 128) of the part's rows into shared memory, where Q, K and V are through: the f32 tile as
+    // [32 columns][row], 128-byte swizzle; and from there, a row of 512 bytes an instruction, to the records.  (By TMA, in
+    // boxes of 8 rows x 32 columns, the tile took 4000 clk.)
+    constexpr int PART_CHUNK = 128 * 128;
+    float* const part_lse = SPLIT ? p.part_lse + (long long)(blockIdx.x / 2 % p.num_splits) * p.batch * p.seq * p.nq : nullptr;
+    auto own_row0 = [&](int part) { return (part * 16 + p.num_splits - 1) / p.num_splits * 8; };  // rows a part's CTA folds
+    auto store_part = [&](const WideWork& w, int quarter, float row_l, int col) {
+        if (!mbar_wait_warp<2>(o_full, 0)) {
+            if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x700u);
+            return;
+        }
+        tc_fence_after_sync();
+        const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
+        const uint32_t tO = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::COL_O + col;
+        const uint32_t tile = smem_u32(smem) + col / 32 * PART_CHUNK, at = tile + (quarter * 32 + lane) * 128;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+            uint32_t v[32];
+            tmem_ld32(tO + c * 32, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + c * PART_CHUNK + ((i ^ (lane & 7)) << 4)),
+                             "f"(__uint_as_float(v[4 * i]) * inv), "f"(__uint_as_float(v[4 * i + 1]) * inv),
+                             "f"(__uint_as_float(v[4 * i + 2]) * inv), "f"(__uint_as_float(v[4 * i + 3]) * inv) : "memory");
+        }
+        __syncwarp();
+        const int keep0 = p.fold ? own_row0(w.part) : 128, keep1 = p.fold ? own_row0(w.part + 1) : 128;
+        const int end = min(quarter * 32 + 32, p.seq - w.q0);
+        const long long step_t = (long long)p.nq * HD;
+        float* dst = p.part_o + ((((long long)w.part * p.batch + w.b) * p.seq + w.q0) * p.nq + w.h) * HD + col + lane * 4;
+#pragma unroll 1
+        for (int i0 = quarter * 32; i0 < end; i0 += 8) {  // (shares begin at multiples of eight rows)
+            if (i0 >= keep0 && i0 < keep1) continue;
+            float4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                v[i] = *reinterpret_cast<const float4*>(smem + (col / 32 + (lane >> 3)) * PART_CHUNK + (i0 + i) * 128 + (((lane & 7) ^ i) << 4));
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i0 + i < end) *reinterpret_cast<float4*>(dst + (i0 + i) * step_t) = v[i];
+        }
+    };
 
     if (warp == C::PRODUCER_WARP) {
         // ------------------------------------------------------------------ TMA producer
-        const uint32_t bq = map_to_cta(smem_u32(q_full), 0), bk = map_to_cta(smem_u32(k_full), 0), bv = map_to_cta(smem_u32(v_full), 0);
+        const uint32_t bq = map_to_cta(smem_u32(q_full), lead), bk = map_to_cta(smem_u32(k_full), lead), bv = map_to_cta(smem_u32(v_full), lead);
         int gk = 0, gv = 0, n = 0;  // K blocks, V blocks and units loaded so far
         bool ok = true;
         auto load_k = [&](const WideWork& w, int j) {
@@ -347,7 +433,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         };
         WideCursor cur(first, step);
         for (; ok && cur.w < total; cur.advance(p)) {
-            const WideWork w = decode_wide<MASKED>(p, cur, rank);
+            const WideWork w = unit_at(cur);
             if (w.hi == w.lo) continue;
             if (n > 0 && !mbar_wait_inline(q_empty, (n - 1) & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u);
@@ -395,16 +481,16 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c, da += C::Q_CHUNK >> 4, db += C::K_CHUNK >> 4, acc = 1u)
                     umma_pair_ss_x4<2, 2>(tmem_base + C::COL_S + st * 128, da, db, IDESC_QK, acc);
-                umma_commit_pair(&s_full[st]);
-                umma_commit_pair(&k_empty[st]);
-                if (j + 1 == w.hi) umma_commit_pair(q_empty);
+                umma_commit_pair(&s_full[st], lead);
+                umma_commit_pair(&k_empty[st], lead);
+                if (j + 1 == w.hi) umma_commit_pair(q_empty, lead);
                 ++gs;
                 return true;
             };
             WideCursor cur(first, step);
             auto next_unit = [&](WideWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
                 for (; cur.w < total; cur.advance(p)) {
-                    w = decode_wide<MASKED>(p, cur, 0);
+                    w = unit_at(cur);
                     if (w.hi > w.lo) {
                         cur.advance(p);
                         return true;
@@ -452,8 +538,8 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                         umma_pair_ts_x4<8, 128>(tmem_base + C::COL_O, tP, dv, IDESC_PV, acc);
                     }
                     if (!ok) break;
-                    if (j + 1 == w.hi) umma_commit_pair(o_full);
-                    umma_commit_pair(&v_empty[st]);
+                    if (j + 1 == w.hi) umma_commit_pair(o_full, lead);
+                    umma_commit_pair(&v_empty[st], lead);
                     ++gp;
                 }
                 w = wn;
@@ -465,18 +551,20 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;
         const uint32_t tO = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::COL_O;
-        const uint32_t b_empty = map_to_cta(smem_u32(o_empty), 0);
+        const uint32_t b_empty = map_to_cta(smem_u32(o_empty), lead);
         int n = 0;  // units with key blocks so far
         OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0};
         WideCursor cur(first, step);
         for (; cur.w < total; cur.advance(p)) {
-            const WideWork w = decode_wide<MASKED>(p, cur, rank);
+            const WideWork w = unit_at(cur);
             const int t0 = w.q0 + quarter * 32, t = t0 + lane;
             const bool store = t < p.seq, warp_store = t0 < p.seq;  // this row / some row of the warp is stored
             const long long row = ((long long)w.b * p.seq + t) * p.nq + w.h;
             const long long eoff = w.b * p.o_stride_b + t * p.o_stride_t + (long long)w.h * HD;
             if (w.hi == w.lo) {  // nothing visible for the pair: zero output
-                if (store) {
+                if (SPLIT) {
+                    if (store) part_lse[row] = -CUDART_INF_F;
+                } else if (store) {
                     for (int c = -1; c < p.n_copies; ++c) {
                         uint4* dst = reinterpret_cast<uint4*>((c < 0 ? p.out : reinterpret_cast<uint16_t*>(p.out_copies[c])) + eoff);
                         for (int i = 0; i < HD / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -485,12 +573,16 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 }
                 continue;
             }
-            if (warp_store) stage_open<GATE, HD>(stage, &tm_gate, lane, w.h, t0, w.b);
+            if (!SPLIT && warp_store) stage_open<GATE, HD>(stage, &tm_gate, lane, w.h, t0, w.b);
             if (!mbar_wait_warp<2>(&fin[n & 3], (n >> 2) & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x500u);
                 break;
             }
             const float row_l = fin_vals[(n & 3) * 128 + r];
+            if constexpr (SPLIT) {
+                store_part(w, quarter, row_l, 0);
+                break;
+            }
             if (!mbar_wait_warp<2>(o_full, n & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, n);
                 break;
@@ -531,14 +623,14 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             }
             if (!ok) break;
         }
-        if (lane == 0) bulk_wait_read<0>();  // the stage may go when its last rows have been read
+        if (!SPLIT && lane == 0) bulk_wait_read<0>();  // the stage may go when its last rows have been read
     } else {
         // ------------------------------------------------------------------ softmax: thread = query row
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;
         const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
         const uint32_t tO = tmem_base + lane_sel + C::COL_O;
-        const uint32_t b_half = map_to_cta(smem_u32(p_half), 0);
+        const uint32_t b_half = map_to_cta(smem_u32(p_half), lead);
         const float sl = p.scale_log2;
         const uint64_t sl2 = pack_f32x2(sl, sl);
         const bool causal = (p.mask_type == 3);
@@ -549,7 +641,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         uint32_t s0[32], s1[32], s2[32], s3[32];  // the row's 128 scores of the current block
         WideCursor cur(first, step);
         for (; ok && cur.w < total; cur.advance(p)) {
-            const WideWork w = decode_wide<MASKED>(p, cur, rank);
+            const WideWork w = unit_at(cur);
             if (w.hi == w.lo) continue;
             const int t = w.q0 + r;
             int row_lo = 0, row_hi = p.kv_len;  // visible keys [row_lo, row_hi)
@@ -608,7 +700,8 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 chunk_max<0>(s1, mr, sl, kc, rm);
                 chunk_max<0>(s2, mr, sl, kc, rm);
                 chunk_max<0>(s3, mr, sl, kc, rm);
-                const float m_new = fmaxf(m, fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sl);
+                const float top = fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3]));
+                const float m_new = fmaxf(m, top * sl);
                 if (j == w.lo) {
                     m = m_new;
                 } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
@@ -640,6 +733,10 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
                 const uint64_t nm2 = pack_f32x2(-m_eff, -m_eff);
                 uint64_t ls2[2] = {0ull, 0ull};
+                // The sum takes the block's largest probability as the second MMA will see it, rounded to bf16: a row that
+                // one key dominates would otherwise be off by that rounding whenever m is stale (2^-9, as much as the output's own).
+                const float p_top = fast_exp2(fmaf(top, sl, -m_eff));
+                l += bf16_round(p_top) - p_top;
                 uint32_t pk[16];
                 exp_chunk(s0, pk, ls2, sl2, nm2);
                 tmem_st16(tS, pk);
@@ -663,10 +760,15 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             }
             if (ok) {
                 fin_vals[(n & 3) * 128 + r] = l;
-                if (p.out_lse && t < p.seq)
-                    p.out_lse[((long long)w.b * p.seq + t) * p.nq + w.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
+                float* lse = SPLIT ? part_lse : p.out_lse;
+                if (lse && t < p.seq)
+                    lse[((long long)w.b * p.seq + t) * p.nq + w.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
                 mbar_arrive_warp(&fin[n & 3]);
                 ++n;
+                if constexpr (SPLIT) {
+                    store_part(w, quarter, l, HD / 2);
+                    break;
+                }
             }
         }
     }
@@ -675,6 +777,82 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();  // neither CTA's barriers or tensor memory go before the other is through with them
+    if constexpr (SPLIT) {
+        if (p.fold && total > 0) {  // every part's records are there; a warp takes a row in ten of the CTA's share
+            constexpr int W = C::THREADS / 32;
+            const long long rows = (long long)p.batch * p.seq * p.nq;
+            const WideWork w = *first_unit;
+            const int parts = p.num_splits, r0 = own_row0(w.part), end = min(own_row0(w.part + 1), p.seq - w.q0);
+            const long long row0 = ((long long)w.b * p.seq + w.q0) * p.nq + w.h;
+            const long long eoff0 = w.b * p.o_stride_b + w.q0 * p.o_stride_t + (long long)w.h * HD + lane * 4;
+            // The other parts' rows go behind the tile (at most 48 rows of two or 64 of one), gate values into rows of
+            // the tile that others fold.
+            constexpr int THEIRS = 8 * PART_CHUNK;
+            auto theirs = [&](int i) { return smem + THEIRS + (i - r0) * (parts - 1) * 1024 + lane * 16; };
+            auto gates = [&](int i) { return smem + (lane >> 4) * PART_CHUNK + ((own_row0(w.part + 1) + i - r0) & 127) * 128 + (lane & 15) * 8; };
+            float lse = -CUDART_INF_F;  // lane = 3 k + part: of the warp's k-th row
+            const int li = r0 + warp + lane / 3 * W;
+            if (li < end && lane % 3 < parts) lse = p.part_lse[lane % 3 * rows + row0 + (long long)li * p.nq];
+#pragma unroll 1
+            for (int i = r0 + warp; i < end; i += W) {
+                uint8_t* dst = theirs(i);
+                const float* src = p.part_o + (row0 + (long long)i * p.nq) * HD + lane * 4;
+#pragma unroll 1
+                for (int u = 0; u < parts; ++u) {
+                    if (u == w.part) continue;
+                    cp_async_16(dst, src + u * rows * HD);
+                    cp_async_16(dst + 512, src + u * rows * HD + 128);
+                    dst += 1024;
+                }
+                if (p.gate) {
+                    cp_async_8(gates(i), p.gate + eoff0 + i * p.o_stride_t);
+                    cp_async_8(gates(i) + 2 * PART_CHUNK, p.gate + eoff0 + i * p.o_stride_t + 128);
+                }
+            }
+            // The parts' weights, for all the warp's rows at once (lanes 30 and 31 hold nothing).
+            const int base = lane / 3 * 3;
+            const float l0 = __shfl_sync(0xffffffffu, lse, base), l1 = __shfl_sync(0xffffffffu, lse, base + 1), l2 = __shfl_sync(0xffffffffu, lse, base + 2);
+            const float mx = fmaxf(fmaxf(l0, l1), l2), at0 = mx == -CUDART_INF_F ? 0.f : mx;
+            const float z = __expf(l0 - at0) + __expf(l1 - at0) + __expf(l2 - at0);
+            const float weight = z > 0.f ? __expf(lse - at0) / z : 0.f;
+            if (p.out_lse && li < end && lane % 3 == 0) p.out_lse[row0 + (long long)li * p.nq] = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
+            cp_async_wait_all();
+            __syncwarp();
+            int k3 = 0;
+#pragma unroll 1
+            for (int i = r0 + warp; i < end; i += W, k3 += 3) {
+                const uint8_t* from = theirs(i);
+                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    const float e = __shfl_sync(0xffffffffu, weight, k3 + u);
+                    const bool own = u == w.part;
+                    const uint8_t* src = own ? smem + (lane >> 3) * PART_CHUNK + i * 128 + (((lane & 7) ^ (i & 7)) << 4) : from;
+                    if (!own) from += 1024;
+                    if (e == 0.f) continue;  // no such part, or an empty one, whose record may hold anything
+                    const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + (own ? 4 * PART_CHUNK : 512));
+                    acc[0] = fmaf(e, a.x, acc[0]), acc[1] = fmaf(e, a.y, acc[1]), acc[2] = fmaf(e, a.z, acc[2]), acc[3] = fmaf(e, a.w, acc[3]);
+                    acc[4] = fmaf(e, b.x, acc[4]), acc[5] = fmaf(e, b.y, acc[5]), acc[6] = fmaf(e, b.z, acc[6]), acc[7] = fmaf(e, b.w, acc[7]);
+                }
+                uint2 o[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    float* a = acc + 4 * c;
+                    if (p.gate) {
+                        const uint2 g = *reinterpret_cast<const uint2*>(gates(i) + c * 2 * PART_CHUNK);
+                        a[0] = sigmoid_gate(a[0], (uint16_t)g.x), a[1] = sigmoid_gate(a[1], (uint16_t)(g.x >> 16));
+                        a[2] = sigmoid_gate(a[2], (uint16_t)g.y), a[3] = sigmoid_gate(a[3], (uint16_t)(g.y >> 16));
+                    }
+                    o[c] = make_uint2(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]));
+                }
+                for (int c = -1; c < p.n_copies; ++c) {
+                    uint16_t* dst = (c < 0 ? p.out : reinterpret_cast<uint16_t*>(p.out_copies[c])) + eoff0 + i * p.o_stride_t;
+                    *reinterpret_cast<uint2*>(dst) = o[0];
+                    *reinterpret_cast<uint2*>(dst + 128) = o[1];
+                }
+            }
+        }
+    }
     if (warp == C::PRODUCER_WARP) tmem_dealloc_pair(tmem_base, 512);
 }
 

@@ -332,6 +332,15 @@ __device__ __forceinline__ void bulk_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory");
 }
 
+// 16 / 8 bytes of global memory to shared memory, asynchronous; this thread's have landed after cp_async_wait_all().
+__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_8(void* smem_dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // 2-D tiled load (c0 innermost, multiple of 8 elements for 16-bit data).
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1) {
     asm volatile(
@@ -554,7 +563,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 
 // ---------------------------------------------------------------------------
-// tcgen05 on a CTA pair (cta_group::2): two CTAs of a cluster of two hold 128 rows of D (and of A) each, and half of
+// tcgen05 on a CTA pair (cta_group::2): two neighbouring CTAs of a cluster hold 128 rows of D (and of A) each, and half of
 // B each; one thread of the leader CTA (rank 0) issues for both.  Allocation and release are done by one warp of each.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t ncols) {
@@ -603,12 +612,13 @@ __device__ __forceinline__ void umma_pair_ts_x4(uint32_t d_tmem, uint32_t a_tmem
 }
 
 // Arrive on the mbarrier at this address in BOTH CTAs once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+// (first: rank of the pair's first CTA in the cluster)
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t first) {
     asm volatile(
-        "{\n\t.reg .pred q;\n\t.reg .b16 m;\n\tmov.b16 m, 3;\n\t"
+        "{\n\t.reg .pred q;\n\t.reg .b16 m;\n\tcvt.u16.u32 m, %1;\n\t"
         "elect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(
-            smem_u32(bar))
+            smem_u32(bar)), "r"(3u << first)
         : "memory");
 }
 

@@ -73,7 +73,9 @@ const char* arc_sdpa_last_error(void);
  * mul_sigmoid_inplace (src/modeling/qwen3_5_moe/kernels.hpp:80-88).
  * `num_splits` > 1 splits the key range over several CTAs per query tile and
  * needs `workspace` of arc_sdpa_prefill_workspace_bytes(); 0 picks a value
- * (ask the size function: a non-zero answer means a workspace is required).
+ * (ask the size function: a non-zero answer means a workspace is wanted; head
+ * dim 256 does without one, more slowly: the key range then stays whole, and an
+ * explicit mask is read by the attention kernel itself).
  * ------------------------------------------------------------------------- */
 typedef struct arc_sdpa_prefill_params {
     const void* q;     /* (batch, seq, nq, hd) bf16 */
@@ -99,8 +101,8 @@ typedef struct arc_sdpa_prefill_params {
      * (seq, kv_len) f32 buffer).  block_ids: device int32 per absolute position, -1 = text token, a
      * non-negative id for each contiguous image / video block; a query inside a block also sees the
      * block's later keys.  block_ids[block_ids_offset + j] belongs to key j, so the array must reach
-     * block_ids_offset + kv_len entries; the same ids serve every sequence of the batch.  Needs
-     * workspace (arc_sdpa_prefill_workspace_bytes()); head dim 128 then runs the one-tile kernel. */
+     * block_ids_offset + kv_len entries; the same ids serve every sequence of the batch.  Head
+     * dim 128 needs workspace (arc_sdpa_prefill_workspace_bytes()) and runs the one-tile kernel. */
     const int32_t* block_ids;
     int32_t block_ids_offset;
     /* Copies of the output (optional; no counterpart in the reference, which is single-device).

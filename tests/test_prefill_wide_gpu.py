@@ -120,3 +120,36 @@ def test_vision_blocks_longer_than_a_search_step():
         # the same visible keys; blocks may be skipped in one form and fully masked in the other
         assert_close(got, want.float(), f"window {window}", rel_tol=2e-3, abs_tol=8e-3)
     assert ops.device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("parts", [2, 3, 4, 8])
+@pytest.mark.parametrize("batch,seq,kv,nq,nkv,window", [
+    (1, 256, 1100, 8, 4, oracle.INT_MAX),  # two row tiles of pairs of heads, the last key block ragged
+    (1, 77, 1030, 4, 2, oracle.INT_MAX),   # one ragged tile: shares of the fold without rows
+    (2, 130, 700, 3, 3, oracle.INT_MAX),   # odd group: 256 tokens of one head, the second tile two rows
+    (1, 300, 900, 4, 2, 60),               # a window: parts without key blocks, rows that see none of a part's keys
+    (3, 200, 600, 24, 4, oracle.INT_MAX),  # more units than clusters or pairs: always a merge launch, several waves
+])
+def test_parts_of_the_key_range(parts, batch, seq, kv, nq, nkv, window):
+    """Two and three parts fold as one cluster where every cluster fits at once, the rest in a launch of their own: the
+    gated output, the plain one with its log-sum-exp and its copy, as the whole range gives them."""
+    from arcaine_b200 import ops
+    ops.clear_device_status()
+    hd, mask = 256, 3 if window != oracle.INT_MAX else 0
+    q, k, v, gate = (seeded_bf16(batch, n, h, hd, seed=70 + i).cuda() for i, (n, h) in enumerate([(seq, nq), (kv, nkv), (kv, nkv), (seq, nq)]))
+    run = lambda n, **kw: ops.sdpa_prefill(q, k, v, scale=0.0625, mask_type=mask, window=window, num_splits=n, **kw)  # noqa: E731
+    copy = torch.empty_like(q)
+    before = ops.launch_count()
+    out, lse = run(parts, return_lse=True, out_copies=torch.tensor([copy.data_ptr()], device="cuda"))
+    units = batch * ((seq + 127) // 128 * nq // 2 if nq // nkv % 2 == 0 else (seq + 255) // 256 * nq)
+    assert ops.launch_count() - before == (1 if parts <= 3 and units <= 20 else 2)
+    want, want_lse = run(1, return_lse=True)
+    # the same values but for the bf16 rounding of the probabilities, whose reference a part chooses for itself
+    assert_close(out, want.float().cpu(), "out", rel_tol=4e-3, abs_tol=1.6e-2)
+    assert torch.equal(copy, out)
+    fin = torch.isfinite(want_lse)
+    assert torch.equal(torch.isfinite(lse), fin) and torch.allclose(lse[fin], want_lse[fin], atol=2e-3)
+    assert_close(run(parts, gate=gate), run(1, gate=gate).float().cpu(), "gated", rel_tol=4e-3, abs_tol=1.6e-2)
+    for _ in range(10):
+        assert torch.equal(run(parts), out)
+    assert ops.device_status() == (0, 0)
