@@ -529,14 +529,14 @@ struct DecodePlan {
     bool cluster = false;  // one launch: a cluster of `ncta` CTAs per sequence and group of KV heads
 };
 
-// Shared memory of a CTA that works on `nkv_cta` KV heads: slices, stages, bytes.  False: not even two stages fit.
-static bool size_decode_cta(int hd, int nkv_cta, int batch, int smem_optin, DecodePlan* plan) {
+// Shared memory of a CTA that works on `nkv_cta` KV heads (and holds `extra` bytes): slices, stages, bytes.  False: not even two stages fit.
+static bool size_decode_cta(int hd, int nkv_cta, int batch, int extra, int smem_optin, DecodePlan* plan) {
     const int row_bytes = nkv_cta * hd * 2;
     int slices = (64 * 1024) / (32 * row_bytes);
     if (slices > 8 / nkv_cta) slices = 8 / nkv_cta;
     if (slices < 1) slices = 1;
     const int stage_bytes = 2 * 16 * slices * row_bytes;
-    const int fixed = 1024 + 2 * 8 * 8 + (batch + 2) * 8;
+    const int fixed = 1024 + 2 * 8 * 8 + (batch + 2) * 8 + extra;
     int stages = (smem_optin - kDecodeStaticSmem - fixed) / stage_bytes;
     if (stages > 4) stages = 4;
     plan->nkv_cta = nkv_cta;
@@ -576,9 +576,9 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
     const double t_shares = 9.0 + 0.12 * p->batch + total * p->nkv * p->hd * 4.0 / 6.9e6;
     if (t_cluster > t_shares) return;
     DecodePlan one = *plan;
-    if (!size_decode_cta(p->hd, heads, 0, ds.smem_optin, &one)) return;
-    const int ncw = heads * one.slices;  // the records must fit where the stages were
-    if ((ncw * one.nt * 8 + heads * G) * (p->hd + 1) * 4 > one.stages * 2 * 16 * one.slices * heads * p->hd * 2) return;
+    // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where
+    // the stages were, at least two: 64 * hd floats a warp, at most 16 * (hd + 5) needed.)
+    if (!size_decode_cta(p->hd, heads, 0, heads * G * (p->hd + csize) * 4, ds.smem_optin, &one)) return;
     one.cluster = true;
     one.groups = p->nkv / heads;
     one.ncta = csize;
@@ -610,7 +610,7 @@ static int plan_decode(const arc_sdpa_decode_params* p, const DeviceState& ds, D
     int nkv_cta = 1;
     for (int c = 1; c <= p->nkv && c <= max_heads; ++c)
         if (p->nkv % c == 0) nkv_cta = c;
-    if (!size_decode_cta(p->hd, nkv_cta, p->batch, smem_optin, plan)) return ARC_ERR_TOO_LARGE;
+    if (!size_decode_cta(p->hd, nkv_cta, p->batch, 0, smem_optin, plan)) return ARC_ERR_TOO_LARGE;
     plan->groups = p->nkv / nkv_cta;
     int ncta = p->num_ctas > 0 ? p->num_ctas : sm_count / plan->groups;
     if (ncta < 1) ncta = 1;
@@ -694,9 +694,14 @@ static int launch_decode(const arc_sdpa_decode_params* p, const DecodePlan& plan
     mp.x_step = p->xchg_step;
     mp.x_wait_cycles = p->xchg_wait_cycles > 0 ? p->xchg_wait_cycles : 2000000000LL;
     mp.fault = ds->fault;
-    dim3 mgrid((unsigned)p->nq, (unsigned)p->batch, 1);
     const bool xchg = mp.x_world > 1;
-    ARC_CUDA(launch_dependent(xchg ? sdpa_decode_merge_kernel<HD, true> : sdpa_decode_merge_kernel<HD, false>, mgrid,
+    // 64 columns a block while that leaves at most one block per SM; with more, every block would repeat the search for
+    // the records for less work of its own.
+    const bool narrow = !xchg && (long long)p->nq * p->batch * (HD / 64) <= ds->sm_count;
+    const dim3 mgrid((unsigned)p->nq, (unsigned)p->batch, narrow ? HD / 64 : 1);
+    ARC_CUDA(launch_dependent(xchg     ? sdpa_decode_merge_kernel<HD, true, HD>
+                              : narrow ? sdpa_decode_merge_kernel<HD, false, 64>
+                                       : sdpa_decode_merge_kernel<HD, false, HD>, mgrid,
                               dim3(MERGE_THREADS), 0, stream, 1, mp));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return ARC_OK;

@@ -66,12 +66,13 @@ struct DecodeParams {
 // Prefix sums of the per-sequence lengths into shared memory: cum[b] = keys before sequence b, cum[batch] = total.
 // Called by the first warp, which scans 32 sequences a step (one thread adding them up in turn took a microsecond for
 // 64); the caller's barrier follows.
-__device__ __forceinline__ void build_len_prefix(const int* kv_len, int kv_len_uniform, int batch, long long* cum) {
+template <typename F>
+__device__ __forceinline__ void build_len_prefix(int batch, long long* cum, F&& len_of) {
     long long run = 0;
     if (threadIdx.x == 0) cum[0] = 0;
     for (int b0 = 0; b0 < batch; b0 += 32) {
         const int b = b0 + threadIdx.x;
-        const int len = b < batch ? (kv_len ? kv_len[b] : kv_len_uniform) : 0;
+        const int len = b < batch ? len_of(b) : 0;
         long long v = len > 0 ? len : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -84,9 +85,12 @@ __device__ __forceinline__ void build_len_prefix(const int* kv_len, int kv_len_u
 }
 
 __device__ __forceinline__ long long share_size(long long total, int ncta, int tile_keys) {
-    long long per = (total + ncta - 1) / ncta;
-    per = (per + tile_keys - 1) / tile_keys * tile_keys;
-    return per > 0 ? per : tile_keys;
+    if (total < (1ll << 30)) {  // (a 64-bit division takes some hundred clk, and every role waits for this one)
+        const uint32_t per = ((uint32_t)total + ncta - 1) / (uint32_t)ncta;
+        return max(1u, (per + tile_keys - 1) / (uint32_t)tile_keys) * tile_keys;
+    }
+    const long long per = (total + ncta - 1) / ncta;
+    return (per + tile_keys - 1) / tile_keys * tile_keys;
 }
 
 __device__ __forceinline__ float sigmoid_gate(float attn, uint16_t gate_bits) {
@@ -100,8 +104,8 @@ __device__ __forceinline__ void consumer_sync(int consumer_warps) {
 }
 
 // CLUSTER: a cluster of CTAs owns one sequence (grid.z) and one group of KV heads (grid.y); its CTAs take equal parts of
-// the sequence's keys, fold their slices as above, then fold each other's records through distributed shared
-// memory and write the result: one launch, no records in global memory, no merge kernel.  For calls so small that the
+// the sequence's keys, fold their slices as above, leave the records in the shared memory of the CTAs that finish them
+// and write the result: one launch, no records in global memory, no merge kernel.  For calls so small that the
 // launches are what they cost; otherwise equal shares over all SMs win.
 template <int HD, int NT, bool CLUSTER>
 __global__ void __launch_bounds__(288, 1)
@@ -139,47 +143,74 @@ __global__ void __launch_bounds__(288, 1)
         }
         fence_mbar_init();
     }
+    long long g0 = 0, g1 = 0;  // this CTA's keys, counted over the sequences laid end to end (CLUSTER: of its own sequence)
+    int b_first = 0, my_len = 0;
+    bool work = true;
+    auto find_share = [&]() {
+        if constexpr (CLUSTER) {
+            b_first = blockIdx.z;
+            const int per = ((my_len + p.ncta - 1) / p.ncta + 15) / 16 * 16;
+            g0 = (long long)blockIdx.x * per;
+            g1 = min((long long)my_len, g0 + per);
+        } else {
+            const long long total = cum[p.batch];
+            const long long per = share_size(total, p.ncta, tk);
+            g0 = (long long)blockIdx.x * per;
+            g1 = min(total, g0 + per);
+            for (int b0 = 0; b0 < p.batch - 1; b0 += 32) {  // sequences that end at or before the share's first key
+                const int n = __popc(__ballot_sync(0xffffffffu, b0 + lane < p.batch - 1 && cum[b0 + lane + 1] <= g0));
+                b_first += n;
+                if (n < 32) break;
+            }
+        }
+    };
+    // Lengths the host knows, and has checked, need no look at memory: the share is found before the wait.
+    const bool known = !p.kv_len && !p.kv_row_offset;
+    if (known) {
+        my_len = max(0, p.kv_len_uniform);
+        if (!CLUSTER && threadIdx.x < 32) build_len_prefix(p.batch, cum, [&](int) { return p.kv_len_uniform; });
+        __syncthreads();
+        find_share();
+    }
+    if (CLUSTER) cluster_sync_all();  // every CTA runs: its shared memory may be written
     // Up to here nothing depends on the kernels in front; everything below may.
     grid_dependency_wait();
     grid_launch_dependents();  // the merge kernel may be scheduled now; it waits for this grid before reading
-    // The status word, the lengths and the row offsets are asked for together: each is a trip to L2 or HBM.
-    // Lengths and row offsets live on the device, so this is where they can be checked: a sequence that reaches past the
-    // cache (the copies would read zero rows and fold them in as score-0 keys) or past the stated bound stops the
-    // launch with a status instead of a wrong result.  Every CTA checks all sequences and so none of them works.
-    bool bad = threadIdx.x == 0 && *reinterpret_cast<volatile uint32_t*>(p.fault) != 0u;
-    for (int b = threadIdx.x; b < p.batch; b += blockDim.x) {
-        const int len = p.kv_len ? p.kv_len[b] : p.kv_len_uniform;
-        const long long row0 = p.kv_row_offset ? p.kv_row_offset[b] : (long long)b * p.kv_stride_b;
-        if ((len > 0 && (row0 < 0 || row0 + len > p.kv_rows_total)) || (p.max_kv_len > 0 && len > p.max_kv_len)) {
-            report_fault(p.fault, FAULT_BAD_KV_RANGE, (uint32_t)b);
-            bad = true;
-        }
+    const uint32_t fault = threadIdx.x == 0 ? *reinterpret_cast<volatile uint32_t*>(p.fault) : 0u;  // (set: no result is written)
+    if (!known) {
+        // The status word, the lengths and the row offsets are asked for together: each is a trip to L2 or HBM.
+        // Lengths and row offsets live on the device, so this is where they can be checked: a sequence that reaches past the
+        // cache (the copies would read zero rows and fold them in as score-0 keys) or past the stated bound stops the
+        // launch with a status instead of a wrong result.  Every CTA checks all sequences and so none of them works.
+        // (The first warp checks and adds up what it has asked for once: a second look was a second trip.)
+        bool bad = fault != 0u;
+        auto checked_len = [&](int b) {
+            const int len = p.kv_len ? p.kv_len[b] : p.kv_len_uniform;
+            const long long row0 = p.kv_row_offset ? p.kv_row_offset[b] : (long long)b * p.kv_stride_b;
+            if ((len > 0 && (row0 < 0 || row0 + len > p.kv_rows_total)) || (p.max_kv_len > 0 && len > p.max_kv_len)) {
+                report_fault(p.fault, FAULT_BAD_KV_RANGE, (uint32_t)b);
+                bad = true;
+            }
+            return len;
+        };
+        if (!CLUSTER && threadIdx.x < 32) build_len_prefix(p.batch, cum, checked_len);
+        if (CLUSTER)
+            for (int b = threadIdx.x; b < p.batch; b += blockDim.x) checked_len(b);
+        if (CLUSTER) my_len = max(0, p.kv_len ? p.kv_len[blockIdx.z] : p.kv_len_uniform);
+        work = !__syncthreads_or(bad);
+        if (work) find_share();
     }
-    if (!CLUSTER && threadIdx.x < 32) build_len_prefix(p.kv_len, p.kv_len_uniform, p.batch, cum);
-    const int my_len = CLUSTER ? max(0, p.kv_len ? p.kv_len[blockIdx.z] : p.kv_len_uniform) : 0;
-    const bool work = !__syncthreads_or(bad);
-    long long g0, g1;  // this CTA's keys, counted over the sequences laid end to end (CLUSTER: of its own sequence)
-    int b_first = 0;
-    if constexpr (CLUSTER) {
-        b_first = blockIdx.z;
-        const int per = ((my_len + p.ncta - 1) / p.ncta + 15) / 16 * 16;
-        g0 = (long long)blockIdx.x * per;
-        g1 = work ? min((long long)my_len, g0 + per) : g0;
-    } else {
-        if (!work) return;
-        const long long total = cum[p.batch];
-        const long long per = share_size(total, p.ncta, tk);
-        g0 = (long long)blockIdx.x * per;
-        g1 = min(total, g0 + per);
-        if (g0 >= g1) return;
-        while (b_first < p.batch - 1 && cum[b_first + 1] <= g0) ++b_first;
-    }
+    if (!CLUSTER && g0 >= g1) return;
     // keys before sequence b / up to its end, in the count g0 and g1 use
     auto seq_begin = [&](int b) { return CLUSTER ? 0ll : cum[b]; };
     auto seq_end = [&](int b) { return CLUSTER ? (long long)my_len : cum[b + 1]; };
-    // CLUSTER: this CTA's folded record of every head of its group, behind the warps' records
-    float* crec = reinterpret_cast<float*>(stage_base) + (size_t)ncw * NT * 8 * (HD + 1);
-    float* crec_lse = crec + (size_t)p.nkv_cta * G * HD;
+    // CLUSTER: CTA c of the cluster finishes columns [c, c + 1) * HD / ncta of all heads; the others leave their folded
+    // records of those here: [CTA][query head of the group][column], and the log-sum-exps behind.
+    float* crec = reinterpret_cast<float*>(cum + 2);
+    const int dc_log2 = (HD == 256 ? 8 : 7) - (CLUSTER ? __ffs(p.ncta) - 1 : 0), dc = 1 << dc_log2;  // (clusters are of 1, 2, 4 or 8)
+    const int rows = p.nkv_cta * G;
+    float* crec_lse = crec + (size_t)rows * HD;
+    constexpr int RS = HD + 4;  // floats from one head's row of a warp's record to the next
 
     if (warp == ncw) {
         // ------------------------------------------------------------------ producer
@@ -295,18 +326,43 @@ __global__ void __launch_bounds__(288, 1)
                         __syncwarp();
                     }
 
-                    float acc[NT][2][4];
+                    // Fragments are fetched AHEAD at a time and a batch before their MMAs: fetched one by one, each MMA
+                    // waited 40 clk for its own, and the 32 of a step of 16 keys at head dim 256 took 1400 clk (now 800).
+                    constexpr int AHEAD = HD * NT > 256 ? 2 : 4, BATCHES = HD / 16 / AHEAD;
+                    constexpr int CHAINS = NT == 1 ? 4 : 2;  // independent sums of S
+                    uint32_t fr[2][AHEAD][4];
+                    auto fetch_k = [&](int bt) {
+#pragma unroll
+                        for (int i = 0; i < AHEAD; ++i) {
+                            const int kk = bt * AHEAD + i;
+                            ldmatrix_x4(fr[bt & 1][i], a_k + (kk >> 2) * chunk_bytes + ((((kk & 3) * 2 + hk) ^ xk) << 4));
+                        }
+                    };
+                    auto fetch_v = [&](int bt) {
+#pragma unroll
+                        for (int i = 0; i < AHEAD; ++i) {
+                            const int mt = bt * AHEAD + i;
+                            ldmatrix_x4_trans(fr[bt & 1][i], a_v + (mt >> 2) * chunk_bytes + ((((mt & 3) * 2 + hv) ^ xv) << 4));
+                        }
+                    };
+                    float acc[NT][CHAINS][4];
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                        for (int hh = 0; hh < 2; ++hh) acc[nt][hh][0] = acc[nt][hh][1] = acc[nt][hh][2] = acc[nt][hh][3] = 0.f;
+                        for (int hh = 0; hh < CHAINS; ++hh) acc[nt][hh][0] = acc[nt][hh][1] = acc[nt][hh][2] = acc[nt][hh][3] = 0.f;
+                    fetch_k(0);
 #pragma unroll
-                    for (int kk = 0; kk < HD / 16; ++kk) {
-                        uint32_t a[4];
-                        ldmatrix_x4(a, a_k + (kk >> 2) * chunk_bytes + ((((kk & 3) * 2 + hk) ^ xk) << 4));
+                    for (int bt = 0; bt < BATCHES; ++bt) {
+                        if (bt + 1 < BATCHES) fetch_k(bt + 1);
+                        else if (NT == 1) fetch_v(0);  // (an even number of batches: into the other half)
 #pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(acc[nt][kk & 1], a, qf[nt][kk][0], qf[nt][kk][1]);
+                        for (int i = 0; i < AHEAD; ++i) {
+                            const int kk = bt * AHEAD + i;
+#pragma unroll
+                            for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(acc[nt][kk % CHAINS], fr[bt & 1][i], qf[nt][kk][0], qf[nt][kk][1]);
+                        }
                     }
+                    static_assert(BATCHES % 2 == 0, "the first batch of V goes where the last one of K is not");
                     const bool v_lo = g4 < nvalid, v_hi = g4 + 8 < nvalid;
                     uint32_t pb[NT][2];
                     bool any_rescale = false;
@@ -316,7 +372,9 @@ __global__ void __launch_bounds__(288, 1)
                         float x[4];
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            const float s = (acc[nt][0][e] + acc[nt][1][e]) * sl;
+                            float s = acc[nt][0][e] + acc[nt][1][e];
+                            if constexpr (CHAINS == 4) s += acc[nt][2][e] + acc[nt][3][e];
+                            s *= sl;
                             x[e] = ((e < 2) ? v_lo : v_hi) ? s : -CUDART_INF_F;
                         }
                         float pr[4];
@@ -349,12 +407,14 @@ __global__ void __launch_bounds__(288, 1)
                                 o[nt][mt][3] *= alpha[nt][1];
                             }
                     }
+                    if (NT > 1) fetch_v(0);
 #pragma unroll
-                    for (int mt = 0; mt < HD / 16; ++mt) {
-                        uint32_t a[4];
-                        ldmatrix_x4_trans(a, a_v + (mt >> 2) * chunk_bytes + ((((mt & 3) * 2 + hv) ^ xv) << 4));
+                    for (int bt = 0; bt < BATCHES; ++bt) {
+                        if (bt + 1 < BATCHES) fetch_v(bt + 1);
 #pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(o[nt][mt], a, pb[nt][0], pb[nt][1]);
+                        for (int i = 0; i < AHEAD; ++i)
+#pragma unroll
+                            for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(o[nt][bt * AHEAD + i], fr[bt & 1][i], pb[nt][0], pb[nt][1]);
                     }
                 }
                 __syncwarp();
@@ -369,8 +429,9 @@ __global__ void __launch_bounds__(288, 1)
             // `slices` times fewer records.  Earlier segments (a sequence boundary inside the share) write
             // one record per slice.
             const bool fold_here = CLUSTER || (p.slices > 1 && seg_end == g1);  // CTA-uniform
-            float* rec = reinterpret_cast<float*>(stage_base);     // [warp][NT * 8 heads][HD]
-            float* rec_lse = rec + (size_t)ncw * NT * 8 * HD;      // [warp][NT * 8]
+            // (rows four floats longer than HD: the four lanes that write the same column of different heads hit different banks)
+            float* rec = reinterpret_cast<float*>(stage_base);     // [warp][NT * 8 heads][RS]
+            float* rec_lse = rec + (size_t)ncw * NT * 8 * RS;      // [warp][NT * 8]
             if (fold_here) {
                 consumer_sync(ncw);  // every warp is through with the stages; no copy is in flight any more
                 folded = true;
@@ -398,7 +459,7 @@ __global__ void __launch_bounds__(288, 1)
                     for (int u = 0; u < 2; ++u) {
                         const int n = nt * 8 + q4 * 2 + u;
                         if (fold_here || n < G) {
-                            float* dst = fold_here ? rec + ((size_t)warp * NT * 8 + n) * HD
+                            float* dst = fold_here ? rec + ((size_t)warp * NT * 8 + n) * RS
                                                    : p.part_o + (part * p.nq + (long long)kvh * G + n) * HD;
 #pragma unroll
                             for (int mt = 0; mt < HD / 16; ++mt) {
@@ -411,39 +472,50 @@ __global__ void __launch_bounds__(288, 1)
             }
             if (fold_here) {
                 consumer_sync(ncw);  // all records of the CTA are in shared memory
-                // The `slices` warps of this KV head share its G x HD output values, four per step.
-                const long long part0 = ((long long)blockIdx.x + b) * p.slices;
-                for (int item = slice * 32 + lane; item < G * (HD / 4); item += p.slices * 32) {
-                    const int n = item / (HD / 4), d = (item % (HD / 4)) * 4;
-                    float mx = -CUDART_INF_F;
-                    for (int sidx = 0; sidx < p.slices; ++sidx)
-                        mx = fmaxf(mx, rec_lse[(sidx * p.nkv_cta + hl) * NT * 8 + n]);
-                    float z = 0.f;
-                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (mx > -CUDART_INF_F) {
-                        for (int sidx = 0; sidx < p.slices; ++sidx) {
-                            const int w = sidx * p.nkv_cta + hl;
-                            const float li = rec_lse[w * NT * 8 + n];
-                            if (li == -CUDART_INF_F) continue;
-                            const float wt = __expf(li - mx);
-                            z += wt;
-                            const float4 ov = *reinterpret_cast<const float4*>(rec + ((size_t)w * NT * 8 + n) * HD + d);
-                            acc.x = fmaf(wt, ov.x, acc.x);
-                            acc.y = fmaf(wt, ov.y, acc.y);
-                            acc.z = fmaf(wt, ov.z, acc.z);
-                            acc.w = fmaf(wt, ov.w, acc.w);
+                // The `slices` (at most eight) warps of this KV head take its rows in turn; the weights of a row's records
+                // are worked out once, a lane each.
+                const long long row0 = ((long long)blockIdx.x + b) * p.slices * p.nq + (long long)kvh * G;
+                for (int n = slice; n < G; n += p.slices) {
+                    const float li = lane < p.slices ? rec_lse[(lane * p.nkv_cta + hl) * NT * 8 + n] : -CUDART_INF_F;
+                    float mx = li;
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                    mx = __shfl_sync(0xffffffffu, mx, 0);
+                    float z = mx > -CUDART_INF_F ? __expf(li - mx) : 0.f;
+                    const float e = z;
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+                    z = __shfl_sync(0xffffffffu, z, 0);
+                    const float weight = z > 0.f ? e / z : 0.f;
+                    float4 acc[HD / 128];
+#pragma unroll
+                    for (int j = 0; j < HD / 128; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+                    for (int sidx = 0; sidx < p.slices; ++sidx) {
+                        const float wt = __shfl_sync(0xffffffffu, weight, sidx);
+                        const float* src = rec + ((size_t)(sidx * p.nkv_cta + hl) * NT * 8 + n) * RS + lane * 4;
+#pragma unroll
+                        for (int j = 0; j < HD / 128; ++j) {  // (an empty slice's record holds zeros)
+                            const float4 ov = *reinterpret_cast<const float4*>(src + 128 * j);
+                            acc[j].x = fmaf(wt, ov.x, acc[j].x);
+                            acc[j].y = fmaf(wt, ov.y, acc[j].y);
+                            acc[j].z = fmaf(wt, ov.z, acc[j].z);
+                            acc[j].w = fmaf(wt, ov.w, acc[j].w);
                         }
-                        const float iz = 1.f / z;
-                        acc = make_float4(acc.x * iz, acc.y * iz, acc.z * iz, acc.w * iz);
                     }
-                    const float rec_l = mx > -CUDART_INF_F ? mx + __logf(z) : -CUDART_INF_F;
+                    const float rec_l = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
                     if constexpr (CLUSTER) {
-                        *reinterpret_cast<float4*>(crec + (size_t)(hl * G + n) * HD + d) = acc;
-                        if (d == 0) crec_lse[hl * G + n] = rec_l;
+                        const uint32_t mine = smem_u32(crec + ((size_t)blockIdx.x * rows + hl * G + n) * dc);
+#pragma unroll
+                        for (int j = 0; j < HD / 128; ++j) {
+                            const int d = lane * 4 + 128 * j;
+                            st_cluster_f32x4(map_to_cta(mine + (d & (dc - 1)) * 4, d >> dc_log2), acc[j]);
+                        }
+                        if (lane < p.ncta) st_cluster_f32(map_to_cta(smem_u32(crec_lse + blockIdx.x * rows + hl * G + n), lane), rec_l);
                     } else {
-                        const long long row = part0 * p.nq + (long long)kvh * G + n;
-                        *reinterpret_cast<float4*>(p.part_o + row * HD + d) = acc;
-                        if (d == 0) p.part_lse[row] = rec_l;
+#pragma unroll
+                        for (int j = 0; j < HD / 128; ++j) *reinterpret_cast<float4*>(p.part_o + (row0 + n) * HD + lane * 4 + 128 * j) = acc[j];
+                        if (lane == 0) p.part_lse[row0 + n] = rec_l;
                     }
                 }
             }
@@ -455,62 +527,56 @@ __global__ void __launch_bounds__(288, 1)
             consumer_sync(ncw);
         }
         // (CLUSTER: no keys: an empty record)
-        if (CLUSTER && !folded)
-            for (int n = slice * 32 + lane; n < G; n += p.slices * 32) crec_lse[hl * G + n] = -CUDART_INF_F;
+        if (CLUSTER && !folded && lane < p.ncta)
+            for (int n = slice; n < G; n += p.slices)
+                st_cluster_f32(map_to_cta(smem_u32(crec_lse + blockIdx.x * rows + hl * G + n), lane), -CUDART_INF_F);
     }
     if constexpr (CLUSTER) {
+        // This CTA's columns, two a thread.  Every record is in its own shared memory by now: read out of the other CTAs
+        // instead, 16 loads a thread, this step took 2100 clk.
+        if (threadIdx.x == 0) cum[0] = work && fault == 0u;
+        const int items = rows * (dc / 2), b = blockIdx.z;
+        auto offset_of = [&](int item) {
+            return (long long)b * p.o_stride_b + (long long)(head0 * G + (item >> (dc_log2 - 1))) * HD + blockIdx.x * dc + (item & (dc / 2 - 1)) * 2;
+        };
+        uint32_t gw = p.gate && (int)threadIdx.x < items ? *reinterpret_cast<const uint32_t*>(p.gate + offset_of(threadIdx.x)) : 0u;
         __syncwarp();
-        cluster_sync_all();  // every CTA's records are in its shared memory
-        // this CTA's part of the (head, 4 columns) items, all records of an item in flight at once
-        const int heads = p.nkv_cta * G, items = heads * (HD / 4), C = p.ncta;
-        const uint32_t a_lse = smem_u32(crec_lse), a_rec = smem_u32(crec);
-        const int b = blockIdx.z;
-        for (int item = blockIdx.x * blockDim.x + threadIdx.x; work && item < items; item += C * blockDim.x) {
-            const int n = item / (HD / 4), d = (item % (HD / 4)) * 4;
-            const int h = head0 * G + n;
-            const long long eoff = (long long)b * p.o_stride_b + (long long)h * HD + d;
-            const uint2 gw = p.gate ? *reinterpret_cast<const uint2*>(p.gate + eoff) : make_uint2(0u, 0u);
-            float li[8];
-            float4 ov[8];
+        cluster_sync_all();  // every CTA's records are where they belong
+        for (int item = threadIdx.x; cum[0] && item < items; item += blockDim.x) {
+            const int n = item >> (dc_log2 - 1), d = (item & (dc / 2 - 1)) * 2;
+            const long long eoff = offset_of(item);
+            if (p.gate && item != (int)threadIdx.x) gw = *reinterpret_cast<const uint32_t*>(p.gate + eoff);
+            float li[8], mx = -CUDART_INF_F;
+            float2 v[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
-                li[c] = -CUDART_INF_F;
-                if (c < C) {
-                    li[c] = ld_cluster_f32(map_to_cta(a_lse + n * 4, c));
-                    ov[c] = ld_cluster_f32x4(map_to_cta(a_rec + (n * HD + d) * 4, c));
-                }
+                li[c] = c < p.ncta ? crec_lse[c * rows + n] : -CUDART_INF_F;
+                v[c] = c < p.ncta ? *reinterpret_cast<const float2*>(crec + (size_t)(c * rows + n) * dc + d) : make_float2(0.f, 0.f);
+                mx = fmaxf(mx, li[c]);
             }
-            float mx = li[0];
-#pragma unroll
-            for (int c = 1; c < 8; ++c) mx = fmaxf(mx, li[c]);
-            float z = 0.f, a[4] = {0.f, 0.f, 0.f, 0.f};
+            float z = 0.f, a0 = 0.f, a1 = 0.f;
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 if (li[c] == -CUDART_INF_F) continue;  // an empty record may hold anything
                 const float wt = __expf(li[c] - mx);
                 z += wt;
-                a[0] = fmaf(wt, ov[c].x, a[0]);
-                a[1] = fmaf(wt, ov[c].y, a[1]);
-                a[2] = fmaf(wt, ov[c].z, a[2]);
-                a[3] = fmaf(wt, ov[c].w, a[3]);
+                a0 = fmaf(wt, v[c].x, a0);
+                a1 = fmaf(wt, v[c].y, a1);
             }
             const float iz = z > 0.f ? 1.f / z : 0.f;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) a[e] *= iz;
-            const long long row = (long long)b * p.nq + h;
-            if (p.out_f32) *reinterpret_cast<float4*>(p.out_f32 + row * HD + d) = make_float4(a[0], a[1], a[2], a[3]);
-            if (p.out_lse && d == 0) p.out_lse[row] = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
+            a0 *= iz;
+            a1 *= iz;
+            const long long row = (long long)b * p.nq + head0 * G + n;
+            if (p.out_f32) *reinterpret_cast<float2*>(p.out_f32 + row * HD + blockIdx.x * dc + d) = make_float2(a0, a1);
+            if (p.out_lse && blockIdx.x == 0 && d == 0) p.out_lse[row] = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
             if (p.out) {
                 if (p.gate) {
-                    a[0] = sigmoid_gate(a[0], (uint16_t)(gw.x & 0xffffu));
-                    a[1] = sigmoid_gate(a[1], (uint16_t)(gw.x >> 16));
-                    a[2] = sigmoid_gate(a[2], (uint16_t)(gw.y & 0xffffu));
-                    a[3] = sigmoid_gate(a[3], (uint16_t)(gw.y >> 16));
+                    a0 = sigmoid_gate(a0, (uint16_t)(gw & 0xffffu));
+                    a1 = sigmoid_gate(a1, (uint16_t)(gw >> 16));
                 }
-                *reinterpret_cast<uint2*>(p.out + eoff) = make_uint2(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]));
+                *reinterpret_cast<uint32_t*>(p.out + eoff) = pack_bf16x2(a0, a1);
             }
         }
-        cluster_sync_all();  // nobody's shared memory goes while another CTA still reads it
     }
 }
 
@@ -564,17 +630,22 @@ __device__ __forceinline__ uint4 ld_volatile_v4(const uint4* p) {
 constexpr int MERGE_THREADS = 256;
 
 // XCHG: the instance that also exchanges records with other GPUs.  It keeps every source's values in
-// registers; the plain merge — hundreds of small blocks for a large batch — stays lean enough for five blocks
-// per SM.
-template <int HD, bool XCHG>
+// registers; the plain merge — hundreds of small blocks for a large batch — stays lean.
+// COLS: columns of the row a block takes.  All of them, unless the rows are so few that most SMs would idle: one token of
+// 24 heads over 6760 keys has 106 records in each of 24 rows, 100 KB a block, and took 7.5 us from the decode kernel's
+// end; 64 columns a block, every load of a batch in flight with the log-sum-exps, take 3.9.
+template <int HD, bool XCHG, int COLS>
 __global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const DecodeMergeParams p) {
     // One row of output per block; what the block does before its one barrier every warp does for itself — where the
     // row's records are, their maximum and weights — because that is a handful of loads, while three block-wide
     // reductions and a list in shared memory made this kernel's tail 5 us.
     constexpr int NW = MERGE_THREADS / 32;
-    __shared__ float acc_sm[NW * HD];
-    const int h = blockIdx.x, b = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int LPR = COLS / 4 < 32 ? COLS / 4 : 32, VPL = COLS / LPR;  // lanes of a record, their output values
+    constexpr int TEAMS = NW * 32 / LPR;                                  // records the block takes at a time
+    __shared__ float acc_sm[TEAMS * COLS];
+    const int h = blockIdx.x, b = blockIdx.y, col0 = XCHG ? 0 : blockIdx.z * COLS;
+    const int team = threadIdx.x / LPR, tl = threadIdx.x % LPR;
+    const int lane = threadIdx.x & 31;
     // (The decode kernel released this one after its own wait for the kernels in front: the lengths are final.)
     long long k_begin = 0, total = 0, k_len = 0;
     if (!p.kv_len) {
@@ -602,14 +673,15 @@ __global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const 
     const long long k_end = k_begin + k_len;
     grid_dependency_wait();                                            // from here on the partial records are read
     grid_launch_dependents();
-    if (*reinterpret_cast<volatile uint32_t*>(p.fault) != 0u) return;  // block-uniform: a status is set, no work
-    constexpr int VPL = HD / 32;  // output values per lane
+    const uint32_t fault = threadIdx.x == 0 ? *reinterpret_cast<volatile uint32_t*>(p.fault) : 0u;
     float acc[VPL];
 #pragma unroll
     for (int j = 0; j < VPL; ++j) acc[j] = 0.f;
     float lse = -CUDART_INF_F, inv = 0.f;
     if (k_len > 0) {  // block-uniform
-        const int c_first = (int)(k_begin / per), c_last = (int)((k_end - 1) / per);
+        const bool small = total < (1ll << 30);
+        const int c_first = small ? (int)((uint32_t)k_begin / (uint32_t)per) : (int)(k_begin / per);
+        const int c_last = small ? (int)((uint32_t)(k_end - 1) / (uint32_t)per) : (int)((k_end - 1) / per);
         const long long part0 = ((long long)c_first + b) * p.slices;
         // Which records exist follows from the shares: a share whose last segment is this sequence's folded its slices
         // into slice 0's record — every share but possibly the last, whose slices wrote one record each if the
@@ -618,30 +690,45 @@ __global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const 
         const int n_rec = n_full + (k_end == min(total, (c_last + 1) * per) ? 1 : p.slices);
         auto rec_of = [&](int j) { return part0 + (j < n_full ? (long long)j * p.slices : (long long)n_full * p.slices + (j - n_full)); };
         const float* lses = p.part_lse + h;
-        float mx = -CUDART_INF_F;
-        for (int j = lane; j < n_rec; j += 32) mx = fmaxf(mx, lses[rec_of(j) * p.nq]);
-        // The records are dealt to the warps in turn, four at a time with their loads in flight together (and beside
-        // those of the weights); a lane owns VPL consecutive output values.  Always the same order of additions.
+        // The records are dealt to the teams in turn, U at a time; a lane owns VPL consecutive output values.  Always the
+        // same order of additions.  The first batch and all log-sum-exps (eight a lane; more is rare) are asked for
+        // together: one trip to L2.
+        constexpr int U = 4, MINE = 8;
+        float wu[U];
+        float4 ov[U][VPL / 4];
+        auto load_batch = [&](int j0) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int j = j0 + u * TEAMS;
+                wu[u] = -CUDART_INF_F;
+                if (j < n_rec) {
+                    const long long rec = rec_of(j);
+                    wu[u] = lses[rec * p.nq];
+                    const float* src = p.part_o + (rec * p.nq + h) * HD + col0 + tl * VPL;
+#pragma unroll
+                    for (int i = 0; i < VPL / 4; ++i) ov[u][i] = *reinterpret_cast<const float4*>(src + 4 * i);
+                }
+            }
+        };
+        load_batch(team);
+        float mine[MINE], mx = -CUDART_INF_F;
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) mine[i] = lane + 32 * i < n_rec ? lses[rec_of(lane + 32 * i) * p.nq] : -CUDART_INF_F;
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) mx = fmaxf(mx, mine[i]);
+        for (int j = lane + 32 * MINE; j < n_rec; j += 32) mx = fmaxf(mx, lses[rec_of(j) * p.nq]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (mx > -CUDART_INF_F) {
             float z = 0.f;
-            for (int j = lane; j < n_rec; j += 32) z += __expf(lses[rec_of(j) * p.nq] - mx);  // exp(-inf) = 0: an empty slice
-            constexpr int U = 4;
-            for (int j0 = warp; j0 < n_rec; j0 += NW * U) {
-                float wu[U];
-                float4 ov[U][VPL / 4];
+#pragma unroll
+            for (int i = 0; i < MINE; ++i) z += __expf(mine[i] - mx);  // exp(-inf) = 0: an empty slice
+            for (int j = lane + 32 * MINE; j < n_rec; j += 32) z += __expf(lses[rec_of(j) * p.nq] - mx);
+            for (int j0 = team; j0 < n_rec; j0 += TEAMS * U) {
+                if (j0 != team) load_batch(j0);
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int j = j0 + u * NW;
-                    const long long rec = rec_of(j < n_rec ? j : j0);
-                    wu[u] = j < n_rec ? lses[rec * p.nq] : -CUDART_INF_F;
-                    const float* src = p.part_o + (rec * p.nq + h) * HD + lane * VPL;
-#pragma unroll
-                    for (int i = 0; i < VPL / 4; ++i) ov[u][i] = *reinterpret_cast<const float4*>(src + 4 * i);
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
+                    if (wu[u] == -CUDART_INF_F) continue;  // an empty slice's record may hold anything
                     const float w = __expf(wu[u] - mx);
 #pragma unroll
                     for (int i = 0; i < VPL / 4; ++i) {
@@ -659,17 +746,18 @@ __global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const 
         }
     }
 #pragma unroll
-    for (int j = 0; j < VPL; ++j) acc_sm[warp * HD + lane * VPL + j] = acc[j];
-    __syncthreads();
+    for (int j = 0; j < VPL; ++j) acc_sm[team * COLS + tl * VPL + j] = acc[j];
+    if (__syncthreads_or(fault != 0u)) return;  // a status is set: no work
     const long long row = (long long)b * p.nq + h;
-    if (p.out_lse && threadIdx.x == 0) p.out_lse[row] = lse;
-    const int d = threadIdx.x * 2;
+    if (p.out_lse && threadIdx.x == 0 && col0 == 0) p.out_lse[row] = lse;
+    const int d = col0 + threadIdx.x * 2;
     float a0 = 0.f, a1 = 0.f;
-    if (threadIdx.x < HD / 2) {
+    if (threadIdx.x < COLS / 2) {
 #pragma unroll
-        for (int w = 0; w < MERGE_THREADS / 32; ++w) {
-            a0 += acc_sm[w * HD + d];
-            a1 += acc_sm[w * HD + d + 1];
+        for (int w = 0; w < TEAMS; ++w) {
+            const float2 v = *reinterpret_cast<const float2*>(acc_sm + w * COLS + threadIdx.x * 2);
+            a0 += v.x;
+            a1 += v.y;
         }
         a0 *= inv;
         a1 *= inv;
@@ -741,7 +829,7 @@ __global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const 
         a0 = b0;
         a1 = b1;
     }
-    if (threadIdx.x < HD / 2) {
+    if (threadIdx.x < COLS / 2) {
         if (p.out) {
             const long long eoff = (long long)b * p.o_stride_b + (long long)h * HD + d;
             if (p.gate) {

@@ -297,3 +297,28 @@ def test_one_launch_form(ops, B, nq, nkv, hd, lens):
         assert_close(o32[b], wf[0], f"seq {b} f32", rel_tol=3e-3, abs_tol=5e-3)
         assert_close(out[b], wgb[0].float(), f"seq {b} gated")
         assert torch.allclose(lse[b].cpu(), wl[0], atol=2e-3)
+
+
+@pytest.mark.parametrize("B,nq,nkv,hd,length,ctas", [
+    (1, 24, 4, 256, 6100, 148),   # few rows: 64 columns of a row per merge block, every share one record
+    (1, 6, 2, 128, 9000, 600),    # more records of a row than a lane of the merge block keeps of their log-sum-exps
+    (2, 16, 16, 128, 700, 64),    # two slices per record at a sequence's end
+    (1, 32, 2, 128, 3000, 40),    # sixteen query heads per KV head
+    (40, 16, 8, 256, 130, 148),   # many rows: whole rows per block
+])
+def test_lengths_known_to_the_host_and_merge_blocks(ops, B, nq, nkv, hd, length, ctas):
+    """A length the host states gives what the same length on the device gives, bit for bit: shares found before or
+    after the wait for the kernels in front, one launch or two; all against the oracle."""
+    q, k, v, g = seeded_bf16(B, nq, hd, seed=1), seeded_bf16(B, length, nkv, hd, seed=2), seeded_bf16(B, length, nkv, hd, seed=3), seeded_bf16(B, nq, hd, seed=4)
+    dev = [t.cuda() for t in (q, k, v)]
+    kl = torch.full((B,), length, dtype=torch.int32, device="cuda")
+    for n in (0, ctas):
+        on_host = ops.sdpa_decode(*dev, scale=hd ** -0.5, gate=g.cuda(), num_ctas=n, return_partial=True)
+        on_device = ops.sdpa_decode(*dev, scale=hd ** -0.5, kv_len=kl, gate=g.cuda(), num_ctas=n, return_partial=True)
+        assert all(torch.equal(a, b) for a, b in zip(on_host, on_device))
+        for b in range(0, B, max(1, B // 4)):
+            wf, _, wl = oracle_decode(q[b], k[b], v[b], hd ** -0.5)
+            _, wgb, _ = oracle_decode(q[b], k[b], v[b], hd ** -0.5, gate=g[b])
+            assert_close(on_host[1][b], wf[0], f"seq {b} f32", rel_tol=3e-3, abs_tol=5e-3)
+            assert_close(on_host[0][b], wgb[0].float(), f"seq {b} gated")
+            assert torch.allclose(on_host[2][b].cpu(), wl[0], atol=2e-3)
