@@ -546,12 +546,13 @@ static bool size_decode_cta(int hd, int nkv_cta, int batch, int extra, int smem_
     return stages >= 2;
 }
 
-// One launch or two?  A cluster of up to eight CTAs per sequence and group of heads finishes alone: 6 us plus the time its
-// CTAs take for their part of the longest sequence, at the 58 GB/s one CTA pulls at head dim 256 (four consumer warps) and
-// 93 at 128 (eight), or their share of the memory's rate.  Equal shares over all SMs read the total at 6.9 TB/s,
-// but cost 9 us and 0.12 us per sequence for the second launch and the records.  (Measured over
-// batches of 1 to 64 and lengths of 32 to 8192 for four head layouts; one token over 513 keys, 24/4 heads: 11.8 -> 7.6 us,
-// 64 sequences of 512 keys, 16/2 heads: 21.7 -> 10.3.)  Lengths on the device are not known here: the longest sequence is
+// One launch or two?  A cluster of up to eight CTAs per sequence and group of heads finishes alone: 5.2 us plus the time its
+// CTAs take for their part of the longest sequence, at the 93 GB/s one CTA pulls at head dim 256 (four consumer warps) and
+// 105 at 128 (eight), or their share of what so many CTAs get out of the memory (less when a CTA's heads fill a row of
+// 2 KB: one slice, as few warps as heads).  Equal shares over all SMs read the total at 7 TB/s, but cost 7.2 us (8 with the
+// lengths on the device) and 0.1 us per sequence for the second launch and the records.  (Measured over
+// batches of 1 to 64 and lengths of 64 to 8192 for five head layouts: one token over 513 keys, 24/4 heads: 6.7 and 6.0 us,
+// 64 sequences of 512 keys, 16/2 heads: 17.8 and 9.9.)  Lengths on the device are not known here: the longest sequence is
 // taken to be as long as its bound says, or twice the mean of a packed cache, the others half of that.
 static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceState& ds, int nkv_cta, DecodePlan* plan) {
     if (p->num_ctas != 0 || p->xchg_world > 1 || p->kv_rows_total == 0 || p->batch > 1024) return;
@@ -569,11 +570,12 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
             longest = 2.0 * (double)p->kv_rows_total / p->batch;
         total = longest * (0.5 * p->batch + 0.5);
     }
-    double rate = p->hd == 256 ? 58e3 : 93e3;
-    const double even = 6.9e6 / ((double)p->batch * (p->nkv / heads) * csize);
+    double rate = p->hd == 256 ? 93e3 : 105e3;
+    const double ctas = (double)p->batch * (p->nkv / heads) * csize;
+    const double even = (heads * p->hd >= 1024 ? 6.0e6 : 6.9e6 - 6e3 * (ds.sm_count - ctas)) / ctas;
     if (rate > even) rate = even;
-    const double t_cluster = 6.0 + longest / csize * heads * p->hd * 4.0 / rate;
-    const double t_shares = 9.0 + 0.12 * p->batch + total * p->nkv * p->hd * 4.0 / 6.9e6;
+    const double t_cluster = 5.2 + longest / csize * heads * p->hd * 4.0 / rate;
+    const double t_shares = (p->kv_len ? 8.0 : 7.2) + 0.1 * p->batch + total * p->nkv * p->hd * 4.0 / 7.0e6;
     if (t_cluster > t_shares) return;
     DecodePlan one = *plan;
     // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where
