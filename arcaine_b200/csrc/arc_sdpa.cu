@@ -132,6 +132,7 @@ static int device_state(DeviceState** out) {
             ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<true, false>, PairCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<false, true>, PairCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<true, true>, PairCfg::SMEM_BYTES));
+            ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<false, false, true>, PairCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, false, false>, PrefillCfg<128>::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, false, true>, PrefillCfg<128>::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, true, true>, PrefillCfg<128>::SMEM_BYTES));
@@ -362,18 +363,19 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     kp.out_lse = p->out_lse;
     kp.part_o = plan.splits > 1 ? static_cast<float*>(p->workspace) : nullptr;
     kp.part_lse = kp.part_o ? kp.part_o + (size_t)plan.splits * plan.rows * HD : nullptr;
-    // CTA pairs (prefill_wide_sm100.cuh) look vision blocks up themselves; the one-tile kernel wants the span end of every
-    // row (a few microseconds instead of a (seq, kv_len) f32 mask).
+    // CTA pairs (prefill_wide_sm100.cuh) and the two-tile kernel look vision blocks up themselves; the one-tile kernel wants
+    // the span end of every row (a few microseconds instead of a (seq, kv_len) f32 mask).
     const bool wide = HD == 256 && (plan.splits == 1 || p->mask_type != ARC_MASK_EXPLICIT);
-    if (p->block_ids && wide) {
-        kp.ids = p->block_ids + p->block_ids_offset;
-    } else if (p->block_ids) {
+    if (p->block_ids) kp.ids = p->block_ids + p->block_ids_offset;
+    auto find_spans = [&]() -> int {
+        if (!kp.ids) return ARC_OK;
         int* vis = reinterpret_cast<int*>(static_cast<unsigned char*>(p->workspace) + plan.split_bytes);
         ARC_CUDA(launch_dependent(vision_span_kernel, dim3((unsigned)((p->seq + 255) / 256)), dim3(256), 0, stream, 1, p->block_ids,
                                   p->block_ids_offset, p->kv_len - p->seq, p->seq, p->kv_len, vis));
         g_launches.fetch_add(1, std::memory_order_relaxed);
         kp.vis_hi = vis;
-    }
+        return ARC_OK;
+    };
     kp.fault = ds->fault;
     kp.batch = p->batch;
     kp.seq = p->seq;
@@ -394,7 +396,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
 
     // Head dim 128: two query tiles per CTA (prefill_pair_sm100.cuh) when that is the faster way to cover
     // the tiles.  ARC_SDPA_PREFILL_KERNEL=single|pair overrides the choice (for A/B measurements).
-    if (HD == 128 && plan.splits == 1 && !(kp.mask_type == 1 && kp.mask != nullptr) && kp.vis_hi == nullptr) {
+    if (HD == 128 && plan.splits == 1 && !(kp.mask_type == 1 && kp.mask != nullptr) && !(kp.ids && (kp.gate || kp.n_copies > 0))) {
         static const int forced = [] {
             const char* e = std::getenv("ARC_SDPA_PREFILL_KERNEL");
             if (!e) return 0;
@@ -415,10 +417,12 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         // one as SMs free up) takes them, and no SM runs a whole pair while the others idle.  A single tile
         // costs about one tile of the one-tile kernel.
         const long long full_waves = pair_tiles / sms, left = pair_tiles - full_waves * sms;
-        const bool cut_tail = head_pair && full_waves > 0 && left > 0 && 2 * left <= sms;
+        const bool cut_tail = !kp.ids && head_pair && full_waves > 0 && left > 0 && 2 * left <= sms;
         const double cost_pair = cut_tail ? 1.7 * (double)full_waves + 1.05 : 1.7 * (double)((pair_tiles + sms - 1) / sms);
         const double cost_single = (double)((single_tiles + sms - 1) / sms);
-        const bool use_pair = forced == 2 || (forced == 0 && cost_pair <= cost_single);
+        // (Vision blocks: the one-tile kernel also needs a launch for the span ends, and takes an SM twice as long per wave:
+        // 1257 tokens of 16 heads 43.7 us, two tiles at a time 24.6.)
+        const bool use_pair = forced == 2 || (forced == 0 && (kp.ids || cost_pair <= cost_single));
         if (use_pair) {
             if (pair_tiles > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
             kp.head_pair = head_pair ? 1 : 0;
@@ -428,7 +432,8 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
             kp.total_tiles = (int)pair_units;
             const unsigned ctas = (unsigned)(pair_units < ds->sm_count ? pair_units : ds->sm_count);
             if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
-            auto kernel = kp.n_copies > 0 ? (kp.gate ? sdpa_prefill_pair_kernel<true, true> : sdpa_prefill_pair_kernel<false, true>)
+            auto kernel = kp.ids          ? sdpa_prefill_pair_kernel<false, false, true>
+                          : kp.n_copies > 0 ? (kp.gate ? sdpa_prefill_pair_kernel<true, true> : sdpa_prefill_pair_kernel<false, true>)
                                           : (kp.gate ? sdpa_prefill_pair_kernel<true, false> : sdpa_prefill_pair_kernel<false, false>);
             ARC_CUDA(launch_dependent(kernel, dim3(ctas), dim3(PairCfg::THREADS), (size_t)PairCfg::SMEM_BYTES, stream, 1, tq, tk, tv, to, tg, kp));
             g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -451,6 +456,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         }
     }
 
+    if (!wide && (rc = find_spans()) != ARC_OK) return rc;
     // Head dim 256, whole tiles, no additive mask: pairs of CTAs (prefill_wide_sm100.cuh) take 2300-2500 clk per key block
     // and pair of tiles where a CTA on its own takes 3700 per tile.
     const bool masked = kp.mask_type == 1 && kp.mask != nullptr;
@@ -546,9 +552,9 @@ static bool size_decode_cta(int hd, int nkv_cta, int batch, int extra, int smem_
     return stages >= 2;
 }
 
-// One launch or two?  A cluster of up to eight CTAs per sequence and group of heads finishes alone: 5.2 us plus the time its
-// CTAs take for their part of the longest sequence, at the 93 GB/s one CTA pulls at head dim 256 (four consumer warps) and
-// 105 at 128 (eight), or their share of what so many CTAs get out of the memory (less when a CTA's heads fill a row of
+// One launch or two?  A cluster of up to eight CTAs per sequence and group of heads finishes alone: 5.2 us and the longer of
+// two times: of the CTAs with the longest sequence, at the 93 GB/s one CTA pulls at head dim 256 (four consumer warps) and
+// 105 at 128 (eight), and of all bytes at what so many CTAs get out of the memory (less when a CTA's heads fill a row of
 // 2 KB: one slice, as few warps as heads).  Equal shares over all SMs read the total at 7 TB/s, but cost 7.2 us (8 with the
 // lengths on the device) and 0.1 us per sequence for the second launch and the records.  (Measured over
 // batches of 1 to 64 and lengths of 64 to 8192 for five head layouts: one token over 513 keys, 24/4 heads: 6.7 and 6.0 us,
@@ -570,11 +576,10 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
             longest = 2.0 * (double)p->kv_rows_total / p->batch;
         total = longest * (0.5 * p->batch + 0.5);
     }
-    double rate = p->hd == 256 ? 93e3 : 105e3;
     const double ctas = (double)p->batch * (p->nkv / heads) * csize;
-    const double even = (heads * p->hd >= 1024 ? 6.0e6 : 6.9e6 - 6e3 * (ds.sm_count - ctas)) / ctas;
-    if (rate > even) rate = even;
-    const double t_cluster = 5.2 + longest / csize * heads * p->hd * 4.0 / rate;
+    const double all = heads * p->hd >= 1024 ? 6.0e6 : 6.9e6 - 6e3 * (ds.sm_count - ctas);
+    const double t_longest = longest / csize * heads * p->hd * 4.0 / (p->hd == 256 ? 93e3 : 105e3);
+    const double t_cluster = 5.2 + std::max(t_longest, total * p->nkv * p->hd * 4.0 / all);
     const double t_shares = (p->kv_len ? 8.0 : 7.2) + 0.1 * p->batch + total * p->nkv * p->hd * 4.0 / 7.0e6;
     if (t_cluster > t_shares) return;
     DecodePlan one = *plan;

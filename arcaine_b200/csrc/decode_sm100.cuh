@@ -634,8 +634,10 @@ constexpr int MERGE_THREADS = 256;
 // COLS: columns of the row a block takes.  All of them, unless the rows are so few that most SMs would idle: one token of
 // 24 heads over 6760 keys has 106 records in each of 24 rows, 100 KB a block, and took 7.5 us from the decode kernel's
 // end; 64 columns a block, every load of a batch in flight with the log-sum-exps, take 3.9.
+// (Whole rows of 256: four blocks per SM, 64 sequences of 24 heads are 1536 of them.  At 128 columns the registers that
+// would take are worth more: 12 sequences of 16 heads 14.8 us, with four blocks per SM 15.6.)
 template <int HD, bool XCHG, int COLS>
-__global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const DecodeMergeParams p) {
+__global__ void __launch_bounds__(MERGE_THREADS, XCHG || COLS < 256 ? 1 : 4) sdpa_decode_merge_kernel(const DecodeMergeParams p) {
     // One row of output per block; what the block does before its one barrier every warp does for itself — where the
     // row's records are, their maximum and weights — because that is a handful of loads, while three block-wide
     // reductions and a list in shared memory made this kernel's tail 5 us.
@@ -693,7 +695,7 @@ __global__ void __launch_bounds__(MERGE_THREADS) sdpa_decode_merge_kernel(const 
         // The records are dealt to the teams in turn, U at a time; a lane owns VPL consecutive output values.  Always the
         // same order of additions.  The first batch and all log-sum-exps (eight a lane; more is rare) are asked for
         // together: one trip to L2.
-        constexpr int U = 4, MINE = 8;
+        constexpr int U = VPL == 8 ? 2 : 4, MINE = 8;
         float wu[U];
         float4 ov[U][VPL / 4];
         auto load_batch = [&](int j0) {

@@ -91,14 +91,55 @@ struct PairWork {
     __device__ __forceinline__ bool live_of(int s) const { return s ? live[1] : live[0]; }
 };
 
-// Key blocks [lo, hi) a 128-row tile starting at token qs can see.
+// ---------------------------------------------------------------------------
+// Vision blocks (a query inside a block of equal non-negative ids also sees the block's later keys).  The ends are looked
+// up where they are needed: a launch of its own for one end per row took 4.5 us in front of a kernel of 20.
+// ---------------------------------------------------------------------------
+// First key after `key` that does not carry `id`.  Whole warps, 128 keys a step.
+__device__ __forceinline__ int run_end(const int* ids, int kv_len, int key, int id) {
+    const int lane = threadIdx.x & 31;
+    for (int k0 = key + 1;; k0 += 128) {
+        bool other[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) other[i] = k0 + 32 * i + lane >= kv_len || ids[k0 + 32 * i + lane] != id;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t found = __ballot_sync(0xffffffffu, other[i]);
+            if (found) return k0 + 32 * i + __ffs(found) - 1;
+        }
+    }
+}
+
+// First key the row at key position `self` does not see.  Same position in every lane.
+__device__ __forceinline__ int vision_end(const PrefillParams& p, int self) {
+    const int plain = min(max(self + 1, 0), p.kv_len);
+    if (self < 0 || self >= p.kv_len) return plain;
+    const int id = p.ids[self];
+    return id >= 0 ? run_end(p.ids, p.kv_len, self, id) : plain;
+}
+
+// The same for a warp's 32 consecutive rows, one per lane (row: t < seq).
+__device__ __forceinline__ int vision_ends(const PrefillParams& p, int self, bool row) {
+    const int lane = threadIdx.x & 31;
+    const int id = row && self >= 0 && self < p.kv_len ? p.ids[self] : -1;
+    const int next_id = __shfl_down_sync(0xffffffffu, id, 1);  // (all lanes take part; lane 31 does not use it)
+    const uint32_t breaks = __ballot_sync(0xffffffffu, lane < 31 && id != next_id);
+    const int last_id = __shfl_sync(0xffffffffu, id, 31), last = __shfl_sync(0xffffffffu, self, 31);
+    const int end = last_id >= 0 ? run_end(p.ids, p.kv_len, last, last_id) : 0;  // of the block that leaves the warp's rows
+    if (id < 0) return min(max(self + 1, 0), p.kv_len);
+    const uint32_t ahead = breaks >> lane;
+    return ahead ? self + __ffs(ahead) : end;
+}
+
+// Key blocks [lo, hi) a 128-row tile starting at token qs can see.  VISION: whole warps.
+template <bool VISION>
 __device__ __forceinline__ void tile_blocks(const PrefillParams& p, int qs, int& blk_lo, int& blk_hi) {
     const int off = p.kv_len - p.seq;
     blk_lo = 0;
     blk_hi = (p.kv_len + PairCfg::BN - 1) / PairCfg::BN;
     if (p.mask_type == 3) {
         const int q_last = min(qs + PairCfg::BM - 1, p.seq - 1);
-        const int last_key = min(p.kv_len - 1, q_last + off);
+        const int last_key = VISION ? vision_end(p, q_last + off) - 1 : min(p.kv_len - 1, q_last + off);  // (monotone in the row)
         blk_hi = last_key >= 0 ? last_key / PairCfg::BN + 1 : 0;
         if (p.window > 0 && p.window != 0x7fffffff) blk_lo = max(0, qs + off - p.window + 1) / PairCfg::BN;
     }
@@ -107,6 +148,7 @@ __device__ __forceinline__ void tile_blocks(const PrefillParams& p, int qs, int&
 
 // Every role runs this once per unit, from code that has long left the instruction caches by
 // then, so it is kept short: one division at most, and nothing computed twice.
+template <bool VISION>
 __device__ __forceinline__ PairWork decode_pair(const PrefillParams& p, const TileCursor& cur) {
     PairWork t;
     t.b = cur.z;
@@ -116,7 +158,7 @@ __device__ __forceinline__ PairWork decode_pair(const PrefillParams& p, const Ti
         t.q0[0] = t.q0[1] = cur.qt * PairCfg::BM;
         t.kvh = p.group_shift >= 0 ? (t.h[0] >> p.group_shift) : t.h[0] / p.group;
         t.live[0] = t.live[1] = true;  // the tile list only holds tiles with rows
-        tile_blocks(p, t.q0[0], t.lo[0], t.hi[0]);
+        tile_blocks<VISION>(p, t.q0[0], t.lo[0], t.hi[0]);
         t.lo[1] = t.ulo = t.lo[0];
         t.hi[1] = t.uhi = t.hi[0];
     } else {
@@ -126,9 +168,9 @@ __device__ __forceinline__ PairWork decode_pair(const PrefillParams& p, const Ti
         t.kvh = p.group_shift >= 0 ? (cur.h >> p.group_shift) : cur.h / p.group;
         t.live[0] = true;
         t.live[1] = t.q0[1] < p.seq;
-        tile_blocks(p, t.q0[0], t.lo[0], t.hi[0]);
+        tile_blocks<VISION>(p, t.q0[0], t.lo[0], t.hi[0]);
         t.lo[1] = t.hi[1] = 0;
-        if (t.live[1]) tile_blocks(p, t.q0[1], t.lo[1], t.hi[1]);
+        if (t.live[1]) tile_blocks<VISION>(p, t.q0[1], t.lo[1], t.hi[1]);
         t.ulo = 0x7fffffff;
         t.uhi = 0;
 #pragma unroll
@@ -275,7 +317,8 @@ __device__ __forceinline__ void stage_turn(const OutStage& s, const void* tm_out
 
 // The gated epilogue and the one that also stores copies of the output are instances of their own: code the
 // common kernel does not carry.
-template <bool GATE, bool COPIES>
+// VISION: causal with vision blocks (p.ids).
+template <bool GATE, bool COPIES, bool VISION = false>
 __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     sdpa_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
@@ -381,7 +424,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             PairWork last{};  // unit and index of the block requested last
             int last_j = 0;
             for (; ok && cur.w < total_tiles; cur.advance(p)) {
-                const PairWork pw = decode_pair(p, cur);
+                const PairWork pw = decode_pair<VISION>(p, cur);
                 for (int j = pw.ulo; ok && j < pw.uhi; ++j, ++r) {
                     if (r == 0) {
                         if (lane == 0) mbar_arrive_expect_tx(k_first, C::TILE_BYTES);
@@ -422,35 +465,37 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             // -------------------------------------------------------------- TMA producer of Q
             // A thread of its own: the next unit's Q tiles are requested the moment the current tiles'
             // last scores are out, whatever the K / V producer is waiting for at that time.
-            if (lane == 0) {
-                prefetch_tensormap(&tm_q);
+            if (VISION || lane == 0) {  // (the look-up of vision blocks takes the whole warp)
+                if (lane == 0) prefetch_tensormap(&tm_q);
                 int tq0 = 0, tq1 = 0;  // tiles with key blocks loaded so far, per pipeline
                 bool ok = true;
                 TileCursor cur = *cursor;
                 for (; ok && cur.w < total_tiles; cur.advance(p)) {
-                    const PairWork pw = decode_pair(p, cur);
+                    const PairWork pw = decode_pair<VISION>(p, cur);
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
                         if (pw.hi[s] == pw.lo[s]) continue;
                         int& tq = s ? tq1 : tq0;
-                        if (tq > 0 && !mbar_wait<1>(&q_empty[s], (tq - 1) & 1)) {
-                            report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u + s);
+                        if (tq > 0 && !(VISION ? mbar_wait_inline(&q_empty[s], (tq - 1) & 1) : mbar_wait<1>(&q_empty[s], (tq - 1) & 1))) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u + s);
                             ok = false;
                             break;
                         }
-                        mbar_arrive_expect_tx(&q_full[s], C::TILE_BYTES);
+                        if (lane == 0) {
+                            mbar_arrive_expect_tx(&q_full[s], C::TILE_BYTES);
 #pragma unroll
-                        for (int c = 0; c < C::CH; ++c)
-                            tma_load_4d(sQ + s * C::TILE_BYTES + c * C::CHUNK_BYTES, &tm_q, &q_full[s], c * 64, pw.h[s],
-                                        pw.q0[s], pw.b);
+                            for (int c = 0; c < C::CH; ++c)
+                                tma_load_4d(sQ + s * C::TILE_BYTES + c * C::CHUNK_BYTES, &tm_q, &q_full[s], c * 64, pw.h[s],
+                                            pw.q0[s], pw.b);
+                        }
                         ++tq;
                     }
                     // The unit after this one: its Q rows (one 256-byte piece per token, far apart in
                     // memory) are asked into L2 now, a whole unit ahead of the load that needs them.
                     TileCursor nx = cur;
                     nx.advance(p);
-                    if (ok && nx.w < total_tiles) {
-                        const PairWork pn = decode_pair(p, nx);
+                    if (ok && !VISION && nx.w < total_tiles) {
+                        const PairWork pn = decode_pair<false>(p, nx);
 #pragma unroll
                         for (int s = 0; s < 2; ++s) {
                             if (pn.hi[s] == pn.lo[s]) continue;
@@ -510,7 +555,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             TileCursor cur = *cursor;
             auto next_unit = [&](PairWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
                 for (; cur.w < total_tiles; cur.advance(p)) {
-                    w = decode_pair(p, cur);
+                    w = decode_pair<VISION>(p, cur);
                     if (w.uhi > w.ulo) {
                         cur.advance(p);
                         return true;
@@ -603,7 +648,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0};
         TileCursor cur = *cursor;
         for (; ok && cur.w < total_tiles; cur.advance(p)) {
-            const PairWork pw = decode_pair(p, cur);
+            const PairWork pw = decode_pair<VISION>(p, cur);
 #pragma unroll 1
             for (int s = 0; s < 2 && ok; ++s) {
                 const int t0 = pw.q0_of(s) + quarter * 32, t = t0 + lane, h = pw.h_of(s);
@@ -695,7 +740,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
 
         TileCursor cur = *cursor;
         for (; ok && cur.w < total_tiles; cur.advance(p)) {
-            const PairWork pw = decode_pair(p, cur);
+            const PairWork pw = decode_pair<VISION>(p, cur);
             if (pw.uhi == pw.ulo) continue;
             const int t = pw.q0_of(s) + r;
             const int lo = pw.lo_of(s), hi = pw.hi_of(s);
@@ -703,6 +748,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             if (causal) {
                 const int diag = t + off;
                 row_hi = min(max(diag + 1, 0), p.kv_len);
+                if (VISION) row_hi = vision_ends(p, diag, t < p.seq);
                 if (windowed) row_lo = max(0, diag - p.window + 1);
                 if (row_lo > row_hi) row_lo = row_hi;
             }

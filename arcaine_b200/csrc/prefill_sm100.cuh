@@ -62,7 +62,7 @@ struct PrefillParams {
     const uint4* mask_bits;      // [row tile][key block][row]: one bit per key, set where the mask is 0
     int mask_blocks;
     int fold;        // prefill_wide_sm100.cuh: the parts of a unit are the pairs of one cluster, which folds them itself
-    const int* ids;  // prefill_wide_sm100.cuh: vision-block ids, ids[j] that of key j (instead of vis_hi)
+    const int* ids;  // vision-block ids, ids[j] that of key j (prefill_wide_sm100.cuh and prefill_pair_sm100.cuh, instead of vis_hi)
 };
 
 // One CTA per SM, persistent: it takes tiles (128 query tokens of one query head) round-robin

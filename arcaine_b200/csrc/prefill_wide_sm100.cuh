@@ -141,46 +141,6 @@ __device__ __forceinline__ void add_mask_values(uint32_t tS, const float* mask_r
     tmem_wait_st();
 }
 
-// ---------------------------------------------------------------------------
-// Vision blocks (a query inside a block of equal non-negative ids also sees the block's later keys).  The ends are looked
-// up where they are needed: a launch of its own for one end per row took 4.5 us in front of a kernel of 20.
-// ---------------------------------------------------------------------------
-// First key after `key` that does not carry `id`.  Whole warps, 128 keys a step.
-__device__ __forceinline__ int run_end(const int* ids, int kv_len, int key, int id) {
-    const int lane = threadIdx.x & 31;
-    for (int k0 = key + 1;; k0 += 128) {
-        bool other[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) other[i] = k0 + 32 * i + lane >= kv_len || ids[k0 + 32 * i + lane] != id;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t found = __ballot_sync(0xffffffffu, other[i]);
-            if (found) return k0 + 32 * i + __ffs(found) - 1;
-        }
-    }
-}
-
-// First key the row at key position `self` does not see.  Same position in every lane.
-__device__ __forceinline__ int vision_end(const PrefillParams& p, int self) {
-    const int plain = min(max(self + 1, 0), p.kv_len);
-    if (self < 0 || self >= p.kv_len) return plain;
-    const int id = p.ids[self];
-    return id >= 0 ? run_end(p.ids, p.kv_len, self, id) : plain;
-}
-
-// The same for a warp's 32 consecutive rows, one per lane (row: t < seq).
-__device__ __forceinline__ int vision_ends(const PrefillParams& p, int self, bool row) {
-    const int lane = threadIdx.x & 31;
-    const int id = row && self >= 0 && self < p.kv_len ? p.ids[self] : -1;
-    const int next_id = __shfl_down_sync(0xffffffffu, id, 1);  // (all lanes take part; lane 31 does not use it)
-    const uint32_t breaks = __ballot_sync(0xffffffffu, lane < 31 && id != next_id);
-    const int last_id = __shfl_sync(0xffffffffu, id, 31), last = __shfl_sync(0xffffffffu, self, 31);
-    const int end = last_id >= 0 ? run_end(p.ids, p.kv_len, last, last_id) : 0;  // of the block that leaves the warp's rows
-    if (id < 0) return min(max(self + 1, 0), p.kv_len);
-    const uint32_t ahead = breaks >> lane;
-    return ahead ? self + __ffs(ahead) : end;
-}
-
 __device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first, int q_last, int& lo, int& hi) {
     const int off = p.kv_len - p.seq;
     lo = 0;

@@ -331,3 +331,23 @@ def test_few_keys_in_the_first_block_repeat_bit_for_bit(ops, window):
     assert_close(first[0], want, f"window {window}")
     for _ in range(40):
         assert torch.equal(first, run())
+
+
+@pytest.mark.parametrize("nq,nkv", [(8, 4), (6, 2)])  # two heads of one tile, two tiles of one head
+def test_vision_blocks_two_tiles_per_cta(ops, nq, nkv):
+    """Block ids looked up in the kernel against the additive buffer of the same rule: blocks of one token, across tiles, up
+    to the last key; with a window that hides a block's first keys; the last tile ragged."""
+    seq, kv, hd = 1150, 1250, 128
+    ids = torch.full((kv,), -1, dtype=torch.int32)
+    for i, (a, b) in enumerate([(30, 31), (31, 100), (140, 160), (227, 260), (300, 711), (840, 1096), (1200, 1250)]):
+        ids[a:b] = i
+    q, k, v = (seeded_bf16(n, h, hd, seed=50 + h).cuda() for n, h in ((seq, nq), (kv, nkv), (kv, nkv)))
+    for window in (oracle.INT_MAX, 200):
+        mask = ops.fill_causal_mask_with_block_ids(ids.cuda(), seq, kv, kv - seq, window)
+        want, want_lse = ops.sdpa_prefill(q, k, v, scale=0.09, mask_type=ops.MASK_EXPLICIT, mask=mask, return_lse=True, num_splits=1)
+        before = ops.launch_count()
+        got, lse = ops.sdpa_prefill(q, k, v, scale=0.09, mask_type=ops.MASK_CAUSAL, window=window, block_ids=ids.cuda(), return_lse=True, num_splits=1)
+        assert ops.launch_count() - before == 1
+        # the same visible keys; blocks may be skipped in one form and fully masked in the other
+        assert_close(got, want.float(), f"window {window}", rel_tol=4e-3, abs_tol=1.6e-2)
+        assert torch.allclose(lse, want_lse, atol=2e-3)
