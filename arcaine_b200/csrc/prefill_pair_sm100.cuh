@@ -33,7 +33,7 @@
 //     the scores in a rolled loop would be smaller still but measured 2-5 % slower.)
 //
 // Lazy rescaling, bounded waits and the device status word are as in the single-tile kernel (prefill_sm100.cuh),
-// which keeps head dim 256, additive masks and key-range splits.
+// which keeps additive masks, key-range splits and small problems.
 #pragma once
 #include "prefill_sm100.cuh"
 

@@ -144,13 +144,6 @@ __device__ __forceinline__ void store_copies_bf16x16(const unsigned long long* c
     for (int c = 0; c < n; ++c) store_bf16x16(reinterpret_cast<uint16_t*>(copies[c]) + off, w);
 }
 
-// bf16(attention) * sigmoid(gate), the rounding order of mul_sigmoid_inplace after a bf16 attention
-// output (src/modeling/qwen3_5_moe/kernels.hpp:80-88).
-__device__ __forceinline__ float sigmoid_gate_bits(float attn, uint16_t gate_bits) {
-    const float g = bf16_bits_to_f32(gate_bits);
-    return bf16_round(attn) * sigmoid(g);
-}
-
 // Maximum of one 32-column chunk, folded into four independent running maxima.
 template <int MODE>
 __device__ __forceinline__ void chunk_max(const uint32_t (&v)[32], float (&mx)[4], float sl, int key0,

@@ -37,12 +37,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ uint32_t lane_id() {
-    uint32_t l;
-    asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
-    return l;
-}
-
 // ---------------------------------------------------------------------------
 // Programmatic dependent launch: a kernel launched with the programmatic-serialization attribute
 // may start (be scheduled, run its prologue) while the kernel before it in the stream is still
@@ -139,19 +133,6 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parit
     return ok != 0;
 }
 
-// Non-blocking: has the phase with the given parity completed?
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
 // Wait for the phase with the given parity to complete.  Gives up after
 // ~`limit_cycles` SM clocks (default: about a second) and returns false; the
 // caller records a fault and unwinds.
@@ -218,8 +199,6 @@ __device__ __forceinline__ void cluster_sync_all() {
 // Ask a line of global memory into L2 (no register, no wait).
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-__device__ __forceinline__ void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
-
 // Address of this CTA's shared-memory location `saddr` in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
     uint32_t r;
@@ -235,12 +214,6 @@ __device__ __forceinline__ void st_cluster_f32x4(uint32_t addr, float4 v) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
-// Arrive on an mbarrier of another CTA of the cluster (address from map_to_cta); release at cluster
-// scope, so this thread's earlier shared-memory writes are visible to whoever acquires the phase.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
-}
-
 // One arrival for a converged warp, without release at cluster scope: for arrivals that announce tensor-memory accesses
 // only (completed by tcgen05.wait and ordered by tcgen05.fence).  The release costs the arriving warp about 600 clk.
 __device__ __forceinline__ void mbar_arrive_remote_warp(uint32_t remote_bar) {
@@ -249,23 +222,6 @@ __device__ __forceinline__ void mbar_arrive_remote_warp(uint32_t remote_bar) {
         "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
         "@q mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(remote_bar)
         : "memory");
-}
-
-// Bounded wait on a local mbarrier whose arrivals come from the whole cluster (acquire at cluster scope).
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, long long limit_cycles = 2000000000LL) {
-    const long long t0 = clock64();
-    for (;;) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity), "r"(200000u)
-            : "memory");
-        if (ok) return true;
-        if (clock64() - t0 > limit_cycles) return false;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -340,16 +296,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, ui
         : "memory");
 }
 
-// Plain 1-D bulk copy global -> shared (both 16-byte aligned, size % 16 == 0).
-__device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes,
-                                             uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(smem_dst)),
-        "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
 // ---------------------------------------------------------------------------
 // tcgen05: tensor memory + 5th-generation MMA (single-CTA group)
 // ---------------------------------------------------------------------------
@@ -399,28 +345,6 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, bool b_mn_m
            | (1u << 10)                    // B format bf16
            | ((b_mn_major ? 1u : 0u) << 16)  // B major
            | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
-}
-
-// D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                        uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                        uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
 }
 
 // Forms for a whole converged warp: every lane executes the statement with identical operands and one elected lane
@@ -482,14 +406,6 @@ __device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
         "elect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
         : "memory");
-}
-
-// Arrive on an mbarrier once every tcgen05 operation issued so far by this
-// thread has completed (implies tcgen05.fence::before_thread_sync).
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
 }
 
 __device__ __forceinline__ void tmem_wait_ld() {
