@@ -59,9 +59,13 @@ struct WideWork {
 // bit per key and a class per 32 rows x 128 keys.  The attention then skips key blocks nobody sees, tests nothing in
 // those everybody sees and selects by bits in the others; only where other values occur does it read the mask itself.
 // ---------------------------------------------------------------------------
-constexpr uint32_t MASK_SEEN = 1;     // some key is not -inf
-constexpr uint32_t MASK_HIDDEN = 2;   // some key is -inf or past the end
-constexpr uint32_t MASK_VALUES = 4;   // some value is neither 0 nor -inf
+constexpr uint32_t MASK_SEEN = 1;     // some key is not hidden
+constexpr uint32_t MASK_HIDDEN = 2;   // some key is hidden or past the end
+constexpr uint32_t MASK_VALUES = 4;   // some value is neither 0 nor hides its key
+
+// A mask value hides its key where the softmax's log2 domain holds no number for it: -inf, and the type's lowest values
+// with it, as in the kernels that add the mask to the scaled score.
+__device__ __forceinline__ bool mask_hides(float value) { return value * 1.4426950408889634f == -CUDART_INF_F; }
 
 // Block = 32 rows x 128 keys, warp = 4 rows; a lane reads keys lane + 32 c, so that reads coalesce whatever the row's
 // alignment and a ballot is the chunk's bits.
@@ -76,7 +80,8 @@ __global__ void __launch_bounds__(256) mask_scan_kernel(const float* mask, int s
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int key = j * 128 + c * 32 + lane;
-            v[i][c] = r0 + i < seq && key < kv_len ? mask[(long long)(r0 + i) * kv_len + key] : -CUDART_INF_F;
+            const float m = r0 + i < seq && key < kv_len ? mask[(long long)(r0 + i) * kv_len + key] : -CUDART_INF_F;
+            v[i][c] = mask_hides(m) ? -CUDART_INF_F : m;
         }
     uint32_t c8 = 0;
 #pragma unroll
@@ -122,9 +127,10 @@ __device__ __forceinline__ void select_chunk(uint32_t (&v)[32], uint32_t bits) {
     for (int e = 0; e < 32; ++e) v[e] = (bits >> e) & 1u ? v[e] : 0xff800000u;
 }
 
-// A block with values: raw score + mask / scale, which the softmax scales like a score, back into tensor memory.
-// (Clamped, so that a large finite mask stays finite.)
-__device__ __forceinline__ void add_mask_values(uint32_t tS, const float* mask_row, int key0, int kv_len, float inv_scale) {
+// A block with values: score * scale + mask in the log2 domain, as the softmax goes on to use it (with a scale of one),
+// back into tensor memory.  (Not mask / scale beside the raw score: where the mask is large, the product with the scale is
+// then off by more than an exponent holds.)
+__device__ __forceinline__ void add_mask_values(uint32_t tS, const float* mask_row, int key0, int kv_len, float sl) {
 #pragma unroll 1
     for (int c = 0; c < 128; c += 32) {
         uint32_t v[32];
@@ -133,8 +139,7 @@ __device__ __forceinline__ void add_mask_values(uint32_t tS, const float* mask_r
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
             const float m = mask_row && key0 + c + e < kv_len ? mask_row[key0 + c + e] : -CUDART_INF_F;
-            const float x = fminf(fmaxf(m * inv_scale, -3.0e38f), 3.0e38f);
-            v[e] = m == -CUDART_INF_F ? 0xff800000u : __float_as_uint(__uint_as_float(v[e]) + x);
+            v[e] = __float_as_uint(__uint_as_float(v[e]) * sl + m * 1.4426950408889634f);
         }
         tmem_st32(tS + c, v);
     }
@@ -635,8 +640,12 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                     break;
                 }
                 tc_fence_after_sync();
-                if (MASKED && (cls & MASK_VALUES))
-                    add_mask_values(tS, t < p.seq ? p.mask + (long long)t * p.kv_len : nullptr, kc, p.kv_len, 1.4426950408889634f / sl);
+                float bl = sl;  // what the block's scores are scaled by
+                uint64_t bl2 = sl2;
+                if (MASKED && (cls & MASK_VALUES)) {
+                    add_mask_values(tS, t < p.seq ? p.mask + (long long)t * p.kv_len : nullptr, kc, p.kv_len, sl);
+                    bl = 1.0f, bl2 = pack_f32x2(1.0f, 1.0f);
+                }
                 tmem_ld32(tS, s0);
                 tmem_ld32(tS + 32, s1);
                 tmem_ld32(tS + 64, s2);
@@ -656,12 +665,12 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                     mask_chunk(s3, kc + 96, rm);
                 }
                 float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                chunk_max<0>(s0, mr, sl, kc, rm);
-                chunk_max<0>(s1, mr, sl, kc, rm);
-                chunk_max<0>(s2, mr, sl, kc, rm);
-                chunk_max<0>(s3, mr, sl, kc, rm);
+                chunk_max<0>(s0, mr, bl, kc, rm);
+                chunk_max<0>(s1, mr, bl, kc, rm);
+                chunk_max<0>(s2, mr, bl, kc, rm);
+                chunk_max<0>(s3, mr, bl, kc, rm);
                 const float top = fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3]));
-                const float m_new = fmaxf(m, top * sl);
+                const float m_new = fmaxf(m, top * bl);
                 if (j == w.lo) {
                     m = m_new;
                 } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
@@ -695,19 +704,19 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 uint64_t ls2[2] = {0ull, 0ull};
                 // The sum takes the block's largest probability as the second MMA will see it, rounded to bf16: a row that
                 // one key dominates would otherwise be off by that rounding whenever m is stale (2^-9, as much as the output's own).
-                const float p_top = fast_exp2(fmaf(top, sl, -m_eff));
+                const float p_top = fast_exp2(fmaf(top, bl, -m_eff));
                 l += bf16_round(p_top) - p_top;
                 uint32_t pk[16];
-                exp_chunk(s0, pk, ls2, sl2, nm2);
+                exp_chunk(s0, pk, ls2, bl2, nm2);
                 tmem_st16(tS, pk);
-                exp_chunk(s1, pk, ls2, sl2, nm2);
+                exp_chunk(s1, pk, ls2, bl2, nm2);
                 tmem_st16(tS + 16, pk);
-                exp_chunk(s2, pk, ls2, sl2, nm2);
+                exp_chunk(s2, pk, ls2, bl2, nm2);
                 tmem_wait_st();
                 tc_fence_before_sync();
                 mbar_arrive_remote_warp(b_half + 16 * st);
                 tmem_st16(tS + 32, pk);
-                exp_chunk(s3, pk, ls2, sl2, nm2);
+                exp_chunk(s3, pk, ls2, bl2, nm2);
                 tmem_st16(tS + 48, pk);
                 cls = next_cls;
                 float l0, l1, l2, l3;

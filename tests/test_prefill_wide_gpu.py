@@ -103,6 +103,47 @@ def test_additive_mask(seq, kv, nq, nkv, kind):
     assert ops.device_status() == (0, 0)
 
 
+@pytest.mark.parametrize("scale", [0.0625, 1.0, 1.5])
+def test_additive_mask_of_the_lowest_value_infinity_and_nan(scale):
+    """Scanned or read by the attention kernel itself (no workspace), a mask means the same: the type's lowest value hides
+    a key as -inf does, NaN and +inf go on to their row only."""
+    from arcaine_b200 import _lib, ops
+    import ctypes as C
+    ops.clear_device_status()
+    seq, kv, nq, nkv, hd, inf, lowest = 40, 300, 4, 2, 256, float("inf"), torch.finfo(torch.float32).min
+    q = (seeded_bf16(seq, nq, hd, seed=1).float() * hd ** -0.5).bfloat16().cuda()
+    k, v = seeded_bf16(kv, nkv, hd, seed=2).cuda(), seeded_bf16(kv, nkv, hd, seed=3).cuda()
+    mask = torch.zeros(seq, kv, device="cuda")
+    mask[0] = lowest
+    mask[1, 20:] = lowest
+    mask[2, 7], mask[3, 8] = float("nan"), inf
+    mask[4] = -2.0e38  # finite, large: the same for every key, so that it changes nothing
+    mask[5], mask[5, 250:] = lowest, 1.0
+    run = lambda m: ops.sdpa_prefill(q, k, v, scale=scale, mask_type=ops.MASK_EXPLICIT, mask=m, num_splits=1, return_lse=True)  # noqa: E731
+    out, lse = run(mask)
+    own, own_lse = torch.empty_like(out), torch.empty_like(lse)
+    p = _lib.PrefillParams()
+    p.q, p.k, p.v, p.out, p.mask, p.out_lse = (t.data_ptr() for t in (q, k, v, own, mask, own_lse))
+    p.batch, p.seq, p.kv_len, p.nq, p.nkv, p.hd = 1, seq, kv, nq, nkv, hd
+    p.q_stride_t = p.o_stride_t = nq * hd
+    p.k_stride_t = p.v_stride_t = nkv * hd
+    p.scale, p.mask_type, p.window, p.num_splits = scale, ops.MASK_EXPLICIT, ops.NO_WINDOW, 1
+    assert _lib.load().arc_sdpa_prefill(C.byref(p), torch.cuda.current_stream().cuda_stream) == _lib.ARC_OK
+    for o, l in ((out, lse), (own, own_lse)):
+        assert torch.count_nonzero(o[0].float()) == 0 and (l[0] == -inf).all()
+        assert torch.isnan(o[2].float()).all() and torch.isnan(o[3].float()).all()
+    hidden = mask.clone()
+    hidden[hidden == lowest] = -inf
+    hidden[2:5] = 0.0
+    want, _ = run(hidden)
+    rows = [1, 4] + list(range(5, seq))
+    # (-2e38 and a score are -2e38 in fp32: row 4 sees all keys alike)
+    want[4] = v.float().mean(0).repeat_interleave(nq // nkv, 0).bfloat16()
+    assert_close(out[rows], want[rows].float(), "scanned", rel_tol=4e-3, abs_tol=1.6e-2)
+    assert_close(own[rows], want[rows].float(), "read by the kernel", rel_tol=4e-3, abs_tol=1.6e-2)
+    assert ops.device_status() == (0, 0)
+
+
 def test_vision_blocks_longer_than_a_search_step():
     """Block ids looked up in the kernel (128 keys a step, 32 rows a warp) against the additive buffer of the same rule:
     blocks of one token, next to each other, across warps and tiles, longer than a step, and up to the last key."""
