@@ -163,9 +163,8 @@ def load() -> C.CDLL:
 _native = None
 
 
-def native(workspace_of):
-    """The compiled tensor binding (``_native.so``, csrc/torch_binding.cpp), loaded once.
-    ``workspace_of(device index)`` gives it the default workspace of a device."""
+def native():
+    """The compiled tensor binding (``_native.so``, csrc/torch_binding.cpp), loaded once."""
     global _native
     if _native is None:
         if not os.path.exists(BINDING_PATH):
@@ -174,7 +173,7 @@ def native(workspace_of):
                 "(there is no CPU or PyTorch fallback for these operators)")
         load()
         from . import _native as module
-        module.setup(check, workspace_of)
+        module.setup(check)
         _native = module
     return _native
 

@@ -11,6 +11,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -150,9 +151,7 @@ Tensor new_cuda(at::IntArrayRef sizes, c10::ScalarType type, c10::Device device)
 
 // --------------------------------------------------------------------------- library calls
 PyObject* g_check = nullptr;          // _lib.check(status, where): raises ArcError
-PyObject* g_workspace_of = nullptr;   // ops.Workspace.for_index(device index)
 PyObject* g_reserve = nullptr;        // "reserve"
-PyObject* g_default_ws[64] = {};      // the default workspace object of every device, once asked for
 
 void check_status(int status, const char* where) {
     if (status == ARC_OK) return;
@@ -161,29 +160,33 @@ void check_status(int status, const char* where) {
     python_failed();
 }
 
-// Scratch of at least `need` bytes from the caller's Workspace, or the device's default one.
-void take_workspace(PyObject* workspace, int device, size_t need, void** ptr, size_t* bytes) {
-    if (is_none(workspace)) {
-        PyObject*& slot = g_default_ws[device & 63];
-        if (!slot) {
-            slot = PyObject_CallFunction(g_workspace_of, "i", device);
-            if (!slot) python_failed();
+// Scratch of a call: from the caller's Workspace, or an allocation of the call's own on its stream, which the caching
+// allocator hands out again behind it, so that two streams, threads or captured graphs never share one (0.2 us more than
+// a buffer per device took).  Held until the launches are enqueued: that happens without the GIL, and a Workspace may let
+// go of its buffer meanwhile.
+struct Scratch {
+    c10::DataPtr own;
+    Tensor borrowed;
+
+    // At least `need` bytes, on the current device and stream.
+    void take(PyObject* workspace, size_t need, void** ptr, size_t* bytes) {
+        if (is_none(workspace)) {
+            own = c10::cuda::CUDACachingAllocator::get()->allocate(need);
+            *ptr = own.get();
+            *bytes = need;
+            return;
         }
-        workspace = slot;
-    }
-    PyObject* n = PyLong_FromSize_t(need);
-    PyObject* buf = n ? PyObject_CallMethodOneArg(workspace, g_reserve, n) : nullptr;
-    Py_XDECREF(n);
-    if (!buf) python_failed();
-    const Tensor* t = tensor_or_null(buf);
-    if (!t) {
+        PyObject* n = PyLong_FromSize_t(need);
+        PyObject* buf = n ? PyObject_CallMethodOneArg(workspace, g_reserve, n) : nullptr;
+        Py_XDECREF(n);
+        if (!buf) python_failed();
+        if (const Tensor* t = tensor_or_null(buf)) borrowed = *t;
         Py_DECREF(buf);
-        bad("workspace.reserve() must return a tensor");
+        if (!borrowed.defined()) bad("workspace.reserve() must return a tensor");
+        *ptr = borrowed.data_ptr();
+        *bytes = static_cast<size_t>(borrowed.numel()) * borrowed.element_size();
     }
-    *ptr = t->data_ptr();
-    *bytes = static_cast<size_t>(t->numel()) * t->element_size();
-    Py_DECREF(buf);  // the workspace object keeps it
-}
+};
 
 template <typename F>
 int without_gil(F&& f) {
@@ -247,7 +250,8 @@ void run_prefill(c10::Device device, const View& q, const View& k, const View& v
     }
     const c10::cuda::CUDAGuard guard(device);
     const size_t need = arc_sdpa_prefill_workspace_bytes(&p);
-    if (need) take_workspace(x.workspace, device.index(), need, &p.workspace, &p.workspace_bytes);
+    Scratch scratch;
+    if (need) scratch.take(x.workspace, need, &p.workspace, &p.workspace_bytes);
     void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
     check_status(without_gil([&] { return arc_sdpa_prefill(&p, stream); }), "arc_sdpa_prefill");
 }
@@ -430,7 +434,8 @@ void run_decode(c10::Device device, const View& q, const View& k, const View& v,
     }
     const c10::cuda::CUDAGuard guard(device);
     const size_t need = arc_sdpa_decode_workspace_bytes(&p);
-    if (need) take_workspace(x.workspace, device.index(), need, &p.workspace, &p.workspace_bytes);
+    Scratch scratch;
+    if (need) scratch.take(x.workspace, need, &p.workspace, &p.workspace_bytes);
     void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
     check_status(without_gil([&] { return arc_sdpa_decode(&p, stream); }), "arc_sdpa_decode");
 }
@@ -652,14 +657,13 @@ PyObject* py_fill_causal_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// setup(check, workspace_of): the Python callables the binding needs.
+// setup(check): the Python callable the binding needs.
 PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 2) {
-        PyErr_SetString(PyExc_TypeError, "setup(check, workspace_of)");
+    if (n != 1) {
+        PyErr_SetString(PyExc_TypeError, "setup(check)");
         return nullptr;
     }
     g_check = again(a[0]);
-    g_workspace_of = again(a[1]);
     g_reserve = PyUnicode_InternFromString("reserve");
     Py_RETURN_NONE;
 }

@@ -36,11 +36,13 @@ def _require(t: torch.Tensor, dtype, name: str) -> None:
 
 
 class Workspace:
-    """Grow-only device scratch for split-KV partials, one per device.
+    """Grow-only device scratch for split-KV partials and scanned masks, to pass as ``workspace=``.
 
-    Reallocates only when a call needs more than any earlier call, so steady
-    state has no allocation on the hot path (the reference measured what
-    per-call attention scratch costs: notes/diffusion_gemma/NVFP4_DPAS_KERNEL.md:243-250).
+    Reallocates only when a call needs more than any earlier call (the reference measured what
+    per-call attention scratch costs: notes/diffusion_gemma/NVFP4_DPAS_KERNEL.md:243-250).  One of them
+    serves the calls of one stream; it is the caller's to keep from being used on two at once.  Calls
+    without one take their scratch from torch's caching allocator on their stream and share it with no
+    other call.
     """
 
     _per_device: dict[int, "Workspace"] = {}
@@ -67,7 +69,7 @@ def _native():
     """The compiled binding: it reads the tensors, checks them, fills the parameter struct and calls the
     library.  Replaced by the module's own getter once loaded, so a call costs one global lookup."""
     global _native
-    module = _lib.native(lambda index: Workspace.for_device(torch.device("cuda", index)))
+    module = _lib.native()
     _native = lambda: module  # noqa: E731
     return module
 
