@@ -494,9 +494,7 @@ PyObject* py_decode_one(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t begin = to_int(a[4]), end = to_int(a[5]), nq = to_int(a[6]), nkv = to_int(a[7]), hd = to_int(a[8]);
     const bool reshape = to_bool(a[11]);
     auto cache = [&](const Tensor& t, const char* name) {
-        const View v = reshape ? view3(t, -1, nkv, hd, name) : view_of(t, name);
-        if (v.dim != 3) bad("k must have 3 or 4 dims");
-        return rows(v, begin, end);
+        return rows(reshape ? view3(t, -1, nkv, hd, name) : view_of(t, name), begin, end);  // (or a block of one sequence)
     };
     Tensor made;
     View out;
@@ -524,13 +522,13 @@ PyObject* py_qwen_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t seq = to_int(a[4]), past = to_int(a[5]), nq = to_int(a[6]), hd = to_int(a[7]);
     const View q = rows(view3(tq, -1, nq, hd, "q"), 0, seq);
     const View o = rows(view3(need_tensor(a[3], at::kBFloat16, "out"), -1, nq, hd, "out"), 0, seq);
-    if (k0.dim != 3 || v0.dim != 3) bad("k must have 3 or 4 dims");
     const View k = rows(k0, 0, past + seq), v = rows(v0, 0, past + seq);
-    if (seq == 1) {
+    if (seq == 1) {  // (also over a block of one sequence)
         DecodeExtra x;
         x.kv_len_known = true, x.kv_len_int = past + 1;
         run_decode(tq.device(), q, k, v, o, to_float(a[8]), x);
     } else {
+        if (k.dim != 3 || v.dim != 3) bad("k must have 3 or 4 dims");
         run_prefill(tq.device(), unsqueeze0(q), unsqueeze0(k), unsqueeze0(v), unsqueeze0(o), to_float(a[8]), ARC_MASK_CAUSAL,
                     ARC_NO_WINDOW, PrefillExtra());
     }

@@ -102,6 +102,22 @@ def test_qwen_single_token_entry_points(ops):
     assert_close(buf, oracle.mul_sigmoid_inplace(want, g).float(), "attention then mul_sigmoid_inplace")
 
 
+def test_qwen_single_token_over_a_block_of_one_sequence(ops):
+    """key and value as (1, capacity, nkv, hd), past + 1 rows of them in use."""
+    nq, nkv, hd, depth = 24, 4, 256, 300
+    q, g = seeded_bf16(1, nq, hd, seed=1).cuda(), seeded_bf16(1, nq, hd, seed=2).cuda()
+    k, v = seeded_bf16(1, depth + 9, nkv, hd, seed=3).cuda(), seeded_bf16(1, depth + 9, nkv, hd, seed=4).cuda()
+    want, got = torch.empty_like(q), torch.empty_like(q)
+    ops.qwen35_xmx_attention_decode_gqa(q, k[0], v[0], want, depth, nq, nkv, hd, 0.0625, gate=g)
+    ops.qwen35_xmx_attention_decode_gqa(q, k, v, got, depth, nq, nkv, hd, 0.0625, gate=g)
+    assert torch.equal(got, want)
+    ops.qwen35_xmx_attention(q, k[0], v[0], want, 1, depth, nq, nkv, hd, 0.0625)
+    ops.qwen35_xmx_attention(q, k, v, got, 1, depth, nq, nkv, hd, 0.0625)
+    assert torch.equal(got, want)
+    with pytest.raises(ValueError):
+        ops.qwen35_xmx_attention(q.expand(2, -1, -1).contiguous(), k, v, torch.empty_like(q).expand(2, -1, -1).contiguous(), 2, depth, nq, nkv, hd, 0.0625)
+
+
 def test_merge_kernel_against_oracle(ops):
     P, rows, hd = 5, 37, 128
     g = torch.Generator().manual_seed(5)
