@@ -317,17 +317,18 @@ PyObject* py_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // One sequence, token-major: attention(Q, seq, nq, hd, K, V, kv_len, nkv, scale, mask_type, window, mask, out,
-//                                      block_ids, block_ids_offset)
+//                                      block_ids, block_ids_offset, flat).  flat: K and V may be one-dimensional.
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    need_args(n, 15, "attention");
+    need_args(n, 16, "attention");
+    const bool flat = to_bool(a[15]);
     const Tensor& tq = need_tensor(a[0], at::kBFloat16, "q");
     const Tensor& tk = need_tensor(a[4], at::kBFloat16, "k");
     const Tensor& tv = need_tensor(a[5], at::kBFloat16, "v");
     const int64_t seq = to_int(a[1]), nq = to_int(a[2]), hd = to_int(a[3]), kv_len = to_int(a[6]), nkv = to_int(a[7]);
     View q = unsqueeze0(view3(tq, seq, nq, hd, "q"));
     auto cache = [&](const Tensor& t, const char* name) {
-        if (t.dim() == 1) return unsqueeze0(view3(t.slice(0, 0, kv_len * nkv * hd), kv_len, nkv, hd, name));
+        if (flat && t.dim() == 1) return unsqueeze0(view3(t.slice(0, 0, kv_len * nkv * hd), kv_len, nkv, hd, name));
         View v = view_of(t, name);
         if (v.dim != 3) bad(std::string(name) + " must have 3 or 4 dims");
         return unsqueeze0(rows(v, 0, kv_len));
@@ -548,9 +549,8 @@ PyObject* py_qkv_prepare(PyObject*, PyObject* const* a, Py_ssize_t n) {
     auto get = [&](int i, const char* name) {
         if (is_none(a[i])) return View();
         View v = view_of(need_tensor(a[i], at::kBFloat16, name), name);
-        if (three && v.dim < 4) v = unsqueeze0(v);
-        if (v.dim != 4) bad(std::string(name) + " must have 3 or 4 dims");
-        return v;
+        if (v.dim != (three ? 3 : 4)) bad(std::string(name) + " must have 3 or 4 dims, as q and k");
+        return three ? unsqueeze0(v) : v;
     };
     const View q = get(0, "q"), k = get(1, "k"), v = get(2, "v"), kc = get(3, "k_cache"), vc = get(4, "v_cache");
     const View& r = q.given() ? q : k;

@@ -200,14 +200,14 @@ def fill_causal_mask_with_block_ids(block_ids: Optional[torch.Tensor], q_len: in
 # ---------------------------------------------------------------------------
 def gqa_attention_sdpa(Q, seq, nq, hd, Kc, Vc, kv_len, nkv, mask=None, mask_type=MASK_NONE, out=None):
     """src/modeling/diffusion_gemma/attention.cpp:930-995 — no scale; mask_type 0 / 1 / 3."""
-    return _native().attention(Q, seq, nq, hd, Kc, Vc, kv_len, nkv, 1.0, mask_type, NO_WINDOW, mask, out, None, 0)
+    return _native().attention(Q, seq, nq, hd, Kc, Vc, kv_len, nkv, 1.0, mask_type, NO_WINDOW, mask, out, None, 0, True)
 
 
 def gqa_attention(Q, seq, nq, hd, Kc, Vc, kv_len, nkv, past_offset, sliding_window, causal, out=None):
     """src/modeling/diffusion_gemma/attention.cpp:706-821 — the matmul/softmax/matmul path's result."""
     del past_offset  # queries and keys share it; the visibility rule does not depend on it
     return _native().attention(Q, seq, nq, hd, Kc, Vc, kv_len, nkv, 1.0, MASK_CAUSAL if causal else MASK_NONE,
-                               sliding_window if causal else NO_WINDOW, None, out, None, 0)
+                               sliding_window if causal else NO_WINDOW, None, out, None, 0, False)
 
 
 def batched_attention(Q, seq_len, nq_heads, q_head_dim, K, V, kv_len, nkv_heads, kv_head_dim, past_offset,
@@ -221,7 +221,7 @@ def batched_attention(Q, seq_len, nq_heads, q_head_dim, K, V, kv_len, nkv_heads,
         block_ids = None  # the reference builds no mask at all in that case
     return _native().attention(Q, seq_len, nq_heads, q_head_dim, K, V, kv_len, nkv_heads, scale,
                                MASK_NONE if skip_mask else MASK_CAUSAL, NO_WINDOW if skip_mask else sliding_window, None, out,
-                               block_ids, past_offset - (kv_len - seq_len) if block_ids is not None else 0)
+                               block_ids, past_offset - (kv_len - seq_len) if block_ids is not None else 0, False)
 
 
 def gemma4_sliding_decode_attention(Q, K_cache, V_cache, kv_len, kv_start, nq_heads, nkv_heads, head_dim, out=None):

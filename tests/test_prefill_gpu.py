@@ -217,6 +217,23 @@ def test_reference_named_entry_points(ops):
                               block_ids=torch.zeros(1, dtype=torch.int32, device="cuda"))
 
 
+def test_caches_of_other_dimensions_stay_refused(ops):
+    """One-dimensional caches belong to gqa_attention_sdpa; pre-processing takes all tensors with the same number of dims."""
+    seq, nq, nkv, hd = 20, 4, 2, 128
+    q, k = seeded_bf16(seq, nq, hd, seed=1).cuda(), seeded_bf16(seq, nkv, hd, seed=2).cuda()
+    want = ops.gqa_attention_sdpa(q, seq, nq, hd, k, k, seq, nkv)
+    assert torch.equal(ops.gqa_attention_sdpa(q, seq, nq, hd, k.flatten(), k.flatten(), seq, nkv), want)
+    with pytest.raises(ValueError):
+        ops.gqa_attention(q, seq, nq, hd, k.flatten(), k.flatten(), seq, nkv, 0, ops.NO_WINDOW, True)
+    with pytest.raises(ValueError):
+        ops.batched_attention(q, seq, nq, hd, k.flatten(), k.flatten(), seq, nkv, hd, 0, ops.NO_WINDOW)
+    cache = torch.zeros(1, seq + 4, nkv, hd, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises((ValueError, IndexError)):
+        ops.qkv_prepare(q, k, k.clone(), k_cache=cache, v_cache=cache.clone(), eps=1e-6, theta=1e4)
+    with pytest.raises((ValueError, IndexError)):
+        ops.qkv_prepare(q[None], k[None], k[None].clone(), k_cache=cache[0], v_cache=cache[0].clone(), eps=1e-6, theta=1e4)
+
+
 def test_error_statuses(ops):
     from arcaine_b200 import _lib
     q = torch.zeros(8, 4, 64, dtype=torch.bfloat16, device="cuda")
