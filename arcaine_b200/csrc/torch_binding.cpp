@@ -69,6 +69,25 @@ float to_float(PyObject* o) {
     return static_cast<float>(v);
 }
 
+// A reference of this function's own.
+struct Held {
+    PyObject* o;
+    explicit Held(PyObject* owned) : o(owned) {}
+    Held(const Held&) = delete;
+    ~Held() { Py_XDECREF(o); }
+};
+
+PyObject* item(PyObject* o, Py_ssize_t i) {  // o[i], of a tuple, a list, an array, a tensor
+    if (PyTuple_Check(o) && i < PyTuple_GET_SIZE(o)) {
+        Py_INCREF(PyTuple_GET_ITEM(o, i));
+        return PyTuple_GET_ITEM(o, i);
+    }
+    const Held index(PyLong_FromSsize_t(i));
+    PyObject* r = index.o ? PyObject_GetItem(o, index.o) : nullptr;
+    if (!r) python_failed();
+    return r;
+}
+
 bool to_bool(PyObject* o) {
     const int v = PyObject_IsTrue(o);
     if (v < 0) python_failed();
@@ -426,11 +445,11 @@ void run_decode(c10::Device device, const View& q, const View& k, const View& v,
     p.q_stride_b = q.st[0];
     p.scale = scale, p.num_ctas = x.num_ctas;
     if (!is_none(x.exchange)) {
-        PyObject *peers, *world, *rank, *step;
-        if (!PyArg_ParseTuple(x.exchange, "OOOO", &peers, &world, &rank, &step)) python_failed();
-        p.xchg_peers = static_cast<const uint64_t*>(need_tensor(peers, at::kLong, "exchange peers").data_ptr());
-        p.xchg_world = (int32_t)to_int(world), p.xchg_rank = (int32_t)to_int(rank);
-        p.xchg_step = (uint32_t)(to_int(step) & 0xFFFFFFFFll);
+        const Held peers(item(x.exchange, 0)), world(item(x.exchange, 1)), rank(item(x.exchange, 2)), step(item(x.exchange, 3));
+        if (PyObject_Size(x.exchange) != 4) bad("exchange must be (peers, world, rank, step)");
+        p.xchg_peers = static_cast<const uint64_t*>(need_tensor(peers.o, at::kLong, "exchange peers").data_ptr());
+        p.xchg_world = (int32_t)to_int(world.o), p.xchg_rank = (int32_t)to_int(rank.o);
+        p.xchg_step = (uint32_t)(to_int(step.o) & 0xFFFFFFFFll);
         p.xchg_wait_cycles = x.exchange_wait;
     }
     const c10::cuda::CUDAGuard guard(device);
@@ -608,14 +627,8 @@ PyObject* py_qkv_prepare(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor& pos = need_tensor(a[16], at::kInt, "mrope_positions");
         if (!pos.is_contiguous() || pos.numel() != B * 3 * S) bad("mrope_positions must be a contiguous (B, 3, S) int32 tensor");
         p.mrope_positions = static_cast<const int32_t*>(pos.data_ptr());
-        if (is_none(a[17]) || PySequence_Size(a[17]) != 3) bad("Qwen3.5 MRoPE needs three sections");
-        for (int i = 0; i < 3; ++i) {
-            PyObject* e = PySequence_GetItem(a[17], i);
-            if (!e) python_failed();
-            const int64_t sec = to_int(e);
-            Py_DECREF(e);
-            p.mrope_section[i] = (int32_t)sec;
-        }
+        if (is_none(a[17]) || PyObject_Size(a[17]) != 3) bad("Qwen3.5 MRoPE needs three sections");
+        for (int i = 0; i < 3; ++i) p.mrope_section[i] = (int32_t)to_int(Held(item(a[17], i)).o);
     }
     p.v_copy = to_bool(a[18]) ? 1 : 0;
     const c10::cuda::CUDAGuard guard(ref.device());

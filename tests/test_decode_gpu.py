@@ -251,6 +251,16 @@ def test_exchange_fold_with_the_other_ranks_record_already_in_place(ops):
     assert (xbuf[step & 1, 0, :, :, 1] == step).all() and (scratch[step & 1, 0, :, :, 1] == step).all()
 
 
+def test_exchange_of_one_rank_as_a_list(ops):
+    q, k, v = seeded_bf16(1, 4, 128, seed=71).cuda(), seeded_bf16(1, 300, 1, 128, seed=72).cuda(), seeded_bf16(1, 300, 1, 128, seed=73).cuda()
+    peers = torch.zeros(1, dtype=torch.int64, device="cuda")
+    want = ops.sdpa_decode(q, k, v, scale=0.1)
+    for exchange in ((peers, 1, 0, 1), [peers, 1, 0, 1]):
+        assert torch.equal(ops.sdpa_decode(q, k, v, scale=0.1, exchange=exchange), want)
+    with pytest.raises((ValueError, IndexError)):
+        ops.sdpa_decode(q, k, v, scale=0.1, exchange=[peers, 1, 0])
+
+
 def test_device_side_length_past_the_cache_is_a_status_not_a_wrong_result(ops):
     from arcaine_b200 import _lib
     B, nq, nkv, hd, cap = 2, 8, 2, 128, 64

@@ -169,3 +169,16 @@ def test_shared_kv_projection_with_in_place_k_is_refused(ops):
     vc = torch.zeros(B, 16, nkv, hd, dtype=torch.bfloat16, device="cuda")
     with pytest.raises(ValueError, match="k_cache"):
         ops.qkv_prepare(q, k, None, v_from_k=True, v_cache=vc)
+
+
+def test_mrope_sections_as_any_sequence(ops):
+    """Three sections as a tuple, a list, an array or a tensor."""
+    import numpy as np
+    pos = torch.arange(30, dtype=torch.int32, device="cuda").view(1, 3, 10)
+    x = seeded_bf16(10, 2, 256, seed=1).cuda()
+    got = []
+    for sec in ((11, 11, 10), [11, 11, 10], np.array([11, 11, 10]), torch.tensor([11, 11, 10])):
+        q = x.clone()
+        ops.qkv_prepare(q, None, None, eps=1e-6, theta=1e6, rotary_dim=64, mrope_positions=pos, mrope_section=sec)
+        got.append(q)
+    assert all(torch.equal(g, got[0]) for g in got) and not torch.equal(got[0], x)
