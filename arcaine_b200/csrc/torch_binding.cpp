@@ -157,6 +157,11 @@ void token_strides(const View& v, const char* name, int64_t* sb, int64_t* st) {
     *st = v.st[1];
 }
 
+// A buffer the library writes (or reads) as (n0, n1, row) must hold that many: it is given addresses and strides only.
+void need_room(const View& v, int64_t n0, int64_t n1, int64_t row, const char* name) {
+    if (v.n[0] < n0 || v.n[1] < n1 || v.n[2] * v.n[3] < row) bad(std::string(name) + " is smaller than the call needs");
+}
+
 bool same_layout(const View& a, const View& b) {
     if (a.dim != b.dim) return false;
     for (int i = 0; i < a.dim; ++i)
@@ -253,6 +258,7 @@ void run_prefill(c10::Device device, const View& q, const View& k, const View& v
     token_strides(k, "k", &p.k_stride_b, &p.k_stride_t);
     token_strides(v, "v", &p.v_stride_b, &p.v_stride_t);
     token_strides(out, "out", &p.o_stride_b, &p.o_stride_t);
+    need_room(out, B, S, q.n[2] * q.n[3], "out");
     p.scale = scale, p.mask_type = mask_type, p.window = (int32_t)window, p.num_splits = x.num_splits;
     if (!is_none(x.block_ids)) {
         const Tensor& ids = need_tensor(x.block_ids, at::kInt, "block_ids");
@@ -662,6 +668,8 @@ PyObject* py_fill_causal_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int q_len = (int)to_int(a[1]), kv_len = (int)to_int(a[2]), past = (int)to_int(a[3]), window = (int)to_int(a[4]);
     const c10::cuda::CUDAGuard guard(out.device());
     void* stream = c10::cuda::getCurrentCUDAStream(out.device().index()).stream();
+    if (!out.is_contiguous() || (q_len > 0 && kv_len > 0 && out.numel() < (int64_t)q_len * kv_len))
+        bad("out must be contiguous and hold q_len * kv_len values");
     float* mask = static_cast<float*>(out.data_ptr());
     check_status(without_gil([&] { return arc_fill_causal_mask(mask, q_len, kv_len, past, window, stream); }), "arc_fill_causal_mask");
     return again(a[0]);

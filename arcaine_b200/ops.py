@@ -184,6 +184,8 @@ def fill_causal_mask_with_block_ids(block_ids: Optional[torch.Tensor], q_len: in
     if out is None:
         out = torch.empty((q_len, kv_len), dtype=torch.float32, device=device)
     _require(out, torch.float32, "out")
+    if not out.is_contiguous() or out.numel() < q_len * kv_len:
+        raise ValueError("out must be contiguous and hold q_len * kv_len values")
     if block_ids is not None:
         _require(block_ids, torch.int32, "block_ids")
         if block_ids.numel() < past_offset + q_len:

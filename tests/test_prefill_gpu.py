@@ -217,6 +217,34 @@ def test_reference_named_entry_points(ops):
                               block_ids=torch.zeros(1, dtype=torch.int32, device="cuda"))
 
 
+def test_outputs_too_small_for_the_result_are_refused(ops):
+    """The library is given addresses and strides: what it would write past its end has to be refused here.  Larger ones
+    are filled from their start."""
+    seq, nq, nkv, hd = 20, 4, 2, 128
+    q, k = seeded_bf16(seq, nq, hd, seed=1).cuda(), seeded_bf16(seq, nkv, hd, seed=2).cuda()
+    new = lambda *n: torch.zeros(*n, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+    want = ops.sdpa_prefill(q, k, k, scale=0.1)
+    for small in (new(seq - 1, nq, hd), new(seq, nq - 1, hd), new(seq, nq, hd - 8)):
+        with pytest.raises(ValueError):
+            ops.sdpa_prefill(q, k, k, scale=0.1, out=small)
+        with pytest.raises(ValueError):
+            ops.sdpa_prefill(q, k, k, scale=0.1, out=small, gate=small.clone())
+        with pytest.raises(ValueError):
+            ops.gqa_attention_sdpa(q, seq, nq, hd, k, k, seq, nkv, out=small)
+    with pytest.raises(ValueError):
+        ops.sdpa_prefill(q[None].repeat(2, 1, 1, 1), k[None].repeat(2, 1, 1, 1), k[None].repeat(2, 1, 1, 1), scale=0.1, out=new(1, seq, nq, hd))
+    with pytest.raises(ValueError):
+        ops.qwen35_xmx_attention(q, k, k, new(seq - 1, nq, hd), seq, 0, nq, nkv, hd, 0.1)
+    large = new(seq + 3, nq + 1, hd)
+    ops.sdpa_prefill(q, k, k, scale=0.1, out=large)
+    assert torch.equal(large[:seq, :nq], want) and not large[seq:].any() and not large[:, nq:].any()
+    for fill in (lambda o: ops.fill_causal_mask(8, 16, 8, out=o), lambda o: ops.fill_causal_mask_with_block_ids(None, 8, 16, 8, out=o)):
+        for bad in (torch.zeros(8, 15, device="cuda"), torch.zeros(16, 8, device="cuda").t()):
+            with pytest.raises(ValueError):
+                fill(bad)
+        assert torch.equal(fill(torch.ones(9, 16, device="cuda"))[:8], ops.fill_causal_mask(8, 16, 8))
+
+
 def test_caches_of_other_dimensions_stay_refused(ops):
     """One-dimensional caches belong to gqa_attention_sdpa; pre-processing takes all tensors with the same number of dims."""
     seq, nq, nkv, hd = 20, 4, 2, 128
