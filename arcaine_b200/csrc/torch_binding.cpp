@@ -581,6 +581,7 @@ PyObject* py_qkv_prepare(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const View& r = q.given() ? q : k;
     const int64_t past = to_int(a[5]), B = r.n[0], S = r.n[1], hd = r.n[3];
     const bool v_from_k = to_bool(a[14]);
+    if (past < 0 && (kc.given() || vc.given())) bad("past_len must not be negative");
     arc_qkv_prepare_params p{};
     if (q.given()) {
         p.q = q.ptr, p.nq = (int32_t)q.n[2];
@@ -588,8 +589,11 @@ PyObject* py_qkv_prepare(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     if (k.given()) {
         p.k_src = k.ptr, p.nkv = (int32_t)k.n[2];
+        const int64_t row = k.n[2] * hd;
+        need_room(k, B, S, row, "k");
         token_strides(k, "k", &p.k_src_stride_b, &p.k_src_stride_t);
         if (kc.given() && past + S > kc.n[1]) bad("KV cache capacity exceeded");
+        if (kc.given()) need_room(kc, B, past + S, row, "k_cache");
         const View& kd = kc.given() ? kc : k;
         token_strides(kd, "k_cache", &p.k_dst_stride_b, &p.k_dst_stride_t);
         p.k_dst = kd.ptr + (kc.given() ? past : 0) * p.k_dst_stride_t * 2;
@@ -598,6 +602,8 @@ PyObject* py_qkv_prepare(PyObject*, PyObject* const* a, Py_ssize_t n) {
             if (!vd.given()) bad("v_from_k needs v_cache");
             if (v_from_k && !kc.given())  // K would be rewritten in place while V is still being read from it
                 bad("v_from_k needs k_cache: K cannot be normalised in place when V is taken from it");
+            need_room(vd, B, vc.given() ? past + S : S, row, vc.given() ? "v_cache" : "v");
+            if (v.given() && !v_from_k) need_room(v, B, S, row, "v");
             token_strides(vd, "v_cache", &p.v_dst_stride_b, &p.v_dst_stride_t);
             p.v_dst = vd.ptr + (vc.given() ? past : 0) * p.v_dst_stride_t * 2;
             if (v.given() && !v_from_k) {
@@ -606,8 +612,12 @@ PyObject* py_qkv_prepare(PyObject*, PyObject* const* a, Py_ssize_t n) {
             }
         }
     }
-    if (!is_none(a[6])) p.q_weight = need_tensor(a[6], at::kBFloat16, "q_weight").data_ptr();
-    if (!is_none(a[7])) p.k_weight = need_tensor(a[7], at::kBFloat16, "k_weight").data_ptr();
+    auto values = [](const Tensor& t, int64_t n, const char* name) {  // the address of n values in a row
+        if (t.numel() < n) bad(std::string(name) + " is smaller than the call needs");
+        return t.data_ptr();
+    };
+    if (!is_none(a[6])) p.q_weight = values(need_tensor(a[6], at::kBFloat16, "q_weight"), hd, "q_weight");
+    if (!is_none(a[7])) p.k_weight = values(need_tensor(a[7], at::kBFloat16, "k_weight"), hd, "k_weight");
     p.batch = (int32_t)B, p.seq = (int32_t)S, p.hd = (int32_t)hd;
     const double partial = PyFloat_AsDouble(a[10]);
     if (partial == -1.0 && PyErr_Occurred()) python_failed();
@@ -616,12 +626,14 @@ PyObject* py_qkv_prepare(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor& c = need_tensor(a[11], at::kFloat, "rope_cos");
         const Tensor& s = need_tensor(a[12], at::kFloat, "rope_sin");
         if (!c.is_contiguous() || !s.is_contiguous()) bad("rope tables must be contiguous");
-        p.rope_cos = static_cast<const float*>(c.data_ptr());
-        p.rope_sin = static_cast<const float*>(s.data_ptr());
         p.rope_stride_b = c.dim() == 3 ? S * p.n_active_pairs : 0;
+        const int64_t pairs = is_none(a[15]) ? p.n_active_pairs : to_int(a[15]) / 2;
+        const int64_t angles = S * pairs + (B - 1) * p.rope_stride_b;
+        p.rope_cos = static_cast<const float*>(values(c, angles, "rope_cos"));
+        p.rope_sin = static_cast<const float*>(values(s, angles, "rope_sin"));
     }
     if (!is_none(a[13]) && tensor_or_null(a[13]))
-        p.pos_offset = static_cast<const int32_t*>(need_tensor(a[13], at::kInt, "pos_offset").data_ptr());
+        p.pos_offset = static_cast<const int32_t*>(values(need_tensor(a[13], at::kInt, "pos_offset"), B, "pos_offset"));
     else
         p.pos0 = (int32_t)(is_none(a[13]) ? past : to_int(a[13]));
     p.eps = to_float(a[8]), p.theta = to_float(a[9]);

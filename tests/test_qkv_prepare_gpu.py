@@ -182,3 +182,33 @@ def test_mrope_sections_as_any_sequence(ops):
         ops.qkv_prepare(q, None, None, eps=1e-6, theta=1e6, rotary_dim=64, mrope_positions=pos, mrope_section=sec)
         got.append(q)
     assert all(torch.equal(g, got[0]) for g in got) and not torch.equal(got[0], x)
+
+
+def test_caches_and_tables_too_small_for_the_call_are_refused(ops):
+    """Everything the kernel would read or write past the end of: both caches, K and V, weights, tables, positions."""
+    B, seq, nq, nkv, hd, past = 2, 10, 4, 2, 128, 3
+    new = lambda *n: torch.zeros(*n, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+    table = torch.zeros(seq, hd // 2, device="cuda")
+    good = dict(q=new(B, seq, nq, hd), k=new(B, seq, nkv, hd), v=new(B, seq, nkv, hd), k_cache=new(B, past + seq, nkv, hd),
+                v_cache=new(B, past + seq, nkv, hd), q_weight=new(hd), k_weight=new(hd), rope_cos=table, rope_sin=table.clone())
+
+    def call(**over):
+        a = {**good, **over}
+        ops.qkv_prepare(a.pop("q"), a.pop("k"), a.pop("v"), past_len=past, eps=1e-6, **a)
+
+    call()
+    call(rope_cos=None, rope_sin=None, pos_offset=torch.zeros(B, dtype=torch.int32, device="cuda"))
+    for name in ("k_cache", "v_cache"):
+        for shape in ((B - 1, past + seq, nkv, hd), (B, past + seq - 1, nkv, hd), (B, past + seq, nkv - 1, hd)):
+            with pytest.raises(ValueError):
+                call(**{name: new(*shape)})
+    for name, t in (("k", new(B - 1, seq, nkv, hd)), ("k", new(B, seq - 1, nkv, hd)), ("v", new(B, seq, nkv - 1, hd)),
+                    ("v", new(B, seq - 1, nkv, hd)), ("q_weight", new(hd - 1)), ("k_weight", new(hd - 1)),
+                    ("rope_cos", table[1:]), ("rope_sin", table[1:])):
+        with pytest.raises(ValueError):
+            call(**{name: t})
+    with pytest.raises(ValueError):
+        call(rope_cos=None, rope_sin=None, pos_offset=torch.zeros(B - 1, dtype=torch.int32, device="cuda"))
+    with pytest.raises(ValueError):
+        ops.qkv_prepare(good["q"], good["k"], good["v"], k_cache=good["k_cache"], v_cache=good["v_cache"], past_len=-1, eps=1e-6)
+    torch.cuda.synchronize()
