@@ -757,7 +757,7 @@ extern "C" int arc_sdpa_prefill(const arc_sdpa_prefill_params* p, void* stream) 
     if (rc != ARC_OK) return rc;
     PrefillPlan plan;
     if ((rc = plan_prefill(p, ds->sm_count, ds->wide, &plan)) != ARC_OK) return rc;
-    if (p->hd == 256 && p->num_splits == 0 && plan.splits > 1 && (!p->workspace || p->workspace_bytes < plan.ws_bytes)) {
+    if (p->hd == 256 && p->num_splits == 0 && plan.splits > 1 && (!p->workspace || !aligned16(p->workspace) || p->workspace_bytes < plan.ws_bytes)) {
         arc_sdpa_prefill_params whole = *p;  // no room for the parts of a split the caller has not asked for: none, then
         whole.num_splits = 1;
         if ((rc = plan_prefill(&whole, ds->sm_count, ds->wide, &plan)) != ARC_OK) return rc;

@@ -144,6 +144,30 @@ def test_additive_mask_of_the_lowest_value_infinity_and_nan(scale):
     assert ops.device_status() == (0, 0)
 
 
+@pytest.mark.parametrize("room,shift", [(0, 0), (4096, 0), (1 << 26, 4)])  # none, too little, not 16-byte aligned
+def test_a_workspace_that_cannot_be_used_costs_time_only(room, shift):
+    """A canvas step whose parts have no place for their records runs over the whole key range."""
+    from arcaine_b200 import _lib, ops
+    import ctypes as C
+    ops.clear_device_status()
+    seq, kv, nq, nkv, hd = 256, 1400, 8, 4, 256
+    q, k, v = (seeded_bf16(n, h, hd, seed=80 + i).cuda() for i, (n, h) in enumerate([(seq, nq), (kv, nkv), (kv, nkv)]))
+    out, ws = torch.empty_like(q), torch.zeros(room + 64, dtype=torch.uint8, device="cuda")
+    p = _lib.PrefillParams()
+    p.q, p.k, p.v, p.out = (t.data_ptr() for t in (q, k, v, out))
+    p.batch, p.seq, p.kv_len, p.nq, p.nkv, p.hd = 1, seq, kv, nq, nkv, hd
+    p.q_stride_t = p.o_stride_t = nq * hd
+    p.k_stride_t = p.v_stride_t = nkv * hd
+    p.scale, p.mask_type, p.window, p.num_splits = 0.0625, ops.MASK_NONE, ops.NO_WINDOW, 0
+    L = _lib.load()
+    assert 4096 < L.arc_sdpa_prefill_workspace_bytes(C.byref(p)) <= 1 << 26
+    if room:
+        p.workspace, p.workspace_bytes = ws.data_ptr() + shift, room
+    assert L.arc_sdpa_prefill(C.byref(p), torch.cuda.current_stream().cuda_stream) == _lib.ARC_OK
+    assert torch.equal(out, ops.sdpa_prefill(q, k, v, scale=0.0625, num_splits=1))
+    assert ops.device_status() == (0, 0) and not ws.any()
+
+
 def test_vision_blocks_longer_than_a_search_step():
     """Block ids looked up in the kernel (128 keys a step, 32 rows a warp) against the additive buffer of the same rule:
     blocks of one token, next to each other, across warps and tiles, longer than a step, and up to the last key."""
