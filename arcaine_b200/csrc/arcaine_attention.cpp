@@ -43,8 +43,9 @@ void run_prefill(cudaStream_t stream, const bf16* q, const bf16* k, const bf16* 
     p.num_splits = 0;
     p.block_ids = block_ids;
     p.block_ids_offset = block_ids_offset;
-    const size_t need = arc_sdpa_prefill_workspace_bytes(&p);
+    size_t need = arc_sdpa_prefill_workspace_bytes(&p);
     if (need) {
+        if (hd == 256 && !ws.can_hold(need, stream)) need = 0;  // with what there is: the call is slower, not refused
         p.workspace = ws.reserve(need);
         p.workspace_bytes = ws.capacity();
     }
@@ -81,6 +82,13 @@ void run_decode(cudaStream_t stream, const bf16* q, const bf16* k, const bf16* v
 
 SdpaWorkspace::~SdpaWorkspace() {
     if (ptr_ && owned_) cudaFree(ptr_);
+}
+
+bool SdpaWorkspace::can_hold(size_t bytes, cudaStream_t stream) const {
+    if (bytes <= bytes_) return true;
+    if (!owned_) return false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;  // (a stream that is being captured must not allocate)
+    return cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
 }
 
 void* SdpaWorkspace::reserve(size_t bytes) {

@@ -28,19 +28,21 @@ struct CudaEngine {
     cudaStream_t stream = nullptr;
 };
 
-// Grow-only device scratch for split-KV partials.  The reference learned that
-// per-call allocation costs throughput (persistent attention scratch, notes/
-// diffusion_gemma/NVFP4_DPAS_KERNEL.md:243-250); this buffer reallocates only
-// when a call needs more than any call before it.
+// Grow-only device scratch for split-KV partials and scanned masks, for the calls
+// of one stream.  The reference learned that per-call allocation costs throughput
+// (persistent attention scratch, notes/diffusion_gemma/NVFP4_DPAS_KERNEL.md:243-250);
+// this buffer reallocates only when a call needs more than any call before it.
 class SdpaWorkspace {
 public:
     SdpaWorkspace() = default;
     // A region the caller owns (an arena slice sized from arc_sdpa_*_workspace_bytes): never freed or grown
-    // here; a call that needs more throws.
+    // here; a call that needs more throws, but for the prefill calls of head dim 256, which do without.
     SdpaWorkspace(void* borrowed, size_t bytes) : ptr_(borrowed), bytes_(bytes), owned_(false) {}
     ~SdpaWorkspace();
     SdpaWorkspace(const SdpaWorkspace&) = delete;
     SdpaWorkspace& operator=(const SdpaWorkspace&) = delete;
+    // reserve(bytes) can succeed now, ahead of work on `stream`.
+    bool can_hold(size_t bytes, cudaStream_t stream) const;
     void* reserve(size_t bytes);  // throws std::runtime_error on allocation failure
     size_t capacity() const { return bytes_; }
 
