@@ -142,6 +142,7 @@ static int device_state(DeviceState** out) {
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, true>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true, true>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, false, true>, WideCfg::SMEM_BYTES));
+            ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, true, true>, WideCfg::SMEM_BYTES));
             s.wide.pairs = clusters_at_once(sdpa_prefill_wide_kernel<false, false>, 2, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
             for (int parts = 2; parts <= WideRoom::MOST_FOLDED; ++parts)
                 s.wide.folded[parts] = clusters_at_once(sdpa_prefill_wide_kernel<false, false, true>, 2 * parts, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
@@ -265,6 +266,10 @@ static long long wide_units(const arc_sdpa_prefill_params* p, int q_tiles) {
 static int choose_wide_splits(const arc_sdpa_prefill_params* p, int q_tiles, const WideRoom& room) {
     const long long units = wide_units(p, q_tiles);
     int most = (p->kv_len + 127) / 128;  // key blocks of the longest unit
+    // What an additive mask hides is not known here.  Over the few blocks of a window the parts of 2048 rows cost 5 us more
+    // than they save (256 queries of 8 heads over 2304 keys: 16.4 us whole and 21.1; with all keys seen 30.3 and 23.9); 1024
+    // rows are even (64 queries of 16 heads over 4096 keys: 15.9 and 15.6; 45 and 20).  A longer cache is worth it in any case.
+    if (p->mask_type == ARC_MASK_EXPLICIT && most <= 32 && (long long)p->batch * p->seq * p->nq > 1024) return 1;
     if (p->mask_type == ARC_MASK_CAUSAL && p->window > 0 && p->window < p->kv_len && !p->block_ids) most = std::min(most, (p->window + 255) / 128 + 1);
     int best = 1;
     double least = 1.13 * most;
@@ -290,7 +295,6 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const Wi
     int splits = p->num_splits;
     const long long tiles = (long long)plan->q_tiles * p->nq * p->batch;
     const bool scanned_mask = p->mask_type == ARC_MASK_EXPLICIT && p->hd == 256 && p->num_splits <= 1;
-    if (splits == 0 && scanned_mask) splits = 1;
     if (splits == 0 && p->hd == 256) splits = choose_wide_splits(p, plan->q_tiles, room);
     if (splits == 0) {
         // Split the key range only when the tiles alone leave most SMs idle and there are enough key blocks
@@ -365,7 +369,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     kp.part_lse = kp.part_o ? kp.part_o + (size_t)plan.splits * plan.rows * HD : nullptr;
     // CTA pairs (prefill_wide_sm100.cuh) and the two-tile kernel look vision blocks up themselves; the one-tile kernel wants
     // the span end of every row (a few microseconds instead of a (seq, kv_len) f32 mask).
-    const bool wide = HD == 256 && (plan.splits == 1 || p->mask_type != ARC_MASK_EXPLICIT);
+    const bool wide = HD == 256 && (plan.splits == 1 || p->mask_type != ARC_MASK_EXPLICIT || plan.mask_bytes > 0);
     if (p->block_ids) kp.ids = p->block_ids + p->block_ids_offset;
     auto find_spans = [&]() -> int {
         if (!kp.ids) return ARC_OK;
@@ -495,7 +499,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         }
         // (a cluster is placed inside one GPC, so fewer fit than pairs / parts)
         kp.fold = split && wide_units(p, plan.q_tiles) <= ds->wide.clusters(plan.splits);
-        auto kernel = split    ? sdpa_prefill_wide_kernel<false, false, true>
+        auto kernel = split    ? (masked ? sdpa_prefill_wide_kernel<false, true, true> : sdpa_prefill_wide_kernel<false, false, true>)
                       : masked ? (kp.gate ? sdpa_prefill_wide_kernel<true, true> : sdpa_prefill_wide_kernel<false, true>)
                                : (kp.gate ? sdpa_prefill_wide_kernel<true, false> : sdpa_prefill_wide_kernel<false, false>);
         ARC_CUDA(launch_dependent(kernel,

@@ -214,7 +214,8 @@ __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int ran
     }
 }
 
-// MASKED: with an additive mask, as mask_scan_kernel has read it.
+// MASKED: with an additive mask, as mask_scan_kernel has read it.  (With SPLIT: few queries over a long cache.  16 of 8 heads
+// over 32768 keys take 299 us as whole units and 59 in parts; 64 over 4096 keys with a bias per key 201 and 43.)
 // SPLIT: a unit is one of num_splits parts of the key blocks, one unit per pair, for calls whose tiles would leave most
 // pairs idle.  The part's normalised rows go to the partial records as f32 with their log-sum-exp.  Two or three parts
 // are the pairs of one cluster (p.fold): each CTA stores only the rows the other parts' CTAs fold, and after a cluster

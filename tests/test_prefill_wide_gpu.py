@@ -103,6 +103,46 @@ def test_additive_mask(seq, kv, nq, nkv, kind):
     assert ops.device_status() == (0, 0)
 
 
+@pytest.mark.parametrize("seq,kv,nq,nkv,kind,launches", [
+    (16, 5000, 8, 4, "causal", 3),     # eight parts, one ragged tile: scan, attention, merge
+    (180, 4200, 24, 4, "random", 3),   # 24 units in three parts
+    (200, 4300, 32, 4, "blocks", 2),   # 32 units in two parts, a cluster each; a row without any key, unseen blocks at a part's ends
+    (64, 4096, 6, 2, "values", 3),     # odd group, finite values
+    (130, 1200, 3, 3, "window", 3),    # odd group, the second tile two rows; parts that see nothing
+    (256, 2304, 8, 4, "causal", 2),    # too many rows for so few blocks: whole units
+])
+def test_additive_mask_over_parts_of_the_key_range(seq, kv, nq, nkv, kind, launches):
+    """Few queries over a long cache: the library splits a masked call as it does others.  Gated, and with log-sum-exp and
+    a copy of the output, as the whole range gives them."""
+    from arcaine_b200 import ops
+    ops.clear_device_status()
+    hd, inf = 256, float("inf")
+    g = torch.Generator().manual_seed(9)
+    mask = torch.from_numpy(oracle.fill_causal_mask(seq, kv, kv - seq, 200 if kind == "window" else oracle.INT_MAX)).clone()
+    if kind == "random":
+        mask[torch.rand(seq, kv, generator=g) < 0.5] = -inf
+    elif kind == "blocks":
+        mask[:, :700], mask[:, 1900:2700], mask[7] = -inf, -inf, -inf
+    elif kind == "values":
+        mask += torch.randn(seq, kv, generator=g) * 2
+    mask = mask.cuda()
+    q, k, v, gate = (seeded_bf16(n, h, hd, seed=90 + i).cuda() for i, (n, h) in enumerate([(seq, nq), (kv, nkv), (kv, nkv), (seq, nq)]))
+    run = lambda n, **kw: ops.sdpa_prefill(q, k, v, scale=0.0625, mask_type=ops.MASK_EXPLICIT, mask=mask, num_splits=n, **kw)  # noqa: E731
+    copy = torch.empty_like(q)
+    before = ops.launch_count()
+    out, lse = run(0, return_lse=True, out_copies=torch.tensor([copy.data_ptr()], device="cuda"))
+    assert ops.launch_count() - before == launches
+    want, want_lse = run(1, return_lse=True)
+    assert_close(out, want.float().cpu(), kind, rel_tol=4e-3, abs_tol=1.6e-2)  # (as in test_parts_of_the_key_range)
+    assert torch.equal(copy, out)
+    fin = torch.isfinite(want_lse)
+    assert torch.equal(torch.isfinite(lse), fin) and torch.allclose(lse[fin], want_lse[fin], atol=2e-3)
+    assert_close(run(0, gate=gate), run(1, gate=gate).float().cpu(), kind + " gated", rel_tol=4e-3, abs_tol=1.6e-2)
+    for _ in range(5):
+        assert torch.equal(run(0), out)
+    assert ops.device_status() == (0, 0)
+
+
 @pytest.mark.parametrize("scale", [0.0625, 1.0, 1.5])
 def test_additive_mask_of_the_lowest_value_infinity_and_nan(scale):
     """Scanned or read by the attention kernel itself (no workspace), a mask means the same: the type's lowest value hides
