@@ -143,6 +143,26 @@ def test_additive_mask_over_parts_of_the_key_range(seq, kv, nq, nkv, kind, launc
     assert ops.device_status() == (0, 0)
 
 
+@pytest.mark.parametrize("hd", [128, 256])
+@pytest.mark.parametrize("kv", [260, 333])  # rows of whole groups of four values, and not
+def test_additive_mask_at_any_alignment(hd, kv):
+    """A mask whose buffer, or whose rows, do not start at multiples of 16 bytes gives the same bits."""
+    from arcaine_b200 import ops
+    ops.clear_device_status()
+    seq, nq, nkv = 150, 4, 2
+    q, k, v = seeded_bf16(seq, nq, hd, seed=1).cuda(), seeded_bf16(kv, nkv, hd, seed=2).cuda(), seeded_bf16(kv, nkv, hd, seed=3).cuda()
+    g = torch.Generator().manual_seed(5)
+    mask = torch.randn(seq, kv, generator=g)
+    mask[torch.rand(seq, kv, generator=g) < 0.2] = -float("inf")
+    got = []
+    for shift in range(4):
+        buf = torch.empty(seq * kv + 4, device="cuda")[shift:shift + seq * kv].view(seq, kv)
+        buf.copy_(mask)
+        got.append(ops.sdpa_prefill(q, k, v, scale=0.0625, mask_type=ops.MASK_EXPLICIT, mask=buf))
+    assert_close(got[0], oracle.sdpa_f32(q.cpu(), k.cpu(), v.cpu(), scale=0.0625, mask_type=1, mask=mask.numpy())[0], f"kv {kv}")
+    assert all(torch.equal(o, got[0]) for o in got) and ops.device_status() == (0, 0)
+
+
 @pytest.mark.parametrize("scale", [0.0625, 1.0, 1.5])
 def test_additive_mask_of_the_lowest_value_infinity_and_nan(scale):
     """Scanned or read by the attention kernel itself (no workspace), a mask means the same: the type's lowest value hides
