@@ -268,8 +268,9 @@ static int choose_wide_splits(const arc_sdpa_prefill_params* p, int q_tiles, con
     int most = (p->kv_len + 127) / 128;  // key blocks of the longest unit
     // What an additive mask hides is not known here.  Over the few blocks of a window the parts of 2048 rows cost 5 us more
     // than they save (256 queries of 8 heads over 2304 keys: 16.4 us whole and 21.1; with all keys seen 30.3 and 23.9); 1024
-    // rows are even (64 queries of 16 heads over 4096 keys: 15.9 and 15.6; 45 and 20).  A longer cache is worth it in any case.
-    if (p->mask_type == ARC_MASK_EXPLICIT && most <= 32 && (long long)p->batch * p->seq * p->nq > 1024) return 1;
+    // rows are even (64 queries of 16 heads over 4096 keys: 15.9 and 15.6; 45 and 20).  A longer cache is worth it in any case (a
+    // bias per key, 128 queries of 16 heads over 4096 keys: 116 us whole).
+    if (p->mask_type == ARC_MASK_EXPLICIT && most <= 24 && (long long)p->batch * p->seq * p->nq > 1024) return 1;
     if (p->mask_type == ARC_MASK_CAUSAL && p->window > 0 && p->window < p->kv_len && !p->block_ids) most = std::min(most, (p->window + 255) / 128 + 1);
     int best = 1;
     double least = 1.13 * most;
