@@ -564,7 +564,9 @@ static bool size_decode_cta(int hd, int nkv_cta, int batch, int extra, int smem_
 // lengths on the device) and 0.1 us per sequence for the second launch and the records.  (Measured over
 // batches of 1 to 64 and lengths of 64 to 8192 for five head layouts: one token over 513 keys, 24/4 heads: 6.7 and 6.0 us,
 // 64 sequences of 512 keys, 16/2 heads: 17.8 and 9.9.)  Lengths on the device are not known here: the longest sequence is
-// taken to be as long as its bound says, or twice the mean of a packed cache, the others half of that.
+// taken to be as long as its bound says, or twice the mean of a packed cache, the others half of that.  If they are not and
+// one sequence holds nearly all keys, its cluster works alone: 20000 keys among 31 sequences of 400 took 52 to 228 us where
+// shares take 16 to 34.  So the form is left alone where that could cost more than 24 us and 1.3 times what shares do.
 static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceState& ds, int nkv_cta, DecodePlan* plan) {
     if (p->num_ctas != 0 || p->xchg_world > 1 || p->kv_rows_total == 0 || p->batch > 1024) return;
     const int G = p->nq / p->nkv;
@@ -583,13 +585,18 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
     }
     const double ctas = (double)p->batch * (p->nkv / heads) * csize;
     const double all = heads * p->hd >= 1024 ? 6.0e6 : 6.9e6 - 6e3 * (ds.sm_count - ctas);
-    const double t_longest = longest / csize * heads * p->hd * 4.0 / (p->hd == 256 ? 93e3 : 105e3);
-    const double t_cluster = 5.2 + std::max(t_longest, total * p->nkv * p->hd * 4.0 / all);
-    const double t_shares = (p->kv_len ? 8.0 : 7.2) + 0.1 * p->batch + total * p->nkv * p->hd * 4.0 / 7.0e6;
-    if (t_cluster > t_shares) return;
+    const double per_longest = heads * p->hd * 4.0 / csize / (p->hd == 256 ? 93e3 : 105e3), per_key = p->nkv * p->hd * 4.0;
+    auto t_cluster = [&](double most, double keys) { return 5.2 + std::max(most * per_longest, keys * per_key / all); };
+    auto t_shares = [&](double keys) { return (p->kv_len ? 8.0 : 7.2) + 0.1 * p->batch + keys * per_key / 7.0e6; };
+    if (t_cluster(longest, total) > t_shares(total)) return;
+    if (p->kv_len) {
+        const double most = p->max_kv_len > 0 ? std::min((double)p->max_kv_len, (double)p->kv_rows_total) : (double)p->kv_rows_total;
+        const double wide_group = G <= 8 ? 1.0 : p->hd == 256 ? 4.0 : 1.6;  // (two tiles of heads a warp: the rates are that much lower)
+        if (t_cluster(most * wide_group, most) > std::max(24.0, 1.3 * t_shares(most))) return;
+    }
     DecodePlan one = *plan;
     // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where
-    // the stages were, at least two: 64 * hd floats a warp, at most 16 * (hd + 5) needed.)
+    // the stages were, at least two: 32 * hd floats a warp, at most 16 * (hd + 5) needed.)
     if (!size_decode_cta(p->hd, heads, 0, heads * G * (p->hd + csize) * 4, ds.smem_optin, &one)) return;
     one.cluster = true;
     one.groups = p->nkv / heads;

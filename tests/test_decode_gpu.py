@@ -325,6 +325,35 @@ def test_one_launch_form(ops, B, nq, nkv, hd, lens):
         assert torch.allclose(lse[b].cpu(), wl[0], atol=2e-3)
 
 
+@pytest.mark.parametrize("lens,nq,nkv,hd,block,packed", [
+    ([20000] + [400] * 31, 16, 2, 128, 2, 2),  # its cluster alone would take three times as long
+    ([8000] + [14] * 15, 24, 4, 256, 2, 2),
+    ([700] * 3, 24, 4, 256, 1, 1),             # whatever the lengths were, a cluster is fast enough
+    ([500, 16000], 8, 4, 128, 1, 1),
+])
+def test_batches_that_may_be_one_long_sequence(ops, lens, nq, nkv, hd, block, packed):
+    """Launches of a call whose lengths only the device knows, over a block cache as long as the longest sequence and over
+    a packed one; the same result either way."""
+    B, cap = len(lens), max(lens)
+    q = seeded_bf16(B, nq, hd, seed=1).cuda()
+    kp, vp = seeded_bf16(sum(lens), nkv, hd, seed=2).cuda(), seeded_bf16(sum(lens), nkv, hd, seed=3).cuda()
+    offs = [sum(lens[:b]) for b in range(B)]
+    k, v = (torch.zeros(B, cap, nkv, hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    for b, n in enumerate(lens):
+        k[b, :n], v[b, :n] = kp[offs[b]:offs[b] + n], vp[offs[b]:offs[b] + n]
+    kl, ko = torch.tensor(lens, dtype=torch.int32, device="cuda"), torch.tensor(offs, dtype=torch.int64, device="cuda")
+    launches = []
+    for call in (lambda: ops.sdpa_decode(q, k, v, scale=hd ** -0.5, kv_len=kl),
+                 lambda: ops.sdpa_decode(q, kp, vp, scale=hd ** -0.5, kv_len=kl, kv_row_offset=ko)):
+        before = ops.launch_count()
+        out = call()
+        launches.append(ops.launch_count() - before)
+        for b in {0, 1, B - 1}:
+            want = oracle_decode(q[b].cpu(), kp[offs[b]:offs[b] + lens[b]].cpu(), vp[offs[b]:offs[b] + lens[b]].cpu(), hd ** -0.5)
+            assert_close(out[b], want[0][0], f"seq {b}")
+    assert launches == [block, packed]
+
+
 @pytest.mark.parametrize("B,nq,nkv,hd,length,ctas", [
     (1, 24, 4, 256, 6100, 148),   # few rows: 64 columns of a row per merge block, every share one record
     (1, 6, 2, 128, 9000, 600),    # more records of a row than a lane of the merge block keeps of their log-sum-exps
