@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(288, 1)
             mbar_init(&empty[s], ncw);
         }
         fence_mbar_init();
+        if (CLUSTER) cum[0] = 1;  // results may be written: until a status or a wait that runs out, in any CTA, clears it
     }
     long long g0 = 0, g1 = 0;  // this CTA's keys, counted over the sequences laid end to end (CLUSTER: of its own sequence)
     int b_first = 0, my_len = 0;
@@ -526,6 +527,8 @@ __global__ void __launch_bounds__(288, 1)
             consumer_sync(ncw);
             consumer_sync(ncw);
         }
+        // (A producer that gives up leaves a consumer waiting, which comes here.)
+        if (CLUSTER && !ok && lane < p.ncta) st_cluster_f32(map_to_cta(smem_u32(cum), lane), 0.0f);
         // (CLUSTER: no keys: an empty record)
         if (CLUSTER && !folded && lane < p.ncta)
             for (int n = slice; n < G; n += p.slices)
@@ -534,7 +537,7 @@ __global__ void __launch_bounds__(288, 1)
     if constexpr (CLUSTER) {
         // This CTA's columns, two a thread.  Every record is in its own shared memory by now: read out of the other CTAs
         // instead, 16 loads a thread, this step took 2100 clk.
-        if (threadIdx.x == 0) cum[0] = work && fault == 0u;
+        if (threadIdx.x == 0 && (!work || fault != 0u)) cum[0] = 0;
         const int items = rows * (dc / 2), b = blockIdx.z;
         auto offset_of = [&](int item) {
             return (long long)b * p.o_stride_b + (long long)(head0 * G + (item >> (dc_log2 - 1))) * HD + blockIdx.x * dc + (item & (dc / 2 - 1)) * 2;

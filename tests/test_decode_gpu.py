@@ -251,6 +251,29 @@ def test_exchange_fold_with_the_other_ranks_record_already_in_place(ops):
     assert (xbuf[step & 1, 0, :, :, 1] == step).all() and (scratch[step & 1, 0, :, :, 1] == step).all()
 
 
+@pytest.mark.parametrize("on_device", [False, True])
+@pytest.mark.parametrize("ctas,launches", [(0, 1), (148, 2)])
+def test_no_form_writes_a_result_under_a_status(ops, on_device, ctas, launches):
+    """Any status keeps a call from its outputs, whichever form it takes and whoever knows the lengths.  (A wait that runs out
+    in the middle of the one-launch form does the same through a flag in every CTA of the cluster; it cannot be made to run
+    out here without a broken kernel.)"""
+    B, nq, nkv, hd, n = 2, 8, 2, 128, 300
+    q, k = seeded_bf16(B, nq, hd, seed=1).cuda(), seeded_bf16(B, n, nkv, hd, seed=2).cuda()
+    lens = torch.full((B,), n, dtype=torch.int32, device="cuda")
+    ops.sdpa_decode(q, k, k, scale=0.1, kv_len=lens + 1)  # past the cache: sets a status
+    assert ops.device_status()[0] == ops.FAULT_BAD_KV_RANGE
+    out, o32, lse = (torch.full(s, 3.0, dtype=t, device="cuda") for s, t in
+                     (((B, nq, hd), torch.bfloat16), ((B, nq, hd), torch.float32), ((B, nq), torch.float32)))
+    before = ops.launch_count()
+    ops.sdpa_decode(q, k, k, scale=0.1, kv_len=lens if on_device else n, num_ctas=ctas, out=out, return_partial=True, partial_out=o32,
+                    partial_lse=lse)
+    assert ops.launch_count() - before == launches
+    torch.cuda.synchronize()
+    assert all((t.float() == 3.0).all() for t in (out, o32, lse))
+    ops.clear_device_status()
+    assert not (ops.sdpa_decode(q, k, k, scale=0.1, kv_len=lens if on_device else n, num_ctas=ctas, out=out).float() == 3.0).all()
+
+
 def test_exchange_of_one_rank_as_a_list(ops):
     q, k, v = seeded_bf16(1, 4, 128, seed=71).cuda(), seeded_bf16(1, 300, 1, 128, seed=72).cuda(), seeded_bf16(1, 300, 1, 128, seed=73).cuda()
     peers = torch.zeros(1, dtype=torch.int64, device="cuda")
