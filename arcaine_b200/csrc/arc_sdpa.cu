@@ -1059,9 +1059,13 @@ static int fill_mask(float* mask, const int32_t* block_ids, int32_t q_len, int32
     if (q_len < 0 || kv_len < 0) return ARC_ERR_BAD_SHAPE;
     if (q_len == 0 || kv_len == 0) return ARC_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // a block writes 1024 keys of a row; a grid's y extent ends at 65535, longer masks loop
-    const dim3 grid((unsigned)((kv_len + 1023) / 1024), (unsigned)(q_len < 65535 ? q_len : 65535));
-    ARC_CUDA(launch_dependent(block_ids ? fill_causal_mask_kernel<true> : fill_causal_mask_kernel<false>, grid, dim3(256), 0, st, 1,
+    // a block writes 1024 keys of a row, or several rows that are shorter; a grid's y extent ends at 65535, longer masks loop
+    unsigned x = 256;
+    while (x > 1 && (int64_t)x * 2 >= kv_len) x /= 2;
+    const unsigned y = 256 / x;
+    const int64_t rows = ((int64_t)q_len + y - 1) / y;
+    const dim3 grid((unsigned)(((int64_t)kv_len + 4 * x - 1) / (4 * x)), (unsigned)(rows < 65535 ? rows : 65535));
+    ARC_CUDA(launch_dependent(block_ids ? fill_causal_mask_kernel<true> : fill_causal_mask_kernel<false>, grid, dim3(x, y), 0, st, 1,
                               mask, block_ids, (int)q_len, (int)kv_len, (int)past_offset, (int)sliding_window));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return ARC_OK;

@@ -228,6 +228,19 @@ def test_a_workspace_that_cannot_be_used_costs_time_only(room, shift):
     assert ops.device_status() == (0, 0) and not ws.any()
 
 
+@pytest.mark.parametrize("seq,kv", [(1, 1), (7, 3), (300, 64), (1000, 65), (513, 512), (65, 1025), (70000, 5), (40000, 513)])
+def test_mask_buffers_of_any_shape(seq, kv):
+    """Rows that share a block, rows of several blocks, more rows than a grid has blocks; nothing beside the buffer."""
+    from arcaine_b200 import ops
+    past = max(0, kv - seq)
+    buf = torch.full((seq * kv + 64,), 7.0, device="cuda")
+    ops.fill_causal_mask(seq, kv, past, 50, out=buf[:seq * kv].view(seq, kv))
+    i = torch.arange(seq, device="cuda")[:, None] + past
+    j = torch.arange(kv, device="cuda")[None] + past - (kv - seq)
+    want = torch.zeros(seq, kv, device="cuda").masked_fill_((j > i) | (j < i - 49), -float("inf"))
+    assert torch.equal(buf[:seq * kv].view(seq, kv), want) and (buf[seq * kv:] == 7.0).all()
+
+
 def test_vision_blocks_longer_than_a_search_step():
     """Block ids looked up in the kernel (128 keys a step, 32 rows a warp) against the additive buffer of the same rule:
     blocks of one token, next to each other, across warps and tiles, longer than a step, and up to the last key."""
