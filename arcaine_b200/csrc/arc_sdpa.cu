@@ -1065,7 +1065,9 @@ static int fill_mask(float* mask, const int32_t* block_ids, int32_t q_len, int32
     const unsigned y = 256 / x;
     const int64_t rows = ((int64_t)q_len + y - 1) / y;
     const dim3 grid((unsigned)(((int64_t)kv_len + 4 * x - 1) / (4 * x)), (unsigned)(rows < 65535 ? rows : 65535));
-    ARC_CUDA(launch_dependent(block_ids ? fill_causal_mask_kernel<true> : fill_causal_mask_kernel<false>, grid, dim3(x, y), 0, st, 1,
+    auto kernel = y > 1 ? (block_ids ? fill_causal_mask_kernel<true, true> : fill_causal_mask_kernel<false, true>)
+                        : (block_ids ? fill_causal_mask_kernel<true, false> : fill_causal_mask_kernel<false, false>);
+    ARC_CUDA(launch_dependent(kernel, grid, dim3(x, y), 0, st, 1,
                               mask, block_ids, (int)q_len, (int)kv_len, (int)past_offset, (int)sliding_window));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return ARC_OK;

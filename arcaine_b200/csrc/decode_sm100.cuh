@@ -999,16 +999,16 @@ __global__ void mul_sigmoid_kernel(uint16_t* a, const uint16_t* gate, long long 
 // block_ids (one int per absolute position, -1 = text) tokens of the same non-negative block also
 // see each other's future: fill_causal_mask_with_block_ids, attention_mask.hpp:44-73.
 // Bound by the stores: a thread writes four consecutive keys of one row, 16 bytes at once where the row allows it, and
-// divides nothing (one element per thread and a division per element took 13 us for 1000 x 1300).  Short rows share a block
-// (blockDim.y of them; one each took 69 us for 70000 x 64).
-template <bool IDS>
+// divides nothing (one element per thread and a division per element took 13 us for 1000 x 1300).  SHORT: rows share a block
+// (blockDim.y of them; one each took 69 us for 70000 x 64.  An instance of its own: the general one was 0.5 us slower with it).
+template <bool IDS, bool SHORT>
 __global__ void fill_causal_mask_kernel(float* mask, const int* block_ids, int q_len, int kv_len, int past_offset, int window) {
     grid_dependency_wait();
     grid_launch_dependents();
     const int j0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (j0 >= kv_len) return;
     const int first = past_offset - (kv_len - q_len);  // absolute position of key 0
-    for (int qi = blockIdx.y * blockDim.y + threadIdx.y; qi < q_len; qi += gridDim.y * blockDim.y) {
+    for (int qi = SHORT ? blockIdx.y * blockDim.y + threadIdx.y : blockIdx.y; qi < q_len; qi += SHORT ? gridDim.y * blockDim.y : gridDim.y) {
         const int q_global = past_offset + qi;
         const int qb = IDS ? block_ids[q_global] : -1;
         float v[4];
