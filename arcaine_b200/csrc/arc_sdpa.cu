@@ -45,9 +45,6 @@ struct DeviceState {
     uint32_t* fault = nullptr;
     int sm_count = 0;
     int smem_optin = 0;
-    // largest cluster size (2, 4 or 8; 0 = none) the cluster form of the prefill kernel can be launched with, per head dim
-    // [head dim 128 / 256][log2(cluster size)]: how many clusters of 2 or 4 CTAs of the cluster form of the
-    // prefill kernel the device can hold at once (0: that size cannot be launched)
     int decode_clusters[4] = {0, 0, 0, 0};  // [log2(size)]: clusters of the one-launch decode the device holds at once
     WideRoom wide;
 };
@@ -298,10 +295,10 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const Wi
     const bool scanned_mask = p->mask_type == ARC_MASK_EXPLICIT && p->hd == 256 && p->num_splits <= 1;
     if (splits == 0 && p->hd == 256) splits = choose_wide_splits(p, plan->q_tiles, room);
     if (splits == 0) {
-        // Split the key range only when the tiles alone leave most SMs idle and there are enough key blocks
-        // to pay for folding the parts again (measured: about 8 us for the fold against 1.3-2 us per key
-        // block; with fewer than ten blocks a tile is faster in one piece, and more than eight parts cost
-        // more than they save).
+        // Head dim 128: split the key range only when the tiles alone leave most SMs idle and there are enough key
+        // blocks to pay for folding the parts again.  A block takes 1.3 us, records and merge 3 to 5 in all (one tile row of
+        // 8 heads: 1024 keys 15.5 us whole, 11.2 in eight parts; 1280 keys 17.9 and 12.4; 512 keys 10.1 and 10.5).  The line
+        // at ten blocks was drawn when the merge took 8 us; five to nine blocks of few tiles would gain too.
         splits = 1;
         if (tiles * 2 <= sm_count && kv_blocks >= 10) {
             splits = (int)(sm_count / tiles);
@@ -412,9 +409,11 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         const bool head_pair = ((p->nq / p->nkv) & 1) == 0;
         const long long pair_tiles = head_pair ? (long long)plan.q_tiles * (p->nq / 2) * p->batch
                                                : (long long)((p->seq + 255) / 256) * p->nq * p->batch;
-        // Measured: a pair of tiles costs 1.7 single tiles.  Tiles come in waves of one per SM, so the
-        // kernel with the cheaper whole number of waves wins (512 pair tiles on 148 SMs are 4 waves,
-        // the same rows as 1024 single tiles are 7: the single-tile kernel is then faster).
+        // Tiles come in waves of one per SM, and the kernel with the cheaper whole number of waves wins, a pair taken for 1.7
+        // single tiles.  That was measured with earlier kernels; with these a wave of pairs costs 1.13 to 1.18 waves of
+        // single tiles (64 pairs 18.9 us, 128 tiles 16.7 over 1024 keys; 57.3 and 49.0 over 4096).  The line is the same for
+        // one wave of single tiles against one of pairs, and for two or more against half as many; it is drawn too high
+        // where three waves stand against two (odd groups).
         const long long single_tiles = (long long)plan.q_tiles * p->nq * p->batch;
         const long long sms = ds->sm_count;
         // The pairs left over after the last whole wave of CTAs are cut into their two heads when every SM then
@@ -425,8 +424,8 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         const bool cut_tail = !kp.ids && head_pair && full_waves > 0 && left > 0 && 2 * left <= sms;
         const double cost_pair = cut_tail ? 1.7 * (double)full_waves + 1.05 : 1.7 * (double)((pair_tiles + sms - 1) / sms);
         const double cost_single = (double)((single_tiles + sms - 1) / sms);
-        // (Vision blocks: the one-tile kernel also needs a launch for the span ends, and takes an SM twice as long per wave:
-        // 1257 tokens of 16 heads 43.7 us, two tiles at a time 24.6.)
+        // (Vision blocks: the one-tile kernel also needs a launch for the span ends and twice as many waves: 1257 tokens of
+        // 16 heads 43.7 us, two tiles at a time 24.6.)
         const bool use_pair = forced == 2 || (forced == 0 && (kp.ids || cost_pair <= cost_single));
         if (use_pair) {
             if (pair_tiles > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;

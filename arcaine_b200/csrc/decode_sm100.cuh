@@ -584,9 +584,9 @@ __global__ void __launch_bounds__(288, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Merge of the decode partials.  grid = (nq, batch); the block recomputes the
-// same share boundaries the decode kernel used to find the records of its
-// sequence: CTAs [c_first, c_last] x slices, record index (cta + b)*slices + s.
+// Merge of the decode partials.  grid = (nq, batch, column blocks); every warp of a
+// block recomputes the share boundaries the decode kernel used, which say where the
+// records of its sequence are: CTAs [c_first, c_last], record index (cta + b)*slices + s.
 // ---------------------------------------------------------------------------
 struct DecodeMergeParams {
     const float* part_o;
@@ -850,9 +850,9 @@ __global__ void __launch_bounds__(MERGE_THREADS, XCHG || COLS < 256 ? 1 : 4) sdp
 // ---------------------------------------------------------------------------
 // Merge of `num_parts` uniformly strided partial sets: part_o (parts, rows, hd),
 // part_lse (parts, rows), consecutive parts o_part_stride / lse_part_stride
-// elements apart (so one packed record per part works too).  One block per row.  Used for split prefill tiles and
+// elements apart (so one packed record per part works too).  One warp per row.  Used for split prefill tiles and
 // for records gathered from other GPUs.  out rows are contiguous (rows, hd)
-// unless row_tokens > 0, in which case row = (b, t, h) is scattered with the
+// unless seq > 0, in which case row = (b, t, h) is scattered with the
 // given strides (prefill output layout).
 // ---------------------------------------------------------------------------
 struct UniformMergeParams {

@@ -170,10 +170,9 @@ template <int MODE>
 __device__ __forceinline__ void chunk_exp(const uint32_t (&v)[32], uint32_t (&pk)[16], float (&ls)[4], float sl,
                                           float m_eff, int key0, const RowMask& rm) {
     if constexpr (MODE == 0) {
-        // Every key visible.  Plain fp32 instructions on purpose: measured on B200, a warp issues an
-        // fma.f32x2 / add.f32x2 only every ~8 clocks (the scalar forms every clock), about as often as
-        // an ex2.approx; both the packed forms and a polynomial 2^x on the FMA pipe for a share of
-        // the scores made the kernel slower.
+        // Every key visible.  Plain fp32 instructions: the packed forms take the pipe no shorter, and where the loop fits
+        // the instruction cache without them, as here, they made the kernel slower; so did a polynomial 2^x on the FMA
+        // pipe for a share of the scores.  (The kernels with two tiles need the shorter code.)
         const float nm = -m_eff;
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {

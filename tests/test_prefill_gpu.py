@@ -89,17 +89,18 @@ def test_key_range_splits_agree(ops, splits):
 
 @pytest.mark.parametrize("hd", [128, 256])
 @pytest.mark.parametrize("seq,kv_len,nq,nkv,mask_type,window,parts", [
+    # (parts: what head dim 128 takes; 256 chooses by units of two tiles)
     (256, 1300, 28, 4, 0, oracle.INT_MAX, 2),   # 56 tiles on 148 SMs, 11 key blocks: two parts
-    (200, 1300, 28, 4, 3, 300, 2),              # the same ragged and windowed: CTAs of a cluster without keys
+    (200, 1300, 28, 4, 3, 300, 2),              # the same ragged and windowed: parts without keys
     (256, 2100, 16, 8, 0, oracle.INT_MAX, 4),   # 32 tiles, 17 key blocks (the last one ragged): four parts
-    (130, 2100, 16, 2, 3, 100, 4),              # 32 tiles, a window: most CTAs of a cluster see no key
+    (130, 2100, 16, 2, 3, 100, 4),              # 32 tiles, a window: most parts see no key
     (130, 2100, 4, 2, 0, oracle.INT_MAX, 8),    # 8 tiles: eight parts, always two launches
     (256, 1200, 8, 4, 3, oracle.INT_MAX, 5),    # 16 tiles, 10 key blocks: five parts, two launches
 ])
 def test_key_range_splits_the_library_chooses(ops, hd, seq, kv_len, nq, nkv, mask_type, window, parts):
-    """Splits the library chooses itself: two or four parts at head dim 256 run as one thread-block cluster per
-    tile whose CTAs fold their accumulators through distributed shared memory (one launch); everything else as
-    partial records and a merge launch.  With the gate and the log-sum-exp output."""
+    """Splits the library chooses itself: at head dim 256 few parts run as one thread-block cluster per unit that folds
+    them itself (one launch), or none at all; everything else as partial records and a merge launch.  With the gate
+    and the log-sum-exp output."""
     before = ops.launch_count()
     run_case(ops, seq, kv_len, nq, nkv, hd, hd ** -0.5, mask_type, window, seed=500 + hd + seq, gate=True, lse=True)
     torch.cuda.synchronize()
@@ -115,7 +116,7 @@ def test_output_copies_are_written_by_every_epilogue(ops, case):
     seq, kv, nq, nkv, hd, mask, win, splits = {
         "hd128": (1024, 1024, 8, 4, 128, 3, 256, 0),         # (the two-tile kernel's copies: test_prefill_pair_gpu.py)
         "single": (300, 300, 4, 2, 256, 3, oracle.INT_MAX, 1),
-        "cluster": (256, 2100, 16, 8, 256, 0, oracle.INT_MAX, 0),    # 32 tiles, 17 key blocks: clusters of four
+        "cluster": (256, 2100, 16, 8, 256, 0, oracle.INT_MAX, 0),    # 16 units, 17 key blocks: three parts, folded in a cluster
         "two_launch": (256, 1200, 4, 2, 128, 0, oracle.INT_MAX, 3),
         "nothing_visible": (200, 100, 4, 2, 128, 3, oracle.INT_MAX, 0),  # the first 100 queries see no key
     }[case]
