@@ -49,18 +49,19 @@ struct PairCfg {
     static constexpr int K_STAGES = 2;
     static constexpr int V_STAGES = 2;
     static constexpr int TMEM_COLS = 512;
-    static constexpr int COL_S = 0;    // + 128 * pipeline
+    static constexpr int COL_S = 0;    // the score buffer, used by the pipelines in turn
+    static constexpr int COL_P = 128;  // + 64 * pipeline
     static constexpr int COL_O = 256;  // + 128 * pipeline
-    // q_full[2] q_empty[2] k_first k_first_used kv_full[2] kv_empty[2] then per pipeline:
-    // s_full p_part[2] o_full o_empty fin[2]; then gate[4][2], two per epilogue warp
-    static constexpr int NUM_BARS = 4 + 2 + 2 * K_STAGES + 22;
+    // q_full[2] q_empty[2] k_first k_first_used kv_full[2] kv_empty[2] s_free then per pipeline:
+    // s_full p_part[2] pv_done o_full o_empty fin[2]; then gate[4][2], two per epilogue warp
+    static constexpr int NUM_BARS = 4 + 2 + 2 * K_STAGES + 1 + 24;
     static constexpr int FIN_FLOATS = 2 * 2 * 128;  // [tile parity][pipeline][row] row sum
     static constexpr int SMEM_BYTES = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 4 * 8192 + NUM_BARS * 8 + 16 + FIN_FLOATS * 4 + 32;  // (4 x 8 KB: output stage; 32: first unit)
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
     static constexpr int SOFTMAX_WARPS = 8;   // four per pipeline
     static constexpr int EPILOGUE_WARP = 8;   // four warps
     static constexpr int PRODUCER_WARP = 12;
-    static constexpr int ISSUER_WARP = 13;    // (warp 14 idles)
+    static constexpr int S_ISSUER_WARP = 13;  // warp 14 issues the P V MMAs
     static constexpr int Q_PRODUCER_WARP = 15;
     static constexpr int THREADS = 32 * 16;
     // The budgets may only redistribute what the CTA holds at launch (threads x the per-thread
@@ -339,9 +340,11 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     uint64_t* k_first_used = bars + 5;  // both pipelines' first scores have been computed
     uint64_t* kv_full = bars + 6;       // [2] V of a block and K of the block after it
     uint64_t* kv_empty = bars + 8;      // [2] both have been used by both pipelines
-    uint64_t* s_full = kv_empty + 2; // [2] per pipeline from here on
+    uint64_t* s_free = kv_empty + 2; // the softmax warps of the pipeline that has had the scores last hold them in registers
+    uint64_t* s_full = s_free + 1;   // [2] per pipeline from here on
     uint64_t* p_part = s_full + 2;   // [pipeline][part]: P of keys 0-95 / 96-127 of the block is in tensor memory
-    uint64_t* o_full = p_part + 4;   // one phase per tile: the tile's last O += P V has completed
+    uint64_t* pv_done = p_part + 4;  // O += P V of the block has completed: P may be replaced, O rescaled
+    uint64_t* o_full = pv_done + 2;  // one phase per tile: the tile's last O += P V has completed
     uint64_t* o_empty = o_full + 2;  // one phase per tile: the epilogue warps have read O out
     // fin[2 * s + (tile & 1)], one phase per second tile: the softmax warps have published the tile's row sums.  Two barriers per pipeline, used in turn, because a tile of one key block needs no
     // O += P V to finish: with one barrier the softmax warps could complete it for tile n + 1 while a slow
@@ -372,6 +375,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             mbar_init(&s_full[s], 1);
             mbar_init(&p_part[2 * s], 4);
             mbar_init(&p_part[2 * s + 1], 4);
+            mbar_init(&pv_done[s], 1);
             mbar_init(&o_full[s], 1);
             mbar_init(&o_empty[s], 4);
             mbar_init(&fin[2 * s], 4);
@@ -380,9 +384,10 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         for (int w = 0; w < 8; ++w) mbar_init(&gate_bar[w], 1);
         mbar_init(k_first, 1);
         mbar_init(k_first_used, 1);
+        mbar_init(s_free, 4);
         for (int s = 0; s < 2; ++s) {
             mbar_init(&kv_full[s], 1);
-            mbar_init(&kv_empty[s], 1);
+            mbar_init(&kv_empty[s], 2);
         }
         fence_mbar_init();
     }
@@ -406,6 +411,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
     tc_fence_after_sync();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
     const int total_tiles = *abort_slot ? 0 : p.total_tiles;  // a status is set: walk an empty list
+    constexpr uint32_t TILE16 = C::TILE_BYTES >> 4, CHUNK16 = C::CHUNK_BYTES >> 4;  // descriptor units
 
     if (warp >= C::PRODUCER_WARP) {
         reg_dealloc<C::REGS_CONTROL>();
@@ -505,134 +511,116 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     }
                 }
             }
-        } else if (warp == C::ISSUER_WARP) {
-            // -------------------------------------------------------------- MMA issuer of both pipelines
-            // The whole warp runs this code and one lane issues: addresses stay in the uniform datapath.  The MMA
-            // loops are rolled (four MMAs a turn), because this code shares an instruction cache of about 8 KB per
-            // scheduler with the softmax loop: unrolled, every MMA waited for its own code (125 clk apart, not 64).
+        } else if (warp == C::S_ISSUER_WARP) {
+            // -------------------------------------------------------------- S = Q K^T of both pipelines
+            // The whole warp runs this code and one lane issues: addresses stay in the uniform datapath.
             //
-            // ONE thread serves both pipelines, A's O += P V and next S, then B's: what the two need next goes
-            // through the tensor pipe one after the other, so A's scores are ready about 800 clk before B's and
-            // the pipelines stay out of phase by themselves.  (With a thread each their MMAs interleaved, both got
-            // their scores at the same time, and softmax and tensor pipe worked in turns: 4400 clk per pair of blocks.)
-            //
-            // A step is one key block of one pipeline: O += P V(j), then S(j+1) over the P just consumed — at the end
-            // of a unit the first scores of the next one.  What a step needs besides P (V, the next K, Q, a free
-            // accumulator; addresses) is seen to before its P is waited for, while the softmax warps still work on it.
+            // The pipelines' scores go through the one buffer in turn: a pipeline's next scores are computed as soon as
+            // the other one's softmax warps have taken theirs into registers, which they do when they are through with
+            // the block before.  So A's scores of block j + 1 are computed while A exponentiates block j and are there
+            // when it is done, and the two are half a period apart by themselves.
             constexpr uint32_t IDESC_QK = make_idesc_bf16(128, 128, false);
-            constexpr uint32_t IDESC_PV = make_idesc_bf16(128, HD, true);
-            constexpr uint32_t TILE16 = C::TILE_BYTES >> 4, CHUNK16 = C::CHUNK_BYTES >> 4;  // descriptor units
             const uint64_t dQ = make_smem_desc_sw128(smem_u32(sQ), 16, 1024);
             const uint64_t dK = make_smem_desc_sw128(smem_u32(sK), 16, 1024);
-            const uint64_t dV = make_smem_desc_sw128(smem_u32(sV), C::CHUNK_BYTES, 1024);
             static_assert(KS == 2 && VS == 2 && HD == 128, "ring arithmetic assumes two stages and head dim 128");
-            int gu = 0;            // ring position: union key blocks passed so far
-            uint32_t g_par = 0u;   // bit s: parity of pipeline s's key blocks whose P V has been issued
-            uint32_t q_par = 0u;   // bit s: parity of its tiles whose first scores have been issued
-            uint32_t o_par = 3u;   // bit s: parity to wait for before its next tile's first P V (starts "complete")
+            int r = 0;            // ring position: key blocks so far
+            int ns = 0;           // score blocks so far, of both pipelines
+            uint32_t q_par = 0u;  // bit s: parity of pipeline s's tiles so far
             bool ok = true;
-            // S = Q K(j)^T of pipeline s at ring position r (a block the pipeline does not use: nothing).
-            auto issue_scores = [&](const PairWork& pw, int s, int j, int r) {
-                if (j >= pw.lo_of(s) && j < pw.hi_of(s)) {
-                    const uint32_t tS = tmem_base + C::COL_S + s * 128;
-                    const uint64_t da = dQ + (uint64_t)(s * TILE16), db = dK + (uint64_t)((r & 1) * TILE16);
-                    umma_ss_x4<2, 2>(tS, da, db, IDESC_QK, 0u);  // 64 head-dim columns
-                    umma_ss_x4<2, 2>(tS, da + CHUNK16, db + CHUNK16, IDESC_QK, 1u);
-                    umma_commit_warp(&s_full[s]);
-                    if (j + 1 == pw.hi_of(s)) umma_commit_warp(&q_empty[s]);
-                }
-            };
-            // Q of a tile whose first scores come next
-            auto await_q = [&](const PairWork& pw, int s, int j) -> bool {
-                if (j != pw.lo_of(s) || j >= pw.hi_of(s)) return true;
-                if (!mbar_wait_inline(&q_full[s], (q_par >> s) & 1u)) {
-                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_Q, s);
-                    return false;
-                }
-                q_par ^= 1u << s;
-                return true;
-            };
             TileCursor cur = *cursor;
-            auto next_unit = [&](PairWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
-                for (; cur.w < total_tiles; cur.advance(p)) {
-                    w = decode_pair<VISION>(p, cur);
-                    if (w.uhi > w.ulo) {
-                        cur.advance(p);
-                        return true;
-                    }
-                }
-                return false;
-            };
-            PairWork pw{};
-            bool have = next_unit(pw);
-            if (have && !mbar_wait_inline(k_first, 0)) {
-                if (lane == 0) report_fault(p.fault, FAULT_WAIT_K, 0u);
-                ok = false;
-            }
-            for (int s = 0; have && ok && s < 2; ++s) {
-                ok = await_q(pw, s, pw.ulo);
-                tc_fence_after_sync();
-                if (ok) issue_scores(pw, s, pw.ulo, 0);
-            }
-            umma_commit_warp(k_first_used);
-            while (have && ok) {
-                PairWork pn = pw;
-                const bool have_next = next_unit(pn);
-                for (int j = pw.ulo; ok && j < pw.uhi; ++j, ++gu) {
-                    const bool more = j + 1 < pw.uhi;           // the next scores belong to this unit
-                    const bool scores = more || have_next;
-                    if (!mbar_wait_inline(&kv_full[gu & 1], (gu >> 1) & 1)) {
-                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_V, gu);
+            for (; ok && cur.w < total_tiles; cur.advance(p)) {
+                const PairWork pw = decode_pair<VISION>(p, cur);
+                for (int j = pw.ulo; ok && j < pw.uhi; ++j, ++r) {
+                    if (!mbar_wait_inline(r ? &kv_full[(r - 1) & 1] : k_first, r ? ((r - 1) >> 1) & 1 : 0)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_K, r);
                         ok = false;
                         break;
                     }
 #pragma unroll 1
                     for (int s = 0; s < 2; ++s) {
-                        const bool act = j >= pw.lo_of(s) && j < pw.hi_of(s);
-                        if (scores && !await_q(more ? pw : pn, s, more ? j + 1 : pn.ulo)) {
+                        if (j < pw.lo_of(s) || j >= pw.hi_of(s)) continue;
+                        if (j == pw.lo_of(s)) {
+                            if (!mbar_wait_inline(&q_full[s], (q_par >> s) & 1u)) {
+                                if (lane == 0) report_fault(p.fault, FAULT_WAIT_Q, s);
+                                ok = false;
+                                break;
+                            }
+                            q_par ^= 1u << s;
+                        }
+                        const uint64_t da = dQ + (uint64_t)(s * TILE16), db = dK + (uint64_t)((r & 1) * TILE16);
+                        if (ns > 0 && !mbar_wait_inline(s_free, (ns - 1) & 1)) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_S, 0x1000u + ns);
                             ok = false;
                             break;
                         }
-                        if (act) {
-                            if (j == pw.lo_of(s)) {
-                                if (!mbar_wait_inline(&o_empty[s], (o_par >> s) & 1u)) {
-                                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x100u + s);
-                                    ok = false;
-                                    break;
-                                }
-                                o_par ^= 1u << s;
-                            }
-                            // P from tensor memory: 16 keys are 8 columns of packed bf16.  V is MN-major:
-                            // 64-element head-dim chunks 16 KB apart, 8-key groups 1024 bytes apart; 16 keys =
-                            // 2048 bytes.  The first 96 keys go to the tensor pipe while the softmax warps are
-                            // still busy with the other 32: what is left for the chain is 128 clk.
-                            const uint32_t tO = tmem_base + C::COL_O + s * 128, tP = tmem_base + C::COL_S + s * 128;
-                            const uint64_t dv = dV + (uint64_t)((gu & 1) * TILE16);
-                            const uint32_t par = (g_par >> s) & 1u;
-                            if (!mbar_wait_inline(&p_part[2 * s], par)) {
-                                if (lane == 0) report_fault(p.fault, FAULT_WAIT_P, gu);
-                                ok = false;
-                                break;
-                            }
-                            tc_fence_after_sync();
-                            umma_ts_x4<8, 128>(tO, tP, dv, IDESC_PV, j > pw.lo_of(s) ? 1u : 0u);
-                            umma_ts_x2<8, 128>(tO, tP + 32, dv + 512, IDESC_PV, 1u);
-                            if (!mbar_wait_inline(&p_part[2 * s + 1], par)) {
-                                if (lane == 0) report_fault(p.fault, FAULT_WAIT_P, 0x1000u + gu);
-                                ok = false;
-                                break;
-                            }
-                            tc_fence_after_sync();
-                            umma_ts_x2<8, 128>(tO, tP + 48, dv + 768, IDESC_PV, 1u);
-                            g_par ^= 1u << s;
-                        }
-                        if (scores) issue_scores(more ? pw : pn, s, more ? j + 1 : pn.ulo, gu + 1);
-                        if (act && j + 1 == pw.hi_of(s)) umma_commit_warp(&o_full[s]);
-                        if (s == 1) umma_commit_warp(&kv_empty[gu & 1]);
+                        ++ns;
+                        tc_fence_after_sync();
+                        umma_ss_x4<2, 2>(tmem_base + C::COL_S, da, db, IDESC_QK, 0u);  // 64 head-dim columns
+                        umma_ss_x4<2, 2>(tmem_base + C::COL_S, da + CHUNK16, db + CHUNK16, IDESC_QK, 1u);
+                        umma_commit_warp(&s_full[s]);
+                        if (j + 1 == pw.hi_of(s)) umma_commit_warp(&q_empty[s]);
                     }
+                    umma_commit_warp(r ? &kv_empty[(r - 1) & 1] : k_first_used);
                 }
-                pw = pn;
-                have = have_next;
+            }
+        } else {
+            // -------------------------------------------------------------- O += P V of both pipelines
+            // A warp of its own: with one warp for all MMAs the tensor pipe ran dry while it looked after the barriers
+            // between two groups (2710 clk per pair of blocks for 2048 of MMAs).
+            constexpr uint32_t IDESC_PV = make_idesc_bf16(128, HD, true);
+            const uint64_t dV = make_smem_desc_sw128(smem_u32(sV), C::CHUNK_BYTES, 1024);
+            int r = 0;             // ring position: key blocks so far
+            uint32_t g_par = 0u;   // bit s: parity of pipeline s's key blocks so far
+            uint32_t o_par = 3u;   // bit s: parity to wait for before its next tile's first P V (starts "complete")
+            bool ok = true;
+            TileCursor cur = *cursor;
+            for (; ok && cur.w < total_tiles; cur.advance(p)) {
+                const PairWork pw = decode_pair<VISION>(p, cur);
+                for (int j = pw.ulo; ok && j < pw.uhi; ++j, ++r) {
+                    if (!mbar_wait_inline(&kv_full[r & 1], (r >> 1) & 1)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_V, r);
+                        ok = false;
+                        break;
+                    }
+#pragma unroll 1
+                    for (int s = 0; s < 2; ++s) {
+                        if (j < pw.lo_of(s) || j >= pw.hi_of(s)) continue;
+                        if (j == pw.lo_of(s)) {
+                            if (!mbar_wait_inline(&o_empty[s], (o_par >> s) & 1u)) {
+                                if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x100u + s);
+                                ok = false;
+                                break;
+                            }
+                            o_par ^= 1u << s;
+                        }
+                        // P from tensor memory: 16 keys are 8 columns of packed bf16.  V is MN-major:
+                        // 64-element head-dim chunks 16 KB apart, 8-key groups 1024 bytes apart; 16 keys =
+                        // 2048 bytes.  The first 96 keys go to the tensor pipe while the softmax warps are
+                        // still busy with the other 32.
+                        const uint32_t tO = tmem_base + C::COL_O + s * 128, tP = tmem_base + C::COL_P + s * 64;
+                        const uint64_t dv = dV + (uint64_t)((r & 1) * TILE16);
+                        const uint32_t par = (g_par >> s) & 1u;
+                        if (!mbar_wait_inline(&p_part[2 * s], par)) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_P, r);
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after_sync();
+                        umma_ts_x4<8, 128>(tO, tP, dv, IDESC_PV, j > pw.lo_of(s) ? 1u : 0u);
+                        umma_ts_x2<8, 128>(tO, tP + 32, dv + 512, IDESC_PV, 1u);
+                        if (!mbar_wait_inline(&p_part[2 * s + 1], par)) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_P, 0x1000u + r);
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after_sync();
+                        umma_ts_x2<8, 128>(tO, tP + 48, dv + 768, IDESC_PV, 1u);
+                        g_par ^= 1u << s;
+                        umma_commit_warp(&pv_done[s]);
+                        if (j + 1 == pw.hi_of(s)) umma_commit_warp(&o_full[s]);
+                    }
+                    umma_commit_warp(&kv_empty[r & 1]);
+                }
             }
         }
     } else if (warp >= C::EPILOGUE_WARP) {
@@ -726,7 +714,8 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;
         const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
-        const uint32_t tS = tmem_base + lane_sel + C::COL_S + s * 128;
+        const uint32_t tS = tmem_base + lane_sel + C::COL_S;
+        const uint32_t tP = tmem_base + lane_sel + C::COL_P + s * 64;
         const uint32_t tO = tmem_base + lane_sel + C::COL_O + s * 128;
         const float sl = p.scale_log2;
         const bool causal = (p.mask_type == 3);
@@ -765,50 +754,55 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 }
                 tc_fence_after_sync();
                 const bool full = __all_sync(0xffffffffu, rm.lo <= kc && kc + C::BN <= rm.hi);
-                for (;;) {
-                    float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                    tmem_ld32(tS, s0);
-                    tmem_ld32(tS + 32, s1);
-                    tmem_wait_ld();
-                    tmem_ld32(tS + 64, s2);  // lands while the maximum of the first half is taken
-                    tmem_ld32(tS + 96, s3);
-                    if (!full) {  // window edge, diagonal, ragged end (two blocks in nine with a 1024-key window)
-                        mask_chunk(s0, kc, rm);
-                        mask_chunk(s1, kc + 32, rm);
-                    }
-                    chunk_max<0>(s0, mr, sl, kc, rm);
-                    chunk_max<0>(s1, mr, sl, kc, rm);
-                    tmem_wait_ld();
-                    if (!full) {
-                        mask_chunk(s2, kc + 64, rm);
-                        mask_chunk(s3, kc + 96, rm);
-                    }
-                    chunk_max<0>(s2, mr, sl, kc, rm);
-                    chunk_max<0>(s3, mr, sl, kc, rm);
-                    const float m_new = fmaxf(m, fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sl);
-                    if (j == lo) {
-                        m = m_new;
-                        break;
-                    }
-                    const bool need = m_new > m + 8.0f;
-                    if (!__any_sync(0xffffffffu, need)) break;
-                    // Rare: some row's maximum grows by more than 2^8.  O += P V of the previous block
-                    // has landed (these scores were issued behind it): rescale those rows of O in
-                    // tensor memory, then take the scores again (their registers were the scratch).
+                float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+                tmem_ld32(tS, s0);
+                tmem_ld32(tS + 32, s1);
+                tmem_wait_ld();
+                tmem_ld32(tS + 64, s2);  // lands while the maximum of the first half is taken
+                tmem_ld32(tS + 96, s3);
+                if (!full) {  // window edge, diagonal, ragged end (two blocks in nine with a 1024-key window)
+                    mask_chunk(s0, kc, rm);
+                    mask_chunk(s1, kc + 32, rm);
+                }
+                chunk_max<0>(s0, mr, sl, kc, rm);
+                chunk_max<0>(s1, mr, sl, kc, rm);
+                tmem_wait_ld();
+                tc_fence_before_sync();
+                mbar_arrive_warp(s_free);  // the buffer may take the other pipeline's scores
+                if (!full) {
+                    mask_chunk(s2, kc + 64, rm);
+                    mask_chunk(s3, kc + 96, rm);
+                }
+                chunk_max<0>(s2, mr, sl, kc, rm);
+                chunk_max<0>(s3, mr, sl, kc, rm);
+                const float m_new = fmaxf(m, fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sl);
+                // O += P V of the block before has long completed, as a rule: its P may be replaced.
+                if (g > 0 && !mbar_wait_warp<3>(&pv_done[s], (g - 1) & 1)) {
+                    report_fault(p.fault, FAULT_WAIT_O, 0x200u + g);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                const bool need = m_new > m + 8.0f;
+                if (j == lo) {
+                    m = m_new;
+                } else if (__any_sync(0xffffffffu, need)) {
+                    // Rare: some row's maximum grows by more than 2^8: rescale those rows of O in tensor memory.
                     const float alpha = need ? fast_exp2(m - m_new) : 1.0f;
 #pragma unroll 1
-                    for (int c = 0; c < HD; c += 32) {
-                        tmem_ld32(tO + c, s0);
+                    for (int c = 0; c < HD; c += 16) {
+                        uint32_t ww[16];
+                        tmem_ld16(tO + c, ww);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) s0[e] = __float_as_uint(__uint_as_float(s0[e]) * alpha);
-                        tmem_st32(tO + c, s0);
+                        for (int e = 0; e < 16; ++e) ww[e] = __float_as_uint(__uint_as_float(ww[e]) * alpha);
+                        tmem_st16(tO + c, ww);
                     }
                     tmem_wait_st();
                     l *= alpha;
                     if (need) m = m_new;
                 }
-                // Probabilities as bf16, packed over the first 64 of the block's score columns; row sum in fp32.
+                // Probabilities as bf16, packed in the pipeline's 64 columns for P; row sum in fp32.
                 // The first 96 keys are announced half a chunk late: by then their stores have landed and the wait
                 // for them costs nothing, and their share of O += P V still runs beside the rest.
                 const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
@@ -816,17 +810,17 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 uint64_t ls2[2] = {0ull, 0ull};
                 uint32_t pk[16];
                 exp_chunk(s0, pk, ls2, sl2, nm2);
-                tmem_st16(tS, pk);
+                tmem_st16(tP, pk);
                 exp_chunk(s1, pk, ls2, sl2, nm2);
-                tmem_st16(tS + 16, pk);
+                tmem_st16(tP + 16, pk);
                 exp_chunk(s2, pk, ls2, sl2, nm2);
-                tmem_st16(tS + 32, pk);
+                tmem_st16(tP + 32, pk);
                 exp_chunk<0, 16>(s3, pk, ls2, sl2, nm2);
                 tmem_wait_st();
                 tc_fence_before_sync();
                 mbar_arrive_warp(&p_part[2 * s]);
                 exp_chunk<16, 32>(s3, pk, ls2, sl2, nm2);
-                tmem_st16(tS + 48, pk);
+                tmem_st16(tP + 48, pk);
                 float l0, l1, l2, l3;
                 unpack_f32x2(ls2[0], l0, l1);
                 unpack_f32x2(ls2[1], l2, l3);
