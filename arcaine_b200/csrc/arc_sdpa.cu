@@ -21,6 +21,7 @@
 #include "qkv_prepare_sm100.cuh"
 #include "prefill_sm100.cuh"
 #include "prefill_wide_sm100.cuh"
+#include "prefill_chains_sm100.cuh"
 
 namespace arc {
 
@@ -100,6 +101,20 @@ static int clusters_at_once(K kernel, int size, int sm_count, int threads, int s
     return n;
 }
 
+// The instances of the kernels of head dim 128 for a call; the common ones carry nothing they do not need.
+using PairKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, PrefillParams);
+static PairKernel pair_kernel(bool gate, bool copies, bool vision) {
+    if (vision) return gate ? sdpa_prefill_pair_kernel<true, true, true> : copies ? sdpa_prefill_pair_kernel<false, true, true> : sdpa_prefill_pair_kernel<false, false, true>;
+    if (copies) return gate ? sdpa_prefill_pair_kernel<true, true> : sdpa_prefill_pair_kernel<false, true>;
+    return gate ? sdpa_prefill_pair_kernel<true, false> : sdpa_prefill_pair_kernel<false, false>;
+}
+using ChainsKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, PrefillParams);
+static ChainsKernel chains_kernel(bool gate, bool vision, bool masked) {
+    if (masked) return gate ? sdpa_prefill_chains_kernel<true, false, true> : sdpa_prefill_chains_kernel<false, false, true>;
+    if (vision) return gate ? sdpa_prefill_chains_kernel<true, true, false> : sdpa_prefill_chains_kernel<false, true, false>;
+    return gate ? sdpa_prefill_chains_kernel<true, false, false> : sdpa_prefill_chains_kernel<false, false, false>;
+}
+
 // One-time set-up for the current device: status-word address, SM count, and the
 // dynamic shared memory opt-in of every kernel.
 static int device_state(DeviceState** out) {
@@ -125,14 +140,10 @@ static int device_state(DeviceState** out) {
                 }
                 g_encode = reinterpret_cast<EncodeTiledFn>(fn);
             }
-            ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<false, false>, PairCfg::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<true, false>, PairCfg::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<false, true>, PairCfg::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<true, true>, PairCfg::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_pair_kernel<false, false, true>, PairCfg::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, false, false>, PrefillCfg<128>::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, false, true>, PrefillCfg<128>::SMEM_BYTES));
-            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<128, true, true>, PrefillCfg<128>::SMEM_BYTES));
+            for (int i = 0; i < 8; ++i) {
+                ARC_CUDA(opt_in_smem(pair_kernel(i & 1, i & 2, i & 4), PairCfg::SMEM_BYTES));
+                ARC_CUDA(opt_in_smem(chains_kernel(i & 1, i & 2, i & 4), ChainsCfg::SMEM_BYTES));
+            }
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<256, true, true>, PrefillCfg<256>::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, false>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true, false>, WideCfg::SMEM_BYTES));
@@ -250,6 +261,15 @@ struct PrefillPlan {
     size_t mask_bytes = 0;   // behind it, if it is there: the classes and bits of an additive mask
 };
 
+// Key blocks that token tile qt (128 rows) of a call sees, block ids apart.
+static int tile_key_blocks(const arc_sdpa_prefill_params* p, int qt) {
+    const int blocks = (p->kv_len + 127) / 128, off = p->kv_len - p->seq;
+    if (p->mask_type != ARC_MASK_CAUSAL) return blocks;
+    const int last = std::min(p->kv_len - 1, std::min(qt * 128 + 127, p->seq - 1) + off);
+    const int hi = last >= 0 ? last / 128 + 1 : 0, lo = p->window > 0 && p->window != 0x7fffffff ? std::max(0, qt * 128 + off - p->window + 1) / 128 : 0;
+    return std::max(0, hi - lo);
+}
+
 // Head dim 256: units of the CTA pairs' list, and how many parts the key range of each is worth when the units alone
 // would leave pairs idle.  Measured (us): a key block of a pair 1.13; records and fold 3 + 0.04 per pair in a cluster, 2.5 +
 // 0.06 per pair with a merge launch (every pair writes its 256 rows as f32, 32 bytes per clk and SM), whatever the number
@@ -295,16 +315,17 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const Wi
     const bool scanned_mask = p->mask_type == ARC_MASK_EXPLICIT && p->hd == 256 && p->num_splits <= 1;
     if (splits == 0 && p->hd == 256) splits = choose_wide_splits(p, plan->q_tiles, room);
     if (splits == 0) {
-        // Head dim 128: split the key range only when the tiles alone leave most SMs idle and there are enough key
-        // blocks to pay for folding the parts again.  A block takes 1.3 us, records and merge 3 to 5 in all (one tile row of
-        // 8 heads: 1024 keys 15.5 us whole, 11.2 in eight parts; 1280 keys 17.9 and 12.4; 512 keys 10.1 and 10.5).  The line
-        // at ten blocks was drawn when the merge took 8 us; five to nine blocks of few tiles would gain too.
+        // Head dim 128: split the key range when the tiles alone leave most SMs idle and there are enough key blocks to pay
+        // for folding the parts again, into as many parts as take least: a key block is 0.71 us, records and merge 0.028 a part.
+        // (8 tiles of 12 / 16 / 32 blocks: 12.4 / 16.1 / 28.9 us whole, 10.6 / 11.3 / 14.5 in four parts, 10.5 / 10.7 / 12.3 in
+        // eight; 32 tiles of 16: 16.8 whole, 16.2 in two, 13.5 in four.)
         splits = 1;
         if (tiles * 2 <= sm_count && kv_blocks >= 10) {
-            splits = (int)(sm_count / tiles);
-            if (splits > kv_blocks / 2) splits = kv_blocks / 2;
-            if (splits > 8) splits = 8;
-            if (splits < 1) splits = 1;
+            double least = 1e30;
+            for (int s = 2; s <= 8 && 2 * s <= kv_blocks && tiles * s <= sm_count; ++s) {
+                const double t = 0.71 * ((kv_blocks + s - 1) / s) + 0.028 * (double)(tiles * s);
+                if (t < least) least = t, splits = s;
+            }
         }
     }
     if (splits > kv_blocks) splits = kv_blocks;
@@ -316,6 +337,7 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const Wi
     if (scanned_mask) plan->mask_bytes = (size_t)plan->q_tiles * kv_blocks * (128 * sizeof(uint4) + sizeof(uint32_t));
     if (p->block_ids) {
         if (p->mask_type != ARC_MASK_CAUSAL || p->block_ids_offset < 0) return ARC_ERR_BAD_SHAPE;
+        // (span ends were kept there once; the call still asks for the room it always did)
         if (p->hd == 128) plan->ws_bytes += ((size_t)p->seq * sizeof(int32_t) + 15) & ~(size_t)15;
     }
     return ARC_OK;
@@ -347,6 +369,36 @@ static int launch_fold(const arc_sdpa_prefill_params* p, const PrefillPlan& plan
     return ARC_OK;
 }
 
+// What the SM with most to do takes for its share of `units` units (`heads` per token tile and sequence, of `tiles` token
+// tiles each), a unit taking per_block for each of its key blocks and per_unit.  Dealt in plain order units count as all as long
+// as the longest; longest first and every second wave in reverse (TileCursor), the load is linear in the SM's index between
+// the ends of the waves, so these are what is looked at.
+static double longest_share(const arc_sdpa_prefill_params* p, long long units, int heads, int tiles, long long sms, bool by_length, double per_block, double per_unit) {
+    const int q_tiles = (p->seq + 127) / 128;
+    const long long waves = (units + sms - 1) / sms, rest = units - (waves - 1) * sms;
+    if (!by_length || waves > 16) return (double)waves * (per_block * tile_key_blocks(p, q_tiles - 1) + per_unit);
+    const long long per = (long long)heads * p->batch, edge = (waves & 1) ? rest : sms - rest;
+    double most = 0.0;
+    for (long long x : {0ll, sms - 1, edge - 1, edge}) {
+        if (x < 0 || x >= sms) continue;
+        double sum = 0.0;
+        for (long long i = 0; i < waves; ++i) {
+            const long long u = i * sms + ((i & 1) ? sms - 1 - x : x);
+            if (u < units) sum += per_block * tile_key_blocks(p, std::min(q_tiles - 1, (int)((q_tiles + tiles - 1) / tiles - 1 - u / per) * tiles + tiles - 1)) + per_unit;
+        }
+        most = std::max(most, sum);
+    }
+    return most;
+}
+
+// Digits of a grid of `ctas` in the tile list, fastest first (TileCursor).
+static void set_step(PrefillParams* kp, long long ctas) {
+    const long long rf = kp->long_first ? kp->cur_heads : kp->q_tiles, rm = kp->long_first ? kp->batch : kp->cur_heads;
+    kp->step[0] = (int)(ctas % rf);
+    kp->step[1] = (int)(ctas / rf % rm);
+    kp->step[2] = (int)(ctas / rf / rm);
+}
+
 template <int HD>
 static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& plan, DeviceState* ds,
                           cudaStream_t stream) {
@@ -365,19 +417,8 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     kp.out_lse = p->out_lse;
     kp.part_o = plan.splits > 1 ? static_cast<float*>(p->workspace) : nullptr;
     kp.part_lse = kp.part_o ? kp.part_o + (size_t)plan.splits * plan.rows * HD : nullptr;
-    // CTA pairs (prefill_wide_sm100.cuh) and the two-tile kernel look vision blocks up themselves; the one-tile kernel wants
-    // the span end of every row (a few microseconds instead of a (seq, kv_len) f32 mask).
     const bool wide = HD == 256 && (plan.splits == 1 || p->mask_type != ARC_MASK_EXPLICIT || plan.mask_bytes > 0);
     if (p->block_ids) kp.ids = p->block_ids + p->block_ids_offset;
-    auto find_spans = [&]() -> int {
-        if (!kp.ids) return ARC_OK;
-        int* vis = reinterpret_cast<int*>(static_cast<unsigned char*>(p->workspace) + plan.split_bytes);
-        ARC_CUDA(launch_dependent(vision_span_kernel, dim3((unsigned)((p->seq + 255) / 256)), dim3(256), 0, stream, 1, p->block_ids,
-                                  p->block_ids_offset, p->kv_len - p->seq, p->seq, p->kv_len, vis));
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        kp.vis_hi = vis;
-        return ARC_OK;
-    };
     kp.fault = ds->fault;
     kp.batch = p->batch;
     kp.seq = p->seq;
@@ -396,74 +437,87 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     for (int sh = 0; sh < 31; ++sh)
         if ((1 << sh) == kp.group) kp.group_shift = sh;
 
-    // Head dim 128: two query tiles per CTA (prefill_pair_sm100.cuh) when that is the faster way to cover
-    // the tiles.  ARC_SDPA_PREFILL_KERNEL=single|pair overrides the choice (for A/B measurements).
-    if (HD == 128 && plan.splits == 1 && !(kp.mask_type == 1 && kp.mask != nullptr) && !(kp.ids && (kp.gate || kp.n_copies > 0))) {
+    const bool masked = kp.mask_type == ARC_MASK_EXPLICIT && kp.mask != nullptr;
+    // Head dim 128: two query tiles per CTA (prefill_pair_sm100.cuh), or one in two chains of key blocks
+    // (prefill_chains_sm100.cuh), whichever covers the tiles faster; the latter for additive masks and parts of a key range.
+    // ARC_SDPA_PREFILL_KERNEL=single|pair overrides the choice (for A/B measurements).
+    if constexpr (HD == 128) {
         static const int forced = [] {
             const char* e = std::getenv("ARC_SDPA_PREFILL_KERNEL");
             if (!e) return 0;
             return std::strcmp(e, "pair") == 0 ? 2 : (std::strcmp(e, "single") == 0 ? 1 : 0);
         }();
+        const bool split = plan.splits > 1;
         // A CTA takes two 128-row tiles: the same tokens of two heads of one KV group when the group
         // size is even (both tiles then see exactly the same key blocks), else 256 tokens of one head.
         const bool head_pair = ((p->nq / p->nkv) & 1) == 0;
         const long long pair_tiles = head_pair ? (long long)plan.q_tiles * (p->nq / 2) * p->batch
                                                : (long long)((p->seq + 255) / 256) * p->nq * p->batch;
-        // Tiles come in waves of one per SM, and the kernel with the cheaper whole number of waves wins, a pair taken for 1.7
-        // single tiles.  That was measured with earlier kernels; with these a wave of pairs costs 1.13 to 1.18 waves of
-        // single tiles (64 pairs 18.9 us, 128 tiles 16.7 over 1024 keys; 57.3 and 49.0 over 4096).  The line is the same for
-        // one wave of single tiles against one of pairs, and for two or more against half as many; it is drawn too high
-        // where three waves stand against two (odd groups).
-        const long long single_tiles = (long long)plan.q_tiles * p->nq * p->batch;
+        const long long single_tiles = (long long)plan.q_tiles * p->nq * p->batch * plan.splits;
         const long long sms = ds->sm_count;
         // The pairs left over after the last whole wave of CTAs are cut into their two heads when every SM then
-        // gets at most one of them: a second launch (the one-tile kernel, one CTA per tile, scheduled behind this
-        // one as SMs free up) takes them, and no SM runs a whole pair while the others idle.  A single tile
-        // costs about one tile of the one-tile kernel.
+        // gets at most one of them: a second launch (a tile per CTA, scheduled behind this
+        // one as SMs free up) takes them, and no SM runs a whole pair while the others idle.
         const long long full_waves = pair_tiles / sms, left = pair_tiles - full_waves * sms;
-        const bool cut_tail = !kp.ids && head_pair && full_waves > 0 && left > 0 && 2 * left <= sms;
-        const double cost_pair = cut_tail ? 1.7 * (double)full_waves + 1.05 : 1.7 * (double)((pair_tiles + sms - 1) / sms);
-        const double cost_single = (double)((single_tiles + sms - 1) / sms);
-        // (Vision blocks: the one-tile kernel also needs a launch for the span ends and twice as many waves: 1257 tokens of
-        // 16 heads 43.7 us, two tiles at a time 24.6.)
-        const bool use_pair = forced == 2 || (forced == 0 && (kp.ids || cost_pair <= cost_single));
-        if (use_pair) {
-            if (pair_tiles > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
-            kp.head_pair = head_pair ? 1 : 0;
-            kp.cur_heads = head_pair ? p->nq / 2 : p->nq;
-            kp.q_tiles = head_pair ? plan.q_tiles : (p->seq + 255) / 256;
-            const long long pair_units = cut_tail ? full_waves * sms : pair_tiles;
-            kp.total_tiles = (int)pair_units;
-            const unsigned ctas = (unsigned)(pair_units < ds->sm_count ? pair_units : ds->sm_count);
-            if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
-            auto kernel = kp.ids          ? sdpa_prefill_pair_kernel<false, false, true>
-                          : kp.n_copies > 0 ? (kp.gate ? sdpa_prefill_pair_kernel<true, true> : sdpa_prefill_pair_kernel<false, true>)
-                                          : (kp.gate ? sdpa_prefill_pair_kernel<true, false> : sdpa_prefill_pair_kernel<false, false>);
-            ARC_CUDA(launch_dependent(kernel, dim3(ctas), dim3(PairCfg::THREADS), (size_t)PairCfg::SMEM_BYTES, stream, 1, tq, tk, tv, to, tg, kp));
-            g_launches.fetch_add(1, std::memory_order_relaxed);
-            if (cut_tail) {
-                PrefillParams tp = kp;
-                tp.head_pair = 0;
-                tp.cur_heads = p->nq;
-                tp.q_tiles = plan.q_tiles;
-                tp.tail_base = (int)pair_units;
-                tp.total_tiles = (int)(2 * left);
-                tp.num_splits = 1;
-                const dim3 grid((unsigned)(2 * left)), block(PrefillCfg<128>::THREADS);
-                if (tp.gate)
-                    ARC_CUDA(launch_dependent(sdpa_prefill_kernel<128, false, true>, grid, block, (size_t)PrefillCfg<128>::SMEM_BYTES, stream, 1, tq, tk, tv, tp));
-                else
-                    ARC_CUDA(launch_dependent(sdpa_prefill_kernel<128, false, false>, grid, block, (size_t)PrefillCfg<128>::SMEM_BYTES, stream, 1, tq, tk, tv, tp));
-                g_launches.fetch_add(1, std::memory_order_relaxed);
+        // Under a causal mask tiles differ in length and go longest first, as at head dim 256 below.
+        const bool windowed = p->window > 0 && p->window < p->kv_len;
+        const auto by_length = [&](long long units) {
+            return !split && p->mask_type == ARC_MASK_CAUSAL && units > sms && (!windowed || units < 8 * sms) &&
+                   (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;
+        };
+        // In steps of a key block of a pair (1.37 us): launches, loads and output apart, a pair's unit takes its blocks and
+        // half a step, a tile in chains 0.52 a block and 0.8.  A second launch for the tail adds 3.6 (it starts when the first
+        // one's CTAs end).  (16 heads, 1152 queries, 512 / 2048 keys: 8.7 / 17.2 us in chains, 11.4 / 27.9 in pairs; 2304
+        // queries 14 / 32, 13 / 31; 2000 causal queries of 28 heads: 29 in pairs, 31 in chains.)
+        bool use_pair = false, cut_tail = false;
+        if (!split && !masked && forced != 1 && (forced == 2 || single_tiles > sms)) {
+            const int heads = head_pair ? p->nq / 2 : p->nq, tiles = head_pair ? 1 : 2;
+            const bool sorted = by_length(pair_tiles);
+            double cost_pair = longest_share(p, pair_tiles, heads, tiles, sms, sorted, 1.0, 0.5);
+            if (head_pair && full_waves > 0 && left > 0 && 2 * left <= sms) {
+                const int first = sorted ? plan.q_tiles - 1 - (int)(full_waves * sms / ((long long)heads * p->batch)) : plan.q_tiles - 1;  // the tail's longest
+                const double cost_cut = longest_share(p, full_waves * sms, heads, 1, sms, sorted, 1.0, 0.5) + 3.6 + 0.52 * tile_key_blocks(p, first);
+                cut_tail = cost_cut < cost_pair;
+                cost_pair = std::min(cost_pair, cost_cut);
             }
-            return ARC_OK;
+            use_pair = forced == 2 || cost_pair <= longest_share(p, single_tiles, p->nq, 1, sms, by_length(single_tiles), 0.52, 0.8);
         }
+        if ((use_pair ? pair_tiles : single_tiles) > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
+        kp.long_first = by_length(use_pair ? pair_tiles : single_tiles);
+        PrefillParams cp = kp;  // tiles one by one
+        cp.head_pair = 0;
+        cp.cur_heads = p->nq;
+        cp.q_tiles = plan.q_tiles;
+        cp.total_tiles = (int)single_tiles;
+        auto launch_chains = [&](long long ctas) -> int {
+            set_step(&cp, ctas);
+            ARC_CUDA(launch_dependent(chains_kernel(cp.gate && !split, cp.ids != nullptr, masked), dim3((unsigned)ctas), dim3(ChainsCfg::THREADS),
+                                      (size_t)ChainsCfg::SMEM_BYTES, stream, 1, tq, tk, tv, cp));
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+            return ARC_OK;
+        };
+        if (!use_pair) {
+            if ((rc = launch_chains(std::min(single_tiles, sms))) != ARC_OK) return rc;
+            return split ? launch_fold<HD>(p, plan, kp, stream) : ARC_OK;
+        }
+        kp.head_pair = head_pair ? 1 : 0;
+        kp.cur_heads = head_pair ? p->nq / 2 : p->nq;
+        kp.q_tiles = head_pair ? plan.q_tiles : (p->seq + 255) / 256;
+        const long long pair_units = cut_tail ? full_waves * sms : pair_tiles;
+        kp.total_tiles = (int)pair_units;
+        set_step(&kp, std::min(pair_units, sms));
+        if ((rc = make_out_maps(&to, &tg, p)) != ARC_OK) return rc;
+        ARC_CUDA(launch_dependent(pair_kernel(kp.gate != nullptr, kp.n_copies > 0, kp.ids != nullptr), dim3((unsigned)std::min(pair_units, sms)), dim3(PairCfg::THREADS),
+                                  (size_t)PairCfg::SMEM_BYTES, stream, 1, tq, tk, tv, to, tg, kp));
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        if (!cut_tail) return ARC_OK;
+        cp.tail_base = (int)pair_units;
+        cp.total_tiles = (int)(2 * left);
+        return launch_chains(2 * left);
     }
 
-    if (!wide && (rc = find_spans()) != ARC_OK) return rc;
     // Head dim 256, whole tiles, no additive mask: pairs of CTAs (prefill_wide_sm100.cuh) take 2300-2500 clk per key block
     // and pair of tiles where a CTA on its own takes 3700 per tile.
-    const bool masked = kp.mask_type == 1 && kp.mask != nullptr;
     // (a caller who brings no workspace for the scanned mask gets the one-tile kernel, which reads the mask itself)
     if (wide &&
         (!masked || (plan.mask_bytes > 0 && plan.q_tiles < 16384 && p->workspace && aligned16(p->workspace) && p->workspace_bytes >= plan.ws_bytes + plan.mask_bytes))) {
@@ -517,12 +571,8 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     if (total_tiles > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
     kp.total_tiles = (int)total_tiles;
     const unsigned ctas = (unsigned)(total_tiles < ds->sm_count ? total_tiles : ds->sm_count);
-    // The additive-mask form is a kernel of its own: the common one stays small.
-    void (*kernel)(CUtensorMap, CUtensorMap, CUtensorMap, PrefillParams) = sdpa_prefill_kernel<HD, true, true>;
-    if constexpr (HD == 128) {
-        if (!masked) kernel = kp.gate && plan.splits == 1 ? sdpa_prefill_kernel<HD, false, true> : sdpa_prefill_kernel<HD, false, false>;
-    }
-    ARC_CUDA(launch_dependent(kernel, dim3(ctas), dim3(PrefillCfg<HD>::THREADS), (size_t)PrefillCfg<HD>::SMEM_BYTES, stream, 1, tq, tk, tv, kp));
+    set_step(&kp, ctas);
+    ARC_CUDA(launch_dependent(sdpa_prefill_kernel<256, true, true>, dim3(ctas), dim3(PrefillCfg<256>::THREADS), (size_t)PrefillCfg<256>::SMEM_BYTES, stream, 1, tq, tk, tv, kp));
     g_launches.fetch_add(1, std::memory_order_relaxed);
 
     return plan.splits > 1 ? launch_fold<HD>(p, plan, kp, stream) : ARC_OK;

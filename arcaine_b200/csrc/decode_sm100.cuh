@@ -1029,32 +1029,4 @@ __global__ void fill_causal_mask_kernel(float* mask, const int* block_ids, int q
     }
 }
 
-// First key each query row can no longer see under the causal rule extended by Gemma4's vision
-// blocks (src/common/kernels/attention_mask.hpp:44-73): a query inside a block (same non-negative id,
-// contiguous) sees the block's later keys as well.  ids[base + j] is key j's id; row t sits at key
-// position t + off.  One thread per row; a warp looks for the ends of its rows' blocks together, 32 keys a step (a
-// thread walking to the end of its own block took 10 us for blocks of 256).
-__global__ void vision_span_kernel(const int* ids, int base, int off, int seq, int kv_len, int* vis_hi) {
-    grid_dependency_wait();
-    grid_launch_dependents();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-    const int self = t + off;  // key index of the query's own position
-    const int id = t < seq && self >= 0 && self < kv_len ? ids[base + self] : -1;
-    int hi = min(max(self + 1, 0), kv_len);
-    bool open = id >= 0;  // the end of this row's block has not been found
-    for (int k0 = t - lane + off; __any_sync(0xffffffffu, open); k0 += 32) {
-        const int key = k0 + lane;
-        const int other = key >= 0 && key < kv_len ? ids[base + key] : -2;  // (past the last key: another id)
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-            const int o = __shfl_sync(0xffffffffu, other, e);
-            if (open && k0 + e > self && o != id) {
-                hi = k0 + e;
-                open = false;
-            }
-        }
-    }
-    if (t < seq) vis_hi[t] = hi;
-}
-
 }  // namespace arc

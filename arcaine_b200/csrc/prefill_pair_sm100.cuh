@@ -56,7 +56,7 @@ struct PairCfg {
     // s_full p_part[2] pv_done o_full o_empty fin[2]; then gate[4][2], two per epilogue warp
     static constexpr int NUM_BARS = 4 + 2 + 2 * K_STAGES + 1 + 24;
     static constexpr int FIN_FLOATS = 2 * 2 * 128;  // [tile parity][pipeline][row] row sum
-    static constexpr int SMEM_BYTES = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 4 * 8192 + NUM_BARS * 8 + 16 + FIN_FLOATS * 4 + 32;  // (4 x 8 KB: output stage; 32: first unit)
+    static constexpr int SMEM_BYTES = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 4 * 8192 + NUM_BARS * 8 + 16 + FIN_FLOATS * 4 + 80;  // (4 x 8 KB: output stage; 80: first unit)
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
     static constexpr int SOFTMAX_WARPS = 8;   // four per pipeline
     static constexpr int EPILOGUE_WARP = 8;   // four warps
@@ -395,6 +395,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
     }
+    static_assert(sizeof(TileCursor) <= 80, "the first unit's place in shared memory");
     // (the divisions, once and ahead of the wait: they took 1000 clk between the kernel's release and its first load)
     if (threadIdx.x == 0) {
         TileCursor cur;

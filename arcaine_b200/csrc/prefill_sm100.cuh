@@ -1,6 +1,6 @@
-// GQA flash-attention prefill kernel for sm_100a, one query tile at a time per CTA: the kernel for small problems, split
-// key ranges, additive masks and vision blocks of head dim 128 (with enough tiles prefill_pair_sm100.cuh runs two per
-// CTA), and at head dim 256 for additive masks without a workspace (prefill_wide_sm100.cuh does the rest).
+// GQA flash-attention prefill kernel for sm_100a, one query tile at a time per CTA: head dim 256 with an additive mask and
+// no workspace for what mask_scan_kernel would read out of it (prefill_wide_sm100.cuh does the rest of head dim 256,
+// prefill_pair_sm100.cuh and prefill_chains_sm100.cuh head dim 128); and what all prefill kernels share.
 //
 // One CTA owns a tile of 128 query tokens of one query head and walks the key
 // blocks (128 keys) that tile can see.  Q, K and V tiles are staged in shared
@@ -40,7 +40,6 @@ struct PrefillParams {
     float* out_lse;
     float* part_o;
     float* part_lse;
-    const int* vis_hi;  // optional [seq]: first key row t can no longer see (causal rule extended by vision blocks)
     uint32_t* fault;
     int batch, seq, kv_len, nq, nkv;
     long long o_stride_b, o_stride_t;
@@ -53,28 +52,24 @@ struct PrefillParams {
     int head_pair;    // prefill_pair_sm100.cuh: 1 = the CTA's two tiles are the same tokens of two heads of one KV group
     int group;        // nq / nkv
     int group_shift;  // log2(group) if it is a power of two, else -1
-    // >= 0 (one-tile kernel): the launch covers the tail of a two-tile launch's unit list — tile w is head (w & 1)
+    // >= 0 (prefill_chains_sm100.cuh): the launch covers the tail of a two-tile launch's unit list — tile w is head (w & 1)
     // of the head pair with unit index tail_base + (w >> 1), one tile per CTA; -1: the plain tile list
     int tail_base;
-    int long_first;  // prefill_wide_sm100.cuh: units in order of falling length
+    int long_first;  // units in order of falling length
+    int step[3];     // digits of the grid's size in the tile list (TileCursor)
     // The additive mask as mask_scan_kernel has read it (prefill_wide_sm100.cuh; mask_blocks key blocks per row tile)
     const uint32_t* mask_class;  // [row tile][key block]: a byte per 32 rows, MASK_* bits
     const uint4* mask_bits;      // [row tile][key block][row]: one bit per key, set where the mask is 0
     int mask_blocks;
     int fold;        // prefill_wide_sm100.cuh: the parts of a unit are the pairs of one cluster, which folds them itself
-    const int* ids;  // vision-block ids, ids[j] that of key j (prefill_wide_sm100.cuh and prefill_pair_sm100.cuh, instead of vis_hi)
+    const int* ids;  // vision-block ids, ids[j] that of key j 
 };
 
 // One CTA per SM, persistent: it takes tiles (128 query tokens of one query head) round-robin
 // and keeps its pipelines running across tile boundaries — the next tile's Q, K and V stream in
 // and its first score blocks are computed while the softmax warps still write the previous
-// tile's output.  The score accumulator is
-// multi-buffered in tensor memory (S0, S1[, S2], then O), so S = Q K^T runs one or two key
-// blocks ahead of the softmax; eight softmax warps (two threads per query row, 64 keys
-// each).  With three score buffers (head dim 128) they look at the next block's maximum
-// before they exponentiate the current one, which hides the exchange of row maxima; with
-// two (head dim 256) every block is taken on its own, because the next block's scores
-// cannot be computed before this block's probabilities have been consumed.
+// tile's output.  Two score buffers in tensor memory, then O, so S = Q K^T runs one key block ahead of
+// the softmax; eight softmax warps (two threads per query row, 64 keys each).
 // Eight rather than sixteen softmax warps on purpose: the
 // single MMA-issuing thread shares an instruction scheduler with them, and with four busy
 // warps per scheduler it could not issue MMAs fast enough to keep the tensor pipe fed.
@@ -85,10 +80,10 @@ struct PrefillCfg {
     static constexpr int CH = HD / 64;
     static constexpr int CHUNK_BYTES = 128 * 128;  // 128 rows x 64 bf16
     static constexpr int TILE_BYTES = CH * CHUNK_BYTES;
-    static constexpr int K_STAGES = (HD == 128) ? 3 : 1;
-    static constexpr int V_STAGES = (HD == 128) ? 2 : 1;
+    static constexpr int K_STAGES = 1;
+    static constexpr int V_STAGES = 1;
     static constexpr int TMEM_COLS = 512;
-    static constexpr int NSB = (HD == 128) ? 3 : 2;  // score buffers: S = Q K^T runs NSB-1 blocks ahead of the softmax
+    static constexpr int NSB = 2;  // score buffers: S = Q K^T runs NSB-1 blocks ahead of the softmax
     static constexpr int COL_S = 0;                  // NSB buffers of 128 fp32 columns; P (bf16) is written over them
     static constexpr int COL_O = NSB * 128;          // HD fp32 columns
     static constexpr int NUM_BARS = 2 + 2 * K_STAGES + 2 * V_STAGES + 2 * NSB + 2 + 2;
@@ -257,43 +252,65 @@ struct TileWork {
     int my_lo, n_my;  // key blocks [my_lo, my_lo + n_my) of this tile and split
 };
 
-// Position of a persistent CTA in the launch's tile list: tile w = ((z * cur_heads) + h) * q_tiles + qt,
-// token tiles fastest (neighbouring CTAs share K/V blocks in L2), then query heads, then
-// z = batch * num_splits + split.  The cursor moves by gridDim.x tiles per step with carries
-// instead of dividing again.
+// Position of a persistent CTA in the launch's tile list.  Plain order: tile w = ((z * cur_heads) + h) * q_tiles + qt,
+// token tiles fastest (neighbouring CTAs share K/V blocks in L2), then query heads, then z = batch * num_splits + split.
+// long_first: the tiles with most key blocks first, all heads of a token tile together, and every second wave of CTAs in
+// reverse, so that the sums of a CTA's tiles are about equal.  A place in the list is added up from the digits of the
+// wave's first place, which move by those of the grid's size (from the host), and of the CTA's place in a wave: divisions
+// are few, and ahead of the kernel's wait — where all of a call's CTAs fill the device they are on its clock all the same
+// (ten of them were 2.8 us).
 struct TileCursor {
     int w, qt, h, z;
-    int dqt, dh, dz, step;
+    int base_w, base[3];      // first place of the wave: index and digits (fastest first)
+    int own_w[2], own[2][3];  // the CTA's place in even / odd waves
+    int odd;
+    __device__ __forceinline__ void place(const PrefillParams& p) {
+        const int rf = p.long_first ? p.cur_heads : p.q_tiles, rm = p.long_first ? p.batch : p.cur_heads;
+        w = base_w + (odd ? own_w[1] : own_w[0]);
+        int fast = base[0] + (odd ? own[1][0] : own[0][0]), carry = fast >= rf ? 1 : 0;
+        fast -= carry * rf;
+        int mid = base[1] + (odd ? own[1][1] : own[0][1]) + carry;
+        carry = mid >= rm ? 1 : 0;
+        mid -= carry * rm;
+        const int slow = base[2] + (odd ? own[1][2] : own[0][2]) + carry;
+        qt = p.long_first ? p.q_tiles - 1 - slow : fast;
+        h = p.long_first ? fast : mid;
+        z = p.long_first ? mid : slow;
+    }
     __device__ __forceinline__ void init(const PrefillParams& p) {
-        w = blockIdx.x;
-        step = gridDim.x;
-        if (p.tail_base >= 0) {  // (the grid holds one CTA per tile: the strides below are never used)
-            const int idx = p.tail_base + (w >> 1);
-            qt = idx % p.q_tiles;
-            const int prest = idx / p.q_tiles, pairs = p.cur_heads >> 1;
-            h = (prest % pairs) * 2 + (w & 1);
-            z = prest / pairs;
-            dqt = dh = dz = 0;
-            return;
+        const bool tail = p.tail_base >= 0;  // (the grid holds one CTA per tile, and never steps)
+        const int heads = tail ? p.cur_heads >> 1 : p.cur_heads;
+        const int rf = p.long_first ? heads : p.q_tiles, rm = p.long_first ? p.batch : heads;
+        auto digits = [&](int idx, int (&d)[3]) {
+            const int rest = idx / rf;
+            d[0] = idx - rest * rf;
+            d[2] = rest / rm;
+            d[1] = rest - d[2] * rm;
+        };
+        base_w = base[0] = base[1] = base[2] = odd = 0;
+        const int first = blockIdx.x;
+        own_w[0] = own_w[1] = first;
+        digits(tail ? p.tail_base + (first >> 1) : first, own[0]);
+        own[1][0] = own[0][0], own[1][1] = own[0][1], own[1][2] = own[0][2];
+        if (p.long_first && !tail) {
+            own_w[1] = (int)gridDim.x - 1 - first;
+            digits(own_w[1], own[1]);
         }
-        qt = w % p.q_tiles;
-        const int rest = w / p.q_tiles;
-        h = rest % p.cur_heads;
-        z = rest / p.cur_heads;
-        dqt = step % p.q_tiles;
-        const int srest = step / p.q_tiles;
-        dh = srest % p.cur_heads;
-        dz = srest / p.cur_heads;
+        place(p);
+        if (tail) h = h * 2 + (first & 1);
     }
     __device__ __forceinline__ void advance(const PrefillParams& p) {
-        w += step;
-        qt += dqt;
-        int carry = qt >= p.q_tiles ? 1 : 0;
-        qt -= carry * p.q_tiles;
-        h += dh + carry;
-        carry = h >= p.cur_heads ? 1 : 0;
-        h -= carry * p.cur_heads;
-        z += dz + carry;
+        const int rf = p.long_first ? p.cur_heads : p.q_tiles, rm = p.long_first ? p.batch : p.cur_heads;
+        base_w += gridDim.x;
+        base[0] += p.step[0];
+        int carry = base[0] >= rf ? 1 : 0;
+        base[0] -= carry * rf;
+        base[1] += p.step[1] + carry;
+        carry = base[1] >= rm ? 1 : 0;
+        base[1] -= carry * rm;
+        base[2] += p.step[2] + carry;
+        odd ^= 1;
+        place(p);
     }
 };
 
@@ -319,7 +336,7 @@ __device__ __forceinline__ TileWork decode_tile(const PrefillParams& p, const Ti
     int blk_lo = 0, blk_hi = (p.kv_len + C::BN - 1) / C::BN;
     if (causal) {
         // the span ends are monotone in the row, so the tile's last row decides
-        const int last_key = p.vis_hi ? p.vis_hi[q_last] - 1 : min(p.kv_len - 1, q_last + off);
+        const int last_key = min(p.kv_len - 1, q_last + off);
         blk_hi = last_key >= 0 ? last_key / C::BN + 1 : 0;
         if (windowed) blk_lo = max(0, t.q0 + off - p.window + 1) / C::BN;
     }
@@ -354,10 +371,7 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     uint64_t* v_empty = v_full + VS;
     uint64_t* s_full = v_empty + VS;    // [NSB] score buffers
     uint64_t* p_full = s_full + NSB;    // [NSB]
-    // [key block & 1]: O += P V of that block has completed.  Two barriers, because with three score buffers a softmax warp
-    // may ask for block g's while that of block g - 1 still runs: on one barrier the parity it waits for is then also
-    // that of block g - 2, and it would rescale O under the MMA.  (P V of block g - 2 has completed: the scores it has of
-    // block g + 1 were computed behind it.)
+    // [key block & 1]: O += P V of that block has completed
     uint64_t* pv_done = p_full + NSB;
     uint64_t* o_full = pv_done + 2;     // one phase per tile: the tile's last O += P V has completed
     uint64_t* o_empty = o_full + 1;     // one phase per tile: the softmax warps have read O out
@@ -412,9 +426,8 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     // (the divisions, ahead of the wait: they took 1000 clk between the kernel's release and its first load)
     TileCursor cursor;
     cursor.init(p);
-    // Up to here nothing depends on the kernels in front; everything below may.  (The tail of a two-tile launch runs
-    // beside that launch, which let it start only when the kernels before it had completed.)
-    if (p.tail_base < 0) grid_dependency_wait();
+    // Up to here nothing depends on the kernels in front; everything below may.
+    grid_dependency_wait();
     grid_launch_dependents();
     if (threadIdx.x == 0) *abort_slot = *reinterpret_cast<volatile uint32_t*>(p.fault) != 0u ? 1u : 0u;
     tc_fence_before_sync();
@@ -610,7 +623,6 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
             if (causal) {
                 const int diag = t + off;
                 row_hi = min(max(diag + 1, 0), p.kv_len);
-                if (p.vis_hi && t < p.seq) row_hi = p.vis_hi[t];  // a vision block's later keys are visible too
                 if (windowed) row_lo = max(0, diag - p.window + 1);
                 if (row_lo > row_hi) row_lo = row_hi;
             }
@@ -620,117 +632,7 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
             float m = -CUDART_INF_F;  // running max, log2 domain, possibly stale by <= 8
             float l = 0.f;            // this thread's share of the row sum
 
-            // Partial maximum of the tile's block u (global block g = gb + u) over this thread's
-            // 64 keys, published for the row's other thread.  False if the scores never arrived.
-            // (The scores are fetched again for the exponentials: holding both blocks' 128 values
-            // in registers at once does not fit next to the working set.)
-            auto publish_max = [&](int u) -> bool {
-                const int g = gb + u;
-                if (!mbar_wait_warp(&s_full[g % NSB], (g / NSB) & 1)) {
-                    report_fault(p.fault, FAULT_WAIT_S, g);
-                    return false;
-                }
-                tc_fence_after_sync();
-                uint32_t wa[32], wb[32];
-                tmem_ld32(tS0 + (g % NSB) * 128, wa);
-                tmem_ld32(tS0 + (g % NSB) * 128 + 32, wb);
-                tmem_wait_ld();
-                const int kc = (tw.my_lo + u) * C::BN + kh * 64;
-                float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                float ms[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                if (has_mask) {
-                    chunk_max_any<true>(wa, mr, ms, sl, kc, rm);
-                    chunk_max_any<true>(wb, mr, ms, sl, kc + 32, rm);
-                } else {
-                    chunk_max_any<false>(wa, mr, ms, sl, kc, rm);
-                    chunk_max_any<false>(wb, mr, ms, sl, kc + 32, rm);
-                }
-                xch_max[(g & 1) * 256 + kh * 128 + r] = fmaxf(fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sl,
-                                                             fmaxf(fmaxf(ms[0], ms[1]), fmaxf(ms[2], ms[3])));
-                return true;
-            };
-
-            if constexpr (NSB >= 3) {
-                // Block 0: publish, meet, adopt the row maximum, fetch the scores.
-                if (ok) ok = publish_max(0);
-                pair_sync(quarter);
-                if (ok) {
-                    const float* xm = xch_max + (gb & 1) * 256;
-                    m = fmaxf(xm[r], xm[128 + r]);
-                    tmem_ld32(tS0 + (gb % NSB) * 128, va);
-                    tmem_ld32(tS0 + (gb % NSB) * 128 + 32, vb);
-                    tmem_wait_ld();
-                }
-
-                for (int i = 0; i < tw.n_my; ++i) {
-                    const int g = gb + i;
-                    const int kc = (tw.my_lo + i) * C::BN + kh * 64;
-                    const uint32_t tS = tS0 + (g % NSB) * 128;
-                    const bool have_next = i + 1 < tw.n_my;
-                    // The next block's scores were computed one or two blocks ago: take their maximum
-                    // now, so that the exchange through shared memory is hidden behind this block's
-                    // exponentials.
-                    if (ok && have_next) ok = publish_max(i + 1);
-                    if (ok) {
-                        // Probabilities of block i as bf16: each 32-key chunk over the first 16 of its
-                        // own 32 score columns; row-sum share in fp32.
-                        const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
-                        float ls4[4] = {0.f, 0.f, 0.f, 0.f};
-                        uint32_t pk[16];
-                        if (has_mask) {
-                            chunk_exp_any<true>(va, pk, ls4, sl, m_eff, kc, rm);
-                            tmem_st16(tS, pk);
-                            chunk_exp_any<true>(vb, pk, ls4, sl, m_eff, kc + 32, rm);
-                            tmem_st16(tS + 32, pk);
-                        } else {
-                            chunk_exp_any<false>(va, pk, ls4, sl, m_eff, kc, rm);
-                            tmem_st16(tS, pk);
-                            chunk_exp_any<false>(vb, pk, ls4, sl, m_eff, kc + 32, rm);
-                            tmem_st16(tS + 32, pk);
-                        }
-                        l += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
-                        tmem_wait_st();
-                        tc_fence_before_sync();
-                        mbar_arrive(&p_full[g % NSB]);
-                        if (have_next) {  // lands during the barrier below
-                            tmem_ld32(tS0 + ((g + 1) % NSB) * 128, va);
-                            tmem_ld32(tS0 + ((g + 1) % NSB) * 128 + 32, vb);
-                        }
-                    }
-                    if (!have_next) break;
-                    pair_sync(quarter);
-                    if (!ok) continue;
-                    const float* xm = xch_max + ((g + 1) & 1) * 256;
-                    const float m_new = fmaxf(m, fmaxf(xm[r], xm[128 + r]));
-                    const bool need = m_new > m + 8.0f;
-                    if (__any_sync(0xffffffffu, need)) {
-                        // Rare: the row maximum grows by more than 2^8 with the next block.  Once
-                        // O += P V of block i has landed, rescale this thread's half of O in tensor
-                        // memory (the row's other thread takes the same decision from the same values).
-                        const float alpha = (m_new == -CUDART_INF_F) ? 1.0f : fast_exp2(m - m_new);
-                        tmem_wait_ld();
-                        if (!mbar_wait_warp(&pv_done[g & 1], (g >> 1) & 1)) {
-                            report_fault(p.fault, FAULT_WAIT_O, g);
-                            ok = false;
-                            continue;
-                        }
-                        tc_fence_after_sync();
-                        uint32_t ww[32];
-    #pragma unroll 1
-                        for (int c = 0; c < OC / 32; ++c) {
-                            tmem_ld32(tO + c * 32, ww);
-                            tmem_wait_ld();
-    #pragma unroll
-                            for (int e = 0; e < 32; ++e) ww[e] = __float_as_uint(__uint_as_float(ww[e]) * alpha);
-                            tmem_st32(tO + c * 32, ww);
-                        }
-                        tmem_wait_st();
-                        l *= alpha;
-                        m = m_new;
-                    }
-                    tmem_wait_ld();
-                }
-            } else {
+            {
                 // Two score buffers leave no room to look ahead: S(i+1) can only be computed once P(i-1) has
                 // been consumed, so waiting for it before the exponentials of block i would put the tensor
                 // pipe and the softmax in series.  Here every block is taken on its own: maximum, exchange,
@@ -879,11 +781,6 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     tc_fence_before_sync();
     __syncthreads();
     if (warp == PRODUCER_WARP) tmem_dealloc(tmem_base, C::TMEM_COLS);
-    // A launch that covers the tail of a two-tile launch's unit list runs beside that launch (programmatic
-    // stream serialization) and reads nothing it writes — but whatever follows in the stream waits for this
-    // grid only, so this grid does not complete before the one in front of it has: every CTA ends on the
-    // grid-dependency wait (a no-op for launches without the attribute).
-    if (p.tail_base >= 0) grid_dependency_wait();
 }
 
 }  // namespace arc
