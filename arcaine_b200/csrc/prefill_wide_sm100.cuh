@@ -37,8 +37,8 @@ struct WideCfg {
     static constexpr int STAGES = 2;               // of K and of V
     static constexpr int COL_S = 0;                // + 128 * buffer
     static constexpr int COL_O = 256;
-    // q_full q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp][2]
-    static constexpr int NUM_BARS = 2 + 8 + 2 + 4 + 2 + 4 + 8;
+    // first[4] q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp][2]
+    static constexpr int NUM_BARS = 5 + 8 + 2 + 4 + 2 + 4 + 8;
     static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4 + 32;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
     static constexpr int MOST_FOLDED = 3;  // parts of a split unit that fold themselves as one cluster
@@ -249,22 +249,24 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     uint8_t* sV = sK + C::STAGES * C::K_BYTES;   // [STAGES]
     uint8_t* sOut = sV + C::STAGES * C::V_BYTES;  // output stage
     uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + STAGE_BYTES);
-    uint64_t* q_full = bars;           // leader
-    uint64_t* q_empty = bars + 1;      // both: the tile's last S = Q K^T has completed
-    uint64_t* k_full = bars + 2;       // [2] leader
-    uint64_t* k_empty = bars + 4;      // [2] both
-    uint64_t* v_full = bars + 6;       // [2] leader
-    uint64_t* v_empty = bars + 8;      // [2] both
-    uint64_t* s_full = bars + 10;      // [2] both
-    uint64_t* p_half = bars + 12;      // [buffer][half] leader: eight warps' probabilities of keys 0-63 / 64-127
-    uint64_t* o_full = bars + 16;      // both: one phase per unit
-    uint64_t* o_empty = bars + 17;     // leader: eight epilogue warps have read O out
+    // [64 head-dim columns] leader: Q and the unit's first K: the first MMAs run while the other columns arrive (96 KB: all of
+    // it first, the first scores of a call came 1000 clk later)
+    uint64_t* first = bars;
+    uint64_t* q_empty = bars + 4;      // both: the tile's last S = Q K^T has completed
+    uint64_t* k_full = bars + 5;       // [2] leader: the other K
+    uint64_t* k_empty = bars + 7;      // [2] both
+    uint64_t* v_full = bars + 9;       // [2] leader
+    uint64_t* v_empty = bars + 11;     // [2] both
+    uint64_t* s_full = bars + 13;      // [2] both
+    uint64_t* p_half = bars + 15;      // [buffer][half] leader: eight warps' probabilities of keys 0-63 / 64-127
+    uint64_t* o_full = bars + 19;      // both: one phase per unit
+    uint64_t* o_empty = bars + 20;     // leader: eight epilogue warps have read O out
     // [unit & 3] own CTA: the softmax warps have published the unit's row sums.  While the epilogue is still busy with
     // unit n - 1, units n, n + 1 and n + 2 may be through the softmax when they have one key block each (scores are
     // computed one block ahead; the first P V of n + 1 waits for the epilogue of n): with fewer slots a phase could
     // complete twice before the epilogue has looked at it, which a parity wait cannot tell from "not yet".
-    uint64_t* fin = bars + 18;
-    uint64_t* gate_bar = bars + 22;    // [epilogue warp][buffer] own CTA
+    uint64_t* fin = bars + 21;
+    uint64_t* gate_bar = bars + 25;    // [epilogue warp][buffer] own CTA
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
     float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [unit & 3][row] row sum
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         prefetch_tensormap(&tm_v);
     }
     if (threadIdx.x == 0) {
-        mbar_init(q_full, 1);
+        for (int i = 0; i < 4; ++i) mbar_init(&first[i], 1);
         mbar_init(q_empty, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&k_full[i], 1);
@@ -305,11 +307,11 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     if (warp == C::PRODUCER_WARP) tmem_alloc_pair(tmem_slot, 512);
     // One warp finds the first unit for all; its divisions, and the code that every role would fetch for them, took 2500 clk
     // between the kernel's release and its first load.
-    const int first = (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
+    const int place = (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
     const bool blocks_in_memory = MASKED || p.ids;
     WideWork w_first{};
-    if (warp == C::EPILOGUE_WARP) {
-        w_first = wide_place<SPLIT>(p, WideCursor(first, step), rank);
+    if (warp == C::PRODUCER_WARP) {
+        w_first = wide_place<SPLIT>(p, WideCursor(place, step), rank);
         if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
     }
     cluster_sync_all();  // both CTAs' barriers exist before anyone arrives on the other's
@@ -317,12 +319,54 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     grid_dependency_wait();
     grid_launch_dependents();
     if (threadIdx.x == 0) *abort_slot = *reinterpret_cast<volatile uint32_t*>(p.fault) != 0u ? 1u : 0u;
-    if (warp == C::EPILOGUE_WARP) {
+    // Q and the first K of a unit, 64 head-dim columns after 64; K or V of another block
+    auto load_first = [&](const WideWork& w, int st) {
+        const uint32_t b_first = map_to_cta(smem_u32(first), lead);
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+            if (leader && lane == 0) mbar_arrive_expect_tx(&first[c], 2 * (C::Q_CHUNK + C::K_CHUNK));
+            __syncwarp();
+            tma_load_4d_pair(sQ + c * C::Q_CHUNK, &tm_q, b_first + c * 8, c * 64, w.h, w.q0, w.b);
+            tma_load_4d_pair(sK + st * C::K_BYTES + c * C::K_CHUNK, &tm_k, b_first + c * 8, c * 64, w.kvh, w.lo * C::BN + rank * 64, w.b);
+        }
+    };
+    auto load_k = [&](const WideWork& w, int j, int st) {
+        const uint32_t b_k = map_to_cta(smem_u32(k_full), lead);
+        if (leader && lane == 0) mbar_arrive_expect_tx(&k_full[st], 2 * C::K_BYTES);
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            tma_load_4d_pair(sK + st * C::K_BYTES + c * C::K_CHUNK, &tm_k, b_k + st * 8, c * 64, w.kvh, j * C::BN + rank * 64, w.b);
+    };
+    auto load_v = [&](const WideWork& w, int j, int st) {
+        const uint32_t b_v = map_to_cta(smem_u32(v_full), lead);
+        if (leader && lane == 0) mbar_arrive_expect_tx(&v_full[st], 2 * C::V_BYTES);
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            tma_load_4d_pair(sV + st * C::V_BYTES + c * C::V_CHUNK, &tm_v, b_v + st * 8, rank * 128 + c * 64, w.kvh, j * C::BN, w.b);
+    };
+    // The first unit's first blocks are asked for before the status word has been looked at (another 500 clk).
+    int ahead_k = 0, ahead_v = 0;
+    // (The others do not wait for that: issuing takes longer than the status word.)
+    static_assert(C::THREADS == 320, "barriers 3 and 4");
+    tc_fence_before_sync();
+    if (warp == C::PRODUCER_WARP) {
         if (blocks_in_memory) wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
         if (lane == 0) *first_unit = w_first;
+        __syncwarp();
+        asm volatile("bar.arrive 3, 320;" ::: "memory");
+        ahead_k = min(w_first.hi - w_first.lo, 2), ahead_v = min(w_first.hi - w_first.lo, 1);
+        if (ahead_k > 0) {
+            load_first(w_first, 0);
+            if (ahead_k > 1) load_k(w_first, w_first.lo + 1, 1);
+            load_v(w_first, w_first.lo, 0);
+        }
+        asm volatile("bar.sync 4, 320;" ::: "memory");
+    } else {
+        asm volatile("bar.sync 3, 320;" ::: "memory");
+        asm volatile("bar.arrive 4, 320;" ::: "memory");
     }
-    tc_fence_before_sync();
-    __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
     const int total = *abort_slot ? 0 : p.total_tiles;  // a status is set: walk an empty list
@@ -379,55 +423,43 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
 
     if (warp == C::PRODUCER_WARP) {
         // ------------------------------------------------------------------ TMA producer
-        const uint32_t bq = map_to_cta(smem_u32(q_full), lead), bk = map_to_cta(smem_u32(k_full), lead), bv = map_to_cta(smem_u32(v_full), lead);
+        if (total == 0 && leader && ahead_k > 0) {  // (what has been asked for lands before the CTAs go)
+            for (int c = 0; c < 4; ++c) mbar_wait_inline(&first[c], 0);
+            if (ahead_k > 1) mbar_wait_inline(&k_full[1], 0);
+            mbar_wait_inline(&v_full[0], 0);
+        }
         int gk = 0, gv = 0, n = 0;  // K blocks, V blocks and units loaded so far
         bool ok = true;
-        auto load_k = [&](const WideWork& w, int j) {
-            const int st = gk & 1;
-            if (gk >= 2 && !mbar_wait_inline(&k_empty[st], ((gk >> 1) - 1) & 1)) {
-                if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x100u);
-                return false;
-            }
-            if (leader && lane == 0) mbar_arrive_expect_tx(&k_full[st], 2 * C::K_BYTES);
-            __syncwarp();
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                tma_load_4d_pair(sK + st * C::K_BYTES + c * C::K_CHUNK, &tm_k, bk + st * 8, c * 64, w.kvh, j * C::BN + rank * 64, w.b);
-            ++gk;
-            return true;
+        auto free_stage = [&](uint64_t* empty, int g) {
+            if (g < 2 || mbar_wait_inline(&empty[g & 1], ((g >> 1) - 1) & 1)) return true;
+            if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x100u);
+            return false;
         };
-        auto load_v = [&](const WideWork& w, int j) {
-            const int st = gv & 1;
-            if (gv >= 2 && !mbar_wait_inline(&v_empty[st], ((gv >> 1) - 1) & 1)) {
-                if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x200u);
-                return false;
-            }
-            if (leader && lane == 0) mbar_arrive_expect_tx(&v_full[st], 2 * C::V_BYTES);
-            __syncwarp();
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-                tma_load_4d_pair(sV + st * C::V_BYTES + c * C::V_CHUNK, &tm_v, bv + st * 8, rank * 128 + c * 64, w.kvh, j * C::BN, w.b);
-            ++gv;
-            return true;
-        };
-        WideCursor cur(first, step);
+        WideCursor cur(place, step);
         for (; ok && cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
             if (w.hi == w.lo) continue;
-            if (n > 0 && !mbar_wait_inline(q_empty, (n - 1) & 1)) {
-                if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u);
-                break;
+            const int have = n == 0 && cur.i == 0 ? ahead_k : 0;  // (asked for above)
+            if (have) {
+                gk = ahead_k, gv = ahead_v;
+            } else {
+                if (n > 0 && !mbar_wait_inline(q_empty, (n - 1) & 1)) {
+                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u);
+                    break;
+                }
+                ok = free_stage(k_empty, gk);
+                if (ok) load_first(w, gk++ & 1);
             }
-            if (leader && lane == 0) mbar_arrive_expect_tx(q_full, 2 * C::Q_BYTES);
-            __syncwarp();
-#pragma unroll
-            for (int c = 0; c < 4; ++c) tma_load_4d_pair(sQ + c * C::Q_CHUNK, &tm_q, bq, c * 64, w.h, w.q0, w.b);
             ++n;
             // in the order of use: K one block ahead of V
-            ok = load_k(w, w.lo);
             for (int j = w.lo; ok && j < w.hi; ++j) {
-                if (j + 1 < w.hi) ok = load_k(w, j + 1);
-                if (ok) ok = load_v(w, j);
+                if (have && j == w.lo) continue;  // (V of the first block, K of the second)
+                if (j + 1 < w.hi) {
+                    ok = free_stage(k_empty, gk);
+                    if (ok) load_k(w, j + 1, gk++ & 1);
+                }
+                if (ok) ok = free_stage(v_empty, gv);
+                if (ok) load_v(w, j, gv++ & 1);
             }
         }
     } else if (warp == C::ISSUER_WARP) {
@@ -439,34 +471,45 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             const uint64_t dK = make_smem_desc_sw128(smem_u32(sK), 16, 1024);
             const uint64_t dV = make_smem_desc_sw128(smem_u32(sV), C::V_CHUNK, 1024);
             int gs = 0, gp = 0, nq = 0, no = 0;  // score blocks, P V blocks issued; units whose scores / P V have begun
+            uint32_t k_par = 0u;                 // bit st: parity of the stage's k_full
             bool ok = true;
             // S(gs) of the unit's block j
             auto scores = [&](const WideWork& w, int j) -> bool {
                 const int st = gs & 1;
-                if (j == w.lo) {
-                    if (!mbar_wait_inline(q_full, nq & 1)) {
-                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_Q, nq);
-                        return false;
-                    }
-                    ++nq;
-                }
-                if (!mbar_wait_inline(&k_full[st], (gs >> 1) & 1)) {
-                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_K, gs);
-                    return false;
-                }
-                tc_fence_after_sync();
                 uint64_t da = dQ, db = dK + (uint64_t)(st * (C::K_BYTES >> 4));
                 uint32_t acc = 0u;
-#pragma unroll 1
-                for (int c = 0; c < 4; ++c, da += C::Q_CHUNK >> 4, db += C::K_CHUNK >> 4, acc = 1u)
+                auto chunk = [&]() {  // 64 head-dim columns
                     umma_pair_ss_x4<2, 2>(tmem_base + C::COL_S + st * 128, da, db, IDESC_QK, acc);
+                    da += C::Q_CHUNK >> 4, db += C::K_CHUNK >> 4, acc = 1u;
+                };
+                if (j == w.lo) {
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        if (!mbar_wait_inline(&first[c], nq & 1)) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_Q, nq);
+                            return false;
+                        }
+                        tc_fence_after_sync();
+                        chunk();
+                    }
+                    ++nq;
+                } else {
+                    if (!mbar_wait_inline(&k_full[st], (k_par >> st) & 1u)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_K, gs);
+                        return false;
+                    }
+                    k_par ^= 1u << st;
+                    tc_fence_after_sync();
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) chunk();
+                }
                 umma_commit_pair(&s_full[st], lead);
                 umma_commit_pair(&k_empty[st], lead);
                 if (j + 1 == w.hi) umma_commit_pair(q_empty, lead);
                 ++gs;
                 return true;
             };
-            WideCursor cur(first, step);
+            WideCursor cur(place, step);
             auto next_unit = [&](WideWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
                 for (; cur.w < total; cur.advance(p)) {
                     w = unit_at(cur);
@@ -533,7 +576,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         const uint32_t b_empty = map_to_cta(smem_u32(o_empty), lead);
         int n = 0;  // units with key blocks so far
         OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0};
-        WideCursor cur(first, step);
+        WideCursor cur(place, step);
         for (; cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
             const int t0 = w.q0 + quarter * 32, t = t0 + lane;
@@ -618,7 +661,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         int g = 0, n = 0;  // key blocks and units so far
         bool ok = true;
         uint32_t s0[32], s1[32], s2[32], s3[32];  // the row's 128 scores of the current block
-        WideCursor cur(first, step);
+        WideCursor cur(place, step);
         for (; ok && cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
             if (w.hi == w.lo) continue;
