@@ -589,12 +589,14 @@ struct DecodePlan {
     bool cluster = false;  // one launch: a cluster of `ncta` CTAs per sequence and group of KV heads
 };
 
-// Shared memory of a CTA that works on `nkv_cta` KV heads (and holds `extra` bytes): slices, stages, bytes.  False: not even two stages fit.
-static bool size_decode_cta(int hd, int nkv_cta, int batch, int extra, int smem_optin, DecodePlan* plan) {
+// Slices of 16 keys in a stage of `kb` KB of a CTA that works on `nkv_cta` KV heads, a consumer warp for each and head.
+static int most_slices(int hd, int nkv_cta, int kb) {
+    return std::max(1, std::min(kb * 1024 / (32 * nkv_cta * hd * 2), 8 / nkv_cta));
+}
+
+// Shared memory of a CTA that works on `nkv_cta` KV heads (and holds `extra` bytes): stages, bytes.  False: not even two stages fit.
+static bool size_decode_cta(int hd, int nkv_cta, int slices, int batch, int extra, int smem_optin, DecodePlan* plan) {
     const int row_bytes = nkv_cta * hd * 2;
-    int slices = (64 * 1024) / (32 * row_bytes);
-    if (slices > 8 / nkv_cta) slices = 8 / nkv_cta;
-    if (slices < 1) slices = 1;
     const int stage_bytes = 2 * 16 * slices * row_bytes;
     const int fixed = 1024 + 2 * 8 * 8 + (batch + 2) * 8 + extra;
     int stages = (smem_optin - kDecodeStaticSmem - fixed) / stage_bytes;
@@ -644,9 +646,19 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
         if (t_cluster(most * wide_group, most) > std::max(24.0, 1.3 * t_shares(most))) return;
     }
     DecodePlan one = *plan;
+    // A step of a CTA is one 16-key slice for each of its warps.  Head dim 256 has room for six a head in two stages instead of
+    // four in three: taken where the longest sequence then needs fewer steps, a step of s slices counted as 2 + s.  (One token
+    // of 24/4 heads over 513 keys, 65 a CTA: 6.74 us in two steps, 6.37 in one; 701: 6.82 and 6.38; 1501: 7.56 and 7.26; over
+    // 1001 keys four slices fill two steps, six read half as much again for nothing: 6.84 and 7.08.)
+    int slices = most_slices(p->hd, heads, 64);
+    const int wide = most_slices(p->hd, heads, 96);
+    if (p->hd == 256 && wide > slices) {
+        const long long units = ((long long)std::min(longest, 1e9) + csize * 16 - 1) / (csize * 16);  // 16-key slices of a CTA
+        if ((units + wide - 1) / wide * (2 + wide) <= (units + slices - 1) / slices * (2 + slices)) slices = wide;
+    }
     // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where
     // the stages were, at least two: 32 * hd floats a warp, at most 16 * (hd + 5) needed.)
-    if (!size_decode_cta(p->hd, heads, 0, heads * G * (p->hd + csize) * 4, ds.smem_optin, &one)) return;
+    if (!size_decode_cta(p->hd, heads, slices, 0, heads * G * (p->hd + csize) * 4, ds.smem_optin, &one)) return;
     one.cluster = true;
     one.groups = p->nkv / heads;
     one.ncta = csize;
@@ -678,7 +690,7 @@ static int plan_decode(const arc_sdpa_decode_params* p, const DeviceState& ds, D
     int nkv_cta = 1;
     for (int c = 1; c <= p->nkv && c <= max_heads; ++c)
         if (p->nkv % c == 0) nkv_cta = c;
-    if (!size_decode_cta(p->hd, nkv_cta, p->batch, 0, smem_optin, plan)) return ARC_ERR_TOO_LARGE;
+    if (!size_decode_cta(p->hd, nkv_cta, most_slices(p->hd, nkv_cta, 64), p->batch, 0, smem_optin, plan)) return ARC_ERR_TOO_LARGE;
     plan->groups = p->nkv / nkv_cta;
     int ncta = p->num_ctas > 0 ? p->num_ctas : sm_count / plan->groups;
     if (ncta < 1) ncta = 1;

@@ -400,3 +400,13 @@ def test_lengths_known_to_the_host_and_merge_blocks(ops, B, nq, nkv, hd, length,
             assert_close(on_host[1][b], wf[0], f"seq {b} f32", rel_tol=3e-3, abs_tol=5e-3)
             assert_close(on_host[0][b], wgb[0].float(), f"seq {b} gated")
             assert torch.allclose(on_host[2][b].cpu(), wl[0], atol=2e-3)
+
+
+@pytest.mark.parametrize("nq,nkv", [(24, 4), (8, 8), (16, 1)])  # groups of six, one and sixteen heads
+@pytest.mark.parametrize("n", [513, 768, 769, 1501])  # one step of six slices, its last full one, two steps, a ragged second one
+def test_one_launch_form_in_steps_of_six_slices(ops, n, nq, nkv):
+    q, k, v, g = (seeded_bf16(*shape, seed=400 + i) for i, shape in enumerate([(1, nq, 256), (n + 30, nkv, 256), (n + 30, nkv, 256), (1, nq, 256)]))
+    before = ops.launch_count()
+    got = ops.sdpa_decode(q.cuda(), k.cuda()[None], v.cuda()[None], scale=0.0625, kv_len=n, gate=g.cuda())
+    assert ops.launch_count() - before == 1
+    assert_close(got[0], oracle_decode(q[0], k[:n], v[:n], 0.0625, gate=g[0])[1][0].float(), f"{n} keys")
