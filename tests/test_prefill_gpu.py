@@ -397,3 +397,11 @@ def test_vision_blocks_two_tiles_per_cta(ops, nq, nkv):
         # the same visible keys; blocks may be skipped in one form and fully masked in the other
         assert_close(got, want.float(), f"window {window}", rel_tol=4e-3, abs_tol=1.6e-2)
         assert torch.allclose(lse, want_lse, atol=2e-3)
+
+
+@pytest.mark.parametrize("q_len,kv_len", [(4100, 1030), (4097, 1000), (2049, 2050)])  # from 4097 blocks of a row on, a block writes four
+@pytest.mark.parametrize("window", [300, oracle.INT_MAX])
+def test_mask_fill_of_many_rows(ops, q_len, kv_len, window):
+    past = max(0, kv_len - q_len)
+    got = ops.fill_causal_mask(q_len, kv_len, past, window).cpu().numpy()
+    assert (got == oracle.fill_causal_mask(q_len, kv_len, past, window)).all()
