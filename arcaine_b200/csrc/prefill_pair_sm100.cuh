@@ -1,39 +1,39 @@
 // GQA flash-attention prefill kernel for sm_100a, head dim 128: two query tiles per CTA.
 //
 // A CTA owns two 128-row query tiles, A and B, that walk the same key blocks.  Each tile is a pipeline of its own:
-// four softmax warps (one query row per thread, TMEM lane = row, so row maxima and sums never leave the thread), one
-// score buffer S and one accumulator O in tensor memory (S_A S_B O_A O_B = 512 columns), one Q buffer in shared
-// memory.  The two pipelines share the K and V rings, which one producer thread fills by TMA, so every key block is
-// fetched once for 256 rows, and one MMA-issuing warp, which keeps them out of phase.
+// four softmax warps (one query row per thread, TMEM lane = row, so row maxima and sums never leave the thread), P and
+// one accumulator O in tensor memory, one Q buffer in shared memory.  The two share the score buffer, which they use in
+// turn (S P_A P_B O_A O_B = 128 + 2 x 64 + 2 x 128 = 512 columns), and the K and V rings, which one producer thread fills
+// by TMA, so every key block is fetched once for 256 rows.
 //
 // Sixteen warps in groups with register budgets of their own (setmaxnreg):
 //   warps 0-3 / 4-7   softmax of tile A / B: a thread takes its row's 128 scores out of tensor
-//                     memory ONCE, masks them in registers where the block needs it, takes the
-//                     maximum, exponentiates and writes P (bf16) back over the scores;
+//                     memory ONCE and frees the score buffer, masks them in registers where the block needs it, takes
+//                     the maximum, exponentiates and writes P (bf16) into the pipeline's own columns;
 //   warps 8-11        epilogue: once a tile's last O += P V has landed they read the accumulator
 //                     out, normalise, gate and store it, while the softmax warps are already
 //                     working on the next tile's first key block;
-//   warps 12-15       TMA producer of K / V, MMA issuer, (idle), TMA producer of Q.
+//   warps 12-15       TMA producer of K / V, issuer of S = Q K^T, issuer of O += P V, TMA producer of Q.
 //
-// What bounds it.  Per key block and tile 1024 clk of the tensor pipe (64 per M128 N128 K16 MMA, both operand forms),
-// 1024 clk of the ex2 unit (16 a clock), and the chain scores -> maximum -> exponentials -> O += P V -> next scores:
-// P is written over S, so the next scores can only follow the P V that reads them.  The two tiles half a period apart
-// hide each other's tensor time.  Measured with stamps in shared memory, a pair of key blocks takes 3000-3200 clk:
-// softmax of one tile 1800-1950 (400 loads and maximum, 3 x 350 and 400 for the four 32-key chunks; the ex2 unit
-// alone would be 1024), then 250 for the second half of P V, 512 for the scores and 2 x 150 for barriers.
-// What made the difference (4 x 8192 tokens, 32 / 16 heads, window 1024: 691 -> 502 us, 0.45 -> 0.62 of the measured
-// bf16 rate; 2 x 8192, no mask: 1030 -> 800 us):
+// What bounds it.  Per key block and tile 1024 clk of the tensor pipe (64 per M128 N128 K16 MMA, both operand forms)
+// and 1024 clk of the ex2 unit (16 a clock), 2048 of either for a pair of blocks, which takes 2490 clk (2 x 8192 tokens of
+// 32/16 heads, no mask).  With P written over S, as it was, a pipeline's next scores had to wait for the P V that
+// reads them, and a pair of blocks took 2950.  Now they are computed while the block before is exponentiated.  The clock
+// gives part of it back: at this density of work the chip holds 1.40 GHz against its power limit, 1.48 before (1833 ->
+// 1660 us, 0.95 of what cuBLAS sustains in bf16; window 1024, 4 x 8192 tokens: 572 -> 526 us).  Tried on it and slower: one
+// warp for all MMAs (2710 clk: the tensor pipe runs dry while it looks after barriers between two groups), scores strictly
+// ahead of P V in the tensor pipe (2-3 %), all 128 scores behind one wait, P announced once a block.
+// What made the difference before that (4 x 8192 tokens, window 1024: 691 -> 502 us at full clock):
 //   - MMA issue: elect.sync inside the asm statement and warp-uniform operands (an
 //     MMA every 64-90 clk instead of every 125);
-//   - one issuer for both pipelines in a fixed order instead of two issuers and a turn protocol between the softmax
-//     warps: a single warp needs 1200 clk for the exponentials of a block on its own, two on one scheduler 2000
-//     for both, so giving them exclusive turns wasted 40 % of the ex2 unit;
+//   - no turns between the softmax warps: a single warp needs 1200 clk for the exponentials of a block on its own, two on
+//     one scheduler 2000 for both, so giving them exclusive turns wasted 40 % of the ex2 unit;
 //   - code size: hot code of a scheduler beyond ~8 KB costs ~50 clk per 128 bytes, so masking is one select per score
 //     from a bit mask, the epilogue and all MMA loops are rolled, packed fp32 arithmetic halves the rest.  (Re-reading
 //     the scores in a rolled loop would be smaller still but measured 2-5 % slower.)
 //
-// Lazy rescaling, bounded waits and the device status word are as in the single-tile kernel (prefill_sm100.cuh),
-// which keeps additive masks, key-range splits and small problems.
+// Lazy rescaling: O is rescaled in tensor memory only where a row's maximum grows by more than 2^8.  Calls with few tiles,
+// parts of a key range and additive masks are prefill_chains_sm100.cuh's.
 #pragma once
 #include "prefill_sm100.cuh"
 
@@ -576,8 +576,6 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
             }
         } else {
             // -------------------------------------------------------------- O += P V of both pipelines
-            // A warp of its own: with one warp for all MMAs the tensor pipe ran dry while it looked after the barriers
-            // between two groups (2710 clk per pair of blocks for 2048 of MMAs).
             constexpr uint32_t IDESC_PV = make_idesc_bf16(128, HD, true);
             const uint64_t dV = make_smem_desc_sw128(smem_u32(sV), C::CHUNK_BYTES, 1024);
             int r = 0;             // ring position: key blocks so far

@@ -17,7 +17,7 @@
 // expects the bytes of both CTAs; empty and score barriers are committed to both (commit with multicast — the loads
 // themselves use none).  The softmax and epilogue warps of both CTAs arrive on the leader's barriers.
 //
-// Masks, lazy rescaling, P over the scores, bounded waits and the status word are as in prefill_pair_sm100.cuh.
+// Masks, lazy rescaling, bounded waits and the status word are as in prefill_pair_sm100.cuh; P is written over the scores.
 #pragma once
 #include "decode_sm100.cuh"
 #include "prefill_pair_sm100.cuh"
