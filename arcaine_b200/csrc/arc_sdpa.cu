@@ -46,7 +46,7 @@ struct DeviceState {
     uint32_t* fault = nullptr;
     int sm_count = 0;
     int smem_optin = 0;
-    int decode_clusters[4] = {0, 0, 0, 0};  // [log2(size)]: clusters of the one-launch decode the device holds at once
+    int decode_clusters[9] = {};  // [size]: clusters of the one-launch decode the device holds at once
     WideRoom wide;
 };
 
@@ -166,8 +166,8 @@ static int device_state(DeviceState** out) {
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, true>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, true>, s.smem_optin - kDecodeStaticSmem));
-            for (int lg = 0; lg < 4; ++lg)
-                s.decode_clusters[lg] = clusters_at_once(sdpa_decode_kernel<256, 1, true>, 1 << lg, s.sm_count, 288, s.smem_optin - kDecodeStaticSmem);
+            for (int size = 1; size <= 8; ++size)
+                s.decode_clusters[size] = clusters_at_once(sdpa_decode_kernel<256, 1, true>, size, s.sm_count, 288, s.smem_optin - kDecodeStaticSmem);
             s.ready.store(true, std::memory_order_release);
         }
     }
@@ -623,9 +623,9 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
     const int G = p->nq / p->nkv;
     int heads = 0, csize = 0;  // the smallest group of heads and then the largest cluster that are all resident at once
     for (int c = 1; c <= nkv_cta && !heads; ++c)
-        if (p->nkv % c == 0 && (long long)p->batch * (p->nkv / c) <= ds.decode_clusters[0]) heads = c;
-    for (int lg = 3; heads && lg >= 0 && !csize; --lg)
-        if ((long long)p->batch * (p->nkv / heads) <= ds.decode_clusters[lg]) csize = 1 << lg;
+        if (p->nkv % c == 0 && (long long)p->batch * (p->nkv / c) <= ds.decode_clusters[1]) heads = c;
+    for (int size = 8; heads && size >= 1 && !csize; --size)
+        if ((long long)p->batch * (p->nkv / heads) <= ds.decode_clusters[size]) csize = size;
     if (!csize) return;
     double longest = (double)p->kv_len_uniform, total = longest * p->batch;
     if (p->kv_len) {
@@ -634,18 +634,32 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
             longest = 2.0 * (double)p->kv_rows_total / p->batch;
         total = longest * (0.5 * p->batch + 0.5);
     }
-    const double ctas = (double)p->batch * (p->nkv / heads) * csize;
-    const double all = heads * p->hd >= 1024 ? 6.0e6 : 6.9e6 - 6e3 * (ds.sm_count - ctas);
-    const double per_longest = heads * p->hd * 4.0 / csize / (p->hd == 256 ? 93e3 : 105e3), per_key = p->nkv * p->hd * 4.0;
-    auto t_cluster = [&](double most, double keys) { return 5.2 + std::max(most * per_longest, keys * per_key / all); };
-    auto t_shares = [&](double keys) { return (p->kv_len ? 8.0 : 7.2) + 0.1 * p->batch + keys * per_key / 7.0e6; };
-    if (t_cluster(longest, total) > t_shares(total)) return;
-    if (p->kv_len) {
+    // Three, five, six or seven CTAs at head dim 128 where the longest sequence then takes fewer steps than in two or four, at
+    // 256 where it would be too long for these.  (12 sequences of 200 to 6000 keys, 16/2 heads of 128: 12.5 us in fours, 11.5 in
+    // sixes; 24 of 100 to 900, 8/1, two steps either way: 7.1 in fours, 7.4 in sixes.  Head dim 256, with six warps a CTA, 24/4: 6
+    // of 300 to 2000 10.3 and 11.2; 5 packed ones of 300 to 3000: 16.8 by shares, 11.5 in sevens.)
+    const int most_ctas = csize;
+    int finishers = 1;  // CTAs that finish columns: the largest power of two there is
+    while (finishers * 2 <= csize) finishers *= 2;
+    const long long keys = (long long)std::min(longest, 1e9), step = 16 * most_slices(p->hd, heads, 64);
+    if (p->hd == 256 || (keys + csize * step - 1) / (csize * step) >= (keys + finishers * step - 1) / (finishers * step)) csize = finishers;
+    const double per_key = p->nkv * p->hd * 4.0;
+    auto t_shares = [&](double k) { return (p->kv_len ? 8.0 : 7.2) + 0.1 * p->batch + k * per_key / 7.0e6; };
+    auto worth_it = [&](int size) {
+        const double ctas = (double)p->batch * (p->nkv / heads) * size;
+        const double all = heads * p->hd >= 1024 ? 6.0e6 : 6.9e6 - 6e3 * (ds.sm_count - ctas);
+        const double per_longest = heads * p->hd * 4.0 / size / (p->hd == 256 ? 93e3 : 105e3);
+        auto t_cluster = [&](double most, double k) { return 5.2 + std::max(most * per_longest, k * per_key / all); };
+        if (t_cluster(longest, total) > t_shares(total)) return false;
+        if (!p->kv_len) return true;
         const double most = p->max_kv_len > 0 ? std::min((double)p->max_kv_len, (double)p->kv_rows_total) : (double)p->kv_rows_total;
         const double wide_group = G <= 8 ? 1.0 : p->hd == 256 ? 4.0 : 1.6;  // (two tiles of heads a warp: the rates are that much lower)
-        if (t_cluster(most * wide_group, most) > std::max(24.0, 1.3 * t_shares(most))) return;
+        return t_cluster(most * wide_group, most) <= std::max(24.0, 1.3 * t_shares(most));
+    };
+    if (!worth_it(csize)) {
+        csize = most_ctas;
+        if (csize == finishers || !worth_it(csize)) return;
     }
-    DecodePlan one = *plan;
     // A step of a CTA is one 16-key slice for each of its warps.  Head dim 256 has room for six a head in two stages instead of
     // four in three: taken where the longest sequence then needs fewer steps, a step of s slices counted as 2 + s.  (One token
     // of 24/4 heads over 513 keys, 65 a CTA: 6.74 us in two steps, 6.37 in one; 701: 6.82 and 6.38; 1501: 7.56 and 7.26; over
@@ -656,9 +670,10 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
         const long long units = ((long long)std::min(longest, 1e9) + csize * 16 - 1) / (csize * 16);  // 16-key slices of a CTA
         if ((units + wide - 1) / wide * (2 + wide) <= (units + slices - 1) / slices * (2 + slices)) slices = wide;
     }
+    DecodePlan one = *plan;
     // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where
     // the stages were, at least two: 32 * hd floats a warp, at most 16 * (hd + 5) needed.)
-    if (!size_decode_cta(p->hd, heads, slices, 0, heads * G * (p->hd + csize) * 4, ds.smem_optin, &one)) return;
+    if (!size_decode_cta(p->hd, heads, slices, 0, heads * G * (p->hd / finishers * csize + csize) * 4, ds.smem_optin, &one)) return;
     one.cluster = true;
     one.groups = p->nkv / heads;
     one.ncta = csize;
@@ -742,6 +757,8 @@ static int launch_decode(const arc_sdpa_decode_params* p, const DecodePlan& plan
         kp.out_f32 = p->out_f32;
         kp.out_lse = p->out_lse;
         kp.o_stride_b = p->o_stride_b;
+        kp.dc_log2 = HD == 256 ? 8 : 7;
+        for (int c = plan.ncta; c > 1; c /= 2) --kp.dc_log2;
         grid.z = (unsigned)p->batch;
         ARC_CUDA(launch_dependent(plan.nt == 1 ? sdpa_decode_kernel<HD, 1, true> : sdpa_decode_kernel<HD, 2, true>, grid, dim3(threads),
                                   (size_t)plan.smem_bytes, stream, plan.ncta, tk, tv, kp));

@@ -55,7 +55,8 @@ struct DecodeParams {
     int ncta;     // grid.x
     int max_kv_len;            // > 0: no sequence may be longer
     long long kv_rows_total;   // rows addressable from k and v
-    // The form that finishes in one launch (sdpa_decode_kernel<.., true>): the results
+    // The form that finishes in one launch (sdpa_decode_kernel<.., true>): log2 of the columns a CTA finishes, the results
+    int dc_log2;
     const uint16_t* gate;
     uint16_t* out;
     float* out_f32;
@@ -205,12 +206,13 @@ __global__ void __launch_bounds__(288, 1)
     // keys before sequence b / up to its end, in the count g0 and g1 use
     auto seq_begin = [&](int b) { return CLUSTER ? 0ll : cum[b]; };
     auto seq_end = [&](int b) { return CLUSTER ? (long long)my_len : cum[b + 1]; };
-    // CLUSTER: CTA c of the cluster finishes columns [c, c + 1) * HD / ncta of all heads; the others leave their folded
-    // records of those here: [CTA][query head of the group][column], and the log-sum-exps behind.
+    // CLUSTER: the first 2^k CTAs of the cluster (all of 1, 2, 4 or 8, four of six) finish an equal number of columns of all
+    // heads each; the others leave their folded records of those here: [CTA][query head of the group][column], and the
+    // log-sum-exps behind.
     float* crec = reinterpret_cast<float*>(cum + 2);
-    const int dc_log2 = (HD == 256 ? 8 : 7) - (CLUSTER ? __ffs(p.ncta) - 1 : 0), dc = 1 << dc_log2;  // (clusters are of 1, 2, 4 or 8)
+    const int dc_log2 = p.dc_log2, dc = 1 << dc_log2;
     const int rows = p.nkv_cta * G;
-    float* crec_lse = crec + (size_t)rows * HD;
+    float* crec_lse = crec + ((p.ncta * rows) << dc_log2);
     constexpr int RS = HD + 4;  // floats from one head's row of a warp's record to the next
 
     if (warp == ncw) {
@@ -538,7 +540,7 @@ __global__ void __launch_bounds__(288, 1)
         // This CTA's columns, two a thread.  Every record is in its own shared memory by now: read out of the other CTAs
         // instead, 16 loads a thread, this step took 2100 clk.
         if (threadIdx.x == 0 && (!work || fault != 0u)) cum[0] = 0;
-        const int items = rows * (dc / 2), b = blockIdx.z;
+        const int items = (int)(blockIdx.x << dc_log2) < HD ? rows * (dc / 2) : 0, b = blockIdx.z;
         auto offset_of = [&](int item) {
             return (long long)b * p.o_stride_b + (long long)(head0 * G + (item >> (dc_log2 - 1))) * HD + blockIdx.x * dc + (item & (dc / 2 - 1)) * 2;
         };

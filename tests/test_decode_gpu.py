@@ -410,3 +410,23 @@ def test_one_launch_form_in_steps_of_six_slices(ops, n, nq, nkv):
     got = ops.sdpa_decode(q.cuda(), k.cuda()[None], v.cuda()[None], scale=0.0625, kv_len=n, gate=g.cuda())
     assert ops.launch_count() - before == 1
     assert_close(got[0], oracle_decode(q[0], k[:n], v[:n], 0.0625, gate=g[0])[1][0].float(), f"{n} keys")
+
+
+@pytest.mark.parametrize("B,nq,nkv,hd,n", [
+    (12, 16, 2, 128, 1700),  # 24 clusters: six CTAs each, four of which finish columns
+    (5, 24, 4, 256, 900),    # 20: as many as fit
+    (7, 24, 4, 256, 1000),   # 28: five
+    (45, 8, 1, 128, 600),    # three
+    (12, 32, 2, 256, 800),   # sixteen heads a KV head
+])
+def test_one_launch_form_in_clusters_of_any_size(ops, B, nq, nkv, hd, n):
+    lens = [max(1, n - 53 * b) for b in range(B)]
+    q, k, v, g = (seeded_bf16(*shape, seed=500 + i) for i, shape in enumerate([(B, nq, hd), (B, n, nkv, hd), (B, n, nkv, hd), (B, nq, hd)]))
+    got, o32, lse = ops.sdpa_decode(q.cuda(), k.cuda(), v.cuda(), scale=hd ** -0.5, kv_len=torch.tensor(lens, dtype=torch.int32, device="cuda"),
+                                    gate=g.cuda(), return_partial=True)
+    for b in range(0, B, max(1, B // 6)):
+        wf, _, wl = oracle_decode(q[b], k[b, :lens[b]], v[b, :lens[b]], hd ** -0.5)
+        _, wgb, _ = oracle_decode(q[b], k[b, :lens[b]], v[b, :lens[b]], hd ** -0.5, gate=g[b])
+        assert_close(o32[b], wf[0], f"seq {b} f32", rel_tol=3e-3, abs_tol=5e-3)
+        assert_close(got[b], wgb[0].float(), f"seq {b} gated")
+        assert torch.allclose(lse[b].cpu(), wl[0], atol=2e-3)
