@@ -412,21 +412,51 @@ def test_one_launch_form_in_steps_of_six_slices(ops, n, nq, nkv):
     assert_close(got[0], oracle_decode(q[0], k[:n], v[:n], 0.0625, gate=g[0])[1][0].float(), f"{n} keys")
 
 
+def check_ragged_batch(ops, q, k, v, g, lens, rows=None):
+    """One launch, and every sixth sequence's results against the oracle; rows: first rows of a packed cache."""
+    hd = q.shape[2]
+    before = ops.launch_count()
+    got, o32, lse = ops.sdpa_decode(q.cuda(), k.cuda(), v.cuda(), scale=hd ** -0.5, kv_len=torch.tensor(lens, dtype=torch.int32, device="cuda"),
+                                    kv_row_offset=None if rows is None else torch.tensor(rows, dtype=torch.int64, device="cuda"),
+                                    gate=g.cuda(), return_partial=True)
+    assert ops.launch_count() - before == 1
+    for b in sorted({*range(0, len(lens), max(1, len(lens) // 6)), len(lens) - 1}):
+        kb, vb = (k[b, :lens[b]], v[b, :lens[b]]) if rows is None else (k[rows[b]:rows[b] + lens[b]], v[rows[b]:rows[b] + lens[b]])
+        if lens[b] == 0:
+            assert torch.count_nonzero(got[b].float()) == 0 and torch.isinf(lse[b]).all()
+            continue
+        wf, _, wl = oracle_decode(q[b], kb, vb, hd ** -0.5)
+        _, wgb, _ = oracle_decode(q[b], kb, vb, hd ** -0.5, gate=g[b])
+        assert_close(o32[b], wf[0], f"seq {b} f32", rel_tol=3e-3, abs_tol=5e-3)
+        assert_close(got[b], wgb[0].float(), f"seq {b} gated")
+        assert torch.allclose(lse[b].cpu(), wl[0], atol=2e-3)
+
+
 @pytest.mark.parametrize("B,nq,nkv,hd,n", [
-    (12, 16, 2, 128, 1700),  # 24 clusters: six CTAs each, four of which finish columns
-    (5, 24, 4, 256, 900),    # 20: as many as fit
-    (7, 24, 4, 256, 1000),   # 28: five
-    (45, 8, 1, 128, 600),    # three
+    (12, 16, 2, 128, 1700),  # 24 clusters: five CTAs each, four of which finish columns
+    (5, 24, 4, 256, 900),    # 20: six would fit, but four are enough for so few keys
+    (7, 24, 4, 256, 1000),   # 28: four of five
+    (45, 8, 1, 128, 600),    # three, two of which finish columns
     (12, 32, 2, 256, 800),   # sixteen heads a KV head
 ])
 def test_one_launch_form_in_clusters_of_any_size(ops, B, nq, nkv, hd, n):
     lens = [max(1, n - 53 * b) for b in range(B)]
     q, k, v, g = (seeded_bf16(*shape, seed=500 + i) for i, shape in enumerate([(B, nq, hd), (B, n, nkv, hd), (B, n, nkv, hd), (B, nq, hd)]))
-    got, o32, lse = ops.sdpa_decode(q.cuda(), k.cuda(), v.cuda(), scale=hd ** -0.5, kv_len=torch.tensor(lens, dtype=torch.int32, device="cuda"),
-                                    gate=g.cuda(), return_partial=True)
-    for b in range(0, B, max(1, B // 6)):
-        wf, _, wl = oracle_decode(q[b], k[b, :lens[b]], v[b, :lens[b]], hd ** -0.5)
-        _, wgb, _ = oracle_decode(q[b], k[b, :lens[b]], v[b, :lens[b]], hd ** -0.5, gate=g[b])
-        assert_close(o32[b], wf[0], f"seq {b} f32", rel_tol=3e-3, abs_tol=5e-3)
-        assert_close(got[b], wgb[0].float(), f"seq {b} gated")
-        assert torch.allclose(lse[b].cpu(), wl[0], atol=2e-3)
+    check_ragged_batch(ops, q, k, v, g, lens)
+
+
+@pytest.mark.parametrize("B,nq,nkv,total", [
+    (5, 24, 4, 7600),   # 20 clusters of six CTAs in steps of six slices
+    (12, 16, 2, 7600),  # 24 of five, groups of eight heads
+    (40, 6, 1, 4300),   # 40 of three, two of which finish columns
+    (10, 32, 2, 1900),  # 20 of six, sixteen heads a KV head
+])
+def test_one_launch_form_in_uneven_clusters_at_head_dim_256(ops, B, nq, nkv, total):
+    """Packed caches in which one sequence could hold so many keys that a power of two of CTAs would be judged too slow for it
+    and equal shares, two launches, taken: one launch says that all CTAs that fit were.  Two sequences have nearly all
+    keys, the others so few that the last CTAs have none."""
+    short = [b * 7 % 40 for b in range(B - 2)]  # (none at all for the first)
+    lens = [*short, (total - sum(short)) // 3, total - sum(short) - (total - sum(short)) // 3]
+    rows = [sum(lens[:b]) for b in range(B)]
+    q, k, v, g = (seeded_bf16(*shape, seed=600 + i) for i, shape in enumerate([(B, nq, 256), (total, nkv, 256), (total, nkv, 256), (B, nq, 256)]))
+    check_ragged_batch(ops, q, k, v, g, lens, rows)
