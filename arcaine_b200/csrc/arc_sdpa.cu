@@ -160,12 +160,16 @@ static int device_state(DeviceState** out) {
             }
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, true>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, true, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, true>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, true, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, true>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, true, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, true>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, true, false>, s.smem_optin - kDecodeStaticSmem));
             for (int size = 1; size <= 8; ++size)
                 s.decode_clusters[size] = clusters_at_once(sdpa_decode_kernel<256, 1, true>, size, s.sm_count, 288, s.smem_optin - kDecodeStaticSmem);
             s.ready.store(true, std::memory_order_release);
@@ -673,7 +677,7 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
     DecodePlan one = *plan;
     // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where
     // the stages were, at least two: 32 * hd floats a warp, at most 16 * (hd + 5) needed.)
-    if (!size_decode_cta(p->hd, heads, slices, 0, heads * G * (p->hd / finishers * csize + csize) * 4, ds.smem_optin, &one)) return;
+    if (!size_decode_cta(p->hd, heads, slices, 0, heads * G * (p->hd / finishers * csize + (csize & (csize - 1) ? 8 : csize)) * 4, ds.smem_optin, &one)) return;
     one.cluster = true;
     one.groups = p->nkv / heads;
     one.ncta = csize;
@@ -757,11 +761,11 @@ static int launch_decode(const arc_sdpa_decode_params* p, const DecodePlan& plan
         kp.out_f32 = p->out_f32;
         kp.out_lse = p->out_lse;
         kp.o_stride_b = p->o_stride_b;
-        kp.dc_log2 = HD == 256 ? 8 : 7;
-        for (int c = plan.ncta; c > 1; c /= 2) --kp.dc_log2;
+        const bool even = (plan.ncta & (plan.ncta - 1)) == 0;
+        auto kernel = plan.nt == 1 ? (even ? sdpa_decode_kernel<HD, 1, true> : sdpa_decode_kernel<HD, 1, true, false>)
+                                   : (even ? sdpa_decode_kernel<HD, 2, true> : sdpa_decode_kernel<HD, 2, true, false>);
         grid.z = (unsigned)p->batch;
-        ARC_CUDA(launch_dependent(plan.nt == 1 ? sdpa_decode_kernel<HD, 1, true> : sdpa_decode_kernel<HD, 2, true>, grid, dim3(threads),
-                                  (size_t)plan.smem_bytes, stream, plan.ncta, tk, tv, kp));
+        ARC_CUDA(launch_dependent(kernel, grid, dim3(threads), (size_t)plan.smem_bytes, stream, plan.ncta, tk, tv, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
         return ARC_OK;
     }

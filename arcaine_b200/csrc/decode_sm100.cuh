@@ -55,8 +55,7 @@ struct DecodeParams {
     int ncta;     // grid.x
     int max_kv_len;            // > 0: no sequence may be longer
     long long kv_rows_total;   // rows addressable from k and v
-    // The form that finishes in one launch (sdpa_decode_kernel<.., true>): log2 of the columns a CTA finishes, the results
-    int dc_log2;
+    // The form that finishes in one launch (sdpa_decode_kernel<.., true>): the results
     const uint16_t* gate;
     uint16_t* out;
     float* out_f32;
@@ -108,7 +107,10 @@ __device__ __forceinline__ void consumer_sync(int consumer_warps) {
 // the sequence's keys, fold their slices as above, leave the records in the shared memory of the CTAs that finish them
 // and write the result: one launch, no records in global memory, no merge kernel.  For calls so small that the
 // launches are what they cost; otherwise equal shares over all SMs win.
-template <int HD, int NT, bool CLUSTER>
+// EVEN (of CLUSTER): a power of two of CTAs, all of which finish columns.  As a case of the other instance these calls were 0.1
+// to 0.2 us slower (one token of 24/4 heads over 256 / 1001 keys 6.31 / 6.96 us, 6.16 / 6.76 so; 16 sequences of 500 keys,
+// 8/4 heads of 128: 7.92 and 7.70).
+template <int HD, int NT, bool CLUSTER, bool EVEN = true>
 __global__ void __launch_bounds__(288, 1)
     sdpa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const DecodeParams p) {
@@ -208,11 +210,11 @@ __global__ void __launch_bounds__(288, 1)
     auto seq_end = [&](int b) { return CLUSTER ? (long long)my_len : cum[b + 1]; };
     // CLUSTER: the first 2^k CTAs of the cluster (all of 1, 2, 4 or 8, four of six) finish an equal number of columns of all
     // heads each; the others leave their folded records of those here: [CTA][query head of the group][column], and the
-    // log-sum-exps behind.
-    float* crec = reinterpret_cast<float*>(cum + 2);
-    const int dc_log2 = p.dc_log2, dc = 1 << dc_log2;
+    // log-sum-exps behind (not EVEN: in front, eight places a head, so that no address waits for p.ncta).
+    const int dc_log2 = (HD == 256 ? 8 : 7) - (!CLUSTER ? 0 : EVEN ? __ffs(p.ncta) - 1 : 31 - __clz(p.ncta)), dc = 1 << dc_log2;
     const int rows = p.nkv_cta * G;
-    float* crec_lse = crec + ((p.ncta * rows) << dc_log2);
+    float* crec = reinterpret_cast<float*>(cum + 2) + (EVEN ? 0 : 8 * rows);
+    float* crec_lse = EVEN ? crec + (size_t)rows * HD : reinterpret_cast<float*>(cum + 2);
     constexpr int RS = HD + 4;  // floats from one head's row of a warp's record to the next
 
     if (warp == ncw) {
@@ -540,7 +542,7 @@ __global__ void __launch_bounds__(288, 1)
         // This CTA's columns, two a thread.  Every record is in its own shared memory by now: read out of the other CTAs
         // instead, 16 loads a thread, this step took 2100 clk.
         if (threadIdx.x == 0 && (!work || fault != 0u)) cum[0] = 0;
-        const int items = (int)(blockIdx.x << dc_log2) < HD ? rows * (dc / 2) : 0, b = blockIdx.z;
+        const int items = EVEN || (int)(blockIdx.x << dc_log2) < HD ? rows * (dc / 2) : 0, b = blockIdx.z;
         auto offset_of = [&](int item) {
             return (long long)b * p.o_stride_b + (long long)(head0 * G + (item >> (dc_log2 - 1))) * HD + blockIdx.x * dc + (item & (dc / 2 - 1)) * 2;
         };
