@@ -96,23 +96,20 @@ struct PairWork {
 // Vision blocks (a query inside a block of equal non-negative ids also sees the block's later keys).  The ends are looked
 // up where they are needed: a launch of its own for one end per row took 4.5 us in front of a kernel of 20.
 // ---------------------------------------------------------------------------
-// The ids of the 512 keys from k0 on, 16 a lane (past the last key: no block's).  Asked for together with the id they are
-// compared with: one trip to memory where runs of 128 keys a step behind the id took four for an image of 256 tokens.
-__device__ __forceinline__ void load_ids(const int* ids, int kv_len, int k0, int (&v)[16]) {
+// First key after `key` that does not carry `id`.  Whole warps, 128 keys a step.  (512 at once, asked for together with `id`, were
+// 5 KB of code in every kernel of head dim 256, which calls without ids jump over: from cold caches a canvas step took 22.1 us,
+// 21.4 so, and vision prompts were no faster for it — 3000 tokens of 16/8 heads of 128 31.2 us, 29.1 so.)
+__device__ __forceinline__ int run_end(const int* ids, int kv_len, int key, int id) {
     const int lane = threadIdx.x & 31;
+    for (int k0 = key + 1;; k0 += 128) {
+        bool other[4];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = k0 + 32 * i + lane < kv_len ? ids[k0 + 32 * i + lane] : -2;
-}
-
-// First key from k0 on that does not carry `id`; v: their ids.  Whole warps.
-__device__ __forceinline__ int run_end(const int* ids, int kv_len, int k0, int id, int (&v)[16]) {
-    for (;; k0 += 512) {
+        for (int i = 0; i < 4; ++i) other[i] = k0 + 32 * i + lane >= kv_len || ids[k0 + 32 * i + lane] != id;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const uint32_t found = __ballot_sync(0xffffffffu, v[i] != id);
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t found = __ballot_sync(0xffffffffu, other[i]);
             if (found) return k0 + 32 * i + __ffs(found) - 1;
         }
-        load_ids(ids, kv_len, k0 + 512, v);
     }
 }
 
@@ -120,23 +117,18 @@ __device__ __forceinline__ int run_end(const int* ids, int kv_len, int k0, int i
 __device__ __forceinline__ int vision_end(const PrefillParams& p, int self) {
     const int plain = min(max(self + 1, 0), p.kv_len);
     if (self < 0 || self >= p.kv_len) return plain;
-    int v[16];
     const int id = p.ids[self];
-    load_ids(p.ids, p.kv_len, self + 1, v);
-    return id >= 0 ? run_end(p.ids, p.kv_len, self + 1, id, v) : plain;
+    return id >= 0 ? run_end(p.ids, p.kv_len, self, id) : plain;
 }
 
 // The same for a warp's 32 consecutive rows, one per lane (row: t < seq).
 __device__ __forceinline__ int vision_ends(const PrefillParams& p, int self, bool row) {
     const int lane = threadIdx.x & 31;
     const int id = row && self >= 0 && self < p.kv_len ? p.ids[self] : -1;
-    const int last = __shfl_sync(0xffffffffu, self, 31);
-    int v[16];
-    load_ids(p.ids, p.kv_len, max(last, -1) + 1, v);
     const int next_id = __shfl_down_sync(0xffffffffu, id, 1);  // (all lanes take part; lane 31 does not use it)
     const uint32_t breaks = __ballot_sync(0xffffffffu, lane < 31 && id != next_id);
-    const int last_id = __shfl_sync(0xffffffffu, id, 31);
-    const int end = last_id >= 0 ? run_end(p.ids, p.kv_len, last + 1, last_id, v) : 0;  // of the block that leaves the warp's rows
+    const int last_id = __shfl_sync(0xffffffffu, id, 31), last = __shfl_sync(0xffffffffu, self, 31);
+    const int end = last_id >= 0 ? run_end(p.ids, p.kv_len, last, last_id) : 0;  // of the block that leaves the warp's rows
     if (id < 0) return min(max(self + 1, 0), p.kv_len);
     const uint32_t ahead = breaks >> lane;
     return ahead ? self + __ffs(ahead) : end;
