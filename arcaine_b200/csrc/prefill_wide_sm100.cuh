@@ -305,14 +305,15 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         fence_mbar_init();
     }
     if (warp == C::PRODUCER_WARP) tmem_alloc_pair(tmem_slot, 512);
-    // One warp finds the first unit for all; its divisions, and the code that every role would fetch for them, took 2500 clk
-    // between the kernel's release and its first load.
+    // One warp finds the first unit for all, beside the tensor memory's allocation; its divisions, and the code that every role
+    // would fetch for them, took 2500 clk between the kernel's release and its first load.
     const int place = (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
     const bool blocks_in_memory = MASKED || p.ids;
     WideWork w_first{};
-    if (warp == C::PRODUCER_WARP) {
+    if (warp == C::EPILOGUE_WARP) {
         w_first = wide_place<SPLIT>(p, WideCursor(place, step), rank);
         if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
+        if (lane == 0) *first_unit = w_first;
     }
     cluster_sync_all();  // both CTAs' barriers exist before anyone arrives on the other's
     // Up to here nothing depends on the kernels in front; everything below may.
@@ -352,8 +353,11 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     static_assert(C::THREADS == 320, "barriers 3 and 4");
     tc_fence_before_sync();
     if (warp == C::PRODUCER_WARP) {
-        if (blocks_in_memory) wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
-        if (lane == 0) *first_unit = w_first;
+        w_first = *first_unit;
+        if (blocks_in_memory) {
+            wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
+            if (lane == 0) *first_unit = w_first;
+        }
         __syncwarp();
         asm volatile("bar.arrive 3, 320;" ::: "memory");
         ahead_k = min(w_first.hi - w_first.lo, 2), ahead_v = min(w_first.hi - w_first.lo, 1);
@@ -381,7 +385,6 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     // [32 columns][row], 128-byte swizzle; and from there, a row of 512 bytes an instruction, to the records.  (By TMA, in
     // boxes of 8 rows x 32 columns, the tile took 4000 clk.)
     constexpr int PART_CHUNK = 128 * 128;
-    float* const part_lse = SPLIT ? p.part_lse + (long long)(blockIdx.x / 2 % p.num_splits) * p.batch * p.seq * p.nq : nullptr;
     auto own_row0 = [&](int part) { return (part * 16 + p.num_splits - 1) / p.num_splits * 8; };  // rows a part's CTA folds
     auto store_part = [&](const WideWork& w, int quarter, float row_l, int col) {
         if (!mbar_wait_warp<2>(o_full, 0)) {
@@ -585,7 +588,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             const long long eoff = w.b * p.o_stride_b + t * p.o_stride_t + (long long)w.h * HD;
             if (w.hi == w.lo) {  // nothing visible for the pair: zero output
                 if (SPLIT) {
-                    if (store) part_lse[row] = -CUDART_INF_F;
+                    if (store) p.part_lse[(long long)w.part * p.batch * p.seq * p.nq + row] = -CUDART_INF_F;
                 } else if (store) {
                     for (int c = -1; c < p.n_copies; ++c) {
                         uint4* dst = reinterpret_cast<uint4*>((c < 0 ? p.out : reinterpret_cast<uint16_t*>(p.out_copies[c])) + eoff);
@@ -664,7 +667,10 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         WideCursor cur(place, step);
         for (; ok && cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
-            if (w.hi == w.lo) continue;
+            if (w.hi == w.lo) {
+                if (SPLIT) break;  // (its only one; with the place read again below, nothing is spilled: a canvas step 17.9 us, 17.6 so)
+                continue;
+            }
             const int t = w.q0 + r;
             int row_lo = 0, row_hi = p.kv_len;  // visible keys [row_lo, row_hi)
             if (causal) {
@@ -786,13 +792,15 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             }
             if (ok) {
                 fin_vals[(n & 3) * 128 + r] = l;
-                float* lse = SPLIT ? part_lse : p.out_lse;
-                if (lse && t < p.seq)
-                    lse[((long long)w.b * p.seq + t) * p.nq + w.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
+                // (SPLIT: the place in the output is read again, not kept in registers through the blocks)
+                const WideWork u = SPLIT ? *first_unit : w;
+                float* lse = SPLIT ? p.part_lse + (long long)u.part * p.batch * p.seq * p.nq : p.out_lse;
+                if (lse && u.q0 + r < p.seq)
+                    lse[((long long)u.b * p.seq + u.q0 + r) * p.nq + u.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
                 mbar_arrive_warp(&fin[n & 3]);
                 ++n;
                 if constexpr (SPLIT) {
-                    store_part(w, quarter, l, HD / 2);
+                    store_part(*first_unit, quarter, l, HD / 2);
                     break;
                 }
             }
