@@ -260,9 +260,8 @@ struct PrefillPlan {
     int q_tiles = 0;
     int splits = 1;
     long long rows = 0;
-    size_t split_bytes = 0;  // partial records of key-range splits, at the start of the workspace
-    size_t ws_bytes = 0;     // what must be there: partial records, then the per-row span ends of block_ids
-    size_t mask_bytes = 0;   // behind it, if it is there: the classes and bits of an additive mask
+    size_t ws_bytes = 0;    // what must be there: partial records of key-range splits
+    size_t mask_bytes = 0;  // behind it, if it is there: the classes and bits of an additive mask
 };
 
 // Key blocks that token tile qt (128 rows) of a call sees, block ids apart.
@@ -335,15 +334,10 @@ static int plan_prefill(const arc_sdpa_prefill_params* p, int sm_count, const Wi
     if (splits > kv_blocks) splits = kv_blocks;
     if (splits > 64) splits = 64;
     plan->splits = splits;
-    plan->split_bytes = splits > 1 ? (size_t)splits * plan->rows * ((size_t)p->hd + 1) * sizeof(float) : 0;
-    plan->split_bytes = (plan->split_bytes + 15) & ~(size_t)15;
-    plan->ws_bytes = plan->split_bytes;
+    plan->ws_bytes = splits > 1 ? (size_t)splits * plan->rows * ((size_t)p->hd + 1) * sizeof(float) : 0;
+    plan->ws_bytes = (plan->ws_bytes + 15) & ~(size_t)15;
     if (scanned_mask) plan->mask_bytes = (size_t)plan->q_tiles * kv_blocks * (128 * sizeof(uint4) + sizeof(uint32_t));
-    if (p->block_ids) {
-        if (p->mask_type != ARC_MASK_CAUSAL || p->block_ids_offset < 0) return ARC_ERR_BAD_SHAPE;
-        // (span ends were kept there once; the call still asks for the room it always did)
-        if (p->hd == 128) plan->ws_bytes += ((size_t)p->seq * sizeof(int32_t) + 15) & ~(size_t)15;
-    }
+    if (p->block_ids && (p->mask_type != ARC_MASK_CAUSAL || p->block_ids_offset < 0)) return ARC_ERR_BAD_SHAPE;
     return ARC_OK;
 }
 

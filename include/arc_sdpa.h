@@ -101,9 +101,8 @@ typedef struct arc_sdpa_prefill_params {
      * (seq, kv_len) f32 buffer).  block_ids: device int32 per absolute position, -1 = text token, a
      * non-negative id for each contiguous image / video block; a query inside a block also sees the
      * block's later keys.  block_ids[block_ids_offset + j] belongs to key j, so the array must reach
-     * block_ids_offset + kv_len entries; the same ids serve every sequence of the batch.  Head
-     * dim 128 asks for a workspace (arc_sdpa_prefill_workspace_bytes()): with a gate, output copies or a
-     * split key range the span end of every row goes there; other calls look the blocks up as they go. */
+     * block_ids_offset + kv_len entries; the same ids serve every sequence of the batch.  The
+     * kernels look the blocks up as they go; no workspace is needed for it. */
     const int32_t* block_ids;
     int32_t block_ids_offset;
     /* Copies of the output (optional; no counterpart in the reference, which is single-device).

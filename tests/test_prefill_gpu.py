@@ -399,6 +399,30 @@ def test_vision_blocks_two_tiles_per_cta(ops, nq, nkv):
         assert torch.allclose(lse, want_lse, atol=2e-3)
 
 
+def test_vision_blocks_need_no_workspace(ops):
+    """The kernels look the ends of vision blocks up themselves: an unsplit call of head dim 128 brings no workspace."""
+    from arcaine_b200 import _lib
+    seq, nq, nkv, hd = 200, 4, 2, 128
+    q, k, v = (seeded_bf16(seq, h, hd, seed=90 + i).cuda() for i, h in enumerate((nq, nkv, nkv)))
+    ids = torch.full((seq,), -1, dtype=torch.int32, device="cuda")
+    ids[30:170] = 3
+    want = ops.sdpa_prefill(q, k, v, scale=0.09, mask_type=ops.MASK_CAUSAL, window=100, block_ids=ids, num_splits=1)
+    out = torch.empty_like(q)
+    p = _lib.PrefillParams()
+    p.q, p.k, p.v, p.out, p.block_ids = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), ids.data_ptr()
+    p.batch, p.seq, p.kv_len, p.nq, p.nkv, p.hd = 1, seq, seq, nq, nkv, hd
+    for f, heads in (("q", nq), ("k", nkv), ("v", nkv), ("o", nq)):
+        setattr(p, f + "_stride_t", heads * hd)
+        setattr(p, f + "_stride_b", seq * heads * hd)
+    p.scale, p.mask_type, p.window, p.num_splits = 0.09, 3, 100, 1
+    L = _lib.load()
+    assert L.arc_sdpa_prefill_workspace_bytes(C.byref(p)) == 0
+    torch.cuda.synchronize()
+    assert L.arc_sdpa_prefill(C.byref(p), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("q_len,kv_len", [(4100, 1030), (4097, 1000), (2049, 2050)])  # from 4097 blocks of a row on, a block writes four
 @pytest.mark.parametrize("window", [300, oracle.INT_MAX])
 def test_mask_fill_of_many_rows(ops, q_len, kv_len, window):
