@@ -144,7 +144,7 @@ static int device_state(DeviceState** out) {
                 ARC_CUDA(opt_in_smem(pair_kernel(i & 1, i & 2, i & 4), PairCfg::SMEM_BYTES));
                 ARC_CUDA(opt_in_smem(chains_kernel(i & 1, i & 2, i & 4), ChainsCfg::SMEM_BYTES));
             }
-            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel<256, true, true>, PrefillCfg<256>::SMEM_BYTES));
+            ARC_CUDA(opt_in_smem(sdpa_prefill_kernel, PrefillCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, false>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<true, false>, WideCfg::SMEM_BYTES));
             ARC_CUDA(opt_in_smem(sdpa_prefill_wide_kernel<false, true>, WideCfg::SMEM_BYTES));
@@ -569,8 +569,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
     if (total_tiles > 0x7fffffffLL) return ARC_ERR_TOO_LARGE;
     kp.total_tiles = (int)total_tiles;
     const unsigned ctas = (unsigned)(total_tiles < ds->sm_count ? total_tiles : ds->sm_count);
-    set_step(&kp, ctas);
-    ARC_CUDA(launch_dependent(sdpa_prefill_kernel<256, true, true>, dim3(ctas), dim3(PrefillCfg<256>::THREADS), (size_t)PrefillCfg<256>::SMEM_BYTES, stream, 1, tq, tk, tv, kp));
+    ARC_CUDA(launch_dependent(sdpa_prefill_kernel, dim3(ctas), dim3(PrefillCfg::THREADS), (size_t)PrefillCfg::SMEM_BYTES, stream, 1, tq, tk, tv, kp));
     g_launches.fetch_add(1, std::memory_order_relaxed);
 
     return plan.splits > 1 ? launch_fold<HD>(p, plan, kp, stream) : ARC_OK;

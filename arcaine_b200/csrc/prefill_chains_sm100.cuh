@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(ChainsCfg::THREADS, 1)
                 if (windowed) row_lo = max(0, diag - p.window + 1);
                 if (row_lo > row_hi) row_lo = row_hi;
             }
-            const RowMask rm{row_lo, row_hi, p.kv_len, nullptr};
+            const RowMask rm{row_lo, row_hi};
 
             float m = -CUDART_INF_F;  // running max of the chain, log2 domain, possibly stale by <= 8
             float l = 0.f;            // its sum
@@ -443,15 +443,15 @@ __global__ void __launch_bounds__(ChainsCfg::THREADS, 1)
                 tmem_ld32(tS + 96, s3);
                 mask(s0, 0);
                 mask(s1, 1);
-                chunk_max<0>(s0, mr, bl, kc, rm);
-                chunk_max<0>(s1, mr, bl, kc, rm);
+                chunk_max(s0, mr);
+                chunk_max(s1, mr);
                 tmem_wait_ld();
                 tc_fence_before_sync();
                 mbar_arrive_warp(s_free);  // the buffer may take the other chain's scores
                 mask(s2, 2);
                 mask(s3, 3);
-                chunk_max<0>(s2, mr, bl, kc, rm);
-                chunk_max<0>(s3, mr, bl, kc, rm);
+                chunk_max(s2, mr);
+                chunk_max(s3, mr);
                 const float m_new = fmaxf(m, fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * bl);
                 // O += P V of the chain's block before has long completed, as a rule: its P may be replaced.
                 if (g > 0 && !mbar_wait_warp<3>(&pv_done[s], (g - 1) & 1)) {

@@ -742,7 +742,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 if (windowed) row_lo = max(0, diag - p.window + 1);
                 if (row_lo > row_hi) row_lo = row_hi;
             }
-            const RowMask rm{row_lo, row_hi, p.kv_len, nullptr};
+            const RowMask rm{row_lo, row_hi};
 
             float m = -CUDART_INF_F;  // running max, log2 domain, possibly stale by <= 8
             float l = 0.f;            // row sum
@@ -765,8 +765,8 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     mask_chunk(s0, kc, rm);
                     mask_chunk(s1, kc + 32, rm);
                 }
-                chunk_max<0>(s0, mr, sl, kc, rm);
-                chunk_max<0>(s1, mr, sl, kc, rm);
+                chunk_max(s0, mr);
+                chunk_max(s1, mr);
                 tmem_wait_ld();
                 tc_fence_before_sync();
                 mbar_arrive_warp(s_free);  // the buffer may take the other pipeline's scores
@@ -774,8 +774,8 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     mask_chunk(s2, kc + 64, rm);
                     mask_chunk(s3, kc + 96, rm);
                 }
-                chunk_max<0>(s2, mr, sl, kc, rm);
-                chunk_max<0>(s3, mr, sl, kc, rm);
+                chunk_max(s2, mr);
+                chunk_max(s3, mr);
                 const float m_new = fmaxf(m, fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sl);
                 // O += P V of the block before has long completed, as a rule: its P may be replaced.
                 if (g > 0 && !mbar_wait_warp<3>(&pv_done[s], (g - 1) & 1)) {

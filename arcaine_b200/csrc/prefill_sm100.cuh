@@ -1,9 +1,10 @@
-// GQA flash-attention prefill kernel for sm_100a, one query tile at a time per CTA: head dim 256 with an additive mask and
-// no workspace for what mask_scan_kernel would read out of it (prefill_wide_sm100.cuh does the rest of head dim 256,
-// prefill_pair_sm100.cuh and prefill_chains_sm100.cuh head dim 128); and what all prefill kernels share.
+// GQA flash-attention prefill kernel for sm_100a, one query tile at a time per CTA: head dim 256 with an additive mask, for
+// calls without a workspace for what mask_scan_kernel would read out of it and for parts of a key range that a caller
+// asks for (prefill_wide_sm100.cuh does the rest of head dim 256, prefill_pair_sm100.cuh and prefill_chains_sm100.cuh head
+// dim 128); and what all prefill kernels share.
 //
-// One CTA owns a tile of 128 query tokens of one query head and walks the key
-// blocks (128 keys) that tile can see.  Q, K and V tiles are staged in shared
+// One CTA owns a tile of 128 query tokens of one query head and walks all key
+// blocks (128 keys).  Q, K and V tiles are staged in shared
 // memory by TMA (128-byte swizzle, one 64-element column chunk per copy);
 // S = Q K^T and O += P V run on the tcgen05 tensor cores with both accumulators
 // in tensor memory; P is written back to tensor memory as bf16 over the S
@@ -14,16 +15,15 @@
 // (warp index mod 4 selects the 32 TMEM lanes, warp index / 4 the 64-key half of each
 // block), then one TMA producer warp (also the TMEM owner) and one MMA issuing warp.
 //
-// Masking follows the reference's rules evaluated inline instead of through a
+// Masking in the other kernels follows the reference's rules evaluated inline instead of through a
 // (q_len, kv_len) f32 buffer: causal aligned bottom-right with an optional
 // window of the W most recent keys, self included
 // (src/common/kernels/attention_mask.hpp:12-38); no mask for the bidirectional
-// canvas-over-prompt call (src/modeling/diffusion_gemma/attention.cpp:1093-1103);
-// an explicit additive buffer is still accepted.  Key blocks wholly outside a
+// canvas-over-prompt call (src/modeling/diffusion_gemma/attention.cpp:1093-1103).
+// Key blocks wholly outside a
 // tile's visible band are never loaded (the band idea of gqa_attention,
 // src/modeling/diffusion_gemma/attention.cpp:721-769, per CTA).
 #pragma once
-#include <type_traits>
 #include <cuda.h>
 #include <math_constants.h>
 
@@ -62,43 +62,12 @@ struct PrefillParams {
     const uint4* mask_bits;      // [row tile][key block][row]: one bit per key, set where the mask is 0
     int mask_blocks;
     int fold;        // prefill_wide_sm100.cuh: the parts of a unit are the pairs of one cluster, which folds them itself
-    const int* ids;  // vision-block ids, ids[j] that of key j 
+    const int* ids;  // vision-block ids, ids[j] that of key j
 };
 
-// One CTA per SM, persistent: it takes tiles (128 query tokens of one query head) round-robin
-// and keeps its pipelines running across tile boundaries — the next tile's Q, K and V stream in
-// and its first score blocks are computed while the softmax warps still write the previous
-// tile's output.  Two score buffers in tensor memory, then O, so S = Q K^T runs one key block ahead of
-// the softmax; eight softmax warps (two threads per query row, 64 keys each).
-// Eight rather than sixteen softmax warps on purpose: the
-// single MMA-issuing thread shares an instruction scheduler with them, and with four busy
-// warps per scheduler it could not issue MMAs fast enough to keep the tensor pipe fed.
-template <int HD>
-struct PrefillCfg {
-    static constexpr int BM = 128;  // query rows per tile
-    static constexpr int BN = 128;  // keys per block
-    static constexpr int CH = HD / 64;
-    static constexpr int CHUNK_BYTES = 128 * 128;  // 128 rows x 64 bf16
-    static constexpr int TILE_BYTES = CH * CHUNK_BYTES;
-    static constexpr int K_STAGES = 1;
-    static constexpr int V_STAGES = 1;
-    static constexpr int TMEM_COLS = 512;
-    static constexpr int NSB = 2;  // score buffers: S = Q K^T runs NSB-1 blocks ahead of the softmax
-    static constexpr int COL_S = 0;                  // NSB buffers of 128 fp32 columns; P (bf16) is written over them
-    static constexpr int COL_O = NSB * 128;          // HD fp32 columns
-    static constexpr int NUM_BARS = 2 + 2 * K_STAGES + 2 * V_STAGES + 2 * NSB + 2 + 2;
-    static constexpr int XCH_FLOATS = 2 * 2 * 128 + 2 * 128;  // row-max exchange (2 phases), row-sum exchange
-    static constexpr int SMEM_BYTES = (1 + K_STAGES + V_STAGES) * TILE_BYTES + NUM_BARS * 8 + 16 + XCH_FLOATS * 4 + 1024;
-    static constexpr int SOFTMAX_WARPS = 8;
-    static constexpr int THREADS = 32 * (SOFTMAX_WARPS + 2);
-    static constexpr int MAX_REGS = 168;  // ten warps put three on some scheduler: 3 x 32 x 168 fits its 16384 registers, 176 does not
-};
-
-// Per-row visibility for blocks that need element masking.
+// A row's visible keys [lo, hi).
 struct RowMask {
-    int lo, hi;            // visible keys [lo, hi)
-    int kv_len;
-    const float* mask_row;  // optional additive mask row (natural-log domain)
+    int lo, hi;
 };
 
 __device__ __forceinline__ float max3f(float a, float b, float c) {
@@ -107,150 +76,13 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
     return d;
 }
 
-// Element masking mode of a key block: 0 = every key visible, 1 = per-row span
-// [lo, hi), 2 = span plus an additive f32 mask row.
-// Scaled (log2-domain) and masked score of one key.
-template <int MODE>
-__device__ __forceinline__ float masked_score(uint32_t raw, float sl, int key, const RowMask& rm) {
-    float x = __uint_as_float(raw) * sl;
-    if (MODE == 2) {
-        if (rm.mask_row && key < rm.kv_len) x += rm.mask_row[key] * 1.4426950408889634f;
-    }
-    return (key >= rm.lo && key < rm.hi) ? x : -CUDART_INF_F;
-}
-
-// 32 bytes (16 bf16) to q: one 256-bit store where q is 32-byte aligned (a whole DRAM sector), else two
-// 128-bit stores.
-__device__ __forceinline__ void store_bf16x16(uint16_t* q, const uint32_t (&w)[8]) {
-    if ((reinterpret_cast<uintptr_t>(q) & 31u) == 0) {
-        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(q), "r"(w[0]), "r"(w[1]), "r"(w[2]),
-                     "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                     : "memory");
-    } else {
-        *reinterpret_cast<uint4*>(q) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(q + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-    }
-}
-
-// The same 32 bytes at element offset `off` of every copy of the output (plain stores; a copy in another
-// GPU's memory travels over NVLink while the kernel computes on).
-__device__ __forceinline__ void store_copies_bf16x16(const unsigned long long* copies, int n, long long off,
-                                                     const uint32_t (&w)[8]) {
-    for (int c = 0; c < n; ++c) store_bf16x16(reinterpret_cast<uint16_t*>(copies[c]) + off, w);
-}
-
 // Maximum of one 32-column chunk, folded into four independent running maxima.
-template <int MODE>
-__device__ __forceinline__ void chunk_max(const uint32_t (&v)[32], float (&mx)[4], float sl, int key0,
-                                          const RowMask& rm) {
+__device__ __forceinline__ void chunk_max(const uint32_t (&v)[32], float (&mx)[4]) {
 #pragma unroll
-    for (int e = 0; e < 32; e += 8) {
+    for (int e = 0; e < 32; e += 8)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            float a, b;
-            if (MODE != 0) {
-                a = masked_score<MODE>(v[e + 2 * u], sl, key0 + e + 2 * u, rm);
-                b = masked_score<MODE>(v[e + 2 * u + 1], sl, key0 + e + 2 * u + 1, rm);
-            } else {
-                a = __uint_as_float(v[e + 2 * u]);
-                b = __uint_as_float(v[e + 2 * u + 1]);
-            }
-            mx[u] = max3f(mx[u], a, b);
-        }
-    }
+        for (int u = 0; u < 4; ++u) mx[u] = max3f(mx[u], __uint_as_float(v[e + 2 * u]), __uint_as_float(v[e + 2 * u + 1]));
 }
-
-// exp2 of one chunk against the running max, packed to bf16x2; four independent partial sums.
-template <int MODE>
-__device__ __forceinline__ void chunk_exp(const uint32_t (&v)[32], uint32_t (&pk)[16], float (&ls)[4], float sl,
-                                          float m_eff, int key0, const RowMask& rm) {
-    if constexpr (MODE == 0) {
-        // Every key visible.  Plain fp32 instructions: the packed forms take the pipe no shorter, and where the loop fits
-        // the instruction cache without them, as here, they made the kernel slower; so did a polynomial 2^x on the FMA
-        // pipe for a share of the scores.  (The kernels with two tiles need the shorter code.)
-        const float nm = -m_eff;
-#pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-            const float p0 = fast_exp2(fmaf(__uint_as_float(v[e]), sl, nm));
-            const float p1 = fast_exp2(fmaf(__uint_as_float(v[e + 1]), sl, nm));
-            ls[e & 3] += p0;
-            ls[(e + 1) & 3] += p1;
-            pk[e >> 1] = pack_bf16x2(p0, p1);
-        }
-    } else if constexpr (MODE == 1) {
-        // Per-row span: one select per score (exp2(-inf) = 0).
-        const float nm = -m_eff;
-        const int lo_rel = rm.lo - key0, hi_rel = rm.hi - key0;  // visible: lo_rel <= e < hi_rel
-#pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-            const float x0 = fmaf(__uint_as_float(v[e]), sl, nm), x1 = fmaf(__uint_as_float(v[e + 1]), sl, nm);
-            const float p0 = fast_exp2((e >= lo_rel && e < hi_rel) ? x0 : -CUDART_INF_F);
-            const float p1 = fast_exp2((e + 1 >= lo_rel && e + 1 < hi_rel) ? x1 : -CUDART_INF_F);
-            ls[e & 3] += p0;
-            ls[(e + 1) & 3] += p1;
-            pk[e >> 1] = pack_bf16x2(p0, p1);
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-            const float p0 = fast_exp2(masked_score<MODE>(v[e], sl, key0 + e, rm) - m_eff);
-            const float p1 = fast_exp2(masked_score<MODE>(v[e + 1], sl, key0 + e + 1, rm) - m_eff);
-            ls[(e >> 1) & 3] += p0 + p1;
-            pk[e >> 1] = pack_bf16x2(p0, p1);
-        }
-    }
-}
-
-// How a 32-key chunk relates to the rows of this warp (warp-uniform, so the
-// warp-collective TMEM instructions stay converged): 0 = every key visible to all
-// 32 rows (no element test needed), 1 = mixed, 2 = no key visible to any row.
-// With a causal diagonal crossing a 128 x 128 block, each warp meets at most one
-// or two mixed chunks; the rest is either plain or skipped.
-__device__ __forceinline__ int chunk_class(int kc, const RowMask& rm) {
-    const bool all = rm.lo <= kc && kc + 32 <= rm.hi;
-    const bool none = rm.hi <= kc || rm.lo >= kc + 32;
-    if (__all_sync(0xffffffffu, all)) return 0;
-    if (__all_sync(0xffffffffu, none)) return 2;
-    return 1;
-}
-
-template <bool ADD_MASK>
-__device__ __forceinline__ void chunk_max_any(const uint32_t (&v)[32], float (&mx_raw)[4], float (&mx_scaled)[4],
-                                              float sl, int kc, const RowMask& rm) {
-    const int cls = ADD_MASK ? 1 : chunk_class(kc, rm);
-    if (cls == 0) chunk_max<0>(v, mx_raw, sl, kc, rm);
-    else if (cls == 1) chunk_max<ADD_MASK ? 2 : 1>(v, mx_scaled, sl, kc, rm);
-}
-
-template <bool ADD_MASK>
-__device__ __forceinline__ void chunk_exp_any(const uint32_t (&v)[32], uint32_t (&pk)[16], float (&ls)[4], float sl,
-                                              float m_eff, int kc, const RowMask& rm) {
-    const int cls = ADD_MASK ? 1 : chunk_class(kc, rm);
-    if (cls == 0) {
-        chunk_exp<0>(v, pk, ls, sl, m_eff, kc, rm);
-    } else if (cls == 1) {
-        chunk_exp<ADD_MASK ? 2 : 1>(v, pk, ls, sl, m_eff, kc, rm);
-    } else {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) pk[e] = 0u;
-    }
-}
-
-
-
-// Barrier between the two warps that share a set of 32 query rows (warps q and q + 4):
-// hardware barrier 1 + q, 64 threads.  Every softmax warp executes the same number of
-// pair_syncs per tile, whatever happened to its waits, so neither warp of a pair can be left
-// waiting here.
-__device__ __forceinline__ void pair_sync(int quarter) {
-    asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
-}
-
-// One unit of work of the persistent kernel.
-struct TileWork {
-    int q0, h, b, split, kvh;
-    int my_lo, n_my;  // key blocks [my_lo, my_lo + n_my) of this tile and split
-};
 
 // Position of a persistent CTA in the launch's tile list.  Plain order: tile w = ((z * cur_heads) + h) * q_tiles + qt,
 // token tiles fastest (neighbouring CTAs share K/V blocks in L2), then query heads, then z = batch * num_splits + split.
@@ -314,46 +146,116 @@ struct TileCursor {
     }
 };
 
-// The split is part of the tile index (z = batch * num_splits + split).
-template <int HD>
-__device__ __forceinline__ TileWork decode_tile(const PrefillParams& p, const TileCursor& cur) {
-    using C = PrefillCfg<HD>;
+// One CTA per SM, persistent: it takes tiles (128 query tokens of one query head) round-robin
+// and keeps its pipelines running across tile boundaries — the next tile's Q, K and V stream in
+// and its first score blocks are computed while the softmax warps still write the previous
+// tile's output.  Two score buffers in tensor memory, then O, so S = Q K^T runs one key block ahead of
+// the softmax; eight softmax warps (two threads per query row, 64 keys each).
+// Eight rather than sixteen softmax warps on purpose: the
+// single MMA-issuing thread shares an instruction scheduler with them, and with four busy
+// warps per scheduler it could not issue MMAs fast enough to keep the tensor pipe fed.
+struct PrefillCfg {
+    static constexpr int HD = 256;
+    static constexpr int BM = 128;  // query rows per tile
+    static constexpr int BN = 128;  // keys per block
+    static constexpr int CH = HD / 64;
+    static constexpr int CHUNK_BYTES = 128 * 128;  // 128 rows x 64 bf16
+    static constexpr int TILE_BYTES = CH * CHUNK_BYTES;
+    static constexpr int K_STAGES = 1;
+    static constexpr int V_STAGES = 1;
+    static constexpr int TMEM_COLS = 512;
+    static constexpr int NSB = 2;  // score buffers: S = Q K^T runs NSB-1 blocks ahead of the softmax
+    static constexpr int COL_S = 0;                  // NSB buffers of 128 fp32 columns; P (bf16) is written over them
+    static constexpr int COL_O = NSB * 128;          // HD fp32 columns
+    static constexpr int NUM_BARS = 2 + 2 * K_STAGES + 2 * V_STAGES + 2 * NSB + 2 + 2;
+    static constexpr int XCH_FLOATS = 2 * 2 * 128 + 2 * 128;  // row-max exchange (2 phases), row-sum exchange
+    static constexpr int SMEM_BYTES = (1 + K_STAGES + V_STAGES) * TILE_BYTES + NUM_BARS * 8 + 16 + XCH_FLOATS * 4 + 1024;
+    static constexpr int SOFTMAX_WARPS = 8;
+    static constexpr int THREADS = 32 * (SOFTMAX_WARPS + 2);
+    static constexpr int MAX_REGS = 168;  // ten warps put three on some scheduler: 3 x 32 x 168 fits its 16384 registers, 176 does not
+};
+
+// One unit of work: a tile, or a part of its key range, in the order tile w = ((z * nq) + h) * q_tiles + qt, z = batch *
+// num_splits + split.
+struct TileWork {
+    int q0, h, b, split, kvh;
+    int my_lo, n_my;  // key blocks [my_lo, my_lo + n_my)
+};
+
+__device__ __forceinline__ TileWork tile_at(const PrefillParams& p, int w) {
     TileWork t;
-    t.h = cur.h;
-    if (p.num_splits == 1) {
-        t.b = cur.z;
-        t.split = 0;
-    } else {
-        t.b = cur.z / p.num_splits;
-        t.split = cur.z % p.num_splits;
-    }
+    const int rest = w / p.q_tiles, z = rest / p.nq;
+    t.q0 = (w - rest * p.q_tiles) * PrefillCfg::BM;
+    t.h = rest - z * p.nq;
+    t.b = z / p.num_splits;
+    t.split = z - t.b * p.num_splits;
     t.kvh = p.group_shift >= 0 ? (t.h >> p.group_shift) : t.h / p.group;
-    t.q0 = cur.qt * C::BM;
-    const int off = p.kv_len - p.seq;
-    const bool causal = (p.mask_type == 3);
-    const bool windowed = causal && p.window > 0 && p.window != 0x7fffffff;
-    const int q_last = min(t.q0 + C::BM - 1, p.seq - 1);
-    int blk_lo = 0, blk_hi = (p.kv_len + C::BN - 1) / C::BN;
-    if (causal) {
-        // the span ends are monotone in the row, so the tile's last row decides
-        const int last_key = min(p.kv_len - 1, q_last + off);
-        blk_hi = last_key >= 0 ? last_key / C::BN + 1 : 0;
-        if (windowed) blk_lo = max(0, t.q0 + off - p.window + 1) / C::BN;
-    }
-    const int nblk = max(0, blk_hi - blk_lo);
-    const int per = p.num_splits == 1 ? nblk : (nblk + p.num_splits - 1) / p.num_splits;
-    t.my_lo = blk_lo + t.split * per;
-    t.n_my = max(0, min(blk_hi, t.my_lo + per) - t.my_lo);
+    const int blocks = (p.kv_len + PrefillCfg::BN - 1) / PrefillCfg::BN, per = (blocks + p.num_splits - 1) / p.num_splits;
+    t.my_lo = t.split * per;
+    t.n_my = max(0, min(blocks, t.my_lo + per) - t.my_lo);
     return t;
 }
 
-// ADD_MASK and GATE select code that most calls do not need (an additive mask row per query, the
-// sigmoid-gated epilogue); the common instance carries neither and stays small.
-template <int HD, bool ADD_MASK, bool GATE>
-__global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
+// Score of one key in the log2 domain, with the mask's value for it (natural-log domain).
+__device__ __forceinline__ float masked_score(uint32_t raw, float sl, const float* mask_row, int key, int kv_len) {
+    return key < kv_len ? __uint_as_float(raw) * sl + mask_row[key] * 1.4426950408889634f : -CUDART_INF_F;
+}
+
+// Maximum of 32 keys from key0 on, in four independent ones.
+__device__ __forceinline__ void masked_max(const uint32_t (&v)[32], float (&mx)[4], float sl, const float* mask_row, int key0, int kv_len) {
+#pragma unroll
+    for (int e = 0; e < 32; e += 8)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            mx[u] = max3f(mx[u], masked_score(v[e + 2 * u], sl, mask_row, key0 + e + 2 * u, kv_len),
+                          masked_score(v[e + 2 * u + 1], sl, mask_row, key0 + e + 2 * u + 1, kv_len));
+}
+
+// exp2 of 32 keys against the running maximum, packed to bf16x2; four independent partial sums.
+__device__ __forceinline__ void masked_exp(const uint32_t (&v)[32], uint32_t (&pk)[16], float (&ls)[4], float sl, float m_eff,
+                                           const float* mask_row, int key0, int kv_len) {
+#pragma unroll
+    for (int e = 0; e < 32; e += 2) {
+        const float p0 = fast_exp2(masked_score(v[e], sl, mask_row, key0 + e, kv_len) - m_eff);
+        const float p1 = fast_exp2(masked_score(v[e + 1], sl, mask_row, key0 + e + 1, kv_len) - m_eff);
+        ls[(e >> 1) & 3] += p0 + p1;
+        pk[e >> 1] = pack_bf16x2(p0, p1);
+    }
+}
+
+// Barrier between the two warps that share a set of 32 query rows (warps q and q + 4):
+// hardware barrier 1 + q, 64 threads.  Every softmax warp executes the same number of
+// pair_syncs per tile, whatever happened to its waits, so neither warp of a pair can be left
+// waiting here.
+__device__ __forceinline__ void pair_sync(int quarter) {
+    asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
+}
+
+// 32 bytes (16 bf16) to q: one 256-bit store where q is 32-byte aligned (a whole DRAM sector), else two
+// 128-bit stores.
+__device__ __forceinline__ void store_bf16x16(uint16_t* q, const uint32_t (&w)[8]) {
+    if ((reinterpret_cast<uintptr_t>(q) & 31u) == 0) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(q), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                     "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
+    } else {
+        *reinterpret_cast<uint4*>(q) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(q + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+// The same 32 bytes at element offset `off` of every copy of the output (plain stores; a copy in another
+// GPU's memory travels over NVLink while the kernel computes on).
+__device__ __forceinline__ void store_copies_bf16x16(const unsigned long long* copies, int n, long long off,
+                                                     const uint32_t (&w)[8]) {
+    for (int c = 0; c < n; ++c) store_bf16x16(reinterpret_cast<uint16_t*>(copies[c]) + off, w);
+}
+
+__global__ void __maxnreg__(PrefillCfg::MAX_REGS)
     sdpa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                         const __grid_constant__ CUtensorMap tm_v, const PrefillParams p) {
-    using C = PrefillCfg<HD>;
+    using C = PrefillCfg;
+    constexpr int HD = C::HD;
     constexpr int KS = C::K_STAGES;
     constexpr int VS = C::V_STAGES;
     constexpr int NSB = C::NSB;
@@ -380,15 +282,11 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
     float* xch_max = reinterpret_cast<float*>(tmem_slot + 4);  // [phase 2][key half 2][row 128]
     float* xch_sum = xch_max + 2 * 2 * 128;                    // [key half 2][row 128]
 
-
     // (broadcast, so that the compiler knows them to be the same in every lane and keeps what follows from them —
     // MMA descriptors above all — in uniform registers)
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     const long long rows_total = (long long)p.batch * p.seq * p.nq;
-    const bool causal = (p.mask_type == 3);
-    const bool windowed = causal && p.window > 0 && p.window != 0x7fffffff;
-    const int off = p.kv_len - p.seq;
 
     constexpr int PRODUCER_WARP = C::SOFTMAX_WARPS;
     constexpr int MMA_WARP = C::SOFTMAX_WARPS + 1;
@@ -424,8 +322,7 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         tmem_relinquish();
     }
     // (the divisions, ahead of the wait: they took 1000 clk between the kernel's release and its first load)
-    TileCursor cursor;
-    cursor.init(p);
+    const TileWork first = tile_at(p, blockIdx.x);
     // Up to here nothing depends on the kernels in front; everything below may.
     grid_dependency_wait();
     grid_launch_dependents();
@@ -443,9 +340,8 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         if (lane == 0) {
             int gk = 0, gv = 0, tc = 0;  // K blocks, V blocks and non-empty tiles loaded so far
             bool ok = true;
-            TileCursor cur = cursor;
-            for (; ok && cur.w < total_tiles; cur.advance(p)) {
-                const TileWork tw = decode_tile<HD>(p, cur);
+            for (int w = blockIdx.x; ok && w < total_tiles; w += gridDim.x) {
+                const TileWork tw = w == (int)blockIdx.x ? first : tile_at(p, w);
                 if (tw.n_my == 0) continue;
                 if (tc > 0 && !mbar_wait(q_empty, (tc - 1) & 1)) {
                     report_fault(p.fault, FAULT_WAIT_EMPTY, 0x300u);
@@ -526,9 +422,8 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
                 return true;
             };
             bool ok = true;
-            TileCursor cur = cursor;
-            for (; ok && cur.w < total_tiles; cur.advance(p)) {
-                const TileWork tw = decode_tile<HD>(p, cur);
+            for (int w = blockIdx.x; ok && w < total_tiles; w += gridDim.x) {
+                const TileWork tw = w == (int)blockIdx.x ? first : tile_at(p, w);
                 if (tw.n_my == 0) continue;
                 if (!mbar_wait_inline(q_full, tc & 1)) {
                     report_fault(p.fault, FAULT_WAIT_Q, tc);
@@ -589,116 +484,93 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
         const uint32_t tS0 = tmem_base + lane_sel + C::COL_S + kh * 64;
         const uint32_t tO = tmem_base + lane_sel + C::COL_O + kh * OC;
         const float sl = p.scale_log2;
-        constexpr bool has_mask = ADD_MASK;  // the additive-mask form is a kernel of its own: the common one stays small
 
         int gb = 0, tc = 0;  // key blocks and non-empty tiles processed so far
         bool ok = true;
         uint32_t va[32], vb[32];  // this thread's 64 scores of the current block
 
-        TileCursor cur = cursor;
-        for (; cur.w < total_tiles; cur.advance(p)) {
-            const TileWork tw = decode_tile<HD>(p, cur);
+        for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
+            const TileWork tw = w == (int)blockIdx.x ? first : tile_at(p, w);
             const int t = tw.q0 + r;
             const long long row = ((long long)tw.b * p.seq + t) * p.nq + tw.h;
             if (tw.n_my == 0) {
-                // Nothing visible: zero output (or an empty partial) for this tile.
+                // Fewer key blocks than parts: an empty record.
                 if (t < p.seq) {
-                    if (p.num_splits > 1) {
-                        float4* dst = reinterpret_cast<float4*>(p.part_o + ((long long)tw.split * rows_total + row) * HD + kh * OC);
-                        for (int i = 0; i < OC / 4; ++i) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (kh == 0) p.part_lse[(long long)tw.split * rows_total + row] = -CUDART_INF_F;
-                    } else {
-                        const long long zoff = tw.b * p.o_stride_b + t * p.o_stride_t + (long long)tw.h * HD + kh * OC;
-                        for (int c = -1; c < p.n_copies; ++c) {
-                            uint4* dst = reinterpret_cast<uint4*>((c < 0 ? p.out : reinterpret_cast<uint16_t*>(p.out_copies[c])) + zoff);
-                            for (int i = 0; i < OC / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
-                        }
-                        if (kh == 0 && p.out_lse) p.out_lse[row] = -CUDART_INF_F;
-                    }
+                    float4* dst = reinterpret_cast<float4*>(p.part_o + ((long long)tw.split * rows_total + row) * HD + kh * OC);
+                    for (int i = 0; i < OC / 4; ++i) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (kh == 0) p.part_lse[(long long)tw.split * rows_total + row] = -CUDART_INF_F;
                 }
                 continue;
             }
 
-            int row_lo = 0, row_hi = p.kv_len;  // visible keys [row_lo, row_hi)
-            if (causal) {
-                const int diag = t + off;
-                row_hi = min(max(diag + 1, 0), p.kv_len);
-                if (windowed) row_lo = max(0, diag - p.window + 1);
-                if (row_lo > row_hi) row_lo = row_hi;
-            }
-            const float* mask_row = has_mask && t < p.seq ? p.mask + (long long)t * p.kv_len : nullptr;
-            const RowMask rm{row_lo, row_hi, p.kv_len, mask_row};
+            const float* mask_row = p.mask + (long long)min(t, p.seq - 1) * p.kv_len;
 
             float m = -CUDART_INF_F;  // running max, log2 domain, possibly stale by <= 8
             float l = 0.f;            // this thread's share of the row sum
 
-            {
-                // Two score buffers leave no room to look ahead: S(i+1) can only be computed once P(i-1) has
-                // been consumed, so waiting for it before the exponentials of block i would put the tensor
-                // pipe and the softmax in series.  Here every block is taken on its own: maximum, exchange,
-                // exponentials; meanwhile the tensor pipe runs O += P(i-1) V(i-1) and S(i+1).
-                for (int i = 0; i < tw.n_my; ++i) {
-                    const int g = gb + i;
-                    const int kc = (tw.my_lo + i) * C::BN + kh * 64;
-                    const uint32_t tS = tS0 + (g % NSB) * 128;
-                    if (ok && !mbar_wait_warp(&s_full[g % NSB], (g / NSB) & 1)) {
-                        report_fault(p.fault, FAULT_WAIT_S, g);
-                        ok = false;
-                    }
-                    if (ok) {
-                        tc_fence_after_sync();
-                        tmem_ld32(tS, va);
-                        tmem_ld32(tS + 32, vb);
-                        tmem_wait_ld();
-                        float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                        float ms[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                        chunk_max_any<has_mask>(va, mr, ms, sl, kc, rm);
-                        chunk_max_any<has_mask>(vb, mr, ms, sl, kc + 32, rm);
-                        xch_max[(g & 1) * 256 + kh * 128 + r] = fmaxf(fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sl,
-                                                                     fmaxf(fmaxf(ms[0], ms[1]), fmaxf(ms[2], ms[3])));
-                    }
-                    pair_sync(quarter);
-                    if (!ok) continue;
-                    const float* xm = xch_max + (g & 1) * 256;
-                    const float m_new = fmaxf(m, fmaxf(xm[r], xm[128 + r]));
-                    if (i == 0) {
-                        m = m_new;  // nothing accumulated yet
-                    } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
-                        // Rare: the row maximum grows by more than 2^8.  Once O += P V of the previous block has
-                        // landed, rescale this thread's half of O in tensor memory (the row's other thread takes
-                        // the same decision from the same values).
-                        const float alpha = (m_new == -CUDART_INF_F) ? 1.0f : fast_exp2(m - m_new);
-                        if (!mbar_wait_warp(&pv_done[(g - 1) & 1], ((g - 1) >> 1) & 1)) {
-                            report_fault(p.fault, FAULT_WAIT_O, g);
-                            ok = false;
-                            continue;
-                        }
-                        tc_fence_after_sync();
-                        uint32_t ww[32];
-#pragma unroll 1
-                        for (int c = 0; c < OC / 32; ++c) {
-                            tmem_ld32(tO + c * 32, ww);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int e = 0; e < 32; ++e) ww[e] = __float_as_uint(__uint_as_float(ww[e]) * alpha);
-                            tmem_st32(tO + c * 32, ww);
-                        }
-                        tmem_wait_st();
-                        l *= alpha;
-                        m = m_new;
-                    }
-                    const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
-                    float ls4[4] = {0.f, 0.f, 0.f, 0.f};
-                    uint32_t pk[16];
-                    chunk_exp_any<has_mask>(va, pk, ls4, sl, m_eff, kc, rm);
-                    tmem_st16(tS, pk);
-                    chunk_exp_any<has_mask>(vb, pk, ls4, sl, m_eff, kc + 32, rm);
-                    tmem_st16(tS + 32, pk);
-                    l += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
-                    tmem_wait_st();
-                    tc_fence_before_sync();
-                    mbar_arrive(&p_full[g % NSB]);
+            // Two score buffers leave no room to look ahead: S(i+1) can only be computed once P(i-1) has
+            // been consumed, so waiting for it before the exponentials of block i would put the tensor
+            // pipe and the softmax in series.  Here every block is taken on its own: maximum, exchange,
+            // exponentials; meanwhile the tensor pipe runs O += P(i-1) V(i-1) and S(i+1).
+            for (int i = 0; i < tw.n_my; ++i) {
+                const int g = gb + i;
+                const int kc = (tw.my_lo + i) * C::BN + kh * 64;
+                const uint32_t tS = tS0 + (g % NSB) * 128;
+                if (ok && !mbar_wait_warp(&s_full[g % NSB], (g / NSB) & 1)) {
+                    report_fault(p.fault, FAULT_WAIT_S, g);
+                    ok = false;
                 }
+                if (ok) {
+                    tc_fence_after_sync();
+                    tmem_ld32(tS, va);
+                    tmem_ld32(tS + 32, vb);
+                    tmem_wait_ld();
+                    float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+                    masked_max(va, mr, sl, mask_row, kc, p.kv_len);
+                    masked_max(vb, mr, sl, mask_row, kc + 32, p.kv_len);
+                    xch_max[(g & 1) * 256 + kh * 128 + r] = fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3]));
+                }
+                pair_sync(quarter);
+                if (!ok) continue;
+                const float* xm = xch_max + (g & 1) * 256;
+                const float m_new = fmaxf(m, fmaxf(xm[r], xm[128 + r]));
+                if (i == 0) {
+                    m = m_new;  // nothing accumulated yet
+                } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
+                    // Rare: the row maximum grows by more than 2^8.  Once O += P V of the previous block has
+                    // landed, rescale this thread's half of O in tensor memory (the row's other thread takes
+                    // the same decision from the same values).
+                    const float alpha = (m_new == -CUDART_INF_F) ? 1.0f : fast_exp2(m - m_new);
+                    if (!mbar_wait_warp(&pv_done[(g - 1) & 1], ((g - 1) >> 1) & 1)) {
+                        report_fault(p.fault, FAULT_WAIT_O, g);
+                        ok = false;
+                        continue;
+                    }
+                    tc_fence_after_sync();
+                    uint32_t ww[32];
+#pragma unroll 1
+                    for (int c = 0; c < OC / 32; ++c) {
+                        tmem_ld32(tO + c * 32, ww);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) ww[e] = __float_as_uint(__uint_as_float(ww[e]) * alpha);
+                        tmem_st32(tO + c * 32, ww);
+                    }
+                    tmem_wait_st();
+                    l *= alpha;
+                    m = m_new;
+                }
+                const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
+                float ls4[4] = {0.f, 0.f, 0.f, 0.f};
+                uint32_t pk[16];
+                masked_exp(va, pk, ls4, sl, m_eff, mask_row, kc, p.kv_len);
+                tmem_st16(tS, pk);
+                masked_exp(vb, pk, ls4, sl, m_eff, mask_row, kc + 32, p.kv_len);
+                tmem_st16(tS + 32, pk);
+                l += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
+                tmem_wait_st();
+                tc_fence_before_sync();
+                mbar_arrive(&p_full[g % NSB]);
             }
             gb += tw.n_my;
             // Row sum = the two threads' shares.
@@ -736,8 +608,8 @@ __global__ void __maxnreg__(PrefillCfg<HD>::MAX_REGS)
             } else {
                 const long long eoff = tw.b * p.o_stride_b + t * p.o_stride_t + (long long)tw.h * HD + kh * OC;
                 uint16_t* dst = p.out + eoff;
-                const uint16_t* gp = (GATE && p.gate) ? p.gate + eoff : nullptr;
-                // One thread writes 128 (or 256) contiguous bytes of its row.
+                const uint16_t* gp = p.gate ? p.gate + eoff : nullptr;
+                // One thread writes 256 contiguous bytes of its row.
 #pragma unroll 1
                 for (int c = 0; c < OC / 32; ++c) {
                     tmem_ld32(tO + c * 32, va);

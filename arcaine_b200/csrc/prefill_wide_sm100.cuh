@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 if (windowed) row_lo = max(0, diag - p.window + 1);
                 if (row_lo > row_hi) row_lo = row_hi;
             }
-            const RowMask rm{row_lo, row_hi, p.kv_len, nullptr};
+            const RowMask rm{row_lo, row_hi};
             float m = -CUDART_INF_F;  // running max, log2 domain, possibly stale by <= 8
             float l = 0.f;            // row sum
             // (MASKED: a block's class is asked for a block ahead, its bits before its scores are waited for)
@@ -728,10 +728,10 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                     mask_chunk(s3, kc + 96, rm);
                 }
                 float mr[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-                chunk_max<0>(s0, mr, bl, kc, rm);
-                chunk_max<0>(s1, mr, bl, kc, rm);
-                chunk_max<0>(s2, mr, bl, kc, rm);
-                chunk_max<0>(s3, mr, bl, kc, rm);
+                chunk_max(s0, mr);
+                chunk_max(s1, mr);
+                chunk_max(s2, mr);
+                chunk_max(s3, mr);
                 const float top = fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3]));
                 const float m_new = fmaxf(m, top * bl);
                 if (j == w.lo) {
