@@ -3,7 +3,7 @@
 The library picks this kernel by a cost model (large problems); ARC_SDPA_PREFILL_KERNEL=pair, read once per
 process, forces it for every head-dim-128 call, so the small cases here run in a child process with that
 variable set: two token tiles of one head (odd GQA group), two heads of one KV group over the same tokens (even
-group), masks, windows, gate and ragged ends.
+group), masks, windows, vision blocks, gate, output copies and ragged ends.
 """
 import os
 import subprocess
@@ -82,6 +82,45 @@ copies = torch.tensor([b.data_ptr() for b in bufs], dtype=torch.int64, device='c
 got = ops.sdpa_prefill(q1, k1, v1, scale=128 ** -0.5, mask_type=3, window=1024, out_copies=copies)
 torch.cuda.synchronize()
 assert torch.equal(got, ref) and all(torch.equal(b, ref) for b in bufs), "output copies"
+# Vision blocks (ids by key): of one token, that start in the past, across tiles, up to the last key; ragged, with a window and
+# without; every instance: plain, gated, copied, both.  Pairs of heads (even groups), pairs of token tiles (odd ones)
+import numpy as np
+for nq, nkv in ((4, 2), (8, 2), (6, 2), (3, 3)):
+    seq, kv, n = 700, 790, 128
+    ids = np.full(kv, -1, dtype=np.int32)
+    for i, (a, b) in enumerate([(10, 11), (60, 130), (131, 190), (200, 470), (600, 610), (740, 790)]):
+        ids[a:b] = i
+    q, k, v, g = (seeded_bf16(r, h, n, seed=1400 + h + j) for j, (r, h) in enumerate(((seq, nq), (kv, nkv), (kv, nkv), (seq, nq))))
+    for w in (oracle.INT_MAX, 150):
+        mask = oracle.fill_causal_mask_with_block_ids(ids, seq, kv, kv - seq, w)
+        want = oracle.sdpa_f32(q, k, v, scale=0.09, mask_type=1, mask=mask, want_lse=True)
+        want_gated = oracle.sdpa_f32(q, k, v, scale=0.09, mask_type=1, mask=mask, gate=g)[1].float()
+        for gate in (False, True):
+            for copied in (False, True):
+                bufs = [torch.zeros(seq, nq, n, dtype=torch.bfloat16, device='cuda') for _ in range(2 * copied)]
+                before = ops.launch_count()
+                out, lse = ops.sdpa_prefill(q.cuda(), k.cuda(), v.cuda(), scale=0.09, mask_type=3, window=w, block_ids=torch.from_numpy(ids).cuda(),
+                                            num_splits=1, gate=g.cuda() if gate else None, return_lse=True,
+                                            out_copies=torch.tensor([b.data_ptr() for b in bufs], dtype=torch.int64, device='cuda') if copied else None)
+                assert ops.launch_count() - before == 1
+                what = f"vision {nq}/{nkv} window {w} gate {gate} copied {copied}"
+                assert_close(out, want_gated if gate else want[0], what)
+                assert torch.allclose(lse.cpu(), want[2], atol=2e-3), what
+                torch.cuda.synchronize()
+                assert all(torch.equal(b, out) for b in bufs), what
+# Units dealt longest first, two sequences: pairs of heads and pairs of token tiles, more than one wave, all rows of both; with
+# vision blocks as well
+for S, nq, nkv in ((1280, 32, 16), (700, 28, 4)):
+    g = torch.Generator().manual_seed(S)
+    q, k, v = (torch.randn(2, S, h, 128, generator=g).bfloat16() for h in (nq, nkv, nkv))
+    ids = np.full(S, -1, dtype=np.int32)
+    ids[100:300], ids[S - 60:] = 0, 1
+    for vision in (False, True):
+        out = ops.sdpa_prefill(q.cuda(), k.cuda(), v.cuda(), scale=0.09, mask_type=3, block_ids=torch.from_numpy(ids).cuda() if vision else None)
+        mask = oracle.fill_causal_mask_with_block_ids(ids, S, S, 0, oracle.INT_MAX) if vision else None
+        for b in range(2):
+            want = oracle.sdpa_f32(q[b], k[b], v[b], scale=0.09, mask_type=1 if vision else 3, mask=mask)[0]
+            assert_close(out[b], want, f"longest first {S} {nq}/{nkv} vision {vision} sequence {b}")
 assert ops.device_status() == (0, 0)
 assert ops.launch_count() > 0
 print("PAIR-OK")
