@@ -1,7 +1,7 @@
 """Head dim 128: one tile per CTA in two chains of key blocks, and tiles dealt longest first, where either can go wrong: one
 to five key blocks (a chain without any), parts of a key range without keys, scores that grow between the blocks of one
-chain only, additive masks with and without values, several tiles per CTA, a tail of single heads.  Against the CPU oracle
-with the tolerance of every attention test (tests/helpers.py)."""
+chain only, additive masks with and without values, several tiles per CTA.  (The tail of single heads behind a launch of
+pairs: test_prefill_gpu.py.)  Against the CPU oracle with the tolerance of every attention test (tests/helpers.py)."""
 import numpy as np
 import pytest
 import torch
@@ -72,8 +72,9 @@ def test_vision_blocks_gated_and_copied(ops, gate, copies):
 @pytest.mark.parametrize("batch,seq,kv_len,nq,nkv,window", [
     (1, 1300, 1300, 16, 8, oracle.INT_MAX),   # 176 tiles, two waves
     (2, 700, 900, 16, 2, oracle.INT_MAX),     # 192 tiles of two sequences
-    (1, 1900, 1900, 28, 4, oracle.INT_MAX),   # odd group: pairs of token tiles, two waves
-    (1, 1664, 3200, 32, 16, oracle.INT_MAX),  # 208 pairs: one wave and a tail of single heads
+    (1, 1900, 1900, 28, 4, oracle.INT_MAX),   # 420 tiles of an odd group, three waves
+    (2, 700, 700, 28, 4, oracle.INT_MAX),     # odd group: 168 pairs of token tiles, two waves
+    (1, 1664, 3200, 32, 16, oracle.INT_MAX),  # 416 tiles, three waves
     (1, 2100, 2100, 32, 16, 300),             # windowed, two waves of pairs
 ])
 def test_tiles_longest_first(ops, batch, seq, kv_len, nq, nkv, window):

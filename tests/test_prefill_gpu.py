@@ -139,25 +139,78 @@ def test_output_copies_are_written_by_every_epilogue(ops, case):
 
 
 @pytest.mark.parametrize("gate", [False, True])
-def test_two_tile_launch_with_a_single_head_tail(ops, gate):
-    """13 token tiles x 16 head pairs = 208 two-tile units on 148 SMs: one whole wave of pairs, and the 60 pairs
-    left over are cut into 120 single heads that a second launch (the one-tile kernel, one CTA per tile) takes
-    behind the first.  Every row must come out exactly once, from either launch."""
+def test_windowed_pairs_worth_of_tiles_in_one_launch(ops, gate):
+    """13 token tiles of 32 heads: 208 pairs of tiles on 148 SMs, but so few key blocks in each that one launch of single
+    tiles, dealt longest first, is judged faster than pairs with or without a tail."""
+    before = ops.launch_count()
     run_case(ops, 1664, 1664, 32, 16, 128, 128 ** -0.5, 3, 300, seed=800, gate=gate, lse=True)
+    assert ops.launch_count() - before == 1
 
 
-def test_consumer_right_behind_the_two_launch_form_sees_finished_rows(ops):
+# Calls that are cut by a clear margin (5 % and more) into whole waves of two-tile CTAs and a second launch for the pairs left
+# over, one CTA for each of their tiles: batch, queries, keys, heads, KV heads, causal, vision blocks.
+CUT = [
+    (3, 1590, 1700, 32, 16, False, False),  # 624 pairs in plain order: the last 32, heads 26 to 31 of the last sequence
+    (4, 1650, 4700, 24, 4, True, False),    # 624 longest first: the first token tile of all sequences but the first
+    (4, 1650, 4700, 24, 4, True, True),
+]
+
+
+def cut_call(B, seq, kv, nq, nkv, causal, vision, seed):
+    g = torch.Generator().manual_seed(seed)
+    q, k, v, gate = (torch.randn(B, n, h, 128, generator=g).bfloat16() for n, h in ((seq, nq), (kv, nkv), (kv, nkv), (seq, nq)))
+    ids = None
+    if vision:  # one that starts in the past, one across the first two tiles, one up to the last key
+        ids = torch.full((kv,), -1, dtype=torch.int32)
+        for i, (a, b) in enumerate([(kv - seq - 50, kv - seq + 30), (kv - seq + 100, kv - seq + 300), (kv - 90, kv)]):
+            ids[a:b] = i
+    return q, k, v, gate, ids
+
+
+@pytest.mark.parametrize("with_gate", [False, True])
+@pytest.mark.parametrize("B,seq,kv,nq,nkv,causal,vision", CUT)
+def test_two_tile_launch_with_a_single_head_tail(ops, B, seq, kv, nq, nkv, causal, vision, with_gate):
+    """Every row must come out exactly once, from either launch: all rows against the same call in parts of the key range
+    (single tiles and a merge), one in 61 — all heads, all tiles — against the oracle; with the log-sum-exp and an output copy."""
+    q, k, v, gate, ids = cut_call(B, seq, kv, nq, nkv, causal, vision, seed=820)
+    dev = [t.cuda() for t in (q, k, v)]
+    args = dict(scale=128 ** -0.5, mask_type=3 if causal else 0, gate=gate.cuda() if with_gate else None, block_ids=ids.cuda() if vision else None,
+                return_lse=True)
+    copy = torch.zeros(B, seq, nq, 128, dtype=torch.bfloat16, device="cuda")
+    before = ops.launch_count()
+    out, lse = ops.sdpa_prefill(*dev, out_copies=torch.tensor([copy.data_ptr()], dtype=torch.int64, device="cuda"), **args)
+    assert ops.launch_count() - before == 2
+    assert torch.equal(copy, out)
+    parts, parts_lse = ops.sdpa_prefill(*dev, num_splits=2, **args)
+    # (both within half a rounding of bf16 of their own result, as in the comparison of vision blocks below)
+    assert_close(out, parts.float(), "parts", rel_tol=4e-3, abs_tol=1.6e-2)
+    assert torch.allclose(lse, parts_lse, atol=2e-3)
+    mask = oracle.fill_causal_mask_with_block_ids(ids.numpy(), seq, kv, kv - seq, oracle.INT_MAX) if vision else None
+    rows = list(range(0, seq * nq, 61))
+    for b in range(B):
+        want = oracle.sdpa_f32(q[b], k[b], v[b], scale=128 ** -0.5, mask_type=1 if vision else args["mask_type"], mask=mask,
+                               gate=gate[b] if with_gate else None, rows=rows, want_lse=True)
+        assert_close(out[b].reshape(-1, 128)[rows], want[1].float() if with_gate else want[0], f"sequence {b}")
+        assert torch.allclose(lse[b].cpu().reshape(-1)[rows], want[2], atol=2e-3)
+
+
+@pytest.mark.parametrize("with_gate", [False, True])
+@pytest.mark.parametrize("B,seq,kv,nq,nkv,causal,vision", CUT)
+def test_consumer_right_behind_the_two_launch_form_sees_finished_rows(ops, B, seq, kv, nq, nkv, causal, vision, with_gate):
     """The single-head tail runs beside the two-tile launch in front of it; what follows in the stream waits for
     the tail launch only, so the tail must not complete first.  A copy enqueued right behind the call, with no
     host synchronisation in between, has to see every row."""
-    q, k, v = seeded_bf16(1664, 32, 128, seed=810).cuda(), seeded_bf16(1664, 16, 128, seed=811).cuda(), \
-        seeded_bf16(1664, 16, 128, seed=812).cuda()
-    ref = ops.sdpa_prefill(q, k, v, scale=128 ** -0.5, mask_type=ops.MASK_CAUSAL, window=300).clone()
+    q, k, v, gate, ids = cut_call(B, seq, kv, nq, nkv, causal, vision, seed=810)
+    q, k, v = (t.cuda() for t in (q, k, v))
+    args = dict(scale=128 ** -0.5, mask_type=3 if causal else 0, gate=gate.cuda() if with_gate else None, block_ids=ids.cuda() if vision else None)
+    ref = ops.sdpa_prefill(q, k, v, **args).clone()
     torch.cuda.synchronize()
     for _ in range(20):
         out = torch.zeros_like(ref)
-        ops.sdpa_prefill(q, k, v, scale=128 ** -0.5, mask_type=ops.MASK_CAUSAL, window=300, out=out)
+        before = ops.launch_count()
+        ops.sdpa_prefill(q, k, v, out=out, **args)
         snap = out.clone()
+        assert ops.launch_count() - before == 2
         torch.cuda.synchronize()
         assert torch.equal(snap, ref)
 
@@ -379,13 +432,17 @@ def test_few_keys_in_the_first_block_repeat_bit_for_bit(ops, window):
         assert torch.equal(first, run())
 
 
-@pytest.mark.parametrize("nq,nkv", [(8, 4), (6, 2)])  # two heads of one tile, two tiles of one head
-def test_vision_blocks_two_tiles_per_cta(ops, nq, nkv):
+@pytest.mark.parametrize("nq,nkv,seq", [
+    (8, 4, 1150), (6, 2, 1150),    # single tiles in two chains
+    (24, 4, 2700), (28, 4, 2450),  # two tiles a CTA, 9 % and more faster by the rule: two heads of one tile, two tiles of one head
+])
+def test_vision_blocks_two_tiles_per_cta(ops, nq, nkv, seq):
     """Block ids looked up in the kernel against the additive buffer of the same rule: blocks of one token, across tiles, up
-    to the last key; with a window that hides a block's first keys; the last tile ragged."""
-    seq, kv, hd = 1150, 1250, 128
+    to the last key; with a window that hides a block's first keys; the last tile ragged.  (That the two-tile kernel
+    runs is certain where it is forced: test_prefill_pair_gpu.py.)"""
+    kv, hd = seq + 100, 128
     ids = torch.full((kv,), -1, dtype=torch.int32)
-    for i, (a, b) in enumerate([(30, 31), (31, 100), (140, 160), (227, 260), (300, 711), (840, 1096), (1200, 1250)]):
+    for i, (a, b) in enumerate([(30, 31), (31, 100), (140, 160), (227, 260), (300, 711), (840, 1096), (kv - 50, kv)]):
         ids[a:b] = i
     q, k, v = (seeded_bf16(n, h, hd, seed=50 + h).cuda() for n, h in ((seq, nq), (kv, nkv), (kv, nkv)))
     for window in (oracle.INT_MAX, 200):
