@@ -98,7 +98,8 @@ struct PairWork {
 // ---------------------------------------------------------------------------
 // First key after `key` that does not carry `id`.  Whole warps, 128 keys a step.  (512 at once, asked for together with `id`, were
 // 5 KB of code in every kernel of head dim 256, which calls without ids jump over: from cold caches a canvas step took 22.1 us,
-// 21.4 so, and vision prompts were no faster for it — 3000 tokens of 16/8 heads of 128 31.2 us, 29.1 so.)
+// 21.4 so.  Prompts of head dim 128, which it did not burden: 3000 tokens of 16/8 heads 31.2 us with it, 29.0 so, cold 38.1 and
+// 34.5; one wave of tiles in chains up to 0.4 us faster with it, warm, and 0.5 to 2.5 slower cold.)
 __device__ __forceinline__ int run_end(const int* ids, int kv_len, int key, int id) {
     const int lane = threadIdx.x & 31;
     for (int k0 = key + 1;; k0 += 128) {
@@ -116,7 +117,7 @@ __device__ __forceinline__ int run_end(const int* ids, int kv_len, int key, int 
 // First key the row at key position `self` does not see.  Same position in every lane.
 __device__ __forceinline__ int vision_end(const PrefillParams& p, int self) {
     const int plain = min(max(self + 1, 0), p.kv_len);
-    if (self < 0 || self >= p.kv_len) return plain;
+    if (self < 0 || self + 1 >= p.kv_len) return plain;  // (behind the last key there is nothing to look up)
     const int id = p.ids[self];
     return id >= 0 ? run_end(p.ids, p.kv_len, self, id) : plain;
 }
