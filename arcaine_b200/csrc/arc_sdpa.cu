@@ -661,11 +661,22 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
     // four in three: taken where the longest sequence then needs fewer steps, a step of s slices counted as 2 + s.  (One token
     // of 24/4 heads over 513 keys, 65 a CTA: 6.74 us in two steps, 6.37 in one; 701: 6.82 and 6.38; 1501: 7.56 and 7.26; over
     // 1001 keys four slices fill two steps, six read half as much again for nothing: 6.84 and 7.08.)
+    // That is with five or six query heads a KV head, which six warps fold in one turn and four in two, or more than eight.  With
+    // others the fold of six takes 0.6 us longer where a cluster folds (two tokens of 16/8 heads over 780 keys 6.0 us in fours, 6.8 in
+    // sixes, of 16/2 over 1500 8.2 and 8.7, four of 16/8 over 1500 12.4 and 12.9), 0.2 where a CTA is alone, and up to four heads
+    // do not make up for that but where a third of the steps goes (16 of 16/8 over 200 / 260 keys 10.3 / 11.3 and 10.7 / 10.9).
+    // Fewer than 100 single CTAs need the third stage over many steps (20 of 24/4 over 780 keys 17.8 and 19.0; 30 22.1 and 21.9).
     int slices = most_slices(p->hd, heads, 64);
     const int wide = most_slices(p->hd, heads, 96);
     if (p->hd == 256 && wide > slices) {
         const long long units = ((long long)std::min(longest, 1e9) + csize * 16 - 1) / (csize * 16);  // 16-key slices of a CTA
-        if ((units + wide - 1) / wide * (2 + wide) <= (units + slices - 1) / slices * (2 + slices)) slices = wide;
+        const long long steps = (units + slices - 1) / slices, wide_steps = (units + wide - 1) / wide;
+        const bool alone = csize == 1, few = alone && (long long)p->batch * (p->nkv / heads) < 100 && steps > 9;
+        if (G > 8 || G == 5 || G == 6 || (alone && G > 4)) {
+            if (wide_steps * (2 + wide) <= steps * (2 + slices) && (G > 8 || !few)) slices = wide;
+        } else if (alone && !few && 3 * wide_steps < 2 * steps) {
+            slices = wide;
+        }
     }
     DecodePlan one = *plan;
     // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where

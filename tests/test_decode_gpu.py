@@ -402,14 +402,20 @@ def test_lengths_known_to_the_host_and_merge_blocks(ops, B, nq, nkv, hd, length,
             assert torch.allclose(on_host[2][b].cpu(), wl[0], atol=2e-3)
 
 
-@pytest.mark.parametrize("nq,nkv", [(24, 4), (8, 8), (16, 1)])  # groups of six, one and sixteen heads
-@pytest.mark.parametrize("n", [513, 768, 769, 1501])  # one step of six slices, its last full one, two steps, a ragged second one
-def test_one_launch_form_in_steps_of_six_slices(ops, n, nq, nkv):
-    q, k, v, g = (seeded_bf16(*shape, seed=400 + i) for i, shape in enumerate([(1, nq, 256), (n + 30, nkv, 256), (n + 30, nkv, 256), (1, nq, 256)]))
+@pytest.mark.parametrize("B,nq,nkv,n", [
+    # groups of six and of sixteen heads, of one, which takes four slices; one step of six slices, its last full one, two steps, a
+    # ragged second one
+    *((1, nq, nkv, n) for nq, nkv in ((24, 4), (8, 8), (16, 1)) for n in (513, 768, 769, 1501)),
+    # a CTA alone a sequence and KV head: one step and three of six slices, groups of one, four and eight heads
+    (16, 8, 8, 65), (16, 8, 8, 270), (60, 8, 2, 288), (40, 16, 2, 257), (110, 8, 1, 96),
+])
+def test_one_launch_form_in_steps_of_six_slices(ops, B, nq, nkv, n):
+    q, k, v, g = (seeded_bf16(*shape, seed=400 + i) for i, shape in enumerate([(B, nq, 256), (B, n + 30, nkv, 256), (B, n + 30, nkv, 256), (B, nq, 256)]))
     before = ops.launch_count()
-    got = ops.sdpa_decode(q.cuda(), k.cuda()[None], v.cuda()[None], scale=0.0625, kv_len=n, gate=g.cuda())
+    got = ops.sdpa_decode(q.cuda(), k.cuda(), v.cuda(), scale=0.0625, kv_len=n, gate=g.cuda())
     assert ops.launch_count() - before == 1
-    assert_close(got[0], oracle_decode(q[0], k[:n], v[:n], 0.0625, gate=g[0])[1][0].float(), f"{n} keys")
+    for b in {0, B // 2, B - 1}:
+        assert_close(got[b], oracle_decode(q[b], k[b, :n], v[b, :n], 0.0625, gate=g[b])[1][0].float(), f"{n} keys, sequence {b}")
 
 
 def check_ragged_batch(ops, q, k, v, g, lens, rows=None):
