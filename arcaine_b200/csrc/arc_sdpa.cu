@@ -453,11 +453,13 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
                                                : (long long)((p->seq + 255) / 256) * p->nq * p->batch;
         const long long single_tiles = (long long)plan.q_tiles * p->nq * p->batch * plan.splits;
         const long long sms = ds->sm_count;
-        // The pairs left over after the last whole wave of CTAs are cut into their two heads when every SM then
+        // The pairs left over after the last whole wave of CTAs may be cut into their two heads when every SM then
         // gets at most one of them: a second launch (a tile per CTA, scheduled behind this
-        // one as SMs free up) takes them, and no SM runs a whole pair while the others idle.
+        // one as SMs free up) takes them, and no SM runs a whole pair while the others idle.  It pays for a few calls in a
+        // hundred, of three waves and more (4 x 1728 tokens of 32/16 heads, no mask, by the measure below: 97.9 cut, 101.5 whole, 105.0 in
+        // chains); in others chains cover the tiles more evenly.
         const long long full_waves = pair_tiles / sms, left = pair_tiles - full_waves * sms;
-        // Under a causal mask tiles differ in length and go longest first, as at head dim 256 below.
+        // Under a causal mask tiles differ in length and go longest first, as at head dim 256 below, with the same two limits.
         const bool windowed = p->window > 0 && p->window < p->kv_len;
         const auto by_length = [&](long long units) {
             return !split && p->mask_type == ARC_MASK_CAUSAL && units > sms && (!windowed || units < 8 * sms) &&
@@ -536,10 +538,12 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         const long long units = wide_units(p, plan.q_tiles) * plan.splits;
         if (units > 0x3fffffffLL) return ARC_ERR_TOO_LARGE;
         kp.total_tiles = (int)units;
-        // Under a causal mask (as most additive ones are, too) units differ in length — with a window only the first tiles are shorter, which matters
-        // while there are few waves of units — and go longest first then, unless the K and V that all heads and
+        // Under a causal mask (as most additive ones are, too) units differ in length and go longest first then, with a window
+        // while there are fewer than eight waves of them, and unless the K and V that all heads and
         // sequences together read would not stay in L2 (126 MB).  (1531 tokens, window 1024, 96 units on 74 pairs:
-        // 36.5 -> 27 us.)
+        // 36.5 -> 27 us.)  Neither limit is sharp: with a window only the first tiles are shorter, but where the count of token tiles
+        // and the grid share a factor they fall to some CTAs only, however many waves there are (64 tiles of 9 blocks at most on 148
+        // CTAs: the fullest has 5 % over the mean), and a windowed wave reads a part of the keys.
         const bool windowed = p->window > 0 && p->window < p->kv_len;
         kp.long_first = !split && p->mask_type != ARC_MASK_NONE && units > ds->wide.pairs && (!windowed || units < 8LL * ds->wide.pairs) &&
                         (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;

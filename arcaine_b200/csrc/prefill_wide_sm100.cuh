@@ -12,7 +12,7 @@
 // is computed while the softmax warps work on S(j), so the tensor pipe only waits when a softmax takes longer than
 // 2048 clk.
 //
-// Warp roles of each CTA (320 threads, 200 registers): 0-3 softmax (one row per thread), 4-7 epilogue, 8 TMA producer
+// Warp roles of each CTA (320 threads): 0-3 softmax (one row per thread), 4-7 epilogue, 8 TMA producer
 // (its CTA's Q tile and halves of K and V), 9 MMA issuer (leader CTA only).  Full barriers live in the leader, which
 // expects the bytes of both CTAs; empty and score barriers are committed to both (commit with multicast — the loads
 // themselves use none).  The softmax and epilogue warps of both CTAs arrive on the leader's barriers.

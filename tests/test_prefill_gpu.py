@@ -420,7 +420,7 @@ def test_gemma4_decode_wrappers(ops):
 @pytest.mark.parametrize("window", [523, 540, 600])
 def test_few_keys_in_the_first_block_repeat_bit_for_bit(ops, window):
     """A window that leaves most rows a few keys of their first key block: the next block raises their maximum by far
-    more than 2^8, so the accumulator is rescaled while earlier P V products may still run.  One-tile kernel."""
+    more than 2^8, so the accumulator is rescaled while earlier P V products may still run.  One tile in two chains."""
     seq, kv_len, nq, nkv, hd = 400, 1466, 16, 8, 128
     q, k, v = seeded_bf16(1, seq, nq, hd, seed=61), seeded_bf16(1, kv_len, nkv, hd, seed=62), seeded_bf16(1, kv_len, nkv, hd, seed=63)
     want = oracle.sdpa_f32(q[0], k[0], v[0], scale=hd ** -0.5, mask_type=3, window=window)[0]
