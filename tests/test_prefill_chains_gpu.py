@@ -39,16 +39,20 @@ def test_scores_that_grow_in_one_chain(ops, at, gain):
 
 @pytest.mark.parametrize("splits", [0, 3])
 @pytest.mark.parametrize("kv_len", [300, 301])  # rows of the mask 16-byte aligned, and not
-def test_additive_mask(ops, kv_len, splits):
-    seq, nq, nkv = 200, 4, 2
+@pytest.mark.parametrize("seq,gate", [(200, False), (203, True), (73, False)])  # the mask is read eight rows at a time
+def test_additive_mask(ops, kv_len, splits, seq, gate):
+    nq, nkv = 4, 2
     q, k, v = seeded_bf16(seq, nq, 128, seed=71), seeded_bf16(kv_len, nkv, 128, seed=72), seeded_bf16(kv_len, nkv, 128, seed=73)
+    g = seeded_bf16(seq, nq, 128, seed=74)
     mask = np.random.default_rng(7).normal(0.0, 2.0, (seq, kv_len)).astype(np.float32)
     mask[:70] = 0.0                    # blocks without values for the first two warps of rows
     mask[:, 20:60] = -np.inf
     mask[10, 128:] = np.finfo(np.float32).min
     mask[40] = -np.inf                 # a row that sees nothing
-    got = ops.sdpa_prefill(q.cuda(), k.cuda(), v.cuda(), scale=0.09, mask_type=ops.MASK_EXPLICIT, mask=torch.from_numpy(mask).cuda(), num_splits=splits)
-    assert_close(got, oracle.sdpa_f32(q, k, v, scale=0.09, mask_type=oracle.MASK_EXPLICIT, mask=mask)[0], f"mask {kv_len}")
+    got = ops.sdpa_prefill(q.cuda(), k.cuda(), v.cuda(), scale=0.09, mask_type=ops.MASK_EXPLICIT, mask=torch.from_numpy(mask).cuda(), num_splits=splits,
+                           gate=g.cuda() if gate else None)
+    want = oracle.sdpa_f32(q, k, v, scale=0.09, mask_type=oracle.MASK_EXPLICIT, mask=mask, gate=g if gate else None)
+    assert_close(got, want[1].float() if gate else want[0], f"mask {kv_len}")
 
 
 @pytest.mark.parametrize("gate", [False, True])
