@@ -685,7 +685,9 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
     DecodePlan one = *plan;
     // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where
     // the stages were, at least two: 32 * hd floats a warp, at most 16 * (hd + 5) needed.)
-    if (!size_decode_cta(p->hd, heads, slices, 0, heads * G * (p->hd / finishers * csize + (csize & (csize - 1) ? 8 : csize)) * 4, ds.smem_optin, &one)) return;
+    const int rows = heads * G;
+    const int extra = 64 + 8 * ((rows + 1) & ~1) * 8 + csize * rows * (p->hd / finishers) * 4 + rows * 32;
+    if (!size_decode_cta(p->hd, heads, slices, 0, extra, ds.smem_optin, &one)) return;
     one.cluster = true;
     one.groups = p->nkv / heads;
     one.ncta = csize;

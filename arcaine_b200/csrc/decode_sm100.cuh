@@ -104,9 +104,15 @@ __device__ __forceinline__ void consumer_sync(int consumer_warps) {
 }
 
 // CLUSTER: a cluster of CTAs owns one sequence (grid.z) and one group of KV heads (grid.y); its CTAs take equal parts of
-// the sequence's keys, fold their slices as above, leave the records in the shared memory of the CTAs that finish them
+// the sequence's keys, fold their slices as above, send the records to the shared memory of the CTAs that finish them
 // and write the result: one launch, no records in global memory, no merge kernel.  For calls so small that the
 // launches are what they cost; otherwise equal shares over all SMs win.
+// What bounds it: a chain of latencies, and behind the last key instructions that run once, fetched cold at 6 clk each.  One token
+// of 24/4 heads over 513 keys: 600 clk to the lengths, 1400 to the keys, 1250 for them, and it was 7000 from there to the result
+// with records normalised and weighted by their log-sum-exps twice and a barrier of the cluster in between.  Records that travel
+// as they are, weights worked out by eight lanes a row, rolled loops and stores that count themselves on an mbarrier of the CTA they
+// go to (st.async) take half of that (us): that call 6.2 -> 5.3, 1001 keys 6.7 -> 5.5, 20 sequences of 780 keys 20.3 -> 18.4, 64 of
+// 100 to 512 keys, 16/2 heads of 128, 9.0 -> 8.1, twelve of up to 6000 12.3 -> 11.8.
 // EVEN (of CLUSTER): a power of two of CTAs, all of which finish columns.  As a case of the other instance these calls were 0.1
 // to 0.2 us slower (one token of 24/4 heads over 256 / 1001 keys 6.31 / 6.96 us, 6.16 / 6.76 so; 16 sequences of 500 keys,
 // 8/4 heads of 128: 7.92 and 7.70).
@@ -134,6 +140,18 @@ __global__ void __launch_bounds__(288, 1)
     const int lane = threadIdx.x & 31;
     const int head0 = blockIdx.y * p.nkv_cta;  // first KV head of this CTA
     const int G = p.nq / p.nkv;
+    // CLUSTER: the first 2^k CTAs of the cluster (all of 1, 2, 4 or 8, four of six) finish an equal number of columns of all
+    // heads each.  All CTAs send them what they have, weights still to come: per CTA [query head of the group][column], in front
+    // of them [CTA][query head] maximum (log2 domain) and sum, and whether all of the CTA's waits ended well.
+    const int dc_log2 = (HD == 256 ? 8 : 7) - (!CLUSTER ? 0 : EVEN ? __ffs(p.ncta) - 1 : 31 - __clz(p.ncta)), dc = 1 << dc_log2;
+    const int finishers = HD >> dc_log2;
+    const int rows = p.nkv_cta * G, rows2 = (rows + 1) & ~1;
+    uint64_t* gathered = empty + p.stages;
+    int* gave_up = reinterpret_cast<int*>(gathered + 1);
+    float* cflag = reinterpret_cast<float*>(gathered + 2);     // [8]
+    float2* cml = reinterpret_cast<float2*>(cflag + 8);         // [8][rows2]
+    float* crec = reinterpret_cast<float*>(cml + 8 * rows2);    // [CTA][rows][dc]
+    float* cweight = crec + (size_t)p.ncta * rows * dc;         // [rows][8]
 
     if (threadIdx.x == 32) {
         prefetch_tensormap(&tm_k);
@@ -144,8 +162,12 @@ __global__ void __launch_bounds__(288, 1)
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], ncw);
         }
+        if constexpr (CLUSTER) {  // what the other CTAs send here, if this one finishes columns
+            mbar_init(gathered, 1);
+            *gave_up = 0;
+        }
         fence_mbar_init();
-        if (CLUSTER) cum[0] = 1;  // results may be written: until a status or a wait that runs out, in any CTA, clears it
+        if (CLUSTER) mbar_arrive_expect_tx(gathered, (uint32_t)(p.ncta * (4 + rows * (8 + dc * 4))));
     }
     long long g0 = 0, g1 = 0;  // this CTA's keys, counted over the sequences laid end to end (CLUSTER: of its own sequence)
     int b_first = 0, my_len = 0;
@@ -208,13 +230,6 @@ __global__ void __launch_bounds__(288, 1)
     // keys before sequence b / up to its end, in the count g0 and g1 use
     auto seq_begin = [&](int b) { return CLUSTER ? 0ll : cum[b]; };
     auto seq_end = [&](int b) { return CLUSTER ? (long long)my_len : cum[b + 1]; };
-    // CLUSTER: the first 2^k CTAs of the cluster (all of 1, 2, 4 or 8, four of six) finish an equal number of columns of all
-    // heads each; the others leave their folded records of those here: [CTA][query head of the group][column], and the
-    // log-sum-exps behind (not EVEN: in front, eight places a head, so that no address waits for p.ncta).
-    const int dc_log2 = (HD == 256 ? 8 : 7) - (!CLUSTER ? 0 : EVEN ? __ffs(p.ncta) - 1 : 31 - __clz(p.ncta)), dc = 1 << dc_log2;
-    const int rows = p.nkv_cta * G;
-    float* crec = reinterpret_cast<float*>(cum + 2) + (EVEN ? 0 : 8 * rows);
-    float* crec_lse = EVEN ? crec + (size_t)rows * HD : reinterpret_cast<float*>(cum + 2);
     constexpr int RS = HD + 4;  // floats from one head's row of a warp's record to the next
 
     if (warp == ncw) {
@@ -271,9 +286,9 @@ __global__ void __launch_bounds__(288, 1)
         bool folded = false;  // this warp has been through the two barriers of the in-CTA fold
         int b = b_first;
         long long g = g0;
-        while (ok && g < g1) {
-            while (seq_end(b) <= g) ++b;
-            const long long seg_end = min(g1, seq_end(b));
+        while (CLUSTER || (ok && g < g1)) {  // (CLUSTER: once, keys or not)
+            while (!CLUSTER && seq_end(b) <= g) ++b;
+            const long long seg_end = CLUSTER ? max(g0, g1) : min(g1, seq_end(b));
             const int seg_keys = (int)(seg_end - g);
 
             // Q^T fragments (B operand, hd x 8 heads) for this head's GQA group.
@@ -426,6 +441,80 @@ __global__ void __launch_bounds__(288, 1)
                 if (lane == 0) mbar_arrive(&empty[st]);
             }
 
+            if constexpr (CLUSTER) {
+                // Everything from here on runs once a call, from instructions fetched cold, so it is kept short: records as they
+                // are, weights worked out once, by eight lanes a row, loops that are not unrolled.
+                float* rec = reinterpret_cast<float*>(stage_base);                     // [warp][NT * 8 heads][RS]
+                float2* rec_ml = reinterpret_cast<float2*>(rec + (size_t)ncw * NT * 8 * RS);  // [warp][NT * 8]
+                float* rec_w = reinterpret_cast<float*>(rec_ml + ncw * NT * 8);
+                if (lane == 0 && (!ok || !work || fault != 0u)) *reinterpret_cast<volatile int*>(gave_up) = 1;  // (no result is written)
+                consumer_sync(ncw);  // every warp is through with the stages; no copy is in flight any more
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        float ls = l[nt][u];
+                        ls += __shfl_xor_sync(0xffffffffu, ls, 4);
+                        ls += __shfl_xor_sync(0xffffffffu, ls, 8);
+                        ls += __shfl_xor_sync(0xffffffffu, ls, 16);
+                        const int n = warp * NT * 8 + nt * 8 + q4 * 2 + u;
+                        if (g4 == 0) rec_ml[n] = make_float2(m[nt][u], ls);
+                        float* dst = rec + (size_t)n * RS + g4;
+#pragma unroll
+                        for (int mt = 0; mt < HD / 16; ++mt) {
+                            dst[mt * 16] = o[nt][mt][u];
+                            dst[mt * 16 + 8] = o[nt][mt][u + 2];
+                        }
+                    }
+                consumer_sync(ncw);
+                const uint32_t bar = smem_u32(gathered);
+                // (A CTA on its own is not launched as a cluster, and st.async is for clusters: plain stores there.)
+                const bool alone = EVEN && p.ncta == 1;
+#pragma unroll 1
+                for (int n0 = slice * 4; n0 < G; n0 += p.slices * 4) {  // four rows of the KV head a turn, a lane per slice
+                    const int n = n0 + (lane >> 3), s = lane & 7, at = (s * p.nkv_cta + hl) * NT * 8 + n;
+                    const bool some = n < G && s < p.slices;
+                    const float2 ml = some ? rec_ml[at] : make_float2(-CUDART_INF_F, 0.f);
+                    float mx = ml.x;
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                    const float wt = ml.x == -CUDART_INF_F ? 0.f : fast_exp2(ml.x - mx);
+                    float z = wt * ml.y;
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+                    if (some) rec_w[at] = wt;
+                    float2* to = cml + blockIdx.x * rows2 + hl * G + n;
+                    if (n < G && s < finishers) {
+                        if (alone) *to = make_float2(mx, z);
+                        else st_async_f32x2(map_to_cta(smem_u32(to), s), make_float2(mx, z), map_to_cta(bar, s));
+                    }
+                }
+                if (warp == 0 && lane < finishers) {
+                    const float good = *reinterpret_cast<volatile int*>(gave_up) ? 0.f : 1.f;
+                    if (alone) cflag[0] = good;
+                    else st_async_f32(map_to_cta(smem_u32(cflag + blockIdx.x), lane), good, map_to_cta(bar, lane));
+                }
+                consumer_sync(ncw);
+#pragma unroll 1
+                for (int i = slice; i < G * (HD / 128); i += p.slices) {  // half a row (head dim 256) a turn
+                    const int n = i / (HD / 128), d = i % (HD / 128) * 128 + lane * 4;
+                    const float* src = rec + (size_t)(hl * NT * 8 + n) * RS + d;
+                    const float* wts = rec_w + hl * NT * 8 + n;
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+                    for (int s = 0; s < p.slices; ++s) {
+                        const float wt = *wts;
+                        const float4 v = *reinterpret_cast<const float4*>(src);
+                        acc.x = fmaf(wt, v.x, acc.x), acc.y = fmaf(wt, v.y, acc.y), acc.z = fmaf(wt, v.z, acc.z), acc.w = fmaf(wt, v.w, acc.w);
+                        src += (size_t)p.nkv_cta * NT * 8 * RS, wts += p.nkv_cta * NT * 8;
+                    }
+                    float* at = crec + (size_t)(blockIdx.x * rows + hl * G + n) * dc + (d & (dc - 1));
+                    const int to = d >> dc_log2;
+                    if (alone) *reinterpret_cast<float4*>(at) = acc;
+                    else st_async_f32x4(map_to_cta(smem_u32(at), to), acc, map_to_cta(bar, to));
+                }
+                break;
+            }
             // Partial record of this (CTA, sequence, slice): normalised out + natural-log lse.
             // The last segment of the share (for most CTAs the only one) is folded across the slices inside
             // the CTA first: the stages are free by then, so each warp leaves its record in shared memory,
@@ -433,7 +522,7 @@ __global__ void __launch_bounds__(288, 1)
             // 0's slot; the other slices' slots stay unwritten.  The merge kernel then reads
             // `slices` times fewer records.  Earlier segments (a sequence boundary inside the share) write
             // one record per slice.
-            const bool fold_here = CLUSTER || (p.slices > 1 && seg_end == g1);  // CTA-uniform
+            const bool fold_here = p.slices > 1 && seg_end == g1;  // CTA-uniform
             // (rows four floats longer than HD: the four lanes that write the same column of different heads hit different banks)
             float* rec = reinterpret_cast<float*>(stage_base);     // [warp][NT * 8 heads][RS]
             float* rec_lse = rec + (size_t)ncw * NT * 8 * RS;      // [warp][NT * 8]
@@ -509,73 +598,72 @@ __global__ void __launch_bounds__(288, 1)
                         }
                     }
                     const float rec_l = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
-                    if constexpr (CLUSTER) {
-                        const uint32_t mine = smem_u32(crec + ((size_t)blockIdx.x * rows + hl * G + n) * dc);
 #pragma unroll
-                        for (int j = 0; j < HD / 128; ++j) {
-                            const int d = lane * 4 + 128 * j;
-                            st_cluster_f32x4(map_to_cta(mine + (d & (dc - 1)) * 4, d >> dc_log2), acc[j]);
-                        }
-                        if (lane < p.ncta) st_cluster_f32(map_to_cta(smem_u32(crec_lse + blockIdx.x * rows + hl * G + n), lane), rec_l);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < HD / 128; ++j) *reinterpret_cast<float4*>(p.part_o + (row0 + n) * HD + lane * 4 + 128 * j) = acc[j];
-                        if (lane == 0) p.part_lse[row0 + n] = rec_l;
-                    }
+                    for (int j = 0; j < HD / 128; ++j) *reinterpret_cast<float4*>(p.part_o + (row0 + n) * HD + lane * 4 + 128 * j) = acc[j];
+                    if (lane == 0) p.part_lse[row0 + n] = rec_l;
                 }
             }
             g = seg_end;
         }
         // A warp that gave up a wait never reached the fold: it still meets the others at both barriers.
-        if (!folded && (CLUSTER || p.slices > 1)) {
+        if (!CLUSTER && !folded && p.slices > 1) {
             consumer_sync(ncw);
             consumer_sync(ncw);
         }
-        // (A producer that gives up leaves a consumer waiting, which comes here.)
-        if (CLUSTER && !ok && lane < p.ncta) st_cluster_f32(map_to_cta(smem_u32(cum), lane), 0.0f);
-        // (CLUSTER: no keys: an empty record)
-        if (CLUSTER && !folded && lane < p.ncta)
-            for (int n = slice; n < G; n += p.slices)
-                st_cluster_f32(map_to_cta(smem_u32(crec_lse + blockIdx.x * rows + hl * G + n), lane), -CUDART_INF_F);
     }
     if constexpr (CLUSTER) {
-        // This CTA's columns, two a thread.  Every record is in its own shared memory by now: read out of the other CTAs
-        // instead, 16 loads a thread, this step took 2100 clk.
-        if (threadIdx.x == 0 && (!work || fault != 0u)) cum[0] = 0;
-        const int items = EVEN || (int)(blockIdx.x << dc_log2) < HD ? rows * (dc / 2) : 0, b = blockIdx.z;
+        // This CTA's columns, two a thread, once every record is in its own shared memory.  (Nothing is sent to a CTA that
+        // finishes none, and what this one has sent is waited for by those it went to: no barrier of the cluster here.)
+        if (!EVEN && (int)(blockIdx.x << dc_log2) >= HD) return;
+        const int items = rows * (dc / 2), b = blockIdx.z;
         auto offset_of = [&](int item) {
             return (long long)b * p.o_stride_b + (long long)(head0 * G + (item >> (dc_log2 - 1))) * HD + blockIdx.x * dc + (item & (dc / 2 - 1)) * 2;
         };
         uint32_t gw = p.gate && (int)threadIdx.x < items ? *reinterpret_cast<const uint32_t*>(p.gate + offset_of(threadIdx.x)) : 0u;
         __syncwarp();
-        cluster_sync_all();  // every CTA's records are where they belong
-        for (int item = threadIdx.x; cum[0] && item < items; item += blockDim.x) {
+        bool fine = true;
+        if (EVEN && p.ncta == 1) __syncthreads();
+        else fine = mbar_wait_cluster(gathered, 0);
+        if (!fine) {
+            if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x10000u);
+            cluster_sync_all();  // (what is still under way here arrives before the other CTAs have gone)
+        }
+        fine = __all_sync(0xffffffffu, fine && ((lane & 7) >= p.ncta || cflag[lane & 7] != 0.f));
+        // The CTAs' weights of a row: eight lanes.
+#pragma unroll 1
+        for (int n0 = warp * 4; n0 < rows; n0 += (ncw + 1) * 4) {
+            const int n = n0 + (lane >> 3), c = lane & 7;
+            const float2 ml = n < rows && c < p.ncta ? cml[c * rows2 + n] : make_float2(-CUDART_INF_F, 0.f);
+            float mx = ml.x;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float wt = ml.x == -CUDART_INF_F ? 0.f : fast_exp2(ml.x - mx);
+            float z = wt * ml.y;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+            if (n < rows) {
+                cweight[n * 8 + c] = z > 0.f ? __fdividef(wt, z) : 0.f;
+                if (p.out_lse && fine && blockIdx.x == 0 && c == 0)
+                    p.out_lse[(long long)b * p.nq + head0 * G + n] = z > 0.f ? (mx + fast_log2(z)) * 0.6931471805599453f : -CUDART_INF_F;
+            }
+        }
+        __syncthreads();
+        if (!fine) return;
+#pragma unroll 1
+        for (int item = threadIdx.x; item < items; item += blockDim.x) {
             const int n = item >> (dc_log2 - 1), d = (item & (dc / 2 - 1)) * 2;
             const long long eoff = offset_of(item);
             if (p.gate && item != (int)threadIdx.x) gw = *reinterpret_cast<const uint32_t*>(p.gate + eoff);
-            float li[8], mx = -CUDART_INF_F;
-            float2 v[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                li[c] = c < p.ncta ? crec_lse[c * rows + n] : -CUDART_INF_F;
-                v[c] = c < p.ncta ? *reinterpret_cast<const float2*>(crec + (size_t)(c * rows + n) * dc + d) : make_float2(0.f, 0.f);
-                mx = fmaxf(mx, li[c]);
+            float a0 = 0.f, a1 = 0.f;
+#pragma unroll 2
+            for (int c = 0; c < p.ncta; ++c) {
+                const float wt = cweight[n * 8 + c];
+                const float2 v = *reinterpret_cast<const float2*>(crec + (size_t)(c * rows + n) * dc + d);
+                a0 = fmaf(wt, v.x, a0);
+                a1 = fmaf(wt, v.y, a1);
             }
-            float z = 0.f, a0 = 0.f, a1 = 0.f;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                if (li[c] == -CUDART_INF_F) continue;  // an empty record may hold anything
-                const float wt = __expf(li[c] - mx);
-                z += wt;
-                a0 = fmaf(wt, v[c].x, a0);
-                a1 = fmaf(wt, v[c].y, a1);
-            }
-            const float iz = z > 0.f ? 1.f / z : 0.f;
-            a0 *= iz;
-            a1 *= iz;
             const long long row = (long long)b * p.nq + head0 * G + n;
             if (p.out_f32) *reinterpret_cast<float2*>(p.out_f32 + row * HD + blockIdx.x * dc + d) = make_float2(a0, a1);
-            if (p.out_lse && blockIdx.x == 0 && d == 0) p.out_lse[row] = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
             if (p.out) {
                 if (p.gate) {
                     a0 = sigmoid_gate(a0, (uint16_t)(gw & 0xffffu));

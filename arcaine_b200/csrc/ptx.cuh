@@ -206,12 +206,19 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
     return r;
 }
 
-// Into another CTA's shared memory (address from map_to_cta).
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+// Into another CTA's shared memory, counted in bytes on an mbarrier of that CTA (both addresses from map_to_cta): who has
+// waited for the phase with mbar_wait_cluster sees the values.
+__device__ __forceinline__ void st_async_f32(uint32_t addr, float v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(v), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void st_cluster_f32x4(uint32_t addr, float4 v) {
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+__device__ __forceinline__ void st_async_f32x2(uint32_t addr, float2 v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(v.x), "f"(v.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async_f32x4(uint32_t addr, float4 v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(v.x), "f"(v.y),
+                 "f"(v.z), "f"(v.w), "r"(bar)
+                 : "memory");
 }
 
 // One arrival for a converged warp, without release at cluster scope: for arrivals that announce tensor-memory accesses
@@ -222,6 +229,23 @@ __device__ __forceinline__ void mbar_arrive_remote_warp(uint32_t remote_bar) {
         "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
         "@q mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(remote_bar)
         : "memory");
+}
+
+// A whole warp waits for a phase that other CTAs of the cluster complete, and sees what they wrote for it.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, long long limit_cycles = 2000000000LL) {
+    const long long t0 = clock64();
+    do {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (__all_sync(0xffffffffu, ok != 0)) return true;
+    } while (clock64() - t0 < limit_cycles);
+    return false;
 }
 
 // ---------------------------------------------------------------------------

@@ -451,6 +451,17 @@ def test_one_launch_form_in_clusters_of_any_size(ops, B, nq, nkv, hd, n):
     check_ragged_batch(ops, q, k, v, g, lens)
 
 
+@pytest.mark.parametrize("B,nq,nkv,hd,n", [
+    (2, 3, 1, 256, 100), (1, 7, 7, 128, 500), (3, 9, 1, 256, 700), (2, 13, 1, 128, 300),  # an odd number of rows, one and two tiles of heads
+    (30, 25, 5, 128, 200),                          # a CTA alone, one KV head
+    (60, 15, 5, 128, 90), (100, 14, 2, 256, 50),    # several
+])
+def test_one_launch_form_of_any_group(ops, B, nq, nkv, hd, n):
+    lens = [max(0, n - 11 * b) for b in range(B)]
+    q, k, v, g = (seeded_bf16(*shape, seed=700 + i) for i, shape in enumerate([(B, nq, hd), (B, n, nkv, hd), (B, n, nkv, hd), (B, nq, hd)]))
+    check_ragged_batch(ops, q, k, v, g, lens)
+
+
 @pytest.mark.parametrize("B,nq,nkv,total", [
     (5, 24, 4, 7600),   # 20 clusters of six CTAs in steps of six slices
     (12, 16, 2, 7600),  # 24 of five, groups of eight heads
