@@ -250,14 +250,15 @@ __device__ __forceinline__ void stage_open(OutStage& s, const void* tm_gate, int
 
 // The epilogue takes STAGE_COLS columns a turn of a rolled loop: its code runs beside the softmax loop out of the same
 // instruction cache, and what does not fit beside it costs 50 clk per 128 bytes on every turn.  (Gated, 32 columns a
-// turn are 6 KB of code and took 2500 clk, 16 columns 2.5 KB.)
+// turn are 6 KB of code and took 2500 clk, 16 columns 2.5 KB.  On CTA pairs, whose softmax loop is shorter, 32 gated columns are
+// the better turn: 1200 clk, and 690 for 16: prefill_wide_sm100.cuh.)
 template <bool GATE>
 constexpr int STAGE_COLS = GATE ? 16 : 32;
 
-// Before turn k of a tile of HD columns.  False: the gate values never came.
-template <bool GATE, int HD>
+// Before turn k, of N columns, of a tile of HD columns.  False: the gate values never came.
+template <bool GATE, int HD, int N = STAGE_COLS<GATE>>
 __device__ __forceinline__ bool stage_before(OutStage& s, const void* tm_gate, int lane, int k) {
-    constexpr int TURNS = 64 / STAGE_COLS<GATE>;  // per round
+    constexpr int TURNS = 64 / N;  // per round
     const int c = k / TURNS, i = c & 1;
     if (k % TURNS == 0) {
         if (GATE) {
@@ -280,7 +281,7 @@ __device__ __forceinline__ bool stage_before(OutStage& s, const void* tm_gate, i
 // Turn k: the accumulator's values times `inv`, gated, as bf16 into the buffer (and into w8 for the caller); after a
 // round's last turn the round is sent off.  taken(): called once acc has been used, so that the next turn's values
 // can be on their way while this turn's are gated.
-template <bool GATE, typename F, int N = STAGE_COLS<GATE>>
+template <bool GATE, typename F, int N>
 __device__ __forceinline__ void stage_turn(const OutStage& s, const void* tm_out, int lane, int k, const uint32_t (&acc)[N], float inv,
                                            uint32_t (&w8)[N / 2], F&& taken) {
     constexpr int TURNS = 64 / N;

@@ -616,12 +616,14 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             ++n;
             const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
             bool ok = true;
-            constexpr int SC = STAGE_COLS<GATE>;
+            // 32 columns a turn.  (Gated, of which a turn of 16 took 690 clk, 1200 so.  us: 1300 tokens of 24/4 heads 33.6 -> 31.5, 2000
+            // 57.5 -> 54, 4 x 1500, window 300, 106 -> 97; cold, 200 x 333 of 8/4, 14.4 -> 13.3.)
+            constexpr int SC = 32;
             uint32_t wa[SC], w8[SC / 2];
             tmem_ld(tO, wa);
 #pragma unroll 1
             for (int c = 0; c < HD / SC; ++c) {
-                if (warp_store && !stage_before<GATE, HD>(stage, &tm_gate, lane, c)) {
+                if (warp_store && !stage_before<GATE, HD, SC>(stage, &tm_gate, lane, c)) {
                     if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x600u);
                     ok = false;
                     break;
