@@ -278,6 +278,16 @@ __device__ __forceinline__ bool stage_before(OutStage& s, const void* tm_gate, i
     return true;
 }
 
+// Round c of the stage is complete: sent off.
+__device__ __forceinline__ void stage_send(const OutStage& s, const void* tm_out, int lane, int c) {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+        tma_store_4d(tm_out, s.buf + (c & 1) * 4096, c * 64, s.h, s.t0, s.b);
+        bulk_commit();
+    }
+}
+
 // Turn k: the accumulator's values times `inv`, gated, as bf16 into the buffer (and into w8 for the caller); after a
 // round's last turn the round is sent off.  taken(): called once acc has been used, so that the next turn's values
 // can be on their way while this turn's are gated.
@@ -310,14 +320,7 @@ __device__ __forceinline__ void stage_turn(const OutStage& s, const void* tm_out
         }
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at[i]), "r"(w8[4 * i]), "r"(w8[4 * i + 1]), "r"(w8[4 * i + 2]), "r"(w8[4 * i + 3]) : "memory");
     }
-    if (k % TURNS == TURNS - 1) {
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-            tma_store_4d(tm_out, s.buf + (c & 1) * 4096, c * 64, s.h, s.t0, s.b);
-            bulk_commit();
-        }
-    }
+    if (k % TURNS == TURNS - 1) stage_send(s, tm_out, lane, c);
 }
 
 // The gated epilogue and the one that also stores copies of the output are instances of their own: code the

@@ -236,7 +236,10 @@ __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int ran
 // read out of the other CTAs' shared memory, 11 bytes per clk and SM, the fold took 5 us.  Every instruction here runs
 // once per launch and is fetched cold, 50 clk per 128 bytes of code, so the loops are rolled: with five rows unrolled
 // the fold itself took 8700 clk.
-template <bool GATE, bool MASKED, bool SPLIT = false>
+// EARLY (not gated): pairs take several units.  The epilogue then empties the accumulator into registers first (1600 clk), for the
+// next unit's P V to go on; in turns, with the way out of the SM between them, it took 3000.  (2 x 5000 tokens of 16/8 heads,
+// window 512, 103 -> 96 us.  Gated rows wait for sigmoids, not for the way out: taken early they cost calls of short units 8 %.)
+template <bool GATE, bool MASKED, bool SPLIT = false, bool EARLY = false>
 __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     sdpa_prefill_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
@@ -616,35 +619,78 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             ++n;
             const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
             bool ok = true;
-            // 32 columns a turn.  (Gated, of which a turn of 16 took 690 clk, 1200 so.  us: 1300 tokens of 24/4 heads 33.6 -> 31.5, 2000
-            // 57.5 -> 54, 4 x 1500, window 300, 106 -> 97; cold, 200 x 333 of 8/4, 14.4 -> 13.3.)
-            constexpr int SC = 32;
-            uint32_t wa[SC], w8[SC / 2];
-            tmem_ld(tO, wa);
-#pragma unroll 1
-            for (int c = 0; c < HD / SC; ++c) {
-                if (warp_store && !stage_before<GATE, HD, SC>(stage, &tm_gate, lane, c)) {
-                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x600u);
-                    ok = false;
-                    break;
-                }
-                tmem_wait_ld();
-                if (c + 1 == HD / SC) {  // O is in registers: the next unit may overwrite the accumulator
-                    tc_fence_before_sync();
-                    mbar_arrive_remote_warp(b_empty);
-                }
-                auto next = [&]() {
-                    if (c + 1 < HD / SC) tmem_ld(tO + (c + 1) * SC, wa);
-                };
-                if (!warp_store) next();
-                if (warp_store) {
-                    stage_turn<GATE>(stage, &tm_out, lane, c, wa, inv, w8, next);
-                    if (store) {
-                        for (int k = 0; k < p.n_copies; ++k) {
-                            uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + eoff + c * SC);
+            auto store_copies = [&](const uint32_t* words, int n, int col) {  // of this thread's row
+                if (stage.t0 + lane >= p.seq) return;
+                const long long at = stage.b * p.o_stride_b + (stage.t0 + lane) * p.o_stride_t + (long long)stage.h * HD + col;
+                for (int k = 0; k < p.n_copies; ++k) {
+                    uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + at);
 #pragma unroll
-                            for (int i = 0; i < SC / 8; ++i) d4[i] = make_uint4(w8[4 * i], w8[4 * i + 1], w8[4 * i + 2], w8[4 * i + 3]);
-                        }
+                    for (int i = 0; i < n / 4; ++i) d4[i] = make_uint4(words[4 * i], words[4 * i + 1], words[4 * i + 2], words[4 * i + 3]);
+                }
+            };
+            if constexpr (EARLY) {
+                // The whole row into registers as bf16 pairs, so that the next unit may overwrite the accumulator before the last
+                // columns have left the SM.
+                uint32_t pk[HD / 2], va[32], vb[32];
+                const uint64_t inv2 = pack_f32x2(inv, inv);
+                auto take = [&](const uint32_t (&v)[32], uint32_t* to) {
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) {
+                        float x0, x1;
+                        unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(v[2 * u]), __uint_as_float(v[2 * u + 1])), inv2), x0, x1);
+                        to[u] = pack_bf16x2(x0, x1);
+                    }
+                };
+                tmem_ld32(tO, va);
+#pragma unroll
+                for (int c = 0; c < HD / 32; c += 2) {
+                    tmem_wait_ld();
+                    tmem_ld32(tO + (c + 1) * 32, vb);
+                    take(va, pk + c * 16);
+                    tmem_wait_ld();
+                    if (c + 2 < HD / 32) tmem_ld32(tO + (c + 2) * 32, va);
+                    take(vb, pk + (c + 1) * 16);
+                }
+                tc_fence_before_sync();
+                mbar_arrive_remote_warp(b_empty);
+                if (warp_store) {
+                    const uint32_t at = smem_u32(stage.buf) + lane * 128;
+#pragma unroll
+                    for (int c = 0; c < HD / 64; ++c) {
+                        stage_before<false, HD>(stage, &tm_gate, lane, 2 * c);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"((at + (c & 1) * 4096) + ((i ^ (lane & 7)) << 4)),
+                                         "r"(pk[c * 32 + 4 * i]), "r"(pk[c * 32 + 4 * i + 1]), "r"(pk[c * 32 + 4 * i + 2]), "r"(pk[c * 32 + 4 * i + 3]) : "memory");
+                        stage_send(stage, &tm_out, lane, c);
+                    }
+                    store_copies(pk, HD / 2, 0);
+                }
+            } else {
+                // 32 columns a turn.  (Gated, of which a turn of 16 took 690 clk, 1200 so.  us: 1300 tokens of 24/4 heads 33.6 -> 31.5, 2000
+                // 57.5 -> 54, 4 x 1500, window 300, 106 -> 97; cold, 200 x 333 of 8/4, 14.4 -> 13.3.)
+                constexpr int SC = 32;
+                uint32_t wa[SC], w8[SC / 2];
+                tmem_ld(tO, wa);
+#pragma unroll 1
+                for (int c = 0; c < HD / SC; ++c) {
+                    if (warp_store && !stage_before<GATE, HD, SC>(stage, &tm_gate, lane, c)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x600u);
+                        ok = false;
+                        break;
+                    }
+                    tmem_wait_ld();
+                    if (c + 1 == HD / SC) {  // O is in registers: the next unit may overwrite the accumulator
+                        tc_fence_before_sync();
+                        mbar_arrive_remote_warp(b_empty);
+                    }
+                    auto next = [&]() {
+                        if (c + 1 < HD / SC) tmem_ld(tO + (c + 1) * SC, wa);
+                    };
+                    if (!warp_store) next();
+                    if (warp_store) {
+                        stage_turn<GATE>(stage, &tm_out, lane, c, wa, inv, w8, next);
+                        store_copies(w8, SC / 2, c * SC);
                     }
                 }
             }
