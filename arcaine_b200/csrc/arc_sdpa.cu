@@ -370,14 +370,13 @@ static int launch_fold(const arc_sdpa_prefill_params* p, const PrefillPlan& plan
     return ARC_OK;
 }
 
-// What the SM with most to do takes for its share of `units` units (`heads` per token tile and sequence, of `tiles` token
-// tiles each), a unit taking per_block for each of its key blocks and per_unit.  Dealt in plain order units count as all as long
-// as the longest; longest first and every second wave in reverse (TileCursor), the load is linear in the SM's index between
-// the ends of the waves, so these are what is looked at.
-static double longest_share(const arc_sdpa_prefill_params* p, long long units, int heads, int tiles, long long sms, bool by_length, double per_block, double per_unit) {
+// What the SM (or CTA pair) with most to do takes for its share of the units [u0, u1) (`heads` per token tile and sequence, of
+// `tiles` token tiles each), which are dealt to `sms` of them longest first and every second wave in reverse, a unit taking
+// per_block for each of its key blocks and per_unit.  The load is linear in the SM's index between the ends of the waves, so
+// these are what is looked at.
+static double longest_sorted_share(const arc_sdpa_prefill_params* p, long long u0, long long u1, int heads, int tiles, long long sms, double per_block, double per_unit) {
     const int q_tiles = (p->seq + 127) / 128;
-    const long long waves = (units + sms - 1) / sms, rest = units - (waves - 1) * sms;
-    if (!by_length || waves > 16) return (double)waves * (per_block * tile_key_blocks(p, q_tiles - 1) + per_unit);
+    const long long units = u1 - u0, waves = (units + sms - 1) / sms, rest = units - (waves - 1) * sms;
     const long long per = (long long)heads * p->batch, edge = (waves & 1) ? rest : sms - rest;
     double most = 0.0;
     for (long long x : {0ll, sms - 1, edge - 1, edge}) {
@@ -385,11 +384,18 @@ static double longest_share(const arc_sdpa_prefill_params* p, long long units, i
         double sum = 0.0;
         for (long long i = 0; i < waves; ++i) {
             const long long u = i * sms + ((i & 1) ? sms - 1 - x : x);
-            if (u < units) sum += per_block * tile_key_blocks(p, std::min(q_tiles - 1, (int)((q_tiles + tiles - 1) / tiles - 1 - u / per) * tiles + tiles - 1)) + per_unit;
+            if (u < units) sum += per_block * tile_key_blocks(p, std::min(q_tiles - 1, (int)((q_tiles + tiles - 1) / tiles - 1 - (u0 + u) / per) * tiles + tiles - 1)) + per_unit;
         }
         most = std::max(most, sum);
     }
     return most;
+}
+
+// The same of all `units` units, or, dealt in plain order, as if all were as long as the longest.
+static double longest_share(const arc_sdpa_prefill_params* p, long long units, int heads, int tiles, long long sms, bool by_length, double per_block, double per_unit) {
+    const long long waves = (units + sms - 1) / sms;
+    if (!by_length || waves > 16) return (double)waves * (per_block * tile_key_blocks(p, (p->seq + 127) / 128 - 1) + per_unit);
+    return longest_sorted_share(p, 0, units, heads, tiles, sms, per_block, per_unit);
 }
 
 // Digits of a grid of `ctas` in the tile list, fastest first (TileCursor).
@@ -550,6 +556,17 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         const bool windowed = p->window > 0 && p->window < p->kv_len;
         kp.long_first = !split && p->mask_type != ARC_MASK_NONE && units > ds->wide.pairs && (!windowed || units < 8LL * ds->wide.pairs) &&
                         (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;
+        // A few waves: with k whole ones, the pairs that get k units may as well have the longest and leave the rest, which are
+        // shorter, to those that get k + 1.  (2048 queries over 5049 keys, 24 heads: 192 units of 25 to 40 blocks on 74 pairs, the fullest with
+        // 96 blocks in one list and 91 so, 84 on average: 165 -> 147 us on a cool chip; 8192 tokens of 24/4 191 -> 184, a vision prompt 25.1 -> 24.7.)
+        const long long pairs = ds->wide.pairs, whole = units / pairs, extra = units % pairs;
+        if (kp.long_first && !masked && extra > 0 && whole <= 8) {
+            const int tiles = kp.head_pair ? 1 : 2;
+            const long long few = pairs - extra, end = whole * few;
+            const double as_one = longest_sorted_share(p, 0, units, kp.cur_heads, tiles, pairs, 1.0, 1.0);
+            if (std::max(longest_sorted_share(p, 0, end, kp.cur_heads, tiles, few, 1.0, 1.0), longest_sorted_share(p, end, units, kp.cur_heads, tiles, extra, 1.0, 1.0)) < as_one)
+                kp.few = (int)few, kp.few_end = (int)end;
+        }
         if ((rc = make_tile_map(&tk, p->k, HD, p->nkv, p->kv_len, p->batch, p->k_stride_t, p->k_stride_b, 64)) != ARC_OK) return rc;
         if (split) {
             to = tg = tq;  // (not used)

@@ -57,6 +57,7 @@ struct PrefillParams {
     int tail_base;
     int long_first;  // units in order of falling length
     int step[3];     // digits of the grid's size in the tile list (TileCursor)
+    int few, few_end;  // CTA pairs that share the longest units [0, few_end) (WideCursor)
     // The additive mask as mask_scan_kernel has read it (prefill_wide_sm100.cuh; mask_blocks key blocks per row tile)
     const uint32_t* mask_class;  // [row tile][key block]: a byte per 32 rows, MASK_* bits
     const uint4* mask_bits;      // [row tile][key block][row]: one bit per key, set where the mask is 0

@@ -177,12 +177,18 @@ __device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first,
 // run side by side share K and V in L2).  long_first (causal without a window, several waves): the units with most key
 // blocks first, all heads of a token tile together, and every second wave in reverse order, so that the sums of a
 // pair's units are about equal.
+// few > 0: the first `few` pairs share the longest units [0, few_end) in that way and the others the rest, of which they take
+// one more each.
 struct WideCursor {
-    int w, i, first, step;
-    __device__ __forceinline__ WideCursor(int first_, int step_) : w(first_), i(0), first(first_), step(step_) {}
+    int w, i;
+    __device__ __forceinline__ explicit WideCursor(const PrefillParams& p) : i(-1) { advance(p); }
     __device__ __forceinline__ void advance(const PrefillParams& p) {
+        const int place = (int)(blockIdx.x >> 1);
+        const bool rest = place >= p.few;  // (few is 0 where nothing is divided in this way)
+        const int base = rest ? p.few_end : 0, first = rest ? place - p.few : place;
+        const int step = rest ? (int)(gridDim.x >> 1) - p.few : p.few;
         ++i;
-        w = i * step + (p.long_first && (i & 1) ? step - 1 - first : first);
+        w = base + i * step + (p.long_first && (i & 1) ? step - 1 - first : first);
     }
 };
 
@@ -310,11 +316,10 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     if (warp == C::PRODUCER_WARP) tmem_alloc_pair(tmem_slot, 512);
     // One warp finds the first unit for all, beside the tensor memory's allocation; its divisions, and the code that every role
     // would fetch for them, took 2500 clk between the kernel's release and its first load.
-    const int place = (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
     const bool blocks_in_memory = MASKED || p.ids;
     WideWork w_first{};
     if (warp == C::EPILOGUE_WARP) {
-        w_first = wide_place<SPLIT>(p, WideCursor(place, step), rank);
+        w_first = wide_place<SPLIT>(p, WideCursor(p), rank);
         if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
         if (lane == 0) *first_unit = w_first;
     }
@@ -376,7 +381,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     }
     tc_fence_after_sync();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
-    const int total = *abort_slot ? 0 : p.total_tiles;  // a status is set: walk an empty list
+    const int total = *abort_slot ? 0 : (int)(blockIdx.x >> 1) < p.few ? p.few_end : p.total_tiles;  // a status is set: walk an empty list
     auto unit_at = [&](const WideCursor& cur) {
         if (SPLIT || cur.i == 0) return *first_unit;
         WideWork w = wide_place<SPLIT>(p, cur, rank);
@@ -441,7 +446,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x100u);
             return false;
         };
-        WideCursor cur(place, step);
+        WideCursor cur(p);
         for (; ok && cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
             if (w.hi == w.lo) continue;
@@ -515,7 +520,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 ++gs;
                 return true;
             };
-            WideCursor cur(place, step);
+            WideCursor cur(p);
             auto next_unit = [&](WideWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
                 for (; cur.w < total; cur.advance(p)) {
                     w = unit_at(cur);
@@ -582,7 +587,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         const uint32_t b_empty = map_to_cta(smem_u32(o_empty), lead);
         int n = 0;  // units with key blocks so far
         OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0};
-        WideCursor cur(place, step);
+        WideCursor cur(p);
         for (; cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
             const int t0 = w.q0 + quarter * 32, t = t0 + lane;
@@ -712,7 +717,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         int g = 0, n = 0;  // key blocks and units so far
         bool ok = true;
         uint32_t s0[32], s1[32], s2[32], s3[32];  // the row's 128 scores of the current block
-        WideCursor cur(place, step);
+        WideCursor cur(p);
         for (; ok && cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
             if (w.hi == w.lo) {
