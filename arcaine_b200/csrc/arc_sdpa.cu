@@ -398,6 +398,19 @@ static double longest_share(const arc_sdpa_prefill_params* p, long long units, i
     return longest_sorted_share(p, 0, units, heads, tiles, sms, per_block, per_unit);
 }
 
+// Longest first, all heads and sequences of a token tile run side by side: do the keys and values that they read together stay in
+// L2 (126 MB)?  All of them may, where there are few waves or no window; behind a window it is the window's and those of the tiles under
+// way that are read at one time.  In plain order the shorter first tiles of a windowed call fall to some CTAs only, however many waves
+// there are, where the count of token tiles and the grid share a factor: 5 to 20 % between the fullest CTA and the mean.  (us, plain and
+// longest first, window 1024 unless said: 8192 tokens of 24/4 heads of 256 184 and 177; 2 x 8192 of 28/4 of 128, window 2048, 399
+// and 378; 4 x 6000 of 16/8, window 300, 120 and 111; but 4 x 8192 of 32/16, whose windows are 48 MB, 534 and 577.)
+static bool stays_in_l2(const arc_sdpa_prefill_params* p, bool few_waves) {
+    const bool windowed = p->window > 0 && p->window < p->kv_len;
+    const long long key = (long long)p->batch * p->nkv * p->hd * 4;
+    if (windowed && std::min<long long>(p->kv_len, (long long)p->window + 512) * key <= 24ll << 20) return true;
+    return (few_waves || !windowed) && p->kv_len * key <= 96ll << 20;
+}
+
 // Digits of a grid of `ctas` in the tile list, fastest first (TileCursor).
 static void set_step(PrefillParams* kp, long long ctas) {
     const long long rf = kp->long_first ? kp->cur_heads : kp->q_tiles, rm = kp->long_first ? kp->batch : kp->cur_heads;
@@ -468,11 +481,9 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         // hundred, of three waves and more (4 x 1728 tokens of 32/16 heads, no mask, by the measure below: 97.9 cut, 101.5 whole, 105.0 in
         // chains); in others chains cover the tiles more evenly.
         const long long full_waves = pair_tiles / sms, left = pair_tiles - full_waves * sms;
-        // Under a causal mask tiles differ in length and go longest first, as at head dim 256 below, with the same two limits.
-        const bool windowed = p->window > 0 && p->window < p->kv_len;
+        // Under a causal mask tiles differ in length and go longest first, as at head dim 256 below, with the same limit.
         const auto by_length = [&](long long units) {
-            return !split && p->mask_type == ARC_MASK_CAUSAL && units > sms && (!windowed || units < 8 * sms) &&
-                   (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;
+            return !split && p->mask_type == ARC_MASK_CAUSAL && units > sms && stays_in_l2(p, units < 8 * sms);
         };
         // In steps of a key block of a pair (1.37 us): launches, loads and output apart, a pair's unit takes its blocks and
         // half a step, a tile in chains 0.52 a block and 0.8.  A second launch for the tail adds 3.6 (it starts when the first
@@ -547,15 +558,9 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         const long long units = wide_units(p, plan.q_tiles) * plan.splits;
         if (units > 0x3fffffffLL) return ARC_ERR_TOO_LARGE;
         kp.total_tiles = (int)units;
-        // Under a causal mask (as most additive ones are, too) units differ in length and go longest first then, with a window
-        // while there are fewer than eight waves of them, and unless the K and V that all heads and
-        // sequences together read would not stay in L2 (126 MB).  (1531 tokens, window 1024, 96 units on 74 pairs:
-        // 36.5 -> 27 us.)  Neither limit is sharp: with a window only the first tiles are shorter, but where the count of token tiles
-        // and the grid share a factor they fall to some CTAs only, however many waves there are (64 tiles of 9 blocks at most on 148
-        // CTAs: the fullest has 5 % over the mean), and a windowed wave reads a part of the keys.
-        const bool windowed = p->window > 0 && p->window < p->kv_len;
-        kp.long_first = !split && p->mask_type != ARC_MASK_NONE && units > ds->wide.pairs && (!windowed || units < 8LL * ds->wide.pairs) &&
-                        (long long)p->batch * p->kv_len * p->nkv * HD * 4 <= 96ll << 20;
+        // Under a causal mask (as most additive ones are, too) units differ in length and go longest first then, unless K and V would
+        // not stay in L2.  (1531 tokens, window 1024, 96 units on 74 pairs: 36.5 -> 27 us.)
+        kp.long_first = !split && p->mask_type != ARC_MASK_NONE && units > ds->wide.pairs && stays_in_l2(p, units < 8LL * ds->wide.pairs);
         // A few waves: with k whole ones, the pairs that get k units may as well have the longest and leave the rest, which are
         // shorter, to those that get k + 1.  (2048 queries over 5049 keys, 24 heads: 192 units of 25 to 40 blocks on 74 pairs, the fullest with
         // 96 blocks in one list and 91 so, 84 on average: 165 -> 147 us on a cool chip; 8192 tokens of 24/4 191 -> 184, a vision prompt 25.1 -> 24.7.)
