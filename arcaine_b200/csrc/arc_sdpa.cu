@@ -116,11 +116,11 @@ static ChainsKernel chains_kernel(bool gate, bool vision, bool masked) {
 }
 
 using WideKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, PrefillParams);
-static WideKernel wide_kernel(bool gate, bool masked, bool split, bool several) {  // (several: units per CTA pair)
-    if (split) return masked ? sdpa_prefill_wide_kernel<false, true, true> : sdpa_prefill_wide_kernel<false, false, true>;
-    if (gate) return masked ? sdpa_prefill_wide_kernel<true, true> : sdpa_prefill_wide_kernel<true, false>;
-    if (masked) return several ? sdpa_prefill_wide_kernel<false, true, false, true> : sdpa_prefill_wide_kernel<false, true>;
-    return several ? sdpa_prefill_wide_kernel<false, false, false, true> : sdpa_prefill_wide_kernel<false, false>;
+static WideKernel wide_kernel(bool gate, bool masked, bool split, bool several, bool vision) {  // (several: units per CTA pair)
+    if (split) return masked ? sdpa_prefill_wide_kernel<false, true, true> : vision ? sdpa_prefill_wide_kernel<false, false, true, false, true> : sdpa_prefill_wide_kernel<false, false, true>;
+    if (masked) return gate ? sdpa_prefill_wide_kernel<true, true> : several ? sdpa_prefill_wide_kernel<false, true, false, true> : sdpa_prefill_wide_kernel<false, true>;
+    if (vision) return gate ? sdpa_prefill_wide_kernel<true, false, false, false, true> : sdpa_prefill_wide_kernel<false, false, false, true, true>;
+    return gate ? sdpa_prefill_wide_kernel<true, false> : several ? sdpa_prefill_wide_kernel<false, false, false, true> : sdpa_prefill_wide_kernel<false, false>;
 }
 
 // One-time set-up for the current device: status-word address, SM count, and the
@@ -153,7 +153,7 @@ static int device_state(DeviceState** out) {
                 ARC_CUDA(opt_in_smem(chains_kernel(i & 1, i & 2, i & 4), ChainsCfg::SMEM_BYTES));
             }
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel, PrefillCfg::SMEM_BYTES));
-            for (int i = 0; i < 16; ++i) ARC_CUDA(opt_in_smem(wide_kernel(i & 1, i & 2, i & 4, i & 8), WideCfg::SMEM_BYTES));
+            for (int i = 0; i < 32; ++i) ARC_CUDA(opt_in_smem(wide_kernel(i & 1, i & 2, i & 4, i & 8, i & 16), WideCfg::SMEM_BYTES));
             s.wide.pairs = clusters_at_once(sdpa_prefill_wide_kernel<false, false>, 2, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
             for (int parts = 2; parts <= WideRoom::MOST_FOLDED; ++parts)
                 s.wide.folded[parts] = clusters_at_once(sdpa_prefill_wide_kernel<false, false, true>, 2 * parts, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
@@ -580,7 +580,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         }
         // (a cluster is placed inside one GPC, so fewer fit than pairs / parts)
         kp.fold = split && wide_units(p, plan.q_tiles) <= ds->wide.clusters(plan.splits);
-        const WideKernel kernel = wide_kernel(kp.gate != nullptr, masked, split, units > ds->wide.pairs);
+        const WideKernel kernel = wide_kernel(kp.gate != nullptr, masked, split, units > ds->wide.pairs, kp.ids != nullptr);
         ARC_CUDA(launch_dependent(kernel,
                                   dim3((unsigned)(2 * (split || units < ds->wide.pairs ? units : ds->wide.pairs))), dim3(WideCfg::THREADS),
                                   (size_t)WideCfg::SMEM_BYTES, stream, kp.fold ? 2 * plan.splits : 2, tq, tk, tv, to, tg, kp));

@@ -37,9 +37,9 @@ struct WideCfg {
     static constexpr int STAGES = 2;               // of K and of V
     static constexpr int COL_S = 0;                // + 128 * buffer
     static constexpr int COL_O = 256;
-    // first[4] q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp][2]
-    static constexpr int NUM_BARS = 5 + 8 + 2 + 4 + 2 + 4 + 8;
-    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4 + 32;
+    // first[4] q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp][2], next_full next_empty
+    static constexpr int NUM_BARS = 5 + 8 + 2 + 4 + 2 + 4 + 8 + 2;
+    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4 + 2 * 32 + 128 * 4;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
     static constexpr int MOST_FOLDED = 3;  // parts of a split unit that fold themselves as one cluster
     static constexpr int EPILOGUE_WARP = 4, PRODUCER_WARP = 8, ISSUER_WARP = 9;
@@ -159,6 +159,7 @@ __device__ __forceinline__ void add_mask_values(uint32_t tS, const float* mask, 
     tmem_wait_st();
 }
 
+template <bool VISION>
 __device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first, int q_last, int& lo, int& hi) {
     const int off = p.kv_len - p.seq;
     lo = 0;
@@ -166,7 +167,7 @@ __device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first,
     if (p.mask_type == 3) {
         q_last = min(q_last, p.seq - 1);
         // (the span ends are monotone in the row, so the last row decides)
-        const int last_key = p.ids ? vision_end(p, q_last + off) - 1 : min(p.kv_len - 1, q_last + off);
+        const int last_key = VISION ? vision_end(p, q_last + off) - 1 : min(p.kv_len - 1, q_last + off);
         hi = last_key >= 0 ? last_key / WideCfg::BN + 1 : 0;
         if (p.window > 0 && p.window != 0x7fffffff) lo = max(0, q_first + off - p.window + 1) / WideCfg::BN;
     }
@@ -220,12 +221,12 @@ __device__ __forceinline__ WideWork wide_place(const PrefillParams& p, const Wid
     return t;
 }
 
-template <bool MASKED, bool SPLIT>
+template <bool MASKED, bool SPLIT, bool VISION>
 __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int rank, WideWork& t) {
     const int rows = p.head_pair ? WideCfg::BM : 2 * WideCfg::BM;  // tokens of the unit
     const int q0 = p.head_pair ? t.q0 : t.q0 - rank * WideCfg::BM;
     if constexpr (MASKED) masked_blocks(p, q0 >> 7, min(q0 + rows, p.seq + 127) >> 7, t.lo, t.hi);
-    else wide_blocks(p, q0, q0 + rows - 1, t.lo, t.hi);
+    else wide_blocks<VISION>(p, q0, q0 + rows - 1, t.lo, t.hi);
     if (SPLIT) {
         const int lo = t.lo, n = t.hi - t.lo;
         t.lo = lo + n * t.part / p.num_splits;
@@ -245,7 +246,10 @@ __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int ran
 // EARLY (not gated): pairs take several units.  The epilogue then empties the accumulator into registers first (1600 clk), for the
 // next unit's P V to go on; in turns, with the way out of the SM between them, it took 3000.  (2 x 5000 tokens of 16/8 heads,
 // window 512, 103 -> 96 us.  Gated rows wait for sigmoids, not for the way out: taken early they cost calls of short units 8 %.)
-template <bool GATE, bool MASKED, bool SPLIT = false, bool EARLY = false>
+// VISION: causal with vision blocks (p.ids).  Where pairs take several units the next unit's blocks and rows are looked up by warps
+// that wait anyway: between two units the look-up cost the softmax warps 2200 clk and the scores behind it as much.  (1531 tokens of
+// 16/8 heads with three images 24.4 -> 23.2 us.)
+template <bool GATE, bool MASKED, bool SPLIT = false, bool EARLY = false, bool VISION = false>
 __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     sdpa_prefill_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
@@ -276,10 +280,15 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     // complete twice before the epilogue has looked at it, which a parity wait cannot tell from "not yet".
     uint64_t* fin = bars + 21;
     uint64_t* gate_bar = bars + 25;    // [epilogue warp][buffer] own CTA
+    uint64_t* next_full = bars + 33;   // own CTA: the epilogue warps have looked up the next unit's vision blocks
+    uint64_t* next_empty = bars + 34;  // the softmax warps have taken them
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
     float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [unit & 3][row] row sum
     WideWork* first_unit = reinterpret_cast<WideWork*>(fin_vals + 4 * 128);
+    WideWork* next_place = first_unit + 1;
+    int* next_end = reinterpret_cast<int*>(fin_vals + 4 * 128 + 16);  // [row] first key the row does not see
+    static_assert(sizeof(WideWork) <= 32, "two units in 64 bytes");
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
@@ -311,16 +320,18 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         }
         mbar_init(o_full, 1);
         mbar_init(o_empty, 8);
+        mbar_init(next_full, 4);
+        mbar_init(next_empty, 4);
         fence_mbar_init();
     }
     if (warp == C::PRODUCER_WARP) tmem_alloc_pair(tmem_slot, 512);
     // One warp finds the first unit for all, beside the tensor memory's allocation; its divisions, and the code that every role
     // would fetch for them, took 2500 clk between the kernel's release and its first load.
-    const bool blocks_in_memory = MASKED || p.ids;
+    constexpr bool blocks_in_memory = MASKED || VISION;
     WideWork w_first{};
     if (warp == C::EPILOGUE_WARP) {
         w_first = wide_place<SPLIT>(p, WideCursor(p), rank);
-        if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
+        if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT, VISION>(p, rank, w_first);
         if (lane == 0) *first_unit = w_first;
     }
     cluster_sync_all();  // both CTAs' barriers exist before anyone arrives on the other's
@@ -363,7 +374,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     if (warp == C::PRODUCER_WARP) {
         w_first = *first_unit;
         if (blocks_in_memory) {
-            wide_find_blocks<MASKED, SPLIT>(p, rank, w_first);
+            wide_find_blocks<MASKED, SPLIT, VISION>(p, rank, w_first);
             if (lane == 0) *first_unit = w_first;
         }
         __syncwarp();
@@ -385,7 +396,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     auto unit_at = [&](const WideCursor& cur) {
         if (SPLIT || cur.i == 0) return *first_unit;
         WideWork w = wide_place<SPLIT>(p, cur, rank);
-        wide_find_blocks<MASKED, SPLIT>(p, rank, w);
+        wide_find_blocks<MASKED, SPLIT, VISION>(p, rank, w);
         return w;
     };
 
@@ -446,10 +457,20 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x100u);
             return false;
         };
+        // (vision blocks: the next unit's are looked up while this one's first blocks are worked on)
         WideCursor cur(p);
+        WideWork w_next{};
+        auto look_ahead = [&]() {
+            WideCursor after = cur;
+            after.advance(p);
+            if (after.w < total) w_next = unit_at(after);
+        };
         for (; ok && cur.w < total; cur.advance(p)) {
-            const WideWork w = unit_at(cur);
-            if (w.hi == w.lo) continue;
+            const WideWork w = VISION && cur.i > 0 ? w_next : unit_at(cur);
+            if (w.hi == w.lo) {
+                if (VISION) look_ahead();
+                continue;
+            }
             const int have = n == 0 && cur.i == 0 ? ahead_k : 0;  // (asked for above)
             if (have) {
                 gk = ahead_k, gv = ahead_v;
@@ -464,13 +485,17 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             ++n;
             // in the order of use: K one block ahead of V
             for (int j = w.lo; ok && j < w.hi; ++j) {
-                if (have && j == w.lo) continue;  // (V of the first block, K of the second)
+                if (have && j == w.lo) {  // (V of the first block, K of the second)
+                    if (VISION) look_ahead();
+                    continue;
+                }
                 if (j + 1 < w.hi) {
                     ok = free_stage(k_empty, gk);
                     if (ok) load_k(w, j + 1, gk++ & 1);
                 }
                 if (ok) ok = free_stage(v_empty, gv);
                 if (ok) load_v(w, j, gv++ & 1);
+                if (VISION && j == w.lo) look_ahead();
             }
         }
     } else if (warp == C::ISSUER_WARP) {
@@ -535,11 +560,12 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             bool have = next_unit(w);
             if (have) ok = scores(w, w.lo);
             while (have && ok) {
-                const bool have_next = next_unit(wn);
+                bool have_next = false;
                 for (int j = w.lo; j < w.hi; ++j) {
                     // the next block's scores first: they run while the softmax warps work on this block's
                     if (j + 1 < w.hi) ok = scores(w, j + 1);
-                    else if (have_next) ok = scores(wn, wn.lo);
+                    if (j == w.lo) have_next = next_unit(wn);
+                    if (ok && j + 1 == w.hi && have_next) ok = scores(wn, wn.lo);
                     if (!ok) break;
                     const int st = gp & 1;
                     const uint32_t par = (gp >> 1) & 1;
@@ -590,6 +616,21 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         WideCursor cur(p);
         for (; cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
+            if (VISION) {  // for the softmax warps, whose look-up would come between two units
+                WideCursor after = cur;
+                after.advance(p);
+                if (after.w < total) {
+                    const WideWork wn = unit_at(after);
+                    const int tn = wn.q0 + quarter * 32 + lane, end = vision_ends(p, tn + p.kv_len - p.seq, tn < p.seq);
+                    if (cur.i > 0 && !mbar_wait_warp<2>(next_empty, (cur.i - 1) & 1)) {
+                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, 0x500u);
+                        break;
+                    }
+                    next_end[r] = end;
+                    if (threadIdx.x == C::EPILOGUE_WARP * 32) *next_place = wn;
+                    mbar_arrive_warp(next_full);
+                }
+            }
             const int t0 = w.q0 + quarter * 32, t = t0 + lane;
             const bool store = t < p.seq, warp_store = t0 < p.seq;  // this row / some row of the warp is stored
             const long long row = ((long long)w.b * p.seq + t) * p.nq + w.h;
@@ -719,7 +760,17 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         uint32_t s0[32], s1[32], s2[32], s3[32];  // the row's 128 scores of the current block
         WideCursor cur(p);
         for (; ok && cur.w < total; cur.advance(p)) {
-            const WideWork w = unit_at(cur);
+            const bool looked_up = VISION && cur.i > 0;
+            int row_end = 0;
+            if (looked_up) {
+                if (!mbar_wait_inline(next_full, (cur.i - 1) & 1)) {
+                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x700u);
+                    break;
+                }
+                row_end = next_end[r];
+            }
+            const WideWork w = looked_up ? *next_place : unit_at(cur);
+            if (looked_up) mbar_arrive_warp(next_empty);
             if (w.hi == w.lo) {
                 if (SPLIT) break;  // (its only one; with the place read again below, nothing is spilled: a canvas step 17.9 us, 17.6 so)
                 continue;
@@ -729,7 +780,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             if (causal) {
                 const int diag = t + off;
                 row_hi = min(max(diag + 1, 0), p.kv_len);
-                if (p.ids) row_hi = vision_ends(p, diag, t < p.seq);
+                if (VISION) row_hi = looked_up ? row_end : vision_ends(p, diag, t < p.seq);
                 if (windowed) row_lo = max(0, diag - p.window + 1);
                 if (row_lo > row_hi) row_lo = row_hi;
             }
