@@ -545,8 +545,8 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
             kp.mask_blocks = (p->kv_len + 127) / 128;
             uint4* bits = reinterpret_cast<uint4*>(static_cast<unsigned char*>(p->workspace) + plan.ws_bytes);
             uint32_t* cls = reinterpret_cast<uint32_t*>(bits + (size_t)plan.q_tiles * kp.mask_blocks * 128);
-            ARC_CUDA(launch_dependent(mask_scan_kernel, dim3((unsigned)kp.mask_blocks, (unsigned)plan.q_tiles * 4), dim3(256), 0, stream, 1,
-                                      kp.mask, (int)p->seq, (int)p->kv_len, kp.mask_blocks, cls, bits));
+            ARC_CUDA(launch_dependent(mask_scan_kernel, dim3((unsigned)kp.mask_blocks, (unsigned)plan.q_tiles * 4), dim3(512), 0, stream, 1,
+                                      kp.mask, (int)p->seq, (int)p->kv_len, kp.mask_blocks, cls, reinterpret_cast<uint32_t*>(bits)));
             g_launches.fetch_add(1, std::memory_order_relaxed);
             kp.mask_bits = bits;
             kp.mask_class = cls;

@@ -260,6 +260,42 @@ def test_vision_blocks_longer_than_a_search_step():
     assert ops.device_status() == (0, 0)
 
 
+@pytest.mark.parametrize("batch,seq,kv,nq,nkv,window,gate,vision", [
+    (1, 1664, 1664, 24, 4, 0, False, False),  # 156 units on 74 pairs: two or three each, the longest to those with two
+    (1, 1024, 2400, 24, 4, 0, True, False),   # 96: one or two, gated
+    (3, 300, 2000, 27, 9, 0, False, False),   # odd groups of 256 tokens, 162
+    (1, 3000, 3000, 48, 8, 150, False, False),  # a window, 576, as long as each other but for the first
+    (1, 1500, 1500, 24, 4, 400, False, True),   # vision blocks, looked up a unit ahead
+    (1, 900, 500, 48, 8, 0, False, True),       # and tiles that see nothing between others
+    (1, 900, 500, 48, 8, 0, True, True),        # gated
+])
+def test_several_units_a_pair(batch, seq, kv, nq, nkv, window, gate, vision):
+    """More units than pairs: the accumulator freed ahead of the output, the two kinds of pairs, the look-up of the next unit."""
+    from arcaine_b200 import ops
+    ops.clear_device_status()
+    hd, win = 256, window or oracle.INT_MAX
+    q, k, v, g = (seeded_bf16(batch, n, h, hd, seed=110 + i) for i, (n, h) in enumerate([(seq, nq), (kv, nkv), (kv, nkv), (seq, nq)]))
+    qd, kd, vd, copy = q.cuda(), k.cuda(), v.cuda(), torch.empty(batch, seq, nq, hd, dtype=torch.bfloat16, device="cuda")
+    ids = torch.full((seq,), -1, dtype=torch.int32)  # (by position of the query; key j is position j + seq - kv)
+    base = max(0, seq - kv)
+    for i, (a, b) in enumerate([(10, 90), (127, 129), (200, 360), (400, 499)]):
+        ids[base + a:base + b] = i
+    run = lambda: ops.sdpa_prefill(qd, kd, vd, scale=hd ** -0.5, mask_type=3, window=win, gate=g.cuda() if gate else None, num_splits=1,  # noqa: E731
+                                   out_copies=torch.tensor([copy.data_ptr()], device="cuda"), block_ids=ids.cuda() if vision else None,
+                                   block_ids_offset=seq - kv if vision else 0)
+    out = run()
+    assert torch.equal(copy, out)
+    for _ in range(5):
+        assert torch.equal(run(), out)
+    assert ops.device_status() == (0, 0)
+    mask = oracle.fill_causal_mask_with_block_ids(ids.numpy(), seq, kv, 0, win) if vision else None
+    for b in range(batch):
+        rows = sorted({t * nq + h for t in (0, 127, 128, 300, 459, seq // 2, seq - 129, seq - 1) if t < seq for h in (0, 1, nq // 2, nq - 1)})
+        want = oracle.sdpa_f32(q[b], k[b], v[b], scale=hd ** -0.5, mask_type=1 if vision else 3, window=win, mask=mask, rows=rows,
+                               gate=g[b] if gate else None)
+        assert_close(out[b].reshape(-1, hd)[rows], want[1].float() if gate else want[0], f"sequence {b}")
+
+
 @pytest.mark.parametrize("parts", [2, 3, 4, 8])
 @pytest.mark.parametrize("batch,seq,kv,nq,nkv,window", [
     (1, 256, 1100, 8, 4, oracle.INT_MAX),  # two row tiles of pairs of heads, the last key block ragged
