@@ -113,6 +113,9 @@ __device__ __forceinline__ void consumer_sync(int consumer_warps) {
 // as they are, weights worked out by eight lanes a row, rolled loops and stores that count themselves on an mbarrier of the CTA they
 // go to (st.async) take half of that (us): that call 6.2 -> 5.3, 1001 keys 6.7 -> 5.5, 20 sequences of 780 keys 20.3 -> 18.4, 64 of
 // 100 to 512 keys, 16/2 heads of 128, 9.0 -> 8.1, twelve of up to 6000 12.3 -> 11.8.
+// A CTA's first keys are asked for while the lengths are: they do not depend on them (1630 clk to the lengths when they are on the
+// device; us: 16 sequences of 500 keys, 8/4 heads of 128, 6.6 -> 5.9, 32 of 64 to 400, 24/4 of 256, 12.9 -> 11.9, twelve of up to 6000,
+// 16/2 of 128, 11.8 -> 11.2, one token over 513 keys 5.34 -> 5.1).  The scores ahead of V, on a barrier of its own, brought nothing.
 // EVEN (of CLUSTER): a power of two of CTAs, all of which finish columns.  As a case of the other instance these calls were 0.1
 // to 0.2 us slower (one token of 24/4 heads over 256 / 1001 keys 6.31 / 6.96 us, 6.16 / 6.76 so; 16 sequences of 500 keys,
 // 8/4 heads of 128: 7.92 and 7.70).
@@ -171,13 +174,16 @@ __global__ void __launch_bounds__(288, 1)
     }
     long long g0 = 0, g1 = 0;  // this CTA's keys, counted over the sequences laid end to end (CLUSTER: of its own sequence)
     int b_first = 0, my_len = 0;
+    // CLUSTER: a CTA's first step begins at key blockIdx.x * tk, whatever the length, so that its keys are asked for before the length
+    // has been looked at; what is left behind the first steps of all is divided evenly.
+    int more_keys = 0, more_at = 0;
     bool work = true;
     auto find_share = [&]() {
         if constexpr (CLUSTER) {
             b_first = blockIdx.z;
-            const int per = ((my_len + p.ncta - 1) / p.ncta + 15) / 16 * 16;
-            g0 = (long long)blockIdx.x * per;
-            g1 = min((long long)my_len, g0 + per);
+            const int rest = max(0, my_len - p.ncta * tk), per = ((rest + p.ncta - 1) / p.ncta + 15) / 16 * 16, at = min(rest, (int)blockIdx.x * per);
+            more_keys = min(rest, at + per) - at;
+            more_at = p.ncta * tk + at;
         } else {
             const long long total = cum[p.batch];
             const long long per = share_size(total, p.ncta, tk);
@@ -199,10 +205,30 @@ __global__ void __launch_bounds__(288, 1)
         find_share();
     }
     if (CLUSTER) cluster_sync_all();  // every CTA runs: its shared memory may be written
+    // The producer's copies of a step.
+    auto ask = [&](int st, int row) {
+        // A stage always carries tk full rows: rows past the segment end
+        // are masked by the consumers, rows past the cache end read as zero.
+        if (lane == 0) mbar_arrive_expect_tx(&full[st], (uint32_t)stage_bytes);
+        __syncwarp();
+        uint8_t* dst = stage_base + (size_t)st * stage_bytes;
+        for (int c = lane; c < 2 * nchunks; c += 32) {
+            const int is_v = c >= nchunks;
+            const int cc = c - is_v * nchunks;
+            tma_load_2d(dst + (size_t)is_v * tile_bytes + (size_t)cc * chunk_bytes, is_v ? &tm_v : &tm_k,
+                        &full[st], head0 * HD + cc * 64, row);
+        }
+    };
     // Up to here nothing depends on the kernels in front; everything below may.
     grid_dependency_wait();
+    int asked = 0;
+    if (CLUSTER && warp == ncw && !p.kv_row_offset) {
+        ask(0, (int)((long long)blockIdx.z * p.kv_stride_b) + (int)blockIdx.x * tk);
+        asked = 1;
+    }
     grid_launch_dependents();  // the merge kernel may be scheduled now; it waits for this grid before reading
     const uint32_t fault = threadIdx.x == 0 ? *reinterpret_cast<volatile uint32_t*>(p.fault) : 0u;  // (set: no result is written)
+    long long own_row = CLUSTER ? (long long)blockIdx.z * p.kv_stride_b : 0ll;  // first row of the cluster's sequence
     if (!known) {
         // The status word, the lengths and the row offsets are asked for together: each is a trip to L2 or HBM.
         // Lengths and row offsets live on the device, so this is where they can be checked: a sequence that reaches past the
@@ -210,6 +236,8 @@ __global__ void __launch_bounds__(288, 1)
         // launch with a status instead of a wrong result.  Every CTA checks all sequences and so none of them works.
         // (The first warp checks and adds up what it has asked for once: a second look was a second trip.)
         bool bad = fault != 0u;
+        const int own_len = CLUSTER && p.kv_len ? p.kv_len[blockIdx.z] : p.kv_len_uniform;
+        if (CLUSTER && p.kv_row_offset) own_row = p.kv_row_offset[blockIdx.z];
         auto checked_len = [&](int b) {
             const int len = p.kv_len ? p.kv_len[b] : p.kv_len_uniform;
             const long long row0 = p.kv_row_offset ? p.kv_row_offset[b] : (long long)b * p.kv_stride_b;
@@ -222,11 +250,12 @@ __global__ void __launch_bounds__(288, 1)
         if (!CLUSTER && threadIdx.x < 32) build_len_prefix(p.batch, cum, checked_len);
         if (CLUSTER)
             for (int b = threadIdx.x; b < p.batch; b += blockDim.x) checked_len(b);
-        if (CLUSTER) my_len = max(0, p.kv_len ? p.kv_len[blockIdx.z] : p.kv_len_uniform);
         work = !__syncthreads_or(bad);
+        if (CLUSTER && work) my_len = max(0, own_len);
         if (work) find_share();
     }
     if (!CLUSTER && g0 >= g1) return;
+    const bool no_step = CLUSTER && p.kv_row_offset && my_len <= (int)blockIdx.x * tk;  // (nothing has been asked for, and there are no keys)
     // keys before sequence b / up to its end, in the count g0 and g1 use
     auto seq_begin = [&](int b) { return CLUSTER ? 0ll : cum[b]; };
     auto seq_end = [&](int b) { return CLUSTER ? (long long)my_len : cum[b + 1]; };
@@ -238,7 +267,18 @@ __global__ void __launch_bounds__(288, 1)
         bool ok = true;
         int b = b_first;
         long long g = g0;
-        while (ok && g < g1) {
+        if constexpr (CLUSTER) {
+            const int steps = no_step ? 0 : 1 + (more_keys + tk - 1) / tk;
+            for (it = asked; it < steps; ++it) {
+                const int st = it % p.stages;
+                if (it >= p.stages && !mbar_wait_warp(&empty[st], ((it / p.stages) - 1) & 1)) {
+                    if (lane == 0) report_fault(p.fault, FAULT_WAIT_EMPTY, it);
+                    break;
+                }
+                ask(st, (int)own_row + (it == 0 ? (int)blockIdx.x * tk : more_at + (it - 1) * tk));
+            }
+        }
+        while (!CLUSTER && ok && g < g1) {
             while (seq_end(b) <= g) ++b;
             const long long seg_end = min(g1, seq_end(b));
             const long long row0 = (p.kv_row_offset ? p.kv_row_offset[b] : (long long)b * p.kv_stride_b) + (g - seq_begin(b));
@@ -250,18 +290,7 @@ __global__ void __launch_bounds__(288, 1)
                     ok = false;
                     break;
                 }
-                // A stage always carries tk full rows: rows past the segment end
-                // are masked by the consumers, rows past the cache end read as zero.
-                if (lane == 0) mbar_arrive_expect_tx(&full[st], (uint32_t)stage_bytes);
-                __syncwarp();
-                uint8_t* dst = stage_base + (size_t)st * stage_bytes;
-                const int row = (int)(row0 + k0);
-                for (int c = lane; c < 2 * nchunks; c += 32) {
-                    const int is_v = c >= nchunks;
-                    const int cc = c - is_v * nchunks;
-                    tma_load_2d(dst + (size_t)is_v * tile_bytes + (size_t)cc * chunk_bytes, is_v ? &tm_v : &tm_k,
-                                &full[st], head0 * HD + cc * 64, row);
-                }
+                ask(st, (int)(row0 + k0));
             }
             g = seg_end;
         }
@@ -288,8 +317,8 @@ __global__ void __launch_bounds__(288, 1)
         long long g = g0;
         while (CLUSTER || (ok && g < g1)) {  // (CLUSTER: once, keys or not)
             while (!CLUSTER && seq_end(b) <= g) ++b;
-            const long long seg_end = CLUSTER ? max(g0, g1) : min(g1, seq_end(b));
-            const int seg_keys = (int)(seg_end - g);
+            const long long seg_end = CLUSTER ? 0 : min(g1, seq_end(b));
+            const int seg_keys = CLUSTER ? (no_step ? 0 : tk + more_keys) : (int)(seg_end - g);  // (CLUSTER: a first step, full or not)
 
             // Q^T fragments (B operand, hd x 8 heads) for this head's GQA group.
             uint32_t qf[NT][HD / 16][2];
@@ -321,7 +350,7 @@ __global__ void __launch_bounds__(288, 1)
                     ok = false;
                     break;
                 }
-                const int nk = min(tk, seg_keys - k0);
+                const int nk = CLUSTER && k0 == 0 ? min(max(my_len - (int)blockIdx.x * tk, 0), tk) : min(tk, seg_keys - k0);
                 const int nvalid = min(16, nk - slice * 16);  // keys of this warp's slice
                 if (nvalid > 0) {
                     // Swizzled addressing: 16-byte unit u of row r sits at unit u ^ (r & 7).
