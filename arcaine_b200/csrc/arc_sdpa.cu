@@ -116,11 +116,13 @@ static ChainsKernel chains_kernel(bool gate, bool vision, bool masked) {
 }
 
 using WideKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, PrefillParams);
-static WideKernel wide_kernel(bool gate, bool masked, bool split, bool several, bool vision) {  // (several: units per CTA pair)
-    if (split) return masked ? sdpa_prefill_wide_kernel<false, true, true> : vision ? sdpa_prefill_wide_kernel<false, false, true, false, true> : sdpa_prefill_wide_kernel<false, false, true>;
-    if (masked) return gate ? sdpa_prefill_wide_kernel<true, true> : several ? sdpa_prefill_wide_kernel<false, true, false, true> : sdpa_prefill_wide_kernel<false, true>;
-    if (vision) return gate ? sdpa_prefill_wide_kernel<true, false, false, false, true> : sdpa_prefill_wide_kernel<false, false, false, true, true>;
-    return gate ? sdpa_prefill_wide_kernel<true, false> : several ? sdpa_prefill_wide_kernel<false, false, false, true> : sdpa_prefill_wide_kernel<false, false>;
+static WideKernel wide_kernel(bool gate, bool masked, int split, bool several, bool vision) {  // (several: units per CTA pair)
+    if (split == 2 && gate) return masked ? sdpa_prefill_wide_kernel<true, true, 2> : vision ? sdpa_prefill_wide_kernel<true, false, 2, false, true> : sdpa_prefill_wide_kernel<true, false, 2>;
+    if (split == 2) return masked ? sdpa_prefill_wide_kernel<false, true, 2> : vision ? sdpa_prefill_wide_kernel<false, false, 2, false, true> : sdpa_prefill_wide_kernel<false, false, 2>;
+    if (split == 1) return masked ? sdpa_prefill_wide_kernel<false, true, 1> : vision ? sdpa_prefill_wide_kernel<false, false, 1, false, true> : sdpa_prefill_wide_kernel<false, false, 1>;
+    if (masked) return gate ? sdpa_prefill_wide_kernel<true, true> : several ? sdpa_prefill_wide_kernel<false, true, 0, true> : sdpa_prefill_wide_kernel<false, true>;
+    if (vision) return gate ? sdpa_prefill_wide_kernel<true, false, 0, false, true> : sdpa_prefill_wide_kernel<false, false, 0, true, true>;
+    return gate ? sdpa_prefill_wide_kernel<true, false> : several ? sdpa_prefill_wide_kernel<false, false, 0, true> : sdpa_prefill_wide_kernel<false, false>;
 }
 
 // One-time set-up for the current device: status-word address, SM count, and the
@@ -153,10 +155,10 @@ static int device_state(DeviceState** out) {
                 ARC_CUDA(opt_in_smem(chains_kernel(i & 1, i & 2, i & 4), ChainsCfg::SMEM_BYTES));
             }
             ARC_CUDA(opt_in_smem(sdpa_prefill_kernel, PrefillCfg::SMEM_BYTES));
-            for (int i = 0; i < 32; ++i) ARC_CUDA(opt_in_smem(wide_kernel(i & 1, i & 2, i & 4, i & 8, i & 16), WideCfg::SMEM_BYTES));
+            for (int i = 0; i < 48; ++i) ARC_CUDA(opt_in_smem(wide_kernel(i & 1, i & 2, i / 16, i & 4, i & 8), WideCfg::SMEM_BYTES));
             s.wide.pairs = clusters_at_once(sdpa_prefill_wide_kernel<false, false>, 2, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
             for (int parts = 2; parts <= WideRoom::MOST_FOLDED; ++parts)
-                s.wide.folded[parts] = clusters_at_once(sdpa_prefill_wide_kernel<false, false, true>, 2 * parts, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
+                s.wide.folded[parts] = clusters_at_once(sdpa_prefill_wide_kernel<false, false, 2>, 2 * parts, s.sm_count, WideCfg::THREADS, WideCfg::SMEM_BYTES);
             if (s.wide.pairs < 1) {
                 std::snprintf(g_last_error, sizeof(g_last_error), "the device cannot hold a CTA pair of the prefill kernel");
                 return ARC_ERR_CUDA;
@@ -277,9 +279,9 @@ static int tile_key_blocks(const arc_sdpa_prefill_params* p, int qt) {
 }
 
 // Head dim 256: units of the CTA pairs' list, and how many parts the key range of each is worth when the units alone
-// would leave pairs idle.  Measured (us): a key block of a pair 1.13; records and fold 3 + 0.04 per pair in a cluster, 2.5 +
+// would leave pairs idle.  Measured (us): a key block of a pair 1.13; records and fold 1.8 (gated 2.7) + 0.04 per pair in a cluster, 2.5 +
 // 0.06 per pair with a merge launch (every pair writes its 256 rows as f32, 32 bytes per clk and SM), whatever the number
-// of parts.  (256 queries of 16 heads over 2304 keys: 26.7 us whole, 19.1 in three parts, 19.6 in four; of 8 heads 26.2,
+// of parts.  (256 queries of 16 heads over 2304 keys: 26.7 us whole, 15.7 in three parts, 19.6 in four; of 8 heads 26.2,
 // 15.6 in six.)
 static long long wide_units(const arc_sdpa_prefill_params* p, int q_tiles) {
     const bool head_pair = ((p->nq / p->nkv) & 1) == 0;
@@ -298,7 +300,7 @@ static int choose_wide_splits(const arc_sdpa_prefill_params* p, int q_tiles, con
     int best = 1;
     double least = 1.13 * most;
     for (int s = 2; s <= 8 && s <= most && units * s <= room.pairs; ++s) {
-        const double t = 1.13 * ((most + s - 1) / s) + (units <= room.clusters(s) ? 3.0 + 0.04 * (units * s) : 2.5 + 0.06 * (units * s));
+        const double t = 1.13 * ((most + s - 1) / s) + (units <= room.clusters(s) ? (p->gate ? 2.7 : 1.8) + 0.04 * (units * s) : 2.5 + 0.06 * (units * s));
         if (t < least) least = t, best = s;
     }
     return best;
@@ -579,13 +581,13 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
             return rc;
         }
         // (a cluster is placed inside one GPC, so fewer fit than pairs / parts)
-        kp.fold = split && wide_units(p, plan.q_tiles) <= ds->wide.clusters(plan.splits);
-        const WideKernel kernel = wide_kernel(kp.gate != nullptr, masked, split, units > ds->wide.pairs, kp.ids != nullptr);
+        const bool fold = split && wide_units(p, plan.q_tiles) <= ds->wide.clusters(plan.splits);
+        const WideKernel kernel = wide_kernel(kp.gate != nullptr, masked, fold ? 2 : split ? 1 : 0, units > ds->wide.pairs, kp.ids != nullptr);
         ARC_CUDA(launch_dependent(kernel,
                                   dim3((unsigned)(2 * (split || units < ds->wide.pairs ? units : ds->wide.pairs))), dim3(WideCfg::THREADS),
-                                  (size_t)WideCfg::SMEM_BYTES, stream, kp.fold ? 2 * plan.splits : 2, tq, tk, tv, to, tg, kp));
+                                  (size_t)WideCfg::SMEM_BYTES, stream, fold ? 2 * plan.splits : 2, tq, tk, tv, to, tg, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);
-        return split && !kp.fold ? launch_fold<HD>(p, plan, kp, stream) : ARC_OK;
+        return split && !fold ? launch_fold<HD>(p, plan, kp, stream) : ARC_OK;
     }
 
     kp.q_tiles = plan.q_tiles;

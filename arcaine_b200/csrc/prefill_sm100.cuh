@@ -62,7 +62,6 @@ struct PrefillParams {
     const uint32_t* mask_class;  // [row tile][key block]: a byte per 32 rows, MASK_* bits
     const uint4* mask_bits;      // [row tile][key block][row]: one bit per key, set where the mask is 0
     int mask_blocks;
-    int fold;        // prefill_wide_sm100.cuh: the parts of a unit are the pairs of one cluster, which folds them itself
     const int* ids;  // vision-block ids, ids[j] that of key j
 };
 

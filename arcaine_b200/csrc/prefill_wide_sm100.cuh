@@ -19,6 +19,8 @@
 //
 // Masks, lazy rescaling, bounded waits and the status word are as in prefill_pair_sm100.cuh; P is written over the scores.
 #pragma once
+#include <type_traits>
+
 #include "decode_sm100.cuh"
 #include "prefill_pair_sm100.cuh"
 
@@ -49,7 +51,7 @@ struct WideCfg {
 // One unit of the pair: this CTA's tile, and the key blocks [lo, hi) the pair walks (the union over both tiles).
 struct WideWork {
     int q0, h, b, kvh, lo, hi;
-    int part;  // SPLIT: which part of the key range
+    int part;  // of the key range
 };
 
 // ---------------------------------------------------------------------------
@@ -252,19 +254,20 @@ __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int ran
 // MASKED: with an additive mask, as mask_scan_kernel has read it.  (With SPLIT: few queries over a long cache.  16 of 8 heads
 // over 32768 keys take 299 us as whole units and 59 in parts; 64 over 4096 keys 45 and 18.)
 // SPLIT: a unit is one of num_splits parts of the key blocks, one unit per pair, for calls whose tiles would leave most
-// pairs idle.  The part's normalised rows go to the partial records as f32 with their log-sum-exp.  Two or three parts
-// are the pairs of one cluster (p.fold): each CTA stores only the rows the other parts' CTAs fold, and after a cluster
-// barrier folds its own share of rows; more parts are folded by sdpa_uniform_merge_kernel.  The rows pass through L2:
+// pairs idle.  The part's normalised rows go to the partial records as f32 with their log-sum-exp.  SPLIT 2: two or three parts
+// are the pairs of one cluster; each CTA stores only the columns the other parts' CTAs finish, and after a cluster
+// barrier finishes its own columns.  SPLIT 1: more parts are folded by sdpa_uniform_merge_kernel.  The values pass through L2:
 // read out of the other CTAs' shared memory, 11 bytes per clk and SM, the fold took 5 us.  Every instruction here runs
-// once per launch and is fetched cold, 50 clk per 128 bytes of code, so the loops are rolled: with five rows unrolled
-// the fold itself took 8700 clk.
+// once per launch and is fetched cold, 50 clk per 128 bytes of code, so there are few: with rows divided instead of columns, which
+// had to go through shared memory on either side, 13000 clk passed from the last P V to the end  (us: 256 queries of 16 heads over
+// 2304 keys 18.0 -> 15.7, 512 over 2560 23.5 -> 20.7, 512 of 8 heads over 1512 15.5 -> 13.1.)
 // EARLY (not gated): pairs take several units.  The epilogue then empties the accumulator into registers first (1600 clk), for the
 // next unit's P V to go on; in turns, with the way out of the SM between them, it took 3000.  (2 x 5000 tokens of 16/8 heads,
 // window 512, 103 -> 96 us.  Gated rows wait for sigmoids, not for the way out: taken early they cost calls of short units 8 %.)
 // VISION: causal with vision blocks (p.ids).  Where pairs take several units the next unit's blocks and rows are looked up by warps
 // that wait anyway: between two units the look-up cost the softmax warps 2200 clk and the scores behind it as much.  (1531 tokens of
 // 16/8 heads with three images 24.4 -> 23.2 us.)
-template <bool GATE, bool MASKED, bool SPLIT = false, bool EARLY = false, bool VISION = false>
+template <bool GATE, bool MASKED, int SPLIT = 0, bool EARLY = false, bool VISION = false>
 __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     sdpa_prefill_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
@@ -345,8 +348,8 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     constexpr bool blocks_in_memory = MASKED || VISION;
     WideWork w_first{};
     if (warp == C::EPILOGUE_WARP) {
-        w_first = wide_place<SPLIT>(p, WideCursor(p), rank);
-        if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT, VISION>(p, rank, w_first);
+        w_first = wide_place<SPLIT != 0>(p, WideCursor(p), rank);
+        if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT != 0, VISION>(p, rank, w_first);
         if (lane == 0) *first_unit = w_first;
     }
     cluster_sync_all();  // both CTAs' barriers exist before anyone arrives on the other's
@@ -389,7 +392,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     if (warp == C::PRODUCER_WARP) {
         w_first = *first_unit;
         if (blocks_in_memory) {
-            wide_find_blocks<MASKED, SPLIT, VISION>(p, rank, w_first);
+            wide_find_blocks<MASKED, SPLIT != 0, VISION>(p, rank, w_first);
             if (lane == 0) *first_unit = w_first;
         }
         __syncwarp();
@@ -410,16 +413,15 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     const int total = *abort_slot ? 0 : (int)(blockIdx.x >> 1) < p.few ? p.few_end : p.total_tiles;  // a status is set: walk an empty list
     auto unit_at = [&](const WideCursor& cur) {
         if (SPLIT || cur.i == 0) return *first_unit;
-        WideWork w = wide_place<SPLIT>(p, cur, rank);
-        wide_find_blocks<MASKED, SPLIT, VISION>(p, rank, w);
+        WideWork w = wide_place<SPLIT != 0>(p, cur, rank);
+        wide_find_blocks<MASKED, SPLIT != 0, VISION>(p, rank, w);
         return w;
     };
 
-    // SPLIT: columns [col, col + 128) of the part's rows into shared memory, where Q, K and V are through: the f32 tile as
+    // SPLIT 1: columns [col, col + 128) of the part's rows into shared memory, where Q, K and V are through: the f32 tile as
     // [32 columns][row], 128-byte swizzle; and from there, a row of 512 bytes an instruction, to the records.  (By TMA, in
     // boxes of 8 rows x 32 columns, the tile took 4000 clk.)
     constexpr int PART_CHUNK = 128 * 128;
-    auto own_row0 = [&](int part) { return (part * 16 + p.num_splits - 1) / p.num_splits * 8; };  // rows a part's CTA folds
     auto store_part = [&](const WideWork& w, int quarter, float row_l, int col) {
         if (!mbar_wait_warp<2>(o_full, 0)) {
             if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x700u);
@@ -441,13 +443,11 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                              "f"(__uint_as_float(v[4 * i + 2]) * inv), "f"(__uint_as_float(v[4 * i + 3]) * inv) : "memory");
         }
         __syncwarp();
-        const int keep0 = p.fold ? own_row0(w.part) : 128, keep1 = p.fold ? own_row0(w.part + 1) : 128;
         const int end = min(quarter * 32 + 32, p.seq - w.q0);
         const long long step_t = (long long)p.nq * HD;
         float* dst = p.part_o + ((((long long)w.part * p.batch + w.b) * p.seq + w.q0) * p.nq + w.h) * HD + col + lane * 4;
 #pragma unroll 1
-        for (int i0 = quarter * 32; i0 < end; i0 += 8) {  // (shares begin at multiples of eight rows)
-            if (i0 >= keep0 && i0 < keep1) continue;
+        for (int i0 = quarter * 32; i0 < end; i0 += 8) {
             float4 v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i)
@@ -455,6 +455,36 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
 #pragma unroll
             for (int i = 0; i < 8; ++i)
                 if (i0 + i < end) *reinterpret_cast<float4*>(dst + (i0 + i) * step_t) = v[i];
+        }
+    };
+
+    // SPLIT 2: the parts of a unit divide the columns, 16 at a time, among their CTAs of the same rows: part u finishes the groups
+    // [group0(u), group0(u + 1)) of all 128.  A record is [four columns][row], so that a thread, which is a row, stores what the others
+    // finish straight from tensor memory and loads what it finishes straight into registers, 512 bytes a warp.
+    constexpr int GROUP = 16, GROUPS = HD / GROUP;
+    auto group0 = [&](int part) { return part * GROUPS / p.num_splits; };
+    auto record_row = [&](const WideWork& w, int part) { return (((long long)part * p.batch + w.b) * p.nq + w.h) * p.seq + w.q0; };
+    auto send_part = [&](const WideWork& w, int quarter, float row_l, int half) {  // of columns [128 half, 128 half + 128)
+        if (!mbar_wait_warp<2>(o_full, 0)) {
+            if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x700u);
+            return;
+        }
+        tc_fence_after_sync();
+        const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
+        const uint32_t tO = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::COL_O;
+        const int g0 = group0(w.part), g1 = group0(w.part + 1), row = quarter * 32 + lane, rows = min(128, p.seq - w.q0);
+        float4* dst = reinterpret_cast<float4*>(p.part_o + record_row(w, w.part) * HD) + row;
+#pragma unroll 1
+        for (int g = half * (GROUPS / 2); g < (half + 1) * (GROUPS / 2); g += 2) {
+            const bool first = g < g0 || g >= g1, second = g + 1 < g0 || g + 1 >= g1;  // (a group that another part finishes)
+            if (!first && !second) continue;
+            uint32_t v[32];
+            tmem_ld32(tO + g * GROUP, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (row < rows && (i < 4 ? first : second))
+                    dst[(long long)(g * 4 + i) * rows] = make_float4(__uint_as_float(v[4 * i]) * inv, __uint_as_float(v[4 * i + 1]) * inv, __uint_as_float(v[4 * i + 2]) * inv, __uint_as_float(v[4 * i + 3]) * inv);
         }
     };
 
@@ -652,7 +682,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             const long long eoff = w.b * p.o_stride_b + t * p.o_stride_t + (long long)w.h * HD;
             if (w.hi == w.lo) {  // nothing visible for the pair: zero output
                 if (SPLIT) {
-                    if (store) p.part_lse[(long long)w.part * p.batch * p.seq * p.nq + row] = -CUDART_INF_F;
+                    if (store) p.part_lse[SPLIT == 2 ? record_row(w, w.part) + quarter * 32 + lane : (long long)w.part * p.batch * p.seq * p.nq + row] = -CUDART_INF_F;
                 } else if (store) {
                     for (int c = -1; c < p.n_copies; ++c) {
                         uint4* dst = reinterpret_cast<uint4*>((c < 0 ? p.out : reinterpret_cast<uint16_t*>(p.out_copies[c])) + eoff);
@@ -668,8 +698,9 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 break;
             }
             const float row_l = fin_vals[(n & 3) * 128 + r];
-            if constexpr (SPLIT) {
-                store_part(w, quarter, row_l, 0);
+            if constexpr (SPLIT != 0) {
+                if constexpr (SPLIT == 1) store_part(w, quarter, row_l, 0);
+                else send_part(w, quarter, row_l, 0);
                 break;
             }
             if (!mbar_wait_warp<2>(o_full, n & 1)) {
@@ -913,97 +944,135 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 fin_vals[(n & 3) * 128 + r] = l;
                 // (SPLIT: the place in the output is read again, not kept in registers through the blocks)
                 const WideWork u = SPLIT ? *first_unit : w;
-                float* lse = SPLIT ? p.part_lse + (long long)u.part * p.batch * p.seq * p.nq : p.out_lse;
+                float* lse = SPLIT == 1 ? p.part_lse + (long long)u.part * p.batch * p.seq * p.nq : SPLIT == 2 ? p.part_lse : p.out_lse;
                 if (lse && u.q0 + r < p.seq)
-                    lse[((long long)u.b * p.seq + u.q0 + r) * p.nq + u.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
+                    lse[SPLIT == 2 ? record_row(u, u.part) + r : ((long long)u.b * p.seq + u.q0 + r) * p.nq + u.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
                 mbar_arrive_warp(&fin[n & 3]);
                 ++n;
-                if constexpr (SPLIT) {
-                    store_part(*first_unit, quarter, l, HD / 2);
+                if constexpr (SPLIT != 0) {
+                    if constexpr (SPLIT == 1) store_part(*first_unit, quarter, l, HD / 2);
+                    else send_part(*first_unit, quarter, l, 1);
                     break;
                 }
             }
         }
     }
 
+    // SPLIT 2: this warp's half of the CTA's columns, of 32 rows, as they are: while what the others finish is on its way
+    constexpr int MOST = SPLIT == 2 ? 4 : 1;
+    uint32_t mine[MOST][GROUP];
+    int my_first = 0, my_count = 0;  // groups
+    if (SPLIT == 2 && warp < C::PRODUCER_WARP && total > 0) {
+        const WideWork w = *first_unit;
+        const int g0 = group0(w.part), g1 = group0(w.part + 1), mid = (g0 + g1 + 1) / 2;
+        my_first = warp < C::EPILOGUE_WARP ? mid : g0, my_count = (warp < C::EPILOGUE_WARP ? g1 : mid) - my_first;
+        const uint32_t tO = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + C::COL_O + my_first * GROUP;
+#pragma unroll
+        for (int k = 0; k < MOST; ++k)
+            if (k < my_count && w.hi > w.lo) tmem_ld16(tO + k * GROUP, mine[k]);
+        tmem_wait_ld();
+    }
     __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();  // neither CTA's barriers or tensor memory go before the other is through with them
-    if constexpr (SPLIT) {
-        if (p.fold && total > 0) {  // every part's records are there; a warp takes a row in ten of the CTA's share
-            constexpr int W = C::THREADS / 32;
-            const long long rows = (long long)p.batch * p.seq * p.nq;
+    if constexpr (SPLIT == 2) {
+        // Every part's records are there; a warp finishes its half of the CTA's columns of 32 rows.
+        auto finish = [&](auto parts_tag) {
+            constexpr int PARTS = decltype(parts_tag)::value, TAKES = PARTS == 3 ? 3 : 4;  // groups a warp takes at most
             const WideWork w = *first_unit;
-            const int parts = p.num_splits, r0 = own_row0(w.part), end = min(own_row0(w.part + 1), p.seq - w.q0);
-            const long long row0 = ((long long)w.b * p.seq + w.q0) * p.nq + w.h;
-            const long long eoff0 = w.b * p.o_stride_b + w.q0 * p.o_stride_t + (long long)w.h * HD + lane * 4;
-            // The other parts' rows go behind the tile (at most 48 rows of two or 64 of one), gate values into rows of
-            // the tile that others fold.
-            constexpr int THEIRS = 8 * PART_CHUNK;
-            auto theirs = [&](int i) { return smem + THEIRS + (i - r0) * (parts - 1) * 1024 + lane * 16; };
-            auto gates = [&](int i) { return smem + (lane >> 4) * PART_CHUNK + ((own_row0(w.part + 1) + i - r0) & 127) * 128 + (lane & 15) * 8; };
-            float lse = -CUDART_INF_F;  // lane = 3 k + part: of the warp's k-th row
-            const int li = r0 + warp + lane / 3 * W;
-            if (li < end && lane % 3 < parts) lse = p.part_lse[lane % 3 * rows + row0 + (long long)li * p.nq];
-#pragma unroll 1
-            for (int i = r0 + warp; i < end; i += W) {
-                uint8_t* dst = theirs(i);
-                const float* src = p.part_o + (row0 + (long long)i * p.nq) * HD + lane * 4;
-#pragma unroll 1
-                for (int u = 0; u < parts; ++u) {
-                    if (u == w.part) continue;
-                    cp_async_16(dst, src + u * rows * HD);
-                    cp_async_16(dst + 512, src + u * rows * HD + 128);
-                    dst += 1024;
-                }
-                if (p.gate) {
-                    cp_async_8(gates(i), p.gate + eoff0 + i * p.o_stride_t);
-                    cp_async_8(gates(i) + 2 * PART_CHUNK, p.gate + eoff0 + i * p.o_stride_t + 128);
+            const int row = (warp & 3) * 32 + lane, rows = min(128, p.seq - w.q0);
+            const bool live = row < rows;
+            // the others' values, all at once, and the parts' log-sum-exps
+            float4 t[PARTS - 1][TAKES][4];
+            float weight[PARTS], mx = -CUDART_INF_F, z = 0.f;
+            auto other = [&](int s) { return w.part + s < PARTS ? w.part + s : w.part + s - PARTS; };
+#pragma unroll
+            for (int s = 1; s < PARTS; ++s) {
+                const float4* src = reinterpret_cast<const float4*>(p.part_o + record_row(w, other(s)) * HD) + (long long)my_first * 4 * rows + row;
+#pragma unroll
+                for (int k = 0; k < TAKES; ++k)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (live && k < my_count) t[s - 1][k][i] = __ldcg(src + (k * 4 + i) * rows);
+            }
+#pragma unroll
+            for (int s = 0; s < PARTS; ++s) {  // (of this part first)
+                weight[s] = live ? __ldcg(p.part_lse + record_row(w, other(s)) + row) : -CUDART_INF_F;
+                mx = fmaxf(mx, weight[s]);
+            }
+#pragma unroll
+            for (int s = 0; s < PARTS; ++s) {
+                weight[s] = mx == -CUDART_INF_F ? 0.f : __expf(weight[s] - mx);
+                z += weight[s];
+            }
+            if (p.out_lse && live && my_first == 0)
+                p.out_lse[((long long)w.b * p.seq + w.q0 + row) * p.nq + w.h] = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
+            const float iz = z > 0.f ? 1.0f / z : 0.f, row_l = fin_vals[row];
+            const float own = row_l > 0.f ? weight[0] * iz / row_l : 0.f;
+            float acc[TAKES][GROUP];
+#pragma unroll
+            for (int k = 0; k < TAKES; ++k)
+#pragma unroll
+                for (int e = 0; e < GROUP; ++e) acc[k][e] = own > 0.f ? __uint_as_float(mine[k][e]) * own : 0.f;  // (an empty part's columns may hold anything)
+#pragma unroll
+            for (int s = 1; s < PARTS; ++s) {
+                const float e = weight[s] * iz;
+                if (e > 0.f) {  // (an empty part's record may hold anything)
+#pragma unroll
+                    for (int k = 0; k < TAKES; ++k)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 v = t[s - 1][k][i];
+                            acc[k][4 * i] = fmaf(e, v.x, acc[k][4 * i]), acc[k][4 * i + 1] = fmaf(e, v.y, acc[k][4 * i + 1]);
+                            acc[k][4 * i + 2] = fmaf(e, v.z, acc[k][4 * i + 2]), acc[k][4 * i + 3] = fmaf(e, v.w, acc[k][4 * i + 3]);
+                        }
                 }
             }
-            // The parts' weights, for all the warp's rows at once (lanes 30 and 31 hold nothing).
-            const int base = lane / 3 * 3;
-            const float l0 = __shfl_sync(0xffffffffu, lse, base), l1 = __shfl_sync(0xffffffffu, lse, base + 1), l2 = __shfl_sync(0xffffffffu, lse, base + 2);
-            const float mx = fmaxf(fmaxf(l0, l1), l2), at0 = mx == -CUDART_INF_F ? 0.f : mx;
-            const float z = __expf(l0 - at0) + __expf(l1 - at0) + __expf(l2 - at0);
-            const float weight = z > 0.f ? __expf(lse - at0) / z : 0.f;
-            if (p.out_lse && li < end && lane % 3 == 0) p.out_lse[row0 + (long long)li * p.nq] = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
-            cp_async_wait_all();
-            __syncwarp();
-            int k3 = 0;
-#pragma unroll 1
-            for (int i = r0 + warp; i < end; i += W, k3 += 3) {
-                const uint8_t* from = theirs(i);
-                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            // Out through shared memory (Q, K and V are through), so that a store writes whole rows of the warp's columns: a thread's
+            // own 16 bytes at a time took 1800 clk.
+            constexpr int PITCH = TAKES * GROUP * 2 + 16;
+            const uint32_t tile = smem_u32(smem) + warp * 32 * PITCH;
+            const long long eoff = w.b * p.o_stride_b + w.q0 * p.o_stride_t + (long long)w.h * HD + my_first * GROUP;
 #pragma unroll
-                for (int u = 0; u < 3; ++u) {
-                    const float e = __shfl_sync(0xffffffffu, weight, k3 + u);
-                    const bool own = u == w.part;
-                    const uint8_t* src = own ? smem + (lane >> 3) * PART_CHUNK + i * 128 + (((lane & 7) ^ (i & 7)) << 4) : from;
-                    if (!own) from += 1024;
-                    if (e == 0.f) continue;  // no such part, or an empty one, whose record may hold anything
-                    const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + (own ? 4 * PART_CHUNK : 512));
-                    acc[0] = fmaf(e, a.x, acc[0]), acc[1] = fmaf(e, a.y, acc[1]), acc[2] = fmaf(e, a.z, acc[2]), acc[3] = fmaf(e, a.w, acc[3]);
-                    acc[4] = fmaf(e, b.x, acc[4]), acc[5] = fmaf(e, b.y, acc[5]), acc[6] = fmaf(e, b.z, acc[6]), acc[7] = fmaf(e, b.w, acc[7]);
-                }
-                uint2 o[2];
+            for (int k = 0; k < TAKES; ++k) {
+                uint32_t o[GROUP / 2];
+                if constexpr (GATE) {
+                    if (live && k < my_count) {
+                        const uint4* g = reinterpret_cast<const uint4*>(p.gate + eoff + row * p.o_stride_t + k * GROUP);
+                        const uint4 ga = g[0], gb = g[1];
+                        const uint32_t gw[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    float* a = acc + 4 * c;
-                    if (p.gate) {
-                        const uint2 g = *reinterpret_cast<const uint2*>(gates(i) + c * 2 * PART_CHUNK);
-                        a[0] = sigmoid_gate(a[0], (uint16_t)g.x), a[1] = sigmoid_gate(a[1], (uint16_t)(g.x >> 16));
-                        a[2] = sigmoid_gate(a[2], (uint16_t)g.y), a[3] = sigmoid_gate(a[3], (uint16_t)(g.y >> 16));
+                        for (int i = 0; i < GROUP / 2; ++i) {
+                            acc[k][2 * i] = sigmoid_gate(acc[k][2 * i], (uint16_t)gw[i]);
+                            acc[k][2 * i + 1] = sigmoid_gate(acc[k][2 * i + 1], (uint16_t)(gw[i] >> 16));
+                        }
                     }
-                    o[c] = make_uint2(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]));
                 }
-                for (int c = -1; c < p.n_copies; ++c) {
-                    uint16_t* dst = (c < 0 ? p.out : reinterpret_cast<uint16_t*>(p.out_copies[c])) + eoff0 + i * p.o_stride_t;
-                    *reinterpret_cast<uint2*>(dst) = o[0];
-                    *reinterpret_cast<uint2*>(dst + 128) = o[1];
-                }
+#pragma unroll
+                for (int i = 0; i < GROUP / 2; ++i) o[i] = pack_bf16x2(acc[k][2 * i], acc[k][2 * i + 1]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + lane * PITCH + k * 32 + i * 16), "r"(o[4 * i]), "r"(o[4 * i + 1]), "r"(o[4 * i + 2]), "r"(o[4 * i + 3]) : "memory");
             }
+            __syncwarp();
+            const int per_row = 2 * my_count, magic = (65536 + per_row - 1) / per_row;  // 16-byte pieces of a row (exact for the 256 there are at most)
+            const int end = min(32, rows - (warp & 3) * 32);
+#pragma unroll 1
+            for (int i = lane; i < 32 * per_row; i += 32) {
+                const int r = i * magic >> 16, c = i - r * per_row;
+                if (r >= end) break;
+                uint4 v;
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(tile + r * PITCH + c * 16));
+                const long long at = eoff + ((warp & 3) * 32 + r) * p.o_stride_t + c * 8;
+                *reinterpret_cast<uint4*>(p.out + at) = v;
+                for (int k = 0; k < p.n_copies; ++k) *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + at) = v;
+            }
+        };
+        static_assert(C::MOST_FOLDED == 3, "two or three parts");
+        if (warp < C::PRODUCER_WARP && total > 0) {
+            if (p.num_splits == 3) finish(std::integral_constant<int, 3>{});
+            else finish(std::integral_constant<int, 2>{});
         }
     }
     if (warp == C::PRODUCER_WARP) tmem_dealloc_pair(tmem_base, 512);

@@ -302,15 +302,6 @@ __device__ __forceinline__ void bulk_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory");
 }
 
-// 16 / 8 bytes of global memory to shared memory, asynchronous; this thread's have landed after cp_async_wait_all().
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_8(void* smem_dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 // 2-D tiled load (c0 innermost, multiple of 8 elements for 16-bit data).
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1) {
     asm volatile(
