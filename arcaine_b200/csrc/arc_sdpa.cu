@@ -37,7 +37,7 @@ constexpr int kDecodeStaticSmem = 1024;
 struct WideRoom {
     static constexpr int MOST_FOLDED = WideCfg::MOST_FOLDED;
     int pairs = 74;
-    int folded[MOST_FOLDED + 1] = {0, 0, 33, 22};  // clusters of that many pairs
+    int folded[MOST_FOLDED + 1] = {0, 0, 33, 22, 15};  // clusters of that many pairs
     int clusters(int parts) const { return parts <= MOST_FOLDED ? folded[parts] : 0; }
 };
 
@@ -279,13 +279,22 @@ static int tile_key_blocks(const arc_sdpa_prefill_params* p, int qt) {
 }
 
 // Head dim 256: units of the CTA pairs' list, and how many parts the key range of each is worth when the units alone
-// would leave pairs idle.  Measured (us): a key block of a pair 1.13; records and fold 1.8 (gated 2.7) + 0.04 per pair in a cluster, 2.5 +
-// 0.06 per pair with a merge launch (every pair writes its 256 rows as f32, 32 bytes per clk and SM), whatever the number
-// of parts.  (256 queries of 16 heads over 2304 keys: 26.7 us whole, 15.7 in three parts, 19.6 in four; of 8 heads 26.2,
-// 15.6 in six.)
+// would leave pairs idle.  Measured over 64 to 512 rows of 4 to 24 heads and 384 to 8000 keys (us, what all calls have in common left
+// out; n pairs, of which those with fewer than 128 rows count in proportion where rows are stored): a key block of a pair 1.11 +
+// 0.0022 n; records and fold 0.6 (four parts 1.2) + 0.045 n in a cluster, 2.2 + 0.073 n with a merge launch.  (256 queries of 16 heads
+// over 2304 keys: 25.6 whole, 17.1 in two parts, 15.6 in three, 18.2 in four with a merge; of 8 heads 25.5, 13.7 in four.)  Gated, the
+// epilogue of whole units takes 3.3 more, the fold in a cluster 0.5 to 1.5, the merge launch nothing (256 of 8 heads over 640 keys: 14.5
+// whole, 11.2 in three parts, 12.1 in five).
 static long long wide_units(const arc_sdpa_prefill_params* p, int q_tiles) {
     const bool head_pair = ((p->nq / p->nkv) & 1) == 0;
     return (head_pair ? (long long)q_tiles * (p->nq / 2) : (long long)((p->seq + 255) / 256) * p->nq) * p->batch;
+}
+
+// Do the parts of a unit fold themselves, as one cluster?  Two and three do where all clusters fit at once; four where the library chose
+// them and there is neither gate nor additive mask (the merge launch gates for nothing, and is as good where most blocks are hidden).
+static bool folds_itself(const arc_sdpa_prefill_params* p, int parts, long long units, const WideRoom& room) {
+    if (parts > 3 && (p->num_splits != 0 || p->gate || p->mask_type == ARC_MASK_EXPLICIT)) return false;
+    return units <= room.clusters(parts);
 }
 
 static int choose_wide_splits(const arc_sdpa_prefill_params* p, int q_tiles, const WideRoom& room) {
@@ -298,9 +307,14 @@ static int choose_wide_splits(const arc_sdpa_prefill_params* p, int q_tiles, con
     if (p->mask_type == ARC_MASK_EXPLICIT && most <= 24 && (long long)p->batch * p->seq * p->nq > 1024) return 1;
     if (p->mask_type == ARC_MASK_CAUSAL && p->window > 0 && p->window < p->kv_len && !p->block_ids) most = std::min(most, (p->window + 255) / 128 + 1);
     int best = 1;
-    double least = 1.13 * most;
+    const double rows = std::min<int>(p->seq, 128) / 128.0;
+    double least = 1.11 * most + (p->gate ? 3.3 : 0.0);
+    const bool masked = p->mask_type == ARC_MASK_EXPLICIT;  // (blocks that nobody sees are not counted off: a merge launch looks better than it is)
     for (int s = 2; s <= 8 && s <= most && units * s <= room.pairs; ++s) {
-        const double t = 1.13 * ((most + s - 1) / s) + (units <= room.clusters(s) ? (p->gate ? 2.7 : 1.8) + 0.04 * (units * s) : 2.5 + 0.06 * (units * s));
+        const double n = (double)(units * s), blocks = (1.11 + 0.0022 * n) * ((most + s - 1) / s);
+        const bool fold = folds_itself(p, s, units, room);
+        const double t = p->gate ? 1.13 * ((most + s - 1) / s) + (fold ? 2.0 + 0.04 * n : 2.5 + 0.06 * n)
+                                 : blocks + (fold ? (masked ? 1.8 : s == 4 ? 1.2 : 0.6) + 0.045 * rows * n : 2.2 + 0.073 * rows * n);
         if (t < least) least = t, best = s;
     }
     return best;
@@ -581,7 +595,7 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
             return rc;
         }
         // (a cluster is placed inside one GPC, so fewer fit than pairs / parts)
-        const bool fold = split && wide_units(p, plan.q_tiles) <= ds->wide.clusters(plan.splits);
+        const bool fold = split && folds_itself(p, plan.splits, wide_units(p, plan.q_tiles), ds->wide);
         const WideKernel kernel = wide_kernel(kp.gate != nullptr, masked, fold ? 2 : split ? 1 : 0, units > ds->wide.pairs, kp.ids != nullptr);
         ARC_CUDA(launch_dependent(kernel,
                                   dim3((unsigned)(2 * (split || units < ds->wide.pairs ? units : ds->wide.pairs))), dim3(WideCfg::THREADS),

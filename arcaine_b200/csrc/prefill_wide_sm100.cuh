@@ -43,7 +43,7 @@ struct WideCfg {
     static constexpr int NUM_BARS = 5 + 8 + 2 + 4 + 2 + 4 + 8 + 2;
     static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4 + 2 * 32 + 128 * 4;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
-    static constexpr int MOST_FOLDED = 3;  // parts of a split unit that fold themselves as one cluster
+    static constexpr int MOST_FOLDED = 4;  // parts of a split unit that fold themselves as one cluster
     static constexpr int EPILOGUE_WARP = 4, PRODUCER_WARP = 8, ISSUER_WARP = 9;
     static constexpr int THREADS = 320;
 };
@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     if constexpr (SPLIT == 2) {
         // Every part's records are there; a warp finishes its half of the CTA's columns of 32 rows.
         auto finish = [&](auto parts_tag) {
-            constexpr int PARTS = decltype(parts_tag)::value, TAKES = PARTS == 3 ? 3 : 4;  // groups a warp takes at most
+            constexpr int PARTS = decltype(parts_tag)::value, TAKES = PARTS == 4 ? 2 : PARTS == 3 ? 3 : 4;  // groups a warp takes at most
             const WideWork w = *first_unit;
             const int row = (warp & 3) * 32 + lane, rows = min(128, p.seq - w.q0);
             const bool live = row < rows;
@@ -1037,41 +1037,49 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
 #pragma unroll
             for (int k = 0; k < TAKES; ++k) {
                 uint32_t o[GROUP / 2];
-                if constexpr (GATE) {
-                    if (live && k < my_count) {
-                        const uint4* g = reinterpret_cast<const uint4*>(p.gate + eoff + row * p.o_stride_t + k * GROUP);
-                        const uint4 ga = g[0], gb = g[1];
-                        const uint32_t gw[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
-#pragma unroll
-                        for (int i = 0; i < GROUP / 2; ++i) {
-                            acc[k][2 * i] = sigmoid_gate(acc[k][2 * i], (uint16_t)gw[i]);
-                            acc[k][2 * i + 1] = sigmoid_gate(acc[k][2 * i + 1], (uint16_t)(gw[i] >> 16));
-                        }
-                    }
-                }
 #pragma unroll
                 for (int i = 0; i < GROUP / 2; ++i) o[i] = pack_bf16x2(acc[k][2 * i], acc[k][2 * i + 1]);
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + lane * PITCH + k * 32 + i * 16), "r"(o[4 * i]), "r"(o[4 * i + 1]), "r"(o[4 * i + 2]), "r"(o[4 * i + 3]) : "memory");
             }
-            __syncwarp();
             const int per_row = 2 * my_count, magic = (65536 + per_row - 1) / per_row;  // 16-byte pieces of a row (exact for the 256 there are at most)
             const int end = min(32, rows - (warp & 3) * 32);
-#pragma unroll 1
-            for (int i = lane; i < 32 * per_row; i += 32) {
-                const int r = i * magic >> 16, c = i - r * per_row;
-                if (r >= end) break;
-                uint4 v;
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(tile + r * PITCH + c * 16));
+            auto place_of = [&](int i, int& r, int& c) {  // piece i of the warp's: row, piece of the row; whether there is one
+                r = i * magic >> 16, c = i - r * per_row;
+                return i < 32 * per_row && r < end;
+            };
+            [[maybe_unused]] uint4 gate[GATE ? 2 * TAKES : 1];  // all asked for at once
+            if constexpr (GATE) {
+#pragma unroll
+                for (int k = 0; k < 2 * TAKES; ++k) {
+                    int r, c;
+                    if (place_of(k * 32 + lane, r, c)) gate[k] = *reinterpret_cast<const uint4*>(p.gate + eoff + ((warp & 3) * 32 + r) * p.o_stride_t + c * 8);
+                }
+            }
+            __syncwarp();
+#pragma unroll GATE ? 2 * TAKES : 1
+            for (int k = 0; k < 2 * TAKES; ++k) {
+                int r, c;
+                if (!place_of(k * 32 + lane, r, c)) break;
+                uint32_t v[4];
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(tile + r * PITCH + c * 16));
+                if constexpr (GATE) {
+                    const uint32_t g[4] = {gate[k].x, gate[k].y, gate[k].z, gate[k].w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)  // bf16(attention) * sigmoid(gate): the rounding order of the two-launch form
+                        v[i] = pack_bf16x2(__uint_as_float(v[i] << 16) * sigmoid(__uint_as_float(g[i] << 16)),
+                                           __uint_as_float(v[i] & 0xffff0000u) * sigmoid(__uint_as_float(g[i] & 0xffff0000u)));
+                }
                 const long long at = eoff + ((warp & 3) * 32 + r) * p.o_stride_t + c * 8;
-                *reinterpret_cast<uint4*>(p.out + at) = v;
-                for (int k = 0; k < p.n_copies; ++k) *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + at) = v;
+                *reinterpret_cast<uint4*>(p.out + at) = make_uint4(v[0], v[1], v[2], v[3]);
+                for (int n = 0; n < p.n_copies; ++n) *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[n]) + at) = make_uint4(v[0], v[1], v[2], v[3]);
             }
         };
-        static_assert(C::MOST_FOLDED == 3, "two or three parts");
+        static_assert(C::MOST_FOLDED == 4, "two to four parts");
         if (warp < C::PRODUCER_WARP && total > 0) {
-            if (p.num_splits == 3) finish(std::integral_constant<int, 3>{});
+            if (p.num_splits == 4) finish(std::integral_constant<int, 4>{});
+            else if (p.num_splits == 3) finish(std::integral_constant<int, 3>{});
             else finish(std::integral_constant<int, 2>{});
         }
     }
