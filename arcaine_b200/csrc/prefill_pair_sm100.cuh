@@ -225,16 +225,17 @@ struct OutStage {
     uint64_t* gate_bar;  // [2] this warp's, one per buffer
     uint32_t gate_par;   // bit i: parity of buffer i's next gate load
     int h, t0, b;        // head, first of the warp's 32 rows, sequence
+    int col0, rounds;    // the columns: [col0, col0 + 64 rounds) of the head
 };
 
 // Gate values of round c (columns [64 c, 64 c + 64)) into the round's buffer, which is free.  One lane.
 __device__ __forceinline__ void stage_load_gate(const OutStage& s, const void* tm_gate, int c) {
     mbar_arrive_expect_tx(&s.gate_bar[c & 1], 4096);
-    tma_load_4d(s.buf + (c & 1) * 4096, tm_gate, &s.gate_bar[c & 1], c * 64, s.h, s.t0, s.b);
+    tma_load_4d(s.buf + (c & 1) * 4096, tm_gate, &s.gate_bar[c & 1], s.col0 + c * 64, s.h, s.t0, s.b);
 }
 
 // Once per tile, before its accumulator is waited for.
-template <bool GATE, int HD>
+template <bool GATE>
 __device__ __forceinline__ void stage_open(OutStage& s, const void* tm_gate, int lane, int h, int t0, int b) {
     s.h = h, s.t0 = t0, s.b = b;
     if (lane == 0) {
@@ -242,7 +243,7 @@ __device__ __forceinline__ void stage_open(OutStage& s, const void* tm_gate, int
         if (GATE) {
             stage_load_gate(s, tm_gate, 0);
             stage_load_gate(s, tm_gate, 1);
-            for (int c = 2; c < HD / 64; ++c) tma_prefetch_4d(tm_gate, c * 64, h, t0, b);  // (the later rounds' into L2)
+            for (int c = 2; c < s.rounds; ++c) tma_prefetch_4d(tm_gate, s.col0 + c * 64, h, t0, b);  // (the later rounds' into L2)
         }
     }
     __syncwarp();
@@ -255,8 +256,8 @@ __device__ __forceinline__ void stage_open(OutStage& s, const void* tm_gate, int
 template <bool GATE>
 constexpr int STAGE_COLS = GATE ? 16 : 32;
 
-// Before turn k, of N columns, of a tile of HD columns.  False: the gate values never came.
-template <bool GATE, int HD, int N = STAGE_COLS<GATE>>
+// Before turn k, of N columns.  False: the gate values never came.
+template <bool GATE, int N = STAGE_COLS<GATE>>
 __device__ __forceinline__ bool stage_before(OutStage& s, const void* tm_gate, int lane, int k) {
     constexpr int TURNS = 64 / N;  // per round
     const int c = k / TURNS, i = c & 1;
@@ -268,7 +269,7 @@ __device__ __forceinline__ bool stage_before(OutStage& s, const void* tm_gate, i
             if (lane == 0) bulk_wait_read<1>();  // round c - 2 has left the buffer
             __syncwarp();
         }
-    } else if (GATE && k % TURNS == TURNS / 2 && c >= 1 && c + 1 < HD / 64) {
+    } else if (GATE && k % TURNS == TURNS / 2 && c >= 1 && c + 1 < s.rounds) {
         if (lane == 0) {
             bulk_wait_read<0>();  // round c - 1 has left its buffer: the one of round c + 1
             stage_load_gate(s, tm_gate, c + 1);
@@ -283,7 +284,7 @@ __device__ __forceinline__ void stage_send(const OutStage& s, const void* tm_out
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
-        tma_store_4d(tm_out, s.buf + (c & 1) * 4096, c * 64, s.h, s.t0, s.b);
+        tma_store_4d(tm_out, s.buf + (c & 1) * 4096, s.col0 + c * 64, s.h, s.t0, s.b);
         bulk_commit();
     }
 }
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
         const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
         int tq0 = 0, tq1 = 0;  // tiles with key blocks so far, per pipeline
         bool ok = true;
-        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0};
+        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0, 0, HD / 64};
         TileCursor cur = *cursor;
         for (; ok && cur.w < total_tiles; cur.advance(p)) {
             const PairWork pw = decode_pair<VISION>(p, cur);
@@ -661,7 +662,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                     }
                     continue;
                 }
-                if (warp_store) stage_open<GATE, HD>(stage, &tm_gate, lane, h, t0, pw.b);
+                if (warp_store) stage_open<GATE>(stage, &tm_gate, lane, h, t0, pw.b);
                 const int tq = s ? tq1 : tq0;
                 if (!mbar_wait_warp<2>(&fin[2 * s + (tq & 1)], (tq >> 1) & 1)) {
                     report_fault(p.fault, FAULT_WAIT_FULL, 0x500u + s);
@@ -683,7 +684,7 @@ __global__ void __launch_bounds__(PairCfg::THREADS, 1)
                 tmem_ld(tO, wa);
 #pragma unroll 1
                 for (int c = 0; c < HD / SC; ++c) {
-                    if (warp_store && !stage_before<GATE, HD>(stage, &tm_gate, lane, c)) {
+                    if (warp_store && !stage_before<GATE>(stage, &tm_gate, lane, c)) {
                         report_fault(p.fault, FAULT_WAIT_FULL, 0x600u + s);
                         ok = false;
                         break;

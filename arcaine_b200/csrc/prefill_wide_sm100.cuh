@@ -39,8 +39,12 @@ struct WideCfg {
     static constexpr int STAGES = 2;               // of K and of V
     static constexpr int COL_S = 0;                // + 128 * buffer
     static constexpr int COL_O = 256;
-    // first[4] q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp][2], next_full next_empty
-    static constexpr int NUM_BARS = 5 + 8 + 2 + 4 + 2 + 4 + 8 + 2;
+    // first[4] q_empty, {k,v}_{full,empty}[2], s_full[2], p_half[buffer][half], o_full o_empty fin[4], gate[epilogue warp][2], next_full next_empty, gate[softmax warp][2]
+    static constexpr int NUM_BARS = 5 + 8 + 2 + 4 + 2 + 4 + 8 + 2 + 8;
+    // Arrivals that complete a phase of barrier i: the eight softmax or epilogue warps of both CTAs, the four of one, or one thread.
+    __device__ static constexpr int arrivals(int i) {
+        return (i >= 15 && i < 19) || i == 20 ? 8 : (i >= 21 && i < 25) || i == 33 || i == 34 ? 4 : 1;  // p_half, o_empty; fin, next_full, next_empty
+    }
     static constexpr int SMEM_BYTES = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + STAGE_BYTES + NUM_BARS * 8 + 16 + 4 * 128 * 4 + 2 * 32 + 128 * 4;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
     static constexpr int MOST_FOLDED = 4;  // parts of a split unit that fold themselves as one cluster
@@ -300,6 +304,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     uint64_t* gate_bar = bars + 25;    // [epilogue warp][buffer] own CTA
     uint64_t* next_full = bars + 33;   // own CTA: the epilogue warps have looked up the next unit's vision blocks
     uint64_t* next_empty = bars + 34;  // the softmax warps have taken them
+    uint64_t* gate_late = bars + 35;   // [softmax warp][buffer] own CTA: of the last unit's second half
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARS);
     uint32_t* abort_slot = tmem_slot + 1;
     float* fin_vals = reinterpret_cast<float*>(tmem_slot + 4);  // [unit & 3][row] row sum
@@ -319,27 +324,8 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
     }
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 4; ++i) mbar_init(&first[i], 1);
-        mbar_init(q_empty, 1);
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&k_full[i], 1);
-            mbar_init(&k_empty[i], 1);
-            mbar_init(&v_full[i], 1);
-            mbar_init(&v_empty[i], 1);
-            mbar_init(&s_full[i], 1);
-            mbar_init(&p_half[2 * i], 8);
-            mbar_init(&p_half[2 * i + 1], 8);
-        }
-        for (int i = 0; i < 4; ++i) {
-            mbar_init(&fin[i], 4);
-            mbar_init(&gate_bar[2 * i], 1);
-            mbar_init(&gate_bar[2 * i + 1], 1);
-        }
-        mbar_init(o_full, 1);
-        mbar_init(o_empty, 8);
-        mbar_init(next_full, 4);
-        mbar_init(next_empty, 4);
+    if (warp == 0) {  // (a lane a barrier: one thread took them in turn, and what stands in front of the cluster's barrier is on every call's clock)
+        for (int i = lane; i < C::NUM_BARS; i += 32) mbar_init(&bars[i], C::arrivals(i));
         fence_mbar_init();
     }
     if (warp == C::PRODUCER_WARP) tmem_alloc_pair(tmem_slot, 512);
@@ -486,6 +472,46 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 if (row < rows && (i < 4 ? first : second))
                     dst[(long long)(g * 4 + i) * rows] = make_float4(__uint_as_float(v[4 * i]) * inv, __uint_as_float(v[4 * i + 1]) * inv, __uint_as_float(v[4 * i + 2]) * inv, __uint_as_float(v[4 * i + 3]) * inv);
         }
+    };
+
+    auto store_copies = [&](const OutStage& stage, const uint32_t* words, int n, int col) {  // of this thread's row
+        if (stage.t0 + lane >= p.seq) return;
+        const long long at = stage.b * p.o_stride_b + (stage.t0 + lane) * p.o_stride_t + (long long)stage.h * HD + col;
+        for (int k = 0; k < p.n_copies; ++k) {
+            uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + at);
+#pragma unroll
+            for (int i = 0; i < n / 4; ++i) d4[i] = make_uint4(words[4 * i], words[4 * i + 1], words[4 * i + 2], words[4 * i + 3]);
+        }
+    };
+    // The stage's columns of the warp's 32 rows, which begin at tO, in turns of 32.  (Gated, of which a turn of 16 took 690 clk, 1200 so.
+    // us: 1300 tokens of 24/4 heads 33.6 -> 31.5, 2000 57.5 -> 54, 4 x 1500, window 300, 106 -> 97; cold, 200 x 333 of 8/4, 14.4 -> 13.3.)
+    // frees: the accumulator may be overwritten behind the last of them.
+    auto write_turns = [&](OutStage& stage, uint32_t tO, float inv, bool warp_store, bool frees) -> bool {
+        constexpr int SC = 32;
+        const int turns = stage.rounds * (64 / SC);
+        uint32_t wa[SC], w8[SC / 2];
+        tmem_ld(tO, wa);
+#pragma unroll 1
+        for (int c = 0; c < turns; ++c) {
+            if (warp_store && !stage_before<GATE, SC>(stage, &tm_gate, lane, c)) {
+                if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x600u);
+                return false;
+            }
+            tmem_wait_ld();
+            if (frees && c + 1 == turns) {  // O is in registers
+                tc_fence_before_sync();
+                mbar_arrive_remote_warp(map_to_cta(smem_u32(o_empty), lead));
+            }
+            auto next = [&]() {
+                if (c + 1 < turns) tmem_ld(tO + (c + 1) * SC, wa);
+            };
+            if (!warp_store) next();
+            if (warp_store) {
+                stage_turn<GATE>(stage, &tm_out, lane, c, wa, inv, w8, next);
+                store_copies(stage, w8, SC / 2, stage.col0 + c * SC);
+            }
+        }
+        return true;
     };
 
     if (warp == C::PRODUCER_WARP) {
@@ -655,9 +681,9 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;
         const uint32_t tO = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::COL_O;
-        const uint32_t b_empty = map_to_cta(smem_u32(o_empty), lead);
+        [[maybe_unused]] const uint32_t b_empty = map_to_cta(smem_u32(o_empty), lead);
         int n = 0;  // units with key blocks so far
-        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0};
+        OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0, 0, HD / 64};
         WideCursor cur(p);
         for (; cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
@@ -692,7 +718,16 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 }
                 continue;
             }
-            if (!SPLIT && warp_store) stage_open<GATE, HD>(stage, &tm_gate, lane, w.h, t0, w.b);
+            // GATE: the softmax warps take the second half of the last unit's columns: four warps alone wrote them in 12000 clk.  (us: 1000
+            // tokens of 16/8 heads 20.2 -> 18.7, 2000 of 8/2 28.9 -> 27.2, 64 10.1 -> 8.4.)
+            bool last = false;
+            if (GATE && !SPLIT) {
+                WideCursor after = cur;
+                after.advance(p);
+                last = after.w >= total;
+                stage.rounds = last ? HD / 128 : HD / 64;
+            }
+            if (!SPLIT && warp_store) stage_open<GATE>(stage, &tm_gate, lane, w.h, t0, w.b);
             if (!mbar_wait_warp<2>(&fin[n & 3], (n >> 2) & 1)) {
                 if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x500u);
                 break;
@@ -711,15 +746,6 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             ++n;
             const float inv = row_l > 0.f ? 1.0f / row_l : 0.f;
             bool ok = true;
-            auto store_copies = [&](const uint32_t* words, int n, int col) {  // of this thread's row
-                if (stage.t0 + lane >= p.seq) return;
-                const long long at = stage.b * p.o_stride_b + (stage.t0 + lane) * p.o_stride_t + (long long)stage.h * HD + col;
-                for (int k = 0; k < p.n_copies; ++k) {
-                    uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out_copies[k]) + at);
-#pragma unroll
-                    for (int i = 0; i < n / 4; ++i) d4[i] = make_uint4(words[4 * i], words[4 * i + 1], words[4 * i + 2], words[4 * i + 3]);
-                }
-            };
             if constexpr (EARLY) {
                 // The whole row into registers as bf16 pairs, so that the next unit may overwrite the accumulator before the last
                 // columns have left the SM.
@@ -749,42 +775,17 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                     const uint32_t at = smem_u32(stage.buf) + lane * 128;
 #pragma unroll
                     for (int c = 0; c < HD / 64; ++c) {
-                        stage_before<false, HD>(stage, &tm_gate, lane, 2 * c);
+                        stage_before<false>(stage, &tm_gate, lane, 2 * c);
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
                             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"((at + (c & 1) * 4096) + ((i ^ (lane & 7)) << 4)),
                                          "r"(pk[c * 32 + 4 * i]), "r"(pk[c * 32 + 4 * i + 1]), "r"(pk[c * 32 + 4 * i + 2]), "r"(pk[c * 32 + 4 * i + 3]) : "memory");
                         stage_send(stage, &tm_out, lane, c);
                     }
-                    store_copies(pk, HD / 2, 0);
+                    store_copies(stage, pk, HD / 2, 0);
                 }
             } else {
-                // 32 columns a turn.  (Gated, of which a turn of 16 took 690 clk, 1200 so.  us: 1300 tokens of 24/4 heads 33.6 -> 31.5, 2000
-                // 57.5 -> 54, 4 x 1500, window 300, 106 -> 97; cold, 200 x 333 of 8/4, 14.4 -> 13.3.)
-                constexpr int SC = 32;
-                uint32_t wa[SC], w8[SC / 2];
-                tmem_ld(tO, wa);
-#pragma unroll 1
-                for (int c = 0; c < HD / SC; ++c) {
-                    if (warp_store && !stage_before<GATE, HD, SC>(stage, &tm_gate, lane, c)) {
-                        if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x600u);
-                        ok = false;
-                        break;
-                    }
-                    tmem_wait_ld();
-                    if (c + 1 == HD / SC) {  // O is in registers: the next unit may overwrite the accumulator
-                        tc_fence_before_sync();
-                        mbar_arrive_remote_warp(b_empty);
-                    }
-                    auto next = [&]() {
-                        if (c + 1 < HD / SC) tmem_ld(tO + (c + 1) * SC, wa);
-                    };
-                    if (!warp_store) next();
-                    if (warp_store) {
-                        stage_turn<GATE>(stage, &tm_out, lane, c, wa, inv, w8, next);
-                        store_copies(w8, SC / 2, c * SC);
-                    }
-                }
+                ok = write_turns(stage, tO, inv, warp_store, !last);
             }
             if (!ok) break;
         }
@@ -949,6 +950,25 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                     lse[SPLIT == 2 ? record_row(u, u.part) + r : ((long long)u.b * p.seq + u.q0 + r) * p.nq + u.h] = l > 0.f ? (m + fast_log2(l)) * 0.6931471805599453f : -CUDART_INF_F;
                 mbar_arrive_warp(&fin[n & 3]);
                 ++n;
+                if constexpr (GATE && SPLIT == 0) {
+                    WideCursor after = cur;
+                    after.advance(p);
+                    if (after.w >= total) {  // (in what was Q's shared memory)
+                        OutStage half{smem + quarter * STAGE_WARP_BYTES, &gate_late[2 * quarter], 0u, 0, 0, 0, HD / 2, HD / 128};
+                        const int t0 = w.q0 + quarter * 32;
+                        // (The unit before may not have got its P V yet, whose parity is the one before; the one before that has: its P V
+                        // went ahead of this unit's scores.)
+                        if ((n > 1 && !mbar_wait_inline(o_full, n & 1)) || !mbar_wait_inline(o_full, (n - 1) & 1)) {
+                            if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x800u);
+                            break;
+                        }
+                        tc_fence_after_sync();
+                        if (t0 < p.seq) stage_open<GATE>(half, &tm_gate, lane, w.h, t0, w.b);
+                        write_turns(half, tO + HD / 2, l > 0.f ? 1.0f / l : 0.f, t0 < p.seq, false);
+                        if (lane == 0) bulk_wait_read<0>();
+                        break;
+                    }
+                }
                 if constexpr (SPLIT != 0) {
                     if constexpr (SPLIT == 1) store_part(*first_unit, quarter, l, HD / 2);
                     else send_part(*first_unit, quarter, l, 1);
