@@ -648,13 +648,14 @@ static bool size_decode_cta(int hd, int nkv_cta, int slices, int batch, int extr
     return stages >= 2;
 }
 
-// One launch or two?  A cluster of up to eight CTAs per sequence and group of heads finishes alone: 5.2 us and the longer of
-// two times: of the CTAs with the longest sequence, at the 93 GB/s one CTA pulls at head dim 256 (four consumer warps) and
-// 105 at 128 (eight), and of all bytes at what so many CTAs get out of the memory (less when a CTA's heads fill a row of
-// 2 KB: one slice, as few warps as heads).  Equal shares over all SMs read the total at 7 TB/s, but cost 7.2 us (8 with the
+// One launch or two?  A cluster of up to eight CTAs per sequence and group of heads finishes alone: 4.1 us (4.7 with the lengths on the
+// device) and the longer of two times: of the CTAs with the longest sequence, at the 93 GB/s one CTA pulls at head dim 256 (four
+// consumer warps) and 105 at 128 (eight), and of all bytes at what so many CTAs get out of the memory (less when a CTA's heads fill a
+// row of 2 KB: one slice, as few warps as heads).  Equal shares over all SMs read the total at 7 TB/s, but cost 7.2 us (8 with the
 // lengths on the device) and 0.1 us per sequence for the second launch and the records.  (Measured over
-// batches of 1 to 64 and lengths of 64 to 8192 for five head layouts: one token over 513 keys, 24/4 heads: 6.7 and 6.0 us,
-// 64 sequences of 512 keys, 16/2 heads: 17.8 and 9.9.)  Lengths on the device are not known here: the longest sequence is
+// batches of 1 to 64 and lengths of 64 to 8192 for five head layouts: one token over 513 keys, 24/4 heads: 6.7 and 5.1 us,
+// 64 sequences of 512 keys, 16/2 heads: 17.8 and 9.9.  With 5.2, as it was before the records' way was shortened, one token over 2929 and
+// 3768 keys, 24/4 heads, took 9.7 and 9.9 by shares, 7.6 and 8.4 so.)  Lengths on the device are not known here: the longest sequence is
 // taken to be as long as its bound says, or twice the mean of a packed cache, the others half of that.  If they are not and
 // one sequence holds nearly all keys, its cluster works alone: 20000 keys among 31 sequences of 400 took 52 to 228 us where
 // shares take 16 to 34.  So the form is left alone where that could cost more than 24 us and 1.3 times what shares do.
@@ -685,20 +686,22 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
     if (p->hd == 256 || (keys + csize * step - 1) / (csize * step) >= (keys + finishers * step - 1) / (finishers * step)) csize = finishers;
     const double per_key = p->nkv * p->hd * 4.0;
     auto t_shares = [&](double k) { return (p->kv_len ? 8.0 : 7.2) + 0.1 * p->batch + k * per_key / 7.0e6; };
-    auto worth_it = [&](int size) {
+    auto worth_it = [&](int size, double more) {  // (more: us that it has to gain besides)
         const double ctas = (double)p->batch * (p->nkv / heads) * size;
         const double all = heads * p->hd >= 1024 ? 6.0e6 : 6.9e6 - 6e3 * (ds.sm_count - ctas);
         const double per_longest = heads * p->hd * 4.0 / size / (p->hd == 256 ? 93e3 : 105e3);
-        auto t_cluster = [&](double most, double k) { return 5.2 + std::max(most * per_longest, k * per_key / all); };
+        auto t_cluster = [&](double most, double k) { return more + (p->kv_len ? 4.7 : 4.1) + std::max(most * per_longest, k * per_key / all); };
         if (t_cluster(longest, total) > t_shares(total)) return false;
         if (!p->kv_len) return true;
         const double most = p->max_kv_len > 0 ? std::min((double)p->max_kv_len, (double)p->kv_rows_total) : (double)p->kv_rows_total;
         const double wide_group = G <= 8 ? 1.0 : p->hd == 256 ? 4.0 : 1.6;  // (two tiles of heads a warp: the rates are that much lower)
         return t_cluster(most * wide_group, most) <= std::max(24.0, 1.3 * t_shares(most));
     };
-    if (!worth_it(csize)) {
+    // (A power of two of CTAs where there could be more has to be well worth it: five sequences of up to 2233 keys, 16/8 heads of 256, take 14.7
+    // us in twos and 12.7 in threes.)
+    if (!worth_it(csize, csize < most_ctas ? (p->kv_len ? 0.5 : 1.1) : 0.0)) {
         csize = most_ctas;
-        if (csize == finishers || !worth_it(csize)) return;
+        if (!worth_it(csize, 0.0)) return;
     }
     // A step of a CTA is one 16-key slice for each of its warps.  Head dim 256 has room for six a head in two stages instead of
     // four in three: taken where the longest sequence then needs fewer steps, a step of s slices counted as 2 + s.  (One token
