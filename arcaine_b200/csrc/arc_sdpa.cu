@@ -283,8 +283,9 @@ static int tile_key_blocks(const arc_sdpa_prefill_params* p, int qt) {
 // out; n pairs, of which those with fewer than 128 rows count in proportion where rows are stored): a key block of a pair 1.11 +
 // 0.0022 n; records and fold 0.6 (four parts 1.2) + 0.045 n in a cluster, 2.2 + 0.073 n with a merge launch.  (256 queries of 16 heads
 // over 2304 keys: 25.6 whole, 17.1 in two parts, 15.6 in three, 18.2 in four with a merge; of 8 heads 25.5, 13.7 in four.)  Gated, the
-// epilogue of whole units takes 3.3 more, the fold in a cluster 0.5 to 1.5, the merge launch nothing (256 of 8 heads over 640 keys: 14.5
-// whole, 11.2 in three parts, 12.1 in five).
+// epilogue of whole units takes 1.4 more, the fold in a cluster as much, the merge launch little (128 of 8 heads over 700 keys: 13.8
+// whole, 10.7 in three parts, 12.1 in five).  Two blocks are not divided: the second one's scores run under the first one's softmax (128
+// queries of 8 heads over 256 keys: 7.6 whole, 7.95 in two parts).
 static long long wide_units(const arc_sdpa_prefill_params* p, int q_tiles) {
     const bool head_pair = ((p->nq / p->nkv) & 1) == 0;
     return (head_pair ? (long long)q_tiles * (p->nq / 2) : (long long)((p->seq + 255) / 256) * p->nq) * p->batch;
@@ -308,12 +309,12 @@ static int choose_wide_splits(const arc_sdpa_prefill_params* p, int q_tiles, con
     if (p->mask_type == ARC_MASK_CAUSAL && p->window > 0 && p->window < p->kv_len && !p->block_ids) most = std::min(most, (p->window + 255) / 128 + 1);
     int best = 1;
     const double rows = std::min<int>(p->seq, 128) / 128.0;
-    double least = 1.11 * most + (p->gate ? 3.3 : 0.0);
+    double least = 1.11 * most + (p->gate ? 1.4 : 0.0);
     const bool masked = p->mask_type == ARC_MASK_EXPLICIT;  // (blocks that nobody sees are not counted off: a merge launch looks better than it is)
-    for (int s = 2; s <= 8 && s <= most && units * s <= room.pairs; ++s) {
+    for (int s = 2; s <= 8 && s <= most && most > 2 && units * s <= room.pairs; ++s) {
         const double n = (double)(units * s), blocks = (1.11 + 0.0022 * n) * ((most + s - 1) / s);
         const bool fold = folds_itself(p, s, units, room);
-        const double t = p->gate ? 1.13 * ((most + s - 1) / s) + (fold ? 2.0 + 0.04 * n : 2.5 + 0.06 * n)
+        const double t = p->gate ? 1.13 * ((most + s - 1) / s) + (fold ? 2.0 + 0.04 * (0.3 + 0.7 * rows) * n : 2.5 + 0.06 * (0.3 + 0.7 * rows) * n)
                                  : blocks + (fold ? (masked ? 1.8 : s == 4 ? 1.2 : 0.6) + 0.045 * rows * n : 2.2 + 0.073 * rows * n);
         if (t < least) least = t, best = s;
     }

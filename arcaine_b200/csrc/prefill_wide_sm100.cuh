@@ -201,10 +201,15 @@ __device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first,
 // pair's units are about equal.
 // few > 0: the first `few` pairs share the longest units [0, few_end) in that way and the others the rest, of which they take
 // one more each.
+template <bool ONE>  // one unit a pair: the walk ends behind it
 struct WideCursor {
     int w, i;
     __device__ __forceinline__ explicit WideCursor(const PrefillParams& p) : i(-1) { advance(p); }
     __device__ __forceinline__ void advance(const PrefillParams& p) {
+        if constexpr (ONE) {
+            w = ++i == 0 ? (int)(blockIdx.x >> 1) : 0x7fffffff;
+            return;
+        }
         const int place = (int)(blockIdx.x >> 1);
         const bool rest = place >= p.few;  // (few is 0 where nothing is divided in this way)
         const int base = rest ? p.few_end : 0, first = rest ? place - p.few : place;
@@ -215,8 +220,8 @@ struct WideCursor {
 };
 
 // The unit at the cursor, without its key blocks: nothing here depends on memory.
-template <bool SPLIT>
-__device__ __forceinline__ WideWork wide_place(const PrefillParams& p, const WideCursor& cur, int rank) {
+template <bool SPLIT, bool ONE>
+__device__ __forceinline__ WideWork wide_place(const PrefillParams& p, const WideCursor<ONE>& cur, int rank) {
     WideWork t;
     int qt;
     t.part = SPLIT ? cur.w % p.num_splits : 0;
@@ -258,8 +263,8 @@ __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int ran
 // MASKED: with an additive mask, as mask_scan_kernel has read it.  (With SPLIT: few queries over a long cache.  16 of 8 heads
 // over 32768 keys take 299 us as whole units and 59 in parts; 64 over 4096 keys 45 and 18.)
 // SPLIT: a unit is one of num_splits parts of the key blocks, one unit per pair, for calls whose tiles would leave most
-// pairs idle.  The part's normalised rows go to the partial records as f32 with their log-sum-exp.  SPLIT 2: two or three parts
-// are the pairs of one cluster; each CTA stores only the columns the other parts' CTAs finish, and after a cluster
+// pairs idle.  The part's normalised rows go to the partial records as f32 with their log-sum-exp.  SPLIT 2: two to four
+// parts are the pairs of one cluster; each CTA stores only the columns the other parts' CTAs finish, and after a cluster
 // barrier finishes its own columns.  SPLIT 1: more parts are folded by sdpa_uniform_merge_kernel.  The values pass through L2:
 // read out of the other CTAs' shared memory, 11 bytes per clk and SM, the fold took 5 us.  Every instruction here runs
 // once per launch and is fetched cold, 50 clk per 128 bytes of code, so there are few: with rows divided instead of columns, which
@@ -271,6 +276,8 @@ __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int ran
 // VISION: causal with vision blocks (p.ids).  Where pairs take several units the next unit's blocks and rows are looked up by warps
 // that wait anyway: between two units the look-up cost the softmax warps 2200 clk and the scores behind it as much.  (1531 tokens of
 // 16/8 heads with three images 24.4 -> 23.2 us.)
+// Parts, and calls without a gate that are not EARLY, have one unit a pair: ONE takes the walks out of every role, which small calls
+// waited for (161 queries of 24/4 heads over 202 keys 8.28 -> 7.74 us, 64 of 16/8 over 64 6.81 -> 6.29).
 template <bool GATE, bool MASKED, int SPLIT = 0, bool EARLY = false, bool VISION = false>
 __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     sdpa_prefill_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -278,6 +285,8 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                              const __grid_constant__ CUtensorMap tm_gate, const PrefillParams p) {
     using C = WideCfg;
     constexpr int HD = C::HD;
+    constexpr bool ONE = SPLIT != 0 || (!GATE && !EARLY);  // one unit a pair
+    using Cursor = WideCursor<ONE>;
     extern __shared__ __align__(1024) uint8_t smem[];  // (the swizzle pattern follows the address bits)
     uint8_t* sQ = smem;
     uint8_t* sK = sQ + C::Q_BYTES;               // [STAGES]
@@ -334,7 +343,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     constexpr bool blocks_in_memory = MASKED || VISION;
     WideWork w_first{};
     if (warp == C::EPILOGUE_WARP) {
-        w_first = wide_place<SPLIT != 0>(p, WideCursor(p), rank);
+        w_first = wide_place<SPLIT != 0>(p, Cursor(p), rank);
         if (!blocks_in_memory) wide_find_blocks<MASKED, SPLIT != 0, VISION>(p, rank, w_first);
         if (lane == 0) *first_unit = w_first;
     }
@@ -397,8 +406,8 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     tc_fence_after_sync();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);
     const int total = *abort_slot ? 0 : (int)(blockIdx.x >> 1) < p.few ? p.few_end : p.total_tiles;  // a status is set: walk an empty list
-    auto unit_at = [&](const WideCursor& cur) {
-        if (SPLIT || cur.i == 0) return *first_unit;
+    auto unit_at = [&](const Cursor& cur) {
+        if (ONE || cur.i == 0) return *first_unit;
         WideWork w = wide_place<SPLIT != 0>(p, cur, rank);
         wide_find_blocks<MASKED, SPLIT != 0, VISION>(p, rank, w);
         return w;
@@ -529,10 +538,10 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             return false;
         };
         // (vision blocks: the next unit's are looked up while this one's first blocks are worked on)
-        WideCursor cur(p);
+        Cursor cur(p);
         WideWork w_next{};
         auto look_ahead = [&]() {
-            WideCursor after = cur;
+            Cursor after = cur;
             after.advance(p);
             if (after.w < total) w_next = unit_at(after);
         };
@@ -616,7 +625,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 ++gs;
                 return true;
             };
-            WideCursor cur(p);
+            Cursor cur(p);
             auto next_unit = [&](WideWork& w) -> bool {  // the cursor's unit, or the first one after it with key blocks
                 for (; cur.w < total; cur.advance(p)) {
                     w = unit_at(cur);
@@ -684,11 +693,11 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         [[maybe_unused]] const uint32_t b_empty = map_to_cta(smem_u32(o_empty), lead);
         int n = 0;  // units with key blocks so far
         OutStage stage{sOut + quarter * STAGE_WARP_BYTES, &gate_bar[2 * quarter], 0u, 0, 0, 0, 0, HD / 64};
-        WideCursor cur(p);
+        Cursor cur(p);
         for (; cur.w < total; cur.advance(p)) {
             const WideWork w = unit_at(cur);
             if (VISION) {  // for the softmax warps, whose look-up would come between two units
-                WideCursor after = cur;
+                Cursor after = cur;
                 after.advance(p);
                 if (after.w < total) {
                     const WideWork wn = unit_at(after);
@@ -722,7 +731,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             // tokens of 16/8 heads 20.2 -> 18.7, 2000 of 8/2 28.9 -> 27.2, 64 10.1 -> 8.4.)
             bool last = false;
             if (GATE && !SPLIT) {
-                WideCursor after = cur;
+                Cursor after = cur;
                 after.advance(p);
                 last = after.w >= total;
                 stage.rounds = last ? HD / 128 : HD / 64;
@@ -805,7 +814,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         int g = 0, n = 0;  // key blocks and units so far
         bool ok = true;
         uint32_t s0[32], s1[32], s2[32], s3[32];  // the row's 128 scores of the current block
-        WideCursor cur(p);
+        Cursor cur(p);
         for (; ok && cur.w < total; cur.advance(p)) {
             const bool looked_up = VISION && cur.i > 0;
             int row_end = 0;
@@ -951,7 +960,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 mbar_arrive_warp(&fin[n & 3]);
                 ++n;
                 if constexpr (GATE && SPLIT == 0) {
-                    WideCursor after = cur;
+                    Cursor after = cur;
                     after.advance(p);
                     if (after.w >= total) {  // (in what was Q's shared memory)
                         OutStage half{smem + quarter * STAGE_WARP_BYTES, &gate_late[2 * quarter], 0u, 0, 0, 0, HD / 2, HD / 128};

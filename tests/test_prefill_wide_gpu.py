@@ -327,3 +327,33 @@ def test_parts_of_the_key_range(parts, batch, seq, kv, nq, nkv, window):
     for _ in range(10):
         assert torch.equal(run(parts), out)
     assert ops.device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("batch,seq,kv,nq,nkv,window", [
+    (1, 128, 1000, 16, 8, oracle.INT_MAX),  # every row of both tiles, the last key block ragged
+    (1, 200, 1500, 3, 3, oracle.INT_MAX),   # odd group, 256 tokens a unit: the second tile ragged
+    (1, 1, 512, 8, 2, oracle.INT_MAX),      # one row in each tile, one key block a part
+    (3, 100, 900, 4, 2, oracle.INT_MAX),    # three sequences
+    (1, 130, 2000, 3, 3, 700),              # a window: rows that see nothing of a part; odd group
+])
+def test_four_parts_fold_themselves(batch, seq, kv, nq, nkv, window):
+    """Where the library chooses four parts, not gated, their cluster folds them: one launch, as the whole range gives it."""
+    from arcaine_b200 import ops
+    ops.clear_device_status()
+    mask = 3 if window != oracle.INT_MAX else 0
+    q, k, v = (seeded_bf16(batch, n, h, 256, seed=130 + i).cuda() for i, (n, h) in enumerate([(seq, nq), (kv, nkv), (kv, nkv)]))
+    copy = torch.empty_like(q)
+    run = lambda n: ops.sdpa_prefill(q, k, v, scale=0.0625, mask_type=mask, window=window, num_splits=n, return_lse=True,  # noqa: E731
+                                     out_copies=torch.tensor([copy.data_ptr()], device="cuda"))
+    want, want_lse = run(1)
+    before = ops.launch_count()
+    out, lse = run(0)
+    assert ops.launch_count() - before == 1 and not torch.equal(lse, want_lse)  # in parts, without a merge launch
+    # the same values but for the bf16 rounding of the probabilities, whose reference a part chooses for itself
+    assert_close(out, want.float().cpu(), "out", rel_tol=4e-3, abs_tol=1.6e-2)
+    assert torch.equal(copy, out)
+    fin = torch.isfinite(want_lse)
+    assert torch.equal(torch.isfinite(lse), fin) and torch.allclose(lse[fin], want_lse[fin], atol=2e-3)
+    for _ in range(10):
+        assert torch.equal(run(0)[0], out)
+    assert ops.device_status() == (0, 0)
