@@ -120,9 +120,13 @@ static WideKernel wide_kernel(bool gate, bool masked, int split, bool several, b
     if (split == 2 && gate) return masked ? sdpa_prefill_wide_kernel<true, true, 2> : vision ? sdpa_prefill_wide_kernel<true, false, 2, false, true> : sdpa_prefill_wide_kernel<true, false, 2>;
     if (split == 2) return masked ? sdpa_prefill_wide_kernel<false, true, 2> : vision ? sdpa_prefill_wide_kernel<false, false, 2, false, true> : sdpa_prefill_wide_kernel<false, false, 2>;
     if (split == 1) return masked ? sdpa_prefill_wide_kernel<false, true, 1> : vision ? sdpa_prefill_wide_kernel<false, false, 1, false, true> : sdpa_prefill_wide_kernel<false, false, 1>;
-    if (masked) return gate ? sdpa_prefill_wide_kernel<true, true> : several ? sdpa_prefill_wide_kernel<false, true, 0, true> : sdpa_prefill_wide_kernel<false, true>;
-    if (vision) return gate ? sdpa_prefill_wide_kernel<true, false, 0, false, true> : sdpa_prefill_wide_kernel<false, false, 0, true, true>;
-    return gate ? sdpa_prefill_wide_kernel<true, false> : several ? sdpa_prefill_wide_kernel<false, false, 0, true> : sdpa_prefill_wide_kernel<false, false>;
+    if (several || vision) {  // (979 tokens with four images, one unit a pair: 17.4 us, 17.75 without the walks)
+        if (masked) return gate ? sdpa_prefill_wide_kernel<true, true, 0, true> : sdpa_prefill_wide_kernel<false, true, 0, true>;
+        if (vision) return gate ? sdpa_prefill_wide_kernel<true, false, 0, true, true> : sdpa_prefill_wide_kernel<false, false, 0, true, true>;
+        return gate ? sdpa_prefill_wide_kernel<true, false, 0, true> : sdpa_prefill_wide_kernel<false, false, 0, true>;
+    }
+    if (masked) return gate ? sdpa_prefill_wide_kernel<true, true> : sdpa_prefill_wide_kernel<false, true>;
+    return gate ? sdpa_prefill_wide_kernel<true, false> : sdpa_prefill_wide_kernel<false, false>;
 }
 
 // One-time set-up for the current device: status-word address, SM count, and the

@@ -270,22 +270,23 @@ __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int ran
 // once per launch and is fetched cold, 50 clk per 128 bytes of code, so there are few: with rows divided instead of columns, which
 // had to go through shared memory on either side, 13000 clk passed from the last P V to the end  (us: 256 queries of 16 heads over
 // 2304 keys 18.0 -> 15.7, 512 over 2560 23.5 -> 20.7, 512 of 8 heads over 1512 15.5 -> 13.1.)
-// EARLY (not gated): pairs take several units.  The epilogue then empties the accumulator into registers first (1600 clk), for the
+// SEVERAL: pairs take several units.  EARLY (SEVERAL, not gated): the epilogue empties the accumulator into registers first (1600 clk), for the
 // next unit's P V to go on; in turns, with the way out of the SM between them, it took 3000.  (2 x 5000 tokens of 16/8 heads,
 // window 512, 103 -> 96 us.  Gated rows wait for sigmoids, not for the way out: taken early they cost calls of short units 8 %.)
 // VISION: causal with vision blocks (p.ids).  Where pairs take several units the next unit's blocks and rows are looked up by warps
 // that wait anyway: between two units the look-up cost the softmax warps 2200 clk and the scores behind it as much.  (1531 tokens of
 // 16/8 heads with three images 24.4 -> 23.2 us.)
-// Parts, and calls without a gate that are not EARLY, have one unit a pair: ONE takes the walks out of every role, which small calls
-// waited for (161 queries of 24/4 heads over 202 keys 8.28 -> 7.74 us, 64 of 16/8 over 64 6.81 -> 6.29).
-template <bool GATE, bool MASKED, int SPLIT = 0, bool EARLY = false, bool VISION = false>
+// ONE: not SEVERAL, one unit a pair.  The walks are then left out of every role; small calls waited for them (161 queries of 24/4 heads over
+// 202 keys 8.28 -> 7.74 us, gated 9.92 -> 9.33; 64 of 16/8 over 64 6.81 -> 6.29).
+template <bool GATE, bool MASKED, int SPLIT = 0, bool SEVERAL = false, bool VISION = false>
 __global__ void __launch_bounds__(WideCfg::THREADS, 1)
     sdpa_prefill_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_out,
                              const __grid_constant__ CUtensorMap tm_gate, const PrefillParams p) {
     using C = WideCfg;
     constexpr int HD = C::HD;
-    constexpr bool ONE = SPLIT != 0 || (!GATE && !EARLY);  // one unit a pair
+    constexpr bool ONE = !SEVERAL, EARLY = SEVERAL && !GATE;
+    static_assert(!(SPLIT && SEVERAL), "a part is a pair's only unit");
     using Cursor = WideCursor<ONE>;
     extern __shared__ __align__(1024) uint8_t smem[];  // (the swizzle pattern follows the address bits)
     uint8_t* sQ = smem;
@@ -828,7 +829,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             const WideWork w = looked_up ? *next_place : unit_at(cur);
             if (looked_up) mbar_arrive_warp(next_empty);
             if (w.hi == w.lo) {
-                if (SPLIT) break;  // (its only one; with the place read again below, nothing is spilled: a canvas step 17.9 us, 17.6 so)
+                if (SPLIT) break;  // (its only one; its place is read again below, not kept through the blocks: a canvas step 17.9 us, 17.6 so)
                 continue;
             }
             const int t = w.q0 + r;
