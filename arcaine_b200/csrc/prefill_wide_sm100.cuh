@@ -966,9 +966,13 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                     if (after.w >= total) {  // (in what was Q's shared memory)
                         OutStage half{smem + quarter * STAGE_WARP_BYTES, &gate_late[2 * quarter], 0u, 0, 0, 0, HD / 2, HD / 128};
                         const int t0 = w.q0 + quarter * 32;
-                        // (The unit before may not have got its P V yet, whose parity is the one before; the one before that has: its P V
-                        // went ahead of this unit's scores.)
-                        if ((n > 1 && !mbar_wait_inline(o_full, n & 1)) || !mbar_wait_inline(o_full, (n - 1) & 1)) {
+                        // The unit's last P V has landed: by the V stage that it releases, not by o_full.  A wait on a parity tells two
+                        // states of a barrier apart.  Of the stage's these two are left, open or released by this block: the block
+                        // before the previous one, which had the stage before, released it ahead of this block's scores, whose MMAs
+                        // came behind its P V.  o_full, a phase a unit, may be in three: the unit before still open (a short unit's
+                        // scores run ahead of it), or done, or this one done as well, which looks like the first: a wait for the unit
+                        // before, and then for this one, ran out where this warp came to it late.
+                        if (!mbar_wait_inline(&v_empty[(g - 1) & 1], ((g - 1) >> 1) & 1)) {
                             if (lane == 0) report_fault(p.fault, FAULT_WAIT_O, 0x800u);
                             break;
                         }
