@@ -650,14 +650,15 @@ __global__ void __launch_bounds__(288, 1)
         };
         uint32_t gw = p.gate && (int)threadIdx.x < items ? *reinterpret_cast<const uint32_t*>(p.gate + offset_of(threadIdx.x)) : 0u;
         __syncwarp();
-        bool fine = true;
-        if (EVEN && p.ncta == 1) __syncthreads();
-        else fine = mbar_wait_cluster(gathered, 0);
-        if (!fine) {
-            if (lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x10000u);
+        // Whether the records came is settled for the whole CTA before any warp goes on: each warp waits by its own clock, and
+        // one that gave up stood at the cluster's barrier while another, whose last look found them, stood at the CTA's.
+        const bool came = (EVEN && p.ncta == 1) || mbar_wait_cluster(gathered, 0);
+        if (!__syncthreads_and(came)) {
+            if (!came && lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x10000u);
             cluster_sync_all();  // (what is still under way here arrives before the other CTAs have gone)
+            return;
         }
-        fine = __all_sync(0xffffffffu, fine && ((lane & 7) >= p.ncta || cflag[lane & 7] != 0.f));
+        const bool fine = __all_sync(0xffffffffu, (lane & 7) >= p.ncta || cflag[lane & 7] != 0.f);  // (the same in every warp)
         // The CTAs' weights of a row: eight lanes.
 #pragma unroll 1
         for (int n0 = warp * 4; n0 < rows; n0 += (ncw + 1) * 4) {

@@ -231,8 +231,9 @@ __device__ __forceinline__ void mbar_arrive_remote_warp(uint32_t remote_bar) {
         : "memory");
 }
 
-// A whole warp waits for a phase that other CTAs of the cluster complete, and sees what they wrote for it.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, long long limit_cycles = 2000000000LL) {
+// A whole warp waits for a phase that other CTAs of the cluster complete, and sees what they wrote for it.  (Three times the limit
+// of the waits for copies: a CTA that gives one of those up still completes its part of the phase.)
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, long long limit_cycles = 6000000000LL) {
     const long long t0 = clock64();
     do {
         uint32_t ok;

@@ -55,3 +55,19 @@ def test_last_unit_of_the_gated_cta_pairs(blocks, wait):
         assert stuck(0, 0, 0, 0)
     else:
         assert not stuck(0, 0, 0, 0)
+
+
+@pytest.mark.parametrize("verdict", ["a warp's", "the CTA's"])
+@pytest.mark.parametrize("came", [(True, True), (True, False), (False, True), (False, False)])
+def test_records_of_a_decode_cluster_that_come_late(verdict, came):
+    """sdpa_decode_kernel, CLUSTER: two warps of a CTA have waited for the other CTAs' records, each by its own clock.  A warp that
+    goes without them takes the cluster's barrier, which takes all threads that have not left; one that goes on takes the
+    CTA's.  (Decided by each warp for itself, the two wait for one another for good.)"""
+    if verdict == "the CTA's":  # __syncthreads_and, and who goes without leaves behind the cluster's barrier
+        ways = [["cta", "cta"] if all(came) else ["cta", "cluster"]] * 2
+    else:
+        ways = [["cta"] if c else ["cluster", "cta"] for c in came]
+    ways = [list(w) for w in ways]
+    while any(ways) and all(w and w[0] == ways[0][0] for w in ways):  # a barrier opens when all who have not left are there
+        ways = [w[1:] for w in ways]
+    assert (not any(ways)) == (verdict == "the CTA's" or len(set(came)) == 1)
