@@ -268,7 +268,7 @@ def test_vision_blocks_longer_than_a_search_step():
     (1, 1500, 1500, 24, 4, 400, False, True),   # vision blocks, looked up a unit ahead
     (1, 900, 500, 48, 8, 0, False, True),       # and tiles that see nothing between others
     (1, 900, 500, 48, 8, 0, True, True),        # gated
-    (40, 100, 100, 8, 4, 0, True, False),       # gated units of one key block, whose scores run ahead of the unit before
+    (20, 130, 128, 8, 4, 0, True, False),       # gated units of one key block, whose scores run ahead of the unit before
 ])
 def test_several_units_a_pair(batch, seq, kv, nq, nkv, window, gate, vision):
     """More units than pairs: the accumulator freed ahead of the output, the two kinds of pairs, the look-up of the next unit."""
