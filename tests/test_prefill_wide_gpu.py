@@ -297,6 +297,22 @@ def test_several_units_a_pair(batch, seq, kv, nq, nkv, window, gate, vision):
         assert_close(out[b].reshape(-1, hd)[rows], want[1].float() if gate else want[0], f"sequence {b}")
 
 
+@pytest.mark.parametrize("seq,kv,nq,nkv,gate,parts", [
+    (1664, 1664, 24, 4, False, 1), (1664, 1664, 24, 4, True, 1),  # several units a pair
+    (161, 202, 24, 4, False, 1), (256, 1100, 8, 4, False, 3), (256, 1100, 8, 4, False, 8),  # one; parts in both forms
+])
+def test_results_below_the_smallest_normal_number(seq, kv, nq, nkv, gate, parts):
+    """V times a power of two: the results times the same, but for the rounding of bf16 down there (half of 2^-133) and of the
+    results it is compared with (2^-9 of 2^-126 at most)."""
+    from arcaine_b200 import ops
+    q, k, v, g = (seeded_bf16(n, h, 256, seed=140 + i).cuda() for i, (n, h) in enumerate([(seq, nq), (kv, nkv), (kv, nkv), (seq, nq)]))
+    v = (v * 2.0 ** -124).bfloat16()
+    run = lambda v: ops.sdpa_prefill(q, k, v, scale=0.0625, mask_type=3 if seq > 256 else 0, num_splits=parts, gate=g if gate else None).double()  # noqa: E731
+    got, want = run(v), run((v.float() * 2.0 ** 124).bfloat16()) * 2.0 ** -124
+    small = want.abs() < 2.0 ** -126
+    assert small.float().mean() > 0.3 and (got - want)[small].abs().max() <= 2.0 ** -133 * (2 if gate else 1)  # (gated: rounded twice)
+
+
 @pytest.mark.parametrize("parts", [2, 3, 4, 8])
 @pytest.mark.parametrize("batch,seq,kv,nq,nkv,window", [
     (1, 256, 1100, 8, 4, oracle.INT_MAX),  # two row tiles of pairs of heads, the last key block ragged
