@@ -511,7 +511,9 @@ __global__ void __launch_bounds__(288, 1)
                     float z = wt * ml.y;
 #pragma unroll
                     for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-                    if (some) rec_w[at] = wt;
+                    // (2^-6, taken back with the CTAs' weights: up to 64 records are added up before their sum of weights is
+                    // divided by, and values that a record of its own can hold must not run over in between.)
+                    if (some) rec_w[at] = wt * 0.015625f;
                     float2* to = cml + blockIdx.x * rows2 + hl * G + n;
                     if (n < G && s < finishers) {
                         if (alone) *to = make_float2(mx, z);
@@ -672,7 +674,7 @@ __global__ void __launch_bounds__(288, 1)
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
             if (n < rows) {
-                cweight[n * 8 + c] = z > 0.f ? __fdividef(wt, z) : 0.f;
+                cweight[n * 8 + c] = z > 0.f ? __fdividef(wt * 64.f, z) : 0.f;
                 if (p.out_lse && fine && blockIdx.x == 0 && c == 0)
                     p.out_lse[(long long)b * p.nq + head0 * G + n] = z > 0.f ? (mx + fast_log2(z)) * 0.6931471805599453f : -CUDART_INF_F;
             }

@@ -462,6 +462,23 @@ def test_one_launch_form_of_any_group(ops, B, nq, nkv, hd, n):
     check_ragged_batch(ops, q, k, v, g, lens)
 
 
+@pytest.mark.parametrize("B,nq,nkv,hd,n,warp_keys", [
+    (12, 16, 2, 128, 1700, 64), (2, 32, 2, 128, 700, 32), (5, 24, 4, 256, 900, 96), (1, 8, 8, 256, 1501, 64),  # clusters
+    (16, 8, 8, 256, 270, 64),  # a CTA alone
+])
+def test_one_launch_form_keeps_values_that_its_records_can_hold(ops, B, nq, nkv, hd, n, warp_keys):
+    """All scores zero, all values as large as the sum over a warp's keys, of which there are `warp_keys` at most, lets them be: the
+    result is that value, whatever the sum over the CTA's keys."""
+    q, k = torch.zeros(B, nq, hd, dtype=torch.bfloat16), seeded_bf16(B, n, nkv, hd, seed=720)
+    value = torch.tensor(3.3e38 / warp_keys).bfloat16()
+    v = value.expand(B, n, nkv, hd).contiguous()
+    before = ops.launch_count()
+    out, o32, lse = ops.sdpa_decode(q.cuda(), k.cuda(), v.cuda(), scale=0.1, kv_len=n, return_partial=True)
+    assert ops.launch_count() - before == 1
+    assert (out == value.cuda()).all() and ((o32 / value.float().cuda() - 1).abs() <= 1e-6).all()
+    assert torch.allclose(lse.cpu(), torch.full((B, nq), n, dtype=torch.float32).log(), atol=1e-6)
+
+
 @pytest.mark.parametrize("B,nq,nkv,total", [
     (5, 24, 4, 7600),   # 20 clusters of six CTAs in steps of six slices
     (12, 16, 2, 7600),  # 24 of five, groups of eight heads
