@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(288, 1)
             if (n < rows) {
                 cweight[n * 8 + c] = z > 0.f ? __fdividef(wt * 64.f, z) : 0.f;
                 if (p.out_lse && fine && blockIdx.x == 0 && c == 0)
-                    p.out_lse[(long long)b * p.nq + head0 * G + n] = z > 0.f ? (mx + fast_log2(z)) * 0.6931471805599453f : -CUDART_INF_F;
+                    p.out_lse[(long long)b * p.nq + head0 * G + n] = z > 0.f ? fmaf(mx, 0.6931471805599453f, logf(z)) : -CUDART_INF_F;
             }
         }
         __syncthreads();

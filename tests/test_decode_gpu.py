@@ -479,6 +479,21 @@ def test_one_launch_form_keeps_values_that_its_records_can_hold(ops, B, nq, nkv,
     assert torch.allclose(lse.cpu(), torch.full((B, nq), n, dtype=torch.float32).log(), atol=1e-6)
 
 
+@pytest.mark.parametrize("B,nq,nkv,hd,n", [(12, 16, 2, 128, 1700), (5, 24, 4, 256, 900), (1, 24, 4, 256, 600)])
+def test_one_launch_form_has_the_log_sum_exps_of_the_shares(ops, B, nq, nkv, hd, n):
+    """They are no further off than those that equal shares and a merge give (1.6 times as far with a rounding and an approximate
+    logarithm more)."""
+    q, k, v = (seeded_bf16(*shape, seed=730 + i).cuda() for i, shape in enumerate([(B, nq, hd), (B, n, nkv, hd), (B, n, nkv, hd)]))
+    want = torch.einsum("bhgd,bnhd->bhgn", q.double().view(B, nkv, -1, hd), k.double()).mul(hd ** -0.5).logsumexp(-1).view(B, nq)
+    off, launches = [], []
+    for ctas in (0, 148):
+        before = ops.launch_count()
+        lse = ops.sdpa_decode(q, k, v, scale=hd ** -0.5, kv_len=n, num_ctas=ctas, return_partial=True)[2]
+        launches.append(ops.launch_count() - before)
+        off.append((lse.double() / want - 1).square().mean().sqrt().item())
+    assert launches == [1, 2] and off[0] <= 1.25 * off[1], off
+
+
 @pytest.mark.parametrize("B,nq,nkv,total", [
     (5, 24, 4, 7600),   # 20 clusters of six CTAs in steps of six slices
     (12, 16, 2, 7600),  # 24 of five, groups of eight heads
