@@ -674,9 +674,11 @@ __global__ void __launch_bounds__(288, 1)
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
             if (n < rows) {
-                cweight[n * 8 + c] = z > 0.f ? __fdividef(wt * 64.f, z) : 0.f;
+                // (A sum of weights that is no number, as scores make it that are none, goes on to the log-sum-exp: -inf beside such
+                // a row would say that it is empty, and who merges it with others would leave it out.)
+                cweight[n * 8 + c] = z == 0.f ? 0.f : __fdividef(wt * 64.f, z);
                 if (p.out_lse && fine && blockIdx.x == 0 && c == 0)
-                    p.out_lse[(long long)b * p.nq + head0 * G + n] = z > 0.f ? fmaf(mx, 0.6931471805599453f, logf(z)) : -CUDART_INF_F;
+                    p.out_lse[(long long)b * p.nq + head0 * G + n] = z == 0.f ? -CUDART_INF_F : fmaf(mx, 0.6931471805599453f, logf(z));
             }
         }
         __syncthreads();

@@ -494,6 +494,27 @@ def test_one_launch_form_has_the_log_sum_exps_of_the_shares(ops, B, nq, nkv, hd,
     assert launches == [1, 2] and off[0] <= 1.25 * off[1], off
 
 
+@pytest.mark.parametrize("B,nq,nkv,hd,n", [(12, 16, 2, 128, 1700), (2, 32, 2, 128, 700), (1, 24, 4, 256, 600), (30, 25, 5, 128, 200)])
+def test_one_launch_form_hands_on_what_is_no_number(ops, B, nq, nkv, hd, n):
+    """A query, or a key, that is none: NaN in the results and in the log-sum-exps of the heads that see it, so that a merge with
+    another part keeps it; the other heads, and a head whose keys all score -inf, as ever."""
+    q, k, v = (seeded_bf16(*shape, seed=740 + i).cuda() for i, shape in enumerate([(B, nq, hd), (B, n, nkv, hd), (B, n, nkv, hd)]))
+    G = nq // nkv
+    q[:, 1, 5] = float("nan")  # a head of the first group
+    k[0, n // 2, nkv - 1, 3] = float("nan")  # the last group of the first sequence
+    out, o32, lse = ops.sdpa_decode(q, k, v, scale=hd ** -0.5, kv_len=n, return_partial=True)
+    bad = torch.zeros(B, nq, dtype=torch.bool, device="cuda")
+    bad[:, 1] = True
+    bad[0, nq - G:] = True
+    assert torch.equal(lse.isnan(), bad) and torch.equal(o32.isnan(), bad[..., None].expand_as(o32)) and torch.equal(out.isnan(), o32.isnan())
+    part = torch.randn(1, B * nq, hd, device="cuda"), torch.zeros(1, B * nq, device="cuda")
+    merged = ops.sdpa_merge(torch.cat([o32.view(1, -1, hd), part[0]]), torch.cat([lse.view(1, -1), part[1]]))
+    assert torch.equal(merged.view(B, nq, hd).isnan(), o32.isnan())
+    q[:, 1], q[..., 0], k[0, n // 2, nkv - 1, 3], k[..., 0] = 0.0, 1.0, 0.0, -float("inf")
+    out, o32, lse = ops.sdpa_decode(q, k, v, scale=hd ** -0.5, kv_len=n, return_partial=True)
+    assert not out.any() and not o32.any() and (lse == -float("inf")).all()
+
+
 @pytest.mark.parametrize("B,nq,nkv,total", [
     (5, 24, 4, 7600),   # 20 clusters of six CTAs in steps of six slices
     (12, 16, 2, 7600),  # 24 of five, groups of eight heads
