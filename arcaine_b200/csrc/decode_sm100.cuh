@@ -222,7 +222,9 @@ __global__ void __launch_bounds__(288, 1)
     // Up to here nothing depends on the kernels in front; everything below may.
     grid_dependency_wait();
     int asked = 0;
-    if (CLUSTER && warp == ncw && !p.kv_row_offset) {
+    // (Not where the sequence is known to end in front of it.)
+    bool no_step = known && my_len <= (int)blockIdx.x * tk;
+    if (CLUSTER && warp == ncw && !p.kv_row_offset && !no_step) {
         ask(0, (int)((long long)blockIdx.z * p.kv_stride_b) + (int)blockIdx.x * tk);
         asked = 1;
     }
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(288, 1)
         if (work) find_share();
     }
     if (!CLUSTER && g0 >= g1) return;
-    const bool no_step = CLUSTER && p.kv_row_offset && my_len <= (int)blockIdx.x * tk;  // (nothing has been asked for, and there are no keys)
+    no_step |= p.kv_row_offset && my_len <= (int)blockIdx.x * tk;  // (CLUSTER: nothing has been asked for, and there are no keys)
     // keys before sequence b / up to its end, in the count g0 and g1 use
     auto seq_begin = [&](int b) { return CLUSTER ? 0ll : cum[b]; };
     auto seq_end = [&](int b) { return CLUSTER ? (long long)my_len : cum[b + 1]; };
