@@ -282,14 +282,7 @@ static int tile_key_blocks(const arc_sdpa_prefill_params* p, int qt) {
     return std::max(0, hi - lo);
 }
 
-// Head dim 256: units of the CTA pairs' list, and how many parts the key range of each is worth when the units alone
-// would leave pairs idle.  Measured over 64 to 512 rows of 4 to 24 heads and 384 to 8000 keys (us, what all calls have in common left
-// out; n pairs, of which those with fewer than 128 rows count in proportion where rows are stored): a key block of a pair 1.11 +
-// 0.0022 n; records and fold 0.6 (four parts 1.2) + 0.045 n in a cluster, 2.2 + 0.073 n with a merge launch.  (256 queries of 16 heads
-// over 2304 keys: 25.6 whole, 17.1 in two parts, 15.6 in three, 18.2 in four with a merge; of 8 heads 25.5, 13.7 in four.)  Gated, the
-// epilogue of whole units takes 1.4 more, the fold in a cluster as much, the merge launch little (128 of 8 heads over 700 keys: 13.8
-// whole, 10.7 in three parts, 12.1 in five).  Two blocks are not divided: the second one's scores run under the first one's softmax (128
-// queries of 8 heads over 256 keys: 7.6 whole, 7.95 in two parts).
+// Head dim 256: units of the CTA pairs' list.
 static long long wide_units(const arc_sdpa_prefill_params* p, int q_tiles) {
     const bool head_pair = ((p->nq / p->nkv) & 1) == 0;
     return (head_pair ? (long long)q_tiles * (p->nq / 2) : (long long)((p->seq + 255) / 256) * p->nq) * p->batch;
@@ -297,29 +290,70 @@ static long long wide_units(const arc_sdpa_prefill_params* p, int q_tiles) {
 
 // Do the parts of a unit fold themselves, as one cluster?  Two and three do where all clusters fit at once; four where the library chose
 // them and there is neither gate nor additive mask (the merge launch gates for nothing, and is as good where most blocks are hidden).
+// Four that the caller asked for keep the two launches, and the bits, that they had before four could fold themselves: who gives a
+// count, unlike who leaves it to the library, may count on either.
 static bool folds_itself(const arc_sdpa_prefill_params* p, int parts, long long units, const WideRoom& room) {
     if (parts > 3 && (p->num_splits != 0 || p->gate || p->mask_type == ARC_MASK_EXPLICIT)) return false;
     return units <= room.clusters(parts);
 }
 
+// How many parts the key range of each unit is worth when the units alone would leave pairs idle: what a call takes besides what all
+// calls have in common (us; n pairs; rows: the part of a tile's 128 that there are, where they are stored).  Fitted to 20 to 512
+// rows of 4 to 24 heads over 384 to 8000 keys in every number of parts.  (256 queries of 16 heads over 2304 keys: 25.6 whole, 17.1 in
+// two parts, 15.6 in three, 18.2 in four with a merge; of 8 heads 25.5, 13.7 in four.  Gated, 128 of 8 heads over 700 keys: 13.8 whole,
+// 10.7 in three parts, 12.1 in five; three sequences of 45 queries, 4 heads, over 1000: 10.8 in three, 10.0 in four, 10.6 in eight.)
+struct WideCosts {
+    double block, block_n;                          // a part's key blocks, each
+    double whole;                                   // the epilogue of whole units
+    double fold, fold_4, fold_n, fold_rows;         // parts that fold themselves: two or three, four, per pair, per pair and rows
+    double merge, merge_more, merge_n, merge_rows;  // a merge launch: up to four parts, more, per pair, per pair and rows
+};
+constexpr WideCosts kWidePlain = {1.11, 0.0022, 0.0, 0.6, 1.2, 0.0, 0.045, 2.2, 2.2, 0.0, 0.073};
+constexpr WideCosts kWideGated = {1.4, 0.0, 1.8, 1.7, 1.7, 0.02, 0.012, 1.5, 1.8, 0.026, 0.06};
+// (Of an additive mask's blocks some are hidden, which is not known here: a block counts less.)
+constexpr WideCosts kWideMasked = {1.11, 0.0022, 0.0, 1.8, 1.8, 0.0, 0.045, 2.2, 2.2, 0.0, 0.073};
+constexpr WideCosts kWideMaskedGated = {1.13, 0.0, 1.4, 2.0, 2.0, 0.012, 0.028, 2.5, 2.5, 0.018, 0.042};
+
 static int choose_wide_splits(const arc_sdpa_prefill_params* p, int q_tiles, const WideRoom& room) {
     const long long units = wide_units(p, q_tiles);
+    if (units * 2 > room.pairs) return 1;
+    const bool masked = p->mask_type == ARC_MASK_EXPLICIT;
+    const bool windowed = p->mask_type == ARC_MASK_CAUSAL && p->window > 0 && p->window < p->kv_len && !p->block_ids;
     int most = (p->kv_len + 127) / 128;  // key blocks of the longest unit
     // What an additive mask hides is not known here.  Over the few blocks of a window the parts of 2048 rows cost 5 us more
     // than they save (256 queries of 8 heads over 2304 keys: 16.4 us whole and 21.1; with all keys seen 30.3 and 23.9); 1024
     // rows are even (64 queries of 16 heads over 4096 keys: 15.9 and 15.6; 45 and 20).  A longer cache is worth it in any case (a
     // bias per key, 128 queries of 16 heads over 4096 keys: 116 us whole).
-    if (p->mask_type == ARC_MASK_EXPLICIT && most <= 24 && (long long)p->batch * p->seq * p->nq > 1024) return 1;
-    if (p->mask_type == ARC_MASK_CAUSAL && p->window > 0 && p->window < p->kv_len && !p->block_ids) most = std::min(most, (p->window + 255) / 128 + 1);
-    int best = 1;
+    if (masked && most <= 24 && (long long)p->batch * p->seq * p->nq > 1024) return 1;
+    if (windowed) {
+        most = std::min(most, (p->window + 255) / 128 + 1);
+        // (That is the most that a window can cover, up to two more than it does.  Gated calls, whose epilogue and merge weigh more, are
+        // divided by what it does: 256 queries of 8 heads over 1500 keys, window 533, 11.5 us in three parts, 13.2 in four.  For the others
+        // the bound is the better guess: 63 of 24 heads over 1000 keys 9.9 in four, 10.4 in three.)
+        if (p->gate) {
+            const int tiles = ((p->nq / p->nkv) & 1) == 0 ? 1 : 2;  // token tiles of a unit
+            int seen = 0;
+            for (int qt = 0; qt < q_tiles; qt += tiles) {
+                const int last = std::min(q_tiles, qt + tiles) - 1, blocks = tile_key_blocks(p, last);
+                seen = std::max(seen, blocks + (last > qt && blocks > 0 ? 1 : 0));
+            }
+            most = std::min(most, seen);
+        }
+    }
+    // Two blocks are not divided: the second one's scores run under the first one's softmax (128 queries of 8 heads over 256 keys: 7.6
+    // whole, 7.95 in two parts).
+    if (most <= 2) return 1;
+    const WideCosts& c = masked ? (p->gate ? kWideMaskedGated : kWideMasked) : p->gate ? kWideGated : kWidePlain;
     const double rows = std::min<int>(p->seq, 128) / 128.0;
-    double least = 1.11 * most + (p->gate ? 1.4 : 0.0);
-    const bool masked = p->mask_type == ARC_MASK_EXPLICIT;  // (blocks that nobody sees are not counted off: a merge launch looks better than it is)
-    for (int s = 2; s <= 8 && s <= most && most > 2 && units * s <= room.pairs; ++s) {
-        const double n = (double)(units * s), blocks = (1.11 + 0.0022 * n) * ((most + s - 1) / s);
-        const bool fold = folds_itself(p, s, units, room);
-        const double t = p->gate ? 1.13 * ((most + s - 1) / s) + (fold ? 2.0 + 0.04 * (0.3 + 0.7 * rows) * n : 2.5 + 0.06 * (0.3 + 0.7 * rows) * n)
-                                 : blocks + (fold ? (masked ? 1.8 : s == 4 ? 1.2 : 0.6) + 0.045 * rows * n : 2.2 + 0.073 * rows * n);
+    // Behind a window a unit's first two blocks are tested key by key, which shows where one part has both.  (45 queries of 8 heads over
+    // 663 keys, window 533: 9.8 in three parts of two blocks, 9.1 in six, 9.0 in four, whose first is one; without a window 9.05, 9.04, 8.9.)
+    const auto edge = [&](int parts) { return windowed && most / parts >= 2 ? 1.0 : 0.0; };
+    int best = 1;
+    double least = c.block * most + c.whole + edge(1);
+    for (int s = 2; s <= 8 && s <= most && units * s <= room.pairs; ++s) {
+        const double n = (double)(units * s), blocks = (c.block + c.block_n * n) * ((most + s - 1) / s) + edge(s);
+        const double t = blocks + (folds_itself(p, s, units, room) ? (s == 4 ? c.fold_4 : c.fold) + (c.fold_n + c.fold_rows * rows) * n
+                                                                   : (s > 4 ? c.merge_more : c.merge) + (c.merge_n + c.merge_rows * rows) * n);
         if (t < least) least = t, best = s;
     }
     return best;

@@ -313,6 +313,38 @@ def test_results_below_the_smallest_normal_number(seq, kv, nq, nkv, gate, parts)
     assert small.float().mean() > 0.3 and (got - want)[small].abs().max() <= 2.0 ** -133 * (2 if gate else 1)  # (gated: rounded twice)
 
 
+def chosen_parts(batch, seq, kv, nq, nkv, window=oracle.INT_MAX, gate=False):
+    """Parts of the key range that the library chooses, told by the workspace that it asks for."""
+    from arcaine_b200 import _lib
+    import ctypes as C
+    room = torch.zeros(4, dtype=torch.uint8, device="cuda")
+    p = _lib.PrefillParams()
+    p.q = p.k = p.v = p.out = room.data_ptr()
+    p.gate = room.data_ptr() if gate else None
+    p.batch, p.seq, p.kv_len, p.nq, p.nkv, p.hd = batch, seq, kv, nq, nkv, 256
+    p.q_stride_t = p.o_stride_t = nq * 256
+    p.k_stride_t = p.v_stride_t = nkv * 256
+    p.q_stride_b = p.o_stride_b = seq * nq * 256
+    p.k_stride_b = p.v_stride_b = kv * nkv * 256
+    p.scale, p.mask_type, p.window = 0.0625, 3 if window != oracle.INT_MAX else 0, window
+    need = []
+    for n in range(9):
+        p.num_splits = n
+        need.append(_lib.load().arc_sdpa_prefill_workspace_bytes(C.byref(p)))
+    return need.index(need[0], 1)
+
+
+@pytest.mark.parametrize("batch,seq,kv,nq,nkv,window,gate,parts", [
+    (1, 45, 663, 8, 4, 533, False, 4),  # behind a window (us): four parts 9.0, six 9.1, three of two masked blocks 9.8
+    (1, 63, 663, 4, 2, 533, False, 4),  # 9.3, three 10.0
+    (3, 45, 1000, 4, 2, oracle.INT_MAX, True, 4),  # gated: four 10.0, eight 10.6
+    (3, 45, 663, 4, 2, 533, True, 6),   # 9.5, three 10.55
+    (1, 256, 2304, 16, 8, oracle.INT_MAX, False, 3),  # 15.6, two 17.1
+])
+def test_parts_that_the_library_chooses(batch, seq, kv, nq, nkv, window, gate, parts):
+    assert chosen_parts(batch, seq, kv, nq, nkv, window, gate) == parts
+
+
 @pytest.mark.parametrize("parts", [2, 3, 4, 8])
 @pytest.mark.parametrize("batch,seq,kv,nq,nkv,window", [
     (1, 256, 1100, 8, 4, oracle.INT_MAX),  # two row tiles of pairs of heads, the last key block ragged
@@ -357,6 +389,7 @@ def test_four_parts_fold_themselves(batch, seq, kv, nq, nkv, window):
     """Where the library chooses four parts, not gated, their cluster folds them: one launch, as the whole range gives it."""
     from arcaine_b200 import ops
     ops.clear_device_status()
+    assert chosen_parts(batch, seq, kv, nq, nkv, window) == 4
     mask = 3 if window != oracle.INT_MAX else 0
     q, k, v = (seeded_bf16(batch, n, h, 256, seed=130 + i).cuda() for i, (n, h) in enumerate([(seq, nq), (kv, nkv), (kv, nkv)]))
     copy = torch.empty_like(q)
