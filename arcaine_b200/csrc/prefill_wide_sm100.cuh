@@ -992,20 +992,6 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
         }
     }
 
-    // SPLIT 2: this warp's half of the CTA's columns, of 32 rows, as they are: while what the others finish is on its way
-    constexpr int MOST = SPLIT == 2 ? 4 : 1;
-    uint32_t mine[MOST][GROUP];
-    int my_first = 0, my_count = 0;  // groups
-    if (SPLIT == 2 && warp < C::PRODUCER_WARP && total > 0) {
-        const WideWork w = *first_unit;
-        const int g0 = group0(w.part), g1 = group0(w.part + 1), mid = (g0 + g1 + 1) / 2;
-        my_first = warp < C::EPILOGUE_WARP ? mid : g0, my_count = (warp < C::EPILOGUE_WARP ? g1 : mid) - my_first;
-        const uint32_t tO = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + C::COL_O + my_first * GROUP;
-#pragma unroll
-        for (int k = 0; k < MOST; ++k)
-            if (k < my_count && w.hi > w.lo) tmem_ld16(tO + k * GROUP, mine[k]);
-        tmem_wait_ld();
-    }
     __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
@@ -1017,6 +1003,8 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
             const WideWork w = *first_unit;
             const int row = (warp & 3) * 32 + lane, rows = min(128, p.seq - w.q0);
             const bool live = row < rows;
+            const int g0 = group0(w.part), g1 = group0(w.part + 1), mid = (g0 + g1 + 1) / 2;
+            const int my_first = warp < C::EPILOGUE_WARP ? mid : g0, my_count = (warp < C::EPILOGUE_WARP ? g1 : mid) - my_first;  // groups
             // the others' values, all at once, and the parts' log-sum-exps
             float4 t[PARTS - 1][TAKES][4];
             float weight[PARTS], mx = -CUDART_INF_F, z = 0.f;
@@ -1044,35 +1032,39 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1)
                 p.out_lse[((long long)w.b * p.seq + w.q0 + row) * p.nq + w.h] = z > 0.f ? mx + __logf(z) : -CUDART_INF_F;
             const float iz = z > 0.f ? 1.0f / z : 0.f, row_l = fin_vals[row];
             const float own = row_l > 0.f ? weight[0] * iz / row_l : 0.f;
-            float acc[TAKES][GROUP];
-#pragma unroll
-            for (int k = 0; k < TAKES; ++k)
-#pragma unroll
-                for (int e = 0; e < GROUP; ++e) acc[k][e] = own > 0.f ? __uint_as_float(mine[k][e]) * own : 0.f;  // (an empty part's columns may hold anything)
-#pragma unroll
-            for (int s = 1; s < PARTS; ++s) {
-                const float e = weight[s] * iz;
-                if (e > 0.f) {  // (an empty part's record may hold anything)
-#pragma unroll
-                    for (int k = 0; k < TAKES; ++k)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float4 v = t[s - 1][k][i];
-                            acc[k][4 * i] = fmaf(e, v.x, acc[k][4 * i]), acc[k][4 * i + 1] = fmaf(e, v.y, acc[k][4 * i + 1]);
-                            acc[k][4 * i + 2] = fmaf(e, v.z, acc[k][4 * i + 2]), acc[k][4 * i + 3] = fmaf(e, v.w, acc[k][4 * i + 3]);
-                        }
-                }
-            }
-            // Out through shared memory (Q, K and V are through), so that a store writes whole rows of the warp's columns: a thread's
-            // own 16 bytes at a time took 1800 clk.
+            // A group at a time: this part's columns as they are, out of tensor memory, and the others' on top.  (One group ahead: all
+            // of them held beside the others' values, and through the barrier, made the kernel spill.)  Out through shared memory
+            // (Q, K and V are through), so that a store writes whole rows of the warp's columns: a thread's own 16 bytes at a time
+            // took 1800 clk.
             constexpr int PITCH = TAKES * GROUP * 2 + 16;
             const uint32_t tile = smem_u32(smem) + warp * 32 * PITCH;
             const long long eoff = w.b * p.o_stride_b + w.q0 * p.o_stride_t + (long long)w.h * HD + my_first * GROUP;
+            const uint32_t tO = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + C::COL_O + my_first * GROUP;
+            const bool any = w.hi > w.lo;
+            uint32_t mine[2][GROUP];
+            if (any && my_count > 0) tmem_ld16(tO, mine[0]);
 #pragma unroll
             for (int k = 0; k < TAKES; ++k) {
+                tmem_wait_ld();
+                if (any && k + 1 < my_count) tmem_ld16(tO + (k + 1) * GROUP, mine[(k + 1) & 1]);
+                float acc[GROUP];
+#pragma unroll
+                for (int e = 0; e < GROUP; ++e) acc[e] = own > 0.f ? __uint_as_float(mine[k & 1][e]) * own : 0.f;  // (an empty part's columns may hold anything)
+#pragma unroll
+                for (int s = 1; s < PARTS; ++s) {
+                    const float e = weight[s] * iz;
+                    if (e > 0.f) {  // (an empty part's record may hold anything)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 v = t[s - 1][k][i];
+                            acc[4 * i] = fmaf(e, v.x, acc[4 * i]), acc[4 * i + 1] = fmaf(e, v.y, acc[4 * i + 1]);
+                            acc[4 * i + 2] = fmaf(e, v.z, acc[4 * i + 2]), acc[4 * i + 3] = fmaf(e, v.w, acc[4 * i + 3]);
+                        }
+                    }
+                }
                 uint32_t o[GROUP / 2];
 #pragma unroll
-                for (int i = 0; i < GROUP / 2; ++i) o[i] = pack_bf16x2(acc[k][2 * i], acc[k][2 * i + 1]);
+                for (int i = 0; i < GROUP / 2; ++i) o[i] = pack_bf16x2(acc[2 * i], acc[2 * i + 1]);
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + lane * PITCH + k * 32 + i * 16), "r"(o[4 * i]), "r"(o[4 * i + 1]), "r"(o[4 * i + 2]), "r"(o[4 * i + 3]) : "memory");
