@@ -378,6 +378,36 @@ def test_parts_of_the_key_range(parts, batch, seq, kv, nq, nkv, window):
     assert ops.device_status() == (0, 0)
 
 
+@pytest.mark.parametrize("parts", [2, 3, 4, 8])
+@pytest.mark.parametrize("batch,seq,kv,nq,nkv,window", [
+    (1, 300, 900, 8, 4, oracle.INT_MAX),  # three row tiles of pairs of heads
+    (1, 256, 700, 3, 3, 200),             # odd group, a window: parts whose keys some rows do not see
+])
+def test_vision_blocks_in_parts(parts, batch, seq, kv, nq, nkv, window):
+    """Two and three parts in a cluster, four and eight with a merge launch, gated and not, as the whole range gives them; the whole
+    range against the oracle."""
+    from arcaine_b200 import ops
+    ops.clear_device_status()
+    q, k, v, g = (seeded_bf16(batch, n, h, 256, seed=150 + i) for i, (n, h) in enumerate([(seq, nq), (kv, nkv), (kv, nkv), (seq, nq)]))
+    ids = torch.full((kv,), -1, dtype=torch.int32)
+    for i, (a, b) in enumerate([(kv - seq + 10, kv - seq + 90), (kv - seq + 127, kv - seq + 129), (kv - seq + 130, kv - 20)]):
+        ids[a:b] = i
+    run = lambda n, gate: ops.sdpa_prefill(q.cuda(), k.cuda(), v.cuda(), scale=0.0625, mask_type=3, window=window, num_splits=n,  # noqa: E731
+                                           gate=g.cuda() if gate else None, block_ids=ids.cuda())
+    mask = oracle.fill_causal_mask_with_block_ids(ids.numpy(), seq, kv, kv - seq, window)
+    rows = sorted({t * nq + h for t in (0, 9, 10, 89, 127, 128, 129, 200, seq - 1) for h in (0, nq - 1)})
+    for gate in (False, True):
+        whole = run(1, gate)
+        want = oracle.sdpa_f32(q[0], k[0], v[0], scale=0.0625, mask_type=1, mask=mask, rows=rows, gate=g[0] if gate else None)
+        assert_close(whole[0].reshape(-1, 256)[rows], want[1].float() if gate else want[0], "whole")
+        before = ops.launch_count()
+        got = run(parts, gate)
+        assert ops.launch_count() - before == (1 if parts <= 3 else 2)
+        assert_close(got, whole.float().cpu(), f"gate {gate}", rel_tol=4e-3, abs_tol=1.6e-2)
+        assert torch.equal(run(parts, gate), got)
+    assert ops.device_status() == (0, 0)
+
+
 @pytest.mark.parametrize("batch,seq,kv,nq,nkv,window", [
     (1, 128, 1000, 16, 8, oracle.INT_MAX),  # every row of both tiles, the last key block ragged
     (1, 200, 1500, 3, 3, oracle.INT_MAX),   # odd group, 256 tokens a unit: the second tile ragged
