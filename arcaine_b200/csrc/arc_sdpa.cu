@@ -169,16 +169,16 @@ static int device_state(DeviceState** out) {
             }
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, true>, s.smem_optin - kDecodeStaticSmem));
-            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, true, false>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 1, true, true>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, true>, s.smem_optin - kDecodeStaticSmem));
-            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, true, false>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<128, 2, true, true>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, true>, s.smem_optin - kDecodeStaticSmem));
-            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, true, false>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 1, true, true>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, false>, s.smem_optin - kDecodeStaticSmem));
             ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, true>, s.smem_optin - kDecodeStaticSmem));
-            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, true, false>, s.smem_optin - kDecodeStaticSmem));
+            ARC_CUDA(opt_in_smem(sdpa_decode_kernel<256, 2, true, true>, s.smem_optin - kDecodeStaticSmem));
             for (int size = 1; size <= 8; ++size)
                 s.decode_clusters[size] = clusters_at_once(sdpa_decode_kernel<256, 1, true>, size, s.sm_count, 288, s.smem_optin - kDecodeStaticSmem);
             s.ready.store(true, std::memory_order_release);
@@ -765,7 +765,7 @@ static void plan_decode_cluster(const arc_sdpa_decode_params* p, const DeviceSta
     }
     DecodePlan one = *plan;
     // (The records the CTA finishes have a place of their own: they come while it still works.  Its warps' records go where
-    // the stages were, at least two: 32 * hd floats a warp, at most 16 * (hd + 5) needed.)
+    // the stages were, of which there are at least two.)
     const int rows = heads * G;
     const int extra = 64 + 8 * ((rows + 1) & ~1) * 8 + csize * rows * (p->hd / finishers) * 4 + rows * 32;
     if (!size_decode_cta(p->hd, heads, slices, 0, extra, ds.smem_optin, &one)) return;
@@ -852,9 +852,9 @@ static int launch_decode(const arc_sdpa_decode_params* p, const DecodePlan& plan
         kp.out_f32 = p->out_f32;
         kp.out_lse = p->out_lse;
         kp.o_stride_b = p->o_stride_b;
-        const bool even = (plan.ncta & (plan.ncta - 1)) == 0;
-        auto kernel = plan.nt == 1 ? (even ? sdpa_decode_kernel<HD, 1, true> : sdpa_decode_kernel<HD, 1, true, false>)
-                                   : (even ? sdpa_decode_kernel<HD, 2, true> : sdpa_decode_kernel<HD, 2, true, false>);
+        const bool alone = plan.ncta == 1;
+        auto kernel = plan.nt == 1 ? (alone ? sdpa_decode_kernel<HD, 1, true, true> : sdpa_decode_kernel<HD, 1, true>)
+                                   : (alone ? sdpa_decode_kernel<HD, 2, true, true> : sdpa_decode_kernel<HD, 2, true>);
         grid.z = (unsigned)p->batch;
         ARC_CUDA(launch_dependent(kernel, grid, dim3(threads), (size_t)plan.smem_bytes, stream, plan.ncta, tk, tv, kp));
         g_launches.fetch_add(1, std::memory_order_relaxed);

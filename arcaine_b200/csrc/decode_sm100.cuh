@@ -103,8 +103,8 @@ __device__ __forceinline__ void consumer_sync(int consumer_warps) {
     asm volatile("bar.sync 1, %0;" ::"r"(consumer_warps * 32) : "memory");
 }
 
-// CLUSTER: a cluster of CTAs owns one sequence (grid.z) and one group of KV heads (grid.y); its CTAs take equal parts of
-// the sequence's keys, fold their slices as above, send the records to the shared memory of the CTAs that finish them
+// CLUSTER: a cluster of CTAs owns one sequence (grid.z) and one group of KV heads (grid.y); its CTAs take a step of the
+// sequence's keys each, in order, and equal parts of the rest, fold their slices as above, send the records to the shared memory of the CTAs that finish them
 // and write the result: one launch, no records in global memory, no merge kernel.  For calls so small that the
 // launches are what they cost; otherwise equal shares over all SMs win.
 // What bounds it: a chain of latencies, and behind the last key instructions that run once, fetched cold at 6 clk each.  One token
@@ -116,10 +116,10 @@ __device__ __forceinline__ void consumer_sync(int consumer_warps) {
 // A CTA's first keys are asked for while the lengths are: they do not depend on them (1630 clk to the lengths when they are on the
 // device; us: 16 sequences of 500 keys, 8/4 heads of 128, 6.6 -> 5.9, 32 of 64 to 400, 24/4 of 256, 12.9 -> 11.9, twelve of up to 6000,
 // 16/2 of 128, 11.8 -> 11.2, one token over 513 keys 5.34 -> 5.1).  The scores ahead of V, on a barrier of its own, brought nothing.
-// EVEN (of CLUSTER): a power of two of CTAs, all of which finish columns.  As a case of the other instance these calls were 0.1
-// to 0.2 us slower (one token of 24/4 heads over 256 / 1001 keys 6.31 / 6.96 us, 6.16 / 6.76 so; 16 sequences of 500 keys,
-// 8/4 heads of 128: 7.92 and 7.70).
-template <int HD, int NT, bool CLUSTER, bool EVEN = true>
+// ALONE (of CLUSTER): one CTA, which is not launched as a cluster.  (Clusters of a power of two, all of whose CTAs finish columns, had an
+// instance of their own with it while records were folded another way; now they are faster as a case of the general one, us: one token of
+// 24/4 heads over 256 / 513 / 1001 keys 4.62 / 5.21 / 5.50 -> 4.47 / 5.11 / 5.42, 16 sequences of 500 keys, 8/4 heads of 128, 5.80 -> 5.65.)
+template <int HD, int NT, bool CLUSTER, bool ALONE = false>
 __global__ void __launch_bounds__(288, 1)
     sdpa_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const DecodeParams p) {
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(288, 1)
     // CLUSTER: the first 2^k CTAs of the cluster (all of 1, 2, 4 or 8, four of six) finish an equal number of columns of all
     // heads each.  All CTAs send them what they have, weights still to come: per CTA [query head of the group][column], in front
     // of them [CTA][query head] maximum (log2 domain) and sum, and whether all of the CTA's waits ended well.
-    const int dc_log2 = (HD == 256 ? 8 : 7) - (!CLUSTER ? 0 : EVEN ? __ffs(p.ncta) - 1 : 31 - __clz(p.ncta)), dc = 1 << dc_log2;
+    const int dc_log2 = (HD == 256 ? 8 : 7) - (CLUSTER && !ALONE ? 31 - __clz(p.ncta) : 0), dc = 1 << dc_log2;
     const int finishers = HD >> dc_log2;
     const int rows = p.nkv_cta * G, rows2 = (rows + 1) & ~1;
     uint64_t* gathered = empty + p.stages;
@@ -478,6 +478,7 @@ __global__ void __launch_bounds__(288, 1)
                 float* rec = reinterpret_cast<float*>(stage_base);                     // [warp][NT * 8 heads][RS]
                 float2* rec_ml = reinterpret_cast<float2*>(rec + (size_t)ncw * NT * 8 * RS);  // [warp][NT * 8]
                 float* rec_w = reinterpret_cast<float*>(rec_ml + ncw * NT * 8);
+                static_assert(NT * 8 * (RS + 3) <= 2 * 16 * HD, "a warp's records, sums and weights in its slices of K and V of two stages");
                 if (lane == 0 && (!ok || !work || fault != 0u)) *reinterpret_cast<volatile int*>(gave_up) = 1;  // (no result is written)
                 consumer_sync(ncw);  // every warp is through with the stages; no copy is in flight any more
 #pragma unroll
@@ -499,8 +500,7 @@ __global__ void __launch_bounds__(288, 1)
                     }
                 consumer_sync(ncw);
                 const uint32_t bar = smem_u32(gathered);
-                // (A CTA on its own is not launched as a cluster, and st.async is for clusters: plain stores there.)
-                const bool alone = EVEN && p.ncta == 1;
+                // (st.async is for clusters: plain stores where a CTA is alone.)
 #pragma unroll 1
                 for (int n0 = slice * 4; n0 < G; n0 += p.slices * 4) {  // four rows of the KV head a turn, a lane per slice
                     const int n = n0 + (lane >> 3), s = lane & 7, at = (s * p.nkv_cta + hl) * NT * 8 + n;
@@ -518,13 +518,13 @@ __global__ void __launch_bounds__(288, 1)
                     if (some) rec_w[at] = wt * 0.015625f;
                     float2* to = cml + blockIdx.x * rows2 + hl * G + n;
                     if (n < G && s < finishers) {
-                        if (alone) *to = make_float2(mx, z);
+                        if (ALONE) *to = make_float2(mx, z);
                         else st_async_f32x2(map_to_cta(smem_u32(to), s), make_float2(mx, z), map_to_cta(bar, s));
                     }
                 }
                 if (warp == 0 && lane < finishers) {
                     const float good = *reinterpret_cast<volatile int*>(gave_up) ? 0.f : 1.f;
-                    if (alone) cflag[0] = good;
+                    if (ALONE) cflag[0] = good;
                     else st_async_f32(map_to_cta(smem_u32(cflag + blockIdx.x), lane), good, map_to_cta(bar, lane));
                 }
                 consumer_sync(ncw);
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(288, 1)
                     }
                     float* at = crec + (size_t)(blockIdx.x * rows + hl * G + n) * dc + (d & (dc - 1));
                     const int to = d >> dc_log2;
-                    if (alone) *reinterpret_cast<float4*>(at) = acc;
+                    if (ALONE) *reinterpret_cast<float4*>(at) = acc;
                     else st_async_f32x4(map_to_cta(smem_u32(at), to), acc, map_to_cta(bar, to));
                 }
                 break;
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(288, 1)
     if constexpr (CLUSTER) {
         // This CTA's columns, two a thread, once every record is in its own shared memory.  (Nothing is sent to a CTA that
         // finishes none, and what this one has sent is waited for by those it went to: no barrier of the cluster here.)
-        if (!EVEN && (int)(blockIdx.x << dc_log2) >= HD) return;
+        if (!ALONE && (int)(blockIdx.x << dc_log2) >= HD) return;
         const int items = rows * (dc / 2), b = blockIdx.z;
         auto offset_of = [&](int item) {
             return (long long)b * p.o_stride_b + (long long)(head0 * G + (item >> (dc_log2 - 1))) * HD + blockIdx.x * dc + (item & (dc / 2 - 1)) * 2;
@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(288, 1)
         __syncwarp();
         // Whether the records came is settled for the whole CTA before any warp goes on: each warp waits by its own clock, and
         // one that gave up stood at the cluster's barrier while another, whose last look found them, stood at the CTA's.
-        const bool came = (EVEN && p.ncta == 1) || mbar_wait_cluster(gathered, 0);
+        const bool came = ALONE || mbar_wait_cluster(gathered, 0);
         if (!__syncthreads_and(came)) {
             if (!came && lane == 0) report_fault(p.fault, FAULT_WAIT_FULL, 0x10000u);
             cluster_sync_all();  // (what is still under way here arrives before the other CTAs have gone)
