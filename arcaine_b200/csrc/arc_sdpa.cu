@@ -618,7 +618,8 @@ static int launch_prefill(const arc_sdpa_prefill_params* p, const PrefillPlan& p
         kp.long_first = !split && p->mask_type != ARC_MASK_NONE && units > ds->wide.pairs && stays_in_l2(p, units < 8LL * ds->wide.pairs);
         // A few waves: with k whole ones, the pairs that get k units may as well have the longest and leave the rest, which are
         // shorter, to those that get k + 1.  (2048 queries over 5049 keys, 24 heads: 192 units of 25 to 40 blocks on 74 pairs, the fullest with
-        // 96 blocks in one list and 91 so, 84 on average: 165 -> 147 us on a cool chip; 8192 tokens of 24/4 191 -> 184, a vision prompt 25.1 -> 24.7.)
+        // 96 blocks in one list and 91 so, 84 on average: 153 -> 147 us, gated 165 -> 158; 1664 tokens of 24/4 34.0 -> 32.5.  Vision prompts of
+        // 96 to 160 units, and 8192 tokens of 24/4 behind a window of 1024, as fast either way.)
         const long long pairs = ds->wide.pairs, whole = units / pairs, extra = units % pairs;
         if (kp.long_first && !masked && extra > 0 && whole <= 8) {
             const int tiles = kp.head_pair ? 1 : 2;

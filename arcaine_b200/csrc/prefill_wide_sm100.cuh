@@ -196,9 +196,9 @@ __device__ __forceinline__ void wide_blocks(const PrefillParams& p, int q_first,
 }
 
 // Position of a CTA pair in the list of units.  Plain order: token tiles fastest, then heads, then sequences (pairs that
-// run side by side share K and V in L2).  long_first (causal without a window, several waves): the units with most key
-// blocks first, all heads of a token tile together, and every second wave in reverse order, so that the sums of a
-// pair's units are about equal.
+// run side by side share K and V in L2).  long_first (causal, with a window or not, more units than pairs,
+// whose keys and values stay in L2): the units with most key blocks first, all heads of a token tile together, and every second wave in
+// reverse order, so that the sums of a pair's units are about equal.
 // few > 0: the first `few` pairs share the longest units [0, few_end) in that way and the others the rest, of which they take
 // one more each.
 template <bool ONE>  // one unit a pair: the walk ends behind it
@@ -269,7 +269,7 @@ __device__ __forceinline__ void wide_find_blocks(const PrefillParams& p, int ran
 // read out of the other CTAs' shared memory, 11 bytes per clk and SM, the fold took 5 us.  Every instruction here runs
 // once per launch and is fetched cold, 50 clk per 128 bytes of code, so there are few: with rows divided instead of columns, which
 // had to go through shared memory on either side, 13000 clk passed from the last P V to the end  (us: 256 queries of 16 heads over
-// 2304 keys 18.0 -> 15.7, 512 over 2560 23.5 -> 20.7, 512 of 8 heads over 1512 15.5 -> 13.1.)
+// 2304 keys 18.0 -> 15.5, 512 over 2560 23.5 -> 21.4, 512 of 8 heads over 1512 15.5 -> 12.6.)
 // SEVERAL: pairs take several units.  EARLY (SEVERAL, not gated): the epilogue empties the accumulator into registers first (1600 clk), for the
 // next unit's P V to go on; in turns, with the way out of the SM between them, it took 3000.  (2 x 5000 tokens of 16/8 heads,
 // window 512, 103 -> 96 us.  Gated rows wait for sigmoids, not for the way out: taken early they cost calls of short units 8 %.)
